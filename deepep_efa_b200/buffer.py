@@ -397,8 +397,9 @@ class Buffer:
                                       topk_weights, expert_alignment, num_worst_tokens)
         req = _DispatchReq(x, handle, num_tokens_per_rank, is_token_in_rank, num_tokens_per_expert, topk_idx, topk_weights,
                            expert_alignment, num_worst_tokens, quantize_fp8, round_scale)
-        config = self.get_dispatch_config(self.group_size) if config is None else config
-        return _dispatch_many([self], [req], config, previous_event, async_finish, allocate_on_comm_stream)[0]
+        own_config = config is not None
+        config = config if own_config else self.get_dispatch_config(self.group_size)
+        return _dispatch_many([self], [req], config, previous_event, async_finish, allocate_on_comm_stream, own_config)[0]
 
     def combine(self, x: torch.Tensor, handle: Tuple, topk_weights: Optional[torch.Tensor] = None,
                 bias: Union[torch.Tensor, Tuple[torch.Tensor, torch.Tensor], None] = None, config: Optional[Config] = None,
@@ -414,9 +415,10 @@ class Buffer:
             return self.internode_combine(x, handle, topk_weights, bias, config, previous_event, async_finish, allocate_on_comm_stream)
         if self._cpu is not None:
             return self._cpu.combine(x, handle, topk_weights, bias)
-        config = self.get_combine_config(self.group_size) if config is None else config
+        own_config = config is not None
+        config = config if own_config else self.get_combine_config(self.group_size)
         return _combine_many([self], [(x, handle, topk_weights, bias)], config, previous_event, async_finish,
-                             allocate_on_comm_stream)[0]
+                             allocate_on_comm_stream, own_config)[0]
 
     # Groups that span several NVLink domains (the reference's "internode" paths).
     def internode_dispatch(self, x, handle: Optional[Tuple] = None, num_tokens_per_rank: Optional[torch.Tensor] = None,
@@ -653,7 +655,11 @@ class _CommScope:
 
     On entry the communication stream waits for ``previous_event`` (or for the caller's stream). Inside the block the
     communication stream is current. On exit either an event is returned (``async_finish``) and the inputs are kept
-    safe with ``record_stream``, or the caller's stream waits for the communication stream."""
+    safe with ``record_stream``, or the caller's stream waits for the communication stream.
+
+    A call without ``previous_event`` and without ``async_finish`` is ordered behind the caller's stream on both sides, so it
+    runs on that stream itself (``direct``): no events, no ``record_stream``, and no hop between two streams, which costs the
+    GPU a few microseconds per hop. The native call keeps it in order with calls on the communication stream."""
 
     def __init__(self, buf: Buffer, previous_event, async_finish, allocate_on_comm_stream, inputs=()):
         if allocate_on_comm_stream:
@@ -664,6 +670,7 @@ class _CommScope:
         self._outputs: List[torch.Tensor] = []
         self._early_outputs: List[torch.Tensor] = []
         self.event = EventOverlap()
+        self.direct = not async_finish and (previous_event is None or previous_event.event is None or previous_event.event.event is None)
 
     def outputs(self, *tensors):
         self._outputs.extend(t for t in tensors if isinstance(t, torch.Tensor))
@@ -677,6 +684,8 @@ class _CommScope:
         self._early_outputs.extend(t for t in tensors if isinstance(t, torch.Tensor))
 
     def __enter__(self):
+        if self.direct:
+            return self
         self.compute = torch.cuda.current_stream()
         comm = self.buf.comm_stream
         if self.prev is not None and self.prev.event is not None and self.prev.event.event is not None:
@@ -688,6 +697,8 @@ class _CommScope:
         return self
 
     def __exit__(self, et, ev, tb):
+        if self.direct:
+            return False
         comm = self.buf.comm_stream
         self._ctx.__exit__(et, ev, tb)
         if et is not None:
@@ -735,130 +746,87 @@ def _clamp_sms(num_sms: int, num_virtual: int) -> int:
     return num_sms if num_virtual == 1 else max(1, min(num_sms, _NUM_SM_B200 // num_virtual - 1))
 
 
+def _normal_sms(config: Config, own_config: bool, bufs: List[Buffer]) -> int:
+    """CTAs of a normal-mode kernel. The configs share the GPU between communication and compute and are tuned for NVLink, which
+    a few dozen SMs saturate. With one rank nothing crosses NVLink: the kernels are copies within this GPU's memory, and unless
+    the caller asked for a share of the SMs with a config of their own they take all of them (4096 x 7168 BF16 cast to FP8 and
+    summed back on one B200: dispatch 80 -> 23 us, combine 94 -> 25 us from 32 to 148 CTAs)."""
+    if bufs[0].group_size == 1 and not own_config:
+        return _NUM_SM_B200
+    return _clamp_sms(config.num_sms if config.num_sms > 0 else Buffer.num_sms, len(bufs))
+
+
 def _dispatch_many(bufs: List[Buffer], reqs: List[_DispatchReq], config: Config, previous_event, async_finish,
-                   allocate_on_comm_stream):
+                   allocate_on_comm_stream, own_config: bool = True):
     C = bufs[0]._C
     rts = [b.runtime for b in bufs]
-    V = len(bufs)
-    R = bufs[0].group_size
     for b in bufs:
         b.check_status()
     inputs = []
     for q in reqs:
         inputs += list(q.x) if isinstance(q.x, tuple) else [q.x]
         inputs += [q.topk_idx, q.topk_weights, q.is_token_in_rank, q.num_tokens_per_rank, q.num_tokens_per_expert]
-    num_sms = _clamp_sms(config.num_sms if config.num_sms > 0 else Buffer.num_sms, V)
+    num_sms = _normal_sms(config, own_config, bufs)
     num_channels = max(1, min(config.num_sms // 2 if config.num_sms >= 2 else 1, 128))
     cached = reqs[0].handle is not None
-    worst = reqs[0].num_worst_tokens
-    results = []
-    with _CommScope(bufs[0], previous_event, async_finish, allocate_on_comm_stream, inputs) as scope, nvtx_range("ep.dispatch"):
+    calls = []
+    for b, q in zip(bufs, reqs):
         if cached:
-            metas = []
-            for q in reqs:
-                assert q.topk_idx is None and q.topk_weights is None, "cached dispatch carries no top-k data"
-                rpm, cpm, rcpm, recv_src_idx, itir, send_head = q.handle
-                if _DEBUG_CHECKS:
-                    validate_handle(q.handle, bufs[len(metas)].rank, R)
-                metas.append((rpm, cpm, rcpm, send_head, itir, recv_src_idx.size(0), []))
+            assert q.topk_idx is None and q.topk_weights is None, "cached dispatch carries no top-k data"
+            if _DEBUG_CHECKS:
+                validate_handle(q.handle, b.rank, b.group_size)
         else:
-            for q in reqs:
-                assert q.num_tokens_per_rank is not None and q.is_token_in_rank is not None and q.num_tokens_per_expert is not None
-            num_experts = reqs[0].num_tokens_per_expert.numel()
-            outs = C.notify(rts, [q.num_tokens_per_rank for q in reqs], [q.num_tokens_per_expert for q in reqs],
-                            [q.is_token_in_rank for q in reqs], num_channels, reqs[0].expert_alignment)
-            metas = []
-            for b, q, (rpm, cpm, rcpm, send_head) in zip(bufs, reqs, outs):
-                if worst > 0:
-                    n_recv, per_expert = worst, []
-                else:
-                    n_recv, per_expert = b.runtime.wait_recv_counts(num_experts // R)
-                metas.append((rpm, cpm, rcpm, send_head, q.is_token_in_rank, n_recv, per_expert))
-        num_experts = reqs[0].num_tokens_per_expert.numel() if not cached else R  # only used for local-id remap
-        per_rank, outs_all = [], []
-        for b, q, (rpm, cpm, rcpm, send_head, itir, n_recv, per_expert) in zip(bufs, reqs, metas):
-            x, x_scales = q.x if isinstance(q.x, tuple) else (q.x, None)
-            x = x.contiguous()
-            if x_scales is not None:
-                x_scales = x_scales.contiguous()  # the reference's tests pass column-major scales (tests/test_intranode.py:29)
-            H = x.size(1)
-            rt = b.runtime
-            quant = q.quantize_fp8
-            out_dtype = torch.float8_e4m3fn if quant else x.dtype
-            recv_x = rt.alloc_symmetric([n_recv, H], out_dtype)
-            recv_scales = rt.alloc_symmetric([n_recv, H // 128], torch.float32) if (quant or x_scales is not None) else None
-            K = q.topk_idx.size(1) if q.topk_idx is not None else 0
-            recv_topk_idx = rt.alloc_symmetric([n_recv, K], torch.int64) if q.topk_idx is not None else None
-            recv_topk_w = rt.alloc_symmetric([n_recv, K], torch.float32) if q.topk_weights is not None else None
-            if cached:
-                recv_src_idx = rt.alloc_symmetric([n_recv], torch.int32)  # rewritten with identical content
-            else:
-                recv_src_idx = rt.alloc_symmetric([n_recv], torch.int32)
-            per_rank.append((x, x_scales, q.topk_idx, q.topk_weights, send_head, rpm, recv_x, recv_scales, recv_topk_idx,
-                             recv_topk_w, recv_src_idx))
-            outs_all.append((recv_x, recv_scales, recv_topk_idx, recv_topk_w, recv_src_idx, rpm, cpm, rcpm, send_head, itir,
-                             per_expert))
-            scope.outputs(rpm, cpm, rcpm, send_head)
-        C.dispatch(rts, per_rank, num_experts, reqs[0].quantize_fp8, reqs[0].round_scale, worst, num_sms)
-    for q, o in zip(reqs, outs_all):
-        recv_x, recv_scales, recv_topk_idx, recv_topk_w, recv_src_idx, rpm, cpm, rcpm, send_head, itir, per_expert = o
+            assert q.num_tokens_per_rank is not None and q.is_token_in_rank is not None and q.num_tokens_per_expert is not None
+        x, x_scales = q.x if isinstance(q.x, tuple) else (q.x, None)
+        calls.append((x, x_scales, q.num_tokens_per_rank, q.num_tokens_per_expert, q.is_token_in_rank, q.topk_idx, q.topk_weights, q.handle))
+    q0 = reqs[0]
+    with _CommScope(bufs[0], previous_event, async_finish, allocate_on_comm_stream, inputs) as scope, nvtx_range("ep.dispatch"):
+        outs = C.normal_dispatch(rts, calls, num_channels, q0.expert_alignment, q0.quantize_fp8, q0.round_scale,
+                                 0 if cached else q0.num_worst_tokens, num_sms)
+        if not cached:
+            for o in outs:
+                rpm, cpm, rcpm, _, _, send_head = o[5]
+                scope.outputs(rpm, cpm, rcpm, send_head)
+    results = []
+    for recv_x, recv_scales, recv_topk_idx, recv_topk_w, per_expert, handle in outs:
         rx = (recv_x, recv_scales) if recv_scales is not None else recv_x
         if cached:
             results.append((rx, None, None, None, None, scope.event))
         else:
-            handle = (rpm, cpm, rcpm, recv_src_idx, itir, send_head)
             results.append((rx, recv_topk_idx, recv_topk_w, per_expert, handle, scope.event))
     return results
 
 
-def _combine_many(bufs: List[Buffer], calls, config: Config, previous_event, async_finish, allocate_on_comm_stream):
+def _combine_many(bufs: List[Buffer], calls, config: Config, previous_event, async_finish, allocate_on_comm_stream, own_config: bool = True):
     C = bufs[0]._C
     rts = [b.runtime for b in bufs]
-    V = len(bufs)
     for b in bufs:
         b.check_status()
-    num_sms = _clamp_sms(config.num_sms if config.num_sms > 0 else Buffer.num_sms, V)
-    inputs = []
-    for x, handle, w, bias in calls:
-        inputs += [x, w] + list(Buffer._unpack_bias(bias))
-    results, per_rank, keep = [], [], []
-    # results are allocated here, on the caller's stream (see _CommScope.outputs_from_caller_stream)
-    early = []
-    if not allocate_on_comm_stream:
-        for x, handle, w, bias in calls:
-            T = handle[5].size(0)
-            early.append((torch.empty((T, x.size(1)), dtype=torch.bfloat16, device=x.device),
-                          torch.empty((T, w.size(1)), dtype=torch.float32, device=x.device) if w is not None else None))
-    with _CommScope(bufs[0], previous_event, async_finish, allocate_on_comm_stream, inputs) as scope, nvtx_range("ep.combine"):
-        for ci, (b, (x, handle, w, bias)) in enumerate(zip(bufs, calls)):
-            rpm, _, _, src_idx, _, send_head = handle
-            if _DEBUG_CHECKS:
-                validate_handle(handle, b.rank, b.group_size)
-            rt = b.runtime
-            assert x.dim() == 2 and x.dtype == torch.bfloat16 and x.size(0) == src_idx.size(0)
-            if rt.symmetric_offset(x) < 0:
-                xs = rt.alloc_symmetric(list(x.shape), x.dtype)
-                xs.copy_(x)
-                x = xs
-            if w is not None and rt.symmetric_offset(w) < 0:
-                ws = rt.alloc_symmetric(list(w.shape), torch.float32)
-                ws.copy_(w)
-                w = ws
-            keep += [x, w]
-            b0, b1 = Buffer._unpack_bias(bias)
+    num_sms = _normal_sms(config, own_config, bufs)
+    inputs, per_rank = [], []
+    scope = _CommScope(bufs[0], previous_event, async_finish, allocate_on_comm_stream)
+    for b, (x, handle, w, bias) in zip(bufs, calls):
+        rpm, _, _, src_idx, _, send_head = handle
+        if _DEBUG_CHECKS:
+            validate_handle(handle, b.rank, b.group_size)
+        assert x.dim() == 2 and x.dtype == torch.bfloat16 and x.size(0) == src_idx.size(0)
+        b0, b1 = Buffer._unpack_bias(bias)
+        inputs += [x, w, b0, b1]
+        out = out_w = None
+        if not scope.direct and not allocate_on_comm_stream:
+            # results are allocated here, on the caller's stream (see _CommScope.outputs_from_caller_stream)
             T = send_head.size(0)
-            if early:
-                out, out_w = early[ci]
-                scope.outputs_from_caller_stream(out, out_w)
-            else:
-                out = torch.empty((T, x.size(1)), dtype=torch.bfloat16, device=x.device)
-                out_w = torch.empty((T, w.size(1)), dtype=torch.float32, device=x.device) if w is not None else None
+            out = torch.empty((T, x.size(1)), dtype=torch.bfloat16, device=x.device)
+            out_w = torch.empty((T, w.size(1)), dtype=torch.float32, device=x.device) if w is not None else None
+            scope.outputs_from_caller_stream(out, out_w)
+        per_rank.append((x, w, send_head, rpm, b0, b1, out, out_w))
+    scope.inputs = [t for t in inputs if t is not None]
+    with scope, nvtx_range("ep.combine"):
+        results = C.normal_combine(rts, per_rank, num_sms)
+        if allocate_on_comm_stream:
+            for out, out_w in results:
                 scope.outputs(out, out_w)
-            per_rank.append((x, w, send_head, rpm, b0, b1, out, out_w))
-            results.append([out, out_w])
-        C.combine(rts, per_rank, num_sms)
-    del keep
-    return [(o, ow, scope.event) for o, ow in results]
+    return [(out, out_w, scope.event) for out, out_w in results]
 
 
 def _parity_of(views, src_info: torch.Tensor) -> int:

@@ -39,25 +39,36 @@ struct Runtime {
     void open_peers(const std::vector<std::string>& handles) { core->open_peers(handles); }
     void set_comm_stream(int64_t s) { comm_stream = reinterpret_cast<cudaStream_t>(s); }
 
+    // A block of the arena; its memory returns when the last tensor in it dies.
+    struct Block {
+        std::shared_ptr<RuntimeCore> core;
+        uint64_t off;
+        cudaStream_t comm;
+        Block(std::shared_ptr<RuntimeCore> c, uint64_t bytes, cudaStream_t s) : core(std::move(c)), off(core->arena_alloc(bytes)), comm(s) {}
+        Block(const Block&) = delete;
+        ~Block() {
+            cudaStream_t streams[2];
+            int n = 0;
+            try {
+                streams[n] = c10::cuda::getCurrentCUDAStream(core->device()).stream();
+                ++n;
+            } catch (...) {
+            }
+            if (comm != nullptr) streams[n++] = comm;
+            core->arena_release(off, streams, n);
+        }
+    };
+    using BlockPtr = std::shared_ptr<Block>;
+    BlockPtr alloc_block(uint64_t bytes) { return std::make_shared<Block>(core, bytes, comm_stream); }
+    torch::Tensor tensor_in(const BlockPtr& block, uint64_t byte_off, at::IntArrayRef sizes, torch::ScalarType dtype) {
+        return torch::from_blob(reinterpret_cast<char*>(core->base()) + block->off + byte_off, sizes, [block](void*) {},
+                                torch::TensorOptions().dtype(dtype).device(torch::kCUDA, core->device()));
+    }
+
     torch::Tensor alloc_symmetric(std::vector<int64_t> sizes, torch::ScalarType dtype) {
         int64_t numel = 1;
         for (auto s : sizes) numel *= s;
-        const uint64_t bytes = (uint64_t)numel * c10::elementSize(dtype);
-        const uint64_t off = core->arena_alloc(bytes);
-        void* p = reinterpret_cast<char*>(core->base()) + off;
-        auto keep = core;
-        cudaStream_t comm = comm_stream;
-        const int dev = core->device();
-        auto deleter = [keep, off, comm, dev](void*) {
-            std::vector<cudaStream_t> streams;
-            try {
-                streams.push_back(c10::cuda::getCurrentCUDAStream(dev).stream());
-            } catch (...) {
-            }
-            if (comm != nullptr) streams.push_back(comm);
-            keep->arena_release(off, streams);
-        };
-        return torch::from_blob(p, sizes, deleter, torch::TensorOptions().dtype(dtype).device(torch::kCUDA, dev));
+        return tensor_in(alloc_block((uint64_t)numel * c10::elementSize(dtype)), 0, sizes, dtype);
     }
 
     // Offset of a tensor inside the symmetric buffer, or -1 when it lives elsewhere.
@@ -76,16 +87,6 @@ struct Runtime {
         auto keep = core;
         return torch::from_blob(reinterpret_cast<char*>(core->base()) + off, sizes, [keep](void*) {},
                                 torch::TensorOptions().dtype(dtype).device(torch::kCUDA, core->device()));
-    }
-
-    std::pair<int, std::vector<int>> wait_recv_counts(int num_local_experts) {
-        std::vector<int> per;
-        int n;
-        {
-            py::gil_scoped_release rel;
-            n = core->wait_recv_counts(num_local_experts, &per);
-        }
-        return {n, per};
     }
 
     void set_mask(int rank_to_mask, bool mask) {
@@ -133,6 +134,17 @@ void check_launch(cudaError_t e, const char* what) {
     }
 }
 
+// One normal-mode call on the current stream, ordered behind the runtime's previous one (RuntimeCore::order_enter).
+struct OrderedCall {
+    RuntimeCore* core;
+    cudaStream_t stream;
+    bool counted;
+    explicit OrderedCall(Runtime* rt) : core(rt->core.get()), stream(cur_stream(rt)), counted(core->order_enter(stream)) {}
+    ~OrderedCall() {
+        if (counted) core->order_leave(stream);
+    }
+};
+
 // ---------------------------------------------------------------------------------------------
 // layout
 // ---------------------------------------------------------------------------------------------
@@ -157,159 +169,227 @@ std::tuple<torch::Tensor, torch::Tensor, torch::Tensor> get_dispatch_layout(Runt
     a.num_tokens_per_expert = per_expert.data_ptr<int>();
     a.is_token_in_rank = in_rank.data_ptr<bool>();
     a.scratch = rt->layout_scratch.data_ptr<int>();
-    check_launch(dx::launch_layout(a, cur_stream(rt)), "get_dispatch_layout");
+    OrderedCall order(rt);
+    check_launch(dx::launch_layout(a, order.stream), "get_dispatch_layout");
     return {per_rank, per_expert, in_rank};
 }
 
-// ---------------------------------------------------------------------------------------------
-// notify: per rank (num_tokens_per_rank, num_tokens_per_expert, is_token_in_rank)
-// returns per rank (rank_prefix_matrix, channel_prefix_matrix, recv_channel_prefix_matrix, send_head)
-// ---------------------------------------------------------------------------------------------
-using NotifyOut = std::tuple<torch::Tensor, torch::Tensor, torch::Tensor, torch::Tensor>;
-std::vector<NotifyOut> notify(std::vector<Runtime*> rts, std::vector<torch::Tensor> ntpr, std::vector<torch::Tensor> ntpe,
-                              std::vector<torch::Tensor> itir, int num_channels, int expert_alignment) {
-    const int V = (int)rts.size();
-    DX_CHECK(V >= 1 && V <= dx::kMaxVirtualRanks && (int)ntpr.size() == V && (int)ntpe.size() == V && (int)itir.size() == V, "notify: one entry per rank");
-    DX_CHECK(num_channels >= 1 && num_channels <= dx::kMaxChannels, "num_channels out of range");
-    DX_CHECK(expert_alignment >= 1, "expert_alignment must be >= 1");
-    c10::cuda::CUDAGuard guard(rts[0]->core->device());
-    std::vector<dx::NotifyArgs> args(V);
-    std::vector<NotifyOut> outs;
-    for (int v = 0; v < V; ++v) {
-        Runtime* rt = rts[v];
-        const int R = rt->core->num_ranks();
-        DX_CHECK(rt->core->available(), "runtime is not synchronised with its peers");
-        DX_CHECK(ntpr[v].scalar_type() == torch::kInt32 && ntpr[v].numel() == R && ntpr[v].is_contiguous(), "num_tokens_per_rank must be int32 [R]");
-        DX_CHECK(ntpe[v].scalar_type() == torch::kInt32 && ntpe[v].is_contiguous() && ntpe[v].numel() % R == 0, "num_tokens_per_expert must be int32 [E]");
-        DX_CHECK(itir[v].scalar_type() == torch::kBool && itir[v].dim() == 2 && itir[v].size(1) == R && itir[v].is_contiguous(), "is_token_in_rank must be bool [T,R]");
-        const int E = (int)ntpe[v].numel(), T = (int)itir[v].size(0);
-        DX_CHECK(E / R <= dx::kMaxLocalExperts, "too many local experts");
-        auto i32 = torch::TensorOptions().dtype(torch::kInt32).device(itir[v].device());
-        auto rpm = torch::empty({R, R}, i32), cpm = torch::empty({R, num_channels}, i32), rcpm = torch::empty({R, num_channels}, i32);
-        auto send_head = torch::empty({T, R}, i32);
-        rt->core->reset_recv_counters(E / R);
-        dx::NotifyArgs& a = args[v];
-        a.ctx = rt->core->ctx();
-        a.num_tokens_per_rank = ntpr[v].data_ptr<int>();
-        a.num_tokens_per_expert = ntpe[v].data_ptr<int>();
-        a.is_token_in_rank = itir[v].data_ptr<bool>();
-        a.num_tokens = T;
-        a.num_experts = E;
-        a.num_channels = num_channels;
-        a.expert_alignment = expert_alignment;
-        a.rank_prefix_matrix = rpm.data_ptr<int>();
-        a.channel_prefix_matrix = cpm.data_ptr<int>();
-        a.recv_channel_prefix_matrix = rcpm.data_ptr<int>();
-        a.send_head = send_head.data_ptr<int>();
-        dxh::HostWords* hw = reinterpret_cast<dxh::HostWords*>(a.ctx.status);  // status is the first member
-        a.host_recv_counter = &hw->recv_counter;
-        a.host_expert_counter = hw->expert_counter;
-        outs.emplace_back(rpm, cpm, rcpm, send_head);
-    }
-    check_launch(dx::launch_notify(args.data(), V, cur_stream(rts[0])), "notify");
-    return outs;
-}
-
-// ---------------------------------------------------------------------------------------------
-// dispatch. Per rank tuple:
-//  (x, x_scales|None, topk_idx|None, topk_weights|None, send_head, rank_prefix_matrix,
-//   recv_x, recv_scales|None, recv_topk_idx|None, recv_topk_weights|None, recv_src_idx)
-// ---------------------------------------------------------------------------------------------
 c10::optional<torch::Tensor> opt_tensor(const py::handle& h) {
     if (h.is_none()) return c10::nullopt;
     return h.cast<torch::Tensor>();
 }
 
-void dispatch(std::vector<Runtime*> rts, std::vector<py::tuple> per_rank, int num_experts, bool quantize, bool round_scale,
-              int num_worst_tokens, int num_sms) {
+// ---------------------------------------------------------------------------------------------
+// normal-mode dispatch: count exchange, host wait for the receive counts, outputs carved from the arena, dispatch kernel.
+// Per rank request: (x, x_scales|None, num_tokens_per_rank|None, num_tokens_per_expert|None, is_token_in_rank|None,
+//                    topk_idx|None, topk_weights|None, handle|None)
+// Per rank result:  (recv_x, recv_scales|None, recv_topk_idx|None, recv_topk_weights|None, rows per local expert (list),
+//                    (rank_prefix_matrix, channel_prefix_matrix, recv_channel_prefix_matrix, recv_src_idx, is_token_in_rank, send_head))
+// ---------------------------------------------------------------------------------------------
+struct DispatchCall {
+    torch::Tensor x, in_rank, rpm, cpm, rcpm, send_head;
+    c10::optional<torch::Tensor> x_scales, topk_idx, topk_w;
+    int T = 0, H = 0, K = 0, num_recv = 0;
+    torch::ScalarType out_type;
+    bool has_scales = false;
+    std::vector<int> per_expert;
+    // outputs: the payload in one block of the arena, the row metadata (part of which lives on in the handle) in another
+    Runtime::BlockPtr payload, meta;
+    uint64_t scales_at = 0, topk_w_at = 0, src_idx_at = 0;  // byte offsets inside the blocks
+
+    void allocate(Runtime* rt, int rows) {
+        const uint64_t x_bytes = (uint64_t)rows * H * c10::elementSize(out_type);
+        scales_at = dxh::align_up(x_bytes, 1024);
+        payload = rt->alloc_block(has_scales ? scales_at + (uint64_t)rows * (H / 128) * 4 : x_bytes);
+        const uint64_t idx_bytes = topk_idx.has_value() ? (uint64_t)rows * K * 8 : 0, w_bytes = topk_w.has_value() ? (uint64_t)rows * K * 4 : 0;
+        topk_w_at = dxh::align_up(idx_bytes, 128);
+        src_idx_at = dxh::align_up(topk_w_at + w_bytes, 128);
+        meta = rt->alloc_block(src_idx_at + (uint64_t)rows * 4);
+    }
+};
+
+void wait_counts(Runtime* rt, DispatchCall& q, int num_local_experts) {
+    py::gil_scoped_release rel;
+    q.num_recv = rt->core->wait_recv_counts(num_local_experts, &q.per_expert);
+}
+
+py::list normal_dispatch(std::vector<Runtime*> rts, const std::vector<py::tuple>& reqs, int num_channels, int expert_alignment, bool quantize,
+                         bool round_scale, int num_worst_tokens, int num_sms) {
     const int V = (int)rts.size();
-    DX_CHECK(V >= 1 && V <= dx::kMaxVirtualRanks && (int)per_rank.size() == V, "dispatch: one entry per rank");
+    DX_CHECK(V >= 1 && V <= dx::kMaxVirtualRanks && (int)reqs.size() == V, "dispatch: one entry per rank");
     DX_CHECK(num_sms >= 1, "num_sms must be >= 1");
+    DX_CHECK(num_channels >= 1 && num_channels <= dx::kMaxChannels, "num_channels out of range");
+    DX_CHECK(expert_alignment >= 1, "expert_alignment must be >= 1");
     c10::cuda::CUDAGuard guard(rts[0]->core->device());
-    std::vector<dx::DispatchArgs> args(V);
+    const int R = rts[0]->core->num_ranks();
+    std::vector<DispatchCall> calls(V);
+    std::vector<dx::NotifyArgs> nargs(V);
+    std::vector<dx::DispatchArgs> dargs(V);
+    OrderedCall order(rts[0]);
+    bool cached = false;
+    int E = R;  // a cached call carries no expert ids to remap
     for (int v = 0; v < V; ++v) {
         Runtime* rt = rts[v];
-        const py::tuple& t = per_rank[v];
-        DX_CHECK(t.size() == 11, "dispatch: per-rank tuple must have 11 entries");
-        const int R = rt->core->num_ranks();
-        auto x = t[0].cast<torch::Tensor>();
-        auto x_scales = opt_tensor(t[1]);
-        auto topk_idx = opt_tensor(t[2]);
-        auto topk_w = opt_tensor(t[3]);
-        auto send_head = t[4].cast<torch::Tensor>();
-        auto rpm = t[5].cast<torch::Tensor>();
-        auto recv_x = t[6].cast<torch::Tensor>();
-        auto recv_scales = opt_tensor(t[7]);
-        auto recv_topk_idx = opt_tensor(t[8]);
-        auto recv_topk_w = opt_tensor(t[9]);
-        auto recv_src_idx = t[10].cast<torch::Tensor>();
-        DX_CHECK(x.dim() == 2 && x.is_contiguous(), "x must be contiguous [T,hidden]");
-        const int T = (int)x.size(0), H = (int)x.size(1);
-        DX_CHECK((H * x.element_size()) % 16 == 0, "hidden bytes must be a multiple of 16");
-        DX_CHECK(send_head.scalar_type() == torch::kInt32 && send_head.is_contiguous() && send_head.size(0) == T && send_head.size(1) == R, "send_head must be int32 [T,R]");
-        DX_CHECK(rpm.scalar_type() == torch::kInt32 && rpm.is_contiguous() && rpm.numel() == R * R, "rank_prefix_matrix must be int32 [R,R]");
-        dx::DispatchArgs& a = args[v];
+        const py::tuple& t = reqs[v];
+        DispatchCall& q = calls[v];
+        DX_CHECK(t.size() == 8, "dispatch: per-rank tuple must have 8 entries");
+        DX_CHECK(rt->core->available(), "runtime is not synchronised with its peers");
+        q.x = t[0].cast<torch::Tensor>().contiguous();
+        q.x_scales = opt_tensor(t[1]);
+        if (q.x_scales.has_value()) q.x_scales = q.x_scales->contiguous();  // column-major scales are accepted (the reference's tests pass them)
+        q.topk_idx = opt_tensor(t[5]);
+        q.topk_w = opt_tensor(t[6]);
+        DX_CHECK(q.x.dim() == 2 && q.x.is_cuda(), "x must be [T,hidden] on the GPU");
+        q.T = (int)q.x.size(0);
+        q.H = (int)q.x.size(1);
+        const int T = q.T, H = q.H;
+        DX_CHECK((H * q.x.element_size()) % 16 == 0, "hidden bytes must be a multiple of 16");
+        q.has_scales = quantize || q.x_scales.has_value();
+        q.out_type = quantize ? torch::kFloat8_e4m3fn : q.x.scalar_type();
+        if (quantize) {
+            DX_CHECK(q.x.scalar_type() == torch::kBFloat16 && H % 128 == 0 && H <= 8192, "fused FP8 dispatch needs bf16 x with hidden % 128 == 0 and hidden <= 8192");
+        } else if (q.x_scales.has_value()) {
+            DX_CHECK(q.x.element_size() == 1 && q.x_scales->scalar_type() == torch::kFloat32 && q.x_scales->size(0) == T, "x_scales must be f32 [T,hidden/128]");
+            DX_CHECK(H % 128 == 0 && q.x_scales->size(1) == H / 128, "x_scales must have hidden/128 columns");
+        } else {
+            DX_CHECK(q.x.scalar_type() == torch::kBFloat16, "x must be bf16 (or an (e4m3, scales) pair)");
+        }
+        if (q.topk_idx.has_value()) {
+            DX_CHECK(q.topk_idx->scalar_type() == torch::kInt64 && q.topk_idx->is_contiguous() && q.topk_idx->dim() == 2 && q.topk_idx->size(0) == T, "topk_idx must be int64 [T,K]");
+            q.K = (int)q.topk_idx->size(1);
+            DX_CHECK(q.K <= dx::kMaxTopk, "num_topk too large");
+            if (q.topk_w.has_value())
+                DX_CHECK(q.topk_w->scalar_type() == torch::kFloat32 && q.topk_w->is_contiguous() && q.topk_w->numel() == q.topk_idx->numel(), "topk_weights must be f32 [T,K]");
+        } else {
+            DX_CHECK(!q.topk_w.has_value(), "topk_weights need topk_idx");
+        }
+        cached = !t[7].is_none();
+        if (cached) {
+            const py::tuple h = t[7].cast<py::tuple>();
+            DX_CHECK(h.size() == 6, "a normal-mode handle has 6 entries");
+            q.rpm = h[0].cast<torch::Tensor>();
+            q.cpm = h[1].cast<torch::Tensor>();
+            q.rcpm = h[2].cast<torch::Tensor>();
+            q.num_recv = (int)h[3].cast<torch::Tensor>().size(0);
+            q.in_rank = h[4].cast<torch::Tensor>();
+            q.send_head = h[5].cast<torch::Tensor>();
+            DX_CHECK(q.send_head.scalar_type() == torch::kInt32 && q.send_head.is_contiguous() && q.send_head.dim() == 2 && q.send_head.size(0) == T && q.send_head.size(1) == R, "send_head must be int32 [T,R]");
+            DX_CHECK(q.rpm.scalar_type() == torch::kInt32 && q.rpm.is_contiguous() && q.rpm.numel() == R * R, "rank_prefix_matrix must be int32 [R,R]");
+            continue;
+        }
+        auto ntpr = t[2].cast<torch::Tensor>(), ntpe = t[3].cast<torch::Tensor>();
+        q.in_rank = t[4].cast<torch::Tensor>();
+        DX_CHECK(ntpr.scalar_type() == torch::kInt32 && ntpr.numel() == R && ntpr.is_contiguous(), "num_tokens_per_rank must be int32 [R]");
+        DX_CHECK(ntpe.scalar_type() == torch::kInt32 && ntpe.is_contiguous() && ntpe.numel() % R == 0, "num_tokens_per_expert must be int32 [E]");
+        DX_CHECK(q.in_rank.scalar_type() == torch::kBool && q.in_rank.dim() == 2 && q.in_rank.size(1) == R && q.in_rank.is_contiguous(), "is_token_in_rank must be bool [T,R]");
+        DX_CHECK(q.in_rank.size(0) == T, "is_token_in_rank must have one row per token of x");
+        E = (int)ntpe.numel();
+        DX_CHECK(E / R <= dx::kMaxLocalExperts, "too many local experts");
+        auto i32 = torch::TensorOptions().dtype(torch::kInt32).device(q.in_rank.device());
+        q.rpm = torch::empty({R, R}, i32);
+        q.cpm = torch::empty({R, num_channels}, i32);
+        q.rcpm = torch::empty({R, num_channels}, i32);
+        q.send_head = torch::empty({T, R}, i32);
+        rt->core->reset_recv_counters(E / R);
+        dx::NotifyArgs& a = nargs[v];
         a.ctx = rt->core->ctx();
-        a.x = x.data_ptr();
-        a.x_elem_bytes = (int)x.element_size();
-        a.x_scales = nullptr;
+        a.num_tokens_per_rank = ntpr.data_ptr<int>();
+        a.num_tokens_per_expert = ntpe.data_ptr<int>();
+        a.is_token_in_rank = q.in_rank.data_ptr<bool>();
+        a.num_tokens = T;
+        a.num_experts = E;
+        a.num_channels = num_channels;
+        a.expert_alignment = expert_alignment;
+        a.rank_prefix_matrix = q.rpm.data_ptr<int>();
+        a.channel_prefix_matrix = q.cpm.data_ptr<int>();
+        a.recv_channel_prefix_matrix = q.rcpm.data_ptr<int>();
+        a.send_head = q.send_head.data_ptr<int>();
+        dxh::HostWords* hw = reinterpret_cast<dxh::HostWords*>(a.ctx.status);  // status is the first member
+        a.host_recv_counter = &hw->recv_counter;
+        a.host_expert_counter = hw->expert_counter;
+    }
+    if (!cached) check_launch(dx::launch_notify(nargs.data(), V, order.stream), "notify");
+
+    // How many rows arrive is known on the host only when the count exchange has run, except that a lone rank receives at most
+    // its own tokens: its outputs are sized for them, the dispatch kernel is queued at once and the host waits beside it.
+    const bool exact = !cached && num_worst_tokens == 0;
+    bool waited = !exact;
+    for (int v = 0; v < V; ++v) {
+        DispatchCall& q = calls[v];
+        int rows = cached ? q.num_recv : num_worst_tokens;
+        if (exact && R == 1) {
+            try {
+                q.allocate(rts[v], q.T);
+            } catch (const std::runtime_error&) {  // the arena may still hold what really arrives
+                q.payload.reset();
+                q.meta.reset();
+            }
+            if (q.meta) continue;
+        }
+        if (exact) {
+            wait_counts(rts[v], q, E / R);
+            rows = q.num_recv;
+            waited = true;
+        }
+        q.num_recv = rows;
+        q.allocate(rts[v], rows);
+    }
+    for (int v = 0; v < V; ++v) {
+        DispatchCall& q = calls[v];
+        dx::DispatchArgs& a = dargs[v];
+        a.ctx = rts[v]->core->ctx();
+        a.x = q.x.data_ptr();
+        a.x_elem_bytes = (int)q.x.element_size();
+        a.x_scales = (!quantize && q.x_scales.has_value()) ? q.x_scales->data_ptr<float>() : nullptr;
         a.quantize = quantize ? 1 : 0;
         a.round_scale = round_scale ? 1 : 0;
-        if (quantize) {
-            DX_CHECK(x.scalar_type() == torch::kBFloat16 && H % 128 == 0 && H <= 8192, "fused FP8 dispatch needs bf16 x with hidden % 128 == 0 and hidden <= 8192");
-            DX_CHECK(recv_scales.has_value(), "fused FP8 dispatch needs a recv_scales output");
-        } else if (x_scales.has_value()) {
-            DX_CHECK(x.element_size() == 1 && x_scales->scalar_type() == torch::kFloat32 && x_scales->is_contiguous() && x_scales->size(0) == T, "x_scales must be f32 [T,hidden/128]");
-            DX_CHECK(H % 128 == 0 && x_scales->size(1) == H / 128, "x_scales must have hidden/128 columns");
-            a.x_scales = x_scales->data_ptr<float>();
-        } else {
-            DX_CHECK(x.scalar_type() == torch::kBFloat16, "x must be bf16 (or an (e4m3, scales) pair)");
-        }
-        a.topk_idx = nullptr;
-        a.topk_weights = nullptr;
-        a.num_topk = 0;
-        if (topk_idx.has_value()) {
-            DX_CHECK(topk_idx->scalar_type() == torch::kInt64 && topk_idx->is_contiguous() && topk_idx->size(0) == T, "topk_idx must be int64 [T,K]");
-            a.num_topk = (int)topk_idx->size(1);
-            DX_CHECK(a.num_topk <= dx::kMaxTopk, "num_topk too large");
-            a.topk_idx = topk_idx->data_ptr<int64_t>();
-            DX_CHECK(recv_topk_idx.has_value(), "recv_topk_idx output missing");
-            if (topk_w.has_value()) {
-                DX_CHECK(topk_w->scalar_type() == torch::kFloat32 && topk_w->is_contiguous() && topk_w->numel() == topk_idx->numel(), "topk_weights must be f32 [T,K]");
-                a.topk_weights = topk_w->data_ptr<float>();
-                DX_CHECK(recv_topk_w.has_value(), "recv_topk_weights output missing");
-            }
-        }
-        a.send_head = send_head.data_ptr<int>();
-        a.rank_prefix_matrix = rpm.data_ptr<int>();
-        a.num_tokens = T;
-        a.hidden = H;
-        a.num_experts = num_experts;
+        a.topk_idx = ptr_or_null<int64_t>(q.topk_idx);
+        a.topk_weights = ptr_or_null<float>(q.topk_w);
+        a.num_topk = q.K;
+        a.send_head = q.send_head.data_ptr<int>();
+        a.rank_prefix_matrix = q.rpm.data_ptr<int>();
+        a.num_tokens = q.T;
+        a.hidden = q.H;
+        a.num_experts = E;
         a.num_sms = num_sms;
-        auto off_of = [&](const torch::Tensor& tt, const char* name) -> uint64_t {
-            const int64_t off = rt->symmetric_offset(tt);
-            DX_CHECK(off >= 0, std::string(name) + " must live in this rank's symmetric buffer");
-            return (uint64_t)off;
-        };
-        a.recv_x_off = off_of(recv_x, "recv_x");
-        a.recv_scales_off = recv_scales.has_value() ? off_of(*recv_scales, "recv_scales") : 0;
-        a.recv_topk_idx_off = recv_topk_idx.has_value() ? off_of(*recv_topk_idx, "recv_topk_idx") : 0;
-        a.recv_topk_w_off = recv_topk_w.has_value() ? off_of(*recv_topk_w, "recv_topk_weights") : 0;
-        a.recv_src_idx_off = off_of(recv_src_idx, "recv_src_idx");
+        a.recv_x_off = q.payload->off;
+        a.recv_scales_off = q.has_scales ? q.payload->off + q.scales_at : 0;
+        a.recv_topk_idx_off = q.topk_idx.has_value() ? q.meta->off : 0;
+        a.recv_topk_w_off = q.topk_w.has_value() ? q.meta->off + q.topk_w_at : 0;
+        a.recv_src_idx_off = q.meta->off + q.src_idx_at;
         a.num_worst_tokens = num_worst_tokens;
     }
-    check_launch(dx::launch_dispatch(args.data(), V, cur_stream(rts[0])), "dispatch");
+    check_launch(dx::launch_dispatch(dargs.data(), V, order.stream), "dispatch");
+
+    py::list out;
+    for (int v = 0; v < V; ++v) {
+        Runtime* rt = rts[v];
+        DispatchCall& q = calls[v];
+        if (!waited) wait_counts(rt, q, E / R);
+        const int64_t n = q.num_recv, H = q.H, K = q.K;
+        auto opt = [](bool there, auto make) -> py::object { return there ? py::cast(make()) : py::object(py::none()); };
+        py::object scales = opt(q.has_scales, [&] { return rt->tensor_in(q.payload, q.scales_at, {n, H / 128}, torch::kFloat32); });
+        py::object idx = opt(q.topk_idx.has_value(), [&] { return rt->tensor_in(q.meta, 0, {n, K}, torch::kInt64); });
+        py::object w = opt(q.topk_w.has_value(), [&] { return rt->tensor_in(q.meta, q.topk_w_at, {n, K}, torch::kFloat32); });
+        out.append(py::make_tuple(rt->tensor_in(q.payload, 0, {n, H}, q.out_type), scales, idx, w, q.per_expert,
+                                  py::make_tuple(q.rpm, q.cpm, q.rcpm, rt->tensor_in(q.meta, q.src_idx_at, {n}, torch::kInt32), q.in_rank, q.send_head)));
+    }
+    return out;
 }
 
 // ---------------------------------------------------------------------------------------------
-// combine. Per rank tuple: (x_sym, topk_weights_sym|None, send_head, rank_prefix_matrix, bias0|None,
-//                           bias1|None, out, out_topk_weights|None)
+// normal-mode combine. Per rank call: (x, topk_weights|None, send_head, rank_prefix_matrix, bias0|None, bias1|None,
+// out|None, out_topk_weights|None); outputs that are not given are allocated on the current stream.
+// Per rank result: (out, out_topk_weights|None)
 // ---------------------------------------------------------------------------------------------
-void combine(std::vector<Runtime*> rts, std::vector<py::tuple> per_rank, int num_sms) {
+py::list normal_combine(std::vector<Runtime*> rts, const std::vector<py::tuple>& per_rank, int num_sms) {
     const int V = (int)rts.size();
     DX_CHECK(V >= 1 && V <= dx::kMaxVirtualRanks && (int)per_rank.size() == V, "combine: one entry per rank");
     c10::cuda::CUDAGuard guard(rts[0]->core->device());
     std::vector<dx::CombineArgs> args(V);
+    std::vector<torch::Tensor> keep;
+    py::list results;
+    OrderedCall order(rts[0]);
     for (int v = 0; v < V; ++v) {
         Runtime* rt = rts[v];
         const py::tuple& t = per_rank[v];
@@ -321,27 +401,41 @@ void combine(std::vector<Runtime*> rts, std::vector<py::tuple> per_rank, int num
         auto rpm = t[3].cast<torch::Tensor>();
         auto b0 = opt_tensor(t[4]);
         auto b1 = opt_tensor(t[5]);
-        auto out = t[6].cast<torch::Tensor>();
-        auto out_w = opt_tensor(t[7]);
-        DX_CHECK(x.dim() == 2 && x.scalar_type() == torch::kBFloat16, "combine: x must be bf16 [N,hidden]");
+        DX_CHECK(x.is_cuda() && x.dim() == 2 && x.scalar_type() == torch::kBFloat16, "combine: x must be bf16 [N,hidden] on the GPU");
+        DX_CHECK(!w.has_value() || (w->is_cuda() && w->scalar_type() == torch::kFloat32 && w->dim() == 2), "combine: topk_weights must be f32 [N,K] on the GPU");
         const int H = (int)x.size(1), T = (int)send_head.size(0);
         DX_CHECK(H % 8 == 0, "hidden must be a multiple of 8");
         DX_CHECK(send_head.scalar_type() == torch::kInt32 && send_head.is_contiguous() && send_head.size(1) == R, "send_head must be int32 [T,R]");
+        // What the peers read must lie in symmetric memory; anything else is staged there. A lone rank reads its own tensor where
+        // it is (an offset that leaves the buffer, which the debug range check would refuse).
+        auto place = [&](const torch::Tensor& given) -> uint64_t {
+            torch::Tensor tt = given.contiguous();
+            int64_t off = rt->symmetric_offset(tt);
+            const bool in_place = R == 1 && !rt->core->debug_checks() && (reinterpret_cast<uintptr_t>(tt.data_ptr()) & 15) == 0;
+            if (off < 0 && !in_place) {
+                const uint64_t bytes = (uint64_t)tt.numel() * tt.element_size();
+                auto staged = rt->tensor_in(rt->alloc_block(bytes), 0, tt.sizes(), tt.scalar_type());
+                DX_CUDA_CHECK(cudaMemcpyAsync(staged.data_ptr(), tt.data_ptr(), bytes, cudaMemcpyDeviceToDevice, order.stream));
+                off = rt->symmetric_offset(staged);
+                keep.push_back(staged);
+            }
+            keep.push_back(tt);
+            return off >= 0 ? (uint64_t)off : (uint64_t)(reinterpret_cast<uintptr_t>(tt.data_ptr()) - reinterpret_cast<uintptr_t>(rt->core->base()));
+        };
+        torch::Tensor out = t[6].is_none() ? torch::empty({T, H}, x.options()) : t[6].cast<torch::Tensor>();
         DX_CHECK(out.scalar_type() == torch::kBFloat16 && out.is_contiguous() && out.size(0) == T && out.size(1) == H, "out must be bf16 [T,hidden]");
+        c10::optional<torch::Tensor> out_w;
         dx::CombineArgs& a = args[v];
         a.ctx = rt->core->ctx();
-        const int64_t xo = rt->symmetric_offset(x);
-        DX_CHECK(xo >= 0, "combine: x must live in the symmetric buffer (stage it first)");
-        a.x_off = (uint64_t)xo;
+        a.x_off = place(x);
         a.topk_w_off = ~0ull;
         a.num_topk = 0;
         a.out_topk_w = nullptr;
         if (w.has_value()) {
-            const int64_t wo = rt->symmetric_offset(*w);
-            DX_CHECK(wo >= 0 && w->scalar_type() == torch::kFloat32 && w->dim() == 2, "combine: topk_weights must be f32 [N,K] in the symmetric buffer");
-            a.topk_w_off = (uint64_t)wo;
+            a.topk_w_off = place(*w);
             a.num_topk = (int)w->size(1);
-            DX_CHECK(out_w.has_value() && out_w->scalar_type() == torch::kFloat32 && out_w->is_contiguous(), "combine: out_topk_weights must be f32");
+            out_w = t[7].is_none() ? torch::empty({T, a.num_topk}, w->options()) : t[7].cast<torch::Tensor>();
+            DX_CHECK(out_w->scalar_type() == torch::kFloat32 && out_w->is_contiguous() && out_w->numel() == (int64_t)T * a.num_topk, "combine: out_topk_weights must be f32 [T,K]");
             a.out_topk_w = out_w->data_ptr<float>();
         }
         a.send_head = send_head.data_ptr<int>();
@@ -357,8 +451,10 @@ void combine(std::vector<Runtime*> rts, std::vector<py::tuple> per_rank, int num
         a.num_tokens = T;
         a.hidden = H;
         a.num_sms = num_sms;
+        results.append(py::make_tuple(out, out_w));
     }
-    check_launch(dx::launch_combine(args.data(), V, cur_stream(rts[0])), "combine");
+    check_launch(dx::launch_combine(args.data(), V, order.stream), "combine");
+    return results;
 }
 
 void barrier(std::vector<Runtime*> rts) {
@@ -650,7 +746,6 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         .def("alloc_symmetric", &Runtime::alloc_symmetric)
         .def("symmetric_offset", &Runtime::symmetric_offset)
         .def("view", &Runtime::view)
-        .def("wait_recv_counts", &Runtime::wait_recv_counts)
         .def("set_mask", &Runtime::set_mask)
         .def("query_mask", &Runtime::query_mask)
         .def("clean_mask", &Runtime::clean_mask)
@@ -678,9 +773,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
 
     m.def("set_local_peers", &set_local_peers);
     m.def("get_dispatch_layout", &get_dispatch_layout);
-    m.def("notify", &notify);
-    m.def("dispatch", &dispatch);
-    m.def("combine", &combine);
+    m.def("normal_dispatch", &normal_dispatch);
+    m.def("normal_combine", &normal_combine);
     m.def("barrier", &barrier);
     m.def("timeout_probe", &timeout_probe);
     m.def("per_token_cast_to_fp8", &per_token_cast_to_fp8, py::arg("x"), py::arg("round_scale") = false, py::arg("use_ue8m0") = false,

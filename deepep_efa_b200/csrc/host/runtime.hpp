@@ -158,6 +158,10 @@ class RuntimeCore {
         cudaSetDevice(device_);
         cudaDeviceSynchronize();
         drain_pending(true);
+        for (cudaEvent_t ev : event_pool_) cudaEventDestroy(ev);
+        event_pool_.clear();
+        if (order_event_ != nullptr) cudaEventDestroy(order_event_);
+        order_event_ = nullptr;
         for (int r = 0; r < num_ranks_; ++r)
             if (ipc_opened_[r]) cudaIpcCloseMemHandle(peers_[r]);
         if (base_) cudaFree(base_);
@@ -210,9 +214,10 @@ class RuntimeCore {
         return (uint64_t)off;
     }
 
-    // Called from tensor deleters (any thread). `streams` are streams whose queued work may still
-    // use the block.
-    void arena_release(uint64_t off, const std::vector<cudaStream_t>& streams) {
+    // Called when the last tensor of a block dies (any thread). `streams` (up to two, nullptr = the default stream) are the
+    // streams whose queued work may still use the block. Events come from a pool: creating and destroying them cost more than
+    // everything else here.
+    void arena_release(uint64_t off, const cudaStream_t* streams, int num_streams) {
         std::lock_guard<std::mutex> g(mu_);
         if (released_) return;
         Pending p;
@@ -220,16 +225,37 @@ class RuntimeCore {
         int prev = -1;
         cudaGetDevice(&prev);
         if (prev != device_) cudaSetDevice(device_);
-        for (cudaStream_t s : streams) {
-            cudaEvent_t ev = nullptr;
-            if (cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) == cudaSuccess) {
-                if (cudaEventRecord(ev, s) == cudaSuccess) p.events.push_back(ev);
-                else cudaEventDestroy(ev);
-            }
+        for (int i = 0; i < num_streams; ++i) {
+            if (i == 1 && streams[1] == streams[0]) break;
+            cudaEvent_t ev = take_event();
+            if (ev == nullptr) continue;
+            if (cudaEventRecord(ev, streams[i]) == cudaSuccess) p.events[p.num_events++] = ev;
+            else event_pool_.push_back(ev);
         }
         cudaGetLastError();
         if (prev != device_ && prev >= 0) cudaSetDevice(prev);
-        pending_.push_back(std::move(p));
+        pending_.push_back(p);
+    }
+
+    // ---- order of the normal-mode kernels -----------------------------------------------------
+    // They share state (sequence numbers, tickets, the layout scratch), so one must not overlap the next one. A call runs on the
+    // caller's stream, or on the communication stream when the caller asked for an event; a call on another stream than the
+    // last one waits for that one's event first. A stream under capture takes no part: an event from outside may not be waited
+    // for there, and the graph's owner orders its replays.
+    bool order_enter(cudaStream_t s) {
+        cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(s, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone) {
+            cudaGetLastError();
+            return false;
+        }
+        if (order_event_ != nullptr && order_stream_ != s) DX_CUDA_CHECK(cudaStreamWaitEvent(s, order_event_, 0));
+        return true;
+    }
+    void order_leave(cudaStream_t s) {
+        if (order_event_ == nullptr && cudaEventCreateWithFlags(&order_event_, cudaEventDisableTiming) != cudaSuccess) order_event_ = nullptr;
+        if (order_event_ != nullptr) cudaEventRecord(order_event_, s);
+        order_stream_ = s;
+        cudaGetLastError();
     }
 
     bool in_symmetric(const void* p, uint64_t bytes, uint64_t* off) const {
@@ -335,22 +361,34 @@ class RuntimeCore {
     static int read_word(const int* p) { return *reinterpret_cast<const volatile int*>(p); }
 
     struct Pending {
-        uint64_t off;
-        std::vector<cudaEvent_t> events;
+        uint64_t off = 0;
+        cudaEvent_t events[2];
+        int num_events = 0;
     };
+
+    cudaEvent_t take_event() {
+        cudaEvent_t ev = nullptr;
+        if (!event_pool_.empty()) {
+            ev = event_pool_.back();
+            event_pool_.pop_back();
+        } else if (cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess) {
+            ev = nullptr;
+        }
+        return ev;
+    }
 
     void drain_pending(bool wait) {
         for (auto it = pending_.begin(); it != pending_.end();) {
             bool done = true;
-            for (cudaEvent_t ev : it->events) {
-                cudaError_t e = wait ? cudaEventSynchronize(ev) : cudaEventQuery(ev);
+            for (int i = 0; i < it->num_events; ++i) {
+                cudaError_t e = wait ? cudaEventSynchronize(it->events[i]) : cudaEventQuery(it->events[i]);
                 if (e == cudaErrorNotReady) {
                     done = false;
                     break;
                 }
             }
             if (done) {
-                for (cudaEvent_t ev : it->events) cudaEventDestroy(ev);
+                for (int i = 0; i < it->num_events; ++i) event_pool_.push_back(it->events[i]);
                 arena_.free(it->off);
                 it = pending_.erase(it);
             } else {
@@ -381,6 +419,9 @@ class RuntimeCore {
     long long timeout_cycles_ = 0;
     Arena arena_;
     std::deque<Pending> pending_;
+    std::vector<cudaEvent_t> event_pool_;  // bounded by the number of blocks that were ever pending at once
+    cudaEvent_t order_event_ = nullptr;    // end of the last normal-mode call, recorded on order_stream_
+    cudaStream_t order_stream_ = nullptr;
     std::mutex mu_;
 };
 

@@ -11,6 +11,23 @@
 
 namespace dx {
 
+// Ordinary kernel whose launch work overlaps the tail of its predecessor in the stream (programmatic dependent launch). The
+// kernel must execute griddepcontrol.wait (pdl_wait_predecessor) before it touches memory that the predecessor may touch.
+template <typename... P, typename... A>
+cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t stream, const A&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 template <typename Args, int V>
 struct ArgPack {
     Args a[V];

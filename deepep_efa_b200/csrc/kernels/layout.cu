@@ -9,6 +9,7 @@
 // re-reading all of topk_idx). Outputs are identical: num_tokens_per_rank[R] i32,
 // num_tokens_per_expert[E] i32, is_token_in_rank[T,R] bool.
 #include "api.h"
+#include "launch.cuh"
 #include "prims.cuh"
 
 namespace dx {
@@ -29,17 +30,25 @@ __global__ void __launch_bounds__(kLayoutThreads) layout_kernel(const LayoutArgs
     const int nodes = a.num_tokens_per_node != nullptr ? R / P : 0;
     const int bins = E + R + nodes;
     for (int i = threadIdx.x; i < bins; i += kLayoutThreads) s_hist[i] = 0;
+    pdl_wait_predecessor();
+    pdl_release_successor();
     __syncthreads();
 
     const int t = blockIdx.x * kLayoutThreads + threadIdx.x;
     uint64_t mask = 0;
     if (t < a.num_tokens) {
         const int64_t* row = a.topk_idx + (size_t)t * K;
-        for (int k = 0; k < K; ++k) {
-            const int64_t e = row[k];
-            if (e >= 0 && e < E) {
-                atomicAdd(&s_hist[(int)e], 1);
-                mask |= 1ull << ((int)e / L);
+        // eight ids are requested before the first one is looked at: one trip to memory per eight selections
+        for (int k0 = 0; k0 < K; k0 += 8) {
+            int64_t ids[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) ids[k] = k0 + k < K ? row[k0 + k] : -1;
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                if (ids[k] >= 0 && ids[k] < E) {
+                    atomicAdd(&s_hist[(int)ids[k]], 1);
+                    mask |= 1ull << ((int)ids[k] / L);
+                }
             }
         }
         if (R == 8) {
@@ -63,16 +72,24 @@ __global__ void __launch_bounds__(kLayoutThreads) layout_kernel(const LayoutArgs
     }
     __syncthreads();
 
+    auto publish = [&](int i, int sum) {
+        if (i < E) a.num_tokens_per_expert[i] = sum;
+        else if (i < E + R) a.num_tokens_per_rank[i - E] = sum;
+        else a.num_tokens_per_node[i - E - R] = sum;
+    };
+    if (gridDim.x == 1) {  // one CTA has seen every token
+        for (int i = threadIdx.x; i < bins; i += kLayoutThreads) publish(i, s_hist[i]);
+        return;
+    }
     int* partial = a.scratch + 1 + (size_t)blockIdx.x * bins;
     for (int i = threadIdx.x; i < bins; i += kLayoutThreads) partial[i] = s_hist[i];
 
     if (cta_is_last(a.scratch, gridDim.x)) {
         for (int i = threadIdx.x; i < bins; i += kLayoutThreads) {
             int sum = 0;
+#pragma unroll 8
             for (int b = 0; b < (int)gridDim.x; ++b) sum += __ldcg(a.scratch + 1 + (size_t)b * bins + i);
-            if (i < E) a.num_tokens_per_expert[i] = sum;
-            else if (i < E + R) a.num_tokens_per_rank[i - E] = sum;
-            else a.num_tokens_per_node[i - E - R] = sum;
+            publish(i, sum);
         }
     }
 }
@@ -82,8 +99,7 @@ cudaError_t launch_layout(const LayoutArgs& a, cudaStream_t stream) {
     if (ctas < 1) ctas = 1;
     if (a.num_ranks > 64) return cudaErrorInvalidValue;
     const size_t smem = (size_t)(a.num_experts + 2 * a.num_ranks) * sizeof(int);  // upper bound of the bins
-    layout_kernel<<<ctas, kLayoutThreads, smem, stream>>>(a);
-    return cudaGetLastError();
+    return launch_dependent(layout_kernel, dim3(ctas), kLayoutThreads, smem, stream, a);
 }
 
 }  // namespace dx

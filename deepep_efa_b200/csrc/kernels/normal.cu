@@ -36,6 +36,8 @@ constexpr int kNotifyThreads = 1024;
 
 template <int V>
 __global__ void __launch_bounds__(kNotifyThreads, 1) notify_kernel(const __grid_constant__ ArgPack<NotifyArgs, V> pack) {
+    pdl_wait_predecessor();
+    pdl_release_successor();
     const NotifyArgs& a = pack.a[blockIdx.y];
     const RankCtx& c = a.ctx;
     const int R = c.num_ranks, me = c.rank;
@@ -56,7 +58,8 @@ __global__ void __launch_bounds__(kNotifyThreads, 1) notify_kernel(const __grid_
                 st_relaxed_sys(&pc->notify_expert_counts[me][i], a.num_tokens_per_expert[d * L + i]);
         }
         __syncthreads();
-        if (tid < R) {
+        // this rank's own counts need no flag: the barrier above orders them for this CTA, their only reader
+        if (tid < R && tid != me) {
             st_release_sys(&c.ctrl(tid)->notify_seq[me], seq);
             if (!wait_ge_sys(&c.my_ctrl()->notify_seq[tid], seq, c.timeout_cycles)) {
                 report(c.status, kTimeoutNotify, me, tid, 0);
@@ -86,9 +89,9 @@ __global__ void __launch_bounds__(kNotifyThreads, 1) notify_kernel(const __grid_
             const int al = a.expert_alignment;
             a.host_expert_counter[e] = (sum + al - 1) / al * al;
         }
-        __threadfence_system();
-        // channel prefix rows pushed by the scan CTAs of my peers
-        if (tid < R) {
+        // (the host polls every one of these words for itself, so they need no order among themselves)
+        // channel prefix rows pushed by the scan CTAs of my peers; my own row is written by my scan CTA
+        if (tid < R && tid != me) {
             uint64_t dummy;
             if (!mailbox_wait(c, kMbChanPrefix, tid, seq, &dummy, 0)) {
                 report(c.status, kTimeoutNotify, me, tid, 1);
@@ -98,7 +101,7 @@ __global__ void __launch_bounds__(kNotifyThreads, 1) notify_kernel(const __grid_
         __syncthreads();
         if (!s_ok) return;
         for (int i = tid; i < R * C; i += kNotifyThreads)
-            a.recv_channel_prefix_matrix[i] = ld_relaxed_sys(&my->chan_prefix_in[i / C][i % C]);
+            if (i / C != me) a.recv_channel_prefix_matrix[i] = ld_relaxed_sys(&my->chan_prefix_in[i / C][i % C]);
         if (cta_is_last(c.local_scratch + kTicketNotify, gridDim.x) && tid == 0) commit_seq(c, kFamNotify, seq);
         return;
     }
@@ -139,17 +142,18 @@ __global__ void __launch_bounds__(kNotifyThreads, 1) notify_kernel(const __grid_
         if (owner < kNotifyThreads)
             for (int t = owner * per; t < b; ++t) prefix += a.is_token_in_rank[(size_t)t * R + d] ? 1 : 0;
         a.channel_prefix_matrix[d * C + tid] = prefix;
-        st_relaxed_sys(&c.ctrl(d)->chan_prefix_in[me][tid], prefix);
+        if (d == me) a.recv_channel_prefix_matrix[me * C + tid] = prefix;
+        else st_relaxed_sys(&c.ctrl(d)->chan_prefix_in[me][tid], prefix);
     }
     __syncthreads();
-    if (tid == 0) {
+    if (tid == 0 && d != me) {
         mailbox_post(c, kMbChanPrefix, d, nullptr, 0, seq);
     }
     if (cta_is_last(c.local_scratch + kTicketNotify, gridDim.x) && tid == 0) commit_seq(c, kFamNotify, seq);
 }
 
 cudaError_t launch_notify(const NotifyArgs* a, int nv, cudaStream_t stream) {
-    return DX_LAUNCH_RANKED(notify_kernel, NotifyArgs, a, nv, 1 + a[0].ctx.num_ranks, kNotifyThreads, 0, stream);
+    return DX_LAUNCH_RANKED_PDL(notify_kernel, NotifyArgs, a, nv, 1 + a[0].ctx.num_ranks, kNotifyThreads, 0, stream);
 }
 
 // =============================================================================================
@@ -167,96 +171,84 @@ struct PeerDst {
     int base_row;  // rows of ranks before me at that peer
 };
 
-template <int V>
-__global__ void __launch_bounds__(kDispatchThreads, 1) dispatch_kernel(const __grid_constant__ ArgPack<DispatchArgs, V> pack) {
-    const DispatchArgs& a = pack.a[blockIdx.y];
+// A warp's share of the rows: item i = (token i / pieces, piece i % pieces). Items are dealt out CTA by CTA, so that every SM
+// gets work when there are fewer items than warps, and a small batch cuts its rows into pieces (each at least kMinPiece 16-byte
+// columns of the row) until there is about one item per warp: a lone warp moves an 8 KB row in four dependent steps, about 4 us.
+constexpr int kMinPiece16 = 64;
+constexpr int kMaxPieces = 8;
+
+__device__ __forceinline__ int row_pieces(int num_tokens, int n16, int total_warps) {
+    int p = 1;
+    while (p < kMaxPieces && 2 * p * num_tokens <= total_warps && n16 / (2 * p) >= kMinPiece16) p *= 2;
+    return p;
+}
+
+// CTAs of a launch: the caller's bound, and no more than have a token to move.
+template <typename Args>
+int grid_ctas(const Args* a, int nv) {
+    int most = 1;
+    for (int i = 0; i < nv; ++i) most = a[i].num_tokens > most ? a[i].num_tokens : most;
+    return a[0].num_sms < most ? a[0].num_sms : most;
+}
+
+template <int kRanks>
+__device__ __forceinline__ void dispatch_rows(const DispatchArgs& a, const PeerDst* s_dst, float* s_scales, int warp, int lane) {
     const RankCtx& c = a.ctx;
-    const int R = c.num_ranks, me = c.rank, T = a.num_tokens, K = a.num_topk;
+    const int R = c.num_ranks, T = a.num_tokens, K = a.num_topk;
     const int L = a.num_experts / R;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const uint64_t seq = next_seq(c, kFamDispatch);
-    __shared__ PeerDst s_dst[kMaxRanks];
-    __shared__ int s_ok;
-    __shared__ float s_scales[kDispatchWarps][64];
-
-    if (tid == 0) s_ok = 1;
-    __syncthreads();
-    // Publish where my rows go, then learn where every peer wants its rows.
-    if (blockIdx.x == 0 && tid < R) {
-        uint64_t w[5] = {a.recv_x_off, a.recv_scales_off, a.recv_topk_idx_off, a.recv_topk_w_off, a.recv_src_idx_off};
-        mailbox_post(c, kMbDispatchDesc, tid, w, 5, seq);
-    }
-    if (tid < R) {
-        uint64_t w[5];
-        if (!mailbox_wait(c, kMbDispatchDesc, tid, seq, w, 5)) {
-            report(c.status, kTimeoutDescriptor, me, tid, 0);
-            s_ok = 0;
-        } else {
-            PeerDst p;
-            p.x = c.at<char>(tid, w[0]);
-            p.scales = c.at<float>(tid, w[1]);
-            p.topk_idx = c.at<int64_t>(tid, w[2]);
-            p.topk_w = c.at<float>(tid, w[3]);
-            p.src_idx = c.at<int>(tid, w[4]);
-            p.base_row = me > 0 ? a.rank_prefix_matrix[(me - 1) * R + tid] : 0;
-            s_dst[tid] = p;
-        }
-    }
-    __syncthreads();
-    if (!s_ok) return;
-
     const int H = a.hidden;
     const bool quant = a.quantize != 0;
-    const int out_elem = quant ? 1 : a.x_elem_bytes;
-    const size_t out_row_bytes = (size_t)H * out_elem;
+    const size_t out_row_bytes = (size_t)H * (quant ? 1 : a.x_elem_bytes);
     const int num_scales = H / 128;
-    const bool has_scales = quant || a.x_scales != nullptr;
-    const int total_warps = a.num_sms * kDispatchWarps;
+    // columns of a row in the unit its pieces are cut in: 16 bytes, or (quantising) the 512 channels a warp converts per step
+    const int n16 = (int)(out_row_bytes / 16);
+    const int pieces = row_pieces(T, quant ? H / 8 : n16, gridDim.x * kDispatchWarps);
 
-    for (int t = blockIdx.x * kDispatchWarps + warp; t < T; t += total_warps) {
+    for (int item = blockIdx.x + gridDim.x * warp; item < T * pieces; item += gridDim.x * kDispatchWarps) {
+        const int t = item / pieces, piece = item % pieces;
         // destination rows
         int head = (lane < R) ? a.send_head[(size_t)t * R + lane] : -1;
         const unsigned dmask = __ballot_sync(0xffffffffu, head >= 0);
         if (dmask == 0) continue;
-        int rows[kMaxRanks];
+        int rows[kRanks];
 #pragma unroll
-        for (int d = 0; d < kMaxRanks; ++d) {
+        for (int d = 0; d < kRanks; ++d) {
             const int h = __shfl_sync(0xffffffffu, head, d);
             rows[d] = (d < R && h >= 0) ? s_dst[d].base_row + h : -1;
-            if (c.debug_extent != 0 && rows[d] >= 0 &&
-                !peer_range_ok(c, d, s_dst[d].x + (size_t)rows[d] * ((size_t)a.hidden * (a.quantize != 0 ? 1 : a.x_elem_bytes)),
-                               (size_t)a.hidden * (a.quantize != 0 ? 1 : a.x_elem_bytes), 1))
-                rows[d] = -1;
+            if (c.debug_extent != 0 && rows[d] >= 0 && !peer_range_ok(c, d, s_dst[d].x + (size_t)rows[d] * out_row_bytes, out_row_bytes, 1)) rows[d] = -1;
         }
 
         if (!quant) {
             // ---- pass-through rows (bf16 or already-quantised e4m3) ----
-            const int n16 = (int)(out_row_bytes / 16);
+            const int per = (((n16 + pieces - 1) / pieces) + 31) & ~31;
+            const int end = min(n16, (piece + 1) * per);
             const int4* src = reinterpret_cast<const int4*>(reinterpret_cast<const char*>(a.x) + (size_t)t * out_row_bytes);
-            constexpr int U = 4;
-            for (int i0 = 0; i0 < n16; i0 += 32 * U) {
+            // loads in flight per lane: a store to a peer occupies the lane for longer than one to this GPU, so the one-rank form
+            // (bound by the latency of its own loads) asks for twice as many
+            constexpr int U = kRanks == 1 ? 8 : 4;
+            for (int i0 = piece * per; i0 < end; i0 += 32 * U) {
                 int4 v[U];
 #pragma unroll
                 for (int u = 0; u < U; ++u) {
                     const int i = i0 + u * 32 + lane;
-                    if (i < n16) v[u] = ld_stream(src + i);
+                    if (i < end) v[u] = ld_stream(src + i);
                 }
 #pragma unroll
-                for (int d = 0; d < kMaxRanks; ++d) {
+                for (int d = 0; d < kRanks; ++d) {
                     if (rows[d] < 0) continue;
                     int4* dst = reinterpret_cast<int4*>(s_dst[d].x + (size_t)rows[d] * out_row_bytes);
 #pragma unroll
                     for (int u = 0; u < U; ++u) {
                         const int i = i0 + u * 32 + lane;
-                        if (i < n16) st_stream(dst + i, v[u]);
+                        if (i < end) st_stream(dst + i, v[u]);
                     }
                 }
             }
-            if (a.x_scales != nullptr) {
+            if (a.x_scales != nullptr && piece == 0) {
                 for (int i = lane; i < num_scales; i += 32) {
                     const float s = a.x_scales[(size_t)t * num_scales + i];
 #pragma unroll
-                    for (int d = 0; d < kMaxRanks; ++d)
+                    for (int d = 0; d < kRanks; ++d)
                         if (rows[d] >= 0) s_dst[d].scales[(size_t)rows[d] * num_scales + i] = s;
                 }
             }
@@ -264,24 +256,26 @@ __global__ void __launch_bounds__(kDispatchThreads, 1) dispatch_kernel(const __g
             // ---- fused BF16 -> e4m3 with one fp32 scale per 128 channels ----
             // A lane owns 16 consecutive channels, 8 lanes own one scale group, a warp covers 512
             // channels per step.
+            const int per = (((H + pieces - 1) / pieces) + 511) & ~511;
+            const int begin = piece * per, end = min(H, begin + per);
             const char* src = reinterpret_cast<const char*>(a.x) + (size_t)t * H * 2;
             // four 16-byte loads per lane in flight: the next 1024 channels are requested before the current ones are converted
             int4 cur[4], nxt[4];
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                const int ch = h * 512 + lane * 16;
+                const int ch = begin + h * 512 + lane * 16;
                 cur[2 * h] = cur[2 * h + 1] = make_int4(0, 0, 0, 0);
-                if (ch < H) {
+                if (ch < end) {
                     cur[2 * h] = ld_cached(reinterpret_cast<const int4*>(src + (size_t)ch * 2));
                     cur[2 * h + 1] = ld_cached(reinterpret_cast<const int4*>(src + (size_t)ch * 2 + 16));
                 }
             }
-            for (int c0 = 0; c0 < H; c0 += 1024) {
+            for (int c0 = begin; c0 < end; c0 += 1024) {
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     const int chn = c0 + 1024 + h * 512 + lane * 16;
                     nxt[2 * h] = nxt[2 * h + 1] = make_int4(0, 0, 0, 0);
-                    if (chn < H) {
+                    if (chn < end) {
                         nxt[2 * h] = ld_cached(reinterpret_cast<const int4*>(src + (size_t)chn * 2));
                         nxt[2 * h + 1] = ld_cached(reinterpret_cast<const int4*>(src + (size_t)chn * 2 + 16));
                     }
@@ -289,7 +283,7 @@ __global__ void __launch_bounds__(kDispatchThreads, 1) dispatch_kernel(const __g
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     const int ch = c0 + h * 512 + lane * 16;
-                    const bool act = ch < H;
+                    const bool act = ch < end;
                     const int4 r0 = cur[2 * h], r1 = cur[2 * h + 1];
                     float f[16];
                     {
@@ -315,10 +309,10 @@ __global__ void __launch_bounds__(kDispatchThreads, 1) dispatch_kernel(const __g
                     q.y = (int)pack_e4m3x4(f[4] * inv, f[5] * inv, f[6] * inv, f[7] * inv);
                     q.z = (int)pack_e4m3x4(f[8] * inv, f[9] * inv, f[10] * inv, f[11] * inv);
                     q.w = (int)pack_e4m3x4(f[12] * inv, f[13] * inv, f[14] * inv, f[15] * inv);
-                    if (act && (lane & 7) == 0) s_scales[warp][ch >> 7] = scale;
+                    if (act && (lane & 7) == 0) s_scales[ch >> 7] = scale;
                     if (act) {
 #pragma unroll
-                        for (int d = 0; d < kMaxRanks; ++d)
+                        for (int d = 0; d < kRanks; ++d)
                             if (rows[d] >= 0) st_stream(reinterpret_cast<int4*>(s_dst[d].x + (size_t)rows[d] * H + ch), q);
                     }
                 }
@@ -326,22 +320,22 @@ __global__ void __launch_bounds__(kDispatchThreads, 1) dispatch_kernel(const __g
                 for (int j = 0; j < 4; ++j) cur[j] = nxt[j];
             }
             __syncwarp();
-            for (int i = lane; i < num_scales; i += 32) {
-                const float s = s_scales[warp][i];
+            for (int i = (begin >> 7) + lane; i < (end >> 7); i += 32) {
+                const float s = s_scales[i];
 #pragma unroll
-                for (int d = 0; d < kMaxRanks; ++d)
+                for (int d = 0; d < kRanks; ++d)
                     if (rows[d] >= 0) s_dst[d].scales[(size_t)rows[d] * num_scales + i] = s;
             }
             __syncwarp();
         }
-        (void)has_scales;
+        if (piece != 0) continue;
 
         // ---- metadata: local expert ids, weights, source token index ----
         if (a.topk_idx != nullptr && lane < K) {
             const int64_t e = a.topk_idx[(size_t)t * K + lane];
             const float w = a.topk_weights != nullptr ? a.topk_weights[(size_t)t * K + lane] : 0.f;
 #pragma unroll
-            for (int d = 0; d < kMaxRanks; ++d) {
+            for (int d = 0; d < kRanks; ++d) {
                 if (rows[d] < 0) continue;
                 const bool mine = e >= (int64_t)d * L && e < (int64_t)(d + 1) * L;
                 s_dst[d].topk_idx[(size_t)rows[d] * K + lane] = mine ? e - (int64_t)d * L : -1;
@@ -350,35 +344,80 @@ __global__ void __launch_bounds__(kDispatchThreads, 1) dispatch_kernel(const __g
         }
         if (lane == 0) {
 #pragma unroll
-            for (int d = 0; d < kMaxRanks; ++d)
+            for (int d = 0; d < kRanks; ++d)
                 if (rows[d] >= 0) s_dst[d].src_idx[rows[d]] = t;
         }
     }
+}
+
+template <int V>
+__global__ void __launch_bounds__(kDispatchThreads, 1) dispatch_kernel(const __grid_constant__ ArgPack<DispatchArgs, V> pack) {
+    pdl_wait_predecessor();
+    pdl_release_successor();
+    const DispatchArgs& a = pack.a[blockIdx.y];
+    const RankCtx& c = a.ctx;
+    const int R = c.num_ranks, me = c.rank, K = a.num_topk;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint64_t seq = next_seq(c, kFamDispatch);
+    __shared__ PeerDst s_dst[kMaxRanks];
+    __shared__ int s_ok;
+    __shared__ float s_scales[kDispatchWarps][64];
+
+    if (tid == 0) s_ok = 1;
+    __syncthreads();
+    // Publish where my rows go, then learn where every peer wants its rows (my own place I know without asking).
+    if (blockIdx.x == 0 && tid < R && tid != me) {
+        uint64_t w[5] = {a.recv_x_off, a.recv_scales_off, a.recv_topk_idx_off, a.recv_topk_w_off, a.recv_src_idx_off};
+        mailbox_post(c, kMbDispatchDesc, tid, w, 5, seq);
+    }
+    if (tid < R) {
+        uint64_t w[5] = {a.recv_x_off, a.recv_scales_off, a.recv_topk_idx_off, a.recv_topk_w_off, a.recv_src_idx_off};
+        if (tid != me && !mailbox_wait(c, kMbDispatchDesc, tid, seq, w, 5)) {
+            report(c.status, kTimeoutDescriptor, me, tid, 0);
+            s_ok = 0;
+        } else {
+            PeerDst p;
+            p.x = c.at<char>(tid, w[0]);
+            p.scales = c.at<float>(tid, w[1]);
+            p.topk_idx = c.at<int64_t>(tid, w[2]);
+            p.topk_w = c.at<float>(tid, w[3]);
+            p.src_idx = c.at<int>(tid, w[4]);
+            p.base_row = me > 0 ? a.rank_prefix_matrix[(me - 1) * R + tid] : 0;
+            s_dst[tid] = p;
+        }
+    }
+    __syncthreads();
+    if (!s_ok) return;
+
+    if (R <= 1) dispatch_rows<1>(a, s_dst, s_scales[warp], warp, lane);
+    else if (R <= 2) dispatch_rows<2>(a, s_dst, s_scales[warp], warp, lane);
+    else if (R <= 4) dispatch_rows<4>(a, s_dst, s_scales[warp], warp, lane);
+    else dispatch_rows<8>(a, s_dst, s_scales[warp], warp, lane);
 
     // worst-case sized outputs: mark the unused tail of my own recv_topk_idx
     if (a.num_worst_tokens > 0 && a.topk_idx != nullptr) {
         const int num_recv = a.rank_prefix_matrix[(R - 1) * R + me];
         int64_t* mine = c.at<int64_t>(me, a.recv_topk_idx_off);
         const size_t lo = (size_t)num_recv * K, hi = (size_t)a.num_worst_tokens * K;
-        for (size_t i = lo + (size_t)blockIdx.x * kDispatchThreads + tid; i < hi; i += (size_t)a.num_sms * kDispatchThreads)
+        for (size_t i = lo + (size_t)blockIdx.x * kDispatchThreads + tid; i < hi; i += (size_t)gridDim.x * kDispatchThreads)
             mine[i] = -1;
     }
 
-    // ---- completion: when my last CTA is done, tell every peer; CTA 0 waits for every peer ----
+    // ---- completion: when my last CTA is done, tell every peer; CTA 0 waits for every peer. A lone rank has nobody to tell
+    // or to wait for (the end of the kernel is its completion), and no sequence number that anybody compares.
+    if (R == 1) return;
     if (cta_is_last(c.local_scratch + kTicketDispatch, gridDim.x)) {
-        if (tid < R) {
-            st_release_sys(&c.ctrl(tid)->barrier_in[kBarDispatch][me], seq);
-        }
+        if (tid < R && tid != me) st_release_sys(&c.ctrl(tid)->barrier_in[kBarDispatch][me], seq);
         if (tid == 0) commit_seq(c, kFamDispatch, seq);
     }
-    if (blockIdx.x == 0 && tid < R) {
+    if (blockIdx.x == 0 && tid < R && tid != me) {
         if (!wait_ge_sys(&c.my_ctrl()->barrier_in[kBarDispatch][tid], seq, c.timeout_cycles))
             report(c.status, kTimeoutBarrier, me, tid, 100);
     }
 }
 
 cudaError_t launch_dispatch(const DispatchArgs* a, int nv, cudaStream_t stream) {
-    return DX_LAUNCH_RANKED(dispatch_kernel, DispatchArgs, a, nv, a[0].num_sms, kDispatchThreads, 0, stream);
+    return DX_LAUNCH_RANKED_PDL(dispatch_kernel, DispatchArgs, a, nv, grid_ctas(a, nv), kDispatchThreads, 0, stream);
 }
 
 // =============================================================================================
@@ -397,9 +436,13 @@ template <int kRanks>
 __device__ __forceinline__ void combine_rows(const CombineArgs& a, const PeerSrc* s_src, int warp, int lane, int R) {
     const int T = a.num_tokens, H = a.hidden, K = a.num_topk;
     const int n16 = H / 8;
-    const int total_warps = a.num_sms * kCombineWarps;
-    constexpr int U = 2;
-    for (int t = blockIdx.x * kCombineWarps + warp; t < T; t += total_warps) {
+    const int pieces = row_pieces(T, n16, gridDim.x * kCombineWarps);
+    const int per = (((n16 + pieces - 1) / pieces) + 31) & ~31;
+    // columns per lane and pass: about sixteen 16-byte loads in flight whatever the number of ranks (eight with one rank, where
+    // two biases may come on top)
+    constexpr int U = kRanks == 1 ? 8 : (kRanks == 2 ? 4 : 2);
+    for (int item = blockIdx.x + gridDim.x * warp; item < T * pieces; item += gridDim.x * kCombineWarps) {
+        const int t = item / pieces, piece = item % pieces;
         int head = (lane < R) ? a.send_head[(size_t)t * R + lane] : -1;
         const int4* rowp[kRanks];
         const float* wp[kRanks];
@@ -411,54 +454,45 @@ __device__ __forceinline__ void combine_rows(const CombineArgs& a, const PeerSrc
             if (a.ctx.debug_extent != 0 && ok && !peer_range_ok(a.ctx, r, rowp[r], (size_t)n16 * 16, 2)) rowp[r] = nullptr;
             wp[r] = (ok && rowp[r] != nullptr && s_src[r].w != nullptr) ? s_src[r].w + (size_t)(s_src[r].base_row + h) * K : nullptr;
         }
-        const int4* b0 = a.bias0 ? reinterpret_cast<const int4*>(a.bias0) + (size_t)t * n16 : nullptr;
-        const int4* b1 = a.bias1 ? reinterpret_cast<const int4*>(a.bias1) + (size_t)t * n16 : nullptr;
+        const int4* bias[2] = {a.bias0 ? reinterpret_cast<const int4*>(a.bias0) + (size_t)t * n16 : nullptr,
+                               a.bias1 ? reinterpret_cast<const int4*>(a.bias1) + (size_t)t * n16 : nullptr};
         int4* out = reinterpret_cast<int4*>(a.out) + (size_t)t * n16;
-        for (int i0 = 0; i0 < n16; i0 += 32 * U) {
+        const int end = min(n16, (piece + 1) * per);
+        for (int i0 = piece * per; i0 < end; i0 += 32 * U) {
             int4 v[kRanks][U];
 #pragma unroll
             for (int r = 0; r < kRanks; ++r) {
 #pragma unroll
                 for (int u = 0; u < U; ++u) {
                     const int i = i0 + u * 32 + lane;
-                    v[r][u] = (rowp[r] != nullptr && i < n16) ? ld_peer(rowp[r] + i) : make_int4(0, 0, 0, 0);
+                    v[r][u] = (rowp[r] != nullptr && i < end) ? ld_peer(rowp[r] + i) : make_int4(0, 0, 0, 0);
                 }
+            }
+            // the first bias is requested together with the rows
+            int4 bv[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int i = i0 + u * 32 + lane;
+                bv[u] = (bias[0] != nullptr && i < end) ? ld_stream(bias[0] + i) : make_int4(0, 0, 0, 0);
             }
 #pragma unroll
             for (int u = 0; u < U; ++u) {
                 const int i = i0 + u * 32 + lane;
-                if (i >= n16) continue;
+                if (i >= end) continue;
                 float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-#pragma unroll
-                for (int r = 0; r < kRanks; ++r) {
-                    const uint32_t w[4] = {(uint32_t)v[r][u].x, (uint32_t)v[r][u].y, (uint32_t)v[r][u].z, (uint32_t)v[r][u].w};
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        const float2 p = bf16x2_to_f2(w[j]);
-                        acc[2 * j] += p.x;
-                        acc[2 * j + 1] += p.y;
-                    }
-                }
-                if (b0 != nullptr) {
-                    const int4 b = ld_cached(b0 + i);
-                    const uint32_t w[4] = {(uint32_t)b.x, (uint32_t)b.y, (uint32_t)b.z, (uint32_t)b.w};
+                auto add = [&](const int4& x) {
+                    const uint32_t w[4] = {(uint32_t)x.x, (uint32_t)x.y, (uint32_t)x.z, (uint32_t)x.w};
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
                         const float2 p = bf16x2_to_f2(w[j]);
                         acc[2 * j] += p.x;
                         acc[2 * j + 1] += p.y;
                     }
-                }
-                if (b1 != nullptr) {
-                    const int4 b = ld_cached(b1 + i);
-                    const uint32_t w[4] = {(uint32_t)b.x, (uint32_t)b.y, (uint32_t)b.z, (uint32_t)b.w};
+                };
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        const float2 p = bf16x2_to_f2(w[j]);
-                        acc[2 * j] += p.x;
-                        acc[2 * j + 1] += p.y;
-                    }
-                }
+                for (int r = 0; r < kRanks; ++r) add(v[r][u]);
+                if (bias[0] != nullptr) add(bv[u]);
+                if (bias[1] != nullptr) add(ld_cached(bias[1] + i));
                 int4 o;
                 o.x = (int)f2_to_bf16x2(acc[0], acc[1]);
                 o.y = (int)f2_to_bf16x2(acc[2], acc[3]);
@@ -467,7 +501,7 @@ __device__ __forceinline__ void combine_rows(const CombineArgs& a, const PeerSrc
                 st_stream(out + i, o);
             }
         }
-        if (a.out_topk_w != nullptr && lane < K) {
+        if (a.out_topk_w != nullptr && piece == 0 && lane < K) {
             float sum = 0.f;
 #pragma unroll
             for (int r = 0; r < kRanks; ++r)
@@ -479,6 +513,8 @@ __device__ __forceinline__ void combine_rows(const CombineArgs& a, const PeerSrc
 
 template <int V>
 __global__ void __launch_bounds__(kCombineThreads, 1) combine_kernel(const __grid_constant__ ArgPack<CombineArgs, V> pack) {
+    pdl_wait_predecessor();
+    pdl_release_successor();
     const CombineArgs& a = pack.a[blockIdx.y];
     const RankCtx& c = a.ctx;
     const int R = c.num_ranks, me = c.rank;
@@ -488,14 +524,14 @@ __global__ void __launch_bounds__(kCombineThreads, 1) combine_kernel(const __gri
     __shared__ int s_ok;
     if (tid == 0) s_ok = 1;
     __syncthreads();
-    // "my expert outputs are final and live at this offset" -> every home rank
-    if (blockIdx.x == 0 && tid < R) {
+    // "my expert outputs are final and live at this offset" -> every other home rank
+    if (blockIdx.x == 0 && tid < R && tid != me) {
         uint64_t w[2] = {a.x_off, a.topk_w_off};
         mailbox_post(c, kMbCombineSrc, tid, w, 2, seq);
     }
     if (tid < R) {
-        uint64_t w[2];
-        if (!mailbox_wait(c, kMbCombineSrc, tid, seq, w, 2)) {
+        uint64_t w[2] = {a.x_off, a.topk_w_off};
+        if (tid != me && !mailbox_wait(c, kMbCombineSrc, tid, seq, w, 2)) {
             report(c.status, kTimeoutCombineReady, me, tid, 0);
             s_ok = 0;
         } else {
@@ -514,21 +550,20 @@ __global__ void __launch_bounds__(kCombineThreads, 1) combine_kernel(const __gri
     else if (R <= 4) combine_rows<4>(a, s_src, warp, lane, R);
     else combine_rows<8>(a, s_src, warp, lane, R);
 
-    // Peers may reuse their expert-output buffers only after every home rank has finished reading.
+    // Peers may reuse their expert-output buffers only after every home rank has finished reading. (A lone rank: see dispatch.)
+    if (R == 1) return;
     if (cta_is_last(c.local_scratch + kTicketCombine, gridDim.x)) {
-        if (tid < R) {
-            st_release_sys(&c.ctrl(tid)->barrier_in[kBarCombine][me], seq);
-        }
+        if (tid < R && tid != me) st_release_sys(&c.ctrl(tid)->barrier_in[kBarCombine][me], seq);
         if (tid == 0) commit_seq(c, kFamCombine, seq);
     }
-    if (blockIdx.x == 0 && tid < R) {
+    if (blockIdx.x == 0 && tid < R && tid != me) {
         if (!wait_ge_sys(&c.my_ctrl()->barrier_in[kBarCombine][tid], seq, c.timeout_cycles))
             report(c.status, kTimeoutBarrier, me, tid, 200);
     }
 }
 
 cudaError_t launch_combine(const CombineArgs* a, int nv, cudaStream_t stream) {
-    return DX_LAUNCH_RANKED(combine_kernel, CombineArgs, a, nv, a[0].num_sms, kCombineThreads, 0, stream);
+    return DX_LAUNCH_RANKED_PDL(combine_kernel, CombineArgs, a, nv, grid_ctas(a, nv), kCombineThreads, 0, stream);
 }
 
 // =============================================================================================

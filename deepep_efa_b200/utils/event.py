@@ -15,6 +15,17 @@ from typing import Any, Optional, Tuple
 import torch
 
 
+_HAS_CUDA: Optional[bool] = None
+
+
+def _has_cuda() -> bool:
+    """``torch.cuda.is_available()``, asked once: it queries the driver on every call."""
+    global _HAS_CUDA
+    if _HAS_CUDA is None:
+        _HAS_CUDA = torch.cuda.is_available()
+    return _HAS_CUDA
+
+
 class EventHandle:
     """A CUDA event recorded on ``stream`` (default: the current stream) when created.
 
@@ -22,7 +33,7 @@ class EventHandle:
 
     def __init__(self, stream: Optional["torch.cuda.Stream"] = None, record: bool = True) -> None:
         self.event = None
-        if torch.cuda.is_available():
+        if _has_cuda():
             self.event = torch.cuda.Event(enable_timing=False)
             if record:
                 self.event.record(stream if stream is not None else torch.cuda.current_stream())

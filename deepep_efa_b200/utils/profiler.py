@@ -26,17 +26,21 @@ PROFILE_WARMUP = int(os.environ.get("DEEPEP_PROFILE_WARMUP", "10"))
 _NVTX = os.environ.get("DEEPEP_NVTX", "0") == "1"
 
 
-@contextlib.contextmanager
+_NO_RANGE = contextlib.nullcontext()
+
+
 def nvtx_range(name: str):
     """NVTX range when ``DEEPEP_NVTX=1`` and CUDA is present; otherwise free."""
-    if _NVTX and torch.cuda.is_available():
-        torch.cuda.nvtx.range_push(name)
-        try:
-            yield
-        finally:
-            torch.cuda.nvtx.range_pop()
-    else:
+    return _nvtx_range(name) if _NVTX and torch.cuda.is_available() else _NO_RANGE
+
+
+@contextlib.contextmanager
+def _nvtx_range(name: str):
+    torch.cuda.nvtx.range_push(name)
+    try:
         yield
+    finally:
+        torch.cuda.nvtx.range_pop()
 
 
 class PhaseProfiler:
