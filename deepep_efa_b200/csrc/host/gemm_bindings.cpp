@@ -2,6 +2,7 @@
 // changes do not rebuild the runtime bindings).
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
+#include <pybind11/stl.h>
 #include <torch/extension.h>
 
 #include <map>
@@ -64,7 +65,7 @@ torch::Tensor grouped_gemm(const torch::Tensor& a, const torch::Tensor& b, const
                            c10::optional<torch::Tensor> ready, c10::optional<torch::Tensor> expected,
                            c10::optional<torch::Tensor> row_info, c10::optional<torch::Tensor> scatter_bases,
                            c10::optional<torch::Tensor> trace, bool mn_major, c10::optional<torch::Tensor> out_fp8,
-                           c10::optional<torch::Tensor> out_atoms) {
+                           c10::optional<torch::Tensor> out_atoms, bool m_ends_are_counts) {
     DXG_CHECK(a.is_cuda() && b.is_cuda() && m_offsets.is_cuda(), "operands must be CUDA tensors");
     DXG_CHECK(a.is_contiguous() && b.is_contiguous() && m_offsets.is_contiguous(), "operands must be contiguous");
     DXG_CHECK(m_offsets.scalar_type() == torch::kInt32 && m_offsets.dim() == 1 && m_offsets.numel() >= 2, "m_offsets must be int32 [G+1]");
@@ -148,6 +149,7 @@ torch::Tensor grouped_gemm(const torch::Tensor& a, const torch::Tensor& b, const
     if (m_ends.has_value()) {
         DXG_CHECK(mode == 0 && m_ends->is_cuda() && m_ends->scalar_type() == torch::kInt32 && m_ends->is_contiguous() && m_ends->numel() == G, "m_ends must be int32 [G] on the GPU (M-grouped mode only)");
         p.m_ends = m_ends->data_ptr<int>();
+        p.m_ends_are_counts = m_ends_are_counts ? 1 : 0;
     }
     p.num_sms = num_sms > 0 ? num_sms : sm_count(device);
     {
@@ -207,38 +209,51 @@ torch::Tensor grouped_gemm(const torch::Tensor& a, const torch::Tensor& b, const
     return c;
 }
 
-std::tuple<torch::Tensor, torch::Tensor, torch::Tensor> build_plan(const torch::Tensor& topk_idx, const torch::Tensor& m_offsets, int64_t m_pad) {
+// counts: 128-aligned rows per local expert. Returns (pos [N,K], src_row [m_pad], src_k [m_pad], m_offsets [L+1], m_pad).
+std::tuple<torch::Tensor, torch::Tensor, torch::Tensor, torch::Tensor, int64_t> build_plan(const torch::Tensor& topk_idx, const std::vector<int>& counts) {
     DXG_CHECK(topk_idx.is_cuda() && topk_idx.dim() == 2 && topk_idx.is_contiguous() && topk_idx.scalar_type() == torch::kInt64, "topk_idx must be contiguous int64 [N,K] on the GPU");
-    DXG_CHECK(m_offsets.is_cuda() && m_offsets.scalar_type() == torch::kInt32 && m_offsets.is_contiguous() && m_offsets.numel() >= 2, "m_offsets must be int32 [L+1] on the GPU");
-    const int64_t N = topk_idx.size(0), K = topk_idx.size(1), L = m_offsets.numel() - 1;
+    const int64_t N = topk_idx.size(0), K = topk_idx.size(1), L = (int64_t)counts.size();
+    DXG_CHECK(L >= 1 && L <= dx::kPlanMaxExperts, "between 1 and 1024 local experts");
+    std::vector<int> offs(L + 1, 0);
+    for (int64_t e = 0; e < L; ++e) offs[e + 1] = offs[e] + counts[e];
+    const int64_t m_pad = offs[L];
     c10::cuda::CUDAGuard guard(topk_idx.device());
     auto i32 = topk_idx.options().dtype(torch::kInt32);
-    auto pos = torch::empty({N, K}, i32), src_row = torch::empty({m_pad}, i32), src_k = torch::empty({m_pad}, i32), counters = torch::empty({L}, i32);
-    const cudaError_t e = dx::launch_build_plan(topk_idx.data_ptr<int64_t>(), m_offsets.data_ptr<int>(), counters.data_ptr<int>(), pos.data_ptr<int>(),
-                                                src_row.data_ptr<int>(), src_k.data_ptr<int>(), (int)N, (int)K, (int)L, (int)m_pad,
+    auto pos = torch::empty({N, K}, i32), src_row = torch::empty({m_pad}, i32), src_k = torch::empty({m_pad}, i32), m_offsets = torch::empty({L + 1}, i32);
+    const cudaError_t e = dx::launch_build_plan(topk_idx.data_ptr<int64_t>(), offs.data(), m_offsets.data_ptr<int>(), pos.data_ptr<int>(),
+                                                src_row.data_ptr<int>(), src_k.data_ptr<int>(), (int)N, (int)K, (int)L,
                                                 at::cuda::getCurrentCUDAStream(topk_idx.device().index()).stream());
     if (e != cudaSuccess) throw std::runtime_error(std::string("build_plan: ") + cudaGetErrorString(e));
-    return {pos, src_row, src_k};
+    return {pos, src_row, src_k, m_offsets, m_pad};
 }
 
-// dst[m] = scale[m] * src[src_row[m]]; rows of any dtype whose byte size is a multiple of 16
+// dst[m] = scale * src[src_row[m]]; rows of any dtype whose byte size is a multiple of 4 (of 16 with a scale, which needs bf16).
+// The scale of row m is scale[m], or with src_k ([M]) scale[src_row[m], src_k[m]] of a matrix.
 torch::Tensor gather_rows(const torch::Tensor& src, const torch::Tensor& src_row, c10::optional<torch::Tensor> scale,
-                          c10::optional<torch::Tensor> out) {
+                          c10::optional<torch::Tensor> out, c10::optional<torch::Tensor> src_k) {
     DXG_CHECK(src.is_cuda() && src.dim() == 2 && src.is_contiguous(), "src must be a contiguous CUDA matrix");
     DXG_CHECK(src_row.scalar_type() == torch::kInt32 && src_row.is_contiguous() && src_row.dim() == 1, "src_row must be int32 [M]");
     const int64_t M = src_row.numel();
     const int64_t row_bytes = src.size(1) * src.element_size();
-    DXG_CHECK(row_bytes % 16 == 0, "row size must be a multiple of 16 bytes");
+    DXG_CHECK(row_bytes % (scale.has_value() ? 16 : 4) == 0, "row size must be a multiple of 4 bytes (16 with a scale)");
     c10::cuda::CUDAGuard guard(src.device());
     torch::Tensor dst = out.has_value() ? *out : torch::empty({M, src.size(1)}, src.options());
     DXG_CHECK(dst.is_contiguous() && dst.scalar_type() == src.scalar_type() && dst.size(0) == M && dst.size(1) == src.size(1), "out has the wrong shape");
     const float* sc = nullptr;
+    int num_k = 0;
     if (scale.has_value()) {
-        DXG_CHECK(src.scalar_type() == torch::kBFloat16 && scale->scalar_type() == torch::kFloat32 && scale->numel() == M && scale->is_contiguous(), "scale needs bf16 rows and f32 [M]");
+        DXG_CHECK(src.scalar_type() == torch::kBFloat16 && scale->scalar_type() == torch::kFloat32 && scale->is_contiguous(), "scale needs bf16 rows and must be f32");
+        if (src_k.has_value()) {
+            DXG_CHECK(scale->dim() == 2 && scale->size(0) == src.size(0) && src_k->scalar_type() == torch::kInt32 && src_k->is_contiguous() && src_k->numel() == M,
+                      "with src_k (int32 [M]) the scale is a matrix with one row per source row");
+            num_k = (int)scale->size(1);
+        } else {
+            DXG_CHECK(scale->numel() == M, "scale must be f32 [M]");
+        }
         sc = scale->data_ptr<float>();
     }
-    const cudaError_t e = dx::launch_gather_rows(src.data_ptr(), dst.data_ptr(), src_row.data_ptr<int>(), sc, (int)M, (int)row_bytes,
-                                                 at::cuda::getCurrentCUDAStream(src.device().index()).stream());
+    const cudaError_t e = dx::launch_gather_rows(src.data_ptr(), dst.data_ptr(), src_row.data_ptr<int>(), sc, num_k > 0 ? src_k->data_ptr<int>() : nullptr, num_k,
+                                                 (int)M, (int)row_bytes, at::cuda::getCurrentCUDAStream(src.device().index()).stream());
     if (e != cudaSuccess) throw std::runtime_error(std::string("gather_rows: ") + cudaGetErrorString(e));
     return dst;
 }
@@ -349,9 +364,10 @@ void bind_gemm(py::module_& m) {
           py::arg("timeout_ms") = 2000.0, py::arg("m_ends") = py::none(), py::arg("sfa_atoms") = py::none(), py::arg("sfb_atoms") = py::none(),
           py::arg("ready") = py::none(), py::arg("expected") = py::none(), py::arg("row_info") = py::none(),
           py::arg("scatter_bases") = py::none(), py::arg("trace") = py::none(), py::arg("mn_major") = false,
-          py::arg("out_fp8") = py::none(), py::arg("out_atoms") = py::none());
+          py::arg("out_fp8") = py::none(), py::arg("out_atoms") = py::none(), py::arg("m_ends_are_counts") = false);
     m.def("build_plan", &build_plan);
-    m.def("gather_rows", &gather_rows, py::arg("src"), py::arg("src_row"), py::arg("scale") = py::none(), py::arg("out") = py::none());
+    m.def("gather_rows", &gather_rows, py::arg("src"), py::arg("src_row"), py::arg("scale") = py::none(), py::arg("out") = py::none(),
+          py::arg("src_k") = py::none());
     m.def("gather_reduce_rows", &gather_reduce_rows, py::arg("src"), py::arg("pos"), py::arg("w") = py::none(), py::arg("out") = py::none());
     m.def("gemm_error", &gemm_error);
     m.def("gemm_clear_error", &gemm_clear_error);

@@ -9,6 +9,7 @@
 // Reference counterpart: per_token_cast_to_fp8_kernel, csrc/kernels/efa_kernels.cu:104-187 (grid
 // (hidden/128, M) x 128 threads, UE8M0 packing through atomicOr).
 #include "api.h"
+#include "launch.cuh"
 #include "prims.cuh"
 
 namespace dx {
@@ -16,6 +17,8 @@ namespace dx {
 constexpr int kCastThreads = 256;
 
 __global__ void __launch_bounds__(kCastThreads) fp8_cast_kernel(const Fp8CastArgs a) {
+    pdl_wait_predecessor();
+    pdl_release_successor();
     const int lane = threadIdx.x & 31;
     const int row = blockIdx.x * (kCastThreads / 32) + (threadIdx.x >> 5);
     if (row >= a.num_rows) return;
@@ -76,8 +79,7 @@ __global__ void __launch_bounds__(kCastThreads) fp8_cast_kernel(const Fp8CastArg
 cudaError_t launch_fp8_cast(const Fp8CastArgs& a, cudaStream_t stream) {
     if (a.num_rows == 0) return cudaSuccess;
     const int rows_per_cta = kCastThreads / 32;
-    fp8_cast_kernel<<<(a.num_rows + rows_per_cta - 1) / rows_per_cta, kCastThreads, 0, stream>>>(a);
-    return cudaGetLastError();
+    return launch_dependent(fp8_cast_kernel, dim3((a.num_rows + rows_per_cta - 1) / rows_per_cta), kCastThreads, 0, stream, a);
 }
 
 }  // namespace dx

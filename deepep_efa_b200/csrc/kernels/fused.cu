@@ -20,81 +20,52 @@
 // The reference dispatches rank-major through ring queues (csrc/kernels/intranode.cu:197-610) and leaves the
 // expert-major permutation to its users; it has no counterpart of the arrival gating.
 #include "api.h"
-#include "prims.cuh"
 #include "launch.cuh"
+#include "prims.cuh"
+#include "row_reduce.cuh"
+#include "select_scan.cuh"
 
 namespace dx {
 
 // One warp per expert scans all selections, so the scan's length is fixed; what varies is how many such warps share an SM's four
 // schedulers. Four warps per CTA (64 CTAs for 256 experts) give every scanning warp a scheduler of its own.
-constexpr int kEmNotifyThreads = 128;
+constexpr int kEmNotifyThreads = kScanThreads;
 constexpr int kEmNotifyWarps = kEmNotifyThreads / 32;
-constexpr int kEmChunk = 16384;          // selections staged in shared memory per pass (uint16 expert ids)
 constexpr int kTicketFused = 5;
 
 __device__ __forceinline__ int align128(int v) { return (v + 127) & ~127; }
 
+// Experts of one CTA: as few as the SMs allow (a CTA scans all selections whatever their number, see select_scan.cuh). 256 experts,
+// 4096 x 8 selections on one B200: 104 us with one warp per expert and the ids staged in shared memory, 14 us this way.
+__host__ __device__ constexpr int em_experts_per_cta(int num_experts, int ctas) { return (num_experts + ctas - 1) / ctas; }
+
 template <int V>
 __global__ void __launch_bounds__(kEmNotifyThreads, 1) em_notify_kernel(const __grid_constant__ ArgPack<EmNotifyArgs, V> pack) {
+    pdl_wait_predecessor();
+    pdl_release_successor();
     const EmNotifyArgs& a = pack.a[blockIdx.y];
     const RankCtx& c = a.ctx;
     const int R = c.num_ranks, me = c.rank, T = a.num_tokens, K = a.num_topk, E = a.num_experts, L = E / R;
-    const int TK = T * K;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint64_t seq = next_seq(c, kFamFused);
     extern __shared__ int s_dyn[];
-    uint16_t* s_sel = reinterpret_cast<uint16_t*>(s_dyn);  // [kEmChunk] expert id of a chunk of selections (0xFFFF = none)
 
-    // ---- every CTA: one warp per expert collects that expert's selections in token order ----
-    const int e = blockIdx.x * kEmNotifyWarps + warp;
-    int run = 0;
-    for (int c0 = 0; c0 < TK; c0 += kEmChunk) {
-        const int n = min(kEmChunk, TK - c0);
-        __syncthreads();
-        if (((reinterpret_cast<uintptr_t>(a.topk_idx + c0)) & 15) == 0) {
-            // two ids per 16-byte load
-            const longlong2* src2 = reinterpret_cast<const longlong2*>(a.topk_idx + c0);
-#pragma unroll 8
-            for (int i = tid; i < n / 2; i += kEmNotifyThreads) {
-                const longlong2 v = src2[i];
-                const uint32_t lo = (v.x >= 0 && v.x < E) ? (uint32_t)v.x : 0xFFFFu, hi = (v.y >= 0 && v.y < E) ? (uint32_t)v.y : 0xFFFFu;
-                reinterpret_cast<uint32_t*>(s_sel)[i] = lo | (hi << 16);
-            }
-            if ((n & 1) && tid == 0) {
-                const int64_t v = a.topk_idx[c0 + n - 1];
-                s_sel[n - 1] = (v >= 0 && v < E) ? (uint16_t)v : (uint16_t)0xFFFF;
-            }
-        } else {
-            for (int i = tid; i < n; i += kEmNotifyThreads) {
-                const int64_t v = a.topk_idx[c0 + i];
-                s_sel[i] = (v >= 0 && v < E) ? (uint16_t)v : (uint16_t)0xFFFF;
-            }
-        }
-        __syncthreads();
-        if (e < E) {
-            // four groups of 32 selections per step, so that four shared-memory loads and votes are in flight at a time
-            for (int i0 = 0; i0 < n; i0 += 128) {
-                bool hit[4];
-                unsigned b[4];
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const int i = i0 + u * 32 + lane;
-                    hit[u] = i < n && s_sel[i] == (uint16_t)e;
-                }
-#pragma unroll
-                for (int u = 0; u < 4; ++u) b[u] = __ballot_sync(0xffffffffu, hit[u]);
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    if (hit[u]) {
-                        const int slot = run + __popc(b[u] & ((1u << lane) - 1));
-                        if (slot < T) a.sel_list[(size_t)e * T + slot] = c0 + i0 + u * 32 + lane;  // an expert is selected at most once per token
-                    }
-                    run += __popc(b[u]);
-                }
-            }
+    // ---- every CTA: the selections of its experts in token order ----
+    const int per_cta = em_experts_per_cta(E, gridDim.x);
+    const int e0 = blockIdx.x * per_cta, ne = max(0, min(per_cta, E - e0));
+    {
+        int* s_run = s_dyn;
+        uint32_t* s_vote = reinterpret_cast<uint32_t*>(s_dyn + kScanBatch);
+        for (int b0 = 0; b0 < ne; b0 += kScanBatch) {
+            const int nb = min(kScanBatch, ne - b0);
+            scan_selections(a.topk_idx, T * K, E, e0 + b0, nb, s_vote, s_run, false,
+                            [&](int j, int n, int i) {
+                                if (n < T) a.sel_list[(size_t)(e0 + b0 + j) * T + n] = i;  // an expert is selected at most once per token
+                            },
+                            [](int) {});
+            for (int j = tid; j < nb; j += kEmNotifyThreads) a.my_counts[e0 + b0 + j] = min(s_run[j], T);
         }
     }
-    if (e < E && lane == 0) a.my_counts[e] = min(run, T);
 
     // ---- the last CTA to finish exchanges the counts and derives the plan ----
     if (!cta_is_last(c.local_scratch + kTicketFused, gridDim.x)) return;
@@ -117,7 +88,7 @@ __global__ void __launch_bounds__(kEmNotifyThreads, 1) em_notify_kernel(const __
         }
     }
     __syncthreads();
-    if (tid < R) {
+    if (tid < R && tid != me) {  // my own words are ordered by the barrier above
         st_release_sys(&c.ctrl(tid)->em_seq[me], seq);
         if (!wait_ge_sys(&c.my_ctrl()->em_seq[tid], seq, c.timeout_cycles)) {
             report(c.status, kTimeoutFusedNotify, me, tid, 0);
@@ -201,9 +172,12 @@ __global__ void __launch_bounds__(kEmNotifyThreads, 1) em_notify_kernel(const __
 cudaError_t launch_em_notify(const EmNotifyArgs* a, int nv, cudaStream_t stream) {
     const int E = a[0].num_experts;
     if (E < 1 || E > kMaxFusedExperts || E % a[0].ctx.num_ranks != 0 || a[0].unit_rows < 1) return cudaErrorInvalidValue;
-    const size_t smem = (size_t)(kEmChunk * 2 > 4 * E * 4 ? kEmChunk * 2 : 4 * E * 4);
-    const int ctas = (E + kEmNotifyWarps - 1) / kEmNotifyWarps;
-    return DX_LAUNCH_RANKED(em_notify_kernel, EmNotifyArgs, a, nv, ctas, kEmNotifyThreads, smem, stream);
+    const int fit = nv == 1 ? 148 : 148 / nv - 1;  // emulated ranks must be co-resident
+    const int per_cta = em_experts_per_cta(E, E < fit ? E : fit);
+    const int ctas = (E + per_cta - 1) / per_cta;
+    const size_t scan = scan_smem_bytes(per_cta), plan = (size_t)4 * E * sizeof(int);
+    const size_t smem = scan > plan ? scan : plan;
+    return DX_LAUNCH_RANKED_PDL(em_notify_kernel, EmNotifyArgs, a, nv, ctas, kEmNotifyThreads, smem, stream);
 }
 
 // =============================================================================================
@@ -220,6 +194,7 @@ __device__ __forceinline__ unsigned long long global_timer() {
 
 template <int V>
 __global__ void __launch_bounds__(kEmDispatchThreads, 6) em_dispatch_kernel(const __grid_constant__ ArgPack<EmDispatchArgs, V> pack) {
+    pdl_wait_predecessor();
     const EmDispatchArgs& a = pack.a[blockIdx.y];
     const RankCtx& c = a.ctx;
     const int R = c.num_ranks, me = c.rank, T = a.num_tokens, K = a.num_topk, E = a.num_experts, L = E / R, H = a.hidden;
@@ -370,7 +345,11 @@ __global__ void __launch_bounds__(kEmDispatchThreads, 6) em_dispatch_kernel(cons
         }
         __syncwarp();
         // one release per unit: everything this warp stored for expert (d, le) is visible before the counter moves
-        if (lane == 0 && sent > 0) red_add_release_sys(&c.ctrl(d)->em_arrived[le], (uint64_t)sent);
+        if (lane == 0 && sent > 0) {
+            // (rows for an expert of this GPU need no more than GPU scope: their reader is a kernel of this GPU)
+            if (d == me) red_add_release_gpu(&c.ctrl(d)->em_arrived[le], (uint64_t)sent);
+            else red_add_release_sys(&c.ctrl(d)->em_arrived[le], (uint64_t)sent);
+        }
     }
     if (a.trace != nullptr) {
         __syncthreads();
@@ -381,89 +360,39 @@ __global__ void __launch_bounds__(kEmDispatchThreads, 6) em_dispatch_kernel(cons
 cudaError_t launch_em_dispatch(const EmDispatchArgs* a, int nv, cudaStream_t stream) {
     if (a[0].hidden % 128 != 0 || a[0].num_sms < 1) return cudaErrorInvalidValue;
     const size_t smem = (size_t)(a[0].num_experts + 1) * sizeof(int);
-    return DX_LAUNCH_RANKED(em_dispatch_kernel, EmDispatchArgs, a, nv, a[0].num_sms, kEmDispatchThreads, smem, stream);
+    return DX_LAUNCH_RANKED_PDL(em_dispatch_kernel, EmDispatchArgs, a, nv, a[0].num_sms, kEmDispatchThreads, smem, stream);
 }
 
 // =============================================================================================
 // home-side reduction of the scattered expert outputs
 // =============================================================================================
-constexpr int kStageReduceThreads = 256;
-
 // out[t] = sum_k w[t,k] * stage[t*K + k] over the valid selections of token t (fp32 accumulate, fixed k order).
-__global__ void __launch_bounds__(kStageReduceThreads) stage_reduce_kernel(const __nv_bfloat16* __restrict__ stage, __nv_bfloat16* __restrict__ out,
-                                                                          const int64_t* __restrict__ topk_idx, const float* __restrict__ w,
-                                                                          int num_tokens, int num_topk, int num_experts, int hidden) {
+__global__ void __launch_bounds__(kReduceThreads) stage_reduce_kernel(const __nv_bfloat16* __restrict__ stage, __nv_bfloat16* __restrict__ out,
+                                                                      const int64_t* __restrict__ topk_idx, const float* __restrict__ w,
+                                                                      int num_tokens, int num_topk, int num_experts, int hidden) {
+    pdl_wait_predecessor();
+    pdl_release_successor();
     const int lane = threadIdx.x & 31;
-    const int t = blockIdx.x * (kStageReduceThreads / 32) + (threadIdx.x >> 5);
+    const int n16 = hidden / 8, spans = reduce_spans(n16);
+    const int item = blockIdx.x * (kReduceThreads / 32) + (threadIdx.x >> 5);
+    const int t = item / spans;
     if (t >= num_tokens) return;
-    const int n16 = hidden / 8;
-    bool ok = false;
+    int row = -1;
     float my_w = 0.f;
     if (lane < num_topk) {
         const int64_t e = topk_idx[(size_t)t * num_topk + lane];
-        ok = e >= 0 && e < num_experts;
-        my_w = ok ? w[(size_t)t * num_topk + lane] : 0.f;
+        my_w = w[(size_t)t * num_topk + lane];
+        if (e >= 0 && e < num_experts) row = t * num_topk + lane;
     }
-    const unsigned valid = __ballot_sync(0xffffffffu, ok);
-    const int4* rows = reinterpret_cast<const int4*>(stage) + (size_t)t * num_topk * n16;
-    int4* d = reinterpret_cast<int4*>(out) + (size_t)t * n16;
-    constexpr int U = 2;
-    for (int i0 = 0; i0 < n16; i0 += 32 * U) {
-        float acc[U][8];
-#pragma unroll
-        for (int u = 0; u < U; ++u)
-#pragma unroll
-            for (int q = 0; q < 8; ++q) acc[u][q] = 0.f;
-        // eight selections x two columns: sixteen 16-byte loads in flight per lane before the first one is consumed
-        for (int k0 = 0; k0 < num_topk; k0 += 8) {
-            int4 v[8][U];
-#pragma unroll
-            for (int kk = 0; kk < 8; ++kk) {
-                const int k = k0 + kk;
-                const bool kv = k < num_topk && ((valid >> k) & 1u);
-#pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    const int i = i0 + u * 32 + lane;
-                    v[kk][u] = (kv && i < n16) ? ld_stream(rows + (size_t)k * n16 + i) : make_int4(0, 0, 0, 0);
-                }
-            }
-#pragma unroll
-            for (int kk = 0; kk < 8; ++kk) {
-                const float wk = __shfl_sync(0xffffffffu, my_w, (k0 + kk) & 31);
-#pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    const uint32_t w4[4] = {(uint32_t)v[kk][u].x, (uint32_t)v[kk][u].y, (uint32_t)v[kk][u].z, (uint32_t)v[kk][u].w};
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        const float2 f = bf16x2_to_f2(w4[q]);
-                        acc[u][2 * q] = fmaf(wk, f.x, acc[u][2 * q]);
-                        acc[u][2 * q + 1] = fmaf(wk, f.y, acc[u][2 * q + 1]);
-                    }
-                }
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int i = i0 + u * 32 + lane;
-            if (i >= n16) continue;
-            int4 o;
-            o.x = (int)f2_to_bf16x2(acc[u][0], acc[u][1]);
-            o.y = (int)f2_to_bf16x2(acc[u][2], acc[u][3]);
-            o.z = (int)f2_to_bf16x2(acc[u][4], acc[u][5]);
-            o.w = (int)f2_to_bf16x2(acc[u][6], acc[u][7]);
-            d[i] = o;
-        }
-    }
+    reduce_row_span(reinterpret_cast<const int4*>(stage), reinterpret_cast<int4*>(out) + (size_t)t * n16, n16, item % spans, num_topk, row, my_w, lane);
 }
 
 cudaError_t launch_stage_reduce(const void* stage, void* out, const int64_t* topk_idx, const float* w, int num_tokens, int num_topk,
                                 int num_experts, int hidden, cudaStream_t stream) {
     if (num_tokens <= 0) return cudaSuccess;
     if (hidden % 8 != 0 || num_topk < 1 || num_topk > 32) return cudaErrorInvalidValue;
-    const int per = kStageReduceThreads / 32;
-    stage_reduce_kernel<<<(num_tokens + per - 1) / per, kStageReduceThreads, 0, stream>>>(
-        static_cast<const __nv_bfloat16*>(stage), static_cast<__nv_bfloat16*>(out), topk_idx, w, num_tokens, num_topk, num_experts, hidden);
-    return cudaGetLastError();
+    return launch_dependent(stage_reduce_kernel, dim3(reduce_ctas(num_tokens, hidden / 8)), kReduceThreads, 0, stream, static_cast<const __nv_bfloat16*>(stage),
+                            static_cast<__nv_bfloat16*>(out), topk_idx, w, num_tokens, num_topk, num_experts, hidden);
 }
 
 }  // namespace dx

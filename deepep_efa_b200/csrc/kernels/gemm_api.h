@@ -35,6 +35,7 @@ struct GroupedGemmArgs {
     const int* m_offsets;     // [G+1] device memory
     const int* m_ends;        // optional [G]: group g covers rows [m_offsets[g], m_ends[g]) instead of up to m_offsets[g+1]
                               // (mode 0 only; the low-latency layout has fixed group starts and a count per expert)
+    int m_ends_are_counts;    // 1 = m_ends[g] is the number of rows of group g instead of its end
     int num_groups;
     int mode;                 // 0 = M-grouped, 1 = K-grouped
     int fp8;                  // 0 = bf16 operands, 1 = e4m3 operands (mode 0 only)
@@ -75,15 +76,17 @@ struct GroupedGemmArgs {
 // Returns cudaErrorInvalidValue for unsupported shapes (divisibility rules are in grouped_gemm.cu).
 cudaError_t launch_grouped_gemm(const GroupedGemmArgs& args, cudaStream_t stream);
 
-// Expert-major plan from local expert ids [N, K] (-1 = unselected) and 128-aligned group offsets [L+1]:
-// pos [N*K], src_row [m_pad] (-1 = padding), src_k [m_pad]; counters is an int[L] scratch.
-cudaError_t launch_build_plan(const int64_t* topk_idx, const int* m_offsets, int* counters, int* pos, int* src_row, int* src_k,
-                              int num_rows, int num_topk, int num_local_experts, int m_pad, cudaStream_t stream);
+// Expert-major plan from local expert ids [N, K] (-1 = unselected) and 128-aligned group offsets [L+1] on the host:
+// m_offsets [L+1] (the offsets on the device), pos [N*K], src_row [m_pad] (-1 = padding), src_k [m_pad] (0 there).
+constexpr int kPlanMaxExperts = 1024;  // local experts; the offsets travel as kernel arguments (4 KiB)
+cudaError_t launch_build_plan(const int64_t* topk_idx, const int* host_offsets, int* m_offsets, int* pos, int* src_row, int* src_k,
+                              int num_rows, int num_topk, int num_local_experts, cudaStream_t stream);
 
 // Row gathers between receive order and the expert-major, 128-row-aligned layout (permute.cu).
-//   dst[m] = scale[m] * src[src_row[m]]   (src_row[m] < 0 -> zero row; scale may be null; bf16 rows when scaled)
-cudaError_t launch_gather_rows(const void* src, void* dst, const int* src_row, const float* scale, int num_dst_rows, int row_bytes,
-                               cudaStream_t stream);
+//   dst[m] = scale * src[src_row[m]]   (src_row[m] < 0 -> zero row; scale may be null; bf16 rows when scaled). The scale of row m is
+//   scale[m], or with num_k > 0 scale[src_row[m] * num_k + src_k[m]]. Rows are multiples of 4 bytes (of 16 when scaled).
+cudaError_t launch_gather_rows(const void* src, void* dst, const int* src_row, const float* scale, const int* src_k, int num_k, int num_dst_rows,
+                               int row_bytes, cudaStream_t stream);
 //   dst[n] = sum_k w[n,k] * src[pos[n,k]]  (bf16 rows, fp32 accumulate; pos < 0 skipped; w may be null = 1)
 cudaError_t launch_gather_reduce_rows(const void* src, void* dst, const int* pos, const float* w, int num_dst_rows, int num_k, int hidden,
                                       cudaStream_t stream);

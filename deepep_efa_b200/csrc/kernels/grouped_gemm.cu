@@ -25,6 +25,7 @@
 #include <cstring>
 
 #include "gemm_api.h"
+#include "launch.cuh"
 #include "prims.cuh"
 
 namespace dx {
@@ -364,6 +365,12 @@ __device__ __forceinline__ void store_rows_256(int4* stage, const int4 (&regs)[1
     }
 }
 
+// Rows of group g (mode 0), which starts at row `begin`.
+__device__ __forceinline__ int group_rows(const GroupedGemmArgs& p, int g, int begin) {
+    if (p.m_ends == nullptr) return max(p.m_offsets[g + 1] - begin, 0);
+    return max(p.m_ends_are_counts ? p.m_ends[g] : p.m_ends[g] - begin, 0);
+}
+
 struct TileInfo {
     int a_row, a_k0, b_row, b_row2, b_k0, num_kb, c_row, c_col, group, nblock, nblock2;
     int c_row_end;  // first output row this tile must not write (end of its group; groups need no 128-row alignment)
@@ -453,23 +460,32 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         tma_prefetch_desc(&map_a);
         tma_prefetch_desc(&map_b);
-        // tile table
-        int run = 0;
+    }
+    // What precedes overlaps the end of the previous kernel (programmatic dependent launch); from here on its results are read.
+    // The successor is released only now, so that a kernel that starts early finds every kernel before this one complete.
+    pdl_wait_predecessor();
+    pdl_release_successor();
+    if (warp == 2) {
+        // tile table: one warp scans the groups (one thread walking 256 groups through dependent loads took about 10 us)
         const int tiles_n = p.mode == 0 ? p.n / kBlockN : 0;
         const int tiles_fixed = p.mode == 1 ? ((p.n + C::kTileRows - 1) / C::kTileRows) * (p.k / kBlockN) : 0;
-        for (int g = 0; g < G; ++g) {
-            tile_start[g] = run;
-            // native block scaling reads one scale atom per 128-row tile, so a group that does not start on a tile boundary
-            // would be scaled with its neighbour's factors: flag it (value 2) instead of returning silently wrong numbers
-            if (kMx && (p.m_offsets[g] & 127) != 0 && p.error_flag != nullptr) atomicExch(p.error_flag, 2);
-            if (p.mode == 0) {
-                const int rows = (p.m_ends != nullptr ? p.m_ends[g] : p.m_offsets[g + 1]) - p.m_offsets[g];
-                run += ((max(rows, 0) + C::kTileRows - 1) / C::kTileRows) * tiles_n;
-            } else {
-                run += tiles_fixed;
+        int run = 0;
+        for (int g0 = 0; g0 < G; g0 += 32) {
+            const int g = g0 + lane;
+            int tiles = 0;
+            if (g < G) {
+                const int begin = p.m_offsets[g];
+                // native block scaling reads one scale atom per 128-row tile, so a group that does not start on a tile boundary
+                // would be scaled with its neighbour's factors: flag it (value 2) instead of returning silently wrong numbers
+                if (kMx && (begin & 127) != 0 && p.error_flag != nullptr) atomicExch(p.error_flag, 2);
+                if (p.mode == 0) tiles = ((group_rows(p, g, begin) + C::kTileRows - 1) / C::kTileRows) * tiles_n;
+                else tiles = tiles_fixed;
             }
+            const int incl = warp_incl_scan(tiles);
+            if (g < G) tile_start[g] = run + incl - tiles;
+            run += __shfl_sync(0xffffffffu, incl, 31);
         }
-        tile_start[G] = run;
+        if (lane == 0) tile_start[G] = run;
     }
     if constexpr (C::kSplitDrain) {
         for (int i = threadIdx.x; i < C::kXchBytes / 8; i += C::kThreads) xch[i] = 0ull;
@@ -492,7 +508,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     auto decode = [&](int tile, int& g, TileInfo& ti) {
         while (tile >= tile_start[g + 1]) ++g;
         const int local = tile - tile_start[g];
-        const int m0 = p.m_offsets[g], m1 = (p.mode == 0 && p.m_ends != nullptr) ? max(p.m_ends[g], m0) : p.m_offsets[g + 1];
+        const int m0 = p.m_offsets[g], m1 = p.mode == 0 ? m0 + group_rows(p, g, m0) : p.m_offsets[g + 1];
         ti.group = g;
         if (p.mode == 0) {
             const int tiles_m = (m1 - m0 + C::kTileRows - 1) / C::kTileRows;
@@ -1229,18 +1245,19 @@ cudaError_t launch_impl(const GroupedGemmArgs& a, cudaStream_t stream) {
         cfg.blockDim = dim3(C::kThreads, 1, 1);
         cfg.dynamicSmemBytes = C::kSmemBytes;
         cfg.stream = stream;
-        cudaLaunchAttribute attr[1];
+        cudaLaunchAttribute attr[2];
         attr[0].id = cudaLaunchAttributeClusterDimension;
         attr[0].val.clusterDim.x = 2;
         attr[0].val.clusterDim.y = 1;
         attr[0].val.clusterDim.z = 1;
+        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[1].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = attr;
-        cfg.numAttrs = 1;
+        cfg.numAttrs = 2;
         if (cfg.gridDim.x < 2) return cudaErrorInvalidValue;
         return cudaLaunchKernelEx(&cfg, kernel, map_a, map_b, map_sfa, map_sfb, a);
     } else {
-        kernel<<<a.num_sms, C::kThreads, C::kSmemBytes, stream>>>(map_a, map_b, map_sfa, map_sfb, a);
-        return cudaGetLastError();
+        return launch_dependent(kernel, dim3(a.num_sms), C::kThreads, C::kSmemBytes, stream, map_a, map_b, map_sfa, map_sfb, a);
     }
 }
 

@@ -12,7 +12,8 @@
 namespace dx {
 
 // Ordinary kernel whose launch work overlaps the tail of its predecessor in the stream (programmatic dependent launch). The
-// kernel must execute griddepcontrol.wait (pdl_wait_predecessor) before it touches memory that the predecessor may touch.
+// kernel must execute griddepcontrol.wait (pdl_wait_predecessor) before it touches memory that the predecessor may touch, and
+// before it releases its own successor: a kernel that starts early can then count on every kernel before its predecessor.
 template <typename... P, typename... A>
 cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t stream, const A&... args) {
     cudaLaunchConfig_t cfg = {};
@@ -25,7 +26,7 @@ cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, int threads, size_
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
 template <typename Args, int V>

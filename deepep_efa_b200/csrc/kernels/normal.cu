@@ -571,6 +571,8 @@ cudaError_t launch_combine(const CombineArgs* a, int nv, cudaStream_t stream) {
 // =============================================================================================
 template <int V>
 __global__ void __launch_bounds__(32, 1) barrier_kernel(const __grid_constant__ ArgPack<BarrierArgs, V> pack) {
+    pdl_wait_predecessor();
+    pdl_release_successor();
     const BarrierArgs& a = pack.a[blockIdx.y];
     const uint64_t seq = next_seq(a.ctx, kFamBarrier);
     cta_rank_barrier(a.ctx, seq);
@@ -578,7 +580,7 @@ __global__ void __launch_bounds__(32, 1) barrier_kernel(const __grid_constant__ 
 }
 
 cudaError_t launch_barrier(const BarrierArgs* a, int nv, cudaStream_t stream) {
-    return DX_LAUNCH_RANKED(barrier_kernel, BarrierArgs, a, nv, 1, 32, 0, stream);
+    return DX_LAUNCH_RANKED_PDL(barrier_kernel, BarrierArgs, a, nv, 1, 32, 0, stream);
 }
 
 __global__ void timeout_probe_kernel(const RankCtx c, uint64_t* flag) {

@@ -54,6 +54,9 @@ __device__ __forceinline__ int ld_relaxed_sys(const int* p) {
 __device__ __forceinline__ void red_add_release_sys(uint64_t* p, uint64_t v) {
     asm volatile("red.release.sys.global.add.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
+__device__ __forceinline__ void red_add_release_gpu(uint64_t* p, uint64_t v) {
+    asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
 __device__ __forceinline__ uint64_t ld_acquire_gpu(const uint64_t* p) {
     uint64_t v;
     asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");

@@ -13,6 +13,7 @@
 //                                    SwiGLU, 128-column tiles: [G][N/128][K/128][512], 64 gate + 64 up rows share one atom
 // The reference has no counterpart (no GEMM).
 #include "gemm_api.h"
+#include "launch.cuh"
 
 namespace dx {
 
@@ -24,6 +25,8 @@ __device__ __forceinline__ uint32_t ue8m0_word(float scale) {
 }
 
 __global__ void sfa_atoms_kernel(const float* __restrict__ scales, uint8_t* __restrict__ atoms, int rows, int num_kb, long long total) {
+    pdl_wait_predecessor();
+    pdl_release_successor();
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
         const int m0 = (int)(i & 31);
         const long long tk = i >> 5;           // tile * num_kb + kb
@@ -41,6 +44,8 @@ __global__ void sfa_atoms_kernel(const float* __restrict__ scales, uint8_t* __re
 
 __global__ void sfb_atoms_kernel(const float* __restrict__ scales, uint8_t* __restrict__ atoms, int n, int num_kb, int tiles, int swiglu,
                                  int wide, long long total) {
+    pdl_wait_predecessor();
+    pdl_release_successor();
     const int nb = n / 128;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
         const int m0 = (int)(i & 31);
@@ -80,8 +85,7 @@ cudaError_t launch_build_sfa_atoms(const float* scales, uint8_t* atoms, int rows
     const long long total = tiles * num_kb * 32;
     if (total <= 0) return cudaSuccess;
     const int blocks = (int)((total + 255) / 256 < 4096 ? (total + 255) / 256 : 4096);
-    sfa_atoms_kernel<<<blocks, 256, 0, stream>>>(scales, atoms, rows, num_kb, total);
-    return cudaGetLastError();
+    return launch_dependent(sfa_atoms_kernel, dim3(blocks), 256, 0, stream, scales, atoms, rows, num_kb, total);
 }
 
 cudaError_t launch_build_sfb_atoms(const float* scales, uint8_t* atoms, int groups, int n, int num_kb, int swiglu, int wide,
@@ -91,8 +95,7 @@ cudaError_t launch_build_sfb_atoms(const float* scales, uint8_t* atoms, int grou
     const long long total = (long long)groups * tiles * num_kb * 32;
     if (total <= 0) return cudaSuccess;
     const int blocks = (int)((total + 255) / 256 < 4096 ? (total + 255) / 256 : 4096);
-    sfb_atoms_kernel<<<blocks, 256, 0, stream>>>(scales, atoms, n, num_kb, tiles, swiglu, wide, total);
-    return cudaGetLastError();
+    return launch_dependent(sfb_atoms_kernel, dim3(blocks), 256, 0, stream, scales, atoms, n, num_kb, tiles, swiglu, wide, total);
 }
 
 }  // namespace dx

@@ -9,6 +9,7 @@
 // The reference has no counterpart (it ships no model code); these replace chains of framework ops whose copies
 // dominated the training step.
 #include "gemm_api.h"
+#include "launch.cuh"
 
 #include <cuda_bf16.h>
 
@@ -50,50 +51,63 @@ __global__ void __launch_bounds__(256) transpose_bf16_kernel(const __nv_bfloat16
 
 __device__ __forceinline__ float silu_f(float x) { return x / (1.f + __expf(-x)); }
 
-__global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ h13, __nv_bfloat16* __restrict__ h, long long rows, int inter) {
-    const int chunks = inter / 8;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < rows * chunks; i += (long long)gridDim.x * blockDim.x) {
-        const long long r = i / chunks;
-        const int c = (int)(i % chunks) * 8;
-        const int4 g = *reinterpret_cast<const int4*>(h13 + r * 2 * inter + c);
-        const int4 u = *reinterpret_cast<const int4*>(h13 + r * 2 * inter + inter + c);
-        const __nv_bfloat16* gp = reinterpret_cast<const __nv_bfloat16*>(&g);
-        const __nv_bfloat16* up = reinterpret_cast<const __nv_bfloat16*>(&u);
-        __align__(16) __nv_bfloat16 o[8];
+// One thread per eight columns; `I` is a 32-bit index wherever the sizes allow (a 64-bit division per thread costs more than the
+// arithmetic of the eight elements).
+template <typename I>
+__global__ void __launch_bounds__(256) swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ h13, __nv_bfloat16* __restrict__ h, I work, int inter) {
+    pdl_wait_predecessor();
+    pdl_release_successor();
+    const I i = (I)blockIdx.x * 256 + threadIdx.x;
+    if (i >= work) return;
+    const I chunks = inter / 8;
+    const I r = i / chunks;
+    const int c = (int)(i - r * chunks) * 8;
+    const __nv_bfloat16* row = h13 + (size_t)r * 2 * inter + c;
+    const int4 g = *reinterpret_cast<const int4*>(row);
+    const int4 u = *reinterpret_cast<const int4*>(row + inter);
+    const __nv_bfloat16* gp = reinterpret_cast<const __nv_bfloat16*>(&g);
+    const __nv_bfloat16* up = reinterpret_cast<const __nv_bfloat16*>(&u);
+    __align__(16) __nv_bfloat16 o[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) o[j] = __float2bfloat16(silu_f(__bfloat162float(gp[j])) * __bfloat162float(up[j]));
-        *reinterpret_cast<int4*>(h + r * inter + c) = *reinterpret_cast<const int4*>(o);
-    }
+    for (int j = 0; j < 8; ++j) o[j] = __float2bfloat16(silu_f(__bfloat162float(gp[j])) * __bfloat162float(up[j]));
+    *reinterpret_cast<int4*>(h + (size_t)r * inter + c) = *reinterpret_cast<const int4*>(o);
 }
 
-__global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ h13, const __nv_bfloat16* __restrict__ dh, __nv_bfloat16* __restrict__ dh13,
-                                  long long rows, int inter) {
-    const int chunks = inter / 8;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < rows * chunks; i += (long long)gridDim.x * blockDim.x) {
-        const long long r = i / chunks;
-        const int c = (int)(i % chunks) * 8;
-        const int4 g = *reinterpret_cast<const int4*>(h13 + r * 2 * inter + c);
-        const int4 u = *reinterpret_cast<const int4*>(h13 + r * 2 * inter + inter + c);
-        const int4 d = *reinterpret_cast<const int4*>(dh + r * inter + c);
-        const __nv_bfloat16* gp = reinterpret_cast<const __nv_bfloat16*>(&g);
-        const __nv_bfloat16* up = reinterpret_cast<const __nv_bfloat16*>(&u);
-        const __nv_bfloat16* dp = reinterpret_cast<const __nv_bfloat16*>(&d);
-        __align__(16) __nv_bfloat16 og[8], ou[8];
+template <typename I>
+__global__ void __launch_bounds__(256) swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ h13, const __nv_bfloat16* __restrict__ dh,
+                                                         __nv_bfloat16* __restrict__ dh13, I work, int inter) {
+    pdl_wait_predecessor();
+    pdl_release_successor();
+    const I i = (I)blockIdx.x * 256 + threadIdx.x;
+    if (i >= work) return;
+    const I chunks = inter / 8;
+    const I r = i / chunks;
+    const int c = (int)(i - r * chunks) * 8;
+    const __nv_bfloat16* row = h13 + (size_t)r * 2 * inter + c;
+    const int4 g = *reinterpret_cast<const int4*>(row);
+    const int4 u = *reinterpret_cast<const int4*>(row + inter);
+    const int4 d = *reinterpret_cast<const int4*>(dh + (size_t)r * inter + c);
+    const __nv_bfloat16* gp = reinterpret_cast<const __nv_bfloat16*>(&g);
+    const __nv_bfloat16* up = reinterpret_cast<const __nv_bfloat16*>(&u);
+    const __nv_bfloat16* dp = reinterpret_cast<const __nv_bfloat16*>(&d);
+    __align__(16) __nv_bfloat16 og[8], ou[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const float x = __bfloat162float(gp[j]), uu = __bfloat162float(up[j]), dd = __bfloat162float(dp[j]);
-            const float sig = 1.f / (1.f + __expf(-x));
-            og[j] = __float2bfloat16(dd * uu * sig * (1.f + x * (1.f - sig)));  // d silu(x)/dx = sig * (1 + x * (1 - sig))
-            ou[j] = __float2bfloat16(dd * x * sig);
-        }
-        *reinterpret_cast<int4*>(dh13 + r * 2 * inter + c) = *reinterpret_cast<const int4*>(og);
-        *reinterpret_cast<int4*>(dh13 + r * 2 * inter + inter + c) = *reinterpret_cast<const int4*>(ou);
+    for (int j = 0; j < 8; ++j) {
+        const float x = __bfloat162float(gp[j]), uu = __bfloat162float(up[j]), dd = __bfloat162float(dp[j]);
+        const float sig = 1.f / (1.f + __expf(-x));
+        og[j] = __float2bfloat16(dd * uu * sig * (1.f + x * (1.f - sig)));  // d silu(x)/dx = sig * (1 + x * (1 - sig))
+        ou[j] = __float2bfloat16(dd * x * sig);
     }
+    __nv_bfloat16* orow = dh13 + (size_t)r * 2 * inter + c;
+    *reinterpret_cast<int4*>(orow) = *reinterpret_cast<const int4*>(og);
+    *reinterpret_cast<int4*>(orow + inter) = *reinterpret_cast<const int4*>(ou);
 }
 
 // one warp per (n, k)
 __global__ void __launch_bounds__(256) rowdot_kernel(const __nv_bfloat16* __restrict__ a, const __nv_bfloat16* __restrict__ b, const int* __restrict__ pos,
                                                      float* __restrict__ out, int n_rows, int num_k, int hidden) {
+    pdl_wait_predecessor();
+    pdl_release_successor();
     const int lane = threadIdx.x & 31;
     const long long total = (long long)n_rows * num_k;
     for (long long p = (long long)blockIdx.x * 8 + (threadIdx.x >> 5); p < total; p += (long long)gridDim.x * 8) {
@@ -103,7 +117,7 @@ __global__ void __launch_bounds__(256) rowdot_kernel(const __nv_bfloat16* __rest
             const int4* ar = reinterpret_cast<const int4*>(a + (size_t)src * hidden);
             const int4* br = reinterpret_cast<const int4*>(b + (size_t)(p / num_k) * hidden);
             const int n16 = hidden / 8;
-            constexpr int U = 4;  // four column chunks of both rows in flight per lane
+            constexpr int U = 8;  // eight column chunks of both rows in flight per lane
             for (int i0 = 0; i0 < n16; i0 += 32 * U) {
                 int4 x[U], y[U];
 #pragma unroll
@@ -145,28 +159,30 @@ cudaError_t launch_swiglu_fwd(const void* h13, void* h, long long rows, int inte
     if (rows <= 0) return cudaSuccess;
     if ((inter & 7) != 0) return cudaErrorInvalidValue;
     const long long work = rows * (inter / 8);
-    const int blocks = (int)((work + 255) / 256 < 148 * 16 ? (work + 255) / 256 : 148 * 16);
-    swiglu_fwd_kernel<<<blocks, 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(h13), static_cast<__nv_bfloat16*>(h), rows, inter);
-    return cudaGetLastError();
+    const dim3 grid((unsigned)((work + 255) / 256));
+    const auto* in = static_cast<const __nv_bfloat16*>(h13);
+    auto* out = static_cast<__nv_bfloat16*>(h);
+    if (work < (1ll << 31)) return launch_dependent(swiglu_fwd_kernel<unsigned>, grid, 256, 0, stream, in, out, (unsigned)work, inter);
+    return launch_dependent(swiglu_fwd_kernel<long long>, grid, 256, 0, stream, in, out, work, inter);
 }
 
 cudaError_t launch_swiglu_bwd(const void* h13, const void* dh, void* dh13, long long rows, int inter, cudaStream_t stream) {
     if (rows <= 0) return cudaSuccess;
     if ((inter & 7) != 0) return cudaErrorInvalidValue;
     const long long work = rows * (inter / 8);
-    const int blocks = (int)((work + 255) / 256 < 148 * 16 ? (work + 255) / 256 : 148 * 16);
-    swiglu_bwd_kernel<<<blocks, 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(h13), static_cast<const __nv_bfloat16*>(dh),
-                                                  static_cast<__nv_bfloat16*>(dh13), rows, inter);
-    return cudaGetLastError();
+    const dim3 grid((unsigned)((work + 255) / 256));
+    const auto *in = static_cast<const __nv_bfloat16*>(h13), *din = static_cast<const __nv_bfloat16*>(dh);
+    auto* out = static_cast<__nv_bfloat16*>(dh13);
+    if (work < (1ll << 31)) return launch_dependent(swiglu_bwd_kernel<unsigned>, grid, 256, 0, stream, in, din, out, (unsigned)work, inter);
+    return launch_dependent(swiglu_bwd_kernel<long long>, grid, 256, 0, stream, in, din, out, work, inter);
 }
 
 cudaError_t launch_rowdot(const void* a, const void* b, const int* pos, float* out, int n_rows, int num_k, int hidden, cudaStream_t stream) {
     const long long total = (long long)n_rows * num_k;
     if (total <= 0) return cudaSuccess;
     if ((hidden & 7) != 0) return cudaErrorInvalidValue;
-    const int blocks = (int)((total + 7) / 8 < 148 * 8 ? (total + 7) / 8 : 148 * 8);
-    rowdot_kernel<<<blocks, 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(a), static_cast<const __nv_bfloat16*>(b), pos, out, n_rows, num_k, hidden);
-    return cudaGetLastError();
+    return launch_dependent(rowdot_kernel, dim3((unsigned)((total + 7) / 8)), 256, 0, stream, static_cast<const __nv_bfloat16*>(a),
+                            static_cast<const __nv_bfloat16*>(b), pos, out, n_rows, num_k, hidden);
 }
 
 }  // namespace dx

@@ -216,7 +216,7 @@ class MoELayer(nn.Module):
             topk_weights=topk_weights, expert_alignment=EXPERT_ALIGNMENT, quantize_fp8=True, round_scale=mx is not None)
         plan = build_expert_plan(recv_idx, counts)
         a = gather_rows(rx, plan.src_row)
-        a_s = gather_rows(rs, plan.src_row) if rs.size(1) % 4 == 0 else rs.index_select(0, plan.src_row.clamp(min=0).long())
+        a_s = gather_rows(rs, plan.src_row)
         if mx is not None:
             # padding rows of the plan carry all-zero data; whatever exponent their zero scale maps to does not matter
             wide = plan.num_rows >= WIDE_TILE_MIN_ROWS_PER_EXPERT * self.num_local_experts
@@ -278,27 +278,31 @@ class MoELayer(nn.Module):
         mx = getattr(self, "_mx", None) if N % 128 == 0 else None  # scale atoms cover whole 128-row tiles
         (px, ps), cnt, handle, _, _ = buf.low_latency_dispatch(x, topk_idx, M, cfg.num_experts, use_fp8=True, round_scale=mx is not None)
         ws = self.__dict__.setdefault("_ll_ws", {})
-        key = (M, x.device)
+        key = (M, x.device, mx is not None)
         if key not in ws:
             dev = x.device
-            ws[key] = dict(starts=(torch.arange(L + 1, device=dev, dtype=torch.int32) * N).contiguous(),
-                           h=torch.empty(L * N, I, dtype=torch.bfloat16, device=dev),
-                           hq=torch.empty(L * N, I, dtype=torch.float8_e4m3fn, device=dev),
-                           hs=torch.empty(L * N, I // 128, dtype=torch.float32, device=dev))
+            w_ = dict(starts=(torch.arange(L + 1, device=dev, dtype=torch.int32) * N).contiguous(),
+                      hq=torch.empty(L * N, I, dtype=torch.float8_e4m3fn, device=dev))
+            if mx is not None:
+                w_["ha"] = torch.empty(L * N // 128, I // 128, 512, dtype=torch.uint8, device=dev)
+            else:
+                w_["h"] = torch.empty(L * N, I, dtype=torch.bfloat16, device=dev)
+                w_["hs"] = torch.empty(L * N, I // 128, dtype=torch.float32, device=dev)
+            ws[key] = w_
         w_ = ws[key]
-        ends = w_["starts"][:L] + cnt
         a, a_s = px.view(L * N, H), ps.view(L * N, H // 128)
         y = buf.get_next_low_latency_combine_buffer(handle)
+        # rows per expert come as counts; both GEMMs read them where the dispatch left them
         if mx is not None:
-            wd = DECODE_WIDE_TILES
-            gg.grouped_gemm(a, w13, w_["starts"], swiglu=True, out=w_["h"], m_ends=ends, sfa_atoms=gg.build_sf_atoms_a(a_s), sfb_atoms=mx[0 if wd else 2])
-            C.per_token_cast_to_fp8(w_["h"], True, False, cnt, N, w_["hq"], w_["hs"])
-            gg.grouped_gemm(w_["hq"], w2, w_["starts"], out=y.view(L * N, H), m_ends=ends, sfa_atoms=gg.build_sf_atoms_a(w_["hs"]),
-                            sfb_atoms=mx[3 if wd else 1])
+            # GEMM1's epilogue quantises its own output (a wide tile holds one whole scale block of a row): e4m3 + scale atoms
+            C.grouped_gemm(a, w13, w_["starts"], 0, True, None, None, None, 0, GEMM_TIMEOUT_MS, cnt, gg.build_sf_atoms_a(a_s), mx[0],
+                           out_fp8=w_["hq"], out_atoms=w_["ha"], m_ends_are_counts=True)
+            C.grouped_gemm(w_["hq"], w2, w_["starts"], 0, False, None, None, y.view(L * N, H), 0, GEMM_TIMEOUT_MS, cnt, w_["ha"], mx[3],
+                           m_ends_are_counts=True)
         else:
-            gg.grouped_gemm(a, w13, w_["starts"], swiglu=True, a_scales=a_s, b_scales=s13, out=w_["h"], m_ends=ends)
+            C.grouped_gemm(a, w13, w_["starts"], 0, True, a_s, s13, w_["h"], 0, GEMM_TIMEOUT_MS, cnt, m_ends_are_counts=True)
             C.per_token_cast_to_fp8(w_["h"], False, False, cnt, N, w_["hq"], w_["hs"])
-            gg.grouped_gemm(w_["hq"], w2, w_["starts"], a_scales=w_["hs"], b_scales=s2, out=y.view(L * N, H), m_ends=ends)
+            C.grouped_gemm(w_["hq"], w2, w_["starts"], 0, False, w_["hs"], s2, y.view(L * N, H), 0, GEMM_TIMEOUT_MS, cnt, m_ends_are_counts=True)
         out, _, _ = buf.low_latency_combine(y, topk_idx, topk_weights, handle, zero_copy=True)
         return out
 
@@ -306,7 +310,6 @@ class MoELayer(nn.Module):
 # ---------------------------------------------------------------------------------------------------------
 # fused forward: expert-major dispatch -> arrival-gated GEMM1 -> cast -> GEMM2 with scatter epilogue -> local reduce
 # ---------------------------------------------------------------------------------------------------------
-DECODE_WIDE_TILES = True  # masked low-latency layout (a handful of valid rows per expert): 128x256 tiles stream the weights faster (1 rank, 256 experts: 1.96 vs 2.25 ms per step)
 UNIT_ROWS = 8  # rows of one expert a dispatch warp sends between two arrival-counter updates
 # SMs the arrival-gated GEMM leaves to the dispatch kernel while the two overlap. Sharing SMs cannot be relied on: a CTA of
 # the promotion kernel (10 warps of 160 registers) leaves no room for a dispatch warp in a scheduler partition's quarter of
@@ -321,6 +324,9 @@ RESERVED_SMS = 16
 # The gated GEMM runs as two launches when it overlaps the dispatch: the first part of the experts (arrival order = expert
 # order) on the SMs the dispatch does not use, the rest on all SMs once the dispatch is about done.
 SPLIT_FRACTION = 0.5
+# CTAs of the expert-major dispatch per SM when nothing runs beside it (four warps each; six fit an SM): with one the copy of 32768
+# rows of 7 KB took 162 us, bound by the loads four warps keep in flight.
+DISPATCH_CTAS_PER_SM = 6
 PREQUANTIZE = True  # cast every token to e4m3 once before the dispatch, which then only copies rows (8 selections share a cast)
 GEMM_TIMEOUT_MS = 2000.0  # bound of every wait inside the gated GEMMs (pipeline barriers and arrival counters)
 
@@ -400,7 +406,10 @@ def fused_forward_many(layers, xs, idxs, ws, overlap: bool = True, num_dispatch_
         wss.append(l.fused_workspace(x.size(0)))
     native = wss[0].native
     cur = torch.cuda.current_stream()
-    comm = bufs[0].comm_stream if (V == 1 and overlap) else cur
+    # a lone rank's rows never leave its memory: the dispatch is a copy at HBM speed, short when it has the GPU to itself, and a GEMM
+    # beside it would only give up SMs for it
+    lone = bufs[0].group_size == 1
+    comm = bufs[0].comm_stream if (V == 1 and overlap and not lone) else cur
     if comm is not cur:
         comm.wait_stream(cur)
     # the quantisation of x (caller's stream) and the count exchange (communication stream) do not depend on each other: side by side
@@ -418,7 +427,7 @@ def fused_forward_many(layers, xs, idxs, ws, overlap: bool = True, num_dispatch_
         planned.record(comm)
         if quantised is not None:
             comm.wait_event(quantised)
-        sms = num_dispatch_sms or (148 if V == 1 else max(1, 148 // V - 1))
+        sms = num_dispatch_sms or (148 * DISPATCH_CTAS_PER_SM if lone else 148 if V == 1 else max(1, 148 // V - 1))
         C.em_dispatch(rts, [(w.xq if PREQUANTIZE else x, w.my_counts, w.sel_list, w.send_base, w.unit_start, w.peer_bases, None,
                              None if w.trace is None else w.trace[0:2], w.xs if PREQUANTIZE else None) for x, w in zip(xs, wss)],
                       E, K, UNIT_ROWS, native, native, sms)
@@ -459,7 +468,8 @@ def fused_forward_many(layers, xs, idxs, ws, overlap: bool = True, num_dispatch_
             C.grouped_gemm(w.hq, w2, w.m_offsets, 0, False, w.hs, s2, None, 0, GEMM_TIMEOUT_MS, w.m_ends, None, None,
                            row_info=w.recv_info, scatter_bases=w.peer_bases[3 * R_:])
     # every rank's second GEMM has finished scattering before anybody sums its stage
-    C.barrier(rts)
+    if not lone:
+        C.barrier(rts)
     for l, x, i, wt, w in zip(layers, xs, idxs, ws, wss):
         out = torch.empty(x.size(0), cfg.hidden, dtype=torch.bfloat16, device=x.device)
         C.stage_reduce(w.stage, out, i, wt, E)

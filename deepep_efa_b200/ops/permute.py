@@ -35,6 +35,8 @@ class ExpertPlan:
 
 def build_expert_plan(recv_topk_idx: torch.Tensor, aligned_counts: List[int]) -> ExpertPlan:
     """``recv_topk_idx`` [N, K] holds local expert ids or -1; ``aligned_counts[e]`` >= rows of expert e."""
+    if recv_topk_idx.is_cuda:
+        return ExpertPlan(*_ext.load().build_plan(recv_topk_idx.contiguous(), aligned_counts))
     dev = recv_topk_idx.device
     N, K = recv_topk_idx.shape
     L = len(aligned_counts)
@@ -42,10 +44,7 @@ def build_expert_plan(recv_topk_idx: torch.Tensor, aligned_counts: List[int]) ->
     for c in aligned_counts:
         offs_host.append(offs_host[-1] + int(c))
     m_pad = offs_host[-1]
-    m_offsets = torch.tensor(offs_host, dtype=torch.int32).to(dev, non_blocking=True)
-    if recv_topk_idx.is_cuda:
-        pos, src_row, src_k = _ext.load().build_plan(recv_topk_idx.contiguous(), m_offsets, m_pad)
-        return ExpertPlan(pos, src_row, src_k, m_offsets, m_pad)
+    m_offsets = torch.tensor(offs_host, dtype=torch.int32)
     flat = recv_topk_idx.reshape(-1)
     valid = flat >= 0
     safe = flat.clamp(min=0)
@@ -117,15 +116,15 @@ class _UnpermuteWeighted(torch.autograd.Function):
         y_perm, weights = ctx.saved_tensors
         plan = ctx.plan
         grad = grad.contiguous()
-        # d y_perm[m] = w[src_row[m], src_k[m]] * grad[src_row[m]]
+        # d y_perm[m] = w[src_row[m], src_k[m]] * grad[src_row[m]];  d w[n, k] = <y_perm[pos[n, k]], grad[n]>
+        if grad.is_cuda and grad.dtype == torch.bfloat16 and y_perm.dtype == torch.bfloat16:
+            d_y_perm = _ext.load().gather_rows(grad, plan.src_row, weights.float().contiguous(), None, plan.src_k)
+            return d_y_perm, _ext.load().rowdot(y_perm, grad, plan.pos).to(weights.dtype), None, None
         w_flat = weights.reshape(-1)
         K = weights.size(1)
         idx = (plan.src_row.clamp(min=0).long() * K + plan.src_k.long())
         row_scale = torch.where(plan.src_row >= 0, w_flat[idx], torch.zeros_like(w_flat[idx])).float().contiguous()
         d_y_perm = gather_rows(grad, plan.src_row, row_scale)
-        # d w[n, k] = <y_perm[pos[n, k]], grad[n]>
-        if grad.is_cuda and grad.dtype == torch.bfloat16 and y_perm.dtype == torch.bfloat16:
-            return d_y_perm, _ext.load().rowdot(y_perm, grad, plan.pos).to(weights.dtype), None, None
         d_w = torch.zeros_like(weights)
         for k in range(K):
             p = plan.pos[:, k]
