@@ -159,8 +159,10 @@ torch::Tensor grouped_gemm(const torch::Tensor& a, const torch::Tensor& b, const
         // window to the epilogue every K block, and the cross-CTA handshake per block costs more than the halved B traffic saves
         const char* pr = std::getenv("DEEPEP_GEMM_PAIR");
         if (pr != nullptr && (pr[0] == '0' || pr[0] == '1')) p.cta_pairs = pr[0] == '1';
-        else p.cta_pairs = (!fp8 && p.m_ends == nullptr && (mode == 1 || (int64_t)p.m_total >= 1024 * (int64_t)G)) ? 1 : 0;
-        if (p.num_sms < 2 || mn_major) p.cta_pairs = 0;
+        // MN-major weight gradients of 64 experts, 4096 x 2816 each, single CTA / pair: 392 / 449 us at 128 rows per expert (a pair's
+        // tile is two row tiles high and the output, not the product, is the work), 1283 / 1263 us at 832, 4192 / 4009 us at 3136
+        else p.cta_pairs = (!fp8 && p.m_ends == nullptr && ((mode == 1 && !mn_major) || (int64_t)p.m_total >= 1024 * (int64_t)G)) ? 1 : 0;
+        if (p.num_sms < 2) p.cta_pairs = 0;
         // natively block-scaled e4m3: a pair instantiation exists for the wide SwiGLU tile only
         if (fp8 && !(p.sfa_atoms != nullptr && p.mx_wide == 1)) p.cta_pairs = (pr != nullptr && pr[0] == '1' && p.sfa_atoms == nullptr) ? 1 : 0;
     }

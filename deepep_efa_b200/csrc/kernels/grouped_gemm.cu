@@ -88,6 +88,13 @@ __device__ __forceinline__ void tma_load_2d(const CUtensorMap* map, uint64_t* ba
         "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(c0), "r"(c1)
         : "memory");
 }
+// An MN-major operand tile in one copy: its chunks of 64 rows are the third dimension of the map (see make_map_mn).
+__device__ __forceinline__ void tma_load_3d(const CUtensorMap* map, uint64_t* bar, void* dst, int c1, int c2) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(smem_u32(dst)),
+        "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(0), "r"(c1), "r"(c2)
+        : "memory");
+}
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* map) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
 }
@@ -196,6 +203,13 @@ __device__ __forceinline__ void tma_load_2d_pair(const CUtensorMap* map, uint32_
         "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(
             smem_u32(dst)),
         "l"(reinterpret_cast<uint64_t>(map)), "r"(bar_cluster_addr), "r"(c0), "r"(c1)
+        : "memory");
+}
+__device__ __forceinline__ void tma_load_3d_pair(const CUtensorMap* map, uint32_t bar_cluster_addr, void* dst, int c1, int c2) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(
+            smem_u32(dst)),
+        "l"(reinterpret_cast<uint64_t>(map)), "r"(bar_cluster_addr), "r"(0), "r"(c1), "r"(c2)
         : "memory");
 }
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t* dst_smem, uint32_t ncols) {
@@ -375,6 +389,7 @@ struct TileInfo {
     int a_row, a_k0, b_row, b_row2, b_k0, num_kb, c_row, c_col, group, nblock, nblock2;
     int c_row_end;  // first output row this tile must not write (end of its group; groups need no 128-row alignment)
     int nt;         // n-tile index inside the group (kMx: selects the B scale atoms)
+    int n_cols;     // columns of this tile: kBlockN, or half of it for the last column tile of an MN-major operand (kRagged)
     // MN-major operands: first tile row inside the tensor's contiguous dimension, and the tensor row of K index 0
     int a_mn0, a_kbase, b_mn0, b_kbase;
 };
@@ -408,11 +423,13 @@ struct Cfg {
     // The single-window wide tile also gets two warps per quarter: each drains half of the columns RAW (128 fp32 registers per
     // thread) and hands the window back at once, so the MMA issuer idles for the TMEM reads only, not for the SwiGLU arithmetic.
     static constexpr bool kSplitDrain = kMx && kBlockN == 256;
+    // plain BF16 with MN-major B: a column count that is an odd multiple of 128 ends in one tile of half the width
+    static constexpr bool kRagged = !kFp8 && !kSwiGLU && kBlockN == 256;
     static constexpr int kEpiWarps = (kPromote || kSplitDrain) ? 8 : 4;
     static constexpr int kThreads = 64 + 32 * kEpiWarps;
     static constexpr int kOutStageBytes = kRowScatter ? 8192 : (kSplitDrain ? 2048 : 4096);    // per epilogue warp: 32 rows x 32 / 64 (128) BF16
     // kSplitDrain with quantised output: the two warps of a quarter exchange their half-row maxima here (two tile parities)
-    static constexpr int kXchBytes = kSplitDrain ? 2 * 2 * kBlockM * 8 : 0;
+    static constexpr int kXchBytes = (kMx && kSwiGLU && kBlockN == 256) ? 2 * 2 * kBlockM * 8 : 0;
     static constexpr size_t kSmemBytes =
         (size_t)kStages * kStageBytes + (size_t)kEpiWarps * kOutStageBytes + 1024 /*align*/ + 256 /*barriers*/ + (kMaxGroups + 1) * 4 + kXchBytes;
 };
@@ -446,6 +463,9 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int G = p.num_groups;
     const int elem_per_kb = kFp8 ? 128 : 64;
+    constexpr bool kMnMajor = !kFp8 && !kSwiGLU;    // instantiations that take MN-major operands
+    const int out_width = p.mode == 0 ? p.n : p.k;  // columns that the column tiles cover
+    const int col_tiles = C::kRagged ? (out_width + kBlockN - 1) / kBlockN : out_width / kBlockN;
 
     if (threadIdx.x == 0) {
         s_abort = 0;
@@ -467,8 +487,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     pdl_release_successor();
     if (warp == 2) {
         // tile table: one warp scans the groups (one thread walking 256 groups through dependent loads took about 10 us)
-        const int tiles_n = p.mode == 0 ? p.n / kBlockN : 0;
-        const int tiles_fixed = p.mode == 1 ? ((p.n + C::kTileRows - 1) / C::kTileRows) * (p.k / kBlockN) : 0;
+        const int tiles_n = p.mode == 0 ? col_tiles : 0;
+        const int tiles_fixed = p.mode == 1 ? ((p.n + C::kTileRows - 1) / C::kTileRows) * col_tiles : 0;
         int run = 0;
         for (int g0 = 0; g0 < G; g0 += 32) {
             const int g = g0 + lane;
@@ -487,7 +507,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         }
         if (lane == 0) tile_start[G] = run;
     }
-    if constexpr (C::kSplitDrain) {
+    if constexpr (C::kXchBytes > 0) {
         for (int i = threadIdx.x; i < C::kXchBytes / 8; i += C::kThreads) xch[i] = 0ull;
     }
     if (warp == 1) {
@@ -512,14 +532,15 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         ti.group = g;
         if (p.mode == 0) {
             const int tiles_m = (m1 - m0 + C::kTileRows - 1) / C::kTileRows;
-            const int tiles_n_ = p.n / kBlockN;
+            const int tiles_n_ = col_tiles;
             // order 0: consecutive tiles share the weight tile (n outer); order 1: they share the activation tile (m outer)
             const int nt = p.tile_order == 0 ? local / tiles_m : local % tiles_n_;
             const int mt = p.tile_order == 0 ? local % tiles_m : local / tiles_n_;
             ti.a_row = m0 + mt * C::kTileRows + (int)cta_rank * kBlockM;
             ti.nt = nt;
+            ti.n_cols = C::kRagged ? min(kBlockN, out_width - nt * kBlockN) : kBlockN;
             ti.a_mn0 = ti.a_kbase = 0;                                          // mode 0: A is always K-major
-            ti.b_mn0 = nt * kBlockN + (int)cta_rank * (kBlockN / 2);            // MN-major B: [G * K, N], N contiguous
+            ti.b_mn0 = nt * kBlockN + (int)cta_rank * (ti.n_cols / 2);          // MN-major B: [G * K, N], N contiguous
             ti.b_kbase = g * p.k;
             ti.a_k0 = 0;
             ti.b_k0 = 0;
@@ -541,10 +562,11 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 ti.nblock2 = ti.nblock;
             }
         } else {
-            const int tiles_j = p.k / kBlockN;
+            const int tiles_j = col_tiles;
             const int it = local / tiles_j, jt = local % tiles_j;
+            ti.n_cols = C::kRagged ? min(kBlockN, out_width - jt * kBlockN) : kBlockN;
             ti.a_row = it * C::kTileRows + (int)cta_rank * kBlockM;
-            ti.b_row = jt * kBlockN + (int)cta_rank * (kBlockN / 2);
+            ti.b_row = jt * kBlockN + (int)cta_rank * (ti.n_cols / 2);
             ti.b_row2 = 0;
             ti.a_mn0 = ti.a_row;                                                // MN-major: A is [M, N_out], B is [M, K_out]
             ti.b_mn0 = ti.b_row;
@@ -616,9 +638,12 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                         // both CTAs fill their own stage and signal the LEADER's barrier, which expects the bytes of both
                         const uint32_t leader_full = mapa_shared(smem_u32(&full[stage]), 0);
                         if (cta_rank == 0) mbar_expect_tx(&full[stage], 2 * C::kStageTxBytes);
-                        tma_load_2d_pair(&map_a, leader_full, sa, ti.a_k0 + kb * elem_per_kb, ti.a_row);
-                        tma_load_2d_pair(&map_b, leader_full, sb, ti.b_k0 + kb * elem_per_kb,
-                                         (kSwiGLU && cta_rank == 1) ? ti.b_row2 : ti.b_row);  // SwiGLU: gate half / up half
+                        if (kMnMajor && p.a_mn) tma_load_3d_pair(&map_a, leader_full, sa, ti.a_kbase + kb * 64, ti.a_mn0 / 64);
+                        else tma_load_2d_pair(&map_a, leader_full, sa, ti.a_k0 + kb * elem_per_kb, ti.a_row);
+                        if (kMnMajor && p.b_mn) tma_load_3d_pair(&map_b, leader_full, sb, ti.b_kbase + kb * 64, ti.b_mn0 / 64);
+                        else
+                            tma_load_2d_pair(&map_b, leader_full, sb, ti.b_k0 + kb * elem_per_kb,
+                                             (kSwiGLU && cta_rank == 1) ? ti.b_row2 : ti.b_row);  // SwiGLU: gate half / up half
                         if constexpr (kMx) {
                             // scale atoms as rows of 32-bit words: this CTA's own 128 rows of A, and the whole tile's B columns
                             uint8_t* ssf = sb + C::kBTileBytes;
@@ -643,33 +668,11 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                         bulk_load_1d(ssf + 512, p.sfb_atoms + (((size_t)ti.group * (p.n / kBlockN) + ti.nt) * nkb + kb) * (512 * C::kSfBAtoms),
                                      512 * C::kSfBAtoms, &full[stage]);
                     }
-                    if constexpr (!kFp8 && !kSwiGLU && !kMx) {
-                        if (p.a_mn | p.b_mn) {
-                            // an MN-major tile arrives as chunks of 64 rows x 64 K-steps (8 KiB each)
-                            if (p.a_mn) {
-#pragma unroll
-                                for (int j = 0; j < kBlockM / 64; ++j)
-                                    tma_load_2d(&map_a, &full[stage], sa + j * 8192, ti.a_mn0 + j * 64, ti.a_kbase + kb * 64);
-                            } else {
-                                tma_load_2d(&map_a, &full[stage], sa, ti.a_k0 + kb * elem_per_kb, ti.a_row);
-                            }
-                            if (p.b_mn) {
-#pragma unroll
-                                for (int j = 0; j < kBlockN / 64; ++j)
-                                    tma_load_2d(&map_b, &full[stage], sb + j * 8192, ti.b_mn0 + j * 64, ti.b_kbase + kb * 64);
-                            } else {
-                                tma_load_2d(&map_b, &full[stage], sb, ti.b_k0 + kb * elem_per_kb, ti.b_row);
-                            }
-                            if (issued < C::kStages) ++issued;
-                            if (++stage == C::kStages) {
-                                stage = 0;
-                                phase ^= 1;
-                            }
-                            continue;
-                        }
-                    }
-                    tma_load_2d(&map_a, &full[stage], sa, ti.a_k0 + kb * elem_per_kb, ti.a_row);
-                    if (kSwiGLU) {
+                    if (kMnMajor && p.a_mn) tma_load_3d(&map_a, &full[stage], sa, ti.a_kbase + kb * 64, ti.a_mn0 / 64);
+                    else tma_load_2d(&map_a, &full[stage], sa, ti.a_k0 + kb * elem_per_kb, ti.a_row);
+                    if (kMnMajor && p.b_mn) {
+                        tma_load_3d(&map_b, &full[stage], sb, ti.b_kbase + kb * 64, ti.b_mn0 / 64);
+                    } else if (kSwiGLU) {
                         tma_load_2d(&map_b, &full[stage], sb, ti.b_k0 + kb * elem_per_kb, ti.b_row);
                         tma_load_2d(&map_b, &full[stage], sb + C::kBTileBytes / 2, ti.b_k0 + kb * elem_per_kb, ti.b_row2);
                     } else {
@@ -708,7 +711,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     } else if (warp == 1) {
         // ================= MMA issuer =================
         if (lane == 0 && cta_rank == 0) {
-            const uint32_t idesc = kMx ? make_idesc_mx(kBlockN, C::kTileRows) : make_idesc<kFp8>(kBlockN, C::kTileRows, p.a_mn, p.b_mn);
+            const uint32_t idesc_full = kMx ? make_idesc_mx(kBlockN, C::kTileRows) : make_idesc<kFp8>(kBlockN, C::kTileRows, p.a_mn, p.b_mn);
+            const uint32_t idesc_half = make_idesc<kFp8>(kBlockN / 2, C::kTileRows, p.a_mn, p.b_mn);
             // bytes (in 16-byte units) one K = 16 step moves the operand's start address: 32 B inside the swizzle atom when K
             // is contiguous, 16 K-steps of 128 B when the rows are
             const uint64_t a_kstep = p.a_mn ? 128 : 2, b_kstep = p.b_mn ? 128 : 2;
@@ -720,6 +724,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             for (int tile = sched_id; tile < total_tiles && ok; tile += sched_stride) {
                 decode(tile, g, ti);
                 if (ti.num_kb == 0) continue;  // epilogue writes zeros on its own
+                const uint32_t idesc = (C::kRagged && ti.n_cols != kBlockN) ? idesc_half : idesc_full;
                 for (int kb = 0; kb < ti.num_kb; ++kb) {
                     const bool new_window = C::kPromote ? true : (kb == 0);
                     if (new_window) {
@@ -829,7 +834,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             if (ti.num_kb == 0) {
                 __nv_bfloat16* zrow = scatter ? scat_ptr : crow;
                 if (row < ti.c_row_end && half == 0 && zrow != nullptr)
-                    for (int c = 0; c < C::kOutCols; c += 8) *reinterpret_cast<int4*>(zrow + c) = make_int4(0, 0, 0, 0);
+                    for (int c = 0; c < (C::kRagged ? ti.n_cols : C::kOutCols); c += 8) *reinterpret_cast<int4*>(zrow + c) = make_int4(0, 0, 0, 0);
                 continue;
             }
             if constexpr (C::kPromote) {
@@ -1098,7 +1103,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                     }
                 } else {
 #pragma unroll 1
-                    for (int c = 0; c < C::kOutCols; c += 64) {
+                    for (int c = 0; c < (C::kRagged ? ti.n_cols : C::kOutCols); c += 64) {
                         uint32_t v[32], u[32];
                         tmem_ld32(taddr + c, v);
                         tmem_ld32(taddr + c + 32, u);
@@ -1178,16 +1183,18 @@ bool make_map(CUtensorMap* map, const void* ptr, bool fp8, uint64_t rows, uint64
     return r == CUDA_SUCCESS;
 }
 
-// 2-D row-major [k_rows, mn_cols] bf16 tensor whose contiguous dimension is the operand's row index (MN-major operand):
-// box = 64 columns (128 bytes) x 64 rows, 128B swizzle.
-bool make_map_mn(CUtensorMap* map, const void* ptr, uint64_t k_rows, uint64_t mn_cols) {
+// Row-major [k_rows, mn_cols] bf16 tensor whose contiguous dimension is the operand's row index (MN-major operand), seen as
+// [mn_cols / 64, k_rows, 64]: a box of `box_rows` operand rows x 64 K-steps lands as chunks of 64 rows (8 KiB each, 128B swizzle),
+// the order the matrix descriptor expects, in one copy. One copy per 64-row chunk cost the loading lane up to six instructions per
+// stage. Chunks past the last column read as zeros and touch no memory.
+bool make_map_mn(CUtensorMap* map, const void* ptr, uint64_t k_rows, uint64_t mn_cols, uint32_t box_rows) {
     EncodeFn fn = get_encode_fn();
     if (fn == nullptr) return false;
-    cuuint64_t dims[2] = {mn_cols, k_rows};
-    cuuint64_t strides[1] = {mn_cols * 2};
-    cuuint32_t box[2] = {64, 64};
-    cuuint32_t estr[2] = {1, 1};
-    const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+    cuuint64_t dims[3] = {64, k_rows, mn_cols / 64};
+    cuuint64_t strides[2] = {mn_cols * 2, 128};
+    cuuint32_t box[3] = {64, 64, box_rows / 64};
+    cuuint32_t estr[3] = {1, 1, 1};
+    const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                           CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS;
 }
@@ -1221,12 +1228,12 @@ cudaError_t launch_impl(const GroupedGemmArgs& a, cudaStream_t stream) {
     bool ok;
     if (a.mode == 0) {
         ok = make_map(&map_a, a.a, kFp8, (uint64_t)a.m_total, (uint64_t)a.k, kBlockM) &&
-             (a.b_mn ? make_map_mn(&map_b, a.b, (uint64_t)a.num_groups * a.k, (uint64_t)a.n)  // B given as [G, K, N]
+             (a.b_mn ? make_map_mn(&map_b, a.b, (uint64_t)a.num_groups * a.k, (uint64_t)a.n, C::kBRows)  // B given as [G, K, N]
                      : make_map(&map_b, a.b, kFp8, (uint64_t)a.num_groups * a.n, (uint64_t)a.k, b_box_rows));
     } else {
-        ok = (a.a_mn ? make_map_mn(&map_a, a.a, (uint64_t)a.m_total, (uint64_t)a.n)   // A given as [M, N_out]
+        ok = (a.a_mn ? make_map_mn(&map_a, a.a, (uint64_t)a.m_total, (uint64_t)a.n, kBlockM)   // A given as [M, N_out]
                      : make_map(&map_a, a.a, kFp8, (uint64_t)a.n, (uint64_t)a.m_total, kBlockM)) &&
-             (a.b_mn ? make_map_mn(&map_b, a.b, (uint64_t)a.m_total, (uint64_t)a.k)   // B given as [M, K_out]
+             (a.b_mn ? make_map_mn(&map_b, a.b, (uint64_t)a.m_total, (uint64_t)a.k, C::kBRows)   // B given as [M, K_out]
                      : make_map(&map_b, a.b, kFp8, (uint64_t)a.k, (uint64_t)a.m_total, b_box_rows));
     }
     if (!ok) return cudaErrorInvalidValue;
@@ -1274,7 +1281,7 @@ cudaError_t launch_grouped_gemm(const GroupedGemmArgs& a, cudaStream_t stream) {
     if (a.num_groups < 1 || a.num_groups > kMaxGroups || a.num_sms < 1) return cudaErrorInvalidValue;
     // MN-major operands: bf16, no swiglu, single CTAs; mode 0 takes B that way (input gradients read the weight in place),
     // mode 1 takes both (weight gradients read the output gradient and the activation in place)
-    if ((a.a_mn || a.b_mn) && (a.fp8 || a.swiglu || a.cta_pairs || (a.mode == 0 && a.a_mn) || (a.mode == 1 && !(a.a_mn && a.b_mn)) || a.n % 64 != 0))
+    if ((a.a_mn || a.b_mn) && (a.fp8 || a.swiglu || (a.mode == 0 && a.a_mn) || (a.mode == 1 && !(a.a_mn && a.b_mn)) || a.n % 64 != 0))
         return cudaErrorInvalidValue;
     if (a.m_total <= 0) return cudaSuccess;
     const int kb = a.fp8 ? 128 : 64;
@@ -1307,13 +1314,16 @@ cudaError_t launch_grouped_gemm(const GroupedGemmArgs& a, cudaStream_t stream) {
             if ((a.n / 2) % 64 == 0) return launch_sel<128, false, true>(a, stream);
             return cudaErrorInvalidValue;
         }
-        if (a.n % 256 == 0) return launch_sel<256, false, false>(a, stream);
+        // MN-major B: 256-column tiles with one half-width tile at the end beat 128-column tiles (input gradient of 53248 rows with 64
+        // experts of 4096 x 1408: 815 -> 635 us); K-major boxes would reach into the next expert's rows, so those stay at 128
+        if (a.n % 256 == 0 || (a.b_mn && a.n > 256 && a.n % 128 == 0)) return launch_sel<256, false, false>(a, stream);
         if (a.n % 128 == 0) return launch_sel<128, false, false>(a, stream);
         return cudaErrorInvalidValue;
     }
     // K-grouped (weight gradients), bf16 only
     if (a.fp8 || a.swiglu || a.n % kBlockM != 0) return cudaErrorInvalidValue;
-    if (a.k % 256 == 0) return launch_sel<256, false, false>(a, stream);
+    // as above (weight gradient of the same layer: 880 -> 680 us; with 128 rows per expert 216 -> 201 us)
+    if (a.k % 256 == 0 || (a.b_mn && a.k > 256 && a.k % 128 == 0)) return launch_sel<256, false, false>(a, stream);
     if (a.k % 128 == 0) return launch_sel<128, false, false>(a, stream);
     return cudaErrorInvalidValue;
 }

@@ -241,6 +241,35 @@ def test_bf16_wgrad_reads_gradient_and_activation_in_place(rows, n_out, k_out):
             assert _rel_err(dw[g], ref) < 1e-2, (g, _rel_err(dw[g], ref))
 
 
+@pytest.mark.parametrize("pair", ["0", "1"])
+@pytest.mark.parametrize("n_out,k_out", [(128, 128), (128, 384), (384, 640), (256, 256)])
+def test_bf16_mn_major_half_width_tiles_and_pairs(monkeypatch, pair, n_out, k_out):
+    """Column counts that are odd multiples of 128 end in a half-width tile, alone or split over a CTA pair; empty and small groups."""
+    from deepep_efa_b200 import _ext
+    from deepep_efa_b200.ops.grouped_gemm import grouped_gemm_dgrad, grouped_gemm_wgrad_inplace
+    monkeypatch.setenv("DEEPEP_GEMM_PAIR", pair)
+    C = _ext.load()
+    C.gemm_clear_error(0)
+    torch.manual_seed(13)
+    rows = [128, 0, 384, 64, 640]
+    dy = torch.randn(sum(rows), n_out, device="cuda").to(torch.bfloat16)
+    x = torch.randn(sum(rows), k_out, device="cuda").to(torch.bfloat16)
+    w = (torch.randn(len(rows), n_out, k_out, device="cuda") * 0.1).to(torch.bfloat16)
+    offs = _offsets(rows)
+    dx, dw = grouped_gemm_dgrad(dy, w, offs), grouped_gemm_wgrad_inplace(dy, x, offs)
+    torch.cuda.synchronize()
+    assert C.gemm_error(0) == 0
+    o = offs.tolist()
+    for g, n in enumerate(rows):
+        d, xx = dy[o[g]:o[g + 1]].float(), x[o[g]:o[g + 1]].float()
+        if n == 0:
+            assert dw[g].float().abs().max().item() == 0
+            continue
+        # fp32 sums of bf16 products, rounded once to bf16 (2^-9 relative)
+        assert _rel_err(dx[o[g]:o[g + 1]], d @ w[g].float()) < 4e-3
+        assert _rel_err(dw[g], d.t() @ xx) < 4e-3
+
+
 def test_fp8_native_wide_swiglu_writes_quantised_output():
     """The wide natively block-scaled SwiGLU kernel can emit e4m3 rows plus UE8M0 scale atoms itself; both must equal what
     the standalone cast makes of the kernel's BF16 output, bit for bit (valid rows only; masked groups stay untouched)."""
