@@ -855,6 +855,22 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 // A warp whose 32 rows all lie past the end of the group (masked low-latency layout: a handful of valid rows
                 // per expert) only keeps the window ring moving; it promotes nothing.
                 const bool warp_has_rows = ti.c_row + q * 32 < ti.c_row_end;
+                // Scales are fetched two K blocks ahead: loaded right before their window's wait they put an L2 round trip into
+                // every K block as soon as the promotion, not the loads, is the slower side (64 experts of 4096 -> 1408, 128 rows each:
+                // first / second GEMM 194 / 103 -> 187 / 93 us; 768 rows each: 1066 / 550 -> 1008 / 523 us). With arrival gating the activation
+                // scales are written by other GPUs during this kernel, and only the accumulator hand-over orders this warp after
+                // the loader's acquire of the group's arrival counter: the first loads then come after the tile's first wait.
+                float s_cur[3] = {0.f, 0.f, 0.f}, s_next[3] = {0.f, 0.f, 0.f}, s_far[3] = {0.f, 0.f, 0.f};
+                auto fetch_scales = [&](int kb, float (&s)[3]) {
+                    if (kb >= ti.num_kb) return;
+                    s[0] = __ldcg(sa_row + kb);
+                    s[1] = __ldg(sb0 + kb);
+                    if (kSwiGLU) s[2] = __ldg(sb1 + kb);
+                };
+                if (warp_has_rows && p.ready == nullptr) {
+                    fetch_scales(0, s_next);
+                    fetch_scales(1, s_far);
+                }
                 for (int kb = 0; kb < ti.num_kb; ++kb) {
                     if (!warp_has_rows) {
                         if (!mbar_wait(&tmem_full[win], win_phase, abort_flag, limit, note, wait_id(7, tile, kb, warp))) {
@@ -869,18 +885,21 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                         }
                         continue;
                     }
-                    // Ungated: the activation scale is fetched ahead of the wait, to hide its latency. With arrival gating the
-                    // scales are written by other GPUs during this kernel, and only the accumulator hand-over orders this warp
-                    // after the loader's acquire of the group's arrival counter: the load has to come after the wait (L2 only).
-                    float sa = 0.f;
-                    if (p.ready == nullptr) sa = __ldcg(sa_row + kb);
-                    const float wb0 = __ldg(sb0 + kb), wb1 = kSwiGLU ? __ldg(sb1 + kb) : 0.f;
                     if (!mbar_wait(&tmem_full[win], win_phase, abort_flag, limit, note, wait_id(5, tile, kb, warp))) {
                         ok = false;
                         break;
                     }
-                    if (p.ready != nullptr) sa = __ldcg(sa_row + kb);
-                    const float s_lo = sa * wb0, s_hi = kSwiGLU ? sa * wb1 : s_lo;
+                    if (kb == 0 && p.ready != nullptr) {
+                        fetch_scales(0, s_next);
+                        fetch_scales(1, s_far);
+                    }
+#pragma unroll
+                    for (int i = 0; i < 3; ++i) {
+                        s_cur[i] = s_next[i];
+                        s_next[i] = s_far[i];
+                    }
+                    fetch_scales(kb + 2, s_far);
+                    const float s_lo = s_cur[0] * s_cur[1], s_hi = kSwiGLU ? s_cur[0] * s_cur[2] : s_lo;
                     tc_fence_after();
                     const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(win * kBlockN);
                     uint32_t v[32], u[32];
