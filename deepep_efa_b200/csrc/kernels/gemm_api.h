@@ -71,6 +71,9 @@ struct GroupedGemmArgs {
     // c_atoms: the activation operand of the next natively block-scaled GEMM, without a cast pass in between.
     uint8_t* c_fp8;
     uint8_t* c_atoms;
+    // Optional [2], zero: tiles are drawn from a counter instead of dealt out in strides (single CTAs only; pairs ignore it). The
+    // kernel leaves both words zero. Launches that may run at the same time need words of their own.
+    int* sched;
 };
 
 // Returns cudaErrorInvalidValue for unsupported shapes (divisibility rules are in grouped_gemm.cu).

@@ -35,6 +35,7 @@ namespace {
 constexpr int kBlockM = 128;
 constexpr int kKBlockBytes = 128;      // one 128B swizzle atom per row
 constexpr int kATileBytes = kBlockM * kKBlockBytes;  // 16 KiB
+constexpr int kTileSlots = 2;          // tiles the loader may hand to the other roles ahead of time
 constexpr int kMaxGroups = 1024;
 
 // ---- PTX wrappers ---------------------------------------------------------------------------
@@ -454,10 +455,14 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     uint64_t* empty = bars + C::kStages;         // [kStages]
     uint64_t* tmem_full = bars + 2 * C::kStages; // [kWindows]
     uint64_t* tmem_empty = tmem_full + C::kWindows;  // [kWindows]
+    uint64_t* tile_full = tmem_empty + C::kWindows;   // [kTileSlots] tiles handed out by the loader (p.sched)
+    uint64_t* tile_free = tile_full + kTileSlots;     // [kTileSlots]
+    static_assert(2 * C::kStages + 2 * C::kWindows + 2 * kTileSlots <= 32, "barrier block");
     int* tile_start = reinterpret_cast<int*>(bars + 32);  // [G+1] first tile index of every group
     volatile unsigned long long* xch = reinterpret_cast<volatile unsigned long long*>(bars + 32 + (kMaxGroups + 2) / 2);  // [2][2][kBlockM] (tile tag << 32 | amax bits)
     __shared__ uint32_t s_tmem_base;
     __shared__ int s_abort;
+    __shared__ volatile int s_tile[kTileSlots];
     __shared__ volatile int s_prod_state[2];  // what the loader is doing (1 = arrival gate, 2 = free stage, 3 = loads issued) and for which tile
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -476,6 +481,10 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         for (int a = 0; a < C::kWindows; ++a) {
             mbar_init(&tmem_full[a], 1);
             mbar_init(&tmem_empty[a], kPair ? 2 * C::kEpiWarps : C::kEpiWarps);  // the leader collects both CTAs' epilogue warps
+        }
+        for (int i = 0; i < kTileSlots; ++i) {
+            mbar_init(&tile_full[i], 1);
+            mbar_init(&tile_free[i], 1 + C::kEpiWarps);
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         tma_prefetch_desc(&map_a);
@@ -581,6 +590,26 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         }
     };
 
+    // Which tile comes next. Without p.sched every CTA walks its share in strides. With it the loader draws tiles from a counter and
+    // passes them on through a small ring: SMs see unequal shares of the L2-to-SM bandwidth, and with equal numbers of tiles the
+    // slowest of them finished tens of microseconds after the first in kernels that stream weights (one B200, decode of 128 tokens
+    // through 256 experts of 7168 -> 2048: first / second GEMM 1243 / 661 -> 1209 / 622 us; the fused layer of 4096 tokens 2700 -> 2600).
+    const bool drawn = !kPair && p.sched != nullptr;
+    int tslot = 0, tphase = 0;  // this role's position in the ring
+    auto next_tile = [&](int tile, bool whole_warp) {
+        if (!drawn) return tile + sched_stride;
+        const bool got = mbar_wait(&tile_full[tslot], tphase, abort_flag, limit, note, wait_id(8, tile, 0, tslot));
+        if (whole_warp ? !__all_sync(0xffffffffu, got) : !got) return total_tiles;
+        const int t = s_tile[tslot];
+        if (whole_warp) __syncwarp();
+        if (lane == 0) mbar_arrive(&tile_free[tslot]);
+        if (++tslot == kTileSlots) {
+            tslot = 0;
+            tphase ^= 1;
+        }
+        return t;
+    };
+
     // An epilogue warp hands an accumulator window back to the MMA issuer: in a pair that is the leader CTA's barrier.
     auto release_window = [&](uint64_t* bar) {
         if constexpr (kPair) {
@@ -600,7 +629,24 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             bool stamped = false;
             TileInfo ti;
             bool ok = true;
-            for (int tile = sched_id; tile < total_tiles && ok; tile += sched_stride) {
+            auto hand_out = [&](int tile, int draw) {
+                if (!drawn) return tile + sched_stride;
+                const int t = min(sched_stride + draw, total_tiles);
+                if (!mbar_wait(&tile_free[tslot], tphase ^ 1, abort_flag, limit, note, wait_id(9, tile, 0, tslot))) {
+                    ok = false;
+                    return total_tiles;
+                }
+                s_tile[tslot] = t;
+                mbar_arrive(&tile_full[tslot]);
+                if (++tslot == kTileSlots) {
+                    tslot = 0;
+                    tphase ^= 1;
+                }
+                return t;
+            };
+            int drawn_tile = 0;
+            for (int tile = sched_id; tile < total_tiles && ok; tile = hand_out(tile, drawn_tile)) {
+                if (drawn) drawn_tile = atomicAdd(p.sched, 1);  // used when this tile's loads have been issued
                 decode(tile, g, ti);
                 s_prod_state[1] = tile;
                 if (p.ready != nullptr && ti.group != gated_group) {
@@ -685,6 +731,13 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                     }
                 }
             }
+            if (drawn) {  // the last CTA to stop drawing leaves the counter as it was found
+                __threadfence();
+                if (atomicAdd(p.sched + 1, 1) == (int)gridDim.x - 1) {
+                    p.sched[1] = 0;
+                    atomicExch(p.sched, 0);
+                }
+            }
             // Own copies in flight land in this CTA's shared memory: before the CTA may exit, wait (bounded) for every stage
             // that was armed but whose completion this lane has not yet seen. `stage`/`phase` point at the next stage to
             // fill, so the kStages stages before it are the candidates, each with the phase it was armed in.
@@ -721,7 +774,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             int win = 0, win_phase = 0;  // accumulator window ring
             TileInfo ti;
             bool ok = true;
-            for (int tile = sched_id; tile < total_tiles && ok; tile += sched_stride) {
+            for (int tile = sched_id; tile < total_tiles && ok; tile = next_tile(tile, false)) {
                 decode(tile, g, ti);
                 if (ti.num_kb == 0) continue;  // epilogue writes zeros on its own
                 const uint32_t idesc = (C::kRagged && ti.n_cols != kBlockN) ? idesc_half : idesc_full;
@@ -820,7 +873,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         __nv_bfloat16* cbase = reinterpret_cast<__nv_bfloat16*>(p.c);
         const int ldc = p.mode == 0 ? (kSwiGLU ? p.n / 2 : p.n) : p.k;
         const bool scatter = !kSwiGLU && p.mode == 0 && p.row_info != nullptr;
-        for (int tile = sched_id; tile < total_tiles && ok; tile += sched_stride) {
+        for (int tile = sched_id; tile < total_tiles && ok; tile = next_tile(tile, true)) {
             decode(tile, g, ti);
             const int row = ti.c_row + row_in_tile;
             __nv_bfloat16* crow = cbase + (size_t)row * ldc + ti.c_col;

@@ -282,7 +282,7 @@ class MoELayer(nn.Module):
         if key not in ws:
             dev = x.device
             w_ = dict(starts=(torch.arange(L + 1, device=dev, dtype=torch.int32) * N).contiguous(),
-                      hq=torch.empty(L * N, I, dtype=torch.float8_e4m3fn, device=dev))
+                      hq=torch.empty(L * N, I, dtype=torch.float8_e4m3fn, device=dev), sched=torch.zeros(2, dtype=torch.int32, device=dev))
             if mx is not None:
                 w_["ha"] = torch.empty(L * N // 128, I // 128, 512, dtype=torch.uint8, device=dev)
             else:
@@ -296,13 +296,13 @@ class MoELayer(nn.Module):
         if mx is not None:
             # GEMM1's epilogue quantises its own output (a wide tile holds one whole scale block of a row): e4m3 + scale atoms
             C.grouped_gemm(a, w13, w_["starts"], 0, True, None, None, None, 0, GEMM_TIMEOUT_MS, cnt, gg.build_sf_atoms_a(a_s), mx[0],
-                           out_fp8=w_["hq"], out_atoms=w_["ha"], m_ends_are_counts=True)
+                           out_fp8=w_["hq"], out_atoms=w_["ha"], m_ends_are_counts=True, sched=w_["sched"])
             C.grouped_gemm(w_["hq"], w2, w_["starts"], 0, False, None, None, y.view(L * N, H), 0, GEMM_TIMEOUT_MS, cnt, w_["ha"], mx[3],
-                           m_ends_are_counts=True)
+                           m_ends_are_counts=True, sched=w_["sched"])
         else:
-            C.grouped_gemm(a, w13, w_["starts"], 0, True, a_s, s13, w_["h"], 0, GEMM_TIMEOUT_MS, cnt, m_ends_are_counts=True)
+            C.grouped_gemm(a, w13, w_["starts"], 0, True, a_s, s13, w_["h"], 0, GEMM_TIMEOUT_MS, cnt, m_ends_are_counts=True, sched=w_["sched"])
             C.per_token_cast_to_fp8(w_["h"], False, False, cnt, N, w_["hq"], w_["hs"])
-            C.grouped_gemm(w_["hq"], w2, w_["starts"], 0, False, w_["hs"], s2, y.view(L * N, H), 0, GEMM_TIMEOUT_MS, cnt, m_ends_are_counts=True)
+            C.grouped_gemm(w_["hq"], w2, w_["starts"], 0, False, w_["hs"], s2, y.view(L * N, H), 0, GEMM_TIMEOUT_MS, cnt, m_ends_are_counts=True, sched=w_["sched"])
         out, _, _ = buf.low_latency_combine(y, topk_idx, topk_weights, handle, zero_copy=True)
         return out
 
@@ -359,6 +359,7 @@ class _FusedWorkspace:
         self.unit_start = torch.zeros(E + 2, **i32)  # prefix of work units [E + 1] and the hand-out counter
         self.m_offsets = torch.zeros(L + 1, **i32)
         self.m_ends = torch.zeros(L, **i32)
+        self.sched = torch.zeros(2, **i32)  # tile counter of the expert GEMMs, which run one after the other
         self.peer_bases = torch.zeros(4 * R, dtype=torch.int64, device=dev)
         self.h = torch.empty(rows, I, dtype=torch.bfloat16, device=dev)
         self.hq = torch.empty(rows, I, dtype=torch.float8_e4m3fn, device=dev)
@@ -447,7 +448,7 @@ def fused_forward_many(layers, xs, idxs, ws, overlap: bool = True, num_dispatch_
         parts = [(0, ga, 148 - RESERVED_SMS), (ga, L - ga, 0)] if (overlapped and ga < L) else [(0, L, (148 - RESERVED_SMS) if overlapped else 0)]
         for pi, (g0, ng, sms1) in enumerate(parts):
             tr = None if (w.trace is None or pi > 0) else w.trace[2:6]
-            gate = dict(ready=w.arrived[g0:g0 + ng], expected=w.expected[g0:g0 + ng], trace=tr)
+            gate = dict(ready=w.arrived[g0:g0 + ng], expected=w.expected[g0:g0 + ng], trace=tr, sched=w.sched)
             mo, me_ = w.m_offsets[g0:g0 + ng + 1], w.m_ends[g0:g0 + ng]
             if native:
                 if fuse_cast:
@@ -462,11 +463,11 @@ def fused_forward_many(layers, xs, idxs, ws, overlap: bool = True, num_dispatch_
             if not fuse_cast:
                 C.per_token_cast_to_fp8(w.h, True, False, None, 1, w.hq, w.hs, w.m_offsets[L:], True)
             C.grouped_gemm(w.hq, w2, w.m_offsets, 0, False, None, None, None, 0, GEMM_TIMEOUT_MS, w.m_ends, w.hs, l._mx[3 if wide else 1],
-                           row_info=w.recv_info, scatter_bases=w.peer_bases[3 * R_:])
+                           row_info=w.recv_info, scatter_bases=w.peer_bases[3 * R_:], sched=w.sched)
         else:
             C.per_token_cast_to_fp8(w.h, False, False, None, 1, w.hq, w.hs, w.m_offsets[L:], False)
             C.grouped_gemm(w.hq, w2, w.m_offsets, 0, False, w.hs, s2, None, 0, GEMM_TIMEOUT_MS, w.m_ends, None, None,
-                           row_info=w.recv_info, scatter_bases=w.peer_bases[3 * R_:])
+                           row_info=w.recv_info, scatter_bases=w.peer_bases[3 * R_:], sched=w.sched)
     # every rank's second GEMM has finished scattering before anybody sums its stage
     if not lone:
         C.barrier(rts)
