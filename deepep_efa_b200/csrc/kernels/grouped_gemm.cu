@@ -35,6 +35,7 @@ namespace {
 constexpr int kBlockM = 128;
 constexpr int kKBlockBytes = 128;      // one 128B swizzle atom per row
 constexpr int kATileBytes = kBlockM * kKBlockBytes;  // 16 KiB
+constexpr int kEdgeRows = 32;          // rows of one copy when a tile of A is fetched in part
 constexpr int kTileSlots = 2;          // tiles the loader may hand to the other roles ahead of time
 constexpr int kMaxGroups = 1024;
 
@@ -490,6 +491,12 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         tma_prefetch_desc(&map_a);
         tma_prefetch_desc(&map_b);
     }
+    if (!kPair && p.mode == 0 && p.m_ends != nullptr) {  // see `edge` below
+        for (int s = 0; s < C::kStages; ++s)
+            for (int i = threadIdx.x; i < kATileBytes / 16; i += C::kThreads)
+                reinterpret_cast<int4*>(stage_base + (size_t)s * C::kStageBytes)[i] = make_int4(0, 0, 0, 0);
+        fence_proxy_async();
+    }
     // What precedes overlaps the end of the previous kernel (programmatic dependent launch); from here on its results are read.
     // The successor is released only now, so that a kernel that starts early finds every kernel before this one complete.
     pdl_wait_predecessor();
@@ -645,6 +652,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 return t;
             };
             int drawn_tile = 0;
+            unsigned stage_rows = 0;  // four bits per stage: 32-row pieces of A that are not zero
             for (int tile = sched_id; tile < total_tiles && ok; tile = hand_out(tile, drawn_tile)) {
                 if (drawn) drawn_tile = atomicAdd(p.sched, 1);  // used when this tile's loads have been issued
                 decode(tile, g, ti);
@@ -672,6 +680,12 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                     atomicMin(&p.trace[0], global_timer_ns());
                     stamped = true;
                 }
+                // Rows past the end of the group are not fetched when m_ends says where that is; the tensor core sees zeros instead.
+                // A stage holds 16 KB of A beside 32 KB of B, and rows that are multiplied for nothing cost power, which lowers the
+                // clock (decode, 20 tokens: 177 us for the first GEMM over stale bytes, 142 with all 128 rows fetched, 138 over
+                // zeros). One or two copies of 32 rows replace the copy of 128; with three or four the loading lane would fall behind.
+                const int valid_rows = max(1, ti.c_row_end - ti.a_row);
+                const int edge = (!kPair && p.mode == 0 && p.m_ends != nullptr && valid_rows <= 2 * kEdgeRows) ? (valid_rows + kEdgeRows - 1) / kEdgeRows : 0;
                 for (int kb = 0; kb < ti.num_kb; ++kb) {
                     s_prod_state[0] = 2;
                     if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag, limit, note, wait_id(1, tile, kb, stage))) {
@@ -705,7 +719,12 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                         continue;
                     }
                     s_prod_state[0] = 3;
-                    mbar_expect_tx(&full[stage], C::kStageTxBytes);
+                    // 32-row pieces of A to write: the valid ones, then pieces an earlier tile left in this stage (zeroed by copies from
+                    // past the last row, which touch no memory)
+                    const int filled = (int)(stage_rows >> (4 * stage)) & 7;
+                    const int pieces = edge == 0 ? kBlockM / kEdgeRows : max(edge, filled);
+                    stage_rows = (stage_rows & ~(7u << (4 * stage))) | ((unsigned)(edge == 0 ? kBlockM / kEdgeRows : edge) << (4 * stage));
+                    mbar_expect_tx(&full[stage], C::kStageTxBytes - kATileBytes + pieces * kEdgeRows * kKBlockBytes);
                     if constexpr (kMx) {
                         // scale atoms: [row tile][K block][512] for A, [group][n tile][K block][512] for B
                         uint8_t* ssf = sb + C::kBTileBytes;
@@ -715,7 +734,11 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                                      512 * C::kSfBAtoms, &full[stage]);
                     }
                     if (kMnMajor && p.a_mn) tma_load_3d(&map_a, &full[stage], sa, ti.a_kbase + kb * 64, ti.a_mn0 / 64);
-                    else tma_load_2d(&map_a, &full[stage], sa, ti.a_k0 + kb * elem_per_kb, ti.a_row);
+                    else if (edge == 0) tma_load_2d(&map_a, &full[stage], sa, ti.a_k0 + kb * elem_per_kb, ti.a_row);
+                    else
+                        for (int j = 0; j < pieces; ++j)
+                            tma_load_2d(&map_sfa, &full[stage], sa + j * kEdgeRows * kKBlockBytes, ti.a_k0 + kb * elem_per_kb,
+                                        j < edge ? ti.a_row + j * kEdgeRows : p.m_total);
                     if (kMnMajor && p.b_mn) {
                         tma_load_3d(&map_b, &full[stage], sb, ti.b_kbase + kb * 64, ti.b_mn0 / 64);
                     } else if (kSwiGLU) {
@@ -1295,6 +1318,9 @@ cudaError_t launch_impl(const GroupedGemmArgs& a, cudaStream_t stream) {
         if (!make_map_sf(&map_sfa, a.sfa_atoms, (((uint64_t)a.m_total + 127) / 128) * nkb, 128) ||
             !make_map_sf(&map_sfb, a.sfb_atoms, (uint64_t)a.num_groups * (a.n / kBlockN) * nkb, 128 * C::kSfBAtoms))
             return cudaErrorInvalidValue;
+    }
+    if constexpr (!kPair) {  // single CTAs read scale atoms without a map; the slot holds the map of A's partial tiles
+        if (a.mode == 0 && a.m_ends != nullptr && !make_map(&map_sfa, a.a, kFp8, (uint64_t)a.m_total, (uint64_t)a.k, kEdgeRows)) return cudaErrorInvalidValue;
     }
     const uint32_t b_box_rows = (kSwiGLU || kPair) ? kBlockN / 2 : kBlockN;
     bool ok;

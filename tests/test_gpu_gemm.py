@@ -241,6 +241,47 @@ def test_bf16_wgrad_reads_gradient_and_activation_in_place(rows, n_out, k_out):
             assert _rel_err(dw[g], ref) < 1e-2, (g, _rel_err(dw[g], ref))
 
 
+@pytest.mark.parametrize("kind", ["bf16", "fp32_scales", "mx_narrow", "mx_wide", "mx_wide_swiglu"])
+def test_partial_tiles_and_drawn_tiles(kind):
+    """Masked groups whose last tile is cut at and around multiples of 32 rows, after full tiles, with NaN bytes in the rows that do
+    not count; tiles drawn from a counter, which comes back zero, must give the same as tiles dealt out in strides."""
+    from deepep_efa_b200 import _ext
+    from deepep_efa_b200.ops.grouped_gemm import build_sf_atoms_a, build_sf_atoms_b, reference_grouped_gemm
+    C = _ext.load()
+    C.gemm_clear_error(0)
+    torch.manual_seed(17)
+    counts, stride, K, N = [1, 31, 256, 32, 0, 33, 160, 64, 65, 129, 128, 161, 97, 96, 200], 256, 512, 512
+    G, swiglu = len(counts), kind == "mx_wide_swiglu"
+    cnt = torch.tensor(counts, device="cuda", dtype=torch.int32)
+    starts = torch.arange(G + 1, device="cuda", dtype=torch.int32) * stride
+    live = (torch.arange(stride, device="cuda").unsqueeze(0) < cnt.unsqueeze(1)).view(-1)
+    x = torch.randn(G * stride, K, device="cuda").to(torch.bfloat16)
+    w = (torch.randn(G, N, K, device="cuda") * 0.1).to(torch.bfloat16)
+    a_s = b_s = sfa = sfb = None
+    if kind == "bf16":
+        a, b = x.clone(), w
+    else:
+        a, a_s = C.per_token_cast_to_fp8(x, kind != "fp32_scales", False)
+        b_s = torch.full((G, N // 128, K // 128), 2.0 ** -9, device="cuda")
+        b = (w.float() / 2.0 ** -9).to(torch.float8_e4m3fn)
+        if kind.startswith("mx"):
+            sfa, sfb = build_sf_atoms_a(a_s), build_sf_atoms_b(b_s, N, swiglu, kind != "mx_narrow")
+    ref = reference_grouped_gemm(a, b, starts, swiglu=swiglu, a_scales=a_s, b_scales=b_s)
+    a.view(torch.uint8)[~live] = 0xFF  # NaN in both types
+    outs = []
+    for sched in (None, torch.zeros(2, dtype=torch.int32, device="cuda")):
+        for sms in (0, 2):
+            out = torch.full((G * stride, N // 2 if swiglu else N), 7.0, device="cuda", dtype=torch.bfloat16)
+            scales = (None, None) if sfa is not None else (a_s, b_s)
+            C.grouped_gemm(a, b, starts, 0, swiglu, *scales, out, sms, 2000.0, cnt, sfa, sfb, m_ends_are_counts=True, sched=sched)
+            outs.append(out)
+    torch.cuda.synchronize()
+    assert C.gemm_error(0) == 0 and sched.tolist() == [0, 0]
+    assert _rel_err(outs[0][live], ref[live]) < (1.5e-2 if swiglu else 1e-2)
+    assert (outs[0][~live] == 7.0).all()
+    assert all(torch.equal(o, outs[0]) for o in outs)
+
+
 @pytest.mark.parametrize("pair", ["0", "1"])
 @pytest.mark.parametrize("n_out,k_out", [(128, 128), (128, 384), (384, 640), (256, 256)])
 def test_bf16_mn_major_half_width_tiles_and_pairs(monkeypatch, pair, n_out, k_out):
