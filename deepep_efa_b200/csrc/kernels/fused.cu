@@ -195,6 +195,7 @@ __device__ __forceinline__ unsigned long long global_timer() {
 template <int V>
 __global__ void __launch_bounds__(kEmDispatchThreads, 6) em_dispatch_kernel(const __grid_constant__ ArgPack<EmDispatchArgs, V> pack) {
     pdl_wait_predecessor();
+    pdl_release_successor();
     const EmDispatchArgs& a = pack.a[blockIdx.y];
     const RankCtx& c = a.ctx;
     const int R = c.num_ranks, me = c.rank, T = a.num_tokens, K = a.num_topk, E = a.num_experts, L = E / R, H = a.hidden;

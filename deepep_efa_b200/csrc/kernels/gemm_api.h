@@ -74,6 +74,9 @@ struct GroupedGemmArgs {
     // Optional [2], zero: tiles are drawn from a counter instead of dealt out in strides (single CTAs only; pairs ignore it). The
     // kernel leaves both words zero. Launches that may run at the same time need words of their own.
     int* sched;
+    // 1 = m_offsets and m_ends were final before the kernel in front of this one in the stream began, and that kernel started only
+    // after everything before it had ended: the tile table is then built without waiting for it (programmatic dependent launch).
+    int early_table;
 };
 
 // Returns cudaErrorInvalidValue for unsupported shapes (divisibility rules are in grouped_gemm.cu).

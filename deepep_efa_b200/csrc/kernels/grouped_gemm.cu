@@ -37,6 +37,7 @@ constexpr int kKBlockBytes = 128;      // one 128B swizzle atom per row
 constexpr int kATileBytes = kBlockM * kKBlockBytes;  // 16 KiB
 constexpr int kEdgeRows = 32;          // rows of one copy when a tile of A is fetched in part
 constexpr int kTileSlots = 2;          // tiles the loader may hand to the other roles ahead of time
+constexpr int kAheadBlocks = 10;       // K blocks of weights per CTA fetched into L2 before the predecessor ends: 48 MB of the 126 MB
 constexpr int kMaxGroups = 1024;
 
 // ---- PTX wrappers ---------------------------------------------------------------------------
@@ -89,6 +90,9 @@ __device__ __forceinline__ void tma_load_2d(const CUtensorMap* map, uint64_t* ba
         "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(smem_u32(dst)),
         "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(c0), "r"(c1)
         : "memory");
+}
+__device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* map, int c0, int c1) {
+    asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global [%0, {%1, %2}];" ::"l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1) : "memory");
 }
 // An MN-major operand tile in one copy: its chunks of 64 rows are the third dimension of the map (see make_map_mn).
 __device__ __forceinline__ void tma_load_3d(const CUtensorMap* map, uint64_t* bar, void* dst, int c1, int c2) {
@@ -499,8 +503,11 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     }
     // What precedes overlaps the end of the previous kernel (programmatic dependent launch); from here on its results are read.
     // The successor is released only now, so that a kernel that starts early finds every kernel before this one complete.
-    pdl_wait_predecessor();
-    pdl_release_successor();
+    // With p.early_table the group table is older than the predecessor, so the tile table and the first weights do not wait for it.
+    if (!p.early_table) {
+        pdl_wait_predecessor();
+        pdl_release_successor();
+    }
     if (warp == 2) {
         // tile table: one warp scans the groups (one thread walking 256 groups through dependent loads took about 10 us)
         const int tiles_n = p.mode == 0 ? col_tiles : 0;
@@ -616,6 +623,22 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         }
         return t;
     };
+
+    if (p.early_table) {
+        if (warp == 0 && lane == 0 && p.mode == 0 && sched_id < total_tiles) {
+            // weights of the first tile -> L2 while the predecessor's last tiles leave most SMs idle
+            int g = 0;
+            TileInfo ti;
+            decode(sched_id, g, ti);
+            for (int kb = 0; kb < min(ti.num_kb, kAheadBlocks); ++kb) {
+                if (kMnMajor && p.b_mn) break;
+                tma_prefetch_2d(&map_b, ti.b_k0 + kb * elem_per_kb, (kSwiGLU && kPair && cta_rank == 1) ? ti.b_row2 : ti.b_row);
+                if (kSwiGLU && !kPair) tma_prefetch_2d(&map_b, ti.b_k0 + kb * elem_per_kb, ti.b_row2);
+            }
+        }
+        pdl_wait_predecessor();
+        pdl_release_successor();
+    }
 
     // An epilogue warp hands an accumulator window back to the MMA issuer: in a pair that is the leader CTA's barrier.
     auto release_window = [&](uint64_t* bar) {

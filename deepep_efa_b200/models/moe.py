@@ -296,9 +296,9 @@ class MoELayer(nn.Module):
         if mx is not None:
             # GEMM1's epilogue quantises its own output (a wide tile holds one whole scale block of a row): e4m3 + scale atoms
             C.grouped_gemm(a, w13, w_["starts"], 0, True, None, None, None, 0, GEMM_TIMEOUT_MS, cnt, gg.build_sf_atoms_a(a_s), mx[0],
-                           out_fp8=w_["hq"], out_atoms=w_["ha"], m_ends_are_counts=True, sched=w_["sched"])
+                           out_fp8=w_["hq"], out_atoms=w_["ha"], m_ends_are_counts=True, sched=w_["sched"], early_table=True)
             C.grouped_gemm(w_["hq"], w2, w_["starts"], 0, False, None, None, y.view(L * N, H), 0, GEMM_TIMEOUT_MS, cnt, w_["ha"], mx[3],
-                           m_ends_are_counts=True, sched=w_["sched"])
+                           m_ends_are_counts=True, sched=w_["sched"], early_table=True)
         else:
             C.grouped_gemm(a, w13, w_["starts"], 0, True, a_s, s13, w_["h"], 0, GEMM_TIMEOUT_MS, cnt, m_ends_are_counts=True, sched=w_["sched"])
             C.per_token_cast_to_fp8(w_["h"], False, False, cnt, N, w_["hq"], w_["hs"])
@@ -448,7 +448,7 @@ def fused_forward_many(layers, xs, idxs, ws, overlap: bool = True, num_dispatch_
         parts = [(0, ga, 148 - RESERVED_SMS), (ga, L - ga, 0)] if (overlapped and ga < L) else [(0, L, (148 - RESERVED_SMS) if overlapped else 0)]
         for pi, (g0, ng, sms1) in enumerate(parts):
             tr = None if (w.trace is None or pi > 0) else w.trace[2:6]
-            gate = dict(ready=w.arrived[g0:g0 + ng], expected=w.expected[g0:g0 + ng], trace=tr, sched=w.sched)
+            gate = dict(ready=w.arrived[g0:g0 + ng], expected=w.expected[g0:g0 + ng], trace=tr, sched=w.sched, early_table=not overlapped)
             mo, me_ = w.m_offsets[g0:g0 + ng + 1], w.m_ends[g0:g0 + ng]
             if native:
                 if fuse_cast:
@@ -463,11 +463,11 @@ def fused_forward_many(layers, xs, idxs, ws, overlap: bool = True, num_dispatch_
             if not fuse_cast:
                 C.per_token_cast_to_fp8(w.h, True, False, None, 1, w.hq, w.hs, w.m_offsets[L:], True)
             C.grouped_gemm(w.hq, w2, w.m_offsets, 0, False, None, None, None, 0, GEMM_TIMEOUT_MS, w.m_ends, w.hs, l._mx[3 if wide else 1],
-                           row_info=w.recv_info, scatter_bases=w.peer_bases[3 * R_:], sched=w.sched)
+                           row_info=w.recv_info, scatter_bases=w.peer_bases[3 * R_:], sched=w.sched, early_table=True)
         else:
             C.per_token_cast_to_fp8(w.h, False, False, None, 1, w.hq, w.hs, w.m_offsets[L:], False)
             C.grouped_gemm(w.hq, w2, w.m_offsets, 0, False, w.hs, s2, None, 0, GEMM_TIMEOUT_MS, w.m_ends, None, None,
-                           row_info=w.recv_info, scatter_bases=w.peer_bases[3 * R_:], sched=w.sched)
+                           row_info=w.recv_info, scatter_bases=w.peer_bases[3 * R_:], sched=w.sched, early_table=True)
     # every rank's second GEMM has finished scattering before anybody sums its stage
     if not lone:
         C.barrier(rts)
