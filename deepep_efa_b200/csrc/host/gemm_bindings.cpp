@@ -234,10 +234,9 @@ std::tuple<torch::Tensor, torch::Tensor, torch::Tensor, torch::Tensor, int64_t> 
     return {pos, src_row, src_k, m_offsets, m_pad};
 }
 
-// dst[m] = scale * src[src_row[m]]; rows of any dtype whose byte size is a multiple of 4 (of 16 with a scale, which needs bf16).
-// The scale of row m is scale[m], or with src_k ([M]) scale[src_row[m], src_k[m]] of a matrix.
+// dst[m] = scale * src[src_row[m]]; rows of any dtype whose byte size is a multiple of 4 (of 16 with a scale, which needs bf16)
 torch::Tensor gather_rows(const torch::Tensor& src, const torch::Tensor& src_row, c10::optional<torch::Tensor> scale,
-                          c10::optional<torch::Tensor> out, c10::optional<torch::Tensor> src_k) {
+                          c10::optional<torch::Tensor> out) {
     DXG_CHECK(src.is_cuda() && src.dim() == 2 && src.is_contiguous(), "src must be a contiguous CUDA matrix");
     DXG_CHECK(src_row.scalar_type() == torch::kInt32 && src_row.is_contiguous() && src_row.dim() == 1, "src_row must be int32 [M]");
     const int64_t M = src_row.numel();
@@ -247,20 +246,13 @@ torch::Tensor gather_rows(const torch::Tensor& src, const torch::Tensor& src_row
     torch::Tensor dst = out.has_value() ? *out : torch::empty({M, src.size(1)}, src.options());
     DXG_CHECK(dst.is_contiguous() && dst.scalar_type() == src.scalar_type() && dst.size(0) == M && dst.size(1) == src.size(1), "out has the wrong shape");
     const float* sc = nullptr;
-    int num_k = 0;
     if (scale.has_value()) {
-        DXG_CHECK(src.scalar_type() == torch::kBFloat16 && scale->scalar_type() == torch::kFloat32 && scale->is_contiguous(), "scale needs bf16 rows and must be f32");
-        if (src_k.has_value()) {
-            DXG_CHECK(scale->dim() == 2 && scale->size(0) == src.size(0) && src_k->scalar_type() == torch::kInt32 && src_k->is_contiguous() && src_k->numel() == M,
-                      "with src_k (int32 [M]) the scale is a matrix with one row per source row");
-            num_k = (int)scale->size(1);
-        } else {
-            DXG_CHECK(scale->numel() == M, "scale must be f32 [M]");
-        }
+        DXG_CHECK(src.scalar_type() == torch::kBFloat16 && scale->scalar_type() == torch::kFloat32 && scale->is_contiguous() && scale->numel() == M,
+                  "scale needs bf16 rows and must be f32 [M]");
         sc = scale->data_ptr<float>();
     }
-    const cudaError_t e = dx::launch_gather_rows(src.data_ptr(), dst.data_ptr(), src_row.data_ptr<int>(), sc, num_k > 0 ? src_k->data_ptr<int>() : nullptr, num_k,
-                                                 (int)M, (int)row_bytes, at::cuda::getCurrentCUDAStream(src.device().index()).stream());
+    const cudaError_t e = dx::launch_gather_rows(src.data_ptr(), dst.data_ptr(), src_row.data_ptr<int>(), sc, (int)M,
+                                                 (int)row_bytes, at::cuda::getCurrentCUDAStream(src.device().index()).stream());
     if (e != cudaSuccess) throw std::runtime_error(std::string("gather_rows: ") + cudaGetErrorString(e));
     return dst;
 }
@@ -321,6 +313,25 @@ torch::Tensor swiglu_bwd(const torch::Tensor& h13, const torch::Tensor& dh) {
     return out;
 }
 
+// Gradients (a's, w's) of y[n] = sum_k w[n, k] * a[pos[n, k]] for the output gradient g
+std::tuple<torch::Tensor, torch::Tensor> unpermute_bwd(const torch::Tensor& a, const torch::Tensor& g, const torch::Tensor& w, const torch::Tensor& pos,
+                                                       const torch::Tensor& src_row) {
+    DXG_CHECK(a.is_cuda() && a.is_contiguous() && a.scalar_type() == torch::kBFloat16 && a.dim() == 2, "unpermute_bwd: a must be contiguous CUDA bf16 [M,H]");
+    auto here = [&](const torch::Tensor& t) { return t.device() == a.device() && t.is_contiguous(); };
+    DXG_CHECK(here(g) && g.scalar_type() == torch::kBFloat16 && g.dim() == 2 && g.size(1) == a.size(1), "unpermute_bwd: g must be bf16 [N,H]");
+    DXG_CHECK(here(pos) && pos.scalar_type() == torch::kInt32 && pos.dim() == 2 && pos.size(0) == g.size(0), "unpermute_bwd: pos must be int32 [N,K]");
+    DXG_CHECK(here(w) && w.scalar_type() == torch::kFloat32 && w.numel() == pos.numel(), "unpermute_bwd: w must be f32 [N,K]");
+    DXG_CHECK(here(src_row) && src_row.scalar_type() == torch::kInt32 && src_row.numel() == a.size(0), "unpermute_bwd: src_row must be int32 [M]");
+    c10::cuda::CUDAGuard guard(a.device());
+    auto da = torch::empty_like(a);
+    auto dw = torch::empty({pos.size(0), pos.size(1)}, a.options().dtype(torch::kFloat32));
+    const cudaError_t e = dx::launch_unpermute_bwd(a.data_ptr(), g.data_ptr(), w.data_ptr<float>(), pos.data_ptr<int>(), src_row.data_ptr<int>(), da.data_ptr(),
+                                                   dw.data_ptr<float>(), (int)pos.size(0), (int)pos.size(1), (int)a.size(0), (int)a.size(1),
+                                                   at::cuda::getCurrentCUDAStream(a.get_device()).stream());
+    DXG_CHECK(e == cudaSuccess, "unpermute_bwd: hidden must be a multiple of 8");
+    return {da, dw};
+}
+
 torch::Tensor rowdot(const torch::Tensor& a, const torch::Tensor& b, const torch::Tensor& pos) {
     DXG_CHECK(a.is_cuda() && a.is_contiguous() && a.scalar_type() == torch::kBFloat16 && a.dim() == 2, "rowdot: a must be contiguous CUDA bf16 [M,H]");
     DXG_CHECK(b.is_cuda() && b.is_contiguous() && b.scalar_type() == torch::kBFloat16 && b.dim() == 2 && b.size(1) == a.size(1), "rowdot: b must be bf16 [N,H]");
@@ -365,6 +376,7 @@ void bind_gemm(py::module_& m) {
     m.def("transpose_bf16", &transpose_bf16);
     m.def("swiglu_fwd", &swiglu_fwd);
     m.def("swiglu_bwd", &swiglu_bwd);
+    m.def("unpermute_bwd", &unpermute_bwd);
     m.def("rowdot", &rowdot);
     m.def("grouped_gemm", &grouped_gemm, py::arg("a"), py::arg("b"), py::arg("m_offsets"), py::arg("mode") = 0, py::arg("swiglu") = false,
           py::arg("a_scales") = py::none(), py::arg("b_scales") = py::none(), py::arg("out") = py::none(), py::arg("num_sms") = 0,
@@ -374,8 +386,7 @@ void bind_gemm(py::module_& m) {
           py::arg("out_fp8") = py::none(), py::arg("out_atoms") = py::none(), py::arg("m_ends_are_counts") = false, py::arg("sched") = py::none(),
           py::arg("early_table") = false);
     m.def("build_plan", &build_plan);
-    m.def("gather_rows", &gather_rows, py::arg("src"), py::arg("src_row"), py::arg("scale") = py::none(), py::arg("out") = py::none(),
-          py::arg("src_k") = py::none());
+    m.def("gather_rows", &gather_rows, py::arg("src"), py::arg("src_row"), py::arg("scale") = py::none(), py::arg("out") = py::none());
     m.def("gather_reduce_rows", &gather_reduce_rows, py::arg("src"), py::arg("pos"), py::arg("w") = py::none(), py::arg("out") = py::none());
     m.def("gemm_error", &gemm_error);
     m.def("gemm_clear_error", &gemm_clear_error);

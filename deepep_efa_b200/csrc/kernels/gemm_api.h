@@ -89,10 +89,10 @@ cudaError_t launch_build_plan(const int64_t* topk_idx, const int* host_offsets, 
                               int num_rows, int num_topk, int num_local_experts, cudaStream_t stream);
 
 // Row gathers between receive order and the expert-major, 128-row-aligned layout (permute.cu).
-//   dst[m] = scale * src[src_row[m]]   (src_row[m] < 0 -> zero row; scale may be null; bf16 rows when scaled). The scale of row m is
-//   scale[m], or with num_k > 0 scale[src_row[m] * num_k + src_k[m]]. Rows are multiples of 4 bytes (of 16 when scaled).
-cudaError_t launch_gather_rows(const void* src, void* dst, const int* src_row, const float* scale, const int* src_k, int num_k, int num_dst_rows,
-                               int row_bytes, cudaStream_t stream);
+//   dst[m] = scale * src[src_row[m]]   (src_row[m] < 0 -> zero row; scale may be null; bf16 rows when scaled, one scale per row m). Rows
+//   are multiples of 4 bytes (of 16 when scaled).
+cudaError_t launch_gather_rows(const void* src, void* dst, const int* src_row, const float* scale, int num_dst_rows, int row_bytes,
+                               cudaStream_t stream);
 //   dst[n] = sum_k w[n,k] * src[pos[n,k]]  (bf16 rows, fp32 accumulate; pos < 0 skipped; w may be null = 1)
 cudaError_t launch_gather_reduce_rows(const void* src, void* dst, const int* pos, const float* w, int num_dst_rows, int num_k, int hidden,
                                       cudaStream_t stream);
@@ -104,6 +104,10 @@ cudaError_t launch_transpose_bf16(const void* in, void* out, int batch, int rows
 cudaError_t launch_swiglu_fwd(const void* h13, void* h, long long rows, int inter, cudaStream_t stream);
 //   dh13 = d/dh13 of the above given dh
 cudaError_t launch_swiglu_bwd(const void* h13, const void* dh, void* dh13, long long rows, int inter, cudaStream_t stream);
+//   gradient of y[n] = sum_k w[n, k] * a[pos[n, k]]: da[m] = w[n, k] * g[n] for the (n, k) with pos[n, k] = m, 0 where src_row[m] < 0;
+//   dw[n, k] = <a[pos[n, k]], g[n]>, 0 where pos < 0
+cudaError_t launch_unpermute_bwd(const void* a, const void* g, const float* w, const int* pos, const int* src_row, void* da, float* dw, int n_rows,
+                                 int num_k, int m_rows, int hidden, cudaStream_t stream);
 //   out[n, k] = <a[pos[n, k]], b[n]>  (f32 out, 0 where pos < 0)
 cudaError_t launch_rowdot(const void* a, const void* b, const int* pos, float* out, int n_rows, int num_k, int hidden, cudaStream_t stream);
 

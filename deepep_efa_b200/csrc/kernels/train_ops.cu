@@ -4,6 +4,7 @@
 //                      the weight-gradient GEMM reduces over tokens and wants them contiguous, the input-gradient GEMM wants
 //                      the weights with their output dimension contiguous
 //   swiglu_fwd / bwd   h = silu(gate) * up from h13 = [gate | up], and its gradient, in one pass each (fp32 math, bf16 I/O)
+//   unpermute_bwd      both gradients of the weighted un-permute in one pass over its input
 //   rowdot             d_w[n, k] = <a[pos[n, k]], b[n]>  (gradient of the gate weights through the weighted un-permute)
 //
 // The reference has no counterpart (it ships no model code); these replace chains of framework ops whose copies
@@ -144,7 +145,71 @@ __global__ void __launch_bounds__(256) rowdot_kernel(const __nv_bfloat16* __rest
     }
 }
 
+// Both gradients of the weighted un-permute. One warp per (n, k): row a[pos] and row g[n] are read once and w * g[n] is written, where a
+// row product and a gather of their own read g twice and could not hide the gather's writes (87 % of its traffic) behind reads. The
+// num_k warps of a token are neighbours, so g[n] comes from L1 or L2 for all but the first. Further warps clear the padding rows.
+__global__ void __launch_bounds__(256) unpermute_bwd_kernel(const __nv_bfloat16* __restrict__ a, const __nv_bfloat16* __restrict__ g,
+                                                            const float* __restrict__ w, const int* __restrict__ pos,
+                                                            const int* __restrict__ src_row, __nv_bfloat16* __restrict__ da, float* __restrict__ dw,
+                                                            long long pairs, long long items, int num_k, int hidden) {
+    pdl_wait_predecessor();
+    pdl_release_successor();
+    const int lane = threadIdx.x & 31, n16 = hidden / 8;
+    const long long p = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (p >= items) return;
+    if (p >= pairs) {
+        const long long m = p - pairs;
+        if (src_row[m] >= 0) return;
+        int4* row = reinterpret_cast<int4*>(da + (size_t)m * hidden);
+        for (int i = lane; i < n16; i += 32) row[i] = make_int4(0, 0, 0, 0);
+        return;
+    }
+    const int src = pos[p];
+    float acc = 0.f;
+    if (src >= 0) {
+        const float sc = w[p];
+        const int4* ar = reinterpret_cast<const int4*>(a + (size_t)src * hidden);
+        const int4* gr = reinterpret_cast<const int4*>(g + (size_t)(p / num_k) * hidden);
+        int4* dr = reinterpret_cast<int4*>(da + (size_t)src * hidden);
+        constexpr int U = 4;  // column chunks of both rows in flight per lane
+        for (int i0 = 0; i0 < n16; i0 += 32 * U) {
+            int4 x[U], y[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int i = i0 + u * 32 + lane;
+                x[u] = i < n16 ? ld_stream(ar + i) : make_int4(0, 0, 0, 0);
+                y[u] = i < n16 ? gr[i] : make_int4(0, 0, 0, 0);
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int i = i0 + u * 32 + lane;
+                const uint32_t xw[4] = {(uint32_t)x[u].x, (uint32_t)x[u].y, (uint32_t)x[u].z, (uint32_t)x[u].w};
+                uint32_t yw[4] = {(uint32_t)y[u].x, (uint32_t)y[u].y, (uint32_t)y[u].z, (uint32_t)y[u].w};
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float2 xf = bf16x2_to_f2(xw[j]), yf = bf16x2_to_f2(yw[j]);
+                    acc = fmaf(xf.x, yf.x, fmaf(xf.y, yf.y, acc));
+                    yw[j] = f2_to_bf16x2(yf.x * sc, yf.y * sc);
+                }
+                if (i < n16) dr[i] = make_int4((int)yw[0], (int)yw[1], (int)yw[2], (int)yw[3]);
+            }
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (lane == 0) dw[p] = acc;
+}
+
 }  // namespace
+
+cudaError_t launch_unpermute_bwd(const void* a, const void* g, const float* w, const int* pos, const int* src_row, void* da, float* dw, int n_rows,
+                                 int num_k, int m_rows, int hidden, cudaStream_t stream) {
+    const long long pairs = (long long)n_rows * num_k, items = pairs + m_rows;
+    if (items <= 0) return cudaSuccess;
+    if ((hidden & 7) != 0) return cudaErrorInvalidValue;
+    return launch_dependent(unpermute_bwd_kernel, dim3((unsigned)((items + 7) / 8)), 256, 0, stream, static_cast<const __nv_bfloat16*>(a),
+                            static_cast<const __nv_bfloat16*>(g), w, pos, src_row, static_cast<__nv_bfloat16*>(da), dw, pairs, items, num_k, hidden);
+}
 
 cudaError_t launch_transpose_bf16(const void* in, void* out, int batch, int rows, int cols, cudaStream_t stream) {
     if (batch <= 0 || rows <= 0 || cols <= 0) return cudaSuccess;

@@ -118,8 +118,8 @@ class _UnpermuteWeighted(torch.autograd.Function):
         grad = grad.contiguous()
         # d y_perm[m] = w[src_row[m], src_k[m]] * grad[src_row[m]];  d w[n, k] = <y_perm[pos[n, k]], grad[n]>
         if grad.is_cuda and grad.dtype == torch.bfloat16 and y_perm.dtype == torch.bfloat16:
-            d_y_perm = _ext.load().gather_rows(grad, plan.src_row, weights.float().contiguous(), None, plan.src_k)
-            return d_y_perm, _ext.load().rowdot(y_perm, grad, plan.pos).to(weights.dtype), None, None
+            d_y_perm, d_w = _ext.load().unpermute_bwd(y_perm, grad, weights.float().contiguous(), plan.pos, plan.src_row)
+            return d_y_perm, d_w.to(weights.dtype), None, None
         w_flat = weights.reshape(-1)
         K = weights.size(1)
         idx = (plan.src_row.clamp(min=0).long() * K + plan.src_k.long())

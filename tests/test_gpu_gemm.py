@@ -168,6 +168,28 @@ def test_rowdot_kernel():
     assert torch.allclose(got, want, rtol=1e-3, atol=1e-2)
 
 
+@pytest.mark.parametrize("N,K,H,pad", [(1, 1, 8, 0), (37, 6, 1032, 5), (120, 8, 4096, 77)])
+def test_unpermute_backward_kernel(N, K, H, pad):
+    """Row gradients bit for bit (one product, rounded once), weight gradients against fp32 sums, padding rows cleared."""
+    from deepep_efa_b200 import _ext
+    torch.manual_seed(10)
+    M = N * K + pad
+    keep = torch.rand(N, K, device="cuda") < 0.8
+    pos = torch.where(keep, torch.randperm(M, device="cuda")[:N * K].view(N, K), torch.full((N, K), -1, device="cuda")).int()
+    src_row = torch.full((M,), -1, device="cuda", dtype=torch.int32)
+    n_of = torch.arange(N, device="cuda").unsqueeze(1).expand(N, K)
+    src_row[pos[keep].long()] = n_of[keep].int()
+    a, g = (torch.randn(r, H, device="cuda").to(torch.bfloat16) for r in (M, N))
+    w = torch.rand(N, K, device="cuda")
+    da, dw = _ext.load().unpermute_bwd(a, g, w, pos, src_row)
+    want = torch.zeros(M, H, device="cuda", dtype=torch.bfloat16)
+    want[pos[keep].long()] = (w[keep].unsqueeze(1) * g[n_of[keep]].float()).to(torch.bfloat16)
+    assert torch.equal(da, want)
+    dot = torch.where(keep, (a[pos.clamp(min=0).long()].double() * g.double().unsqueeze(1)).sum(-1), torch.zeros(N, K, device="cuda", dtype=torch.double))
+    # fp32 sum of H products of unit variance: error well below H * 2^-24 * max |partial sum|
+    assert (dw.double() - dot).abs().max().item() < 1e-3
+
+
 @pytest.mark.parametrize("swiglu,wide", [(False, True), (False, False), (True, True), (True, False)])
 def test_fp8_native_block_scaling(swiglu, wide):
     """tcgen05 block-scaled MMA with UE8M0 scale atoms against the dequantised fp32 reference; the row scales differ by
