@@ -65,7 +65,7 @@ torch::Tensor grouped_gemm(const torch::Tensor& a, const torch::Tensor& b, const
                            c10::optional<torch::Tensor> ready, c10::optional<torch::Tensor> expected,
                            c10::optional<torch::Tensor> row_info, c10::optional<torch::Tensor> scatter_bases,
                            c10::optional<torch::Tensor> trace, bool mn_major, c10::optional<torch::Tensor> out_fp8,
-                           c10::optional<torch::Tensor> out_atoms, bool m_ends_are_counts, c10::optional<torch::Tensor> sched, bool early_table) {
+                           c10::optional<torch::Tensor> out_atoms, bool m_ends_are_counts, c10::optional<torch::Tensor> sched, bool early_table, bool tokens_as_columns) {
     DXG_CHECK(a.is_cuda() && b.is_cuda() && m_offsets.is_cuda(), "operands must be CUDA tensors");
     DXG_CHECK(a.is_contiguous() && b.is_contiguous() && m_offsets.is_contiguous(), "operands must be contiguous");
     DXG_CHECK(m_offsets.scalar_type() == torch::kInt32 && m_offsets.dim() == 1 && m_offsets.numel() >= 2, "m_offsets must be int32 [G+1]");
@@ -200,6 +200,9 @@ torch::Tensor grouped_gemm(const torch::Tensor& a, const torch::Tensor& b, const
         DXG_CHECK(trace->element_size() == 8 && trace->is_contiguous() && trace->numel() >= 4, "trace must be 64-bit [4]");
         p.trace = reinterpret_cast<unsigned long long*>(trace->data_ptr());
     }
+    // The caller says that groups have few rows. Only the natively block-scaled 256-column tiles without a scatter have the form with
+    // the weights as M; SwiGLU then quantises its output.
+    p.swap = (tokens_as_columns && p.m_ends != nullptr && p.sfa_atoms != nullptr && p.mx_wide && !p.cta_pairs && p.row_info == nullptr && (!swiglu || p.c_fp8 != nullptr)) ? 1 : 0;
     p.error_flag = error_flag(device).data_ptr<int>();
     p.timeout_cycles = (long long)(timeout_ms * (double)clock_khz(device));
     const cudaError_t e = dx::launch_grouped_gemm(p, at::cuda::getCurrentCUDAStream(device).stream());
@@ -384,7 +387,7 @@ void bind_gemm(py::module_& m) {
           py::arg("ready") = py::none(), py::arg("expected") = py::none(), py::arg("row_info") = py::none(),
           py::arg("scatter_bases") = py::none(), py::arg("trace") = py::none(), py::arg("mn_major") = false,
           py::arg("out_fp8") = py::none(), py::arg("out_atoms") = py::none(), py::arg("m_ends_are_counts") = false, py::arg("sched") = py::none(),
-          py::arg("early_table") = false);
+          py::arg("early_table") = false, py::arg("tokens_as_columns") = false);
     m.def("build_plan", &build_plan);
     m.def("gather_rows", &gather_rows, py::arg("src"), py::arg("src_row"), py::arg("scale") = py::none(), py::arg("out") = py::none());
     m.def("gather_reduce_rows", &gather_reduce_rows, py::arg("src"), py::arg("pos"), py::arg("w") = py::none(), py::arg("out") = py::none());

@@ -77,6 +77,8 @@ struct GroupedGemmArgs {
     // 1 = m_offsets and m_ends were final before the kernel in front of this one in the stream began, and that kernel started only
     // after everything before it had ended: the tile table is then built without waiting for it (programmatic dependent launch).
     int early_table;
+    // 1 = natively block-scaled 256-column tiles with the weights as the M operand and the tokens as N (see launch_grouped_gemm)
+    int swap;
 };
 
 // Returns cudaErrorInvalidValue for unsupported shapes (divisibility rules are in grouped_gemm.cu).

@@ -146,6 +146,15 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
         : "r"(taddr)
         : "memory");
 }
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
+          "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+        : "r"(taddr)
+        : "memory");
+}
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 // K-major operand tile in 128B-swizzled shared memory: rows are 128 bytes apart, 8-row groups 1024 bytes
@@ -385,6 +394,15 @@ __device__ __forceinline__ void store_rows_256(int4* stage, const int4 (&regs)[1
     }
 }
 
+// Four lanes hold one byte of each of four tokens (byte t of the word) for neighbouring features: afterwards lane j of the four holds
+// the four features of token j.
+__device__ __forceinline__ uint32_t transpose_bytes_4x4(uint32_t w, int lane) {
+    uint32_t o = __shfl_xor_sync(0xffffffffu, w, 1);
+    w = __byte_perm(w, o, (lane & 1) ? 0x3715 : 0x6240);
+    o = __shfl_xor_sync(0xffffffffu, w, 2);
+    return __byte_perm(w, o, (lane & 2) ? 0x3276 : 0x5410);
+}
+
 // Rows of group g (mode 0), which starts at row `begin`.
 __device__ __forceinline__ int group_rows(const GroupedGemmArgs& p, int g, int begin) {
     if (p.m_ends == nullptr) return max(p.m_offsets[g + 1] - begin, 0);
@@ -440,11 +458,12 @@ struct Cfg {
         (size_t)kStages * kStageBytes + (size_t)kEpiWarps * kOutStageBytes + 1024 /*align*/ + 256 /*barriers*/ + (kMaxGroups + 1) * 4 + kXchBytes;
 };
 
-template <int kBlockN, bool kFp8, bool kSwiGLU, bool kPair, bool kMx = false, bool kRowScatter = false>
+template <int kBlockN, bool kFp8, bool kSwiGLU, bool kPair, bool kMx = false, bool kRowScatter = false, bool kSwap = false>
 __global__ void __launch_bounds__((Cfg<kBlockN, kFp8, kSwiGLU, kPair, kMx, kRowScatter>::kThreads), 1)
 grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                     const __grid_constant__ CUtensorMap map_sfa, const __grid_constant__ CUtensorMap map_sfb, const GroupedGemmArgs p) {
     using C = Cfg<kBlockN, kFp8, kSwiGLU, kPair, kMx, kRowScatter>;
+    static_assert(!kSwap || (kMx && !kPair && kBlockN == 256), "weights as M: natively block-scaled 256-column tiles on single CTAs");
     static_assert(!kRowScatter || (kMx && !kSwiGLU && !kPair && kBlockN == 128), "whole-row scatter: natively block-scaled 128-column tiles");
     static_assert(!kMx || (kFp8 && ((!kPair && kBlockN == 128) || (kBlockN == 256 && (kSwiGLU || !kPair)))),
                   "native block scaling: e4m3 operands; 128-column tiles, 256-column tiles, or 256-column SwiGLU tiles on a CTA pair");
@@ -640,6 +659,13 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         pdl_release_successor();
     }
 
+    // kSwap: the weights are the M operand and the tokens the N operand, in steps of 32 columns up to the tile's valid rows. A group of
+    // four rows as M is 128 rows of products for four, and the power they take lowers the clock: streaming 256 experts of 7168 -> 2048
+    // for 128 tokens back to back ran at 1.2 GHz of 1.97 and 2053 us per layer that way, 1850 us this way. Everything up to the MMA
+    // (tiles, copies, scale atoms) is the same; the epilogue finds features in lanes and tokens in columns. An instantiation of its
+    // own: with both epilogues in one kernel the spills of either made 20-token steps 5 % slower instead of 9 % faster.
+    auto token_cols = [&](const TileInfo& t) { return min(kBlockM, (max(1, t.c_row_end - t.a_row) + 31) & ~31); };
+
     // An epilogue warp hands an accumulator window back to the MMA issuer: in a pair that is the leader CTA's barrier.
     auto release_window = [&](uint64_t* bar) {
         if constexpr (kPair) {
@@ -823,7 +849,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             for (int tile = sched_id; tile < total_tiles && ok; tile = next_tile(tile, false)) {
                 decode(tile, g, ti);
                 if (ti.num_kb == 0) continue;  // epilogue writes zeros on its own
-                const uint32_t idesc = (C::kRagged && ti.n_cols != kBlockN) ? idesc_half : idesc_full;
+                const uint32_t idesc = kSwap ? make_idesc_mx(token_cols(ti), kBlockM) : (C::kRagged && ti.n_cols != kBlockN) ? idesc_half : idesc_full;
                 for (int kb = 0; kb < ti.num_kb; ++kb) {
                     const bool new_window = C::kPromote ? true : (kb == 0);
                     if (new_window) {
@@ -860,10 +886,20 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                             tmem_cp_sf(t_sfa, make_sf_desc(ssf));
 #pragma unroll
                             for (int at = 0; at < C::kSfBAtoms; ++at) tmem_cp_sf(t_sfb + 4 * at, make_sf_desc(ssf + 512 + 512 * at));
+                            if constexpr (kSwap) {
+                                // weight rows as M (two tiles of 128), token rows as N
 #pragma unroll
-                            for (int j = 0; j < 4; ++j)
-                                umma_mx(tmem_d, adesc + (uint64_t)(j * 2), bdesc + (uint64_t)(j * 2), idesc, t_sfa, t_sfb,
-                                        (new_window && j == 0) ? 0u : 1u);
+                                for (int hw = 0; hw < kBlockN / kBlockM; ++hw)
+#pragma unroll
+                                    for (int j = 0; j < 4; ++j)
+                                        umma_mx(tmem_d + hw * kBlockM, bdesc + (uint64_t)(hw * (kATileBytes >> 4) + j * 2), adesc + (uint64_t)(j * 2), idesc,
+                                                t_sfb + 4 * hw, t_sfa, (new_window && j == 0) ? 0u : 1u);
+                            } else {
+#pragma unroll
+                                for (int j = 0; j < 4; ++j)
+                                    umma_mx(tmem_d, adesc + (uint64_t)(j * 2), bdesc + (uint64_t)(j * 2), idesc, t_sfa, t_sfb,
+                                            (new_window && j == 0) ? 0u : 1u);
+                            }
                         }
                         sf_buf ^= 1;
                     } else {
@@ -1050,7 +1086,103 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(win * kBlockN);
                 __nv_bfloat16* wbase = cbase + (size_t)(ti.c_row + q * 32) * ldc + ti.c_col;
                 const int rows_valid = min(32, ti.c_row_end - (ti.c_row + q * 32));
-                if constexpr (kSwiGLU && C::kWindows == 1) {
+                if constexpr (kSwap) {
+                    // TMEM lane = weight row, column = token. The two warps of a quarter take alternate chunks of 16 tokens; a thread
+                    // has one feature of the gate (or first) half and one of the up (second) half of every token.
+                    const int n_tok = token_cols(ti), tok_valid = ti.c_row_end - ti.c_row;
+                    const unsigned tag = (unsigned)(++xch_iter & 0xffff) << 16;
+                    volatile uint32_t* xs = reinterpret_cast<volatile uint32_t*>(xch) + (xch_iter & 1) * (kBlockM * 4);
+#pragma unroll 1
+                    for (int tb = 0; tb < n_tok && ok; tb += 64) {  // two chunks at a time: all four would not fit the registers
+                        uint32_t v[2][16], u[2][16];
+#pragma unroll
+                        for (int c = 0; c < 2; ++c) {
+                            const int t0 = tb + (2 * c + half) * 16;
+                            if (t0 < n_tok) {
+                                tmem_ld16(taddr + t0, v[c]);
+                                tmem_ld16(taddr + kBlockM + t0, u[c]);
+                            }
+                        }
+                        tmem_ld_wait();
+                        if (tb + 64 >= n_tok) {
+                            tc_fence_before();
+                            __syncwarp();
+                            if (lane == 0) release_window(&tmem_empty[win]);
+                        }
+#pragma unroll
+                        for (int c = 0; c < 2; ++c) {
+                            const int t0 = tb + (2 * c + half) * 16;
+                            if (t0 >= n_tok) break;
+                            if constexpr (kSwiGLU) {
+                                // same arithmetic as the row-wise epilogue: BF16-rounded product, power-of-two scale from the amax of the
+                                // token's 128 features. NaN does not count, as with fmaxf. Four warps hold 32 features each and exchange
+                                // their maxima (exact in BF16) through tagged words, two tile parities.
+                                float h[16];
+                                uint32_t mine = 0;
+#pragma unroll
+                                for (int t = 0; t < 16; ++t) {
+                                    h[t] = __bfloat162float(__float2bfloat16(silu(__uint_as_float(v[c][t])) * __uint_as_float(u[c][t])));
+                                    const uint32_t bits = (__float_as_uint(h[t]) >> 16) & 0x7fffu;
+                                    const uint32_t m = __reduce_max_sync(0xffffffffu, bits > 0x7f80u ? 0u : bits);
+                                    if (lane == t) mine = m;
+                                }
+                                volatile uint32_t* slot = xs + (t0 + (lane & 15)) * 4;
+                                if (lane < 16) slot[q] = tag | mine;
+                                if (lane < 16) {
+                                    const long long w0 = clock64();
+                                    for (int i = 0; i < 4 && ok; ++i) {
+                                        uint32_t w = slot[i];
+                                        while ((w & 0xffff0000u) != tag) {
+                                            if (*abort_flag || clock64() - w0 > limit) {
+                                                if (!*abort_flag && note != nullptr) atomicCAS(note, 0ull, wait_id(7, tile, 0, warp));
+                                                *abort_flag = 1;
+                                                ok = false;
+                                                break;
+                                            }
+                                            w = slot[i];
+                                        }
+                                        mine = max(mine, w & 0xffffu);
+                                    }
+                                }
+                                ok = __all_sync(0xffffffffu, ok);
+                                if (!ok) break;
+                                float scale, inv;
+                                fp8_scale_from_amax(__uint_as_float(mine << 16), true, scale, inv);
+                                if (q == 0 && lane < 16 && t0 + lane < tok_valid) {
+                                    const int trow = ti.c_row + t0 + lane;
+                                    *reinterpret_cast<uint32_t*>(p.c_atoms + ((size_t)(trow >> 7) * (ldc / 128) + (ti.c_col >> 7)) * 512 + (trow & 31) * 16 +
+                                                                 ((trow >> 5) & 3) * 4) = ((__float_as_uint(scale) >> 23) & 0xffu) * 0x01010101u;
+                                }
+#pragma unroll
+                                for (int t = 0; t < 16; t += 4) {
+                                    float x[4];
+#pragma unroll
+                                    for (int j = 0; j < 4; ++j) x[j] = h[t + j] * __shfl_sync(0xffffffffu, inv, t + j);
+                                    const uint32_t w = transpose_bytes_4x4(pack_e4m3x4(x[0], x[1], x[2], x[3]), lane);
+                                    const int tok = t0 + t + (lane & 3);
+                                    if (tok < tok_valid)
+                                        *reinterpret_cast<uint32_t*>(p.c_fp8 + (size_t)(ti.c_row + tok) * ldc + ti.c_col + q * 32 + (lane & ~3)) = w;
+                                }
+                            } else {
+#pragma unroll
+                                for (int hw = 0; hw < 2; ++hw)
+#pragma unroll
+                                    for (int t = 0; t < 16; t += 2) {
+                                        const uint32_t* a = hw == 0 ? v[c] : u[c];
+                                        const uint32_t w = f2_to_bf16x2(__uint_as_float(a[t]), __uint_as_float(a[t + 1]));
+                                        const uint32_t o = __shfl_xor_sync(0xffffffffu, w, 1);
+                                        const int tok = t0 + t + (lane & 1);
+                                        if (tok < tok_valid)
+                                            *reinterpret_cast<uint32_t*>(cbase + (size_t)(ti.c_row + tok) * ldc + ti.c_col + hw * kBlockM + q * 32 + (lane & ~1)) =
+                                                __byte_perm(w, o, (lane & 1) ? 0x3276 : 0x5410);
+                                    }
+                            }
+                        }
+                    }
+                    if (!ok) break;
+                    win_phase ^= 1;
+                    continue;
+                } else if constexpr (kSwiGLU && C::kWindows == 1) {
                     // Single window, two warps per lane quarter: this warp takes 64 of the tile's 128 output columns. Their gate
                     // and up accumulators go to registers raw, the window returns to the MMA issuer right away, and the
                     // arithmetic and the stores run while the next tile accumulates.
@@ -1330,7 +1462,7 @@ bool make_map_sf(CUtensorMap* map, const void* ptr, uint64_t rows, uint32_t word
     return r == CUDA_SUCCESS;
 }
 
-template <int kBlockN, bool kFp8, bool kSwiGLU, bool kPair, bool kMx = false, bool kRowScatter = false>
+template <int kBlockN, bool kFp8, bool kSwiGLU, bool kPair, bool kMx = false, bool kRowScatter = false, bool kSwap = false>
 cudaError_t launch_impl(const GroupedGemmArgs& a, cudaStream_t stream) {
     using C = Cfg<kBlockN, kFp8, kSwiGLU, kPair, kMx, kRowScatter>;
     CUtensorMap map_a, map_b, map_sfa, map_sfb;
@@ -1358,7 +1490,7 @@ cudaError_t launch_impl(const GroupedGemmArgs& a, cudaStream_t stream) {
                      : make_map(&map_b, a.b, kFp8, (uint64_t)a.k, (uint64_t)a.m_total, b_box_rows));
     }
     if (!ok) return cudaErrorInvalidValue;
-    auto kernel = grouped_gemm_kernel<kBlockN, kFp8, kSwiGLU, kPair, kMx, kRowScatter>;
+    auto kernel = grouped_gemm_kernel<kBlockN, kFp8, kSwiGLU, kPair, kMx, kRowScatter, kSwap>;
     static bool smem_opted_in[64] = {};  // per device, once: the attribute is sticky
     int dev = 0;
     cudaGetDevice(&dev);
@@ -1414,9 +1546,11 @@ cudaError_t launch_grouped_gemm(const GroupedGemmArgs& a, cudaStream_t stream) {
             if (a.swiglu) {
                 if ((a.n / 2) % 128 != 0) return cudaErrorInvalidValue;  // gate/up halves start on scale-block boundaries
                 if (a.mx_wide && a.cta_pairs) return launch_impl<256, true, true, true, true>(a, stream);
+                if (a.mx_wide && a.swap) return launch_impl<256, true, true, false, true, false, true>(a, stream);
                 if (a.mx_wide) return launch_impl<256, true, true, false, true>(a, stream);
                 return launch_impl<128, true, true, false, true>(a, stream);
             }
+            if (a.mx_wide && a.swap && a.n % 256 == 0) return launch_impl<256, true, false, false, true, false, true>(a, stream);
             if (a.mx_wide) return (a.n % 256 == 0) ? launch_impl<256, true, false, false, true>(a, stream) : cudaErrorInvalidValue;
             if (a.row_info != nullptr) return launch_impl<128, true, false, false, true, true>(a, stream);
             return launch_impl<128, true, false, false, true>(a, stream);

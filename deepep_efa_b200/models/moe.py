@@ -291,14 +291,15 @@ class MoELayer(nn.Module):
             ws[key] = w_
         w_ = ws[key]
         a, a_s = px.view(L * N, H), ps.view(L * N, H // 128)
+        few_rows = R * x.size(0) * cfg.num_topk <= TOKEN_COLUMNS_MAX_ROWS * cfg.num_experts
         y = buf.get_next_low_latency_combine_buffer(handle)
         # rows per expert come as counts; both GEMMs read them where the dispatch left them
         if mx is not None:
             # GEMM1's epilogue quantises its own output (a wide tile holds one whole scale block of a row): e4m3 + scale atoms
             C.grouped_gemm(a, w13, w_["starts"], 0, True, None, None, None, 0, GEMM_TIMEOUT_MS, cnt, gg.build_sf_atoms_a(a_s), mx[0],
-                           out_fp8=w_["hq"], out_atoms=w_["ha"], m_ends_are_counts=True, sched=w_["sched"], early_table=True)
+                           out_fp8=w_["hq"], out_atoms=w_["ha"], m_ends_are_counts=True, sched=w_["sched"], early_table=True, tokens_as_columns=few_rows)
             C.grouped_gemm(w_["hq"], w2, w_["starts"], 0, False, None, None, y.view(L * N, H), 0, GEMM_TIMEOUT_MS, cnt, w_["ha"], mx[3],
-                           m_ends_are_counts=True, sched=w_["sched"], early_table=True)
+                           m_ends_are_counts=True, sched=w_["sched"], early_table=True, tokens_as_columns=few_rows)
         else:
             C.grouped_gemm(a, w13, w_["starts"], 0, True, a_s, s13, w_["h"], 0, GEMM_TIMEOUT_MS, cnt, m_ends_are_counts=True, sched=w_["sched"])
             C.per_token_cast_to_fp8(w_["h"], False, False, cnt, N, w_["hq"], w_["hs"])
@@ -316,6 +317,10 @@ UNIT_ROWS = 8  # rows of one expert a dispatch warp sends between two arrival-co
 # the register file, and next to the natively block-scaled kernel the dispatch was measured several times slower than on
 # SMs of its own. A GEMM that got every SM before the dispatch CTAs were placed would wait for rows that nobody can send.
 FUSE_CAST_INTO_GEMM1 = True  # wide natively block-scaled tiles: GEMM1's epilogue emits e4m3 + scale atoms itself
+# Decode, natively block-scaled: average rows per expert up to which the GEMMs take the tokens as columns (a tile then multiplies 32 of
+# them at a time instead of 128 rows). One step back to back, rows / columns, us: 64 experts with 12 rows 251 / 226, 16 rows 252 / 227;
+# 32 experts with 24 rows 152 / 149, 32 rows 152 / 162; 16 experts with 64 rows 119 / 144.
+TOKEN_COLUMNS_MAX_ROWS = 20
 # Natively block-scaled GEMMs: average rows per expert from which the 128x256 tiles are used instead of the 128x128 ones. Since the
 # wide tiles drain their accumulator in two halves they win from the smallest sizes measured on (8 experts x 4096 rows down to 256
 # experts x 128 rows: +22 % to +54 %); below one tile of rows per expert the narrow tiles stay (fewer wasted columns per padded tile).

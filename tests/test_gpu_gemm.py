@@ -292,16 +292,47 @@ def test_partial_tiles_and_drawn_tiles(kind):
     a.view(torch.uint8)[~live] = 0xFF  # NaN in both types
     outs = []
     for sched in (None, torch.zeros(2, dtype=torch.int32, device="cuda")):
-        for sms in (0, 2):
+        for sms, columns in ((0, False), (2, False), (0, True), (2, True)):
             out = torch.full((G * stride, N // 2 if swiglu else N), 7.0, device="cuda", dtype=torch.bfloat16)
             scales = (None, None) if sfa is not None else (a_s, b_s)
-            C.grouped_gemm(a, b, starts, 0, swiglu, *scales, out, sms, 2000.0, cnt, sfa, sfb, m_ends_are_counts=True, sched=sched)
+            C.grouped_gemm(a, b, starts, 0, swiglu, *scales, out, sms, 2000.0, cnt, sfa, sfb, m_ends_are_counts=True, sched=sched, tokens_as_columns=columns)
             outs.append(out)
     torch.cuda.synchronize()
     assert C.gemm_error(0) == 0 and sched.tolist() == [0, 0]
     assert _rel_err(outs[0][live], ref[live]) < (1.5e-2 if swiglu else 1e-2)
     assert (outs[0][~live] == 7.0).all()
     assert all(torch.equal(o, outs[0]) for o in outs)
+
+
+def test_quantised_output_with_tokens_as_columns():
+    """The kernel that takes the weights as M quantises like the row-wise one, bit for bit."""
+    from deepep_efa_b200 import _ext
+    from deepep_efa_b200.ops.grouped_gemm import build_sf_atoms_a, build_sf_atoms_b
+    C = _ext.load()
+    C.gemm_clear_error(0)
+    torch.manual_seed(19)
+    counts, stride, K, I = [1, 15, 16, 17, 31, 32, 33, 0, 64, 65, 96, 97, 128, 129, 256, 200], 256, 384, 384
+    G = len(counts)
+    cnt = torch.tensor(counts, device="cuda", dtype=torch.int32)
+    starts = torch.arange(G + 1, device="cuda", dtype=torch.int32) * stride
+    live = (torch.arange(stride, device="cuda").unsqueeze(0) < cnt.unsqueeze(1)).view(-1)
+    x = torch.randn(G * stride, K, device="cuda").to(torch.bfloat16)
+    x[starts[4]:starts[5]] = 0  # a group whose maxima are all zero
+    a, a_s = C.per_token_cast_to_fp8(x, True, False)
+    b = torch.randn(G, 2 * I, K, device="cuda").to(torch.float8_e4m3fn)
+    b_s = torch.exp2(torch.randint(-8, -4, (G, 2 * I // 128, K // 128), device="cuda").float())
+    sfa, sfb = build_sf_atoms_a(a_s), build_sf_atoms_b(b_s, 2 * I, True, True)
+    got = []
+    for columns in (True, False):
+        q = torch.zeros(G * stride, I, dtype=torch.uint8, device="cuda")
+        atoms = torch.zeros(G * stride // 128, I // 128, 512, dtype=torch.uint8, device="cuda")
+        C.grouped_gemm(a, b, starts, 0, True, None, None, None, 0, 2000.0, cnt, sfa, sfb, out_fp8=q.view(torch.float8_e4m3fn), out_atoms=atoms,
+                       m_ends_are_counts=True, tokens_as_columns=columns)
+        got.append((q, atoms))
+    torch.cuda.synchronize()
+    assert C.gemm_error(0) == 0
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+    assert (got[0][0][~live] == 0).all() and got[0][0][live].any()
 
 
 @pytest.mark.parametrize("pair", ["0", "1"])
