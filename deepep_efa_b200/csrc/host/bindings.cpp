@@ -7,6 +7,7 @@
 // Reference counterpart: the pybind module at csrc/deep_ep.cpp:4310-4479 and the host halves of
 // get_dispatch_layout / intranode_dispatch / intranode_combine (csrc/deep_ep.cpp:517-1035).
 #include <ATen/cuda/CUDAContext.h>
+#include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <pybind11/functional.h>
@@ -132,6 +133,13 @@ void check_launch(cudaError_t e, const char* what) {
         cudaGetLastError();
         throw std::runtime_error(std::string(what) + ": launch failed: " + cudaGetErrorString(e));
     }
+}
+
+// Counts, membership and handles come from earlier calls, each allocated on the stream that call ran on. A call that reads them on
+// another stream marks them there, so that their memory is not handed out again before its kernels have run, whoever drops them and
+// when. On the stream they came from this does nothing.
+void used_here(const torch::Tensor& t) {
+    if (t.is_cuda()) c10::cuda::CUDACachingAllocator::recordStream(t.storage().data_ptr(), c10::cuda::getCurrentCUDAStream(t.get_device()));
 }
 
 // One normal-mode call on the current stream, ordered behind the runtime's previous one (RuntimeCore::order_enter).
@@ -275,6 +283,8 @@ py::list normal_dispatch(std::vector<Runtime*> rts, const std::vector<py::tuple>
             q.send_head = h[5].cast<torch::Tensor>();
             DX_CHECK(q.send_head.scalar_type() == torch::kInt32 && q.send_head.is_contiguous() && q.send_head.dim() == 2 && q.send_head.size(0) == T && q.send_head.size(1) == R, "send_head must be int32 [T,R]");
             DX_CHECK(q.rpm.scalar_type() == torch::kInt32 && q.rpm.is_contiguous() && q.rpm.numel() == R * R, "rank_prefix_matrix must be int32 [R,R]");
+            used_here(q.rpm);
+            used_here(q.send_head);
             continue;
         }
         auto ntpr = t[2].cast<torch::Tensor>(), ntpe = t[3].cast<torch::Tensor>();
@@ -285,6 +295,9 @@ py::list normal_dispatch(std::vector<Runtime*> rts, const std::vector<py::tuple>
         DX_CHECK(q.in_rank.size(0) == T, "is_token_in_rank must have one row per token of x");
         E = (int)ntpe.numel();
         DX_CHECK(E / R <= dx::kMaxLocalExperts, "too many local experts");
+        used_here(ntpr);
+        used_here(ntpe);
+        used_here(q.in_rank);
         auto i32 = torch::TensorOptions().dtype(torch::kInt32).device(q.in_rank.device());
         q.rpm = torch::empty({R, R}, i32);
         q.cpm = torch::empty({R, num_channels}, i32);
@@ -406,6 +419,8 @@ py::list normal_combine(std::vector<Runtime*> rts, const std::vector<py::tuple>&
         const int H = (int)x.size(1), T = (int)send_head.size(0);
         DX_CHECK(H % 8 == 0, "hidden must be a multiple of 8");
         DX_CHECK(send_head.scalar_type() == torch::kInt32 && send_head.is_contiguous() && send_head.size(1) == R, "send_head must be int32 [T,R]");
+        used_here(send_head);
+        used_here(rpm);
         // What the peers read must lie in symmetric memory; anything else is staged there. A lone rank reads its own tensor where
         // it is (an offset that leaves the buffer, which the debug range check would refuse).
         auto place = [&](const torch::Tensor& given) -> uint64_t {
