@@ -142,14 +142,21 @@ void used_here(const torch::Tensor& t) {
     if (t.is_cuda()) c10::cuda::CUDACachingAllocator::recordStream(t.storage().data_ptr(), c10::cuda::getCurrentCUDAStream(t.get_device()));
 }
 
-// One normal-mode call on the current stream, ordered behind the runtime's previous one (RuntimeCore::order_enter).
+// The launches of a normal-mode call on the current stream, ordered behind the previous call's (RuntimeCore::order_enter).
 struct OrderedCall {
     RuntimeCore* core;
     cudaStream_t stream;
-    bool counted;
-    explicit OrderedCall(Runtime* rt) : core(rt->core.get()), stream(cur_stream(rt)), counted(core->order_enter(stream)) {}
-    ~OrderedCall() {
-        if (counted) core->order_leave(stream);
+    bool inside = false;
+    explicit OrderedCall(Runtime* rt) : core(rt->core.get()), stream(cur_stream(rt)) {}
+    OrderedCall(const OrderedCall&) = delete;
+    ~OrderedCall() { leave(); }
+    void enter() {
+        if (!inside) core->order_enter(stream);
+        inside = true;
+    }
+    void leave() {
+        if (inside) core->order_leave(stream);
+        inside = false;
     }
 };
 
@@ -178,6 +185,7 @@ std::tuple<torch::Tensor, torch::Tensor, torch::Tensor> get_dispatch_layout(Runt
     a.is_token_in_rank = in_rank.data_ptr<bool>();
     a.scratch = rt->layout_scratch.data_ptr<int>();
     OrderedCall order(rt);
+    order.enter();
     check_launch(dx::launch_layout(a, order.stream), "get_dispatch_layout");
     return {per_rank, per_expert, in_rank};
 }
@@ -216,6 +224,7 @@ struct DispatchCall {
     }
 };
 
+// Lets other host threads run: the caller has left its OrderedCall.
 void wait_counts(Runtime* rt, DispatchCall& q, int num_local_experts) {
     py::gil_scoped_release rel;
     q.num_recv = rt->core->wait_recv_counts(num_local_experts, &q.per_expert);
@@ -321,7 +330,10 @@ py::list normal_dispatch(std::vector<Runtime*> rts, const std::vector<py::tuple>
         a.host_recv_counter = &hw->recv_counter;
         a.host_expert_counter = hw->expert_counter;
     }
-    if (!cached) check_launch(dx::launch_notify(nargs.data(), V, order.stream), "notify");
+    if (!cached) {
+        order.enter();
+        check_launch(dx::launch_notify(nargs.data(), V, order.stream), "notify");
+    }
 
     // How many rows arrive is known on the host only when the count exchange has run, except that a lone rank receives at most
     // its own tokens: its outputs are sized for them, the dispatch kernel is queued at once and the host waits beside it.
@@ -340,6 +352,7 @@ py::list normal_dispatch(std::vector<Runtime*> rts, const std::vector<py::tuple>
             if (q.meta) continue;
         }
         if (exact) {
+            order.leave();
             wait_counts(rts[v], q, E / R);
             rows = q.num_recv;
             waited = true;
@@ -372,7 +385,9 @@ py::list normal_dispatch(std::vector<Runtime*> rts, const std::vector<py::tuple>
         a.recv_src_idx_off = q.meta->off + q.src_idx_at;
         a.num_worst_tokens = num_worst_tokens;
     }
+    order.enter();
     check_launch(dx::launch_dispatch(dargs.data(), V, order.stream), "dispatch");
+    order.leave();
 
     py::list out;
     for (int v = 0; v < V; ++v) {
@@ -468,6 +483,7 @@ py::list normal_combine(std::vector<Runtime*> rts, const std::vector<py::tuple>&
         a.num_sms = num_sms;
         results.append(py::make_tuple(out, out_w));
     }
+    order.enter();
     check_launch(dx::launch_combine(args.data(), V, order.stream), "combine");
     return results;
 }

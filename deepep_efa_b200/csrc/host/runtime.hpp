@@ -160,8 +160,10 @@ class RuntimeCore {
         drain_pending(true);
         for (cudaEvent_t ev : event_pool_) cudaEventDestroy(ev);
         event_pool_.clear();
-        if (order_event_ != nullptr) cudaEventDestroy(order_event_);
-        order_event_ = nullptr;
+        for (Order* o : {&order_, &capture_order_}) {
+            if (o->event != nullptr) cudaEventDestroy(o->event);
+            *o = Order{};
+        }
         for (int r = 0; r < num_ranks_; ++r)
             if (ipc_opened_[r]) cudaIpcCloseMemHandle(peers_[r]);
         if (base_) cudaFree(base_);
@@ -240,21 +242,25 @@ class RuntimeCore {
     // ---- order of the normal-mode kernels -----------------------------------------------------
     // They share state (sequence numbers, tickets, the layout scratch), so one must not overlap the next one. A call runs on the
     // caller's stream, or on the communication stream when the caller asked for an event; a call on another stream than the
-    // last one waits for that one's event first. A stream under capture takes no part: an event from outside may not be waited
-    // for there, and the graph's owner orders its replays.
-    bool order_enter(cudaStream_t s) {
-        cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-        if (cudaStreamIsCapturing(s, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone) {
-            cudaGetLastError();
-            return false;
-        }
-        if (order_event_ != nullptr && order_stream_ != s) DX_CUDA_CHECK(cudaStreamWaitEvent(s, order_event_, 0));
-        return true;
+    // last one waits for that one's event first. Enter before the first launch of a call and leave after the last one, with
+    // nothing in between that lets another host thread in (a wait for the GPU): a call that waits leaves before it does.
+    // Calls under stream capture are ordered among those of the same capture. With calls outside of it they are not: an event
+    // from outside may not be waited for there, and the graph's owner orders its replays.
+    void order_enter(cudaStream_t s) {
+        std::lock_guard<std::mutex> g(mu_);
+        unsigned long long id = 0;
+        Order* o = order_of(s, &id);
+        if (o != nullptr && o->event != nullptr && o->capture == id && o->stream != s) DX_CUDA_CHECK(cudaStreamWaitEvent(s, o->event, 0));
     }
     void order_leave(cudaStream_t s) {
-        if (order_event_ == nullptr && cudaEventCreateWithFlags(&order_event_, cudaEventDisableTiming) != cudaSuccess) order_event_ = nullptr;
-        if (order_event_ != nullptr) cudaEventRecord(order_event_, s);
-        order_stream_ = s;
+        std::lock_guard<std::mutex> g(mu_);
+        unsigned long long id = 0;
+        Order* o = order_of(s, &id);
+        if (o == nullptr) return;
+        if (o->event == nullptr && cudaEventCreateWithFlags(&o->event, cudaEventDisableTiming) != cudaSuccess) o->event = nullptr;
+        if (o->event != nullptr) cudaEventRecord(o->event, s);
+        o->stream = s;
+        o->capture = id;
         cudaGetLastError();
     }
 
@@ -366,6 +372,23 @@ class RuntimeCore {
         int num_events = 0;
     };
 
+    struct Order {
+        cudaEvent_t event = nullptr;  // end of the last call, recorded on `stream`
+        cudaStream_t stream = nullptr;
+        unsigned long long capture = 0;  // the capture it belongs to, 0 = none
+    };
+    // What a call on `s` is ordered by; nullptr when the driver will not say (the default stream while another stream captures).
+    Order* order_of(cudaStream_t s, unsigned long long* capture) {
+        cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+        if (cudaStreamGetCaptureInfo(s, &st, capture) != cudaSuccess || st == cudaStreamCaptureStatusInvalidated) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        if (st == cudaStreamCaptureStatusActive) return &capture_order_;
+        *capture = 0;
+        return &order_;
+    }
+
     cudaEvent_t take_event() {
         cudaEvent_t ev = nullptr;
         if (!event_pool_.empty()) {
@@ -420,8 +443,7 @@ class RuntimeCore {
     Arena arena_;
     std::deque<Pending> pending_;
     std::vector<cudaEvent_t> event_pool_;  // bounded by the number of blocks that were ever pending at once
-    cudaEvent_t order_event_ = nullptr;    // end of the last normal-mode call, recorded on order_stream_
-    cudaStream_t order_stream_ = nullptr;
+    Order order_, capture_order_;
     std::mutex mu_;
 };
 

@@ -100,3 +100,65 @@ def test_handle_of_an_asynchronous_call_used_and_dropped_elsewhere():
             del keep
     finally:
         vc.destroy()
+
+
+def test_call_of_another_thread_during_the_wait_for_the_counts():
+    """A dispatch waits on the host for its receive counts and lets other threads run; what they launch on another stream comes
+    after what the dispatch has launched."""
+    import threading
+    import time
+    vc, buf = _buffer()
+    try:
+        idx, _ = make_routing(T, E, K, "cuda", seed=3)
+        x = make_tokens(T, H, "cuda", seed=3)
+        lay, _ = _layout(buf, idx)
+        y, _, _, want_counts, handle, _ = buf.dispatch(x, **lay)
+        want = buf.combine(y, handle)[0].clone()
+        first, second = torch.cuda.Stream(), torch.cuda.Stream()
+        torch.cuda.synchronize()
+        with torch.cuda.stream(first):
+            torch.cuda._sleep(8 * DELAY)
+        started, got = threading.Event(), []
+
+        def waiter():
+            with torch.cuda.stream(first):
+                started.set()
+                got.append(buf.dispatch(x, **lay))
+
+        thread = threading.Thread(target=waiter)
+        thread.start()
+        started.wait()
+        time.sleep(0.05)  # the other thread is waiting for its counts by now
+        with torch.cuda.stream(second):
+            out, _, _ = buf.combine(y, handle)
+        early = second.query()
+        thread.join()
+        torch.cuda.synchronize()
+        buf.check_status()
+        assert not early
+        assert torch.equal(out, want) and got[0][3] == want_counts and torch.equal(got[0][0], x)
+    finally:
+        vc.destroy()
+
+
+def test_calls_of_one_capture_on_two_streams():
+    """Inside one capture, a layout on the communication stream and one on the capturing stream share the scratch: they come one
+    after the other although nothing else orders them."""
+    vc, buf = _buffer()
+    try:
+        n = 5000  # several CTAs, so that the scratch is used
+        idx = [make_routing(n, E, K, "cuda", seed=4 + i, masked_fraction=0.1 * i)[0] for i in range(2)]
+        want = [[t.clone() for t in (lay["num_tokens_per_expert"], lay["is_token_in_rank"])] for lay in (_layout(buf, i)[0] for i in idx)]
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            first, ev = _layout(buf, idx[0], async_finish=True)
+            second, _ = _layout(buf, idx[1])
+            ev.current_stream_wait()
+        for _ in range(20):
+            graph.replay()
+            torch.cuda.synchronize()
+            for lay, w in zip((first, second), want):
+                assert torch.equal(lay["num_tokens_per_expert"], w[0]) and torch.equal(lay["is_token_in_rank"], w[1])
+    finally:
+        vc.destroy()
