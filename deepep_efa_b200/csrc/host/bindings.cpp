@@ -142,20 +142,23 @@ void used_here(const torch::Tensor& t) {
     if (t.is_cuda()) c10::cuda::CUDACachingAllocator::recordStream(t.storage().data_ptr(), c10::cuda::getCurrentCUDAStream(t.get_device()));
 }
 
-// The launches of a normal-mode call on the current stream, ordered behind the previous call's (RuntimeCore::order_enter).
+// The launches of a normal-mode call on the current stream, ordered behind the previous call's (RuntimeCore::order_enter) of every
+// rank that takes part.
 struct OrderedCall {
-    RuntimeCore* core;
+    std::vector<Runtime*> rts;
     cudaStream_t stream;
     bool inside = false;
-    explicit OrderedCall(Runtime* rt) : core(rt->core.get()), stream(cur_stream(rt)) {}
+    explicit OrderedCall(std::vector<Runtime*> r) : rts(std::move(r)), stream(cur_stream(rts[0])) {}
     OrderedCall(const OrderedCall&) = delete;
     ~OrderedCall() { leave(); }
     void enter() {
-        if (!inside) core->order_enter(stream);
+        if (inside) return;
+        for (Runtime* rt : rts) rt->core->order_enter(stream);
         inside = true;
     }
     void leave() {
-        if (inside) core->order_leave(stream);
+        if (!inside) return;
+        for (Runtime* rt : rts) rt->core->order_leave(stream);
         inside = false;
     }
 };
@@ -184,7 +187,7 @@ std::tuple<torch::Tensor, torch::Tensor, torch::Tensor> get_dispatch_layout(Runt
     a.num_tokens_per_expert = per_expert.data_ptr<int>();
     a.is_token_in_rank = in_rank.data_ptr<bool>();
     a.scratch = rt->layout_scratch.data_ptr<int>();
-    OrderedCall order(rt);
+    OrderedCall order({rt});
     order.enter();
     check_launch(dx::launch_layout(a, order.stream), "get_dispatch_layout");
     return {per_rank, per_expert, in_rank};
@@ -242,7 +245,7 @@ py::list normal_dispatch(std::vector<Runtime*> rts, const std::vector<py::tuple>
     std::vector<DispatchCall> calls(V);
     std::vector<dx::NotifyArgs> nargs(V);
     std::vector<dx::DispatchArgs> dargs(V);
-    OrderedCall order(rts[0]);
+    OrderedCall order(rts);
     bool cached = false;
     int E = R;  // a cached call carries no expert ids to remap
     for (int v = 0; v < V; ++v) {
@@ -417,7 +420,7 @@ py::list normal_combine(std::vector<Runtime*> rts, const std::vector<py::tuple>&
     std::vector<dx::CombineArgs> args(V);
     std::vector<torch::Tensor> keep;
     py::list results;
-    OrderedCall order(rts[0]);
+    OrderedCall order(rts);
     for (int v = 0; v < V; ++v) {
         Runtime* rt = rts[v];
         const py::tuple& t = per_rank[v];

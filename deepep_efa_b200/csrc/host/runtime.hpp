@@ -160,10 +160,7 @@ class RuntimeCore {
         drain_pending(true);
         for (cudaEvent_t ev : event_pool_) cudaEventDestroy(ev);
         event_pool_.clear();
-        for (Order* o : {&order_, &capture_order_}) {
-            if (o->event != nullptr) cudaEventDestroy(o->event);
-            *o = Order{};
-        }
+        order_ = capture_order_ = Order{};
         for (int r = 0; r < num_ranks_; ++r)
             if (ipc_opened_[r]) cudaIpcCloseMemHandle(peers_[r]);
         if (base_) cudaFree(base_);
@@ -217,8 +214,9 @@ class RuntimeCore {
     }
 
     // Called when the last tensor of a block dies (any thread). `streams` (up to two, nullptr = the default stream) are the
-    // streams whose queued work may still use the block. Events come from a pool: creating and destroying them cost more than
-    // everything else here.
+    // streams whose queued work may still use the block. So may the normal-mode calls, on whatever stream they ran: the last of
+    // them is behind all others, so when it was on neither of these streams its event is waited for as well. Events come from a
+    // pool: creating and destroying them cost more than everything else here.
     void arena_release(uint64_t off, const cudaStream_t* streams, int num_streams) {
         std::lock_guard<std::mutex> g(mu_);
         if (released_) return;
@@ -227,13 +225,19 @@ class RuntimeCore {
         int prev = -1;
         cudaGetDevice(&prev);
         if (prev != device_) cudaSetDevice(device_);
+        bool covered = order_.event == nullptr;
         for (int i = 0; i < num_streams; ++i) {
             if (i == 1 && streams[1] == streams[0]) break;
             cudaEvent_t ev = take_event();
             if (ev == nullptr) continue;
-            if (cudaEventRecord(ev, streams[i]) == cudaSuccess) p.events[p.num_events++] = ev;
-            else event_pool_.push_back(ev);
+            if (cudaEventRecord(ev, streams[i]) == cudaSuccess) {
+                p.events[p.num_events++] = ev;
+                covered = covered || streams[i] == order_.stream;
+            } else {
+                event_pool_.push_back(ev);
+            }
         }
+        if (!covered) p.last_call = order_.event;
         cudaGetLastError();
         if (prev != device_ && prev >= 0) cudaSetDevice(prev);
         pending_.push_back(p);
@@ -250,15 +254,18 @@ class RuntimeCore {
         std::lock_guard<std::mutex> g(mu_);
         unsigned long long id = 0;
         Order* o = order_of(s, &id);
-        if (o != nullptr && o->event != nullptr && o->capture == id && o->stream != s) DX_CUDA_CHECK(cudaStreamWaitEvent(s, o->event, 0));
+        if (o != nullptr && o->event != nullptr && o->capture == id && o->stream != s) DX_CUDA_CHECK(cudaStreamWaitEvent(s, *o->event, 0));
     }
     void order_leave(cudaStream_t s) {
         std::lock_guard<std::mutex> g(mu_);
         unsigned long long id = 0;
         Order* o = order_of(s, &id);
         if (o == nullptr) return;
-        if (o->event == nullptr && cudaEventCreateWithFlags(&o->event, cudaEventDisableTiming) != cudaSuccess) o->event = nullptr;
-        if (o->event != nullptr) cudaEventRecord(o->event, s);
+        if (o->event == nullptr || o->event.use_count() > 1) {  // a block released meanwhile waits for that call, not for this one
+            auto fresh = std::make_shared<OwnedEvent>();
+            o->event = fresh->ev != nullptr ? std::shared_ptr<cudaEvent_t>(fresh, &fresh->ev) : nullptr;
+        }
+        if (o->event != nullptr) cudaEventRecord(*o->event, s);
         o->stream = s;
         o->capture = id;
         cudaGetLastError();
@@ -370,10 +377,21 @@ class RuntimeCore {
         uint64_t off = 0;
         cudaEvent_t events[2];
         int num_events = 0;
+        std::shared_ptr<cudaEvent_t> last_call;  // of the normal-mode calls, where the events do not cover it
     };
 
+    struct OwnedEvent {
+        cudaEvent_t ev = nullptr;
+        OwnedEvent() {
+            if (cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess) ev = nullptr;
+        }
+        OwnedEvent(const OwnedEvent&) = delete;
+        ~OwnedEvent() {
+            if (ev != nullptr) cudaEventDestroy(ev);
+        }
+    };
     struct Order {
-        cudaEvent_t event = nullptr;  // end of the last call, recorded on `stream`
+        std::shared_ptr<cudaEvent_t> event;  // end of the last call, recorded on `stream`
         cudaStream_t stream = nullptr;
         unsigned long long capture = 0;  // the capture it belongs to, 0 = none
     };
@@ -402,14 +420,9 @@ class RuntimeCore {
 
     void drain_pending(bool wait) {
         for (auto it = pending_.begin(); it != pending_.end();) {
-            bool done = true;
-            for (int i = 0; i < it->num_events; ++i) {
-                cudaError_t e = wait ? cudaEventSynchronize(it->events[i]) : cudaEventQuery(it->events[i]);
-                if (e == cudaErrorNotReady) {
-                    done = false;
-                    break;
-                }
-            }
+            auto passed = [&](cudaEvent_t ev) { return (wait ? cudaEventSynchronize(ev) : cudaEventQuery(ev)) != cudaErrorNotReady; };
+            bool done = it->last_call == nullptr || passed(*it->last_call);
+            for (int i = 0; done && i < it->num_events; ++i) done = passed(it->events[i]);
             if (done) {
                 for (int i = 0; i < it->num_events; ++i) event_pool_.push_back(it->events[i]);
                 arena_.free(it->off);

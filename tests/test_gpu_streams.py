@@ -162,3 +162,43 @@ def test_calls_of_one_capture_on_two_streams():
                 assert torch.equal(lay["num_tokens_per_expert"], w[0]) and torch.equal(lay["is_token_in_rank"], w[1])
     finally:
         vc.destroy()
+
+
+@pytest.mark.parametrize("call", ["dispatch", "combine"])
+def test_symmetric_memory_dropped_under_another_stream(call):
+    """A direct call still has to write (dispatch) or read (combine) symmetric memory on its stream when the last tensor in it dies
+    under another one: what is allocated next must lie elsewhere, or come after the call."""
+    vc, buf = _buffer(nvl=64 << 20)
+    try:
+        idx, _ = make_routing(T, E, K, "cuda", seed=5)
+        x = make_tokens(T, H, "cuda", seed=5)
+        lay, _ = _layout(buf, idx)
+        y, _, _, _, handle, _ = buf.dispatch(x, **lay)
+        want = buf.combine(y, handle)[0].clone()
+        side = torch.cuda.Stream()
+        torch.cuda.synchronize()
+        _delay(side)
+        with torch.cuda.stream(side):
+            if call == "dispatch":
+                late = buf.dispatch(x, handle=handle)[0]
+            else:
+                late = buf.empty_symmetric([T, H], torch.bfloat16)
+                late.copy_(y)
+                out = buf.combine(late, handle)[0]
+        late_at = late.data_ptr()
+        del late
+        fresh = [buf.empty_symmetric([T, H], torch.bfloat16) for _ in range(4)]
+        for f in fresh:
+            f.fill_(3.0)
+        assert late_at not in [f.data_ptr() for f in fresh]
+        torch.cuda.synchronize()
+        buf.check_status()
+        assert all(bool((f == 3.0).all()) for f in fresh)
+        if call == "combine":
+            assert torch.equal(out, want)
+        # the memory comes back once the call is over
+        del fresh
+        again = [buf.empty_symmetric([T, H], torch.bfloat16) for _ in range(8)]
+        assert late_at in [f.data_ptr() for f in again]
+    finally:
+        vc.destroy()
