@@ -175,8 +175,13 @@ std::tuple<torch::Tensor, torch::Tensor, torch::Tensor> get_dispatch_layout(Runt
     auto i32 = torch::TensorOptions().dtype(torch::kInt32).device(topk_idx.device());
     auto per_rank = torch::empty({R}, i32), per_expert = torch::empty({num_experts}, i32);
     auto in_rank = torch::empty({T, R}, i32.dtype(torch::kBool));
+    // The scratch belongs to whichever call runs: it is replaced only behind the previous one, and marked on the stream that uses it,
+    // so that an outgrown one is not handed out while a call on another stream is still to use it.
+    OrderedCall order({rt});
+    order.enter();
     const int64_t need = (int64_t)dx::layout_scratch_ints(num_experts, R, T);
     if (!rt->layout_scratch.defined() || rt->layout_scratch.numel() < need) rt->layout_scratch = torch::zeros({need}, i32);
+    used_here(rt->layout_scratch);
     dx::LayoutArgs a{};
     a.topk_idx = topk_idx.data_ptr<int64_t>();
     a.num_tokens = T;
@@ -187,8 +192,6 @@ std::tuple<torch::Tensor, torch::Tensor, torch::Tensor> get_dispatch_layout(Runt
     a.num_tokens_per_expert = per_expert.data_ptr<int>();
     a.is_token_in_rank = in_rank.data_ptr<bool>();
     a.scratch = rt->layout_scratch.data_ptr<int>();
-    OrderedCall order({rt});
-    order.enter();
     check_launch(dx::launch_layout(a, order.stream), "get_dispatch_layout");
     return {per_rank, per_expert, in_rank};
 }

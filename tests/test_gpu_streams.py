@@ -202,3 +202,34 @@ def test_symmetric_memory_dropped_under_another_stream(call):
         assert late_at in [f.data_ptr() for f in again]
     finally:
         vc.destroy()
+
+
+def test_layout_scratch_outgrown_while_another_stream_uses_it():
+    """Layouts of growing size on the caller's, the delayed communication and a third stream: each call has the scratch to itself, and
+    what is allocated in between does not get the outgrown one too early."""
+    vc, buf = _buffer()
+    try:
+        sizes = [2500, 2500, 5000, 9000, 9000, 20000]
+        idx = [make_routing(n, E, K, "cuda", seed=6 + i)[0] for i, n in enumerate(sizes)]
+        want = [torch.bincount(i.flatten(), minlength=E) for i in idx]
+        torch.cuda.synchronize()
+        side, got, keep = torch.cuda.Stream(), [], []
+        for i, n in enumerate(sizes):
+            if i % 3 == 1:
+                _delay(buf.comm_stream)
+                lay, ev = _layout(buf, idx[i], async_finish=True)
+                got.append(lay["num_tokens_per_expert"])
+                keep.append(ev)
+            else:
+                with torch.cuda.stream(side if i % 3 == 2 else torch.cuda.current_stream()):
+                    got.append(_layout(buf, idx[i])[0]["num_tokens_per_expert"])
+            for stream in (torch.cuda.current_stream(), side, buf.comm_stream):
+                with torch.cuda.stream(stream):
+                    keep.append([torch.full((m,), 7, dtype=torch.int32, device="cuda") for m in (250, 500, 1000, 2000)])
+        torch.cuda.synchronize()
+        for g, w in zip(got, want):
+            assert torch.equal(g.long(), w)
+        for k in keep:
+            assert not isinstance(k, list) or all(bool((t == 7).all()) for t in k)
+    finally:
+        vc.destroy()
