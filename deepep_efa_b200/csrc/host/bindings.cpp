@@ -142,26 +142,11 @@ void used_here(const torch::Tensor& t) {
     if (t.is_cuda()) c10::cuda::CUDACachingAllocator::recordStream(t.storage().data_ptr(), c10::cuda::getCurrentCUDAStream(t.get_device()));
 }
 
-// The launches of a normal-mode call on the current stream, ordered behind the previous call's (RuntimeCore::order_enter) of every
-// rank that takes part.
-struct OrderedCall {
-    std::vector<Runtime*> rts;
-    cudaStream_t stream;
-    bool inside = false;
-    explicit OrderedCall(std::vector<Runtime*> r) : rts(std::move(r)), stream(cur_stream(rts[0])) {}
-    OrderedCall(const OrderedCall&) = delete;
-    ~OrderedCall() { leave(); }
-    void enter() {
-        if (inside) return;
-        for (Runtime* rt : rts) rt->core->order_enter(stream);
-        inside = true;
-    }
-    void leave() {
-        if (!inside) return;
-        for (Runtime* rt : rts) rt->core->order_leave(stream);
-        inside = false;
-    }
-};
+dxh::OrderedCall ordered_call(const std::vector<Runtime*>& rts) {
+    std::vector<RuntimeCore*> cores;
+    for (Runtime* rt : rts) cores.push_back(rt->core.get());
+    return dxh::OrderedCall(std::move(cores), cur_stream(rts[0]));
+}
 
 // ---------------------------------------------------------------------------------------------
 // layout
@@ -177,7 +162,7 @@ std::tuple<torch::Tensor, torch::Tensor, torch::Tensor> get_dispatch_layout(Runt
     auto in_rank = torch::empty({T, R}, i32.dtype(torch::kBool));
     // The scratch belongs to whichever call runs: it is replaced only behind the previous one, and marked on the stream that uses it,
     // so that an outgrown one is not handed out while a call on another stream is still to use it.
-    OrderedCall order({rt});
+    dxh::OrderedCall order = ordered_call({rt});
     order.enter();
     const int64_t need = (int64_t)dx::layout_scratch_ints(num_experts, R, T);
     if (!rt->layout_scratch.defined() || rt->layout_scratch.numel() < need) rt->layout_scratch = torch::zeros({need}, i32);
@@ -248,7 +233,7 @@ py::list normal_dispatch(std::vector<Runtime*> rts, const std::vector<py::tuple>
     std::vector<DispatchCall> calls(V);
     std::vector<dx::NotifyArgs> nargs(V);
     std::vector<dx::DispatchArgs> dargs(V);
-    OrderedCall order(rts);
+    dxh::OrderedCall order = ordered_call(rts);
     bool cached = false;
     int E = R;  // a cached call carries no expert ids to remap
     for (int v = 0; v < V; ++v) {
@@ -423,7 +408,7 @@ py::list normal_combine(std::vector<Runtime*> rts, const std::vector<py::tuple>&
     std::vector<dx::CombineArgs> args(V);
     std::vector<torch::Tensor> keep;
     py::list results;
-    OrderedCall order(rts);
+    dxh::OrderedCall order = ordered_call(rts);
     for (int v = 0; v < V; ++v) {
         Runtime* rt = rts[v];
         const py::tuple& t = per_rank[v];

@@ -49,10 +49,12 @@ void em_notify(std::vector<py::object> rts, std::vector<py::tuple> per_rank, int
     const int V = (int)rts.size();
     DXF_CHECK(V >= 1 && V <= dx::kMaxVirtualRanks && (int)per_rank.size() == V, "em_notify: one entry per rank");
     std::vector<dx::EmNotifyArgs> args(V);
+    std::vector<dxh::RuntimeCore*> cores;
     dxh::RuntimeCore* core0 = dx_core_of(rts[0]);
     c10::cuda::CUDAGuard guard(core0->device());
     for (int v = 0; v < V; ++v) {
         dxh::RuntimeCore* core = dx_core_of(rts[v]);
+        cores.push_back(core);
         const py::tuple& t = per_rank[v];
         DXF_CHECK(t.size() == 12, "em_notify: per-rank tuple must have 12 entries");
         auto topk_idx = t[0].cast<torch::Tensor>();
@@ -104,7 +106,9 @@ void em_notify(std::vector<py::object> rts, std::vector<py::tuple> per_rank, int
         a.m_ends = m_ends.data_ptr<int>();
         a.peer_bases = reinterpret_cast<uint64_t*>(peer_bases.data_ptr());
     }
-    check(dx::launch_em_notify(args.data(), V, at::cuda::getCurrentCUDAStream(core0->device()).stream()), "em_notify");
+    dxh::OrderedCall order(std::move(cores), at::cuda::getCurrentCUDAStream(core0->device()).stream());
+    order.enter();
+    check(dx::launch_em_notify(args.data(), V, order.stream), "em_notify");
 }
 
 // Per rank tuple: (x, my_counts, sel_list, send_base, unit_start, peer_bases, dst_row|None, trace|None, x_scales|None)
@@ -115,10 +119,12 @@ void em_dispatch(std::vector<py::object> rts, std::vector<py::tuple> per_rank, i
     DXF_CHECK(V >= 1 && V <= dx::kMaxVirtualRanks && (int)per_rank.size() == V, "em_dispatch: one entry per rank");
     DXF_CHECK(num_sms >= 1 && unit_rows >= 1, "num_sms and unit_rows must be positive");
     std::vector<dx::EmDispatchArgs> args(V);
+    std::vector<dxh::RuntimeCore*> cores;
     dxh::RuntimeCore* core0 = dx_core_of(rts[0]);
     c10::cuda::CUDAGuard guard(core0->device());
     for (int v = 0; v < V; ++v) {
         dxh::RuntimeCore* core = dx_core_of(rts[v]);
+        cores.push_back(core);
         const py::tuple& t = per_rank[v];
         DXF_CHECK(t.size() == 9, "em_dispatch: per-rank tuple must have 9 entries");
         auto x = t[0].cast<torch::Tensor>();
@@ -173,7 +179,9 @@ void em_dispatch(std::vector<py::object> rts, std::vector<py::tuple> per_rank, i
         }
         a.num_sms = num_sms;
     }
-    check(dx::launch_em_dispatch(args.data(), V, at::cuda::getCurrentCUDAStream(core0->device()).stream()), "em_dispatch");
+    dxh::OrderedCall order(std::move(cores), at::cuda::getCurrentCUDAStream(core0->device()).stream());
+    order.enter();
+    check(dx::launch_em_dispatch(args.data(), V, order.stream), "em_dispatch");
 }
 
 // Views of the expert-major control words of this rank: (arrival counters [kMaxLocalExperts] u64 inside the symmetric

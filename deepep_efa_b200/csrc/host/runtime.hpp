@@ -214,7 +214,7 @@ class RuntimeCore {
     }
 
     // Called when the last tensor of a block dies (any thread). `streams` (up to two, nullptr = the default stream) are the
-    // streams whose queued work may still use the block. So may the normal-mode calls, on whatever stream they ran: the last of
+    // streams whose queued work may still use the block. So may the ordered calls (below), on whatever stream they ran: the last of
     // them is behind all others, so when it was on neither of these streams its event is waited for as well. Events come from a
     // pool: creating and destroying them cost more than everything else here.
     void arena_release(uint64_t off, const cudaStream_t* streams, int num_streams) {
@@ -243,8 +243,8 @@ class RuntimeCore {
         pending_.push_back(p);
     }
 
-    // ---- order of the normal-mode kernels -----------------------------------------------------
-    // They share state (sequence numbers, tickets, the layout scratch), so one must not overlap the next one. A call runs on the
+    // ---- order of the normal-mode and expert-major kernels ------------------------------------
+    // They share state (sequence numbers, tickets, count words, the layout scratch), so one must not overlap the next one. A call runs on the
     // caller's stream, or on the communication stream when the caller asked for an event; a call on another stream than the
     // last one waits for that one's event first. Enter before the first launch of a call and leave after the last one, with
     // nothing in between that lets another host thread in (a wait for the GPU): a call that waits leaves before it does.
@@ -377,7 +377,7 @@ class RuntimeCore {
         uint64_t off = 0;
         cudaEvent_t events[2];
         int num_events = 0;
-        std::shared_ptr<cudaEvent_t> last_call;  // of the normal-mode calls, where the events do not cover it
+        std::shared_ptr<cudaEvent_t> last_call;  // of the ordered calls, where the events do not cover it
     };
 
     struct OwnedEvent {
@@ -458,6 +458,29 @@ class RuntimeCore {
     std::vector<cudaEvent_t> event_pool_;  // bounded by the number of blocks that were ever pending at once
     Order order_, capture_order_;
     std::mutex mu_;
+};
+
+// The launches of one call on one stream, ordered behind the previous call's (RuntimeCore::order_enter) of every rank that takes part.
+class OrderedCall {
+  public:
+    OrderedCall(std::vector<RuntimeCore*> cores, cudaStream_t s) : stream(s), cores_(std::move(cores)) {}
+    OrderedCall(const OrderedCall&) = delete;
+    ~OrderedCall() { leave(); }
+    void enter() {
+        if (inside_) return;
+        for (RuntimeCore* c : cores_) c->order_enter(stream);
+        inside_ = true;
+    }
+    void leave() {
+        if (!inside_) return;
+        for (RuntimeCore* c : cores_) c->order_leave(stream);
+        inside_ = false;
+    }
+    const cudaStream_t stream;
+
+  private:
+    std::vector<RuntimeCore*> cores_;
+    bool inside_ = false;
 };
 
 }  // namespace dxh

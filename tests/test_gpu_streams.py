@@ -233,3 +233,31 @@ def test_layout_scratch_outgrown_while_another_stream_uses_it():
             assert not isinstance(k, list) or all(bool((t == 7).all()) for t in k)
     finally:
         vc.destroy()
+
+
+def test_fused_layers_of_one_buffer_on_two_streams():
+    """Two layers that share a buffer, each on a stream of its own: the count exchanges and dispatches share the buffer's words."""
+    from deepep_efa_b200.models.moe import MoEConfig, MoELayer
+    vc, buf = _buffer(nvl=512 << 20)
+    try:
+        layers = [MoELayer(MoEConfig(hidden=512, intermediate=256, num_experts=e, num_topk=k, init_std=0.05), buf, seed=e) for e, k in ((64, 6), (16, 2))]
+        tokens = (4000, 700)
+        data = []
+        for i, (layer, n) in enumerate(zip(layers, tokens)):
+            layer.prepare_fp8(native_block_scaling=i == 0)
+            idx, w = make_routing(n, layer.cfg.num_experts, layer.cfg.num_topk, "cuda", seed=20 + i, masked_fraction=0.1)
+            data.append((make_tokens(n, 512, "cuda", seed=20 + i), idx, w))
+        want = [layer.forward_fused(*d).clone() for layer, d in zip(layers, data)]
+        streams = [torch.cuda.Stream() for _ in layers]
+        torch.cuda.synchronize()
+        for _ in range(10):
+            got = []
+            for _ in range(3):
+                for layer, d, stream in zip(layers, data, streams):
+                    with torch.cuda.stream(stream):
+                        got.append(layer.forward_fused(*d))
+            torch.cuda.synchronize()
+            buf.check_status(sync=True)
+            assert all(torch.equal(g, want[i % 2]) for i, g in enumerate(got))
+    finally:
+        vc.destroy()
