@@ -347,8 +347,8 @@ __global__ void __launch_bounds__(kEmDispatchThreads, 6) em_dispatch_kernel(cons
         __syncwarp();
         // one release per unit: everything this warp stored for expert (d, le) is visible before the counter moves
         if (lane == 0 && sent > 0) {
-            // (rows for an expert of this GPU need no more than GPU scope: their reader is a kernel of this GPU)
-            if (d == me) red_add_release_gpu(&c.ctrl(d)->em_arrived[le], (uint64_t)sent);
+            // (GPU scope is enough only where nobody else adds to the counter: additions of two scopes to one word are not atomic to each other)
+            if (R == 1) red_add_release_gpu(&c.ctrl(d)->em_arrived[le], (uint64_t)sent);
             else red_add_release_sys(&c.ctrl(d)->em_arrived[le], (uint64_t)sent);
         }
     }
