@@ -77,6 +77,9 @@ struct GroupedGemmArgs {
     // 1 = m_offsets and m_ends were final before the kernel in front of this one in the stream began, and that kernel started only
     // after everything before it had ended: the tile table is then built without waiting for it (programmatic dependent launch).
     int early_table;
+    // 1 = the next kernel in the stream gets no SM before this one has ended, also where it is a programmatic dependent launch: the SMs
+    // that this launch leaves free are meant for another stream.
+    int hold_successor;
     // 1 = natively block-scaled 256-column tiles with the weights as the M operand and the tokens as N (see launch_grouped_gemm)
     int swap;
 };

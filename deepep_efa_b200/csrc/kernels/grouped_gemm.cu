@@ -525,7 +525,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     // With p.early_table the group table is older than the predecessor, so the tile table and the first weights do not wait for it.
     if (!p.early_table) {
         pdl_wait_predecessor();
-        pdl_release_successor();
+        if (!p.hold_successor) pdl_release_successor();
     }
     if (warp == 2) {
         // tile table: one warp scans the groups (one thread walking 256 groups through dependent loads took about 10 us)
@@ -656,7 +656,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             }
         }
         pdl_wait_predecessor();
-        pdl_release_successor();
+        if (!p.hold_successor) pdl_release_successor();
     }
 
     // kSwap: the weights are the M operand and the tokens the N operand, in steps of 32 columns up to the tile's valid rows. A group of

@@ -453,7 +453,8 @@ def fused_forward_many(layers, xs, idxs, ws, overlap: bool = True, num_dispatch_
         parts = [(0, ga, 148 - RESERVED_SMS), (ga, L - ga, 0)] if (overlapped and ga < L) else [(0, L, (148 - RESERVED_SMS) if overlapped else 0)]
         for pi, (g0, ng, sms1) in enumerate(parts):
             tr = None if (w.trace is None or pi > 0) else w.trace[2:6]
-            gate = dict(trace=tr, sched=w.sched, early_table=not overlapped)
+            # what follows a part that leaves SMs to the dispatch must not take them early, while that part still waits for rows
+            gate = dict(trace=tr, sched=w.sched, early_table=not overlapped, hold_successor=sms1 > 0)
             if not lone:
                 # (a lone rank's rows are in place when its dispatch has run, which this stream already waits for. The words are the
                 # buffer's: the next call of another layer on another stream raises what is expected, and a GEMM on every SM that

@@ -441,3 +441,31 @@ def test_fp8_native_wide_swiglu_cta_pairs(monkeypatch):
     assert _rel_err(single, ref) < 1.5e-2
     assert _rel_err(paired, ref) < 1.5e-2, _rel_err(paired, ref)
     assert torch.equal(paired, single) and torch.equal(paired_small_grid, single)
+
+
+def test_held_successor_leaves_the_free_sms_to_another_stream():
+    """A GEMM on four SMs that holds its successor: the one behind it in the stream must not occupy the other SMs meanwhile, so a GEMM
+    of another stream, launched last, ends before it begins."""
+    from deepep_efa_b200 import _ext
+    C = _ext.load()
+    C.gemm_clear_error(0)
+    torch.manual_seed(23)
+    big = torch.randn(8192, 4096, device="cuda").to(torch.bfloat16)
+    big_w = (torch.randn(1, 4096, 4096, device="cuda") * 0.02).to(torch.bfloat16)
+    small = torch.randn(148 * 128, 256, device="cuda").to(torch.bfloat16)
+    small_w = torch.randn(1, 256, 256, device="cuda").to(torch.bfloat16)
+    offs, offs_small = _offsets([8192]), _offsets([148 * 128])
+    big_id = torch.iinfo(torch.int64).max
+    stamps = [torch.tensor([big_id, 0, 0, 0], dtype=torch.int64, device="cuda") for _ in range(2)]
+    side = torch.cuda.Stream()
+    outs = []
+    for warm in (True, False):  # (once without stamps, so that no allocation or module load falls between the launches)
+        outs = [torch.empty(8192, 4096, dtype=torch.bfloat16, device="cuda")] + [torch.empty(148 * 128, 256, dtype=torch.bfloat16, device="cuda") for _ in range(2)]
+        torch.cuda.synchronize()
+        C.grouped_gemm(big, big_w, offs, 0, False, None, None, outs[0], 4, 2000.0, hold_successor=True)
+        C.grouped_gemm(small, small_w, offs_small, 0, False, None, None, outs[1], 0, 2000.0, trace=None if warm else stamps[0])
+        with torch.cuda.stream(side):
+            C.grouped_gemm(small, small_w, offs_small, 0, False, None, None, outs[2], 100, 2000.0, trace=None if warm else stamps[1])
+        torch.cuda.synchronize()
+    assert C.gemm_error(0) == 0 and torch.equal(outs[1], outs[2])
+    assert stamps[1][1].item() < stamps[0][0].item()
