@@ -70,6 +70,17 @@ class Arena {
         free_[off] = size;
     }
 
+    // Gives back what lies past the first `bytes` bytes of a block.
+    void shrink(uint64_t off, uint64_t bytes) {
+        auto u = used_.find(off);
+        if (u == used_.end()) throw std::runtime_error("Arena::shrink: offset " + std::to_string(off) + " is not an allocated block");
+        const uint64_t keep = bytes == 0 ? align_ : (bytes + align_ - 1) / align_ * align_;
+        if (keep >= u->second) return;
+        used_[off + keep] = u->second - keep;
+        u->second = keep;
+        free(off + keep);
+    }
+
     bool owns(uint64_t off) const { return used_.count(off) != 0; }
     uint64_t base() const { return base_; }
     uint64_t capacity() const { return size_; }

@@ -31,6 +31,7 @@ struct Runtime {
     std::shared_ptr<RuntimeCore> core;
     cudaStream_t comm_stream = nullptr;
     torch::Tensor layout_scratch;  // grows on demand
+    bool all_tokens_sent = true;   // by the last dispatch of a lone rank (see normal_dispatch)
 
     Runtime(int rank, int num_ranks, int64_t num_nvl_bytes, int64_t num_ll_bytes, int device, double timeout_ms, bool mask_on_timeout)
         : core(std::make_shared<RuntimeCore>(rank, num_ranks, (uint64_t)num_nvl_bytes, (uint64_t)num_ll_bytes, device, timeout_ms,
@@ -61,15 +62,15 @@ struct Runtime {
     };
     using BlockPtr = std::shared_ptr<Block>;
     BlockPtr alloc_block(uint64_t bytes) { return std::make_shared<Block>(core, bytes, comm_stream); }
-    torch::Tensor tensor_in(const BlockPtr& block, uint64_t byte_off, at::IntArrayRef sizes, torch::ScalarType dtype) {
-        return torch::from_blob(reinterpret_cast<char*>(core->base()) + block->off + byte_off, sizes, [block](void*) {},
+    torch::Tensor tensor_in(const BlockPtr& block, at::IntArrayRef sizes, torch::ScalarType dtype) {
+        return torch::from_blob(reinterpret_cast<char*>(core->base()) + block->off, sizes, [block](void*) {},
                                 torch::TensorOptions().dtype(dtype).device(torch::kCUDA, core->device()));
     }
 
     torch::Tensor alloc_symmetric(std::vector<int64_t> sizes, torch::ScalarType dtype) {
         int64_t numel = 1;
         for (auto s : sizes) numel *= s;
-        return tensor_in(alloc_block((uint64_t)numel * c10::elementSize(dtype)), 0, sizes, dtype);
+        return tensor_in(alloc_block((uint64_t)numel * c10::elementSize(dtype)), sizes, dtype);
     }
 
     // Offset of a tensor inside the symmetric buffer, or -1 when it lives elsewhere.
@@ -200,18 +201,38 @@ struct DispatchCall {
     torch::ScalarType out_type;
     bool has_scales = false;
     std::vector<int> per_expert;
-    // outputs: the payload in one block of the arena, the row metadata (part of which lives on in the handle) in another
-    Runtime::BlockPtr payload, meta;
-    uint64_t scales_at = 0, topk_w_at = 0, src_idx_at = 0;  // byte offsets inside the blocks
+    // One block of the arena per output: some outlive the others (the source indices live on in the handle).
+    struct Out {
+        Runtime::BlockPtr block;
+        uint64_t row_bytes = 0;
+        bool there = false;
+        uint64_t off() const { return there ? block->off : 0; }
+    };
+    Out recv_x, recv_scales, recv_idx, recv_w, src_idx;
 
+    template <typename F>
+    void each_out(F f) {
+        for (Out* o : {&recv_x, &recv_scales, &recv_idx, &recv_w, &src_idx})
+            if (o->there) f(*o);
+    }
+    void describe() {
+        recv_x = {nullptr, (uint64_t)H * c10::elementSize(out_type), true};
+        recv_scales = {nullptr, (uint64_t)(H / 128) * 4, has_scales};
+        recv_idx = {nullptr, (uint64_t)K * 8, topk_idx.has_value()};
+        recv_w = {nullptr, (uint64_t)K * 4, topk_w.has_value()};
+        src_idx = {nullptr, 4, true};
+    }
     void allocate(Runtime* rt, int rows) {
-        const uint64_t x_bytes = (uint64_t)rows * H * c10::elementSize(out_type);
-        scales_at = dxh::align_up(x_bytes, 1024);
-        payload = rt->alloc_block(has_scales ? scales_at + (uint64_t)rows * (H / 128) * 4 : x_bytes);
-        const uint64_t idx_bytes = topk_idx.has_value() ? (uint64_t)rows * K * 8 : 0, w_bytes = topk_w.has_value() ? (uint64_t)rows * K * 4 : 0;
-        topk_w_at = dxh::align_up(idx_bytes, 128);
-        src_idx_at = dxh::align_up(topk_w_at + w_bytes, 128);
-        meta = rt->alloc_block(src_idx_at + (uint64_t)rows * 4);
+        each_out([&](Out& o) { o.block = rt->alloc_block((uint64_t)rows * o.row_bytes); });
+    }
+    uint64_t bytes(int rows) {
+        uint64_t sum = 0;
+        each_out([&](Out& o) { sum += dxh::align_up((uint64_t)rows * o.row_bytes + 1, 1024); });
+        return sum;
+    }
+    // The kernel writes no row past the received ones, so the rest is as good as never allocated.
+    void trim(Runtime* rt, int rows) {
+        each_out([&](Out& o) { rt->core->arena_shrink(o.block->off, (uint64_t)rows * o.row_bytes); });
     }
 };
 
@@ -271,6 +292,7 @@ py::list normal_dispatch(std::vector<Runtime*> rts, const std::vector<py::tuple>
         } else {
             DX_CHECK(!q.topk_w.has_value(), "topk_weights need topk_idx");
         }
+        q.describe();
         cached = !t[7].is_none();
         if (cached) {
             const py::tuple h = t[7].cast<py::tuple>();
@@ -327,20 +349,17 @@ py::list normal_dispatch(std::vector<Runtime*> rts, const std::vector<py::tuple>
     }
 
     // How many rows arrive is known on the host only when the count exchange has run, except that a lone rank receives at most
-    // its own tokens: its outputs are sized for them, the dispatch kernel is queued at once and the host waits beside it.
+    // its own tokens: its outputs are sized for them and cut to what has arrived afterwards; the dispatch kernel is queued at once
+    // and the host waits beside it. Cutting leaves holes in the arena, so this is done only where a row per token is a small part of
+    // it (a quarter of the largest free block) and while all tokens are sent: a caller whose last dispatch left some out waits first.
     const bool exact = !cached && num_worst_tokens == 0;
     bool waited = !exact;
     for (int v = 0; v < V; ++v) {
         DispatchCall& q = calls[v];
         int rows = cached ? q.num_recv : num_worst_tokens;
-        if (exact && R == 1) {
-            try {
-                q.allocate(rts[v], q.T);
-            } catch (const std::runtime_error&) {  // the arena may still hold what really arrives
-                q.payload.reset();
-                q.meta.reset();
-            }
-            if (q.meta) continue;
+        if (exact && R == 1 && rts[v]->all_tokens_sent && 4 * q.bytes(q.T) <= rts[v]->core->arena_largest_free()) {
+            q.allocate(rts[v], q.T);
+            continue;
         }
         if (exact) {
             order.leave();
@@ -369,11 +388,11 @@ py::list normal_dispatch(std::vector<Runtime*> rts, const std::vector<py::tuple>
         a.hidden = q.H;
         a.num_experts = E;
         a.num_sms = num_sms;
-        a.recv_x_off = q.payload->off;
-        a.recv_scales_off = q.has_scales ? q.payload->off + q.scales_at : 0;
-        a.recv_topk_idx_off = q.topk_idx.has_value() ? q.meta->off : 0;
-        a.recv_topk_w_off = q.topk_w.has_value() ? q.meta->off + q.topk_w_at : 0;
-        a.recv_src_idx_off = q.meta->off + q.src_idx_at;
+        a.recv_x_off = q.recv_x.off();
+        a.recv_scales_off = q.recv_scales.off();
+        a.recv_topk_idx_off = q.recv_idx.off();
+        a.recv_topk_w_off = q.recv_w.off();
+        a.recv_src_idx_off = q.src_idx.off();
         a.num_worst_tokens = num_worst_tokens;
     }
     order.enter();
@@ -384,14 +403,18 @@ py::list normal_dispatch(std::vector<Runtime*> rts, const std::vector<py::tuple>
     for (int v = 0; v < V; ++v) {
         Runtime* rt = rts[v];
         DispatchCall& q = calls[v];
-        if (!waited) wait_counts(rt, q, E / R);
+        if (!waited) {
+            wait_counts(rt, q, E / R);
+            q.trim(rt, q.num_recv);
+        }
+        if (exact && R == 1) rt->all_tokens_sent = q.num_recv == q.T;
         const int64_t n = q.num_recv, H = q.H, K = q.K;
-        auto opt = [](bool there, auto make) -> py::object { return there ? py::cast(make()) : py::object(py::none()); };
-        py::object scales = opt(q.has_scales, [&] { return rt->tensor_in(q.payload, q.scales_at, {n, H / 128}, torch::kFloat32); });
-        py::object idx = opt(q.topk_idx.has_value(), [&] { return rt->tensor_in(q.meta, 0, {n, K}, torch::kInt64); });
-        py::object w = opt(q.topk_w.has_value(), [&] { return rt->tensor_in(q.meta, q.topk_w_at, {n, K}, torch::kFloat32); });
-        out.append(py::make_tuple(rt->tensor_in(q.payload, 0, {n, H}, q.out_type), scales, idx, w, q.per_expert,
-                                  py::make_tuple(q.rpm, q.cpm, q.rcpm, rt->tensor_in(q.meta, q.src_idx_at, {n}, torch::kInt32), q.in_rank, q.send_head)));
+        auto tensor = [&](const DispatchCall::Out& o, std::initializer_list<int64_t> sizes, torch::ScalarType dtype) -> py::object {
+            return o.there ? py::cast(rt->tensor_in(o.block, sizes, dtype)) : py::object(py::none());
+        };
+        out.append(py::make_tuple(tensor(q.recv_x, {n, H}, q.out_type), tensor(q.recv_scales, {n, H / 128}, torch::kFloat32),
+                                  tensor(q.recv_idx, {n, K}, torch::kInt64), tensor(q.recv_w, {n, K}, torch::kFloat32), q.per_expert,
+                                  py::make_tuple(q.rpm, q.cpm, q.rcpm, tensor(q.src_idx, {n}, torch::kInt32), q.in_rank, q.send_head)));
     }
     return out;
 }
@@ -435,7 +458,7 @@ py::list normal_combine(std::vector<Runtime*> rts, const std::vector<py::tuple>&
             const bool in_place = R == 1 && !rt->core->debug_checks() && (reinterpret_cast<uintptr_t>(tt.data_ptr()) & 15) == 0;
             if (off < 0 && !in_place) {
                 const uint64_t bytes = (uint64_t)tt.numel() * tt.element_size();
-                auto staged = rt->tensor_in(rt->alloc_block(bytes), 0, tt.sizes(), tt.scalar_type());
+                auto staged = rt->tensor_in(rt->alloc_block(bytes), tt.sizes(), tt.scalar_type());
                 DX_CUDA_CHECK(cudaMemcpyAsync(staged.data_ptr(), tt.data_ptr(), bytes, cudaMemcpyDeviceToDevice, order.stream));
                 off = rt->symmetric_offset(staged);
                 keep.push_back(staged);
@@ -750,6 +773,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         .def(py::init<uint64_t, uint64_t, uint64_t>(), py::arg("base"), py::arg("size"), py::arg("align") = 1024)
         .def("alloc", &dxh::Arena::alloc)
         .def("free", &dxh::Arena::free)
+        .def("shrink", &dxh::Arena::shrink)
         .def("owns", &dxh::Arena::owns)
         .def_property_readonly("capacity", &dxh::Arena::capacity)
         .def_property_readonly("in_use", &dxh::Arena::in_use)

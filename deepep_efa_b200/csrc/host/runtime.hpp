@@ -213,6 +213,18 @@ class RuntimeCore {
         return (uint64_t)off;
     }
 
+    uint64_t arena_largest_free() {
+        std::lock_guard<std::mutex> g(mu_);
+        drain_pending(false);
+        return arena_.largest_free();
+    }
+
+    // Gives back the end of a block that nothing has used or will use.
+    void arena_shrink(uint64_t off, uint64_t bytes) {
+        std::lock_guard<std::mutex> g(mu_);
+        if (!released_) arena_.shrink(off, bytes);
+    }
+
     // Called when the last tensor of a block dies (any thread). `streams` (up to two, nullptr = the default stream) are the
     // streams whose queued work may still use the block. So may the ordered calls (below), on whatever stream they ran: the last of
     // them is behind all others, so when it was on neither of these streams its event is waited for as well. Events come from a

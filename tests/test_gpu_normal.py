@@ -229,3 +229,41 @@ def test_handle_validation_catches_foreign_and_corrupt_handles():
             validate_handle(tuple(h), 0, R)
     finally:
         vc.destroy()
+
+
+@pytest.mark.parametrize("mode", ["bf16", "fp8_fused"])
+def test_dispatch_holds_the_rows_that_arrived(mode):
+    """A lone rank whose tokens are mostly unselected: results hold as much symmetric memory as their rows, each tensor its own, up to
+    where the arena could not hold a row per token."""
+    vc = _cluster(1, nvl=24 << 20)
+    try:
+        buf = vc.buffers[0]
+        T, H, E, K = 2000, 2048, 8, 2
+        x = make_tokens(T, H, "cuda", seed=3)
+        idx, w = make_routing(T, E, K, "cuda", seed=3)
+        idx[torch.arange(T, device="cuda") % 20 != 7] = -1
+        rows = T // 20
+        up = lambda b: (b + 1023) // 1024 * 1024
+        elem = 1 if mode == "fp8_fused" else 2
+        each = up(rows * H * elem) + (up(rows * H // 128 * 4) if elem == 1 else 0) + up(rows * K * 8) + up(rows * K * 4) + up(rows * 4)
+        per_rank, _, per_expert, in_rank, _ = buf.get_dispatch_layout(idx, E)
+        base, held = buf.runtime.arena_in_use(), []
+        fits = (buf.runtime.arena_capacity() - base) // each
+        for i in range(fits - 1):  # the last ones find no room for T rows
+            held.append(buf.dispatch(x, num_tokens_per_rank=per_rank, is_token_in_rank=in_rank, num_tokens_per_expert=per_expert, topk_idx=idx,
+                                     topk_weights=w, quantize_fp8=elem == 1))
+            assert buf.runtime.arena_in_use() - base == (i + 1) * each
+        assert len(held) * each + T * H * elem > buf.runtime.arena_capacity()
+        for recv, recv_idx, recv_w, _, _, _ in (held[0], held[-1]):
+            assert torch.equal(recv_w, w[7::20]) and torch.equal(recv_idx, idx[7::20])
+            assert elem == 1 or torch.equal(recv, x[7::20])
+        # the handle keeps the source indices, and nothing else
+        handles = [h[4] for h in held]
+        del held, recv, recv_idx, recv_w
+        torch.cuda.synchronize()
+        buf.empty_symmetric([1], torch.int32)  # takes back what is free
+        assert buf.runtime.arena_in_use() - base == len(handles) * up(rows * 4) + 1024
+        y = make_tokens(rows, H, "cuda", seed=4)
+        assert torch.equal(buf.combine(y, handles[-1])[0][7::20], y)
+    finally:
+        vc.destroy()

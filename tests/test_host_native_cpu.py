@@ -68,6 +68,22 @@ def test_arena_random_stress():
     assert a.in_use == 0 and a.num_free_blocks == 1
 
 
+def test_arena_shrink_gives_back_the_end_of_a_block():
+    a = C.Arena(0, 64 << 10, 1024)
+    first, second = a.alloc(10 << 10), a.alloc(4 << 10)
+    a.shrink(first, 3000)
+    assert a.in_use == (3 << 10) + (4 << 10)
+    assert a.alloc(7 << 10) == first + (3 << 10)
+    a.shrink(second, 1 << 20)  # never grows
+    a.shrink(second, 0)        # the smallest block
+    assert a.in_use == (3 << 10) + (7 << 10) + (1 << 10)
+    for off in (first, first + (3 << 10), second):
+        a.free(off)
+    assert a.in_use == 0 and a.num_free_blocks == 1
+    with pytest.raises(RuntimeError):
+        a.shrink(first, 0)
+
+
 def test_low_latency_layout_class():
     import deepep_efa_b200 as ep
     lay = ep.LowLatencyLayout(C.CONTROL_BYTES, 128, 7168, 8, 256)
