@@ -444,18 +444,22 @@ py::list normal_combine(std::vector<Runtime*> rts, const std::vector<py::tuple>&
         auto b0 = opt_tensor(t[4]);
         auto b1 = opt_tensor(t[5]);
         DX_CHECK(x.is_cuda() && x.dim() == 2 && x.scalar_type() == torch::kBFloat16, "combine: x must be bf16 [N,hidden] on the GPU");
-        DX_CHECK(!w.has_value() || (w->is_cuda() && w->scalar_type() == torch::kFloat32 && w->dim() == 2), "combine: topk_weights must be f32 [N,K] on the GPU");
+        if (w.has_value()) {
+            // weights of another type, or on the host, are converted on the way to where the peers read them
+            if (rt->symmetric_offset(*w) < 0) w = w->to(x.device(), torch::kFloat32);
+            DX_CHECK(w->scalar_type() == torch::kFloat32 && w->dim() == 2, "combine: topk_weights must be [N,K], and f32 in the symmetric buffer");
+        }
         const int H = (int)x.size(1), T = (int)send_head.size(0);
         DX_CHECK(H % 8 == 0, "hidden must be a multiple of 8");
         DX_CHECK(send_head.scalar_type() == torch::kInt32 && send_head.is_contiguous() && send_head.size(1) == R, "send_head must be int32 [T,R]");
         used_here(send_head);
         used_here(rpm);
         // What the peers read must lie in symmetric memory; anything else is staged there. A lone rank reads its own tensor where
-        // it is (an offset that leaves the buffer, which the debug range check would refuse).
+        // it is (an offset that leaves the buffer, which the debug range check would refuse), given a row for every row of x.
         auto place = [&](const torch::Tensor& given) -> uint64_t {
             torch::Tensor tt = given.contiguous();
             int64_t off = rt->symmetric_offset(tt);
-            const bool in_place = R == 1 && !rt->core->debug_checks() && (reinterpret_cast<uintptr_t>(tt.data_ptr()) & 15) == 0;
+            const bool in_place = R == 1 && !rt->core->debug_checks() && tt.size(0) >= x.size(0) && (reinterpret_cast<uintptr_t>(tt.data_ptr()) & 15) == 0;
             if (off < 0 && !in_place) {
                 const uint64_t bytes = (uint64_t)tt.numel() * tt.element_size();
                 auto staged = rt->tensor_in(rt->alloc_block(bytes), tt.sizes(), tt.scalar_type());
@@ -478,7 +482,7 @@ py::list normal_combine(std::vector<Runtime*> rts, const std::vector<py::tuple>&
         if (w.has_value()) {
             a.topk_w_off = place(*w);
             a.num_topk = (int)w->size(1);
-            out_w = t[7].is_none() ? torch::empty({T, a.num_topk}, w->options()) : t[7].cast<torch::Tensor>();
+            out_w = t[7].is_none() ? torch::empty({T, a.num_topk}, x.options().dtype(torch::kFloat32)) : t[7].cast<torch::Tensor>();
             DX_CHECK(out_w->scalar_type() == torch::kFloat32 && out_w->is_contiguous() && out_w->numel() == (int64_t)T * a.num_topk, "combine: out_topk_weights must be f32 [T,K]");
             a.out_topk_w = out_w->data_ptr<float>();
         }

@@ -267,3 +267,33 @@ def test_dispatch_holds_the_rows_that_arrived(mode):
         assert torch.equal(buf.combine(y, handles[-1])[0][7::20], y)
     finally:
         vc.destroy()
+
+
+@pytest.mark.parametrize("R", [1, 2])
+@pytest.mark.parametrize("kind", ["bf16", "f64", "cpu", "strided", "misaligned"])
+def test_combine_takes_weights_of_any_type_and_place(R, kind):
+    vc = _cluster(R)
+    try:
+        T, H, E, K = 65, 512, 4 * R, 3
+        xs, idxs, ws = _inputs(R, T, H, E, K, seed=11)
+        lay = vc.get_dispatch_layout(idxs, E)
+        res = vc.dispatch(xs, layouts=lay, topk_idxs=idxs, topk_weights=[w.to(torch.bfloat16).float() for w in ws])
+        ys, handles, rws = [r[0] for r in res], [r[4] for r in res], [r[2] for r in res]
+        want = vc.combine(ys, handles, topk_weights=rws)
+
+        def given(w):
+            if kind == "strided":
+                return torch.stack([w, w], dim=2)[:, :, 0]
+            if kind == "misaligned":
+                flat = torch.empty(w.numel() + 1, device="cuda")
+                flat[1:] = w.flatten()
+                return flat[1:].view_as(w)
+            return {"bf16": w.to(torch.bfloat16), "f64": w.double(), "cpu": w.cpu()}[kind]
+
+        got = vc.combine(ys, handles, topk_weights=[given(w) for w in rws])
+        torch.cuda.synchronize()
+        for a, b in zip(got, want):
+            assert a[1].dtype == torch.float32 and a[1].is_cuda
+            assert torch.equal(a[0], b[0]) and torch.equal(a[1], b[1])
+    finally:
+        vc.destroy()
