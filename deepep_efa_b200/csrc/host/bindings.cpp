@@ -289,9 +289,7 @@ py::list normal_dispatch(std::vector<Runtime*> rts, const std::vector<py::tuple>
             DX_CHECK(q.K <= dx::kMaxTopk, "num_topk too large");
             if (q.topk_w.has_value())
                 DX_CHECK(q.topk_w->scalar_type() == torch::kFloat32 && q.topk_w->is_contiguous() && q.topk_w->numel() == q.topk_idx->numel(), "topk_weights must be f32 [T,K]");
-        } else {
-            DX_CHECK(!q.topk_w.has_value(), "topk_weights need topk_idx");
-        }
+        }  // (weights without ids do not travel: the result is [rows, 0])
         q.describe();
         cached = !t[7].is_none();
         if (cached) {
@@ -380,7 +378,7 @@ py::list normal_dispatch(std::vector<Runtime*> rts, const std::vector<py::tuple>
         a.quantize = quantize ? 1 : 0;
         a.round_scale = round_scale ? 1 : 0;
         a.topk_idx = ptr_or_null<int64_t>(q.topk_idx);
-        a.topk_weights = ptr_or_null<float>(q.topk_w);
+        a.topk_weights = q.topk_idx.has_value() ? ptr_or_null<float>(q.topk_w) : nullptr;
         a.num_topk = q.K;
         a.send_head = q.send_head.data_ptr<int>();
         a.rank_prefix_matrix = q.rpm.data_ptr<int>();

@@ -297,3 +297,19 @@ def test_combine_takes_weights_of_any_type_and_place(R, kind):
             assert torch.equal(a[0], b[0]) and torch.equal(a[1], b[1])
     finally:
         vc.destroy()
+
+
+@pytest.mark.parametrize("R", [1, 2])
+def test_dispatch_with_weights_but_no_ids(R):
+    vc = _cluster(R)
+    try:
+        T, H, E, K = 40, 256, 4 * R, 2
+        xs, idxs, ws = _inputs(R, T, H, E, K, seed=12)
+        lay = vc.get_dispatch_layout(idxs, E)
+        want = vc.dispatch(xs, layouts=lay)
+        got = vc.dispatch(xs, layouts=lay, topk_weights=ws)
+        torch.cuda.synchronize()
+        for a, b in zip(got, want):
+            assert torch.equal(a[0], b[0]) and a[1] is None and a[2].shape == (a[0].size(0), 0) and a[2].dtype == torch.float32
+    finally:
+        vc.destroy()
