@@ -293,7 +293,7 @@ py::list normal_dispatch(std::vector<Runtime*> rts, const std::vector<py::tuple>
         q.describe();
         cached = !t[7].is_none();
         if (cached) {
-            const py::tuple h = t[7].cast<py::tuple>();
+            const py::tuple h(py::reinterpret_borrow<py::object>(t[7]));  // any sequence: a saved handle may come back as a list
             DX_CHECK(h.size() == 6, "a normal-mode handle has 6 entries");
             q.rpm = h[0].cast<torch::Tensor>();
             q.cpm = h[1].cast<torch::Tensor>();

@@ -313,3 +313,14 @@ def test_dispatch_with_weights_but_no_ids(R):
             assert torch.equal(a[0], b[0]) and a[1] is None and a[2].shape == (a[0].size(0), 0) and a[2].dtype == torch.float32
     finally:
         vc.destroy()
+
+
+def test_cached_dispatch_takes_a_handle_that_was_saved_as_a_list():
+    vc = _cluster(1)
+    try:
+        xs, idxs, _ = _inputs(1, 50, 256, 4, 2, seed=13)
+        res = vc.dispatch(xs, layouts=vc.get_dispatch_layout(idxs, 4))[0]
+        again = vc.buffers[0].dispatch(xs[0], handle=[t.clone() for t in res[4]])
+        assert torch.equal(again[0], res[0])
+    finally:
+        vc.destroy()
