@@ -225,7 +225,7 @@ torch::Tensor grouped_gemm(const torch::Tensor& a, const torch::Tensor& b, const
 std::tuple<torch::Tensor, torch::Tensor, torch::Tensor, torch::Tensor, int64_t> build_plan(const torch::Tensor& topk_idx, const std::vector<int>& counts) {
     DXG_CHECK(topk_idx.is_cuda() && topk_idx.dim() == 2 && topk_idx.is_contiguous() && topk_idx.scalar_type() == torch::kInt64, "topk_idx must be contiguous int64 [N,K] on the GPU");
     const int64_t N = topk_idx.size(0), K = topk_idx.size(1), L = (int64_t)counts.size();
-    DXG_CHECK(L >= 1 && L <= dx::kPlanMaxExperts, "between 1 and 1024 local experts");
+    DXG_CHECK(L >= 1, "at least one local expert");
     std::vector<int> offs(L + 1, 0);
     for (int64_t e = 0; e < L; ++e) offs[e + 1] = offs[e] + counts[e];
     const int64_t m_pad = offs[L];

@@ -89,7 +89,7 @@ cudaError_t launch_grouped_gemm(const GroupedGemmArgs& args, cudaStream_t stream
 
 // Expert-major plan from local expert ids [N, K] (-1 = unselected) and 128-aligned group offsets [L+1] on the host:
 // m_offsets [L+1] (the offsets on the device), pos [N*K], src_row [m_pad] (-1 = padding), src_k [m_pad] (0 there).
-constexpr int kPlanMaxExperts = 1024;  // local experts; the offsets travel as kernel arguments (4 KiB)
+constexpr int kPlanMaxExperts = 1024;  // local experts of one launch; the offsets travel as kernel arguments (4 KiB)
 cudaError_t launch_build_plan(const int64_t* topk_idx, const int* host_offsets, int* m_offsets, int* pos, int* src_row, int* src_k,
                               int num_rows, int num_topk, int num_local_experts, cudaStream_t stream);
 

@@ -102,7 +102,8 @@ __global__ void __launch_bounds__(kReduceThreads, kGatherReduceCtasPerSm) gather
 
 // Expert-major slot assignment: the selections of local expert e get the rows m_offsets[e], m_offsets[e] + 1, ... in token order;
 // the rest of the expert's 128-aligned segment is padding (src_row -1). One launch: the group offsets arrive in the arguments, a
-// CTA lists the selections of its experts (select_scan.cuh) and pads their segments, and CTA 0 marks the unselected ones.
+// CTA lists the selections of its experts (select_scan.cuh) and pads their segments, and CTA 0 marks the unselected ones. More experts
+// than the arguments hold take a launch per kPlanMaxExperts of them.
 struct PlanOffsets {
     int v[kPlanMaxExperts + 1];
 };
@@ -110,7 +111,7 @@ struct PlanOffsets {
 __global__ void __launch_bounds__(kScanThreads, 1) build_plan_kernel(const int64_t* __restrict__ topk_idx, const __grid_constant__ PlanOffsets offs,
                                                                      int* __restrict__ m_offsets, int* __restrict__ pos, int* __restrict__ src_row,
                                                                      int* __restrict__ src_k, int num_pairs, int num_topk, int num_local_experts,
-                                                                     int per_cta) {
+                                                                     int first, int count, int per_cta) {
     pdl_wait_predecessor();
     pdl_release_successor();
     extern __shared__ int s_dyn[];
@@ -118,11 +119,11 @@ __global__ void __launch_bounds__(kScanThreads, 1) build_plan_kernel(const int64
     uint32_t* s_vote = reinterpret_cast<uint32_t*>(s_dyn + kScanBatch);
     const int tid = threadIdx.x;
     if (blockIdx.x == 0)
-        for (int e = tid; e <= num_local_experts; e += kScanThreads) m_offsets[e] = offs.v[e];
-    const int e0 = blockIdx.x * per_cta, ne = max(0, min(per_cta, num_local_experts - e0));
+        for (int e = tid; e <= count; e += kScanThreads) m_offsets[first + e] = offs.v[e];
+    const int e0 = blockIdx.x * per_cta, ne = max(0, min(per_cta, count - e0));  // of the launch's experts [first, first + count)
     for (int b0 = 0; b0 < ne; b0 += kScanBatch) {
         const int nb = min(kScanBatch, ne - b0);
-        scan_selections(topk_idx, num_pairs, num_local_experts, e0 + b0, nb, s_vote, s_run, blockIdx.x == 0 && b0 == 0,
+        scan_selections(topk_idx, num_pairs, num_local_experts, first + e0 + b0, nb, s_vote, s_run, first == 0 && blockIdx.x == 0 && b0 == 0,
                         [&](int j, int n, int i) {
                             const int row = offs.v[e0 + b0 + j] + n;
                             const bool fits = row < offs.v[e0 + b0 + j + 1];  // always, when the offsets come from the dispatch counts
@@ -146,18 +147,21 @@ __global__ void __launch_bounds__(kScanThreads, 1) build_plan_kernel(const int64
 
 cudaError_t launch_build_plan(const int64_t* topk_idx, const int* host_offsets, int* m_offsets, int* pos, int* src_row, int* src_k,
                               int num_rows, int num_topk, int num_local_experts, cudaStream_t stream) {
-    if (num_local_experts < 1 || num_local_experts > kPlanMaxExperts) return cudaErrorInvalidValue;
-    PlanOffsets offs;
-    for (int e = 0; e <= num_local_experts; ++e) offs.v[e] = host_offsets[e];
-    const int ctas = num_local_experts < 148 ? num_local_experts : 148;
-    const int per_cta = (num_local_experts + ctas - 1) / ctas;
-    const size_t smem = scan_smem_bytes(per_cta);
-    if (smem > 48 * 1024) {
-        const cudaError_t e = cudaFuncSetAttribute(build_plan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (num_local_experts < 1) return cudaErrorInvalidValue;
+    for (int first = 0; first < num_local_experts; first += kPlanMaxExperts) {
+        const int count = std::min(num_local_experts - first, kPlanMaxExperts);
+        PlanOffsets offs;
+        for (int e = 0; e <= count; ++e) offs.v[e] = host_offsets[first + e];
+        const int per_cta = (count + 147) / 148;
+        const size_t smem = scan_smem_bytes(per_cta);
+        cudaError_t e = cudaSuccess;
+        if (smem > 48 * 1024) e = cudaFuncSetAttribute(build_plan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e == cudaSuccess)
+            e = launch_dependent(build_plan_kernel, dim3((count + per_cta - 1) / per_cta), kScanThreads, smem, stream, topk_idx, offs, m_offsets, pos, src_row,
+                                 src_k, num_rows * num_topk, num_topk, num_local_experts, first, count, per_cta);
         if (e != cudaSuccess) return e;
     }
-    return launch_dependent(build_plan_kernel, dim3((num_local_experts + per_cta - 1) / per_cta), kScanThreads, smem, stream, topk_idx, offs, m_offsets, pos,
-                            src_row, src_k, num_rows * num_topk, num_topk, num_local_experts, per_cta);
+    return cudaSuccess;
 }
 
 // Rows that are no multiple of 16 bytes (scale rows of some hidden sizes), word by word.

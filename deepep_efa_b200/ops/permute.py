@@ -36,7 +36,10 @@ class ExpertPlan:
 def build_expert_plan(recv_topk_idx: torch.Tensor, aligned_counts: List[int]) -> ExpertPlan:
     """``recv_topk_idx`` [N, K] holds local expert ids or -1; ``aligned_counts[e]`` >= rows of expert e."""
     if recv_topk_idx.is_cuda:
-        return ExpertPlan(*_ext.load().build_plan(recv_topk_idx.contiguous(), aligned_counts))
+        try:
+            return ExpertPlan(*_ext.load().build_plan(recv_topk_idx.contiguous(), aligned_counts))
+        except TypeError:  # anything else that int() takes
+            return ExpertPlan(*_ext.load().build_plan(recv_topk_idx.contiguous(), [int(c) for c in aligned_counts]))
     dev = recv_topk_idx.device
     N, K = recv_topk_idx.shape
     L = len(aligned_counts)

@@ -469,3 +469,27 @@ def test_held_successor_leaves_the_free_sms_to_another_stream():
         torch.cuda.synchronize()
     assert C.gemm_error(0) == 0 and torch.equal(outs[1], outs[2])
     assert stamps[1][1].item() < stamps[0][0].item()
+
+
+@pytest.mark.parametrize("L", [1, 3, 147, 149, 300, 1024, 1025, 2500])
+@pytest.mark.parametrize("N,K", [(1, 1), (700, 3), (8200, 4), (10923, 6)])
+def test_expert_plan_matches_the_cpu_plan(L, N, K):
+    """More experts than CTAs, than a pass over the ids takes and than one launch takes; selections past a chunk of 32768."""
+    import numpy as np
+    from deepep_efa_b200.ops.permute import build_expert_plan
+    if L * N * K > 70_000_000:
+        pytest.skip("the CPU plan holds a word per selection and expert")
+    g = torch.Generator().manual_seed(L + N)
+    idx = torch.randint(-1, L + 1, (N, K), generator=g)
+    idx[idx == L] = -1
+    counts = (torch.bincount(idx[idx >= 0], minlength=L) + 127) // 128 * 128
+    want = build_expert_plan(idx, counts.tolist())
+    for given in (counts.tolist(), counts.double().numpy(), [np.int64(c) for c in counts.tolist()]):
+        got = build_expert_plan(idx.cuda(), given)
+        assert got.num_rows == want.num_rows and torch.equal(got.m_offsets.cpu(), want.m_offsets)
+        assert torch.equal(got.pos.cpu(), want.pos) and torch.equal(got.src_row.cpu(), want.src_row)
+        filled = want.src_row >= 0
+        assert torch.equal(got.src_k.cpu()[filled], want.src_k[filled]) and bool((got.src_k.cpu()[~filled] == 0).all())
+    beyond = idx.clone()
+    beyond[idx < 0] = L  # an id past the last expert is as good as none
+    assert torch.equal(build_expert_plan(beyond.cuda(), counts.tolist()).pos.cpu(), want.pos)
