@@ -18,6 +18,8 @@
 //
 // Reference counterparts: notify_dispatch / cached_notify_dispatch (intranode.cu:11-195),
 // dispatch (:197-610), cached_notify_combine / combine (:612-1099), intranode::barrier (runtime.cu:13-26).
+#include <algorithm>
+
 #include "api.h"
 #include "prims.cuh"
 #include "launch.cuh"
@@ -417,7 +419,11 @@ __global__ void __launch_bounds__(kDispatchThreads, 1) dispatch_kernel(const __g
 }
 
 cudaError_t launch_dispatch(const DispatchArgs* a, int nv, cudaStream_t stream) {
-    return DX_LAUNCH_RANKED_PDL(dispatch_kernel, DispatchArgs, a, nv, grid_ctas(a, nv), kDispatchThreads, 0, stream);
+    // few tokens with outputs for many rows: enough CTAs that no thread marks more than eight unused ids
+    const long long ids = (long long)a[0].num_worst_tokens * (a[0].topk_idx != nullptr ? a[0].num_topk : 0);
+    const long long marking = (ids + 8 * kDispatchThreads - 1) / (8 * kDispatchThreads);
+    const int ctas = (int)std::max<long long>(grid_ctas(a, nv), std::min<long long>(marking, a[0].num_sms));
+    return DX_LAUNCH_RANKED_PDL(dispatch_kernel, DispatchArgs, a, nv, ctas, kDispatchThreads, 0, stream);
 }
 
 // =============================================================================================

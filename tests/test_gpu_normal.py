@@ -324,3 +324,21 @@ def test_cached_dispatch_takes_a_handle_that_was_saved_as_a_list():
         assert torch.equal(again[0], res[0])
     finally:
         vc.destroy()
+
+
+@pytest.mark.parametrize("R,worst", [(1, 9), (1, 70000), (2, 5000)])
+def test_few_tokens_with_outputs_for_many_rows(R, worst):
+    vc = _cluster(R)
+    try:
+        T, H, E, K = 3, 128, 4 * R, 4
+        xs, idxs, ws = _inputs(R, T, H, E, K, seed=14)
+        lay = vc.get_dispatch_layout(idxs, E)
+        want = vc.dispatch(xs, layouts=lay, topk_idxs=idxs, topk_weights=ws)
+        got = vc.dispatch(xs, layouts=lay, topk_idxs=idxs, topk_weights=ws, num_worst_tokens=worst)
+        torch.cuda.synchronize()
+        for a, b in zip(got, want):
+            n = b[0].size(0)
+            assert a[0].size(0) == worst and torch.equal(a[0][:n], b[0]) and torch.equal(a[1][:n], b[1]) and torch.equal(a[2][:n], b[2])
+            assert bool((a[1][n:] == -1).all())
+    finally:
+        vc.destroy()
