@@ -392,6 +392,7 @@ cudaError_t launch_stage_reduce(const void* stage, void* out, const int64_t* top
                                 int num_experts, int hidden, cudaStream_t stream) {
     if (num_tokens <= 0) return cudaSuccess;
     if (hidden % 8 != 0 || num_topk < 1 || num_topk > 32) return cudaErrorInvalidValue;
+    if (hidden == 0) return cudaSuccess;
     return launch_dependent(stage_reduce_kernel, dim3(reduce_ctas(num_tokens, hidden / 8)), kReduceThreads, 0, stream, static_cast<const __nv_bfloat16*>(stage),
                             static_cast<__nv_bfloat16*>(out), topk_idx, w, num_tokens, num_topk, num_experts, hidden);
 }

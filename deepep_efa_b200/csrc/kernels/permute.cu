@@ -177,7 +177,7 @@ __global__ void __launch_bounds__(kPermThreads) gather_words_kernel(const uint32
 
 cudaError_t launch_gather_rows(const void* src, void* dst, const int* src_row, const float* scale, int num_dst_rows, int row_bytes,
                                cudaStream_t stream) {
-    if (num_dst_rows <= 0) return cudaSuccess;
+    if (num_dst_rows <= 0 || row_bytes == 0) return cudaSuccess;
     if (row_bytes % 16 != 0) {
         if (row_bytes % 4 != 0 || scale != nullptr) return cudaErrorInvalidValue;
         return launch_dependent(gather_words_kernel, dim3((num_dst_rows + kPermThreads / 32 - 1) / (kPermThreads / 32)), kPermThreads, 0, stream,
@@ -193,6 +193,7 @@ cudaError_t launch_gather_reduce_rows(const void* src, void* dst, const int* pos
                                       cudaStream_t stream) {
     if (num_dst_rows <= 0) return cudaSuccess;
     if (hidden % 8 != 0 || num_k > 32 || num_k < 1) return cudaErrorInvalidValue;
+    if (hidden == 0) return cudaSuccess;
     return launch_dependent(gather_reduce_rows_kernel, dim3(std::min(reduce_ctas(num_dst_rows, hidden / 8), 148 * kGatherReduceCtasPerSm)), kReduceThreads, 0, stream,
                             static_cast<const __nv_bfloat16*>(src), static_cast<__nv_bfloat16*>(dst), pos, w, num_dst_rows, num_k, hidden);
 }

@@ -493,3 +493,16 @@ def test_expert_plan_matches_the_cpu_plan(L, N, K):
     beyond = idx.clone()
     beyond[idx < 0] = L  # an id past the last expert is as good as none
     assert torch.equal(build_expert_plan(beyond.cuda(), counts.tolist()).pos.cpu(), want.pos)
+
+
+def test_gathers_of_rows_without_columns():
+    """Nothing to move, as with the scale rows of fewer than 128 channels: no launch, and no error from one."""
+    from deepep_efa_b200 import _ext
+    from deepep_efa_b200.ops.permute import gather_reduce_rows, gather_rows
+    rows = torch.zeros(5, dtype=torch.int32, device="cuda")
+    pos = torch.zeros(5, 2, dtype=torch.int32, device="cuda")
+    empty = torch.empty(3, 0, dtype=torch.bfloat16, device="cuda")
+    assert gather_rows(empty, rows).shape == (5, 0) and gather_reduce_rows(empty, pos).shape == (5, 0)
+    out = torch.empty(5, 0, dtype=torch.bfloat16, device="cuda")
+    _ext.load().stage_reduce(torch.empty(10, 0, dtype=torch.bfloat16, device="cuda"), out, pos.long(), torch.ones(5, 2, device="cuda"), 4)
+    torch.cuda.synchronize()
