@@ -46,7 +46,7 @@ struct Runtime {
         std::shared_ptr<RuntimeCore> core;
         uint64_t off;
         cudaStream_t comm;
-        Block(std::shared_ptr<RuntimeCore> c, uint64_t bytes, cudaStream_t s) : core(std::move(c)), off(core->arena_alloc(bytes)), comm(s) {}
+        Block(std::shared_ptr<RuntimeCore> c, uint64_t at, cudaStream_t s) : core(std::move(c)), off(at), comm(s) {}
         Block(const Block&) = delete;
         ~Block() {
             cudaStream_t streams[2];
@@ -61,16 +61,27 @@ struct Runtime {
         }
     };
     using BlockPtr = std::shared_ptr<Block>;
-    BlockPtr alloc_block(uint64_t bytes) { return std::make_shared<Block>(core, bytes, comm_stream); }
-    torch::Tensor tensor_in(const BlockPtr& block, at::IntArrayRef sizes, torch::ScalarType dtype) {
-        return torch::from_blob(reinterpret_cast<char*>(core->base()) + block->off, sizes, [block](void*) {},
+    bool alloc_blocks(const uint64_t* bytes, int n, BlockPtr* blocks, uint64_t roomy = 0) {
+        uint64_t offs[8];
+        DX_CHECK(n <= 8, "at most 8 blocks at a time");
+        if (!core->arena_alloc(bytes, n, offs, roomy)) return false;
+        for (int i = 0; i < n; ++i) blocks[i] = std::make_shared<Block>(core, offs[i], comm_stream);
+        return true;
+    }
+    BlockPtr alloc_block(uint64_t bytes) {
+        BlockPtr b;
+        alloc_blocks(&bytes, 1, &b);
+        return b;
+    }
+    torch::Tensor tensor_in(const BlockPtr& block, uint64_t byte_off, at::IntArrayRef sizes, torch::ScalarType dtype) {
+        return torch::from_blob(reinterpret_cast<char*>(core->base()) + block->off + byte_off, sizes, [block](void*) {},
                                 torch::TensorOptions().dtype(dtype).device(torch::kCUDA, core->device()));
     }
 
     torch::Tensor alloc_symmetric(std::vector<int64_t> sizes, torch::ScalarType dtype) {
         int64_t numel = 1;
         for (auto s : sizes) numel *= s;
-        return tensor_in(alloc_block((uint64_t)numel * c10::elementSize(dtype)), sizes, dtype);
+        return tensor_in(alloc_block((uint64_t)numel * c10::elementSize(dtype)), 0, sizes, dtype);
     }
 
     // Offset of a tensor inside the symmetric buffer, or -1 when it lives elsewhere.
@@ -201,38 +212,51 @@ struct DispatchCall {
     torch::ScalarType out_type;
     bool has_scales = false;
     std::vector<int> per_expert;
-    // One block of the arena per output: some outlive the others (the source indices live on in the handle).
+    // Outputs with lives of their own (the source indices live on in the handle, the weights in a backward pass) are blocks of their
+    // own; the scales are in front of the rows they belong to.
     struct Out {
-        Runtime::BlockPtr block;
-        uint64_t row_bytes = 0;
+        uint64_t head_bytes = 0, row_bytes = 0;  // per row: what lies in front (of all rows), and the rows
         bool there = false;
-        uint64_t off() const { return there ? block->off : 0; }
+        Runtime::BlockPtr block;
+        uint64_t head_rows = 0;  // rows the front part was sized for
+        uint64_t bytes(int rows) const { return there ? front(rows) + (uint64_t)rows * row_bytes : 0; }
+        uint64_t front(uint64_t rows) const { return dxh::align_up(rows * head_bytes, 1024); }
+        uint64_t off() const { return there ? block->off + front(head_rows) : 0; }
     };
-    Out recv_x, recv_scales, recv_idx, recv_w, src_idx;
+    enum { kRecvX, kRecvIdx, kRecvW, kSrcIdx, kOuts };
+    Out outs[kOuts];
 
-    template <typename F>
-    void each_out(F f) {
-        for (Out* o : {&recv_x, &recv_scales, &recv_idx, &recv_w, &src_idx})
-            if (o->there) f(*o);
-    }
     void describe() {
-        recv_x = {nullptr, (uint64_t)H * c10::elementSize(out_type), true};
-        recv_scales = {nullptr, (uint64_t)(H / 128) * 4, has_scales};
-        recv_idx = {nullptr, (uint64_t)K * 8, topk_idx.has_value()};
-        recv_w = {nullptr, (uint64_t)K * 4, topk_w.has_value()};
-        src_idx = {nullptr, 4, true};
+        outs[kRecvX] = {has_scales ? (uint64_t)(H / 128) * 4 : 0, (uint64_t)H * c10::elementSize(out_type), true};
+        outs[kRecvIdx] = {0, (uint64_t)K * 8, topk_idx.has_value()};
+        outs[kRecvW] = {0, (uint64_t)K * 4, topk_w.has_value()};
+        outs[kSrcIdx] = {0, 4, true};
     }
-    void allocate(Runtime* rt, int rows) {
-        each_out([&](Out& o) { o.block = rt->alloc_block((uint64_t)rows * o.row_bytes); });
-    }
-    uint64_t bytes(int rows) {
-        uint64_t sum = 0;
-        each_out([&](Out& o) { sum += dxh::align_up((uint64_t)rows * o.row_bytes + 1, 1024); });
-        return sum;
+    // With `only_if_roomy`: only where they take at most a quarter of the largest free block.
+    bool allocate(Runtime* rt, int rows, bool only_if_roomy = false) {
+        uint64_t bytes[kOuts], sum = 0;
+        Out* of[kOuts];
+        int n = 0;
+        for (Out& o : outs)
+            if (o.there) {
+                of[n] = &o;
+                bytes[n] = o.bytes(rows);
+                sum += dxh::align_up(bytes[n] + 1, 1024);
+                ++n;
+            }
+        Runtime::BlockPtr blocks[kOuts];
+        if (!rt->alloc_blocks(bytes, n, blocks, only_if_roomy ? 4 * sum : 0)) return false;
+        for (int i = 0; i < n; ++i) {
+            of[i]->block = std::move(blocks[i]);
+            of[i]->head_rows = (uint64_t)rows;
+        }
+        return true;
     }
     // The kernel writes no row past the received ones, so the rest is as good as never allocated.
     void trim(Runtime* rt, int rows) {
-        each_out([&](Out& o) { rt->core->arena_shrink(o.block->off, (uint64_t)rows * o.row_bytes); });
+        for (Out& o : outs) {
+            if (o.there) rt->core->arena_shrink(o.block->off, o.front(o.head_rows) + (uint64_t)rows * o.row_bytes);
+        }
     }
 };
 
@@ -355,10 +379,7 @@ py::list normal_dispatch(std::vector<Runtime*> rts, const std::vector<py::tuple>
     for (int v = 0; v < V; ++v) {
         DispatchCall& q = calls[v];
         int rows = cached ? q.num_recv : num_worst_tokens;
-        if (exact && R == 1 && rts[v]->all_tokens_sent && 4 * q.bytes(q.T) <= rts[v]->core->arena_largest_free()) {
-            q.allocate(rts[v], q.T);
-            continue;
-        }
+        if (exact && R == 1 && rts[v]->all_tokens_sent && q.allocate(rts[v], q.T, true)) continue;
         if (exact) {
             order.leave();
             wait_counts(rts[v], q, E / R);
@@ -386,11 +407,11 @@ py::list normal_dispatch(std::vector<Runtime*> rts, const std::vector<py::tuple>
         a.hidden = q.H;
         a.num_experts = E;
         a.num_sms = num_sms;
-        a.recv_x_off = q.recv_x.off();
-        a.recv_scales_off = q.recv_scales.off();
-        a.recv_topk_idx_off = q.recv_idx.off();
-        a.recv_topk_w_off = q.recv_w.off();
-        a.recv_src_idx_off = q.src_idx.off();
+        a.recv_x_off = q.outs[DispatchCall::kRecvX].off();
+        a.recv_scales_off = q.has_scales ? q.outs[DispatchCall::kRecvX].block->off : 0;
+        a.recv_topk_idx_off = q.outs[DispatchCall::kRecvIdx].off();
+        a.recv_topk_w_off = q.outs[DispatchCall::kRecvW].off();
+        a.recv_src_idx_off = q.outs[DispatchCall::kSrcIdx].off();
         a.num_worst_tokens = num_worst_tokens;
     }
     order.enter();
@@ -403,16 +424,17 @@ py::list normal_dispatch(std::vector<Runtime*> rts, const std::vector<py::tuple>
         DispatchCall& q = calls[v];
         if (!waited) {
             wait_counts(rt, q, E / R);
-            q.trim(rt, q.num_recv);
+            if (q.num_recv < q.T) q.trim(rt, q.num_recv);
         }
         if (exact && R == 1) rt->all_tokens_sent = q.num_recv == q.T;
         const int64_t n = q.num_recv, H = q.H, K = q.K;
-        auto tensor = [&](const DispatchCall::Out& o, std::initializer_list<int64_t> sizes, torch::ScalarType dtype) -> py::object {
-            return o.there ? py::cast(rt->tensor_in(o.block, sizes, dtype)) : py::object(py::none());
+        auto tensor = [&](int which, std::initializer_list<int64_t> sizes, torch::ScalarType dtype, bool front = false) -> py::object {
+            const DispatchCall::Out& o = q.outs[which];
+            return o.there && (!front || q.has_scales) ? py::cast(rt->tensor_in(o.block, front ? 0 : o.front(o.head_rows), sizes, dtype)) : py::object(py::none());
         };
-        out.append(py::make_tuple(tensor(q.recv_x, {n, H}, q.out_type), tensor(q.recv_scales, {n, H / 128}, torch::kFloat32),
-                                  tensor(q.recv_idx, {n, K}, torch::kInt64), tensor(q.recv_w, {n, K}, torch::kFloat32), q.per_expert,
-                                  py::make_tuple(q.rpm, q.cpm, q.rcpm, tensor(q.src_idx, {n}, torch::kInt32), q.in_rank, q.send_head)));
+        out.append(py::make_tuple(tensor(DispatchCall::kRecvX, {n, H}, q.out_type), tensor(DispatchCall::kRecvX, {n, H / 128}, torch::kFloat32, true),
+                                  tensor(DispatchCall::kRecvIdx, {n, K}, torch::kInt64), tensor(DispatchCall::kRecvW, {n, K}, torch::kFloat32), q.per_expert,
+                                  py::make_tuple(q.rpm, q.cpm, q.rcpm, tensor(DispatchCall::kSrcIdx, {n}, torch::kInt32), q.in_rank, q.send_head)));
     }
     return out;
 }
@@ -460,7 +482,7 @@ py::list normal_combine(std::vector<Runtime*> rts, const std::vector<py::tuple>&
             const bool in_place = R == 1 && !rt->core->debug_checks() && tt.size(0) >= x.size(0) && (reinterpret_cast<uintptr_t>(tt.data_ptr()) & 15) == 0;
             if (off < 0 && !in_place) {
                 const uint64_t bytes = (uint64_t)tt.numel() * tt.element_size();
-                auto staged = rt->tensor_in(rt->alloc_block(bytes), tt.sizes(), tt.scalar_type());
+                auto staged = rt->tensor_in(rt->alloc_block(bytes), 0, tt.sizes(), tt.scalar_type());
                 DX_CUDA_CHECK(cudaMemcpyAsync(staged.data_ptr(), tt.data_ptr(), bytes, cudaMemcpyDeviceToDevice, order.stream));
                 off = rt->symmetric_offset(staged);
                 keep.push_back(staged);

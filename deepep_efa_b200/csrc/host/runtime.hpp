@@ -157,7 +157,7 @@ class RuntimeCore {
         released_ = true;
         cudaSetDevice(device_);
         cudaDeviceSynchronize();
-        drain_pending(true);
+        drain_pending(Drain::kWait);
         for (cudaEvent_t ev : event_pool_) cudaEventDestroy(ev);
         event_pool_.clear();
         order_ = capture_order_ = Order{};
@@ -190,33 +190,37 @@ class RuntimeCore {
     }
 
     // ---- arena ------------------------------------------------------------------------------
-    // Returns the offset of a fresh block. Blocks released earlier become reusable once the streams
-    // that may still touch them have passed the events recorded at release time.
-    uint64_t arena_alloc(uint64_t bytes) {
+    // Fresh blocks of the given sizes. Blocks released earlier become reusable once the streams that may still touch them have passed
+    // the events recorded at release time. With `roomy`, nothing happens and false is returned unless the largest free block is at
+    // least that large.
+    bool arena_alloc(const uint64_t* bytes, int n, uint64_t* offs, uint64_t roomy = 0) {
         std::lock_guard<std::mutex> g(mu_);
-        drain_pending(false);
-        int64_t off = arena_.alloc(bytes);
-        if (off < 0) {
-            drain_pending(true);
-            off = arena_.alloc(bytes);
-        }
-        if (off < 0) {
+        for (Drain how : {Drain::kFront, Drain::kAll, Drain::kWait}) {
+            drain_pending(how);
+            if (roomy > 0 && arena_.largest_free() < roomy) {
+                if (how == Drain::kFront) continue;
+                return false;
+            }
+            int i = 0;
+            for (; i < n; ++i) {
+                const int64_t off = arena_.alloc(bytes[i]);
+                if (off < 0) break;
+                offs[i] = (uint64_t)off;
+            }
+            if (i == n) return true;
+            const uint64_t need = bytes[i];
+            while (i-- > 0) arena_.free(offs[i]);
+            if (how != Drain::kWait) continue;
             char buf[512];
             std::snprintf(buf, sizeof(buf),
                           "symmetric arena exhausted: need %llu B, capacity %llu B, in use %llu B, largest free block %llu B. "
                           "Create the Buffer with a larger num_nvl_bytes (Config.get_nvl_buffer_size_hint) or drop references "
                           "to earlier dispatch results.",
-                          (unsigned long long)bytes, (unsigned long long)arena_.capacity(), (unsigned long long)arena_.in_use(),
+                          (unsigned long long)need, (unsigned long long)arena_.capacity(), (unsigned long long)arena_.in_use(),
                           (unsigned long long)arena_.largest_free());
             throw std::runtime_error(buf);
         }
-        return (uint64_t)off;
-    }
-
-    uint64_t arena_largest_free() {
-        std::lock_guard<std::mutex> g(mu_);
-        drain_pending(false);
-        return arena_.largest_free();
+        return false;
     }
 
     // Gives back the end of a block that nothing has used or will use.
@@ -430,7 +434,11 @@ class RuntimeCore {
         return ev;
     }
 
-    void drain_pending(bool wait) {
+    // kFront stops at the first release that has not passed: they pass nearly in order, and every look at an event costs the host more
+    // than the rest of an allocation.
+    enum class Drain { kFront, kAll, kWait };
+    void drain_pending(Drain how) {
+        const bool wait = how == Drain::kWait;
         for (auto it = pending_.begin(); it != pending_.end();) {
             auto passed = [&](cudaEvent_t ev) { return (wait ? cudaEventSynchronize(ev) : cudaEventQuery(ev)) != cudaErrorNotReady; };
             bool done = it->last_call == nullptr || passed(*it->last_call);
@@ -439,6 +447,8 @@ class RuntimeCore {
                 for (int i = 0; i < it->num_events; ++i) event_pool_.push_back(it->events[i]);
                 arena_.free(it->off);
                 it = pending_.erase(it);
+            } else if (how == Drain::kFront) {
+                break;
             } else {
                 ++it;
             }

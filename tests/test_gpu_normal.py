@@ -233,7 +233,7 @@ def test_handle_validation_catches_foreign_and_corrupt_handles():
 
 @pytest.mark.parametrize("mode", ["bf16", "fp8_fused"])
 def test_dispatch_holds_the_rows_that_arrived(mode):
-    """A lone rank whose tokens are mostly unselected: results hold as much symmetric memory as their rows, each tensor its own, up to
+    """A lone rank whose tokens are mostly unselected: results hold as much symmetric memory as their rows, the handle its own, up to
     where the arena could not hold a row per token."""
     vc = _cluster(1, nvl=24 << 20)
     try:
@@ -249,10 +249,12 @@ def test_dispatch_holds_the_rows_that_arrived(mode):
         per_rank, _, per_expert, in_rank, _ = buf.get_dispatch_layout(idx, E)
         base, held = buf.runtime.arena_in_use(), []
         fits = (buf.runtime.arena_capacity() - base) // each
-        for i in range(fits - 1):  # the last ones find no room for T rows
+        # FP8: the first result was laid out for T rows, with the scales in front, and is cut behind the rows that arrived
+        slack = up(T * H // 32) - up(rows * H // 32) if elem == 1 else 0
+        for i in range(fits - 3):  # the last ones find no room for T rows
             held.append(buf.dispatch(x, num_tokens_per_rank=per_rank, is_token_in_rank=in_rank, num_tokens_per_expert=per_expert, topk_idx=idx,
                                      topk_weights=w, quantize_fp8=elem == 1))
-            assert buf.runtime.arena_in_use() - base == (i + 1) * each
+            assert buf.runtime.arena_in_use() - base == (i + 1) * each + slack
         assert len(held) * each + T * H * elem > buf.runtime.arena_capacity()
         for recv, recv_idx, recv_w, _, _, _ in (held[0], held[-1]):
             assert torch.equal(recv_w, w[7::20]) and torch.equal(recv_idx, idx[7::20])
