@@ -160,3 +160,8 @@ def test_fused_dispatch_overflow_is_reported_not_written():
             b.runtime.clear_status()
     finally:
         vc.destroy()
+
+
+def test_expert_major_dispatch_with_many_experts_per_cta():
+    """More experts than a CTA lists in one pass over the ids (two emulated ranks share the SMs)."""
+    test_expert_major_dispatch_places_rows(2, 9, 128, 2048, 4, False)

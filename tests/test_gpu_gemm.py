@@ -506,3 +506,46 @@ def test_gathers_of_rows_without_columns():
     out = torch.empty(5, 0, dtype=torch.bfloat16, device="cuda")
     _ext.load().stage_reduce(torch.empty(10, 0, dtype=torch.bfloat16, device="cuda"), out, pos.long(), torch.ones(5, 2, device="cuda"), 4)
     torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("kind", ["bf16", "mx_wide"])
+def test_tile_counter_after_a_launch_that_gave_up(kind):
+    """An arrival gate that nobody opens ends in an error after its limit; the tile counter is zero again, and the next launch, whose
+    table is built early, is right."""
+    from deepep_efa_b200 import _ext
+    from deepep_efa_b200.ops.grouped_gemm import build_sf_atoms_a, build_sf_atoms_b
+    C = _ext.load()
+    C.gemm_clear_error(0)
+    torch.manual_seed(29)
+    counts, stride, K, N = [200, 0, 33, 128], 256, 512, 512
+    G = len(counts)
+    cnt = torch.tensor(counts, device="cuda", dtype=torch.int32)
+    starts = torch.arange(G + 1, device="cuda", dtype=torch.int32) * stride
+    live = (torch.arange(stride, device="cuda").unsqueeze(0) < cnt.unsqueeze(1)).view(-1)
+    x = torch.randn(G * stride, K, device="cuda").to(torch.bfloat16)
+    w = (torch.randn(G, N, K, device="cuda") * 0.1).to(torch.bfloat16)
+    scales = (None, None)
+    if kind == "mx_wide":
+        x, a_s = C.per_token_cast_to_fp8(x, True, False)
+        w = (w.float() / 2.0 ** -9).to(torch.float8_e4m3fn)
+        scales = (build_sf_atoms_a(a_s), build_sf_atoms_b(torch.full((G, N // 128, K // 128), 2.0 ** -9, device="cuda"), N, False, True))
+
+    def run(timeout_ms, **how):
+        out = torch.zeros(G * stride, N, device="cuda", dtype=torch.bfloat16)
+        C.grouped_gemm(x, w, starts, 0, False, None, None, out, 0, timeout_ms, cnt, *scales, m_ends_are_counts=True, **how)
+        return out
+
+    want = run(2000.0)
+    sched = torch.zeros(2, dtype=torch.int32, device="cuda")
+    ready, expected = torch.zeros(G, dtype=torch.int64, device="cuda"), torch.tensor([0, 0, 0, 1], dtype=torch.int64, device="cuda")
+    torch.cuda.synchronize()
+    for _ in range(2):
+        run(20.0, sched=sched, ready=ready, expected=expected)
+        torch.cuda.synchronize()
+        assert C.gemm_error(0) == 1 and sched.tolist() == [0, 0]
+        C.gemm_clear_error(0)
+        run(2000.0, sched=sched)
+        got = run(2000.0, sched=sched, early_table=True)
+        torch.cuda.synchronize()
+        assert C.gemm_error(0) == 0 and sched.tolist() == [0, 0]
+        assert torch.equal(got[live], want[live])

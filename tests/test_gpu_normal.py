@@ -344,3 +344,37 @@ def test_few_tokens_with_outputs_for_many_rows(R, worst):
             assert bool((a[1][n:] == -1).all())
     finally:
         vc.destroy()
+
+
+@pytest.mark.parametrize("T", [1, 2, 5, 37, 149])
+@pytest.mark.parametrize("H,mode", [(128, "fp8_fused"), (1152, "fp8_fused"), (7168, "fp8_fused"), (2048, "fp8_pair"), (8, "bf16"), (520, "bf16"), (7168, "bf16")])
+def test_small_batches_cut_rows_into_pieces(T, H, mode):
+    """A lone rank with fewer tokens than warps: rows are moved in pieces, down to one column each, with two biases on the way back."""
+    from deepep_efa_b200.reference import oracle
+    vc = _cluster(1, nvl=64 << 20)
+    try:
+        E, K = 8, 3
+        (x,), (idx,), (w,) = _inputs(1, T, H, E, K, masked=0.2, seed=T)
+        pair = oracle.per_token_cast_to_fp8(x.cpu()) if mode != "bf16" else None
+        send = x if mode != "fp8_pair" else (pair[0].cuda(), pair[1].cuda())
+        recv, recv_idx, recv_w, _, handle, _ = vc.dispatch([send], layouts=vc.get_dispatch_layout([idx], E), topk_idxs=[idx], topk_weights=[w],
+                                                           quantize_fp8=mode == "fp8_fused")[0]
+        sent = (idx >= 0).any(1)
+        assert torch.equal(recv_idx, idx[sent]) and torch.equal(recv_w, (w * (idx >= 0))[sent])
+        if mode == "bf16":
+            assert torch.equal(recv, x[sent])
+        else:
+            assert torch.equal(recv[0].cpu().view(torch.uint8), pair[0][sent.cpu()].view(torch.uint8)) and torch.equal(recv[1].cpu(), pair[1][sent.cpu()])
+        y, biases = make_tokens(int(sent.sum()), H, "cuda", seed=50), tuple(make_tokens(T, H, "cuda", seed=51 + i) for i in range(2))
+        want = torch.zeros(T, H, device="cuda")
+        want[sent] = y.float()
+        want = (want + biases[0].float() + biases[1].float()).to(torch.bfloat16)  # the kernel's order of sums
+        symmetric = vc.buffers[0].empty_symmetric(list(y.shape), torch.bfloat16)
+        symmetric.copy_(y)
+        shifted = torch.empty(y.numel() + 1, dtype=torch.bfloat16, device="cuda")[1:].view_as(y).copy_(y)  # not on 16 bytes: staged
+        strided = torch.stack([y, y], dim=1)[:, 0]
+        for given in (y, symmetric, shifted, strided):
+            assert torch.equal(vc.combine([given], [handle], biases=[biases])[0][0], want)
+        vc.buffers[0].check_status(sync=True)
+    finally:
+        vc.destroy()

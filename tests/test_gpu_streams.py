@@ -261,3 +261,37 @@ def test_fused_layers_of_one_buffer_on_two_streams():
             assert all(torch.equal(g, want[i % 2]) for i, g in enumerate(got))
     finally:
         vc.destroy()
+
+
+def test_calls_that_alternate_between_streams():
+    """Direct calls on two streams and asynchronous ones on the communication stream, the host never waiting in between."""
+    vc, buf = _buffer()
+    try:
+        sets = []
+        for i, n in enumerate((300, 4000, 37)):
+            idx, w = make_routing(n, E, K, "cuda", seed=30 + i, masked_fraction=0.2)
+            x = make_tokens(n, H, "cuda", seed=30 + i)
+            want = x.float() * (idx >= 0).any(1, keepdim=True)
+            sets.append((x, idx, w, want.to(torch.bfloat16)))
+        side = torch.cuda.Stream()
+        torch.cuda.synchronize()
+        got = []
+        for step in range(30):
+            x, idx, w, want = sets[step % 3]
+            how = dict(async_finish=True) if step % 4 in (1, 2) else {}
+            with torch.cuda.stream(side if step % 5 == 3 else torch.cuda.default_stream()):
+                lay, ev = _layout(buf, idx, **how)
+                ev.current_stream_wait()
+                y, _, rw, _, handle, ev = buf.dispatch(x, topk_weights=w, **lay, **how)
+                ev.current_stream_wait()
+                how = dict(async_finish=True) if step % 4 in (2, 3) else {}
+                out, out_w, ev = buf.combine(y, handle, topk_weights=rw, **how)
+                ev.current_stream_wait()
+                got.append((out, out_w, want, w * (idx >= 0)))
+            del lay, handle, y, rw
+        torch.cuda.synchronize()
+        buf.check_status(sync=True)
+        for out, out_w, want, want_w in got:
+            assert torch.equal(out, want) and torch.equal(out_w, want_w)
+    finally:
+        vc.destroy()
