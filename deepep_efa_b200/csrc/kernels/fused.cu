@@ -1,9 +1,9 @@
 // Expert-major dispatch for the fused MoE layer: rows land at the receiver already grouped by expert, 128-row
 // aligned, in the order the grouped GEMM consumes them, and the GEMM starts on an expert as soon as its rows are in.
 //
-//   em_notify   every rank histograms its selections per GLOBAL expert (one warp per expert, rows of an expert keep
-//               token order), all-gathers the E counts (+ the offsets of its receive buffers) with one release flag
-//               per peer, and derives from the R x E matrix everything the layer needs without a host round trip:
+//   em_notify   every rank lists its selections per GLOBAL expert (a CTA votes over all of them for its share of the experts;
+//               rows of an expert keep token order), all-gathers the E counts (+ the offsets of its receive buffers) with one
+//               release flag per peer, and derives from the R x E matrix everything the layer needs without a host round trip:
 //               where each of its (token, expert) rows goes, the group offsets of its own experts, and how many rows
 //               each of its experts will receive (added to a monotonic expectation that the GEMM compares with the
 //               arrival counter).
@@ -27,8 +27,6 @@
 
 namespace dx {
 
-// One warp per expert scans all selections, so the scan's length is fixed; what varies is how many such warps share an SM's four
-// schedulers. Four warps per CTA (64 CTAs for 256 experts) give every scanning warp a scheduler of its own.
 constexpr int kEmNotifyThreads = kScanThreads;
 constexpr int kEmNotifyWarps = kEmNotifyThreads / 32;
 constexpr int kTicketFused = 5;

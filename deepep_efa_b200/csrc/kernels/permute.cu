@@ -1,11 +1,13 @@
 // Row gather kernels that move dispatch results into the expert-major, 128-row-aligned layout the grouped
 // GEMM wants, and back (weighted) into receive order for combine.
 //
+//   build_plan:           the maps between the two orders, in one launch
 //   gather_rows:          dst[m] = scale[m] * src[src_row[m]]            (src_row < 0 -> zero row)
 //   gather_reduce_rows:   dst[n] = sum_k w[n,k] * src[pos[n,k]]          (pos < 0 skipped), fp32 accumulate
 //
-// Both are pure bandwidth kernels: one warp per output row, 16-byte accesses, no atomics. They are each
-// other's backward pass, so training needs nothing else.
+// The gathers are pure bandwidth kernels: a warp per span of columns of an output row, 16-byte accesses, no atomics. The
+// unweighted ones are each other's backward pass; that of the weighted sum is unpermute_bwd in train_ops.cu, which reads each
+// row once for both of its gradients.
 //
 // The reference has no counterpart: its users permute with framework indexing ops between dispatch and
 // their expert GEMMs.

@@ -392,10 +392,14 @@ def fused_forward_many(layers, xs, idxs, ws, overlap: bool = True, num_dispatch_
     """Fused FP8 forward of one MoE layer on every given rank (one entry per rank: a single entry in a real job, one per
     emulated rank on a single GPU, where the collectives run as one cooperative launch each and nothing overlaps).
 
-    Streams: the count exchange and the dispatch run on the buffer's communication stream; the expert GEMMs run on the
+    Streams, with peers: the count exchange and the dispatch run on the buffer's communication stream; the expert GEMMs run on the
     caller's stream as soon as the exchange is done, concurrently with the dispatch, and gate every expert on its arrival
-    counter. The dispatch kernel is launched first and never waits for the GEMM, so the pair cannot deadlock; its small
-    CTAs share the SMs with the GEMM's persistent CTAs."""
+    counter. The dispatch kernel never waits for the GEMM, and the parts of the first GEMM that may have to wait for rows leave it
+    SMs of its own. A lone rank, the emulated ranks and ``overlap=False`` run everything on the caller's stream, one kernel after
+    the other.
+
+    Calls of one buffer keep their order whatever streams they come from (the exchange and the dispatch wait for the previous
+    call's); the workspace belongs to the layer, so one layer is called on one stream at a time."""
     V = len(layers)
     l0 = layers[0]
     C = l0._C()
