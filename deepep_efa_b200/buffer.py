@@ -131,7 +131,7 @@ class Buffer:
                 use_fabric, True, enable_shrink, timeout_ms=timeout_ms, num_nvl_ranks=nvl))
             nb = self._hier.node_buf
             if nb._cpu is None:
-                self._C, self.device, self.comm_stream = nb._C, nb.device, nb.comm_stream
+                self._C, self.device, self._comm_stream = nb._C, nb.device, nb.comm_stream
             return
 
         if not torch.cuda.is_available():
@@ -146,8 +146,8 @@ class Buffer:
         self.device = torch.device("cuda", device)
         self.runtime = self._C.Runtime(self.rank, self.group_size, self.num_nvl_bytes, self.num_rdma_bytes, device,
                                        timeout_ms if timeout_ms is not None else _env_timeout_ms(), bool(enable_shrink))
-        self.comm_stream = torch.cuda.Stream(device=self.device, priority=-1)
-        self.runtime.set_comm_stream(self.comm_stream.cuda_stream)
+        self._comm_stream = torch.cuda.Stream(device=self.device, priority=-1)
+        self.runtime.set_comm_stream(self._comm_stream.cuda_stream)
         if _virtual is None:
             from .utils.nvlink import check_nvlink_connections
             check_nvlink_connections(group)
@@ -249,6 +249,14 @@ class Buffer:
         if self._hier is not None:
             return self._hier.node_buf.get_local_ipc_handle()
         return bytes(self.runtime.ipc_handle())
+
+    @property
+    def comm_stream(self) -> "torch.cuda.Stream":
+        """The stream of the asynchronous calls. Whoever asks for it may run work of their own there, which every later release of
+        symmetric memory then waits for as well."""
+        if self.runtime is not None:
+            self.runtime.share_comm_stream()
+        return self._comm_stream
 
     def get_comm_stream(self) -> "torch.cuda.Stream":
         return self.comm_stream
@@ -687,7 +695,7 @@ class _CommScope:
         if self.direct:
             return self
         self.compute = torch.cuda.current_stream()
-        comm = self.buf.comm_stream
+        comm = self.buf._comm_stream
         if self.prev is not None and self.prev.event is not None and self.prev.event.event is not None:
             comm.wait_event(self.prev.event.event)
         else:
@@ -699,7 +707,7 @@ class _CommScope:
     def __exit__(self, et, ev, tb):
         if self.direct:
             return False
-        comm = self.buf.comm_stream
+        comm = self.buf._comm_stream
         self._ctx.__exit__(et, ev, tb)
         if et is not None:
             return False

@@ -56,7 +56,7 @@ struct Runtime {
                 ++n;
             } catch (...) {
             }
-            if (comm != nullptr) streams[n++] = comm;
+            if (comm != nullptr && core->comm_stream_shared()) streams[n++] = comm;
             core->arena_release(off, streams, n);
         }
     };
@@ -813,6 +813,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         .def("ipc_handle", &Runtime::ipc_handle)
         .def("open_peers", &Runtime::open_peers)
         .def("set_comm_stream", &Runtime::set_comm_stream)
+        .def("share_comm_stream", [](Runtime& r) { r.core->share_comm_stream(); })
         .def("alloc_symmetric", &Runtime::alloc_symmetric)
         .def("symmetric_offset", &Runtime::symmetric_offset)
         .def("view", &Runtime::view)

@@ -158,9 +158,9 @@ class RuntimeCore {
         cudaSetDevice(device_);
         cudaDeviceSynchronize();
         drain_pending(Drain::kWait);
+        order_ = capture_order_ = Order{};
         for (cudaEvent_t ev : event_pool_) cudaEventDestroy(ev);
         event_pool_.clear();
-        order_ = capture_order_ = Order{};
         for (int r = 0; r < num_ranks_; ++r)
             if (ipc_opened_[r]) cudaIpcCloseMemHandle(peers_[r]);
         if (base_) cudaFree(base_);
@@ -278,14 +278,23 @@ class RuntimeCore {
         Order* o = order_of(s, &id);
         if (o == nullptr) return;
         if (o->event == nullptr || o->event.use_count() > 1) {  // a block released meanwhile waits for that call, not for this one
-            auto fresh = std::make_shared<OwnedEvent>();
-            o->event = fresh->ev != nullptr ? std::shared_ptr<cudaEvent_t>(fresh, &fresh->ev) : nullptr;
+            const cudaEvent_t ev = take_event();
+            o->event = ev == nullptr ? nullptr : std::shared_ptr<cudaEvent_t>(new cudaEvent_t(ev), [this](cudaEvent_t* e) {
+                event_pool_.push_back(*e);  // (under mu_, like every use of these pointers)
+                delete e;
+            });
         }
         if (o->event != nullptr) cudaEventRecord(*o->event, s);
+        else comm_shared_ = true;
         o->stream = s;
         o->capture = id;
         cudaGetLastError();
     }
+
+    // The communication stream runs ordered calls, which a release waits for by their event. Once it is shared (a caller has asked for it,
+    // or other kernels of this library run there) a release records an event of its own on it.
+    void share_comm_stream() { comm_shared_ = true; }
+    bool comm_stream_shared() const { return comm_shared_; }
 
     bool in_symmetric(const void* p, uint64_t bytes, uint64_t* off) const {
         const char* b = reinterpret_cast<const char*>(base_);
@@ -396,16 +405,6 @@ class RuntimeCore {
         std::shared_ptr<cudaEvent_t> last_call;  // of the ordered calls, where the events do not cover it
     };
 
-    struct OwnedEvent {
-        cudaEvent_t ev = nullptr;
-        OwnedEvent() {
-            if (cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess) ev = nullptr;
-        }
-        OwnedEvent(const OwnedEvent&) = delete;
-        ~OwnedEvent() {
-            if (ev != nullptr) cudaEventDestroy(ev);
-        }
-    };
     struct Order {
         std::shared_ptr<cudaEvent_t> event;  // end of the last call, recorded on `stream`
         cudaStream_t stream = nullptr;
@@ -479,6 +478,7 @@ class RuntimeCore {
     std::deque<Pending> pending_;
     std::vector<cudaEvent_t> event_pool_;  // bounded by the number of blocks that were ever pending at once
     Order order_, capture_order_;
+    std::atomic<bool> comm_shared_{false};
     std::mutex mu_;
 };
 

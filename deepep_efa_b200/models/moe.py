@@ -419,7 +419,7 @@ def fused_forward_many(layers, xs, idxs, ws, overlap: bool = True, num_dispatch_
     # a lone rank's rows never leave its memory: the dispatch is a copy at HBM speed, short when it has the GPU to itself, and a GEMM
     # beside it would only give up SMs for it
     lone = bufs[0].group_size == 1
-    comm = bufs[0].comm_stream if (V == 1 and overlap and not lone) else cur
+    comm = bufs[0]._comm_stream if (V == 1 and overlap and not lone) else cur
     if comm is not cur:
         comm.wait_stream(cur)
     # the quantisation of x (caller's stream) and the count exchange (communication stream) do not depend on each other: side by side

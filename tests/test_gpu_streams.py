@@ -295,3 +295,44 @@ def test_calls_that_alternate_between_streams():
             assert torch.equal(out, want) and torch.equal(out_w, want_w)
     finally:
         vc.destroy()
+
+
+@pytest.mark.parametrize("how", ["asynchronous", "own_work"])
+def test_symmetric_memory_dropped_while_the_communication_stream_uses_it(how):
+    """By an asynchronous call of the library, or by work of the caller who asked for the stream."""
+    vc, buf = _buffer(nvl=64 << 20)
+    try:
+        idx, _ = make_routing(T, E, K, "cuda", seed=40)
+        x = make_tokens(T, H, "cuda", seed=40)
+        lay, _ = _layout(buf, idx)
+        y, _, _, _, handle, _ = buf.dispatch(x, **lay)
+        late = buf.empty_symmetric([T, H], torch.bfloat16)
+        late.copy_(y)
+        want, late_at = buf.combine(late, handle)[0].clone(), late.data_ptr()
+        start = torch.cuda.Event()
+        side = torch.cuda.Stream()
+        torch.cuda.synchronize()
+        _delay(side)
+        start.record(side)
+        if how == "asynchronous":  # (without asking for the stream)
+            from deepep_efa_b200 import EventOverlap
+            from deepep_efa_b200.utils.event import EventHandle
+            handle_of_side = EventHandle(record=False)
+            handle_of_side.event = start
+            out, _, ev = buf.combine(late, handle, previous_event=EventOverlap(handle_of_side), async_finish=True)
+        else:
+            out, ev = torch.empty_like(want), None
+            buf.comm_stream.wait_event(start)
+            with torch.cuda.stream(buf.comm_stream):
+                out.copy_(late)
+            want = y.clone()
+        del late
+        if ev is not None:
+            ev.extra_tensors = ()
+        fresh = [buf.empty_symmetric([T, H], torch.bfloat16).fill_(3.0) for _ in range(4)]
+        assert late_at not in [f.data_ptr() for f in fresh]
+        torch.cuda.synchronize()
+        buf.check_status()
+        assert torch.equal(out, want)
+    finally:
+        vc.destroy()
