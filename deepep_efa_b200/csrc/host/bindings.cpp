@@ -347,7 +347,7 @@ py::list normal_dispatch(std::vector<Runtime*> rts, const std::vector<py::tuple>
         q.cpm = torch::empty({R, num_channels}, i32);
         q.rcpm = torch::empty({R, num_channels}, i32);
         q.send_head = torch::empty({T, R}, i32);
-        rt->core->reset_recv_counters(E / R);
+        if (num_worst_tokens == 0) rt->core->reset_recv_counters(E / R);
         dx::NotifyArgs& a = nargs[v];
         a.ctx = rt->core->ctx();
         a.num_tokens_per_rank = ntpr.data_ptr<int>();
@@ -361,9 +361,10 @@ py::list normal_dispatch(std::vector<Runtime*> rts, const std::vector<py::tuple>
         a.channel_prefix_matrix = q.cpm.data_ptr<int>();
         a.recv_channel_prefix_matrix = q.rcpm.data_ptr<int>();
         a.send_head = q.send_head.data_ptr<int>();
+        // A call whose host does not wait must not publish: its words could land after a later call has reset them.
         dxh::HostWords* hw = reinterpret_cast<dxh::HostWords*>(a.ctx.status);  // status is the first member
-        a.host_recv_counter = &hw->recv_counter;
-        a.host_expert_counter = hw->expert_counter;
+        a.host_recv_counter = num_worst_tokens > 0 ? nullptr : &hw->recv_counter;
+        a.host_expert_counter = num_worst_tokens > 0 ? nullptr : hw->expert_counter;
     }
     if (!cached) {
         order.enter();

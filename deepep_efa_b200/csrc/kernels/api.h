@@ -46,7 +46,7 @@ struct NotifyArgs {
     int* channel_prefix_matrix;         // [R,C] out
     int* recv_channel_prefix_matrix;    // [R,C] out
     int* send_head;                     // [T,R] out: position inside the (me -> r) stream or -1
-    volatile int* host_recv_counter;    // mapped host: total rows I will receive
+    volatile int* host_recv_counter;    // mapped host: total rows I will receive (both null when the host does not wait for them)
     volatile int* host_expert_counter;  // mapped host [L]: rows per local expert (aligned)
 };
 cudaError_t launch_notify(const NotifyArgs* a, int num_virtual, cudaStream_t stream);

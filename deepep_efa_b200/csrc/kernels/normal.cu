@@ -70,7 +70,7 @@ __global__ void __launch_bounds__(kNotifyThreads, 1) notify_kernel(const __grid_
         }
         __syncthreads();
         if (!s_ok) {
-            if (tid == 0) {
+            if (tid == 0 && a.host_recv_counter != nullptr) {
                 *a.host_recv_counter = -2;  // tells the host to stop waiting
                 __threadfence_system();
             }
@@ -83,9 +83,9 @@ __global__ void __launch_bounds__(kNotifyThreads, 1) notify_kernel(const __grid_
                 running += ld_relaxed_sys(&my->notify_rank_counts[i][tid]);
                 a.rank_prefix_matrix[i * R + tid] = running;
             }
-            if (tid == me) *a.host_recv_counter = running;
+            if (tid == me && a.host_recv_counter != nullptr) *a.host_recv_counter = running;
         }
-        for (int e = tid; e < L; e += kNotifyThreads) {
+        for (int e = tid; e < L && a.host_expert_counter != nullptr; e += kNotifyThreads) {
             int sum = 0;
             for (int i = 0; i < R; ++i) sum += ld_relaxed_sys(&my->notify_expert_counts[i][e]);
             const int al = a.expert_alignment;

@@ -336,3 +336,22 @@ def test_symmetric_memory_dropped_while_the_communication_stream_uses_it(how):
         assert torch.equal(out, want)
     finally:
         vc.destroy()
+
+
+def test_counts_of_a_call_that_did_not_wait_do_not_reach_the_next_one():
+    """A dispatch with num_worst_tokens is still queued when the next dispatch waits on the host for its own, larger counts."""
+    vc, buf = _buffer()
+    try:
+        sets = [(make_tokens(n, H, "cuda", seed=50 + n), make_routing(n, E, K, "cuda", seed=50 + n)[0]) for n in (20, 300)]
+        lays = [_layout(buf, idx)[0] for _, idx in sets]
+        want = buf.dispatch(sets[1][0], **lays[1])[3]
+        torch.cuda.synchronize()
+        _delay(torch.cuda.current_stream())
+        few = buf.dispatch(sets[0][0], num_worst_tokens=64, **lays[0])
+        many = buf.dispatch(sets[1][0], **lays[1])
+        torch.cuda.synchronize()
+        buf.check_status()
+        assert torch.equal(many[0], sets[1][0]) and many[3] == want
+        assert torch.equal(few[0][:20], sets[0][0]) and few[3] == []
+    finally:
+        vc.destroy()
