@@ -173,12 +173,21 @@ std::tuple<torch::Tensor, torch::Tensor, torch::Tensor> get_dispatch_layout(Runt
     auto per_rank = torch::empty({R}, i32), per_expert = torch::empty({num_experts}, i32);
     auto in_rank = torch::empty({T, R}, i32.dtype(torch::kBool));
     // The scratch belongs to whichever call runs: it is replaced only behind the previous one, and marked on the stream that uses it,
-    // so that an outgrown one is not handed out while a call on another stream is still to use it.
+    // so that an outgrown one is not handed out while a call on another stream is still to use it. A captured call has one of its own
+    // in the graph's memory: the shared one may be outgrown by the time of a replay.
     dxh::OrderedCall order = ordered_call({rt});
     order.enter();
     const int64_t need = (int64_t)dx::layout_scratch_ints(num_experts, R, T);
-    if (!rt->layout_scratch.defined() || rt->layout_scratch.numel() < need) rt->layout_scratch = torch::zeros({need}, i32);
-    used_here(rt->layout_scratch);
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    DX_CUDA_CHECK(cudaStreamIsCapturing(order.stream, &capture));
+    torch::Tensor scratch;
+    if (capture != cudaStreamCaptureStatusNone) {
+        scratch = torch::zeros({need}, i32);
+    } else {
+        if (!rt->layout_scratch.defined() || rt->layout_scratch.numel() < need) rt->layout_scratch = torch::zeros({need}, i32);
+        scratch = rt->layout_scratch;
+        used_here(scratch);
+    }
     dx::LayoutArgs a{};
     a.topk_idx = topk_idx.data_ptr<int64_t>();
     a.num_tokens = T;
@@ -188,7 +197,7 @@ std::tuple<torch::Tensor, torch::Tensor, torch::Tensor> get_dispatch_layout(Runt
     a.num_tokens_per_rank = per_rank.data_ptr<int>();
     a.num_tokens_per_expert = per_expert.data_ptr<int>();
     a.is_token_in_rank = in_rank.data_ptr<bool>();
-    a.scratch = rt->layout_scratch.data_ptr<int>();
+    a.scratch = scratch.data_ptr<int>();
     check_launch(dx::launch_layout(a, order.stream), "get_dispatch_layout");
     return {per_rank, per_expert, in_rank};
 }

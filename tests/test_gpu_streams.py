@@ -355,3 +355,28 @@ def test_counts_of_a_call_that_did_not_wait_do_not_reach_the_next_one():
         assert torch.equal(few[0][:20], sets[0][0]) and few[3] == []
     finally:
         vc.destroy()
+
+
+@pytest.mark.parametrize("warm", [False, True])
+def test_captured_layout_replayed_after_larger_ones(warm):
+    """A captured layout keeps scratch memory of its own, whether the buffer had some before or needs more later."""
+    vc, buf = _buffer()
+    try:
+        small, large = (make_routing(n, E, K, "cuda", seed=n)[0] for n in (5000, 40000))
+        want = [torch.bincount(i.flatten(), minlength=E) for i in (small, large)]
+        if warm:
+            _layout(buf, small)
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            captured = _layout(buf, small)[0]["num_tokens_per_expert"]
+        for _ in range(3):
+            eager = _layout(buf, large)[0]["num_tokens_per_expert"]
+            keep = [torch.full((n,), 7, dtype=torch.int32, device="cuda") for n in (512, 1024, 2048, 4096) for _ in range(8)]
+            captured.zero_()
+            graph.replay()
+            torch.cuda.synchronize()
+            assert torch.equal(captured.long(), want[0]) and torch.equal(eager.long(), want[1])
+            assert all(bool((t == 7).all()) for t in keep)
+    finally:
+        vc.destroy()
