@@ -179,7 +179,10 @@ std::tuple<torch::Tensor, torch::Tensor, torch::Tensor> get_dispatch_layout(Runt
     order.enter();
     const int64_t need = (int64_t)dx::layout_scratch_ints(num_experts, R, T);
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    DX_CUDA_CHECK(cudaStreamIsCapturing(order.stream, &capture));
+    if (cudaStreamIsCapturing(order.stream, &capture) != cudaSuccess) {
+        cudaGetLastError();  // (the default stream while another one captures: not a captured call)
+        capture = cudaStreamCaptureStatusNone;
+    }
     torch::Tensor scratch;
     if (capture != cudaStreamCaptureStatusNone) {
         scratch = torch::zeros({need}, i32);
