@@ -154,12 +154,6 @@ void used_here(const torch::Tensor& t) {
     if (t.is_cuda()) c10::cuda::CUDACachingAllocator::recordStream(t.storage().data_ptr(), c10::cuda::getCurrentCUDAStream(t.get_device()));
 }
 
-dxh::OrderedCall ordered_call(const std::vector<Runtime*>& rts) {
-    std::vector<RuntimeCore*> cores;
-    for (Runtime* rt : rts) cores.push_back(rt->core.get());
-    return dxh::OrderedCall(std::move(cores), cur_stream(rts[0]));
-}
-
 // ---------------------------------------------------------------------------------------------
 // layout
 // ---------------------------------------------------------------------------------------------
@@ -175,16 +169,12 @@ std::tuple<torch::Tensor, torch::Tensor, torch::Tensor> get_dispatch_layout(Runt
     // The scratch belongs to whichever call runs: it is replaced only behind the previous one, and marked on the stream that uses it,
     // so that an outgrown one is not handed out while a call on another stream is still to use it. A captured call has one of its own
     // in the graph's memory: the shared one may be outgrown by the time of a replay.
-    dxh::OrderedCall order = ordered_call({rt});
+    dxh::OrderedCall order(cur_stream(rt));
+    order.add(rt->core.get());
     order.enter();
     const int64_t need = (int64_t)dx::layout_scratch_ints(num_experts, R, T);
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(order.stream, &capture) != cudaSuccess) {
-        cudaGetLastError();  // (the default stream while another one captures: not a captured call)
-        capture = cudaStreamCaptureStatusNone;
-    }
     torch::Tensor scratch;
-    if (capture != cudaStreamCaptureStatusNone) {
+    if (order.captured()) {
         scratch = torch::zeros({need}, i32);
     } else {
         if (!rt->layout_scratch.defined() || rt->layout_scratch.numel() < need) rt->layout_scratch = torch::zeros({need}, i32);
@@ -290,7 +280,8 @@ py::list normal_dispatch(std::vector<Runtime*> rts, const std::vector<py::tuple>
     std::vector<DispatchCall> calls(V);
     std::vector<dx::NotifyArgs> nargs(V);
     std::vector<dx::DispatchArgs> dargs(V);
-    dxh::OrderedCall order = ordered_call(rts);
+    dxh::OrderedCall order(cur_stream(rts[0]));
+    for (Runtime* rt : rts) order.add(rt->core.get());
     bool cached = false;
     int E = R;  // a cached call carries no expert ids to remap
     for (int v = 0; v < V; ++v) {
@@ -464,7 +455,8 @@ py::list normal_combine(std::vector<Runtime*> rts, const std::vector<py::tuple>&
     std::vector<dx::CombineArgs> args(V);
     std::vector<torch::Tensor> keep;
     py::list results;
-    dxh::OrderedCall order = ordered_call(rts);
+    dxh::OrderedCall order(cur_stream(rts[0]));
+    for (Runtime* rt : rts) order.add(rt->core.get());
     for (int v = 0; v < V; ++v) {
         Runtime* rt = rts[v];
         const py::tuple& t = per_rank[v];

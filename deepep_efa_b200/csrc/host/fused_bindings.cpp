@@ -49,12 +49,12 @@ void em_notify(std::vector<py::object> rts, std::vector<py::tuple> per_rank, int
     const int V = (int)rts.size();
     DXF_CHECK(V >= 1 && V <= dx::kMaxVirtualRanks && (int)per_rank.size() == V, "em_notify: one entry per rank");
     std::vector<dx::EmNotifyArgs> args(V);
-    std::vector<dxh::RuntimeCore*> cores;
     dxh::RuntimeCore* core0 = dx_core_of(rts[0]);
     c10::cuda::CUDAGuard guard(core0->device());
+    dxh::OrderedCall order(at::cuda::getCurrentCUDAStream(core0->device()).stream());
     for (int v = 0; v < V; ++v) {
         dxh::RuntimeCore* core = dx_core_of(rts[v]);
-        cores.push_back(core);
+        order.add(core);
         const py::tuple& t = per_rank[v];
         DXF_CHECK(t.size() == 12, "em_notify: per-rank tuple must have 12 entries");
         auto topk_idx = t[0].cast<torch::Tensor>();
@@ -106,7 +106,6 @@ void em_notify(std::vector<py::object> rts, std::vector<py::tuple> per_rank, int
         a.m_ends = m_ends.data_ptr<int>();
         a.peer_bases = reinterpret_cast<uint64_t*>(peer_bases.data_ptr());
     }
-    dxh::OrderedCall order(std::move(cores), at::cuda::getCurrentCUDAStream(core0->device()).stream());
     order.enter();
     check(dx::launch_em_notify(args.data(), V, order.stream), "em_notify");
 }
@@ -119,12 +118,12 @@ void em_dispatch(std::vector<py::object> rts, std::vector<py::tuple> per_rank, i
     DXF_CHECK(V >= 1 && V <= dx::kMaxVirtualRanks && (int)per_rank.size() == V, "em_dispatch: one entry per rank");
     DXF_CHECK(num_sms >= 1 && unit_rows >= 1, "num_sms and unit_rows must be positive");
     std::vector<dx::EmDispatchArgs> args(V);
-    std::vector<dxh::RuntimeCore*> cores;
     dxh::RuntimeCore* core0 = dx_core_of(rts[0]);
     c10::cuda::CUDAGuard guard(core0->device());
+    dxh::OrderedCall order(at::cuda::getCurrentCUDAStream(core0->device()).stream());
     for (int v = 0; v < V; ++v) {
         dxh::RuntimeCore* core = dx_core_of(rts[v]);
-        cores.push_back(core);
+        order.add(core);
         const py::tuple& t = per_rank[v];
         DXF_CHECK(t.size() == 9, "em_dispatch: per-rank tuple must have 9 entries");
         auto x = t[0].cast<torch::Tensor>();
@@ -179,7 +178,6 @@ void em_dispatch(std::vector<py::object> rts, std::vector<py::tuple> per_rank, i
         }
         a.num_sms = num_sms;
     }
-    dxh::OrderedCall order(std::move(cores), at::cuda::getCurrentCUDAStream(core0->device()).stream());
     order.enter();
     check(dx::launch_em_dispatch(args.data(), V, order.stream), "em_dispatch");
 }

@@ -266,16 +266,22 @@ class RuntimeCore {
     // nothing in between that lets another host thread in (a wait for the GPU): a call that waits leaves before it does.
     // Calls under stream capture are ordered among those of the same capture. With calls outside of it they are not: an event
     // from outside may not be waited for there, and the graph's owner orders its replays.
-    void order_enter(cudaStream_t s) {
+    struct Order;
+    struct Place {  // of one call, from enter to leave
+        Order* order = nullptr;
+        unsigned long long capture = 0;
+        bool captured = false;
+    };
+    Place order_enter(cudaStream_t s) {
         std::lock_guard<std::mutex> g(mu_);
-        unsigned long long id = 0;
-        Order* o = order_of(s, &id);
-        if (o != nullptr && o->event != nullptr && o->capture == id && o->stream != s) DX_CUDA_CHECK(cudaStreamWaitEvent(s, *o->event, 0));
+        const Place at = place_of(s);
+        const Order* o = at.order;
+        if (o != nullptr && o->event != nullptr && o->capture == at.capture && o->stream != s) DX_CUDA_CHECK(cudaStreamWaitEvent(s, *o->event, 0));
+        return at;
     }
-    void order_leave(cudaStream_t s) {
+    void order_leave(cudaStream_t s, const Place& at) {
         std::lock_guard<std::mutex> g(mu_);
-        unsigned long long id = 0;
-        Order* o = order_of(s, &id);
+        Order* o = at.order;
         if (o == nullptr) return;
         if (o->event == nullptr || o->event.use_count() > 1) {  // a block released meanwhile waits for that call, not for this one
             const cudaEvent_t ev = take_event();
@@ -287,9 +293,14 @@ class RuntimeCore {
         if (o->event != nullptr) cudaEventRecord(*o->event, s);
         else comm_shared_ = true;
         o->stream = s;
-        o->capture = id;
+        o->capture = at.capture;
         cudaGetLastError();
     }
+    struct Order {
+        std::shared_ptr<cudaEvent_t> event;  // end of the last call, recorded on `stream`
+        cudaStream_t stream = nullptr;
+        unsigned long long capture = 0;  // the capture it belongs to, 0 = none
+    };
 
     // The communication stream runs ordered calls, which a release waits for by their event. Once it is shared (a caller has asked for it,
     // or other kernels of this library run there) a release records an event of its own on it.
@@ -405,21 +416,15 @@ class RuntimeCore {
         std::shared_ptr<cudaEvent_t> last_call;  // of the ordered calls, where the events do not cover it
     };
 
-    struct Order {
-        std::shared_ptr<cudaEvent_t> event;  // end of the last call, recorded on `stream`
-        cudaStream_t stream = nullptr;
-        unsigned long long capture = 0;  // the capture it belongs to, 0 = none
-    };
-    // What a call on `s` is ordered by; nullptr when the driver will not say (the default stream while another stream captures).
-    Order* order_of(cudaStream_t s, unsigned long long* capture) {
+    // What a call on `s` is ordered by; nothing when the driver will not say (the default stream while another stream captures).
+    Place place_of(cudaStream_t s) {
+        Place at;
         cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-        if (cudaStreamGetCaptureInfo(s, &st, capture) != cudaSuccess || st == cudaStreamCaptureStatusInvalidated) {
-            cudaGetLastError();
-            return nullptr;
-        }
-        if (st == cudaStreamCaptureStatusActive) return &capture_order_;
-        *capture = 0;
-        return &order_;
+        if (cudaStreamIsCapturing(s, &st) != cudaSuccess) cudaGetLastError();
+        else if (st == cudaStreamCaptureStatusNone) at.order = &order_;
+        else if (cudaStreamGetCaptureInfo(s, &st, &at.capture) == cudaSuccess && st == cudaStreamCaptureStatusActive) at.order = &capture_order_;
+        at.captured = st != cudaStreamCaptureStatusNone;
+        return at;
     }
 
     cudaEvent_t take_event() {
@@ -485,23 +490,30 @@ class RuntimeCore {
 // The launches of one call on one stream, ordered behind the previous call's (RuntimeCore::order_enter) of every rank that takes part.
 class OrderedCall {
   public:
-    OrderedCall(std::vector<RuntimeCore*> cores, cudaStream_t s) : stream(s), cores_(std::move(cores)) {}
+    explicit OrderedCall(cudaStream_t s) : stream(s) {}
     OrderedCall(const OrderedCall&) = delete;
     ~OrderedCall() { leave(); }
+    void add(RuntimeCore* core) {
+        if (n_ == dx::kMaxRanks) throw std::invalid_argument("OrderedCall: too many ranks");
+        cores_[n_++] = core;
+    }
     void enter() {
         if (inside_) return;
-        for (RuntimeCore* c : cores_) c->order_enter(stream);
+        for (int i = 0; i < n_; ++i) places_[i] = cores_[i]->order_enter(stream);
         inside_ = true;
     }
     void leave() {
         if (!inside_) return;
-        for (RuntimeCore* c : cores_) c->order_leave(stream);
+        for (int i = 0; i < n_; ++i) cores_[i]->order_leave(stream, places_[i]);
         inside_ = false;
     }
+    bool captured() const { return inside_ && places_[0].captured; }
     const cudaStream_t stream;
 
   private:
-    std::vector<RuntimeCore*> cores_;
+    RuntimeCore* cores_[dx::kMaxRanks];
+    RuntimeCore::Place places_[dx::kMaxRanks];
+    int n_ = 0;
     bool inside_ = false;
 };
 
