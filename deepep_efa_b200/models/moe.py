@@ -319,7 +319,11 @@ UNIT_ROWS = 8  # rows of one expert a dispatch warp sends between two arrival-co
 FUSE_CAST_INTO_GEMM1 = True  # wide natively block-scaled tiles: GEMM1's epilogue emits e4m3 + scale atoms itself
 # Decode, natively block-scaled: average rows per expert up to which the GEMMs take the tokens as columns (a tile then multiplies 32 of
 # them at a time instead of 128 rows). One step back to back, rows / columns, us: 64 experts with 12 rows 251 / 226, 16 rows 252 / 227;
-# 32 experts with 24 rows 152 / 149, 32 rows 152 / 162; 16 experts with 64 rows 119 / 144.
+# 32 experts with 24 rows 152 / 149, 32 rows 152 / 162; 16 experts with 64 rows 119 / 144. The average is all the host knows. With skewed
+# routing (popularity 1 / (e + 1)^1.2) a few experts hold most rows, and as columns their tiles take two to four steps of 32; on average /
+# at most, rows, columns, us: 64 experts 12 / 116 227, 225; 128 experts 6 / 97 277, 283; 32 experts 8 / 55 145, 146 and 12 / 82 147, 163; 32
+# smaller ones (2048 -> 1024) 12 / 62 90, 90 and 19 / 93 90, 97; 16 experts 16 / 78 172, 185. (The same layers uniformly: 230, 224; 312, 301;
+# 146, 145 and 146, 146; 91, 80 and 91, 80; 172, 169.)
 TOKEN_COLUMNS_MAX_ROWS = 20
 # Natively block-scaled GEMMs: average rows per expert from which the 128x256 tiles are used instead of the 128x128 ones. Since the
 # wide tiles drain their accumulator in two halves they win from the smallest sizes measured on (8 experts x 4096 rows down to 256
