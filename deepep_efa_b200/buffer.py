@@ -862,11 +862,12 @@ def _ll_stream_exit(buf: Buffer, ctx, tensors) -> EventOverlap:
     return EventOverlap(EventHandle(buf.comm_stream))
 
 
-def _ll_num_sms(num_tokens: int, num_virtual: int) -> int:
+def _ll_num_sms(num_virtual: int) -> int:
+    """SMs a low-latency kernel may take; the launch takes fewer where it has less to do."""
     cap = _NUM_SM_B200 if num_virtual == 1 else _NUM_SM_B200 // num_virtual
     if Buffer.ll_num_sms is not None:
         cap = min(cap, Buffer.ll_num_sms)
-    return max(2, min(num_tokens + 1, cap))
+    return max(2, cap)
 
 
 def _ll_dispatch_many(bufs: List[Buffer], calls, num_max_tokens: int, num_experts: int, use_fp8: bool, round_scale: bool,
@@ -887,7 +888,7 @@ def _ll_dispatch_many(bufs: List[Buffer], calls, num_max_tokens: int, num_expert
         else:
             rx = v["x_bf16"]
         results.append((rx, v["count"], (v["src_info"], v["layout_range"], num_max_tokens, hidden, num_experts)))
-    num_sms = _ll_num_sms(max(c[0].size(0) for c in calls), V)
+    num_sms = _ll_num_sms(V)
 
     def launch(phases: int):
         C.ll_dispatch(rts, per_rank, num_max_tokens, num_experts, use_fp8, round_scale, use_ue8m0, parity, phases, num_sms)
@@ -926,7 +927,7 @@ def _ll_combine_many(bufs: List[Buffer], calls, zero_copy: bool, async_finish: b
         per_rank.append((x, topk_idx, topk_w, src_info, layout_range, out, wait, views[parity]["send_row"]))
         outs.append(out)
     _, _, num_max_tokens, hidden, num_experts = calls[0][3]
-    num_sms = _ll_num_sms(_NUM_SM_B200, V)
+    num_sms = _ll_num_sms(V)
 
     def launch(phases: int):
         C.ll_combine(rts, per_rank, num_max_tokens, num_experts, parity, phases, num_sms, pull, close_barrier)

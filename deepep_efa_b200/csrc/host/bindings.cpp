@@ -735,13 +735,16 @@ void ll_combine(std::vector<Runtime*> rts, std::vector<py::tuple> per_rank, int 
         a.close_barrier = (pull && close_barrier) ? 1 : 0;
         a.x_off = 0;
         a.send_row = nullptr;
+        if (send_row.has_value()) {
+            DX_CHECK(send_row->is_cuda() && send_row->scalar_type() == torch::kInt32 && send_row->is_contiguous() &&
+                         send_row->numel() >= (int64_t)T * topk_idx.size(1), "send_row must be int32 [T,K] on the GPU");
+            a.send_row = send_row->data_ptr<int>();
+        }
         if (pull) {
             const int64_t xo = rt->symmetric_offset(x);
             DX_CHECK(xo >= 0 && xo % 16 == 0, "pull combine: x must live in this rank's symmetric buffer");
-            DX_CHECK(send_row.has_value() && send_row->is_cuda() && send_row->scalar_type() == torch::kInt32 && send_row->is_contiguous() &&
-                         send_row->numel() >= (int64_t)T * topk_idx.size(1), "pull combine: send_row must be int32 [T,K] on the GPU");
+            DX_CHECK(send_row.has_value(), "pull combine: send_row is missing");
             a.x_off = (uint64_t)xo;
-            a.send_row = send_row->data_ptr<int>();
         }
     }
     check_launch(dx::launch_ll_combine(args.data(), V, cur_stream(rts[0])), "low_latency_combine");

@@ -20,6 +20,7 @@
 //     [E][max_tokens] stage (address = (expert, token), so no metadata travels), the home rank waits per source,
 //     then reduces as above.
 //   Both are deterministic (fixed k order, no atomics) and may write the result to pinned host memory.
+// A lone rank has kernels of its own for both directions (dispatch_lone, combine_lone), which keep none of the signalling.
 //
 // `phases` splits either kernel into its send (bit 0) and receive (bit 1) half for the
 // return_recv_hook contract. Sequence numbers and expected-arrival totals live on the device, so a
@@ -35,6 +36,8 @@
 // atomics + cast pass (efa_kernels.cu:1413-1486), and the cooperative send/recv kernels
 // (csrc/kernels/coop_dispatch_send.cuh, coop_dispatch_recv.cuh, coop_combine_send.cuh,
 // coop_combine_recv.cuh).
+#include <algorithm>
+
 #include "api.h"
 #include "prims.cuh"
 #include "launch.cuh"
@@ -45,6 +48,11 @@ constexpr int kLLThreads = 512;
 constexpr int kLLWarps = kLLThreads / 32;
 constexpr int kTicketLLDispatch = 3;
 constexpr int kTicketLLCombine = 4;
+constexpr int kNumSms = 148;
+// The kernels for a lone rank count the earlier selections of a token by looking at all of them. Up to this many (512 tokens with eight
+// experts each) that is a handful of loads per thread; longer batches keep the running histogram of the general kernel.
+constexpr int kLoneMaxSelections = 4096;
+constexpr int kLoneMaxExperts = 8192;  // their counts stay in the shared memory that needs no opt-in
 // rank-local u64 words after the family sequence numbers (RankCtx::seq + kNumFamilies):
 // expected cumulative arrivals [2 kinds][2 parities][kMaxRanks]
 __device__ __forceinline__ uint64_t* expected_word(const RankCtx& c, int kind, int parity, int src) {
@@ -57,13 +65,8 @@ struct QuantChunk {
     uint32_t packed_exp;
 };
 
-// BF16 -> e4m3 for the 16 channels [ch, ch+16) of a row; 8 lanes share a scale, a warp covers four.
-__device__ __forceinline__ QuantChunk quantize_chunk(const char* row, int ch, bool act, bool pow2, bool ue8m0) {
-    int4 r0 = make_int4(0, 0, 0, 0), r1 = r0;
-    if (act) {
-        r0 = ld_cached(reinterpret_cast<const int4*>(row + (size_t)ch * 2));
-        r1 = ld_cached(reinterpret_cast<const int4*>(row + (size_t)ch * 2 + 16));
-    }
+// BF16 -> e4m3 for 16 channels of a row in two registers of 16 bytes; 8 lanes share a scale, a warp covers four.
+__device__ __forceinline__ QuantChunk quantize_regs(const int4& r0, const int4& r1, bool pow2, bool ue8m0) {
     const uint32_t w[8] = {(uint32_t)r0.x, (uint32_t)r0.y, (uint32_t)r0.z, (uint32_t)r0.w,
                            (uint32_t)r1.x, (uint32_t)r1.y, (uint32_t)r1.z, (uint32_t)r1.w};
     float f[16];
@@ -92,6 +95,15 @@ __device__ __forceinline__ QuantChunk quantize_chunk(const char* row, int ch, bo
                        (__shfl_sync(0xffffffffu, ex, 16) << 16) | (__shfl_sync(0xffffffffu, ex, 24) << 24);
     }
     return o;
+}
+// The same for the channels [ch, ch+16) of a row in memory (zeros unless `act`).
+__device__ __forceinline__ QuantChunk quantize_chunk(const char* row, int ch, bool act, bool pow2, bool ue8m0) {
+    int4 r0 = make_int4(0, 0, 0, 0), r1 = r0;
+    if (act) {
+        r0 = ld_cached(reinterpret_cast<const int4*>(row + (size_t)ch * 2));
+        r1 = ld_cached(reinterpret_cast<const int4*>(row + (size_t)ch * 2 + 16));
+    }
+    return quantize_regs(r0, r1, pow2, ue8m0);
 }
 
 // =============================================================================================
@@ -388,11 +400,176 @@ __global__ void __launch_bounds__(kLLThreads, 1) dispatch(const __grid_constant_
     }
 }
 
+// A lone rank knows every count from its own selections and is the only writer and reader of its rows, so nothing is published or
+// waited for: no count words, no arrival counters, no completion ticket. What bounds it is a chain of memory round trips (selections
+// -> slots -> rows); the kernel above went through about eight of them, two at system scope, this one through two. One B200, hidden 7168,
+// 256 experts, top-8, two pairs of dispatch and combine_lone in a CUDA graph: one token 29.4 -> 12.3 us. (77 tokens of 4096 BF16
+// channels with expert outputs in ordinary memory, launched one by one: 23.6 -> 17.9 us, where the host is what takes the time.)
+//   CTA 0      counts per expert and the layout;
+//   CTA 1 + i  slice (i mod slices) of token (i / slices): every thread has 16 channels, loaded while the CTA counts the earlier
+//              selections of the token's experts (read straight from topk_idx: a few thousand words that stay in L2).
+// Sequence numbers, the started word and the tags of send_row are those of the kernel above, so calls of either kind follow each other
+// in any order; the sequence number advances when the last CTA has read it.
+template <bool kFp8>
+__global__ void __launch_bounds__(kLLThreads) dispatch_lone(const __grid_constant__ LLDispatchArgs a, const int slices) {
+    pdl_wait_predecessor();
+    const RankCtx& c = a.ctx;
+    const int T = a.num_tokens, K = a.num_topk, E = a.num_experts, H = a.hidden, P = a.parity, N = a.num_max_tokens;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, num_warps = blockDim.x >> 5;
+    extern __shared__ int s_mem[];                        // CTA 0: [E] selections per expert
+    __shared__ int s_part[kLLWarps][kMaxTopk];            // earlier selections of the token's experts, per warp
+    uint64_t seq = 0;  // only the first warp needs it
+    if (warp == 0) seq = __shfl_sync(0xffffffffu, lane == 0 ? next_seq(c, kFamLLDispatch) : 0ull, 0);
+    const bool masked = __ldcg(&c.my_ctrl()->ll_mask[0]) != 0;
+    unsigned long long* in_flight = reinterpret_cast<unsigned long long*>(c.seq + kLLInFlightWord0 + P);
+    if (blockIdx.x == 0) {
+        trace_stamp(c, kFamLLDispatch, 1, 0);
+        if (tid == 0) {
+            // both words are in memory before this CTA allows the successor's launch (see combine_lone)
+            *reinterpret_cast<volatile uint64_t*>(c.seq + kLLStartedWord0 + P) = seq;
+            atomicAdd(in_flight, (unsigned long long)gridDim.x);
+            __threadfence();
+        }
+        __syncthreads();
+    } else if (blockIdx.x == 1) {
+        trace_stamp(c, kFamLLDispatch, 0, 0);
+    }
+    pdl_release_successor();
+    int order = 0;
+    // counts the CTAs that have read the sequence number: the addend (always 1) depends on it
+    if (tid == 0) order = atomicAdd(c.local_scratch + kTicketLLDispatch, 1 + (int)(seq >> 63));
+    if (blockIdx.x == 0) {
+        for (int i = tid; i < E; i += blockDim.x) s_mem[i] = 0;
+        __syncthreads();
+        for (int i = tid; i < T * K; i += blockDim.x) {
+            const int64_t e = __ldg(a.topk_idx + i);
+            if (e >= 0 && e < E) atomicAdd(&s_mem[e], 1);
+        }
+        __syncthreads();
+        for (int e = tid; e < E; e += blockDim.x) {
+            const int n = masked ? 0 : s_mem[e];
+            a.packed_recv_count[e] = n;
+            a.layout_range[e] = n;
+            if (a.cumulative_stats != nullptr) a.cumulative_stats[e] += n;
+        }
+        trace_stamp(c, kFamLLDispatch, 1, 6);
+    } else {
+        const bool pow2 = a.round_scale != 0 || a.use_ue8m0 != 0;
+        char* rows = c.at<char>(0, a.region.recv_x_off[P]);
+        for (int item = blockIdx.x - 1; item < T * slices; item += gridDim.x - 1) {
+            const int t = item / slices, slice = item % slices;
+            const char* xrow = reinterpret_cast<const char*>(a.x) + (size_t)t * H * 2;
+            // FP8: 16 neighbouring channels; BF16: two 16-byte columns, a CTA's width apart
+            const int ch = (slice * blockDim.x + tid) * 16;
+            const int n16 = H / 8, col0 = slice * 2 * blockDim.x + tid, col1 = col0 + blockDim.x;
+            int4 v0 = make_int4(0, 0, 0, 0), v1 = v0;
+            if constexpr (kFp8) {
+                if (ch < H) {
+                    v0 = ld_cached(reinterpret_cast<const int4*>(xrow + (size_t)ch * 2));
+                    v1 = ld_cached(reinterpret_cast<const int4*>(xrow + (size_t)ch * 2 + 16));
+                }
+            } else {
+                if (col0 < n16) v0 = ld_cached(reinterpret_cast<const int4*>(xrow) + col0);
+                if (col1 < n16) v1 = ld_cached(reinterpret_cast<const int4*>(xrow) + col1);
+            }
+            // lane k: expert of selection (t, k), or -1
+            int e = -1;
+            if (lane < K) {
+                const int64_t e64 = __ldg(a.topk_idx + (size_t)t * K + lane);
+                if (e64 >= 0 && e64 < E) e = (int)e64;
+            }
+            for (int k0 = 0; k0 < K; k0 += 8) {
+                int ek[8], n[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    ek[j] = __shfl_sync(0xffffffffu, e, (k0 + j) & 31);
+                    n[j] = 0;
+                }
+#pragma unroll 4
+                for (int i = tid; i < t * K; i += blockDim.x) {
+                    const int64_t v64 = __ldg(a.topk_idx + i);
+                    const int v = (v64 >= 0 && v64 < E) ? (int)v64 : -2;
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) n[j] += v == ek[j] ? 1 : 0;
+                }
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    n[j] = __reduce_add_sync(0xffffffffu, n[j]);
+                    if (lane == j && k0 + j < K) s_part[warp][k0 + j] = n[j];
+                }
+            }
+            QuantChunk qc;
+            if constexpr (kFp8) qc = quantize_regs(v0, v1, pow2, a.use_ue8m0 != 0);
+            __syncthreads();
+            int row = -1;
+            if (e >= 0 && !masked) {
+                row = 0;
+                for (int w = 0; w < num_warps; ++w) row += s_part[w][lane];
+            }
+            for (int k = 0; k < K; ++k) {
+                const int o = __shfl_sync(0xffffffffu, e, k);
+                if (row >= 0 && k < lane && o == e) ++row;
+            }
+            const size_t row_bytes = (size_t)H * (kFp8 ? 1 : 2);
+            if (row >= N || (row >= 0 && !peer_range_ok(c, 0, rows + ((size_t)e * N + row) * row_bytes, row_bytes, 3))) row = -1;
+            if (slice == 0 && warp == 0 && lane < K) {
+                if (row >= 0) c.at<int>(0, a.region.recv_src_info_off[P])[(size_t)e * N + row] = t;
+                if (a.send_row != nullptr) a.send_row[t * K + lane] = (ll_count_tag(seq) << 16) | (row + 1);
+            }
+            const int slot_of = row >= 0 ? e * N + row : -1;
+#pragma unroll 4
+            for (int k = 0; k < K; ++k) {
+                const int slot = __shfl_sync(0xffffffffu, slot_of, k);
+                if (slot < 0) continue;
+                if constexpr (kFp8) {
+                    if (ch < H) st_stream(reinterpret_cast<int4*>(rows + (size_t)slot * H + ch), qc.q);
+                    if (a.use_ue8m0) {
+                        if (lane == 0 && ch < H) c.at<uint32_t>(0, a.region.recv_scales_off[P])[(size_t)slot * (H / 512) + (ch >> 9)] = qc.packed_exp;
+                    } else if ((lane & 7) == 0 && ch < H) {
+                        c.at<float>(0, a.region.recv_scales_off[P])[(size_t)slot * (H / 128) + (ch >> 7)] = qc.scale;
+                    }
+                } else {
+                    int4* dst = reinterpret_cast<int4*>(rows) + (size_t)slot * n16;
+                    if (col0 < n16) st_stream(dst + col0, v0);
+                    if (col1 < n16) st_stream(dst + col1, v1);
+                }
+            }
+            if (item + (int)gridDim.x - 1 < T * slices) __syncthreads();  // s_part is reused
+        }
+        if (blockIdx.x == 1) trace_stamp(c, kFamLLDispatch, 0, 6);
+    }
+    if (tid == 0) {
+        if (order == (int)gridDim.x - 1) {
+            c.local_scratch[kTicketLLDispatch] = 0;
+            commit_seq(c, kFamLLDispatch, seq);
+        }
+        atomicAdd(in_flight, ~0ull);  // minus one
+    }
+}
+
 }  // namespace ll
 
 cudaError_t launch_ll_dispatch(const LLDispatchArgs* a, int nv, cudaStream_t stream) {
+    int max_tokens = 0;
+    for (int v = 0; v < nv; ++v) max_tokens = std::max(max_tokens, a[v].num_tokens);
+    if (nv == 1 && a->ctx.num_ranks == 1 && a->phases == 3 && a->hidden > 0 && a->num_tokens * a->num_topk <= kLoneMaxSelections && a->num_experts <= kLoneMaxExperts) {
+        int slices = (a->hidden + kLLThreads * 16 - 1) / (kLLThreads * 16);
+        int grid = a->num_tokens * slices + 1;
+        if (a->num_sms >= kNumSms) {
+            // few tokens: slices of a row as small as 1024 channels, as long as every one of them has an SM for itself
+            while (slices * 1024 < a->hidden && a->num_tokens * (slices + 1) < kNumSms) ++slices;
+            grid = a->num_tokens * slices + 1;
+        } else {
+            grid = std::min(grid, std::max(2, a->num_sms));
+        }
+        const int threads = ((a->hidden + 16 * slices - 1) / (16 * slices) + 31) / 32 * 32;
+        const size_t smem = (size_t)a->num_experts * sizeof(int);
+        return a->use_fp8 ? launch_dependent(ll::dispatch_lone<true>, dim3(grid), threads, smem, stream, *a, slices)
+                          : launch_dependent(ll::dispatch_lone<false>, dim3(grid), threads, smem, stream, *a, slices);
+    }
+    const int grid = std::max(2, std::min(max_tokens + 1, a[0].num_sms));
     const size_t smem = ((size_t)a[0].num_tokens * a[0].num_topk + a[0].num_experts) * sizeof(int);
-    return DX_LAUNCH_RANKED_PDL(ll::dispatch, LLDispatchArgs, a, nv, a[0].num_sms, kLLThreads, smem, stream);
+    return DX_LAUNCH_RANKED_PDL(ll::dispatch, LLDispatchArgs, a, nv, grid, kLLThreads, smem, stream);
 }
 
 // =============================================================================================
@@ -778,9 +955,120 @@ __global__ void __launch_bounds__(kLLThreads, 1) combine_pull(const __grid_const
     if (early) pdl_wait_predecessor();  // this kernel may not complete before its predecessor has
 }
 
+// A lone rank's expert outputs are in its own memory wherever x lives, so the rows are read in place: no announcement, no copy into a
+// stage, no closing round. One thread has one 16-byte column of a token, with the loads of eight rows in flight; warps do not wait for
+// each other. A combine that directly follows the dispatch of its handle gathers beside it, as combine_pull does: the dispatch raises the
+// parity's in-flight word by its number of CTAs before any of them allows this launch, and each takes one off as its last act, so the
+// word is zero whenever anything came in between. Only reads happen early; results are stored after the predecessor has completed, because
+// their memory may be a block that the predecessor still reads (freed by the caller between the two calls).
+// kFind (x is an ordinary tensor): src_info decides which row of the expert is the token's, so that the selections of a token may come in
+// another order than at the dispatch, as with the staged form. It is loaded with the row itself; the search is for the odd case.
+template <bool kFind>
+__global__ void __launch_bounds__(kLLThreads) combine_lone(const __grid_constant__ LLCombineArgs a, const int slices) {
+    pdl_release_successor();
+    const RankCtx& c = a.ctx;
+    const int T = a.num_tokens, K = a.num_topk, E = a.num_experts, N = a.num_max_tokens, n16 = a.hidden / 8;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const bool traced = blockIdx.x == 0 || blockIdx.x == gridDim.x - 1;
+    const int tslot = blockIdx.x == 0 ? 0 : 1;
+    if (traced) trace_stamp(c, kFamLLCombine, tslot, 0);
+    bool early = *reinterpret_cast<volatile uint64_t*>(c.seq + kLLInFlightWord0 + a.parity) != 0;
+    early = __any_sync(0xffffffffu, early);
+    if (!early) pdl_wait_predecessor();
+    const int tag = ll_count_tag(*reinterpret_cast<volatile uint64_t*>(c.seq + kLLStartedWord0 + a.parity));
+    const bool masked = __ldcg(&c.my_ctrl()->ll_mask[0]) != 0;
+    const int4* x = reinterpret_cast<const int4*>(a.x);
+    for (int item = blockIdx.x; item < T * slices; item += gridDim.x) {
+        const int t = item / slices, col = (item % slices) * blockDim.x + tid;
+        // lane k: row of selection (t, k) in x, or -1, and its weight
+        int e = -1, slot = -1;
+        float weight = 0.f;
+        if (lane < K) {
+            const int64_t e64 = __ldg(a.topk_idx + (size_t)t * K + lane);
+            unsigned word = (unsigned)ld_relaxed_sys(a.send_row + (size_t)t * K + lane);
+            weight = __ldg(a.topk_weights + (size_t)t * K + lane);
+            if ((word >> 16) != (unsigned)tag) {
+                const long long t0 = clock64();
+                while (early && ((word = (unsigned)ld_relaxed_sys(a.send_row + (size_t)t * K + lane)) >> 16) != (unsigned)tag && clock64() - t0 <= c.timeout_cycles) {
+                }
+                if ((word >> 16) != (unsigned)tag) {
+                    report(c.status, kTimeoutCombineReady, 0, 0, 2);
+                    word = 0;
+                }
+            }
+            const int row = (int)(word & 0xffffu) - 1;
+            if (e64 >= 0 && e64 < E && !masked) e = (int)e64;
+            if (e >= 0 && row >= 0 && row < N) slot = e * N + row;
+        }
+        float acc[8];
+        auto gather = [&]() {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) acc[j] = 0.f;
+            for (int k0 = 0; k0 < K; k0 += 8) {
+                int4 v[8];
+#pragma unroll
+                for (int kk = 0; kk < 8; ++kk) {
+                    const int s = __shfl_sync(0xffffffffu, slot, (k0 + kk) & 31);
+                    v[kk] = (k0 + kk < K && s >= 0 && col < n16) ? ld_stream(x + (size_t)s * n16 + col) : make_int4(0, 0, 0, 0);
+                }
+#pragma unroll
+                for (int kk = 0; kk < 8; ++kk) {
+                    const int s = __shfl_sync(0xffffffffu, slot, (k0 + kk) & 31);
+                    const float w0 = __shfl_sync(0xffffffffu, weight, (k0 + kk) & 31);
+                    const float w = (k0 + kk < K && s >= 0) ? w0 : 0.f;
+                    const uint32_t u[4] = {(uint32_t)v[kk].x, (uint32_t)v[kk].y, (uint32_t)v[kk].z, (uint32_t)v[kk].w};
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const float2 p = bf16x2_to_f2(u[j]);
+                        acc[2 * j] = fmaf(w, p.x, acc[2 * j]);
+                        acc[2 * j + 1] = fmaf(w, p.y, acc[2 * j + 1]);
+                    }
+                }
+            }
+        };
+        int info = t;
+        if (kFind && !early && slot >= 0) info = __ldcg(a.src_info + slot);
+        gather();
+        if (early) pdl_wait_predecessor();  // from here on everything is final; returns at once in later rounds of the loop
+        if constexpr (kFind) {
+            if (early && slot >= 0) info = __ldcg(a.src_info + slot);
+            const bool wrong = e >= 0 && (slot < 0 || info != t);
+            if (__any_sync(0xffffffffu, wrong)) {
+                if (wrong) {
+                    slot = -1;
+                    const int rows = min((int)(a.layout_range[e] & 0xffffffff), N);
+                    for (int n = 0; n < rows && slot < 0; ++n)
+                        if (__ldcg(a.src_info + (size_t)e * N + n) == t) slot = e * N + n;
+                }
+                gather();
+            }
+        }
+        if (col < n16) {
+            int4 o;
+            o.x = (int)f2_to_bf16x2(acc[0], acc[1]);
+            o.y = (int)f2_to_bf16x2(acc[2], acc[3]);
+            o.z = (int)f2_to_bf16x2(acc[4], acc[5]);
+            o.w = (int)f2_to_bf16x2(acc[6], acc[7]);
+            st_stream(reinterpret_cast<int4*>(a.out) + (size_t)t * n16 + col, o);
+        }
+    }
+    if (traced) trace_stamp(c, kFamLLCombine, tslot, 6);
+    if (early) pdl_wait_predecessor();  // also without an item: this kernel may not complete before its predecessor has
+}
+
 }  // namespace ll
 
 cudaError_t launch_ll_combine(const LLCombineArgs* a, int nv, cudaStream_t stream) {
+    if (nv == 1 && a->ctx.num_ranks == 1 && a->phases == 3 && a->send_row != nullptr) {
+        if (a->num_tokens == 0 || a->hidden == 0) return cudaSuccess;
+        // one column per thread in CTAs of 128 threads; a bounded grid takes as wide ones as there are
+        const bool bounded = a->num_sms < kNumSms;
+        const int threads = bounded ? kLLThreads : 128;
+        const int slices = (a->hidden / 8 + threads - 1) / threads;
+        const int grid = bounded ? std::min(a->num_tokens * slices, std::max(1, a->num_sms)) : std::min(a->num_tokens * slices, 16 * kNumSms);
+        return a->pull ? launch_dependent(ll::combine_lone<false>, dim3(grid), threads, 0, stream, *a, slices)
+                       : launch_dependent(ll::combine_lone<true>, dim3(grid), threads, 0, stream, *a, slices);
+    }
     if (a[0].pull) return DX_LAUNCH_RANKED_PDL(ll::combine_pull, LLCombineArgs, a, nv, a[0].num_sms, kLLThreads, 0, stream);
     const size_t smem = ((size_t)a[0].num_experts / a[0].ctx.num_ranks + 1) * sizeof(int);
     return DX_LAUNCH_RANKED_PDL(ll::combine, LLCombineArgs, a, nv, a[0].num_sms, kLLThreads, smem, stream);

@@ -125,5 +125,8 @@ enum Family : int { kFamNotify = 0, kFamDispatch = 1, kFamCombine = 2, kFamBarri
 static_assert(kFusedExpectedWord0 == kNumFamilies + 2 * 2 * kMaxRanks, "layout of the rank-local sequence words");
 // after the fused layer's expected-arrival words: per parity, the sequence number of the low-latency dispatch that last used it
 constexpr int kLLStartedWord0 = kFusedExpectedWord0 + kMaxLocalExperts;
+// per parity: CTAs of a lone rank's low-latency dispatch that have not finished (zero whenever none runs)
+constexpr int kLLInFlightWord0 = kLLStartedWord0 + 2;
+constexpr int kNumLocalSeqWords = kLLInFlightWord0 + 2;
 
 }  // namespace dx

@@ -1,0 +1,131 @@
+"""Low-latency kernels of a lone rank against the general kernels (which the hook form still runs) and the oracle."""
+import pytest
+import torch
+
+from helpers import make_routing, make_tokens
+
+pytestmark = pytest.mark.gpu
+
+
+def _cluster(T, H, E, arena=2 << 20):
+    from deepep_efa_b200 import Buffer
+    from deepep_efa_b200.parallel.virtual import VirtualCluster
+    return VirtualCluster(1, num_nvl_bytes=arena, num_rdma_bytes=Buffer.get_low_latency_rdma_size_hint(T, H, 1, E), timeout_ms=2000)
+
+
+def _valid(res):
+    """Everything the dispatch defines: counts, layout, and the valid rows of data, scales and source tokens."""
+    rx, cnt, handle = res[:3]
+    parts = [cnt, handle[1]]
+    for e, n in enumerate(cnt.tolist()):
+        parts.append(handle[0][e, :n])
+        parts += [r[e, :n].view(torch.uint8) for r in (rx if isinstance(rx, tuple) else (rx,))]
+    return [p.clone() for p in parts]
+
+
+# one token and one selection; slices of a row (few tokens), whole rows, rows wider than a CTA, the last batch of the lone kernel
+# (512 x 8 selections) and the first past it, more selections than a group of eight, hidden sizes that end inside a slice
+@pytest.mark.parametrize("T,H,E,K,masked,sms", [(1, 7168, 256, 8, 0.0, None), (1, 128, 1, 1, 0.0, None), (5, 1152, 60, 6, 0.1, None), (77, 4096, 64, 6, 0.05, None),
+                                                 (128, 7168, 16, 8, 0.0, None), (128, 7168, 16, 8, 0.1, 7), (20, 8320, 8, 3, 0.0, None),
+                                                 (40, 1024, 64, 32, 0.2, None), (512, 512, 32, 8, 0.0, None), (513, 512, 32, 8, 0.0, None), (33, 512, 8, 2, 1.0, None)])
+@pytest.mark.parametrize("wire", ["bf16", "fp8", "fp8_pow2", "fp8_ue8m0"])
+def test_lone_rank_matches_general_kernels(T, H, E, K, masked, sms, wire):
+    from deepep_efa_b200 import Buffer
+    if wire == "fp8_ue8m0" and H % 512:
+        pytest.skip("UE8M0 scales come in words of 512 channels")
+    vc = _cluster(T, H, E, arena=(2 << 20) + E * T * H * 2)
+    Buffer.set_low_latency_num_sms(sms)
+    try:
+        buf = vc.buffers[0]
+        how = dict(use_fp8=wire != "bf16", round_scale=wire in ("fp8_pow2", "fp8_ue8m0"), use_ue8m0=wire == "fp8_ue8m0")
+        idx, w = make_routing(T, E, K, "cuda", seed=T + K, masked_fraction=masked)
+        x = make_tokens(T, H, "cuda", seed=H)
+        stats = [torch.zeros(E, dtype=torch.int32, device="cuda") for _ in range(2)]
+        general = vc.low_latency_dispatch([x], [idx], T, E, return_recv_hook=True, cumulative_stats=[stats[0]], **how)[0]
+        general[4]()
+        want = _valid(general)
+        y = torch.randn(E, T, H, device="cuda").to(torch.bfloat16)
+        out = vc.low_latency_combine([y], [idx], [w], [general[2]], return_recv_hook=True)[0]
+        out[2]()
+        want_y = out[0].clone()
+        got = vc.low_latency_dispatch([x], [idx], T, E, cumulative_stats=[stats[1]], **how)[0]
+        for a, b in zip(want, _valid(got)):
+            assert torch.equal(a, b)
+        assert torch.equal(stats[0], stats[1])
+        sym = buf.empty_symmetric([E, T, H], torch.bfloat16)
+        sym.copy_(y)
+        order = torch.randperm(K, device="cuda")  # selections in another order than at the dispatch: ordinary tensors allow it
+        for _ in range(3):  # behind a finished dispatch, then right behind one that may still run, in either parity
+            assert torch.equal(vc.low_latency_combine([y], [idx], [w], [got[2]])[0][0], want_y)
+            assert torch.equal(vc.low_latency_combine([sym], [idx], [w], [got[2]])[0][0], want_y)
+            turned = idx[:, order].contiguous(), w[:, order].contiguous()
+            got = vc.low_latency_dispatch([x], [idx], T, E, **how)[0]
+            z = vc.low_latency_combine([y], [turned[0]], [turned[1]], [got[2]])[0][0]
+            # K products summed in another order in fp32, then rounded to BF16
+            assert (z.float() - want_y.float()).norm() <= 4e-3 * want_y.float().norm()
+            got = vc.low_latency_dispatch([x], [idx], T, E, **how)[0]
+            assert torch.equal(vc.low_latency_combine([sym], [idx], [w], [got[2]])[0][0], want_y)
+            got = vc.low_latency_dispatch([x], [idx], T, E, **how)[0]
+        buf.check_status()
+    finally:
+        Buffer.set_low_latency_num_sms(None)
+        vc.destroy()
+
+
+def test_lone_rank_pairs_back_to_back():
+    """Pairs with other data each time, alternately of the lone and of the general kernels, the combine right behind its dispatch and its
+    result in memory that the caller gave back after the dispatch."""
+    T, H, E, K = 96, 2048, 32, 4
+    vc = _cluster(T, H, E, arena=(2 << 20) + E * T * H * 2)
+    try:
+        sym = vc.buffers[0].empty_symmetric([E, T, H], torch.bfloat16)
+        sym.copy_(torch.randn(E, T, H, device="cuda"))
+        batches = [(make_tokens(T, H, "cuda", seed=s), *make_routing(T, E, K, "cuda", seed=s, masked_fraction=0.05)) for s in range(6)]
+        outs = []
+        for i in range(48):
+            x, idx, w = batches[i % 6]
+            x = x.clone()
+            hook = i % 5 == 4
+            res = vc.low_latency_dispatch([x], [idx], T, E, return_recv_hook=hook)[0]
+            if hook:
+                res[4]()
+            del x
+            outs.append((i % 6, [r.clone() for r in (res[1], res[2][1])] if i % 7 == 0 else None,
+                         vc.low_latency_combine([sym], [idx], [w], [res[2]])[0][0]))
+        torch.cuda.synchronize()
+        vc.buffers[0].check_status()
+        first = {}
+        for b, meta, y in outs:
+            idx, w = batches[b][1:]
+            if b not in first:
+                want = torch.zeros(T, H, device="cuda")
+                rows = {}
+                for t, es in enumerate(idx.tolist()):
+                    for k, e in enumerate(es):
+                        if e >= 0:
+                            want[t] += w[t, k] * sym[e, rows.setdefault(e, 0)].float()
+                            rows[e] += 1
+                assert (y.float() - want).norm() <= 4e-3 * want.norm()
+                first[b] = y
+            assert torch.equal(y, first[b])
+            if meta is not None:
+                n = torch.bincount(idx[idx >= 0], minlength=E)
+                assert torch.equal(meta[0].long(), n) and torch.equal(meta[1].view(-1), n)
+    finally:
+        vc.destroy()
+
+
+def test_lone_rank_that_masks_itself_sends_nothing():
+    T, H, E, K = 16, 1024, 8, 4
+    vc = _cluster(T, H, E)
+    try:
+        buf = vc.buffers[0]
+        idx, w = make_routing(T, E, K, "cuda", seed=3)
+        buf.low_latency_update_mask_buffer(0, True)
+        res = vc.low_latency_dispatch([make_tokens(T, H, "cuda")], [idx], T, E)[0]
+        assert res[1].sum().item() == 0 and res[2][1].sum().item() == 0
+        y = torch.randn(E, T, H, device="cuda").to(torch.bfloat16)
+        assert vc.low_latency_combine([y], [idx], [w], [res[2]])[0][0].abs().sum().item() == 0
+        buf.check_status()
+    finally:
+        vc.destroy()
