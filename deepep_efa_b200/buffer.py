@@ -27,9 +27,9 @@ import torch.distributed as dist
 
 from . import _ext
 from .config import Config
-from .utils.event import EventHandle, EventOverlap
+from .utils.event import EventHandle, EventOverlap, current_stream
 from .utils.logging import log as _log
-from .utils.profiler import PROFILE_ENABLED, PhaseProfiler, nvtx_range
+from .utils.profiler import NVTX_ENABLED, PROFILE_ENABLED, PhaseProfiler, nvtx_range
 import logging as _logging
 
 topk_idx_t = torch.int64
@@ -499,6 +499,10 @@ class Buffer:
                 # (words are (call tag << 16) | (row + 1); zero = never written)
                 send_row=torch.zeros(num_max_tokens * 32, dtype=torch.int32, device=self.device),
             )
+            # what a dispatch returns, and how a combine finds the parity of its handle
+            d["fp8"], d["fp8_ue8m0"] = (d["x_fp8"], d["scales"]), (d["x_fp8"], d["scales_ue8m0"])
+            d["handle"] = (d["src_info"], d["layout_range"], num_max_tokens, hidden, num_experts)
+            d["src_info_ptr"] = d["src_info"].data_ptr()
             v.append(d)
         self._ll_cache[key] = v
         return v
@@ -529,6 +533,15 @@ class Buffer:
             return self._cpu.low_latency_dispatch(x, topk_idx, num_max_dispatch_tokens_per_rank, num_experts, use_fp8,
                                                   round_scale, use_ue8m0, cumulative_local_expert_recv_stats, return_recv_hook)
         assert not (async_finish and return_recv_hook)
+        if not (async_finish or return_recv_hook or PROFILE_ENABLED or NVTX_ENABLED):
+            parity = self._ll_parity
+            self._ll_parity ^= 1
+            v = self._ll_views(num_max_dispatch_tokens_per_rank, x.size(1), num_experts)[parity]
+            self._C.ll_dispatch_one(self.runtime, x, topk_idx, v["count"], v["layout_range"], cumulative_local_expert_recv_stats,
+                                    dispatch_wait_recv_cost_stats, v["send_row"], num_max_dispatch_tokens_per_rank, num_experts, use_fp8,
+                                    round_scale, use_ue8m0, parity, _ll_num_sms(1))
+            rx = v["x_bf16"] if not use_fp8 else v["fp8_ue8m0"] if use_ue8m0 else v["fp8"]
+            return rx, v["count"], v["handle"], EventOverlap(), None
         if PROFILE_ENABLED:
             prof = self.__dict__.setdefault("_ll_dispatch_profiler", PhaseProfiler("LL-DISPATCH", self.rank))
             prof.mark("start")
@@ -561,6 +574,15 @@ class Buffer:
         if self._cpu is not None:
             return self._cpu.low_latency_combine(x, topk_idx, topk_weights, handle, out, return_recv_hook)
         assert not (async_finish and return_recv_hook)
+        if not (async_finish or return_recv_hook or PROFILE_ENABLED or NVTX_ENABLED):
+            src_info, layout_range, num_max_tokens, hidden, num_experts = handle
+            views = self._ll_views(num_max_tokens, hidden, num_experts)
+            parity = _parity_of(views, src_info)
+            v = views[parity]
+            out = self._C.ll_combine_one(self.runtime, v["combine_src"] if zero_copy else x, topk_idx, topk_weights, src_info, layout_range, out,
+                                         combine_wait_recv_cost_stats, v["send_row"], v["combine_src"], num_max_tokens, num_experts, parity,
+                                         _ll_num_sms(1))
+            return out, EventOverlap(), None
         if PROFILE_ENABLED:
             prof = self.__dict__.setdefault("_ll_combine_profiler", PhaseProfiler("LL-COMBINE", self.rank))
             prof.mark("start")
@@ -694,21 +716,29 @@ class _CommScope:
     def __enter__(self):
         if self.direct:
             return self
-        self.compute = torch.cuda.current_stream()
+        self.compute = current_stream()
         comm = self.buf._comm_stream
         if self.prev is not None and self.prev.event is not None and self.prev.event.event is not None:
             comm.wait_event(self.prev.event.event)
         else:
             comm.wait_stream(self.compute)
-        self._ctx = torch.cuda.stream(comm)
-        self._ctx.__enter__()
+        # the same as entering torch.cuda.stream(comm), which asks for the current streams again on both ways
+        self._ctx = None
+        if self.compute.device == comm.device:
+            torch.cuda.set_stream(comm)
+        else:
+            self._ctx = torch.cuda.stream(comm)
+            self._ctx.__enter__()
         return self
 
     def __exit__(self, et, ev, tb):
         if self.direct:
             return False
         comm = self.buf._comm_stream
-        self._ctx.__exit__(et, ev, tb)
+        if self._ctx is None:
+            torch.cuda.set_stream(self.compute)
+        else:
+            self._ctx.__exit__(et, ev, tb)
         if et is not None:
             return False
         # outputs were allocated while the communication stream was current; they will be used on the caller's stream
@@ -838,7 +868,7 @@ def _combine_many(bufs: List[Buffer], calls, config: Config, previous_event, asy
 
 
 def _parity_of(views, src_info: torch.Tensor) -> int:
-    return 0 if src_info.data_ptr() == views[0]["src_info"].data_ptr() else 1
+    return 0 if src_info.data_ptr() == views[0]["src_info_ptr"] else 1
 
 
 def _ll_stream_enter(buf: Buffer, async_finish: bool):

@@ -611,6 +611,54 @@ dx::LLRegion make_region(const dxh::LowLatencyLayout& l) {
     return r;
 }
 
+using OptTensor = c10::optional<torch::Tensor>;
+
+void fill_ll_dispatch(dx::LLDispatchArgs& a, Runtime* rt, const torch::Tensor& x, const torch::Tensor& topk_idx, const torch::Tensor& count,
+                      const torch::Tensor& range, const OptTensor& cum, const OptTensor& wait, const OptTensor& slot, int num_max_tokens, int num_experts,
+                      bool use_fp8, bool round_scale, bool use_ue8m0, int parity, int phases, int num_sms) {
+    const int R = rt->core->num_ranks();
+    // x may also sit in pinned host memory: the token CTAs then read their rows over PCIe themselves (each row is read
+    // exactly once), which is the host-to-device transfer without a copy in front of the kernel
+    const bool x_on_gpu = x.is_cuda() && x.device().index() == rt->core->device();
+    const bool x_pinned = x.device().is_cpu() && x.is_pinned();
+    DX_CHECK((x_on_gpu || x_pinned) && x.dim() == 2 && x.is_contiguous() && x.scalar_type() == torch::kBFloat16,
+             "x must be contiguous bf16 [T,hidden] on this rank's GPU or in pinned host memory");
+    DX_CHECK(topk_idx.is_cuda() && topk_idx.device().index() == rt->core->device() && count.is_cuda() && range.is_cuda(),
+             "low_latency_dispatch: every tensor but x must live on this rank's GPU");
+    const int T = (int)x.size(0), H = (int)x.size(1);
+    DX_CHECK(T <= num_max_tokens, "more tokens than num_max_dispatch_tokens_per_rank");
+    DX_CHECK(num_max_tokens <= 65535, "num_max_dispatch_tokens_per_rank must fit the 16-bit count field of the count exchange");
+    DX_CHECK((int64_t)R * num_max_tokens < 65535, "rows per expert (ranks x num_max_dispatch_tokens_per_rank) must fit the 16-bit row field of send_row");
+    DX_CHECK(H % 128 == 0 && (!use_ue8m0 || H % 512 == 0), "hidden must be a multiple of 128 (512 with UE8M0)");
+    DX_CHECK(topk_idx.scalar_type() == torch::kInt64 && topk_idx.is_contiguous() && topk_idx.dim() == 2 && topk_idx.size(0) == T, "topk_idx must be int64 [T,K]");
+    DX_CHECK(topk_idx.size(1) <= dx::kMaxTopk, "num_topk too large");
+    DX_CHECK(num_experts % R == 0 && count.numel() == num_experts / R && range.numel() == (int64_t)(num_experts / R) * R, "bad output shapes");
+    dxh::LowLatencyLayout lay(rt->core->ll_base(), num_max_tokens, H, R, num_experts);
+    DX_CHECK(lay.total_bytes <= rt->core->ll_bytes(), "low-latency region too small: create the Buffer with num_rdma_bytes >= get_low_latency_rdma_size_hint(...)");
+    a.ctx = rt->core->ctx();
+    a.parity = parity;
+    a.region = make_region(lay);
+    a.x = reinterpret_cast<const __nv_bfloat16*>(x.data_ptr());
+    a.topk_idx = topk_idx.data_ptr<int64_t>();
+    a.num_tokens = T;
+    a.hidden = H;
+    a.num_topk = (int)topk_idx.size(1);
+    a.num_experts = num_experts;
+    a.num_max_tokens = num_max_tokens;
+    a.use_fp8 = use_fp8;
+    a.round_scale = round_scale;
+    a.use_ue8m0 = use_ue8m0;
+    a.phases = phases;
+    a.packed_recv_count = count.data_ptr<int>();
+    a.layout_range = range.data_ptr<int64_t>();
+    a.cumulative_stats = ptr_or_null<int>(cum);
+    a.wait_cost_stats = ptr_or_null<int64_t>(wait);
+    if (slot.has_value())
+        DX_CHECK(slot->is_cuda() && slot->scalar_type() == torch::kInt32 && slot->is_contiguous() && slot->numel() >= (int64_t)T * topk_idx.size(1), "send_row must be int32 [T,K] on the GPU");
+    a.send_row = ptr_or_null<int>(slot);
+    a.num_sms = num_sms;
+}
+
 // Per rank tuple: (x, topk_idx, packed_recv_count, layout_range, cumulative_stats|None, wait_stats|None, send_row|None)
 void ll_dispatch(std::vector<Runtime*> rts, std::vector<py::tuple> per_rank, int num_max_tokens, int num_experts, bool use_fp8,
                  bool round_scale, bool use_ue8m0, int parity, int phases, int num_sms) {
@@ -619,65 +667,81 @@ void ll_dispatch(std::vector<Runtime*> rts, std::vector<py::tuple> per_rank, int
     c10::cuda::CUDAGuard guard(rts[0]->core->device());
     std::vector<dx::LLDispatchArgs> args(V);
     for (int v = 0; v < V; ++v) {
-        Runtime* rt = rts[v];
         const py::tuple& t = per_rank[v];
         DX_CHECK(t.size() == 7, "ll_dispatch: per-rank tuple must have 7 entries");
-        auto x = t[0].cast<torch::Tensor>();
-        auto topk_idx = t[1].cast<torch::Tensor>();
-        auto count = t[2].cast<torch::Tensor>();
-        auto range = t[3].cast<torch::Tensor>();
-        auto cum = opt_tensor(t[4]);
-        auto wait = opt_tensor(t[5]);
-        auto slot = opt_tensor(t[6]);
-        const int R = rt->core->num_ranks();
-        // x may also sit in pinned host memory: the token CTAs then read their rows over PCIe themselves (each row is read
-        // exactly once), which is the host-to-device transfer without a copy in front of the kernel
-        const bool x_on_gpu = x.is_cuda() && x.device().index() == rt->core->device();
-        const bool x_pinned = x.device().is_cpu() && x.is_pinned();
-        DX_CHECK((x_on_gpu || x_pinned) && x.dim() == 2 && x.is_contiguous() && x.scalar_type() == torch::kBFloat16,
-                 "x must be contiguous bf16 [T,hidden] on this rank's GPU or in pinned host memory");
-        DX_CHECK(topk_idx.is_cuda() && topk_idx.device().index() == rt->core->device() && count.is_cuda() && range.is_cuda(),
-                 "low_latency_dispatch: every tensor but x must live on this rank's GPU");
-        const int T = (int)x.size(0), H = (int)x.size(1);
-        DX_CHECK(T <= num_max_tokens, "more tokens than num_max_dispatch_tokens_per_rank");
-        DX_CHECK(num_max_tokens <= 65535, "num_max_dispatch_tokens_per_rank must fit the 16-bit count field of the count exchange");
-        DX_CHECK((int64_t)R * num_max_tokens < 65535, "rows per expert (ranks x num_max_dispatch_tokens_per_rank) must fit the 16-bit row field of send_row");
-        DX_CHECK(H % 128 == 0 && (!use_ue8m0 || H % 512 == 0), "hidden must be a multiple of 128 (512 with UE8M0)");
-        DX_CHECK(topk_idx.scalar_type() == torch::kInt64 && topk_idx.is_contiguous() && topk_idx.dim() == 2 && topk_idx.size(0) == T, "topk_idx must be int64 [T,K]");
-        DX_CHECK(topk_idx.size(1) <= dx::kMaxTopk, "num_topk too large");
-        DX_CHECK(num_experts % R == 0 && count.numel() == num_experts / R && range.numel() == (int64_t)(num_experts / R) * R, "bad output shapes");
-        dxh::LowLatencyLayout lay(rt->core->ll_base(), num_max_tokens, H, R, num_experts);
-        DX_CHECK(lay.total_bytes <= rt->core->ll_bytes(), "low-latency region too small: create the Buffer with num_rdma_bytes >= get_low_latency_rdma_size_hint(...)");
-        dx::LLDispatchArgs& a = args[v];
-        a.ctx = rt->core->ctx();
-        a.parity = parity;
-        a.region = make_region(lay);
-        a.x = reinterpret_cast<const __nv_bfloat16*>(x.data_ptr());
-        a.topk_idx = topk_idx.data_ptr<int64_t>();
-        a.num_tokens = T;
-        a.hidden = H;
-        a.num_topk = (int)topk_idx.size(1);
-        a.num_experts = num_experts;
-        a.num_max_tokens = num_max_tokens;
-        a.use_fp8 = use_fp8;
-        a.round_scale = round_scale;
-        a.use_ue8m0 = use_ue8m0;
-        a.phases = phases;
-        a.packed_recv_count = count.data_ptr<int>();
-        a.layout_range = range.data_ptr<int64_t>();
-        a.cumulative_stats = ptr_or_null<int>(cum);
-        a.wait_cost_stats = ptr_or_null<int64_t>(wait);
-        if (slot.has_value())
-            DX_CHECK(slot->is_cuda() && slot->scalar_type() == torch::kInt32 && slot->is_contiguous() && slot->numel() >= (int64_t)T * topk_idx.size(1), "send_row must be int32 [T,K] on the GPU");
-        a.send_row = ptr_or_null<int>(slot);
-        a.num_sms = num_sms;
+        fill_ll_dispatch(args[v], rts[v], t[0].cast<torch::Tensor>(), t[1].cast<torch::Tensor>(), t[2].cast<torch::Tensor>(), t[3].cast<torch::Tensor>(),
+                         opt_tensor(t[4]), opt_tensor(t[5]), opt_tensor(t[6]), num_max_tokens, num_experts, use_fp8, round_scale, use_ue8m0, parity, phases, num_sms);
     }
     check_launch(dx::launch_ll_dispatch(args.data(), V, cur_stream(rts[0])), "low_latency_dispatch");
 }
 
-// Per rank tuple: (x, topk_idx, topk_weights, src_info, layout_range, out, wait_stats|None, send_row|None)
+// One rank and both halves, the call of a decode step: its arguments come one by one instead of in lists and tuples.
+void ll_dispatch_one(Runtime* rt, const torch::Tensor& x, const torch::Tensor& topk_idx, const torch::Tensor& count, const torch::Tensor& range,
+                     const OptTensor& cum, const OptTensor& wait, const torch::Tensor& slot, int num_max_tokens, int num_experts, bool use_fp8,
+                     bool round_scale, bool use_ue8m0, int parity, int num_sms) {
+    c10::cuda::CUDAGuard guard(rt->core->device());
+    dx::LLDispatchArgs a{};
+    fill_ll_dispatch(a, rt, x, topk_idx, count, range, cum, wait, slot, num_max_tokens, num_experts, use_fp8, round_scale, use_ue8m0, parity, 3, num_sms);
+    check_launch(dx::launch_ll_dispatch(&a, 1, cur_stream(rt)), "low_latency_dispatch");
+}
+
 // pull: x of every rank lives in its symmetric buffer and send_row comes from the dispatch of the same handle; the home
 // ranks read the rows in place. close_barrier: readers report back before the kernel ends (x is not the zero-copy buffer).
+void fill_ll_combine(dx::LLCombineArgs& a, Runtime* rt, const torch::Tensor& x, const torch::Tensor& topk_idx, const torch::Tensor& topk_w,
+                     const torch::Tensor& src_info, const torch::Tensor& range, const torch::Tensor& out, const OptTensor& wait, const OptTensor& send_row,
+                     int num_max_tokens, int num_experts, int parity, int phases, int num_sms, bool pull, bool close_barrier) {
+    const int R = rt->core->num_ranks();
+    const int L = num_experts / R;
+    DX_CHECK(x.is_cuda() && x.dim() == 3 && x.is_contiguous() && x.scalar_type() == torch::kBFloat16 && x.size(0) == L && x.size(1) == (int64_t)R * num_max_tokens, "x must be contiguous bf16 [L, R*max_tokens, hidden] on the GPU");
+    DX_CHECK(x.device().index() == rt->core->device() && topk_idx.is_cuda() && topk_w.is_cuda() && src_info.is_cuda() && range.is_cuda() &&
+                 topk_idx.device() == x.device() && topk_w.device() == x.device(), "low_latency_combine: inputs must live on this rank's GPU");
+    // the result may go to device memory or straight to pinned (page-locked, device-mapped) host memory
+    DX_CHECK((out.is_cuda() && out.device() == x.device()) || (out.device().is_cpu() && out.is_pinned()), "out must be on this rank's GPU or in pinned host memory");
+    const int H = (int)x.size(2);
+    DX_CHECK(topk_idx.scalar_type() == torch::kInt64 && topk_idx.is_contiguous() && topk_idx.dim() == 2, "topk_idx must be int64 [T,K]");
+    const int T = (int)topk_idx.size(0);
+    DX_CHECK(T <= num_max_tokens && topk_idx.size(1) <= dx::kMaxTopk, "too many tokens or top-k entries");
+    DX_CHECK(topk_w.scalar_type() == torch::kFloat32 && topk_w.is_contiguous() && topk_w.numel() == topk_idx.numel(), "topk_weights must be f32 [T,K]");
+    DX_CHECK(src_info.scalar_type() == torch::kInt32 && src_info.is_contiguous() && src_info.numel() == (int64_t)L * R * num_max_tokens, "src_info must be int32 [L,N]");
+    DX_CHECK(range.scalar_type() == torch::kInt64 && range.is_contiguous() && range.numel() == (int64_t)L * R, "layout_range must be int64 [L,R]");
+    DX_CHECK(out.scalar_type() == torch::kBFloat16 && out.is_contiguous() && out.size(0) == T && out.size(1) == H, "out must be bf16 [T,hidden]");
+    dxh::LowLatencyLayout lay(rt->core->ll_base(), num_max_tokens, H, R, num_experts);
+    DX_CHECK(lay.total_bytes <= rt->core->ll_bytes(), "low-latency region too small");
+    a.ctx = rt->core->ctx();
+    a.parity = parity;
+    a.region = make_region(lay);
+    a.x = reinterpret_cast<const __nv_bfloat16*>(x.data_ptr());
+    a.topk_idx = topk_idx.data_ptr<int64_t>();
+    a.topk_weights = topk_w.data_ptr<float>();
+    a.src_info = src_info.data_ptr<int>();
+    a.layout_range = range.data_ptr<int64_t>();
+    a.out = reinterpret_cast<__nv_bfloat16*>(out.data_ptr());
+    a.wait_cost_stats = ptr_or_null<int64_t>(wait);
+    a.num_tokens = T;
+    a.hidden = H;
+    a.num_topk = (int)topk_idx.size(1);
+    a.num_experts = num_experts;
+    a.num_max_tokens = num_max_tokens;
+    a.phases = phases;
+    a.num_sms = num_sms;
+    a.pull = pull ? 1 : 0;
+    a.close_barrier = (pull && close_barrier) ? 1 : 0;
+    a.x_off = 0;
+    a.send_row = nullptr;
+    if (send_row.has_value()) {
+        DX_CHECK(send_row->is_cuda() && send_row->scalar_type() == torch::kInt32 && send_row->is_contiguous() &&
+                     send_row->numel() >= (int64_t)T * topk_idx.size(1), "send_row must be int32 [T,K] on the GPU");
+        a.send_row = send_row->data_ptr<int>();
+    }
+    if (pull) {
+        const int64_t xo = rt->symmetric_offset(x);
+        DX_CHECK(xo >= 0 && xo % 16 == 0, "pull combine: x must live in this rank's symmetric buffer");
+        DX_CHECK(send_row.has_value(), "pull combine: send_row is missing");
+        a.x_off = (uint64_t)xo;
+    }
+}
+
+// Per rank tuple: (x, topk_idx, topk_weights, src_info, layout_range, out, wait_stats|None, send_row|None)
 void ll_combine(std::vector<Runtime*> rts, std::vector<py::tuple> per_rank, int num_max_tokens, int num_experts, int parity, int phases,
                 int num_sms, bool pull, bool close_barrier) {
     const int V = (int)rts.size();
@@ -685,69 +749,28 @@ void ll_combine(std::vector<Runtime*> rts, std::vector<py::tuple> per_rank, int 
     c10::cuda::CUDAGuard guard(rts[0]->core->device());
     std::vector<dx::LLCombineArgs> args(V);
     for (int v = 0; v < V; ++v) {
-        Runtime* rt = rts[v];
         const py::tuple& t = per_rank[v];
         DX_CHECK(t.size() == 8, "ll_combine: per-rank tuple must have 8 entries");
-        auto x = t[0].cast<torch::Tensor>();
-        auto send_row = opt_tensor(t[7]);
-        auto topk_idx = t[1].cast<torch::Tensor>();
-        auto topk_w = t[2].cast<torch::Tensor>();
-        auto src_info = t[3].cast<torch::Tensor>();
-        auto range = t[4].cast<torch::Tensor>();
-        auto out = t[5].cast<torch::Tensor>();
-        auto wait = opt_tensor(t[6]);
-        const int R = rt->core->num_ranks();
-        const int L = num_experts / R;
-        DX_CHECK(x.is_cuda() && x.dim() == 3 && x.is_contiguous() && x.scalar_type() == torch::kBFloat16 && x.size(0) == L && x.size(1) == (int64_t)R * num_max_tokens, "x must be contiguous bf16 [L, R*max_tokens, hidden] on the GPU");
-        DX_CHECK(x.device().index() == rt->core->device() && topk_idx.is_cuda() && topk_w.is_cuda() && src_info.is_cuda() && range.is_cuda() &&
-                     topk_idx.device() == x.device() && topk_w.device() == x.device(), "low_latency_combine: inputs must live on this rank's GPU");
-        // the result may go to device memory or straight to pinned (page-locked, device-mapped) host memory
-        DX_CHECK((out.is_cuda() && out.device() == x.device()) || (out.device().is_cpu() && out.is_pinned()), "out must be on this rank's GPU or in pinned host memory");
-        const int H = (int)x.size(2);
-        DX_CHECK(topk_idx.scalar_type() == torch::kInt64 && topk_idx.is_contiguous() && topk_idx.dim() == 2, "topk_idx must be int64 [T,K]");
-        const int T = (int)topk_idx.size(0);
-        DX_CHECK(T <= num_max_tokens && topk_idx.size(1) <= dx::kMaxTopk, "too many tokens or top-k entries");
-        DX_CHECK(topk_w.scalar_type() == torch::kFloat32 && topk_w.is_contiguous() && topk_w.numel() == topk_idx.numel(), "topk_weights must be f32 [T,K]");
-        DX_CHECK(src_info.scalar_type() == torch::kInt32 && src_info.is_contiguous() && src_info.numel() == (int64_t)L * R * num_max_tokens, "src_info must be int32 [L,N]");
-        DX_CHECK(range.scalar_type() == torch::kInt64 && range.is_contiguous() && range.numel() == (int64_t)L * R, "layout_range must be int64 [L,R]");
-        DX_CHECK(out.scalar_type() == torch::kBFloat16 && out.is_contiguous() && out.size(0) == T && out.size(1) == H, "out must be bf16 [T,hidden]");
-        dxh::LowLatencyLayout lay(rt->core->ll_base(), num_max_tokens, H, R, num_experts);
-        DX_CHECK(lay.total_bytes <= rt->core->ll_bytes(), "low-latency region too small");
-        dx::LLCombineArgs& a = args[v];
-        a.ctx = rt->core->ctx();
-        a.parity = parity;
-        a.region = make_region(lay);
-        a.x = reinterpret_cast<const __nv_bfloat16*>(x.data_ptr());
-        a.topk_idx = topk_idx.data_ptr<int64_t>();
-        a.topk_weights = topk_w.data_ptr<float>();
-        a.src_info = src_info.data_ptr<int>();
-        a.layout_range = range.data_ptr<int64_t>();
-        a.out = reinterpret_cast<__nv_bfloat16*>(out.data_ptr());
-        a.wait_cost_stats = ptr_or_null<int64_t>(wait);
-        a.num_tokens = T;
-        a.hidden = H;
-        a.num_topk = (int)topk_idx.size(1);
-        a.num_experts = num_experts;
-        a.num_max_tokens = num_max_tokens;
-        a.phases = phases;
-        a.num_sms = num_sms;
-        a.pull = pull ? 1 : 0;
-        a.close_barrier = (pull && close_barrier) ? 1 : 0;
-        a.x_off = 0;
-        a.send_row = nullptr;
-        if (send_row.has_value()) {
-            DX_CHECK(send_row->is_cuda() && send_row->scalar_type() == torch::kInt32 && send_row->is_contiguous() &&
-                         send_row->numel() >= (int64_t)T * topk_idx.size(1), "send_row must be int32 [T,K] on the GPU");
-            a.send_row = send_row->data_ptr<int>();
-        }
-        if (pull) {
-            const int64_t xo = rt->symmetric_offset(x);
-            DX_CHECK(xo >= 0 && xo % 16 == 0, "pull combine: x must live in this rank's symmetric buffer");
-            DX_CHECK(send_row.has_value(), "pull combine: send_row is missing");
-            a.x_off = (uint64_t)xo;
-        }
+        fill_ll_combine(args[v], rts[v], t[0].cast<torch::Tensor>(), t[1].cast<torch::Tensor>(), t[2].cast<torch::Tensor>(), t[3].cast<torch::Tensor>(),
+                        t[4].cast<torch::Tensor>(), t[5].cast<torch::Tensor>(), opt_tensor(t[6]), opt_tensor(t[7]), num_max_tokens, num_experts, parity, phases,
+                        num_sms, pull, close_barrier);
     }
     check_launch(dx::launch_ll_combine(args.data(), V, cur_stream(rts[0])), "low_latency_combine");
+}
+
+// One rank and both halves; `zero_copy` is this parity's zero-copy buffer. Returns the result, allocated here unless given.
+torch::Tensor ll_combine_one(Runtime* rt, const torch::Tensor& x, const torch::Tensor& topk_idx, const torch::Tensor& topk_w, const torch::Tensor& src_info,
+                             const torch::Tensor& range, const OptTensor& out, const OptTensor& wait, const torch::Tensor& send_row,
+                             const torch::Tensor& zero_copy, int num_max_tokens, int num_experts, int parity, int num_sms) {
+    c10::cuda::CUDAGuard guard(rt->core->device());
+    const bool pull = rt->symmetric_offset(x) >= 0;
+    // a caller-owned tensor: its owner may rewrite it as soon as the call returns
+    const bool close_barrier = pull && x.data_ptr() != zero_copy.data_ptr();
+    const torch::Tensor result = out.has_value() ? *out : torch::empty({topk_idx.size(0), zero_copy.size(2)}, topk_idx.options().dtype(torch::kBFloat16));
+    dx::LLCombineArgs a{};
+    fill_ll_combine(a, rt, x, topk_idx, topk_w, src_info, range, result, wait, send_row, num_max_tokens, num_experts, parity, 3, num_sms, pull, close_barrier);
+    check_launch(dx::launch_ll_combine(&a, 1, cur_stream(rt)), "low_latency_combine");
+    return result;
 }
 
 // Offsets of the low-latency region for the Python layer (views are created there once and cached).
@@ -860,6 +883,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
           py::arg("group_counts") = py::none(), py::arg("rows_per_group") = 1, py::arg("out_q") = py::none(), py::arg("out_s") = py::none(),
           py::arg("num_rows_dev") = py::none(), py::arg("atoms") = false);
     m.def("ll_dispatch", &ll_dispatch);
+    m.def("ll_dispatch_one", &ll_dispatch_one);
+    m.def("ll_combine_one", &ll_combine_one);
     m.def("ll_combine", &ll_combine, py::arg("runtimes"), py::arg("per_rank"), py::arg("num_max_tokens"), py::arg("num_experts"),
           py::arg("parity"), py::arg("phases"), py::arg("num_sms"), py::arg("pull") = false, py::arg("close_barrier") = false);
     m.def("ll_layout", &ll_layout);

@@ -26,6 +26,12 @@ def _has_cuda() -> bool:
     return _HAS_CUDA
 
 
+def current_stream() -> "torch.cuda.Stream":
+    """``torch.cuda.current_stream()``. Told the device by number it need not work out which one is meant, which takes longer (about 4 us)
+    than all the rest."""
+    return torch.cuda.current_stream(torch.cuda.current_device())
+
+
 class EventHandle:
     """A CUDA event recorded on ``stream`` (default: the current stream) when created.
 
@@ -36,11 +42,11 @@ class EventHandle:
         if _has_cuda():
             self.event = torch.cuda.Event(enable_timing=False)
             if record:
-                self.event.record(stream if stream is not None else torch.cuda.current_stream())
+                self.event.record(stream if stream is not None else current_stream())
 
     def current_stream_wait(self) -> None:
         if self.event is not None:
-            torch.cuda.current_stream().wait_event(self.event)
+            current_stream().wait_event(self.event)
 
 
 class EventOverlap:

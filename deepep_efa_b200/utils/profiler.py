@@ -23,7 +23,7 @@ PROFILE_ENABLED = os.environ.get("DEEPEP_PROFILE", "0") == "1"
 PROFILE_INTERVAL = int(os.environ.get("DEEPEP_PROFILE_INTERVAL", "50"))
 PROFILE_WARMUP = int(os.environ.get("DEEPEP_PROFILE_WARMUP", "10"))
 
-_NVTX = os.environ.get("DEEPEP_NVTX", "0") == "1"
+NVTX_ENABLED = os.environ.get("DEEPEP_NVTX", "0") == "1"
 
 
 _NO_RANGE = contextlib.nullcontext()
@@ -31,7 +31,7 @@ _NO_RANGE = contextlib.nullcontext()
 
 def nvtx_range(name: str):
     """NVTX range when ``DEEPEP_NVTX=1`` and CUDA is present; otherwise free."""
-    return _nvtx_range(name) if _NVTX and torch.cuda.is_available() else _NO_RANGE
+    return _nvtx_range(name) if NVTX_ENABLED and torch.cuda.is_available() else _NO_RANGE
 
 
 @contextlib.contextmanager
