@@ -418,7 +418,118 @@ __global__ void __launch_bounds__(kDispatchThreads, 1) dispatch_kernel(const __g
     }
 }
 
+// A lone rank that may use the whole GPU: the rows only move within its memory, at the speed of a copy. A warp takes one piece of one row
+// (2 KB to read when it casts, 4 KB otherwise), asks for all of it together with the row's place, stores it and ends; five or six CTAs of eight
+// such warps share an SM. With a warp per row that walked over its columns, 32 to an SM, a row of 14 KB was seven dependent steps (one B200,
+// 4096 x 7168: cast to FP8 31.4 -> 19.2 us, back in BF16 27.4 -> 17.5 us with what overlaps the predecessor; 3001 x 4096 in BF16 with one
+// bias 11.5 -> 8.0 and 18.3 -> 12.0 us).
+constexpr int kLoneThreads = 256;
+constexpr int kLoneWarps = kLoneThreads / 32;
+
+template <bool kQuant>
+__global__ void __launch_bounds__(kLoneThreads, kQuant ? 5 : 4) dispatch_lone_kernel(const __grid_constant__ DispatchArgs a, const int pieces) {
+    pdl_wait_predecessor();
+    pdl_release_successor();
+    const RankCtx& c = a.ctx;
+    const int T = a.num_tokens, K = a.num_topk, H = a.hidden;
+    const int lane = threadIdx.x & 31;
+    const long long item = (long long)blockIdx.x * kLoneWarps + (threadIdx.x >> 5);
+    if (item < (long long)T * pieces) {
+        const int t = (int)(item / pieces), piece = (int)(item % pieces);
+        const size_t out_row_bytes = (size_t)H * (kQuant ? 1 : a.x_elem_bytes);
+        char* out = c.at<char>(0, a.recv_x_off);
+        float* scales = c.at<float>(0, a.recv_scales_off);
+        constexpr int U = kQuant ? 4 : 8;
+        int4 v[U];
+        const int n16 = (int)(out_row_bytes / 16);
+        const int ch = piece * 1024 + lane * 16;  // casting: 16 channels here and 16 in the other half of the piece
+        const int col = piece * 32 * U + lane;    // copying
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            v[u] = make_int4(0, 0, 0, 0);
+            if constexpr (kQuant) {
+                const int at = ch + (u >> 1) * 512;
+                if (at < H) v[u] = ld_stream(reinterpret_cast<const int4*>(reinterpret_cast<const char*>(a.x) + ((size_t)t * H + at) * 2) + (u & 1));
+            } else {
+                if (col + u * 32 < n16) v[u] = ld_stream(reinterpret_cast<const int4*>(reinterpret_cast<const char*>(a.x) + (size_t)t * out_row_bytes) + col + u * 32);
+            }
+        }
+        int row = a.send_head[t];
+        if (row >= 0 && !peer_range_ok(c, 0, out + (size_t)row * out_row_bytes, out_row_bytes, 1)) row = -1;
+        if (row >= 0) {
+            char* dst = out + (size_t)row * out_row_bytes;
+            if constexpr (kQuant) {
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int at = ch + h * 512;
+                    const int4 r0 = v[2 * h], r1 = v[2 * h + 1];
+                    const uint32_t w[8] = {(uint32_t)r0.x, (uint32_t)r0.y, (uint32_t)r0.z, (uint32_t)r0.w,
+                                           (uint32_t)r1.x, (uint32_t)r1.y, (uint32_t)r1.z, (uint32_t)r1.w};
+                    float f[16];
+                    float amax = 0.f;
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        const float2 p = bf16x2_to_f2(w[j]);
+                        f[2 * j] = p.x;
+                        f[2 * j + 1] = p.y;
+                        amax = fmaxf(amax, fmaxf(fabsf(p.x), fabsf(p.y)));
+                    }
+                    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+                    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+                    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 4));
+                    float scale, inv;
+                    fp8_scale_from_amax(amax, a.round_scale != 0, scale, inv);
+                    int4 q;
+                    q.x = (int)pack_e4m3x4(f[0] * inv, f[1] * inv, f[2] * inv, f[3] * inv);
+                    q.y = (int)pack_e4m3x4(f[4] * inv, f[5] * inv, f[6] * inv, f[7] * inv);
+                    q.z = (int)pack_e4m3x4(f[8] * inv, f[9] * inv, f[10] * inv, f[11] * inv);
+                    q.w = (int)pack_e4m3x4(f[12] * inv, f[13] * inv, f[14] * inv, f[15] * inv);
+                    if (at < H) {
+                        st_stream(reinterpret_cast<int4*>(dst + at), q);
+                        if ((lane & 7) == 0) scales[(size_t)row * (H / 128) + (at >> 7)] = scale;
+                    }
+                }
+            } else {
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    if (col + u * 32 < n16) st_stream(reinterpret_cast<int4*>(dst) + col + u * 32, v[u]);
+                if (a.x_scales != nullptr && piece == 0)
+                    for (int i = lane; i < H / 128; i += 32) scales[(size_t)row * (H / 128) + i] = a.x_scales[(size_t)t * (H / 128) + i];
+            }
+            if (piece == 0) {
+                if (a.topk_idx != nullptr && lane < K) {
+                    const int64_t e = a.topk_idx[(size_t)t * K + lane];
+                    const bool mine = e >= 0 && e < a.num_experts;
+                    c.at<int64_t>(0, a.recv_topk_idx_off)[(size_t)row * K + lane] = mine ? e : -1;
+                    if (a.topk_weights != nullptr) c.at<float>(0, a.recv_topk_w_off)[(size_t)row * K + lane] = mine ? a.topk_weights[(size_t)t * K + lane] : 0.f;
+                }
+                if (lane == 0) c.at<int>(0, a.recv_src_idx_off)[row] = t;
+            }
+        }
+    }
+    if (a.num_worst_tokens > 0 && a.topk_idx != nullptr) {  // see dispatch_kernel
+        const int num_recv = a.rank_prefix_matrix[0];
+        int64_t* mine = c.at<int64_t>(0, a.recv_topk_idx_off);
+        const size_t lo = (size_t)num_recv * K, hi = (size_t)a.num_worst_tokens * K;
+        for (size_t i = lo + (size_t)blockIdx.x * kLoneThreads + threadIdx.x; i < hi; i += (size_t)gridDim.x * kLoneThreads) mine[i] = -1;
+    }
+}
+
+// Whether the call is a lone rank's that nobody asked to leave SMs to something else.
+template <typename Args>
+bool lone_and_unbounded(const Args* a, int nv) { return nv == 1 && a->ctx.num_ranks == 1 && a->num_sms >= 148; }
+
 cudaError_t launch_dispatch(const DispatchArgs* a, int nv, cudaStream_t stream) {
+    if (lone_and_unbounded(a, nv)) {
+        const bool quant = a->quantize != 0;
+        const int pieces = quant ? (a->hidden + 1023) / 1024 : (a->hidden * a->x_elem_bytes / 16 + 255) / 256;
+        const long long ids = (long long)a->num_worst_tokens * (a->topk_idx != nullptr ? a->num_topk : 0);
+        const long long moving = ((long long)a->num_tokens * std::max(pieces, 1) + kLoneWarps - 1) / kLoneWarps;
+        const long long marking = std::min<long long>((ids + 8 * kLoneThreads - 1) / (8 * kLoneThreads), 4 * 148);
+        const unsigned ctas = (unsigned)std::max<long long>(1, std::max(moving, marking));
+        return quant ? launch_dependent(dispatch_lone_kernel<true>, dim3(ctas), kLoneThreads, 0, stream, *a, std::max(pieces, 1))
+                     : launch_dependent(dispatch_lone_kernel<false>, dim3(ctas), kLoneThreads, 0, stream, *a, std::max(pieces, 1));
+    }
     // few tokens with outputs for many rows: enough CTAs that no thread marks more than eight unused ids
     const long long ids = (long long)a[0].num_worst_tokens * (a[0].topk_idx != nullptr ? a[0].num_topk : 0);
     const long long marking = (ids + 8 * kDispatchThreads - 1) / (8 * kDispatchThreads);
@@ -568,7 +679,73 @@ __global__ void __launch_bounds__(kCombineThreads, 1) combine_kernel(const __gri
     }
 }
 
+// The lone rank's form, as in dispatch: a warp takes 256 sixteen-byte columns of a row, or 128 where biases come on top, and has all of
+// its loads in flight.
+template <int kBiases>
+constexpr int kCombineLoneLoads = kBiases == 0 ? 8 : 4;
+
+template <int kBiases>
+__global__ void __launch_bounds__(kLoneThreads, kBiases == 2 ? 3 : 4) combine_lone_kernel(const __grid_constant__ CombineArgs a, const int pieces) {
+    pdl_wait_predecessor();
+    pdl_release_successor();
+    const RankCtx& c = a.ctx;
+    const int T = a.num_tokens, K = a.num_topk, n16 = a.hidden / 8;
+    const int lane = threadIdx.x & 31;
+    const long long item = (long long)blockIdx.x * kLoneWarps + (threadIdx.x >> 5);
+    if (item >= (long long)T * pieces) return;
+    const int t = (int)(item / pieces), piece = (int)(item % pieces);
+    constexpr int U = kCombineLoneLoads<kBiases>;
+    const int col = piece * 32 * U + lane;
+    const int4* bias[2] = {reinterpret_cast<const int4*>(a.bias0 != nullptr ? a.bias0 : a.bias1) + (size_t)t * n16,
+                           reinterpret_cast<const int4*>(a.bias1) + (size_t)t * n16};
+    int4 v[1 + kBiases][U];
+#pragma unroll
+    for (int b = 0; b < kBiases; ++b)
+#pragma unroll
+        for (int u = 0; u < U; ++u) v[1 + b][u] = col + u * 32 < n16 ? ld_stream(bias[b] + col + u * 32) : make_int4(0, 0, 0, 0);
+    const int head = a.send_head[t];
+    const int4* row = head >= 0 ? c.at<const int4>(0, a.x_off) + (size_t)head * n16 : nullptr;
+    if (row != nullptr && !peer_range_ok(c, 0, row, (size_t)n16 * 16, 2)) row = nullptr;
+#pragma unroll
+    for (int u = 0; u < U; ++u) v[0][u] = row != nullptr && col + u * 32 < n16 ? ld_stream(row + col + u * 32) : make_int4(0, 0, 0, 0);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        if (col + u * 32 >= n16) continue;
+        float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll
+        for (int b = 0; b <= kBiases; ++b) {
+            const uint32_t w[4] = {(uint32_t)v[b][u].x, (uint32_t)v[b][u].y, (uint32_t)v[b][u].z, (uint32_t)v[b][u].w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float2 p = bf16x2_to_f2(w[j]);
+                acc[2 * j] += p.x;
+                acc[2 * j + 1] += p.y;
+            }
+        }
+        int4 o;
+        o.x = (int)f2_to_bf16x2(acc[0], acc[1]);
+        o.y = (int)f2_to_bf16x2(acc[2], acc[3]);
+        o.z = (int)f2_to_bf16x2(acc[4], acc[5]);
+        o.w = (int)f2_to_bf16x2(acc[6], acc[7]);
+        st_stream(reinterpret_cast<int4*>(a.out) + (size_t)t * n16 + col + u * 32, o);
+    }
+    if (a.out_topk_w != nullptr && piece == 0 && lane < K)
+        a.out_topk_w[(size_t)t * K + lane] = row != nullptr && a.topk_w_off != ~0ull ? 0.f + c.at<const float>(0, a.topk_w_off)[(size_t)head * K + lane] : 0.f;
+}
+
+template <int kBiases>
+cudaError_t launch_combine_lone(const CombineArgs& a, cudaStream_t stream) {
+    const int span = 32 * kCombineLoneLoads<kBiases>, pieces = std::max((a.hidden / 8 + span - 1) / span, 1);
+    const long long ctas = ((long long)a.num_tokens * pieces + kLoneWarps - 1) / kLoneWarps;
+    if (ctas == 0) return cudaSuccess;
+    return launch_dependent(combine_lone_kernel<kBiases>, dim3((unsigned)ctas), kLoneThreads, 0, stream, a, pieces);
+}
+
 cudaError_t launch_combine(const CombineArgs* a, int nv, cudaStream_t stream) {
+    if (lone_and_unbounded(a, nv)) {
+        const int biases = (a->bias0 != nullptr ? 1 : 0) + (a->bias1 != nullptr ? 1 : 0);
+        return biases == 0 ? launch_combine_lone<0>(*a, stream) : biases == 1 ? launch_combine_lone<1>(*a, stream) : launch_combine_lone<2>(*a, stream);
+    }
     return DX_LAUNCH_RANKED_PDL(combine_kernel, CombineArgs, a, nv, grid_ctas(a, nv), kCombineThreads, 0, stream);
 }
 

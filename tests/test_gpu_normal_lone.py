@@ -1,0 +1,53 @@
+"""Normal mode of a lone rank: the kernels that take the whole GPU against the general ones, which a caller's own config still selects."""
+import pytest
+import torch
+
+from helpers import make_routing, make_tokens
+
+pytestmark = pytest.mark.gpu
+
+
+# fewer tokens than a CTA has warps, hidden sizes below, at and past the pieces of a row (1024 channels when casting, 256 and 128 columns of 16
+# bytes otherwise) and not a multiple of them, tokens that nobody selected
+@pytest.mark.parametrize("T,H,masked", [(1, 128, 0.0), (3, 896, 0.5), (7, 1024, 0.0), (61, 1152, 0.6), (200, 2048, 0.6), (33, 2176, 0.0), (129, 4224, 0.5),
+                                        (64, 8192, 0.0)])
+@pytest.mark.parametrize("wire", ["bf16", "fp8", "cast", "cast_pow2"])
+def test_lone_rank_matches_general_kernels(T, H, masked, wire):
+    from deepep_efa_b200 import Config
+    from deepep_efa_b200.parallel.virtual import VirtualCluster
+    E, K = 8, 2
+    vc = VirtualCluster(1, num_nvl_bytes=64 << 20, timeout_ms=2000)
+    try:
+        buf = vc.buffers[0]
+        idx, w = make_routing(T, E, K, "cuda", seed=T, masked_fraction=masked)
+        x = make_tokens(T, H, "cuda", seed=H)
+        if wire == "fp8":
+            x = (x.to(torch.float8_e4m3fn), torch.rand(T, H // 128, device="cuda"))
+        per_rank, _, per_expert, in_rank, _ = buf.get_dispatch_layout(idx, E)
+        res = []
+        for config in (Config(24), None):
+            for worst in (0, T + 5):
+                rx, ri, rw, counts, handle, _ = buf.dispatch(
+                    x, num_tokens_per_rank=per_rank, is_token_in_rank=in_rank, num_tokens_per_expert=per_expert, topk_idx=idx, topk_weights=w, config=config,
+                    quantize_fp8=wire.startswith("cast"), round_scale=wire == "cast_pow2", num_worst_tokens=worst)
+                n = int(per_rank.item())
+                flat = list(rx) if isinstance(rx, tuple) else [rx]
+                out = [t[:n].view(torch.uint8).clone() for t in flat] + [ri.clone() if worst else ri[:n].clone(), rw[:n].clone(), handle[3][:n].clone()]
+                if worst:
+                    assert (ri[n:] == -1).all()
+                    res.append(out)
+                    continue
+                y = torch.randn(n, H, device="cuda", generator=torch.Generator("cuda").manual_seed(1)).to(torch.bfloat16)
+                bias = [make_tokens(T, H, "cuda", seed=s) for s in (5, 6)]
+                for b in (None, bias[0], tuple(bias)):
+                    for placed in (y, buf.empty_symmetric([n, H], torch.bfloat16).copy_(y)):
+                        z, zw, _ = buf.combine(placed, handle, topk_weights=rw, bias=b, config=config)
+                        out += [z.clone(), zw.clone()]
+                cached = buf.dispatch(x, handle=handle, config=config)[0]
+                out += [t.view(torch.uint8).clone() for t in (cached if isinstance(cached, tuple) else (cached,))]
+                res.append(out)
+        buf.check_status(sync=True)
+        for a, b in zip(res[:2], res[2:]):
+            assert len(a) == len(b) and all(torch.equal(p, q) for p, q in zip(a, b))
+    finally:
+        vc.destroy()
