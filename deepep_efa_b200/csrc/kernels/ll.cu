@@ -963,8 +963,9 @@ __global__ void __launch_bounds__(kLLThreads, 1) combine_pull(const __grid_const
 // their memory may be a block that the predecessor still reads (freed by the caller between the two calls).
 // kFind (x is an ordinary tensor): src_info decides which row of the expert is the token's, so that the selections of a token may come in
 // another order than at the dispatch, as with the staged form. It is loaded with the row itself; the search is for the odd case.
+// (Two CTAs of 512 threads to an SM: the 64 registers that leaves let the 896 CTAs of 128 threads of 128 tokens x 7168 be resident at once.)
 template <bool kFind>
-__global__ void __launch_bounds__(kLLThreads) combine_lone(const __grid_constant__ LLCombineArgs a, const int slices) {
+__global__ void __launch_bounds__(kLLThreads, 2) combine_lone(const __grid_constant__ LLCombineArgs a, const int slices) {
     pdl_release_successor();
     const RankCtx& c = a.ctx;
     const int T = a.num_tokens, K = a.num_topk, E = a.num_experts, N = a.num_max_tokens, n16 = a.hidden / 8;
@@ -1000,8 +1001,10 @@ __global__ void __launch_bounds__(kLLThreads) combine_lone(const __grid_constant
             if (e64 >= 0 && e64 < E && !masked) e = (int)e64;
             if (e >= 0 && row >= 0 && row < N) slot = e * N + row;
         }
+        int info = t;
+        if (kFind && !early && slot >= 0) info = __ldcg(a.src_info + slot);
         float acc[8];
-        auto gather = [&]() {
+        for (bool sure = !kFind;; sure = true) {
 #pragma unroll
             for (int j = 0; j < 8; ++j) acc[j] = 0.f;
             for (int k0 = 0; k0 < K; k0 += 8) {
@@ -1025,22 +1028,16 @@ __global__ void __launch_bounds__(kLLThreads) combine_lone(const __grid_constant
                     }
                 }
             }
-        };
-        int info = t;
-        if (kFind && !early && slot >= 0) info = __ldcg(a.src_info + slot);
-        gather();
-        if (early) pdl_wait_predecessor();  // from here on everything is final; returns at once in later rounds of the loop
-        if constexpr (kFind) {
+            if (early) pdl_wait_predecessor();  // from here on everything is final; returns at once in later rounds
+            if (sure) break;
             if (early && slot >= 0) info = __ldcg(a.src_info + slot);
             const bool wrong = e >= 0 && (slot < 0 || info != t);
-            if (__any_sync(0xffffffffu, wrong)) {
-                if (wrong) {
-                    slot = -1;
-                    const int rows = min((int)(a.layout_range[e] & 0xffffffff), N);
-                    for (int n = 0; n < rows && slot < 0; ++n)
-                        if (__ldcg(a.src_info + (size_t)e * N + n) == t) slot = e * N + n;
-                }
-                gather();
+            if (!__any_sync(0xffffffffu, wrong)) break;
+            if (wrong) {
+                slot = -1;
+                const int rows = min((int)(a.layout_range[e] & 0xffffffff), N);
+                for (int n = 0; n < rows && slot < 0; ++n)
+                    if (__ldcg(a.src_info + (size_t)e * N + n) == t) slot = e * N + n;
             }
         }
         if (col < n16) {
