@@ -65,7 +65,7 @@ torch::Tensor grouped_gemm(const torch::Tensor& a, const torch::Tensor& b, const
                            c10::optional<torch::Tensor> ready, c10::optional<torch::Tensor> expected,
                            c10::optional<torch::Tensor> row_info, c10::optional<torch::Tensor> scatter_bases,
                            c10::optional<torch::Tensor> trace, bool mn_major, c10::optional<torch::Tensor> out_fp8,
-                           c10::optional<torch::Tensor> out_atoms, bool m_ends_are_counts, c10::optional<torch::Tensor> sched, bool early_table, bool tokens_as_columns,
+                           c10::optional<torch::Tensor> out_atoms, bool m_ends_are_counts, c10::optional<torch::Tensor> sched, bool early_table, int tokens_as_columns,
                            bool hold_successor) {
     DXG_CHECK(a.is_cuda() && b.is_cuda() && m_offsets.is_cuda(), "operands must be CUDA tensors");
     DXG_CHECK(a.is_contiguous() && b.is_contiguous() && m_offsets.is_contiguous(), "operands must be contiguous");
@@ -182,6 +182,13 @@ torch::Tensor grouped_gemm(const torch::Tensor& a, const torch::Tensor& b, const
         p.row_info = row_info->data_ptr<int>();
         p.scatter_bases = reinterpret_cast<const unsigned long long*>(scatter_bases->data_ptr());
     }
+    // The caller says that groups have few rows, and how many a tile may have (1: the ordinary choice). The natively block-scaled 256-column
+    // tiles have the form with the weights as M; SwiGLU then quantises its output.
+    const bool columns = tokens_as_columns != 0 && p.m_ends != nullptr && p.sfa_atoms != nullptr && p.mx_wide && p.n % 256 == 0 && (!swiglu || out_fp8.has_value());
+    if (columns) {
+        p.token_cap = tokens_as_columns == 1 ? 128 : tokens_as_columns;
+        DXG_CHECK(p.token_cap >= 64 && p.token_cap <= 224 && p.token_cap % 32 == 0, "tokens_as_columns must be 0, 1 or a multiple of 32 from 64 to 224");
+    }
     if (out_fp8.has_value() || out_atoms.has_value()) {
         DXG_CHECK(out_fp8.has_value() && out_atoms.has_value() && same_dev(out_fp8) && same_dev(out_atoms), "out_fp8 and out_atoms go together, on A's device");
         DXG_CHECK(mode == 0 && swiglu && p.sfa_atoms != nullptr && p.mx_wide == 1, "quantised output needs the natively block-scaled kernel with wide SwiGLU tiles");
@@ -202,12 +209,9 @@ torch::Tensor grouped_gemm(const torch::Tensor& a, const torch::Tensor& b, const
         DXG_CHECK(trace->element_size() == 8 && trace->is_contiguous() && trace->numel() >= 4, "trace must be 64-bit [4]");
         p.trace = reinterpret_cast<unsigned long long*>(trace->data_ptr());
     }
-    // The caller says that groups have few rows. Only the natively block-scaled 256-column tiles without a scatter have the form with
-    // the weights as M; SwiGLU then quantises its output.
-    p.swap = (tokens_as_columns && p.m_ends != nullptr && p.sfa_atoms != nullptr && p.mx_wide && !p.cta_pairs && p.row_info == nullptr && (!swiglu || p.c_fp8 != nullptr)) ? 1 : 0;
     p.error_flag = error_flag(device).data_ptr<int>();
     p.timeout_cycles = (long long)(timeout_ms * (double)clock_khz(device));
-    const cudaError_t e = dx::launch_grouped_gemm(p, at::cuda::getCurrentCUDAStream(device).stream());
+    const cudaError_t e = (columns ? dx::launch_token_cols_gemm : dx::launch_grouped_gemm)(p, at::cuda::getCurrentCUDAStream(device).stream());
     if (e == cudaErrorInvalidValue) {
         cudaGetLastError();
         throw std::invalid_argument(
@@ -221,8 +225,8 @@ torch::Tensor grouped_gemm(const torch::Tensor& a, const torch::Tensor& b, const
     return c;
 }
 
-// counts: 128-aligned rows per local expert. Returns (pos [N,K], src_row [m_pad], src_k [m_pad], m_offsets [L+1], m_pad).
-std::tuple<torch::Tensor, torch::Tensor, torch::Tensor, torch::Tensor, int64_t> build_plan(const torch::Tensor& topk_idx, const std::vector<int>& counts) {
+// counts: 128-aligned rows per local expert. Returns (pos [N,K], src_row [m_pad], src_k [m_pad], m_offsets [L+1], m_pad, m_ends [L]).
+std::tuple<torch::Tensor, torch::Tensor, torch::Tensor, torch::Tensor, int64_t, torch::Tensor> build_plan(const torch::Tensor& topk_idx, const std::vector<int>& counts) {
     DXG_CHECK(topk_idx.is_cuda() && topk_idx.dim() == 2 && topk_idx.is_contiguous() && topk_idx.scalar_type() == torch::kInt64, "topk_idx must be contiguous int64 [N,K] on the GPU");
     const int64_t N = topk_idx.size(0), K = topk_idx.size(1), L = (int64_t)counts.size();
     DXG_CHECK(L >= 1, "at least one local expert");
@@ -231,12 +235,13 @@ std::tuple<torch::Tensor, torch::Tensor, torch::Tensor, torch::Tensor, int64_t> 
     const int64_t m_pad = offs[L];
     c10::cuda::CUDAGuard guard(topk_idx.device());
     auto i32 = topk_idx.options().dtype(torch::kInt32);
-    auto pos = torch::empty({N, K}, i32), src_row = torch::empty({m_pad}, i32), src_k = torch::empty({m_pad}, i32), m_offsets = torch::empty({L + 1}, i32);
-    const cudaError_t e = dx::launch_build_plan(topk_idx.data_ptr<int64_t>(), offs.data(), m_offsets.data_ptr<int>(), pos.data_ptr<int>(),
+    auto pos = torch::empty({N, K}, i32), src_row = torch::empty({m_pad}, i32), src_k = torch::empty({m_pad}, i32), m_offsets = torch::empty({L + 1}, i32),
+         m_ends = torch::empty({L}, i32);
+    const cudaError_t e = dx::launch_build_plan(topk_idx.data_ptr<int64_t>(), offs.data(), m_offsets.data_ptr<int>(), m_ends.data_ptr<int>(), pos.data_ptr<int>(),
                                                 src_row.data_ptr<int>(), src_k.data_ptr<int>(), (int)N, (int)K, (int)L,
                                                 at::cuda::getCurrentCUDAStream(topk_idx.device().index()).stream());
     if (e != cudaSuccess) throw std::runtime_error(std::string("build_plan: ") + cudaGetErrorString(e));
-    return {pos, src_row, src_k, m_offsets, m_pad};
+    return {pos, src_row, src_k, m_offsets, m_pad, m_ends};
 }
 
 // dst[m] = scale * src[src_row[m]]; rows of any dtype whose byte size is a multiple of 4 (of 16 with a scale, which needs bf16)
@@ -349,13 +354,16 @@ torch::Tensor rowdot(const torch::Tensor& a, const torch::Tensor& b, const torch
     return out;
 }
 
-torch::Tensor build_sf_atoms_a(const torch::Tensor& scales) {
+torch::Tensor build_sf_atoms_a(const torch::Tensor& scales, c10::optional<torch::Tensor> group_counts, int rows_per_group) {
     DXG_CHECK(scales.is_cuda() && scales.scalar_type() == torch::kFloat32 && scales.is_contiguous() && scales.dim() == 2, "scales must be contiguous CUDA f32 [M, K/128]");
     c10::cuda::CUDAGuard guard(scales.device());
     const int64_t M = scales.size(0), nkb = scales.size(1);
     auto atoms = torch::empty({(M + 127) / 128, nkb, 512}, scales.options().dtype(torch::kUInt8));
+    if (group_counts.has_value())
+        DXG_CHECK(group_counts->device() == scales.device() && group_counts->scalar_type() == torch::kInt32 && group_counts->is_contiguous() && rows_per_group > 0 &&
+                      rows_per_group % 128 == 0 && group_counts->numel() * (int64_t)rows_per_group == M, "group_counts must be int32 [M / rows_per_group], groups of whole tiles");
     const cudaError_t e = dx::launch_build_sfa_atoms(scales.data_ptr<float>(), atoms.data_ptr<uint8_t>(), (int)M, (int)nkb,
-                                                     at::cuda::getCurrentCUDAStream(scales.get_device()).stream());
+                                                     group_counts.has_value() ? group_counts->data_ptr<int>() : nullptr, rows_per_group, at::cuda::getCurrentCUDAStream(scales.get_device()).stream());
     DXG_CHECK(e == cudaSuccess, "build_sf_atoms_a launch failed");
     return atoms;
 }
@@ -376,7 +384,7 @@ torch::Tensor build_sf_atoms_b(const torch::Tensor& scales, int64_t n, bool swig
 }
 
 void bind_gemm(py::module_& m) {
-    m.def("build_sf_atoms_a", &build_sf_atoms_a);
+    m.def("build_sf_atoms_a", &build_sf_atoms_a, py::arg("scales"), py::arg("group_counts") = py::none(), py::arg("rows_per_group") = 0);
     m.def("build_sf_atoms_b", &build_sf_atoms_b, py::arg("scales"), py::arg("n"), py::arg("swiglu") = false, py::arg("wide") = false);
     m.def("transpose_bf16", &transpose_bf16);
     m.def("swiglu_fwd", &swiglu_fwd);
@@ -389,7 +397,7 @@ void bind_gemm(py::module_& m) {
           py::arg("ready") = py::none(), py::arg("expected") = py::none(), py::arg("row_info") = py::none(),
           py::arg("scatter_bases") = py::none(), py::arg("trace") = py::none(), py::arg("mn_major") = false,
           py::arg("out_fp8") = py::none(), py::arg("out_atoms") = py::none(), py::arg("m_ends_are_counts") = false, py::arg("sched") = py::none(),
-          py::arg("early_table") = false, py::arg("tokens_as_columns") = false, py::arg("hold_successor") = false);
+          py::arg("early_table") = false, py::arg("tokens_as_columns") = 0, py::arg("hold_successor") = false);
     m.def("build_plan", &build_plan);
     m.def("gather_rows", &gather_rows, py::arg("src"), py::arg("src_row"), py::arg("scale") = py::none(), py::arg("out") = py::none());
     m.def("gather_reduce_rows", &gather_reduce_rows, py::arg("src"), py::arg("pos"), py::arg("w") = py::none(), py::arg("out") = py::none());

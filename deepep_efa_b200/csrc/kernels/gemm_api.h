@@ -80,17 +80,21 @@ struct GroupedGemmArgs {
     // 1 = the next kernel in the stream gets no SM before this one has ended, also where it is a programmatic dependent launch: the SMs
     // that this launch leaves free are meant for another stream.
     int hold_successor;
-    // 1 = natively block-scaled 256-column tiles with the weights as the M operand and the tokens as N (see launch_grouped_gemm)
-    int swap;
+    // launch_token_cols_gemm: tokens of one tile at most (a multiple of 32 from 64 to 224)
+    int token_cap;
 };
 
 // Returns cudaErrorInvalidValue for unsupported shapes (divisibility rules are in grouped_gemm.cu).
 cudaError_t launch_grouped_gemm(const GroupedGemmArgs& args, cudaStream_t stream);
+// The same product for groups of few to some hundred rows (gemm_cols.cu): natively block-scaled operands with 256-column weight atoms,
+// mode 0, n % 256 == 0; SwiGLU writes c_fp8 and c_atoms, otherwise bf16 rows to c or through the scatter epilogue.
+cudaError_t launch_token_cols_gemm(const GroupedGemmArgs& args, cudaStream_t stream);
 
 // Expert-major plan from local expert ids [N, K] (-1 = unselected) and 128-aligned group offsets [L+1] on the host:
-// m_offsets [L+1] (the offsets on the device), pos [N*K], src_row [m_pad] (-1 = padding), src_k [m_pad] (0 there).
+// m_offsets [L+1] (the offsets on the device), m_ends [L] (end of every group's rows in front of its padding), pos [N*K], src_row [m_pad]
+// (-1 = padding), src_k [m_pad] (0 there).
 constexpr int kPlanMaxExperts = 1024;  // local experts of one launch; the offsets travel as kernel arguments (4 KiB)
-cudaError_t launch_build_plan(const int64_t* topk_idx, const int* host_offsets, int* m_offsets, int* pos, int* src_row, int* src_k,
+cudaError_t launch_build_plan(const int64_t* topk_idx, const int* host_offsets, int* m_offsets, int* m_ends, int* pos, int* src_row, int* src_k,
                               int num_rows, int num_topk, int num_local_experts, cudaStream_t stream);
 
 // Row gathers between receive order and the expert-major, 128-row-aligned layout (permute.cu).
@@ -117,7 +121,9 @@ cudaError_t launch_unpermute_bwd(const void* a, const void* g, const float* w, c
 cudaError_t launch_rowdot(const void* a, const void* b, const int* pos, float* out, int n_rows, int num_k, int hidden, cudaStream_t stream);
 
 // Scale atoms of the natively block-scaled FP8 GEMM (sf_atoms.cu); scales must be powers of two.
-cudaError_t launch_build_sfa_atoms(const float* scales, uint8_t* atoms, int rows, int num_kb, cudaStream_t stream);
+// With group_counts only the rows r with r % rows_per_group < group_counts[r / rows_per_group] are looked at (rows_per_group % 128 == 0).
+cudaError_t launch_build_sfa_atoms(const float* scales, uint8_t* atoms, int rows, int num_kb, const int* group_counts, int rows_per_group,
+                                   cudaStream_t stream);
 cudaError_t launch_build_sfb_atoms(const float* scales, uint8_t* atoms, int groups, int n, int num_kb, int swiglu, int wide,
                                    cudaStream_t stream);
 

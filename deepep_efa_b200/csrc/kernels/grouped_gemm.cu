@@ -2,8 +2,8 @@
 // 128-byte-swizzled shared memory by TMA (from this GPU's own memory only, never multicast), a
 // persistent warp-specialised CTA per SM.
 //
-//   warp 0   : TMA producer   (one lane)  global -> smem ring, mbarrier complete_tx
-//   warp 1   : MMA issuer     (one lane)  tcgen05.mma, tcgen05.commit frees smem stages and publishes
+//   warp 0   : TMA producer   (one elected lane issues)  global -> smem ring, mbarrier complete_tx
+//   warp 1   : MMA issuer     (one elected lane issues)  tcgen05.mma, tcgen05.commit frees smem stages and publishes
 //                                         accumulator windows; also owns TMEM alloc / dealloc
 //   warps 2.. : epilogue (4 warps for BF16, 8 for FP8)  tcgen05.ld -> registers -> (scale | SwiGLU) -> BF16 ->
 //                                         per-warp smem transpose -> coalesced global stores
@@ -19,306 +19,17 @@
 // loops, TMEM is released and the kernel returns.
 //
 // The reference has no GEMM: its users run their expert FFN between dispatch and combine themselves.
-#include <cuda.h>
-#include <cuda_bf16.h>
-
 #include <cstring>
 
-#include "gemm_api.h"
 #include "launch.cuh"
-#include "prims.cuh"
+#include "tc_prims.cuh"
 
 namespace dx {
 
 namespace {
 
-constexpr int kBlockM = 128;
-constexpr int kKBlockBytes = 128;      // one 128B swizzle atom per row
-constexpr int kATileBytes = kBlockM * kKBlockBytes;  // 16 KiB
 constexpr int kEdgeRows = 32;          // rows of one copy when a tile of A is fetched in part
-constexpr int kTileSlots = 2;          // tiles the loader may hand to the other roles ahead of time
 constexpr int kAheadBlocks = 10;       // K blocks of weights per CTA fetched into L2 before the predecessor ends: 48 MB of the 126 MB
-constexpr int kMaxGroups = 1024;
-
-// ---- PTX wrappers ---------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void mbar_init(uint64_t* bar, int count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-// Bounded wait: returns false (and raises the CTA abort flag) when the limit runs out or another role
-// has already aborted.
-// `note` (optional, device memory) keeps the first wait that gave up: `what` = (role code << 56 | tile << 24 | k block << 8 | slot).
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, long long limit,
-                                          unsigned long long* note = nullptr, unsigned long long what = 0) {
-    if (mbar_try_wait(bar, parity)) return true;
-    const long long t0 = clock64();
-    while (!mbar_try_wait(bar, parity)) {
-        if (*abort_flag) return false;
-        if (clock64() - t0 > limit) {
-            *abort_flag = 1;
-            if (note != nullptr) atomicCAS(note, 0ull, what);
-            return false;
-        }
-    }
-    return true;
-}
-__device__ __forceinline__ unsigned long long wait_id(int role, int tile, int kb, int slot) {
-    return ((unsigned long long)role << 56) | ((unsigned long long)(tile & 0xffffffff) << 24) | ((unsigned long long)(kb & 0xffff) << 8) |
-           (unsigned long long)(slot & 0xff);
-}
-
-__device__ __forceinline__ void tma_load_2d(const CUtensorMap* map, uint64_t* bar, void* dst, int c0, int c1) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(smem_u32(dst)),
-        "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(c0), "r"(c1)
-        : "memory");
-}
-__device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* map, int c0, int c1) {
-    asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global [%0, {%1, %2}];" ::"l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1) : "memory");
-}
-// An MN-major operand tile in one copy: its chunks of 64 rows are the third dimension of the map (see make_map_mn).
-__device__ __forceinline__ void tma_load_3d(const CUtensorMap* map, uint64_t* bar, void* dst, int c1, int c2) {
-    asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(smem_u32(dst)),
-        "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(0), "r"(c1), "r"(c2)
-        : "memory");
-}
-__device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* map) {
-    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
-}
-
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-
-__device__ __forceinline__ void tmem_alloc(uint32_t* dst_smem, uint32_t ncols) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(dst_smem)), "r"(ncols) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_dealloc(uint32_t addr, uint32_t ncols) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(addr), "r"(ncols) : "memory");
-}
-__device__ __forceinline__ void umma_commit(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-template <bool kFp8>
-__device__ __forceinline__ void umma(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-    if constexpr (kFp8) {
-        asm volatile(
-            "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-            "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-            "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-            : "memory");
-    } else {
-        asm volatile(
-            "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-            "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-            : "memory");
-    }
-}
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
-          "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]),
-          "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]),
-          "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-        : "r"(taddr)
-        : "memory");
-}
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
-          "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-        : "r"(taddr)
-        : "memory");
-}
-__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-
-// K-major operand tile in 128B-swizzled shared memory: rows are 128 bytes apart, 8-row groups 1024 bytes
-// apart (stride byte offset), descriptor version 1 (Blackwell), layout type 2 (SWIZZLE_128B).
-__device__ __forceinline__ uint64_t make_smem_desc(uint32_t smem_addr) {
-    uint64_t d = 0;
-    d |= (uint64_t)((smem_addr & 0x3FFFF) >> 4);   // start address, 16-byte units
-    d |= (uint64_t)1 << 16;                        // leading byte offset (unused with swizzle)
-    d |= (uint64_t)(1024 >> 4) << 32;              // stride byte offset
-    d |= (uint64_t)1 << 46;                        // descriptor version
-    d |= (uint64_t)2 << 61;                        // SWIZZLE_128B
-    return d;
-}
-// MN-major operand tile (the tensor's contiguous dimension is the tile's row index, not K): the tile is stored as chunks of
-// 64 rows; a chunk is 64 K-steps of 128 bytes (64 BF16 row elements), 128B-swizzled in groups of 8 K-steps. Stride byte
-// offset = distance between 8-K-step groups (1024), leading byte offset = distance between 64-row chunks (8192).
-__device__ __forceinline__ uint64_t make_smem_desc_mn(uint32_t smem_addr) {
-    uint64_t d = 0;
-    d |= (uint64_t)((smem_addr & 0x3FFFF) >> 4);
-    d |= (uint64_t)(8192 >> 4) << 16;              // leading byte offset: next 64-row chunk
-    d |= (uint64_t)(1024 >> 4) << 32;              // stride byte offset: next group of 8 K-steps
-    d |= (uint64_t)1 << 46;
-    d |= (uint64_t)2 << 61;                        // SWIZZLE_128B
-    return d;
-}
-// Instruction descriptor: fp32 accumulate, M = 128, N = n; bit 15 / 16 = A / B is MN-major instead of K-major.
-template <bool kFp8>
-__device__ __forceinline__ uint32_t make_idesc(int n, int m = kBlockM, int a_mn = 0, int b_mn = 0) {
-    uint32_t d = 0;
-    d |= 1u << 4;                          // D format = F32
-    d |= (kFp8 ? 0u : 1u) << 7;            // A format: E4M3 (f8f6f4) or BF16 (f16)
-    d |= (kFp8 ? 0u : 1u) << 10;           // B format
-    d |= (a_mn ? 1u : 0u) << 15;           // A major
-    d |= (b_mn ? 1u : 0u) << 16;           // B major
-    d |= (uint32_t)(n >> 3) << 17;         // N / 8
-    d |= (uint32_t)(m >> 4) << 24;         // M / 16 (256 for a CTA pair)
-    return d;
-}
-
-// ---- CTA pairs (cta_group::2): two CTAs of a cluster share one 256-row MMA; each stages its own 128 rows of A and HALF
-// of the B tile, so the bytes every SM pulls from L2 per FLOP drop by a third. No load here is a multicast: each CTA's TMA
-// writes only its own shared memory and signals the leader CTA's mbarrier.
-__device__ __forceinline__ uint32_t cluster_ctarank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ uint32_t mapa_shared(uint32_t addr, uint32_t cta_rank) {
-    uint32_t r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(cta_rank));
-    return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
-}
-__device__ __forceinline__ void tma_load_2d_pair(const CUtensorMap* map, uint32_t bar_cluster_addr, void* dst, int c0, int c1) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(
-            smem_u32(dst)),
-        "l"(reinterpret_cast<uint64_t>(map)), "r"(bar_cluster_addr), "r"(c0), "r"(c1)
-        : "memory");
-}
-__device__ __forceinline__ void tma_load_3d_pair(const CUtensorMap* map, uint32_t bar_cluster_addr, void* dst, int c1, int c2) {
-    asm volatile(
-        "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(
-            smem_u32(dst)),
-        "l"(reinterpret_cast<uint64_t>(map)), "r"(bar_cluster_addr), "r"(0), "r"(c1), "r"(c2)
-        : "memory");
-}
-__device__ __forceinline__ void tmem_alloc_pair(uint32_t* dst_smem, uint32_t ncols) {
-    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(dst_smem)), "r"(ncols) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_dealloc_pair(uint32_t addr, uint32_t ncols) {
-    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(addr), "r"(ncols) : "memory");
-}
-__device__ __forceinline__ void umma_commit_pair(uint32_t bar_cluster_addr) {
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar_cluster_addr) : "memory");
-}
-template <bool kFp8>
-__device__ __forceinline__ void umma_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-    if constexpr (kFp8) {
-        asm volatile(
-            "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-            "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-            "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-            : "memory");
-    } else {
-        asm volatile(
-            "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-            "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-            "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-            : "memory");
-    }
-}
-
-// ---- native block scaling (kind::mxf8f6f4.block_scale): UE8M0 scale factors live in TMEM, one byte per 32 K-elements and
-// row. A 128-row x 128-K scale tile is a 512-byte atom in shared memory: the byte of row (m0 + 32*m1), K sub-block kb sits at
-// m0*16 + m1*4 + kb; tcgen05.cp moves it to four TMEM columns (lane m0, column m1, byte kb), replicated to all four lane
-// quarters. With one scale per 128 K-elements the four bytes of a word are equal.
-__device__ __forceinline__ void bulk_load_1d(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)), "l"(src),
-                 "r"(bytes), "r"(smem_u32(bar))
-                 : "memory");
-}
-// 32 rows of 16 bytes, contiguous: no swizzle, 8-row groups 128 bytes apart
-__device__ __forceinline__ uint64_t make_sf_desc(uint32_t smem_addr) {
-    uint64_t d = 0;
-    d |= (uint64_t)((smem_addr & 0x3FFFF) >> 4);
-    d |= (uint64_t)1 << 16;            // leading byte offset (one 16-byte column only)
-    d |= (uint64_t)(128 >> 4) << 32;   // stride byte offset between 8-row groups
-    d |= (uint64_t)1 << 46;            // descriptor version
-    return d;                          // layout type 0: no swizzle
-}
-__device__ __forceinline__ void tmem_cp_sf(uint32_t taddr, uint64_t sdesc) {
-    asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(taddr), "l"(sdesc) : "memory");
-}
-__device__ __forceinline__ void umma_mx(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t sfa, uint32_t sfb,
-                                        uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::mxf8f6f4.block_scale [%0], %1, %2, %3, [%5], [%6], p;\n\t}" ::"r"(tmem_d),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(sfa), "r"(sfb)
-        : "memory");
-}
-// Instruction descriptor of the block-scaled kind: E4M3 operands (format 0), K-major, UE8M0 scales, scale-factor ids 0.
-__device__ __forceinline__ uint32_t make_idesc_mx(int n, int m = kBlockM) {
-    uint32_t d = 0;
-    d |= (uint32_t)(n >> 3) << 17;         // N / 8
-    d |= 1u << 23;                         // scale format: E8M0
-    d |= (uint32_t)(m >> 4) << 24;         // M / 16 (256 for a CTA pair)
-    return d;
-}
-// CTA-pair forms: one instruction makes BOTH CTAs copy their own scale atoms (same shared-memory offset) into their own TMEM,
-// and one MMA covers the 256 rows of the pair; every CTA holds the scale factors of its own 128 rows of A and of ALL columns.
-__device__ __forceinline__ void tmem_cp_sf_pair(uint32_t taddr, uint64_t sdesc) {
-    asm volatile("tcgen05.cp.cta_group::2.32x128b.warpx4 [%0], %1;" ::"r"(taddr), "l"(sdesc) : "memory");
-}
-__device__ __forceinline__ void umma_mx_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t sfa, uint32_t sfb,
-                                             uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::mxf8f6f4.block_scale [%0], %1, %2, %3, [%5], [%6], p;\n\t}" ::"r"(tmem_d),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(sfa), "r"(sfb)
-        : "memory");
-}
-
-__device__ __forceinline__ unsigned long long ld_acquire_sys_u64(const unsigned long long* p) {
-    unsigned long long v;
-    asm volatile("ld.acquire.sys.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-    return v;
-}
-// Orders what this thread observed through ordinary loads (the arrival counter) before its later TMA reads of the rows.
-__device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async;" ::: "memory"); }
-__device__ __forceinline__ unsigned long long global_timer_ns() {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-
-__device__ __forceinline__ float silu(float x) { return x / (1.f + __expf(-x)); }
 
 __device__ __forceinline__ int4 pack8_bf16(const float* o) {
     int4 w;
@@ -394,21 +105,6 @@ __device__ __forceinline__ void store_rows_256(int4* stage, const int4 (&regs)[1
     }
 }
 
-// Four lanes hold one byte of each of four tokens (byte t of the word) for neighbouring features: afterwards lane j of the four holds
-// the four features of token j.
-__device__ __forceinline__ uint32_t transpose_bytes_4x4(uint32_t w, int lane) {
-    uint32_t o = __shfl_xor_sync(0xffffffffu, w, 1);
-    w = __byte_perm(w, o, (lane & 1) ? 0x3715 : 0x6240);
-    o = __shfl_xor_sync(0xffffffffu, w, 2);
-    return __byte_perm(w, o, (lane & 2) ? 0x3276 : 0x5410);
-}
-
-// Rows of group g (mode 0), which starts at row `begin`.
-__device__ __forceinline__ int group_rows(const GroupedGemmArgs& p, int g, int begin) {
-    if (p.m_ends == nullptr) return max(p.m_offsets[g + 1] - begin, 0);
-    return max(p.m_ends_are_counts ? p.m_ends[g] : p.m_ends[g] - begin, 0);
-}
-
 struct TileInfo {
     int a_row, a_k0, b_row, b_row2, b_k0, num_kb, c_row, c_col, group, nblock, nblock2;
     int c_row_end;  // first output row this tile must not write (end of its group; groups need no 128-row alignment)
@@ -458,12 +154,11 @@ struct Cfg {
         (size_t)kStages * kStageBytes + (size_t)kEpiWarps * kOutStageBytes + 1024 /*align*/ + 256 /*barriers*/ + (kMaxGroups + 1) * 4 + kXchBytes;
 };
 
-template <int kBlockN, bool kFp8, bool kSwiGLU, bool kPair, bool kMx = false, bool kRowScatter = false, bool kSwap = false>
+template <int kBlockN, bool kFp8, bool kSwiGLU, bool kPair, bool kMx = false, bool kRowScatter = false>
 __global__ void __launch_bounds__((Cfg<kBlockN, kFp8, kSwiGLU, kPair, kMx, kRowScatter>::kThreads), 1)
 grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                     const __grid_constant__ CUtensorMap map_sfa, const __grid_constant__ CUtensorMap map_sfb, const GroupedGemmArgs p) {
     using C = Cfg<kBlockN, kFp8, kSwiGLU, kPair, kMx, kRowScatter>;
-    static_assert(!kSwap || (kMx && !kPair && kBlockN == 256), "weights as M: natively block-scaled 256-column tiles on single CTAs");
     static_assert(!kRowScatter || (kMx && !kSwiGLU && !kPair && kBlockN == 128), "whole-row scatter: natively block-scaled 128-column tiles");
     static_assert(!kMx || (kFp8 && ((!kPair && kBlockN == 128) || (kBlockN == 256 && (kSwiGLU || !kPair)))),
                   "native block scaling: e4m3 operands; 128-column tiles, 256-column tiles, or 256-column SwiGLU tiles on a CTA pair");
@@ -629,12 +324,11 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     // through 256 experts of 7168 -> 2048: first / second GEMM 1243 / 661 -> 1209 / 622 us; the fused layer of 4096 tokens 2700 -> 2600).
     const bool drawn = !kPair && p.sched != nullptr;
     int tslot = 0, tphase = 0;  // this role's position in the ring
-    auto next_tile = [&](int tile, bool whole_warp) {
+    auto next_tile = [&](int tile) {
         if (!drawn) return tile + sched_stride;
-        const bool got = mbar_wait(&tile_full[tslot], tphase, abort_flag, limit, note, wait_id(8, tile, 0, tslot));
-        if (whole_warp ? !__all_sync(0xffffffffu, got) : !got) return total_tiles;
+        if (!__all_sync(0xffffffffu, mbar_wait(&tile_full[tslot], tphase, abort_flag, limit, note, wait_id(8, tile, 0, tslot)))) return total_tiles;
         const int t = s_tile[tslot];
-        if (whole_warp) __syncwarp();
+        __syncwarp();
         if (lane == 0) mbar_arrive(&tile_free[tslot]);
         if (++tslot == kTileSlots) {
             tslot = 0;
@@ -659,13 +353,6 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         if (!p.hold_successor) pdl_release_successor();
     }
 
-    // kSwap: the weights are the M operand and the tokens the N operand, in steps of 32 columns up to the tile's valid rows. A group of
-    // four rows as M is 128 rows of products for four, and the power they take lowers the clock: streaming 256 experts of 7168 -> 2048
-    // for 128 tokens back to back ran at 1.2 GHz of 1.97 and 2053 us per layer that way, 1850 us this way. Everything up to the MMA
-    // (tiles, copies, scale atoms) is the same; the epilogue finds features in lanes and tokens in columns. An instantiation of its
-    // own: with both epilogues in one kernel the spills of either made 20-token steps 5 % slower instead of 9 % faster.
-    auto token_cols = [&](const TileInfo& t) { return min(kBlockM, (max(1, t.c_row_end - t.a_row) + 31) & ~31); };
-
     // An epilogue warp hands an accumulator window back to the MMA issuer: in a pair that is the leader CTA's barrier.
     auto release_window = [&](uint64_t* bar) {
         if constexpr (kPair) {
@@ -678,7 +365,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 
     if (warp == 0) {
         // ================= TMA producer =================
-        if (lane == 0) {
+        {
             int stage = 0, phase = 0, g = 0;
             int issued = 0;  // stages armed so far (saturating), for the drain on the abort path
             int gated_group = -1;
@@ -687,13 +374,16 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             bool ok = true;
             auto hand_out = [&](int tile, int draw) {
                 if (!drawn) return tile + sched_stride;
-                const int t = min(sched_stride + draw, total_tiles);
-                if (!mbar_wait(&tile_free[tslot], tphase ^ 1, abort_flag, limit, note, wait_id(9, tile, 0, tslot))) {
+                const int t = min(sched_stride + __shfl_sync(0xffffffffu, draw, 0), total_tiles);
+                if (!__all_sync(0xffffffffu, mbar_wait(&tile_free[tslot], tphase ^ 1, abort_flag, limit, note, wait_id(9, tile, 0, tslot)))) {
                     ok = false;
                     return total_tiles;
                 }
-                s_tile[tslot] = t;
-                mbar_arrive(&tile_full[tslot]);
+                if (lane == 0) {
+                    s_tile[tslot] = t;
+                    mbar_arrive(&tile_full[tslot]);
+                }
+                __syncwarp();
                 if (++tslot == kTileSlots) {
                     tslot = 0;
                     tphase ^= 1;
@@ -703,11 +393,11 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             int drawn_tile = 0;
             unsigned stage_rows = 0;  // four bits per stage: 32-row pieces of A that are not zero
             for (int tile = sched_id; tile < total_tiles && ok; tile = hand_out(tile, drawn_tile)) {
-                if (drawn) drawn_tile = atomicAdd(p.sched, 1);  // used when this tile's loads have been issued
+                if (drawn && lane == 0) drawn_tile = atomicAdd(p.sched, 1);  // used when this tile's loads have been issued
                 decode(tile, g, ti);
-                s_prod_state[1] = tile;
+                if (lane == 0) s_prod_state[1] = tile;
                 if (p.ready != nullptr && ti.group != gated_group) {
-                    s_prod_state[0] = 1;
+                    if (lane == 0) s_prod_state[0] = 1;
                     // the rows of this group come from other GPUs: wait until all of them have landed
                     const unsigned long long want = p.expected[ti.group];
                     if (ld_acquire_sys_u64(p.ready + ti.group) < want) {
@@ -720,13 +410,14 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                                 break;
                             }
                         }
-                        if (!ok) break;
                     }
+                    ok = __all_sync(0xffffffffu, ok);
+                    if (!ok) break;
                     fence_proxy_async();
                     gated_group = ti.group;
                 }
                 if (p.trace != nullptr && !stamped) {
-                    atomicMin(&p.trace[0], global_timer_ns());
+                    if (lane == 0) atomicMin(&p.trace[0], global_timer_ns());
                     stamped = true;
                 }
                 // Rows past the end of the group are not fetched when m_ends says where that is; the tensor core sees zeros instead.
@@ -736,8 +427,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 const int valid_rows = max(1, ti.c_row_end - ti.a_row);
                 const int edge = (!kPair && p.mode == 0 && p.m_ends != nullptr && valid_rows <= 2 * kEdgeRows) ? (valid_rows + kEdgeRows - 1) / kEdgeRows : 0;
                 for (int kb = 0; kb < ti.num_kb; ++kb) {
-                    s_prod_state[0] = 2;
-                    if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag, limit, note, wait_id(1, tile, kb, stage))) {
+                    if (lane == 0) s_prod_state[0] = 2;
+                    if (!__all_sync(0xffffffffu, mbar_wait(&empty[stage], phase ^ 1, abort_flag, limit, note, wait_id(1, tile, kb, stage)))) {
                         ok = false;
                         break;
                     }
@@ -746,20 +437,23 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                     if constexpr (kPair) {
                         // both CTAs fill their own stage and signal the LEADER's barrier, which expects the bytes of both
                         const uint32_t leader_full = mapa_shared(smem_u32(&full[stage]), 0);
-                        if (cta_rank == 0) mbar_expect_tx(&full[stage], 2 * C::kStageTxBytes);
-                        if (kMnMajor && p.a_mn) tma_load_3d_pair(&map_a, leader_full, sa, ti.a_kbase + kb * 64, ti.a_mn0 / 64);
-                        else tma_load_2d_pair(&map_a, leader_full, sa, ti.a_k0 + kb * elem_per_kb, ti.a_row);
-                        if (kMnMajor && p.b_mn) tma_load_3d_pair(&map_b, leader_full, sb, ti.b_kbase + kb * 64, ti.b_mn0 / 64);
-                        else
-                            tma_load_2d_pair(&map_b, leader_full, sb, ti.b_k0 + kb * elem_per_kb,
-                                             (kSwiGLU && cta_rank == 1) ? ti.b_row2 : ti.b_row);  // SwiGLU: gate half / up half
-                        if constexpr (kMx) {
-                            // scale atoms as rows of 32-bit words: this CTA's own 128 rows of A, and the whole tile's B columns
-                            uint8_t* ssf = sb + C::kBTileBytes;
-                            const int nkb = p.k / 128;
-                            tma_load_2d_pair(&map_sfa, leader_full, ssf, 0, (ti.a_row >> 7) * nkb + kb);
-                            tma_load_2d_pair(&map_sfb, leader_full, ssf + 512, 0, (ti.group * (p.n / kBlockN) + ti.nt) * nkb + kb);
+                        if (elect_one()) {
+                            if (cta_rank == 0) mbar_expect_tx(&full[stage], 2 * C::kStageTxBytes);
+                            if (kMnMajor && p.a_mn) tma_load_3d_pair(&map_a, leader_full, sa, ti.a_kbase + kb * 64, ti.a_mn0 / 64);
+                            else tma_load_2d_pair(&map_a, leader_full, sa, ti.a_k0 + kb * elem_per_kb, ti.a_row);
+                            if (kMnMajor && p.b_mn) tma_load_3d_pair(&map_b, leader_full, sb, ti.b_kbase + kb * 64, ti.b_mn0 / 64);
+                            else
+                                tma_load_2d_pair(&map_b, leader_full, sb, ti.b_k0 + kb * elem_per_kb,
+                                                 (kSwiGLU && cta_rank == 1) ? ti.b_row2 : ti.b_row);  // SwiGLU: gate half / up half
+                            if constexpr (kMx) {
+                                // scale atoms as rows of 32-bit words: this CTA's own 128 rows of A, and the whole tile's B columns
+                                uint8_t* ssf = sb + C::kBTileBytes;
+                                const int nkb = p.k / 128;
+                                tma_load_2d_pair(&map_sfa, leader_full, ssf, 0, (ti.a_row >> 7) * nkb + kb);
+                                tma_load_2d_pair(&map_sfb, leader_full, ssf + 512, 0, (ti.group * (p.n / kBlockN) + ti.nt) * nkb + kb);
+                            }
                         }
+                        __syncwarp();
                         if (issued < C::kStages) ++issued;
                         if (++stage == C::kStages) {
                             stage = 0;
@@ -767,35 +461,38 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                         }
                         continue;
                     }
-                    s_prod_state[0] = 3;
+                    if (lane == 0) s_prod_state[0] = 3;
                     // 32-row pieces of A to write: the valid ones, then pieces an earlier tile left in this stage (zeroed by copies from
                     // past the last row, which touch no memory)
                     const int filled = (int)(stage_rows >> (4 * stage)) & 7;
                     const int pieces = edge == 0 ? kBlockM / kEdgeRows : max(edge, filled);
                     stage_rows = (stage_rows & ~(7u << (4 * stage))) | ((unsigned)(edge == 0 ? kBlockM / kEdgeRows : edge) << (4 * stage));
-                    mbar_expect_tx(&full[stage], C::kStageTxBytes - kATileBytes + pieces * kEdgeRows * kKBlockBytes);
-                    if constexpr (kMx) {
-                        // scale atoms: [row tile][K block][512] for A, [group][n tile][K block][512] for B
-                        uint8_t* ssf = sb + C::kBTileBytes;
-                        const size_t nkb = (size_t)(p.k / 128);
-                        bulk_load_1d(ssf, p.sfa_atoms + ((size_t)(ti.a_row >> 7) * nkb + kb) * 512, 512, &full[stage]);
-                        bulk_load_1d(ssf + 512, p.sfb_atoms + (((size_t)ti.group * (p.n / kBlockN) + ti.nt) * nkb + kb) * (512 * C::kSfBAtoms),
-                                     512 * C::kSfBAtoms, &full[stage]);
+                    if (elect_one()) {
+                        mbar_expect_tx(&full[stage], C::kStageTxBytes - kATileBytes + pieces * kEdgeRows * kKBlockBytes);
+                        if constexpr (kMx) {
+                            // scale atoms: [row tile][K block][512] for A, [group][n tile][K block][512] for B
+                            uint8_t* ssf = sb + C::kBTileBytes;
+                            const size_t nkb = (size_t)(p.k / 128);
+                            bulk_load_1d(ssf, p.sfa_atoms + ((size_t)(ti.a_row >> 7) * nkb + kb) * 512, 512, &full[stage]);
+                            bulk_load_1d(ssf + 512, p.sfb_atoms + (((size_t)ti.group * (p.n / kBlockN) + ti.nt) * nkb + kb) * (512 * C::kSfBAtoms),
+                                         512 * C::kSfBAtoms, &full[stage]);
+                        }
+                        if (kMnMajor && p.a_mn) tma_load_3d(&map_a, &full[stage], sa, ti.a_kbase + kb * 64, ti.a_mn0 / 64);
+                        else if (edge == 0) tma_load_2d(&map_a, &full[stage], sa, ti.a_k0 + kb * elem_per_kb, ti.a_row);
+                        else
+                            for (int j = 0; j < pieces; ++j)
+                                tma_load_2d(&map_sfa, &full[stage], sa + j * kEdgeRows * kKBlockBytes, ti.a_k0 + kb * elem_per_kb,
+                                            j < edge ? ti.a_row + j * kEdgeRows : p.m_total);
+                        if (kMnMajor && p.b_mn) {
+                            tma_load_3d(&map_b, &full[stage], sb, ti.b_kbase + kb * 64, ti.b_mn0 / 64);
+                        } else if (kSwiGLU) {
+                            tma_load_2d(&map_b, &full[stage], sb, ti.b_k0 + kb * elem_per_kb, ti.b_row);
+                            tma_load_2d(&map_b, &full[stage], sb + C::kBTileBytes / 2, ti.b_k0 + kb * elem_per_kb, ti.b_row2);
+                        } else {
+                            tma_load_2d(&map_b, &full[stage], sb, ti.b_k0 + kb * elem_per_kb, ti.b_row);
+                        }
                     }
-                    if (kMnMajor && p.a_mn) tma_load_3d(&map_a, &full[stage], sa, ti.a_kbase + kb * 64, ti.a_mn0 / 64);
-                    else if (edge == 0) tma_load_2d(&map_a, &full[stage], sa, ti.a_k0 + kb * elem_per_kb, ti.a_row);
-                    else
-                        for (int j = 0; j < pieces; ++j)
-                            tma_load_2d(&map_sfa, &full[stage], sa + j * kEdgeRows * kKBlockBytes, ti.a_k0 + kb * elem_per_kb,
-                                        j < edge ? ti.a_row + j * kEdgeRows : p.m_total);
-                    if (kMnMajor && p.b_mn) {
-                        tma_load_3d(&map_b, &full[stage], sb, ti.b_kbase + kb * 64, ti.b_mn0 / 64);
-                    } else if (kSwiGLU) {
-                        tma_load_2d(&map_b, &full[stage], sb, ti.b_k0 + kb * elem_per_kb, ti.b_row);
-                        tma_load_2d(&map_b, &full[stage], sb + C::kBTileBytes / 2, ti.b_k0 + kb * elem_per_kb, ti.b_row2);
-                    } else {
-                        tma_load_2d(&map_b, &full[stage], sb, ti.b_k0 + kb * elem_per_kb, ti.b_row);
-                    }
+                    __syncwarp();
                     if (issued < C::kStages) ++issued;
                     if (++stage == C::kStages) {
                         stage = 0;
@@ -803,7 +500,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                     }
                 }
             }
-            if (drawn) {  // the last CTA to stop drawing leaves the counter as it was found
+            if (drawn && lane == 0) {  // the last CTA to stop drawing leaves the counter as it was found
                 __threadfence();
                 if (atomicAdd(p.sched + 1, 1) == (int)gridDim.x - 1) {
                     p.sched[1] = 0;
@@ -835,100 +532,95 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         }
     } else if (warp == 1) {
         // ================= MMA issuer =================
-        if (lane == 0 && cta_rank == 0) {
+        if (cta_rank == 0) {
             const uint32_t idesc_full = kMx ? make_idesc_mx(kBlockN, C::kTileRows) : make_idesc<kFp8>(kBlockN, C::kTileRows, p.a_mn, p.b_mn);
             const uint32_t idesc_half = make_idesc<kFp8>(kBlockN / 2, C::kTileRows, p.a_mn, p.b_mn);
             // bytes (in 16-byte units) one K = 16 step moves the operand's start address: 32 B inside the swizzle atom when K
             // is contiguous, 16 K-steps of 128 B when the rows are
             const uint64_t a_kstep = p.a_mn ? 128 : 2, b_kstep = p.b_mn ? 128 : 2;
-            int sf_buf = 0;
+            int sf_buf = 0;  // native block scaling: which set of scale columns
             int stage = 0, phase = 0, g = 0;
             int win = 0, win_phase = 0;  // accumulator window ring
             TileInfo ti;
             bool ok = true;
-            for (int tile = sched_id; tile < total_tiles && ok; tile = next_tile(tile, false)) {
+            for (int tile = sched_id; tile < total_tiles && ok; tile = next_tile(tile)) {
                 decode(tile, g, ti);
                 if (ti.num_kb == 0) continue;  // epilogue writes zeros on its own
-                const uint32_t idesc = kSwap ? make_idesc_mx(token_cols(ti), kBlockM) : (C::kRagged && ti.n_cols != kBlockN) ? idesc_half : idesc_full;
+                const uint32_t idesc = (C::kRagged && ti.n_cols != kBlockN) ? idesc_half : idesc_full;
                 for (int kb = 0; kb < ti.num_kb; ++kb) {
                     const bool new_window = C::kPromote ? true : (kb == 0);
                     if (new_window) {
-                        if (!mbar_wait(&tmem_empty[win], win_phase ^ 1, abort_flag, limit, note, wait_id(3, tile, kb, win))) {
+                        if (!__all_sync(0xffffffffu, mbar_wait(&tmem_empty[win], win_phase ^ 1, abort_flag, limit, note, wait_id(3, tile, kb, win)))) {
                             ok = false;
                             break;
                         }
                         tc_fence_after();
                     }
-                    if (!mbar_wait(&full[stage], phase, abort_flag, limit, note, wait_id(4, tile, kb, stage))) {
-                        if (note != nullptr) atomicCAS(note + 1, 0ull, ((unsigned long long)s_prod_state[0] << 32) | (unsigned)s_prod_state[1]);
+                    if (!__all_sync(0xffffffffu, mbar_wait(&full[stage], phase, abort_flag, limit, note, wait_id(4, tile, kb, stage)))) {
+                        if (note != nullptr && lane == 0) atomicCAS(note + 1, 0ull, ((unsigned long long)s_prod_state[0] << 32) | (unsigned)s_prod_state[1]);
                         ok = false;
                         break;
                     }
                     tc_fence_after();
-                    const uint32_t sa = smem_u32(stage_base + (size_t)stage * C::kStageBytes);
+                    const uint32_t sa = smem_u32(stage_base) + (uint32_t)(stage * C::kStageBytes);
                     const uint32_t sb = sa + kATileBytes;
                     const uint64_t adesc = p.a_mn ? make_smem_desc_mn(sa) : make_smem_desc(sa);
                     const uint64_t bdesc = p.b_mn ? make_smem_desc_mn(sb) : make_smem_desc(sb);
                     const uint32_t tmem_d = tmem_base + (uint32_t)(win * kBlockN);
-                    if constexpr (kMx) {
-                        // scale atoms of this stage -> TMEM (alternating column sets), then four K=32 MMAs that read them
-                        const uint32_t ssf = sb + C::kBTileBytes;
-                        const uint32_t t_sfa = tmem_base + (uint32_t)(C::kSfCol0 + sf_buf * C::kSfColsPerBuf), t_sfb = t_sfa + 4;
-                        if constexpr (kPair) {
-                            tmem_cp_sf_pair(t_sfa, make_sf_desc(ssf));
+                    const bool window_done = C::kPromote ? true : (kb == ti.num_kb - 1);
+                    if (elect_one()) {
+                        if constexpr (kMx) {
+                            // scale atoms of this stage -> TMEM (alternating column sets), then four K=32 MMAs that read them
+                            const uint32_t ssf = sb + C::kBTileBytes;
+                            const uint32_t t_sfa = tmem_base + (uint32_t)(C::kSfCol0 + sf_buf * C::kSfColsPerBuf), t_sfb = t_sfa + 4;
+                            if constexpr (kPair) {
+                                tmem_cp_sf_pair(t_sfa, make_sf_desc(ssf));
 #pragma unroll
-                            for (int at = 0; at < C::kSfBAtoms; ++at) tmem_cp_sf_pair(t_sfb + 4 * at, make_sf_desc(ssf + 512 + 512 * at));
+                                for (int at = 0; at < C::kSfBAtoms; ++at) tmem_cp_sf_pair(t_sfb + 4 * at, make_sf_desc(ssf + 512 + 512 * at));
 #pragma unroll
-                            for (int j = 0; j < 4; ++j)
-                                umma_mx_pair(tmem_d, adesc + (uint64_t)(j * 2), bdesc + (uint64_t)(j * 2), idesc, t_sfa, t_sfb,
-                                             (new_window && j == 0) ? 0u : 1u);
-                        } else {
-                            tmem_cp_sf(t_sfa, make_sf_desc(ssf));
-#pragma unroll
-                            for (int at = 0; at < C::kSfBAtoms; ++at) tmem_cp_sf(t_sfb + 4 * at, make_sf_desc(ssf + 512 + 512 * at));
-                            if constexpr (kSwap) {
-                                // weight rows as M (two tiles of 128), token rows as N
-#pragma unroll
-                                for (int hw = 0; hw < kBlockN / kBlockM; ++hw)
-#pragma unroll
-                                    for (int j = 0; j < 4; ++j)
-                                        umma_mx(tmem_d + hw * kBlockM, bdesc + (uint64_t)(hw * (kATileBytes >> 4) + j * 2), adesc + (uint64_t)(j * 2), idesc,
-                                                t_sfb + 4 * hw, t_sfa, (new_window && j == 0) ? 0u : 1u);
+                                for (int j = 0; j < 4; ++j)
+                                    umma_mx_pair(tmem_d, adesc + (uint64_t)(j * 2), bdesc + (uint64_t)(j * 2), idesc, t_sfa, t_sfb,
+                                                 (new_window && j == 0) ? 0u : 1u);
                             } else {
+                                tmem_cp_sf(t_sfa, make_sf_desc(ssf));
+#pragma unroll
+                                for (int at = 0; at < C::kSfBAtoms; ++at) tmem_cp_sf(t_sfb + 4 * at, make_sf_desc(ssf + 512 + 512 * at));
 #pragma unroll
                                 for (int j = 0; j < 4; ++j)
                                     umma_mx(tmem_d, adesc + (uint64_t)(j * 2), bdesc + (uint64_t)(j * 2), idesc, t_sfa, t_sfb,
                                             (new_window && j == 0) ? 0u : 1u);
                             }
-                        }
-                        sf_buf ^= 1;
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            // +32 bytes along K inside the swizzle atom = +2 in the 16-byte start-address field
-                            if constexpr (kPair)
-                                umma_pair<kFp8>(tmem_d, adesc + (uint64_t)j * a_kstep, bdesc + (uint64_t)j * b_kstep, idesc,
-                                                (new_window && j == 0) ? 0u : 1u);
-                            else
-                                umma<kFp8>(tmem_d, adesc + (uint64_t)j * a_kstep, bdesc + (uint64_t)j * b_kstep, idesc,
-                                           (new_window && j == 0) ? 0u : 1u);
-                        }
-                    }
-                    // smem stage reusable once these MMAs have read it (in both CTAs of a pair)
-                    if constexpr (kPair) {
-                        umma_commit_pair(smem_u32(&empty[stage]));
-                        umma_commit_pair(mapa_shared(smem_u32(&empty[stage]), 1));
-                    } else {
-                        umma_commit(&empty[stage]);
-                    }
-                    const bool window_done = C::kPromote ? true : (kb == ti.num_kb - 1);
-                    if (window_done) {
-                        if constexpr (kPair) {
-                            umma_commit_pair(smem_u32(&tmem_full[win]));
-                            umma_commit_pair(mapa_shared(smem_u32(&tmem_full[win]), 1));
                         } else {
-                            umma_commit(&tmem_full[win]);
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) {
+                                // +32 bytes along K inside the swizzle atom = +2 in the 16-byte start-address field
+                                if constexpr (kPair)
+                                    umma_pair<kFp8>(tmem_d, adesc + (uint64_t)j * a_kstep, bdesc + (uint64_t)j * b_kstep, idesc,
+                                                    (new_window && j == 0) ? 0u : 1u);
+                                else
+                                    umma<kFp8>(tmem_d, adesc + (uint64_t)j * a_kstep, bdesc + (uint64_t)j * b_kstep, idesc,
+                                               (new_window && j == 0) ? 0u : 1u);
+                            }
                         }
+                        // smem stage reusable once these MMAs have read it (in both CTAs of a pair)
+                        if constexpr (kPair) {
+                            umma_commit_pair(smem_u32(&empty[stage]));
+                            umma_commit_pair(mapa_shared(smem_u32(&empty[stage]), 1));
+                        } else {
+                            umma_commit(&empty[stage]);
+                        }
+                        if (window_done) {
+                            if constexpr (kPair) {
+                                umma_commit_pair(smem_u32(&tmem_full[win]));
+                                umma_commit_pair(mapa_shared(smem_u32(&tmem_full[win]), 1));
+                            } else {
+                                umma_commit(&tmem_full[win]);
+                            }
+                        }
+                    }
+                    __syncwarp();
+                    sf_buf ^= 1;
+                    if (window_done) {
                         if (++win == C::kWindows) {
                             win = 0;
                             win_phase ^= 1;
@@ -955,7 +647,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         __nv_bfloat16* cbase = reinterpret_cast<__nv_bfloat16*>(p.c);
         const int ldc = p.mode == 0 ? (kSwiGLU ? p.n / 2 : p.n) : p.k;
         const bool scatter = !kSwiGLU && p.mode == 0 && p.row_info != nullptr;
-        for (int tile = sched_id; tile < total_tiles && ok; tile = next_tile(tile, true)) {
+        for (int tile = sched_id; tile < total_tiles && ok; tile = next_tile(tile)) {
             decode(tile, g, ti);
             const int row = ti.c_row + row_in_tile;
             __nv_bfloat16* crow = cbase + (size_t)row * ldc + ti.c_col;
@@ -1086,103 +778,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(win * kBlockN);
                 __nv_bfloat16* wbase = cbase + (size_t)(ti.c_row + q * 32) * ldc + ti.c_col;
                 const int rows_valid = min(32, ti.c_row_end - (ti.c_row + q * 32));
-                if constexpr (kSwap) {
-                    // TMEM lane = weight row, column = token. The two warps of a quarter take alternate chunks of 16 tokens; a thread
-                    // has one feature of the gate (or first) half and one of the up (second) half of every token.
-                    const int n_tok = token_cols(ti), tok_valid = ti.c_row_end - ti.c_row;
-                    const unsigned tag = (unsigned)(++xch_iter & 0xffff) << 16;
-                    volatile uint32_t* xs = reinterpret_cast<volatile uint32_t*>(xch) + (xch_iter & 1) * (kBlockM * 4);
-#pragma unroll 1
-                    for (int tb = 0; tb < n_tok && ok; tb += 64) {  // two chunks at a time: all four would not fit the registers
-                        uint32_t v[2][16], u[2][16];
-#pragma unroll
-                        for (int c = 0; c < 2; ++c) {
-                            const int t0 = tb + (2 * c + half) * 16;
-                            if (t0 < n_tok) {
-                                tmem_ld16(taddr + t0, v[c]);
-                                tmem_ld16(taddr + kBlockM + t0, u[c]);
-                            }
-                        }
-                        tmem_ld_wait();
-                        if (tb + 64 >= n_tok) {
-                            tc_fence_before();
-                            __syncwarp();
-                            if (lane == 0) release_window(&tmem_empty[win]);
-                        }
-#pragma unroll
-                        for (int c = 0; c < 2; ++c) {
-                            const int t0 = tb + (2 * c + half) * 16;
-                            if (t0 >= n_tok) break;
-                            if constexpr (kSwiGLU) {
-                                // same arithmetic as the row-wise epilogue: BF16-rounded product, power-of-two scale from the amax of the
-                                // token's 128 features. NaN does not count, as with fmaxf. Four warps hold 32 features each and exchange
-                                // their maxima (exact in BF16) through tagged words, two tile parities.
-                                float h[16];
-                                uint32_t mine = 0;
-#pragma unroll
-                                for (int t = 0; t < 16; ++t) {
-                                    h[t] = __bfloat162float(__float2bfloat16(silu(__uint_as_float(v[c][t])) * __uint_as_float(u[c][t])));
-                                    const uint32_t bits = (__float_as_uint(h[t]) >> 16) & 0x7fffu;
-                                    const uint32_t m = __reduce_max_sync(0xffffffffu, bits > 0x7f80u ? 0u : bits);
-                                    if (lane == t) mine = m;
-                                }
-                                volatile uint32_t* slot = xs + (t0 + (lane & 15)) * 4;
-                                if (lane < 16) slot[q] = tag | mine;
-                                if (lane < 16) {
-                                    const long long w0 = clock64();
-                                    for (int i = 0; i < 4 && ok; ++i) {
-                                        uint32_t w = slot[i];
-                                        while ((w & 0xffff0000u) != tag) {
-                                            if (*abort_flag || clock64() - w0 > limit) {
-                                                if (!*abort_flag && note != nullptr) atomicCAS(note, 0ull, wait_id(7, tile, 0, warp));
-                                                *abort_flag = 1;
-                                                ok = false;
-                                                break;
-                                            }
-                                            w = slot[i];
-                                        }
-                                        mine = max(mine, w & 0xffffu);
-                                    }
-                                }
-                                ok = __all_sync(0xffffffffu, ok);
-                                if (!ok) break;
-                                float scale, inv;
-                                fp8_scale_from_amax(__uint_as_float(mine << 16), true, scale, inv);
-                                if (q == 0 && lane < 16 && t0 + lane < tok_valid) {
-                                    const int trow = ti.c_row + t0 + lane;
-                                    *reinterpret_cast<uint32_t*>(p.c_atoms + ((size_t)(trow >> 7) * (ldc / 128) + (ti.c_col >> 7)) * 512 + (trow & 31) * 16 +
-                                                                 ((trow >> 5) & 3) * 4) = ((__float_as_uint(scale) >> 23) & 0xffu) * 0x01010101u;
-                                }
-#pragma unroll
-                                for (int t = 0; t < 16; t += 4) {
-                                    float x[4];
-#pragma unroll
-                                    for (int j = 0; j < 4; ++j) x[j] = h[t + j] * __shfl_sync(0xffffffffu, inv, t + j);
-                                    const uint32_t w = transpose_bytes_4x4(pack_e4m3x4(x[0], x[1], x[2], x[3]), lane);
-                                    const int tok = t0 + t + (lane & 3);
-                                    if (tok < tok_valid)
-                                        *reinterpret_cast<uint32_t*>(p.c_fp8 + (size_t)(ti.c_row + tok) * ldc + ti.c_col + q * 32 + (lane & ~3)) = w;
-                                }
-                            } else {
-#pragma unroll
-                                for (int hw = 0; hw < 2; ++hw)
-#pragma unroll
-                                    for (int t = 0; t < 16; t += 2) {
-                                        const uint32_t* a = hw == 0 ? v[c] : u[c];
-                                        const uint32_t w = f2_to_bf16x2(__uint_as_float(a[t]), __uint_as_float(a[t + 1]));
-                                        const uint32_t o = __shfl_xor_sync(0xffffffffu, w, 1);
-                                        const int tok = t0 + t + (lane & 1);
-                                        if (tok < tok_valid)
-                                            *reinterpret_cast<uint32_t*>(cbase + (size_t)(ti.c_row + tok) * ldc + ti.c_col + hw * kBlockM + q * 32 + (lane & ~1)) =
-                                                __byte_perm(w, o, (lane & 1) ? 0x3276 : 0x5410);
-                                    }
-                            }
-                        }
-                    }
-                    if (!ok) break;
-                    win_phase ^= 1;
-                    continue;
-                } else if constexpr (kSwiGLU && C::kWindows == 1) {
+                if constexpr (kSwiGLU && C::kWindows == 1) {
                     // Single window, two warps per lane quarter: this warp takes 64 of the tile's 128 output columns. Their gate
                     // and up accumulators go to registers raw, the window returns to the MMA issuer right away, and the
                     // arithmetic and the stores run while the next tile accumulates.
@@ -1402,37 +998,6 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 }
 
 // ---- host side ------------------------------------------------------------------------------
-using EncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                              const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                              CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeFn get_encode_fn() {
-    static EncodeFn fn = nullptr;
-    if (fn == nullptr) {
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult qres;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &qres) == cudaSuccess &&
-            qres == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<EncodeFn>(p);
-    }
-    return fn;
-}
-
-// 2-D row-major [rows, cols] tensor, box = 128 bytes of columns x box_rows rows, 128B swizzle.
-bool make_map(CUtensorMap* map, const void* ptr, bool fp8, uint64_t rows, uint64_t cols, uint32_t box_rows) {
-    EncodeFn fn = get_encode_fn();
-    if (fn == nullptr) return false;
-    const uint64_t esz = fp8 ? 1 : 2;
-    cuuint64_t dims[2] = {cols, rows};
-    cuuint64_t strides[1] = {cols * esz};
-    cuuint32_t box[2] = {(cuuint32_t)(kKBlockBytes / esz), box_rows};
-    cuuint32_t estr[2] = {1, 1};
-    const CUresult r = fn(map, fp8 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims,
-                          strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    return r == CUDA_SUCCESS;
-}
-
 // Row-major [k_rows, mn_cols] bf16 tensor whose contiguous dimension is the operand's row index (MN-major operand), seen as
 // [mn_cols / 64, k_rows, 64]: a box of `box_rows` operand rows x 64 K-steps lands as chunks of 64 rows (8 KiB each, 128B swizzle),
 // the order the matrix descriptor expects, in one copy. One copy per 64-row chunk cost the loading lane up to six instructions per
@@ -1462,7 +1027,7 @@ bool make_map_sf(CUtensorMap* map, const void* ptr, uint64_t rows, uint32_t word
     return r == CUDA_SUCCESS;
 }
 
-template <int kBlockN, bool kFp8, bool kSwiGLU, bool kPair, bool kMx = false, bool kRowScatter = false, bool kSwap = false>
+template <int kBlockN, bool kFp8, bool kSwiGLU, bool kPair, bool kMx = false, bool kRowScatter = false>
 cudaError_t launch_impl(const GroupedGemmArgs& a, cudaStream_t stream) {
     using C = Cfg<kBlockN, kFp8, kSwiGLU, kPair, kMx, kRowScatter>;
     CUtensorMap map_a, map_b, map_sfa, map_sfb;
@@ -1490,7 +1055,7 @@ cudaError_t launch_impl(const GroupedGemmArgs& a, cudaStream_t stream) {
                      : make_map(&map_b, a.b, kFp8, (uint64_t)a.k, (uint64_t)a.m_total, b_box_rows));
     }
     if (!ok) return cudaErrorInvalidValue;
-    auto kernel = grouped_gemm_kernel<kBlockN, kFp8, kSwiGLU, kPair, kMx, kRowScatter, kSwap>;
+    auto kernel = grouped_gemm_kernel<kBlockN, kFp8, kSwiGLU, kPair, kMx, kRowScatter>;
     static bool smem_opted_in[64] = {};  // per device, once: the attribute is sticky
     int dev = 0;
     cudaGetDevice(&dev);
@@ -1546,11 +1111,9 @@ cudaError_t launch_grouped_gemm(const GroupedGemmArgs& a, cudaStream_t stream) {
             if (a.swiglu) {
                 if ((a.n / 2) % 128 != 0) return cudaErrorInvalidValue;  // gate/up halves start on scale-block boundaries
                 if (a.mx_wide && a.cta_pairs) return launch_impl<256, true, true, true, true>(a, stream);
-                if (a.mx_wide && a.swap) return launch_impl<256, true, true, false, true, false, true>(a, stream);
                 if (a.mx_wide) return launch_impl<256, true, true, false, true>(a, stream);
                 return launch_impl<128, true, true, false, true>(a, stream);
             }
-            if (a.mx_wide && a.swap && a.n % 256 == 0) return launch_impl<256, true, false, false, true, false, true>(a, stream);
             if (a.mx_wide) return (a.n % 256 == 0) ? launch_impl<256, true, false, false, true>(a, stream) : cudaErrorInvalidValue;
             if (a.row_info != nullptr) return launch_impl<128, true, false, false, true, true>(a, stream);
             return launch_impl<128, true, false, false, true>(a, stream);

@@ -111,7 +111,7 @@ struct PlanOffsets {
 };
 
 __global__ void __launch_bounds__(kScanThreads, 1) build_plan_kernel(const int64_t* __restrict__ topk_idx, const __grid_constant__ PlanOffsets offs,
-                                                                     int* __restrict__ m_offsets, int* __restrict__ pos, int* __restrict__ src_row,
+                                                                     int* __restrict__ m_offsets, int* __restrict__ m_ends, int* __restrict__ pos, int* __restrict__ src_row,
                                                                      int* __restrict__ src_k, int num_pairs, int num_topk, int num_local_experts,
                                                                      int first, int count, int per_cta) {
     pdl_wait_predecessor();
@@ -138,6 +138,7 @@ __global__ void __launch_bounds__(kScanThreads, 1) build_plan_kernel(const int64
                         [&](int i) { pos[i] = -1; });
         for (int j = 0; j < nb; ++j) {
             const int end = offs.v[e0 + b0 + j + 1];
+            if (tid == 0) m_ends[first + e0 + b0 + j] = min(offs.v[e0 + b0 + j] + s_run[j], end);
             for (int row = offs.v[e0 + b0 + j] + s_run[j] + tid; row < end; row += kScanThreads) {
                 src_row[row] = -1;
                 src_k[row] = 0;
@@ -147,7 +148,7 @@ __global__ void __launch_bounds__(kScanThreads, 1) build_plan_kernel(const int64
     }
 }
 
-cudaError_t launch_build_plan(const int64_t* topk_idx, const int* host_offsets, int* m_offsets, int* pos, int* src_row, int* src_k,
+cudaError_t launch_build_plan(const int64_t* topk_idx, const int* host_offsets, int* m_offsets, int* m_ends, int* pos, int* src_row, int* src_k,
                               int num_rows, int num_topk, int num_local_experts, cudaStream_t stream) {
     if (num_local_experts < 1) return cudaErrorInvalidValue;
     for (int first = 0; first < num_local_experts; first += kPlanMaxExperts) {
@@ -159,7 +160,7 @@ cudaError_t launch_build_plan(const int64_t* topk_idx, const int* host_offsets, 
         cudaError_t e = cudaSuccess;
         if (smem > 48 * 1024) e = cudaFuncSetAttribute(build_plan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e == cudaSuccess)
-            e = launch_dependent(build_plan_kernel, dim3((count + per_cta - 1) / per_cta), kScanThreads, smem, stream, topk_idx, offs, m_offsets, pos, src_row,
+            e = launch_dependent(build_plan_kernel, dim3((count + per_cta - 1) / per_cta), kScanThreads, smem, stream, topk_idx, offs, m_offsets, m_ends, pos, src_row,
                                  src_k, num_rows * num_topk, num_topk, num_local_experts, first, count, per_cta);
         if (e != cudaSuccess) return e;
     }

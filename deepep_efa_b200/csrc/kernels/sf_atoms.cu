@@ -24,7 +24,8 @@ __device__ __forceinline__ uint32_t ue8m0_word(float scale) {
     return e * 0x01010101u;
 }
 
-__global__ void sfa_atoms_kernel(const float* __restrict__ scales, uint8_t* __restrict__ atoms, int rows, int num_kb, long long total) {
+__global__ void sfa_atoms_kernel(const float* __restrict__ scales, uint8_t* __restrict__ atoms, int rows, int num_kb, const int* __restrict__ group_counts,
+                                 int rows_per_group, long long total) {
     pdl_wait_predecessor();
     pdl_release_successor();
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -32,11 +33,19 @@ __global__ void sfa_atoms_kernel(const float* __restrict__ scales, uint8_t* __re
         const long long tk = i >> 5;           // tile * num_kb + kb
         const int kb = (int)(tk % num_kb);
         const long long tile = tk / num_kb;
+        // low-latency layout: most rows of most groups hold nothing (256 experts of 128 rows with four each, 56 K blocks: 7.3 MB of
+        // scales to read otherwise)
+        long long end = rows;
+        if (group_counts != nullptr) {
+            const long long group = tile * 128 / rows_per_group;
+            end = group * rows_per_group + group_counts[group];
+            if (tile * 128 + m0 >= end) continue;
+        }
         uint32_t w[4];
 #pragma unroll
         for (int m1 = 0; m1 < 4; ++m1) {
             const long long row = tile * 128 + m0 + 32 * m1;
-            w[m1] = row < rows ? ue8m0_word(scales[row * num_kb + kb]) : 127u * 0x01010101u;  // 2^0 for padding rows
+            w[m1] = row < end ? ue8m0_word(scales[row * num_kb + kb]) : 127u * 0x01010101u;  // 2^0 for padding rows
         }
         *reinterpret_cast<uint4*>(atoms + tk * 512 + m0 * 16) = make_uint4(w[0], w[1], w[2], w[3]);
     }
@@ -80,12 +89,14 @@ __global__ void sfb_atoms_kernel(const float* __restrict__ scales, uint8_t* __re
 
 }  // namespace
 
-cudaError_t launch_build_sfa_atoms(const float* scales, uint8_t* atoms, int rows, int num_kb, cudaStream_t stream) {
+cudaError_t launch_build_sfa_atoms(const float* scales, uint8_t* atoms, int rows, int num_kb, const int* group_counts, int rows_per_group,
+                                   cudaStream_t stream) {
+    if (group_counts != nullptr && (rows_per_group <= 0 || rows_per_group % 128 != 0 || rows % rows_per_group != 0)) return cudaErrorInvalidValue;
     const long long tiles = (rows + 127) / 128;
     const long long total = tiles * num_kb * 32;
     if (total <= 0) return cudaSuccess;
     const int blocks = (int)((total + 255) / 256 < 4096 ? (total + 255) / 256 : 4096);
-    return launch_dependent(sfa_atoms_kernel, dim3(blocks), 256, 0, stream, scales, atoms, rows, num_kb, total);
+    return launch_dependent(sfa_atoms_kernel, dim3(blocks), 256, 0, stream, scales, atoms, rows, num_kb, group_counts, rows_per_group, total);
 }
 
 cudaError_t launch_build_sfb_atoms(const float* scales, uint8_t* atoms, int groups, int n, int num_kb, int swiglu, int wide,

@@ -217,16 +217,25 @@ class MoELayer(nn.Module):
         plan = build_expert_plan(recv_idx, counts)
         a = gather_rows(rx, plan.src_row)
         a_s = gather_rows(rs, plan.src_row)
+        how = dict(m_ends=plan.m_ends, timeout_ms=GEMM_TIMEOUT_MS)
         if mx is not None:
             # padding rows of the plan carry all-zero data; whatever exponent their zero scale maps to does not matter
-            wide = plan.num_rows >= WIDE_TILE_MIN_ROWS_PER_EXPERT * self.num_local_experts
-            h = gg.grouped_gemm(a, w13, plan.m_offsets, swiglu=True, sfa_atoms=gg.build_sf_atoms_a(a_s), sfb_atoms=mx[0 if wide else 2])
-            hq, hs = C.per_token_cast_to_fp8(h, True, False)
-            y_perm = gg.grouped_gemm(hq, w2, plan.m_offsets, sfa_atoms=gg.build_sf_atoms_a(hs), sfb_atoms=mx[3 if wide else 1])
+            columns = _token_columns(buf.group_size * x.size(0) * self.cfg.num_topk / self.cfg.num_experts)
+            a_atoms = gg.build_sf_atoms_a(a_s)
+            if columns or plan.num_rows >= WIDE_TILE_MIN_ROWS_PER_EXPERT * self.num_local_experts:
+                # the first GEMM quantises its own output: a wide tile holds one whole scale block of a row
+                hq = torch.empty(plan.num_rows, self.cfg.intermediate, dtype=torch.float8_e4m3fn, device=a.device)
+                ha = torch.empty(plan.num_rows // 128, self.cfg.intermediate // 128, 512, dtype=torch.uint8, device=a.device)
+                C.grouped_gemm(a, w13, plan.m_offsets, 0, True, sfa_atoms=a_atoms, sfb_atoms=mx[0], out_fp8=hq, out_atoms=ha, tokens_as_columns=columns, **how)
+                y_perm = C.grouped_gemm(hq, w2, plan.m_offsets, 0, False, sfa_atoms=ha, sfb_atoms=mx[3], tokens_as_columns=columns, **how)
+            else:
+                h = C.grouped_gemm(a, w13, plan.m_offsets, 0, True, sfa_atoms=a_atoms, sfb_atoms=mx[2], **how)
+                hq, hs = C.per_token_cast_to_fp8(h, True, False)
+                y_perm = C.grouped_gemm(hq, w2, plan.m_offsets, 0, False, sfa_atoms=gg.build_sf_atoms_a(hs), sfb_atoms=mx[1], **how)
         else:
-            h = gg.grouped_gemm(a, w13, plan.m_offsets, swiglu=True, a_scales=a_s, b_scales=s13)
+            h = C.grouped_gemm(a, w13, plan.m_offsets, 0, True, a_s, s13, **how)
             hq, hs = C.per_token_cast_to_fp8(h, False, False)
-            y_perm = gg.grouped_gemm(hq, w2, plan.m_offsets, a_scales=hs, b_scales=s2)
+            y_perm = C.grouped_gemm(hq, w2, plan.m_offsets, 0, False, hs, s2, **how)
         y_recv = unpermute_weighted(y_perm, recv_w, plan, buf.empty_symmetric([rx.size(0), self.cfg.hidden], torch.bfloat16))
         out, _, _ = buf.combine(y_recv, handle)
         return out
@@ -291,19 +300,20 @@ class MoELayer(nn.Module):
             ws[key] = w_
         w_ = ws[key]
         a, a_s = px.view(L * N, H), ps.view(L * N, H // 128)
-        few_rows = R * x.size(0) * cfg.num_topk <= TOKEN_COLUMNS_MAX_ROWS * cfg.num_experts
+        columns = _token_columns(R * x.size(0) * cfg.num_topk / cfg.num_experts)
         y = buf.get_next_low_latency_combine_buffer(handle)
         # rows per expert come as counts; both GEMMs read them where the dispatch left them
         if mx is not None:
             # GEMM1's epilogue quantises its own output (a wide tile holds one whole scale block of a row): e4m3 + scale atoms
-            C.grouped_gemm(a, w13, w_["starts"], 0, True, None, None, None, 0, GEMM_TIMEOUT_MS, cnt, gg.build_sf_atoms_a(a_s), mx[0],
-                           out_fp8=w_["hq"], out_atoms=w_["ha"], m_ends_are_counts=True, sched=w_["sched"], early_table=True, tokens_as_columns=few_rows)
+            C.grouped_gemm(a, w13, w_["starts"], 0, True, None, None, None, 0, GEMM_TIMEOUT_MS, cnt, C.build_sf_atoms_a(a_s, cnt, N), mx[0],
+                           out_fp8=w_["hq"], out_atoms=w_["ha"], m_ends_are_counts=True, sched=w_["sched"], early_table=True, tokens_as_columns=columns)
             C.grouped_gemm(w_["hq"], w2, w_["starts"], 0, False, None, None, y.view(L * N, H), 0, GEMM_TIMEOUT_MS, cnt, w_["ha"], mx[3],
-                           m_ends_are_counts=True, sched=w_["sched"], early_table=True, tokens_as_columns=few_rows)
+                           m_ends_are_counts=True, sched=w_["sched"], early_table=True, tokens_as_columns=columns)
         else:
             C.grouped_gemm(a, w13, w_["starts"], 0, True, a_s, s13, w_["h"], 0, GEMM_TIMEOUT_MS, cnt, m_ends_are_counts=True, sched=w_["sched"])
             C.per_token_cast_to_fp8(w_["h"], False, False, cnt, N, w_["hq"], w_["hs"])
-            C.grouped_gemm(w_["hq"], w2, w_["starts"], 0, False, w_["hs"], s2, y.view(L * N, H), 0, GEMM_TIMEOUT_MS, cnt, m_ends_are_counts=True, sched=w_["sched"])
+            C.grouped_gemm(w_["hq"], w2, w_["starts"], 0, False, w_["hs"], s2, y.view(L * N, H), 0, GEMM_TIMEOUT_MS, cnt, m_ends_are_counts=True, sched=w_["sched"],
+                           early_table=True)
         out, _, _ = buf.low_latency_combine(y, topk_idx, topk_weights, handle, zero_copy=True)
         return out
 
@@ -317,14 +327,20 @@ UNIT_ROWS = 8  # rows of one expert a dispatch warp sends between two arrival-co
 # the register file, and next to the natively block-scaled kernel the dispatch was measured several times slower than on
 # SMs of its own. A GEMM that got every SM before the dispatch CTAs were placed would wait for rows that nobody can send.
 FUSE_CAST_INTO_GEMM1 = True  # wide natively block-scaled tiles: GEMM1's epilogue emits e4m3 + scale atoms itself
-# Decode, natively block-scaled: average rows per expert up to which the GEMMs take the tokens as columns (a tile then multiplies 32 of
-# them at a time instead of 128 rows). One step back to back, rows / columns, us: 64 experts with 12 rows 251 / 226, 16 rows 252 / 227;
-# 32 experts with 24 rows 152 / 149, 32 rows 152 / 162; 16 experts with 64 rows 119 / 144. The average is all the host knows. With skewed
-# routing (popularity 1 / (e + 1)^1.2) a few experts hold most rows, and as columns their tiles take two to four steps of 32; on average /
-# at most, rows, columns, us: 64 experts 12 / 116 227, 225; 128 experts 6 / 97 277, 283; 32 experts 8 / 55 145, 146 and 12 / 82 147, 163; 32
-# smaller ones (2048 -> 1024) 12 / 62 90, 90 and 19 / 93 90, 97; 16 experts 16 / 78 172, 185. (The same layers uniformly: 230, 224; 312, 301;
-# 146, 145 and 146, 146; 91, 80 and 91, 80; 172, 169.)
-TOKEN_COLUMNS_MAX_ROWS = 20
+# Average rows per expert up to which the natively block-scaled GEMMs take the tokens as columns, and up to which a tile has at most 64 of
+# them instead of 128 (five stages in flight instead of four). Both GEMMs of a layer, us, rows / columns by 64 / by 128: 256 experts of 7168 -> 2048 with 4
+# rows 1804 / 1692 / 1723; 64 experts of 4096 -> 1408 with 2 rows 219 / 191 / 191, 36 rows 220 / - / 219, 48 rows 224 / - / 224, 66 rows 226 / - / 245.
+# Skewed routing (popularity 1 / (e + 1)^1.2), average / most rows of an expert: 64 experts 19 / 192 224 / 222 / 218, 38 / 377 237 / 233 / 225; 32 experts
+# 24 / 125 160 / 147 / 135; 128 experts 6 / 121 331 / 319 / 319. The average is all the host knows.
+TOKEN_COLUMNS_MAX_ROWS = 44
+TOKEN_COLUMNS_SMALL_ROWS = 8
+
+
+def _token_columns(rows: float) -> int:
+    """Tokens of a tile for the natively block-scaled GEMMs that take them as columns, or 0 for the form with tokens as rows."""
+    return 0 if rows > TOKEN_COLUMNS_MAX_ROWS else 64 if rows <= TOKEN_COLUMNS_SMALL_ROWS else 128
+
+
 # Natively block-scaled GEMMs: average rows per expert from which the 128x256 tiles are used instead of the 128x128 ones. Since the
 # wide tiles drain their accumulator in two halves they win from the smallest sizes measured on (8 experts x 4096 rows down to 256
 # experts x 128 rows: +22 % to +54 %); below one tile of rows per expert the narrow tiles stay (fewer wasted columns per padded tile).
@@ -454,7 +470,8 @@ def fused_forward_many(layers, xs, idxs, ws, overlap: bool = True, num_dispatch_
         overlapped = comm is not cur
         ga = min(L, max(1, int(round(L * SPLIT_FRACTION)))) if overlapped else L
         if native:
-            wide = R_ * w.num_tokens * K >= WIDE_TILE_MIN_ROWS_PER_EXPERT * E
+            columns = _token_columns(R_ * w.num_tokens * K / E)
+            wide = R_ * w.num_tokens * K >= WIDE_TILE_MIN_ROWS_PER_EXPERT * E or columns != 0
             sfb = l._mx[0 if wide else 2]
             fuse_cast = wide and FUSE_CAST_INTO_GEMM1
         # (first group, number of groups, SMs): the early experts next to the dispatch, the rest on the whole GPU
@@ -473,7 +490,7 @@ def fused_forward_many(layers, xs, idxs, ws, overlap: bool = True, num_dispatch_
                 if fuse_cast:
                     # a wide tile holds one whole scale block of the intermediate per row: the epilogue writes e4m3 + scale atoms itself
                     C.grouped_gemm(w.recv_x, w13[g0:g0 + ng], mo, 0, True, None, None, None, sms1, GEMM_TIMEOUT_MS, me_, w.recv_scales, sfb[g0:g0 + ng],
-                                   out_fp8=w.hq, out_atoms=w.hs, **gate)
+                                   out_fp8=w.hq, out_atoms=w.hs, tokens_as_columns=columns, **gate)
                 else:
                     C.grouped_gemm(w.recv_x, w13[g0:g0 + ng], mo, 0, True, None, None, w.h, sms1, GEMM_TIMEOUT_MS, me_, w.recv_scales, sfb[g0:g0 + ng], **gate)
             else:
@@ -482,7 +499,9 @@ def fused_forward_many(layers, xs, idxs, ws, overlap: bool = True, num_dispatch_
             if not fuse_cast:
                 C.per_token_cast_to_fp8(w.h, True, False, None, 1, w.hq, w.hs, w.m_offsets[L:], True)
             C.grouped_gemm(w.hq, w2, w.m_offsets, 0, False, None, None, None, 0, GEMM_TIMEOUT_MS, w.m_ends, w.hs, l._mx[3 if wide else 1],
-                           row_info=w.recv_info, scatter_bases=w.peer_bases[3 * R_:], sched=w.sched, early_table=True)
+                           row_info=w.recv_info, scatter_bases=w.peer_bases[3 * R_:], sched=w.sched, early_table=True,
+                           # (as columns a row leaves in pieces of 64 bytes: fine for this GPU's memory, too short for NVLink)
+                           tokens_as_columns=columns if R_ == 1 else 0)
         else:
             C.per_token_cast_to_fp8(w.h, False, False, None, 1, w.hq, w.hs, w.m_offsets[L:], False)
             C.grouped_gemm(w.hq, w2, w.m_offsets, 0, False, w.hs, s2, None, 0, GEMM_TIMEOUT_MS, w.m_ends, None, None,

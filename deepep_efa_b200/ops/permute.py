@@ -31,6 +31,7 @@ class ExpertPlan:
     src_k: torch.Tensor      # [M_pad] int32 (0 where padding)
     m_offsets: torch.Tensor  # [L+1] int32
     num_rows: int            # M_pad
+    m_ends: Optional[torch.Tensor] = None  # [L] int32: end of each expert's rows, in front of its padding
 
 
 def build_expert_plan(recv_topk_idx: torch.Tensor, aligned_counts: List[int]) -> ExpertPlan:
@@ -61,7 +62,8 @@ def build_expert_plan(recv_topk_idx: torch.Tensor, aligned_counts: List[int]) ->
     src_row.scatter_(0, tgt, (ids // K).to(torch.int32))
     src_k.scatter_(0, tgt, (ids % K).to(torch.int32))
     src_row[m_pad] = -1
-    return ExpertPlan(pos.to(torch.int32).view(N, K).contiguous(), src_row[:m_pad].contiguous(), src_k[:m_pad].contiguous(), m_offsets, m_pad)
+    return ExpertPlan(pos.to(torch.int32).view(N, K).contiguous(), src_row[:m_pad].contiguous(), src_k[:m_pad].contiguous(), m_offsets, m_pad,
+                      m_offsets[:-1] + torch.bincount(safe[valid], minlength=L).to(torch.int32).cpu())
 
 
 # ---- raw ops with a CPU fallback -------------------------------------------------------------------

@@ -335,6 +335,64 @@ def test_quantised_output_with_tokens_as_columns():
     assert (got[0][0][~live] == 0).all() and got[0][0][live].any()
 
 
+@pytest.mark.parametrize("cap", [64, 128, 160, 192, 224])
+@pytest.mark.parametrize("scatter", [False, True])
+def test_token_columns_tile_sizes(cap, scatter):
+    """Groups at and around every cut of the tiles that take tokens as columns, K blocks fewer than, as many as and more than the ring's
+    stages: bit for bit the rows form, rows that do not count left alone, rows scattered to where their words say."""
+    from deepep_efa_b200 import _ext
+    from deepep_efa_b200.ops.grouped_gemm import build_sf_atoms_a, build_sf_atoms_b
+    C = _ext.load()
+    C.gemm_clear_error(0)
+    torch.manual_seed(cap)
+    step = 64 if cap < 128 else 128
+    counts = [1, 0, 16, 17, step - 1, step, step + 1, cap - 16, cap - 15, cap, cap + 1, cap + 15, cap + 16, step + cap, step + cap + 1, 384]
+    G, stride, I = len(counts), 512, 256
+    cnt = torch.tensor(counts, device="cuda", dtype=torch.int32)
+    starts = torch.arange(G + 1, device="cuda", dtype=torch.int32) * stride
+    live = (torch.arange(stride, device="cuda").unsqueeze(0) < cnt.unsqueeze(1)).view(-1)
+    for K in (128, 512, 1152):
+        a, a_s = C.per_token_cast_to_fp8(torch.randn(G * stride, K, device="cuda").to(torch.bfloat16), True, False)
+        a_s = a_s * torch.exp2(torch.randint(-3, 4, a_s.shape, device="cuda").float())  # another factor in every row and K block
+        sfa = build_sf_atoms_a(a_s)
+        a.view(torch.uint8)[~live] = 0xFF
+        b = torch.randn(G, 2 * I, K, device="cuda").to(torch.float8_e4m3fn)
+        b_s = torch.exp2(torch.randint(-8, -4, (G, 2 * I // 128, K // 128), device="cuda").float())
+        info = torch.full((G * stride,), -1, dtype=torch.int32, device="cuda")
+        info[live] = torch.randperm(sum(counts), device="cuda").int()
+        got = []
+        for columns in (cap, 0):
+            how = dict(m_ends_are_counts=True, tokens_as_columns=columns)
+            q = torch.zeros(G * stride, I, dtype=torch.uint8, device="cuda")
+            atoms = torch.zeros(G * stride // 128, I // 128, 512, dtype=torch.uint8, device="cuda")
+            if not scatter:
+                C.grouped_gemm(a, b, starts, 0, True, None, None, None, 0, 2000.0, cnt, sfa, build_sf_atoms_b(b_s, 2 * I, True, True),
+                               out_fp8=q.view(torch.float8_e4m3fn), out_atoms=atoms, **how)
+            out = torch.full((sum(counts) if scatter else G * stride, 2 * I), 7.0, device="cuda", dtype=torch.bfloat16)
+            extra = dict(row_info=info, scatter_bases=torch.tensor([out.data_ptr()], dtype=torch.int64, device="cuda")) if scatter else {}
+            C.grouped_gemm(a, b, starts, 0, False, None, None, None if scatter else out, 3, 2000.0, cnt, sfa, build_sf_atoms_b(b_s, 2 * I, False, True),
+                           **how, **extra)
+            torch.cuda.synchronize()
+            got.append((q, atoms, out))
+        assert C.gemm_error(0) == 0
+        assert all(torch.equal(x, y) for x, y in zip(*got))
+        out = got[0][2]
+        assert torch.isfinite(out.float()).all() and (scatter or ((out[~live] == 7.0).all() and got[0][0][live].any()))
+
+
+def test_scale_atoms_of_counted_rows():
+    from deepep_efa_b200 import _ext
+    C = _ext.load()
+    counts, stride, nkb = [0, 1, 31, 32, 33, 127, 128, 129, 256], 256, 5
+    s = torch.exp2(torch.randint(-9, 9, (len(counts) * stride, nkb), device="cuda").float())
+    full = C.build_sf_atoms_a(s).view(-1, nkb, 32, 4, 4)
+    some = C.build_sf_atoms_a(s, torch.tensor(counts, dtype=torch.int32, device="cuda"), stride).view(-1, nkb, 32, 4, 4)
+    for g, n in enumerate(counts):
+        for r in range(n):
+            tile, m0, m1 = (g * stride + r) // 128, r % 32, r % 128 // 32
+            assert torch.equal(full[tile, :, m0, m1], some[tile, :, m0, m1])
+
+
 @pytest.mark.parametrize("pair", ["0", "1"])
 @pytest.mark.parametrize("n_out,k_out", [(128, 128), (128, 384), (384, 640), (256, 256)])
 def test_bf16_mn_major_half_width_tiles_and_pairs(monkeypatch, pair, n_out, k_out):
