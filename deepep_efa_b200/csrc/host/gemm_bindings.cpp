@@ -156,13 +156,16 @@ torch::Tensor grouped_gemm(const torch::Tensor& a, const torch::Tensor& b, const
     {
         const char* o = std::getenv("DEEPEP_GEMM_ORDER");
         p.tile_order = (o != nullptr && o[0] == '1') ? 1 : 0;
-        // CTA pairs (cta_group::2) pay off for BF16 with about a thousand rows per expert or more (+1-3 % in a power-limited loop); the FP8 path hands a
-        // window to the epilogue every K block, and the cross-CTA handshake per block costs more than the halved B traffic saves
+        // CTA pairs (cta_group::2), BF16: half of the weight tile per CTA, so a third less to pull from L2. A pair's tile is two row tiles
+        // high, and with few rows per expert (the average of the padded ones is what the host knows) its second half multiplies nothing, or
+        // the output of a weight gradient is the work. Single / pair, us, 64 experts of 4096 -> 2 x 1408 (first product, its input gradient,
+        // its weight gradient), uniform but where noted: 128 rows 255 / 316, 242 / 298, 359 / 567; 242 rows 346 / 329, 403 / 331, 582 / 726; 308 rows 426 /
+        // 406, 485 / 460, 683 / 778; 430 rows, skewed, 581 / 547, 661 / 617, 880 / 884; 512 rows 689 / 565, 754 / 619, 918 / 798; 838 rows, skewed, 1005 / 921,
+        // 1129 / 967, 1287 / 1226. The FP8 promotion hands a window to the epilogue every K block, and the cross-CTA handshake per
+        // block costs more than the halved B traffic saves.
         const char* pr = std::getenv("DEEPEP_GEMM_PAIR");
         if (pr != nullptr && (pr[0] == '0' || pr[0] == '1')) p.cta_pairs = pr[0] == '1';
-        // MN-major weight gradients of 64 experts, 4096 x 2816 each, single CTA / pair: 392 / 449 us at 128 rows per expert (a pair's
-        // tile is two row tiles high and the output, not the product, is the work), 1283 / 1263 us at 832, 4192 / 4009 us at 3136
-        else p.cta_pairs = (!fp8 && p.m_ends == nullptr && ((mode == 1 && !mn_major) || (int64_t)p.m_total >= 1024 * (int64_t)G)) ? 1 : 0;
+        else if (!fp8 && p.m_ends == nullptr) p.cta_pairs = (mode == 1 ? !mn_major || (int64_t)p.m_total >= 480 * (int64_t)G : (int64_t)p.m_total >= 224 * (int64_t)G) ? 1 : 0;
         if (p.num_sms < 2) p.cta_pairs = 0;
         // natively block-scaled e4m3: a pair instantiation exists for the wide SwiGLU tile only
         if (fp8 && !(p.sfa_atoms != nullptr && p.mx_wide == 1)) p.cta_pairs = (pr != nullptr && pr[0] == '1' && p.sfa_atoms == nullptr) ? 1 : 0;
