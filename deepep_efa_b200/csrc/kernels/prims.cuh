@@ -166,7 +166,14 @@ constexpr float kFp8AmaxFloor = 1e-4f;
 
 __device__ __forceinline__ void fp8_scale_from_amax(float amax, bool round_pow2, float& scale, float& inv_scale) {
     amax = fmaxf(amax, kFp8AmaxFloor);
-    if (round_pow2) {
+    const uint32_t bits = __float_as_uint(amax);
+    if (round_pow2 && bits < 0x7f800000u) {
+        // 448 = 1.75 * 2^8, so the smallest power of two >= amax / 448 is eight exponents below amax's own, or seven where amax's
+        // significand is above 1.75 (a quotient above 1 never rounds to 1 here: the first one is 1.14 half steps above it)
+        const uint32_t e = (bits >> 23) - 8u + ((bits & 0x7fffffu) > 0x600000u ? 1u : 0u);
+        scale = __uint_as_float(e << 23);
+        inv_scale = __uint_as_float((254u - e) << 23);
+    } else if (round_pow2) {
         // smallest power of two >= amax/448
         const float s = amax / kFp8Max;
         int e;
