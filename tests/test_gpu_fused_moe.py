@@ -165,3 +165,31 @@ def test_fused_dispatch_overflow_is_reported_not_written():
 def test_expert_major_dispatch_with_many_experts_per_cta():
     """More experts than a CTA lists in one pass over the ids (two emulated ranks share the SMs)."""
     test_expert_major_dispatch_places_rows(2, 9, 128, 2048, 4, False)
+
+
+@pytest.mark.parametrize("T,H,E,K,native", [(1, 128, 4, 1, True), (5, 512, 300, 3, False), (77, 4224, 6, 4, True), (130, 7296, 5, 5, False), (40, 7168, 16, 8, True)])
+def test_lone_dispatch_places_rows_like_the_general_one(T, H, E, K, native):
+    """The dispatch of a lone rank that may use the whole GPU against the one with a bounded number of CTAs: rows, scales, row words, places
+    and arrival counts; hidden sizes below, at and past one pass of a warp, fewer and more experts than a CTA has threads."""
+    import deepep_efa_b200 as ep
+    from deepep_efa_b200.models.moe import UNIT_ROWS
+    vc, layers, xs, idxs, ws = _setup(1, T, H, 256, E, K, native)
+    try:
+        C = ep._ext.load()
+        rt, w, idx = vc.buffers[0].runtime, layers[0].fused_workspace(T), idxs[0]
+        q, s = C.per_token_cast_to_fp8(xs[0], native, False)
+        got = []
+        for sms in (7, 148 * 6):
+            for t in (w.recv_x.view(torch.uint8), w.recv_scales_raw, w.recv_info):
+                t.zero_()
+            C.em_notify([rt], [(idx, w.recv_x, w.recv_scales_raw, w.recv_info, w.stage, w.my_counts, w.sel_list, w.send_base, w.unit_start, w.m_offsets,
+                                w.m_ends, w.peer_bases)], E, UNIT_ROWS)
+            dst = torch.full((T * K,), -1, dtype=torch.int32, device="cuda")
+            C.em_dispatch([rt], [(q, w.my_counts, w.sel_list, w.send_base, w.unit_start, w.peer_bases, dst, None, s)], E, K, UNIT_ROWS, native, native, sms)
+            torch.cuda.synchronize()
+            assert torch.equal(w.arrived, w.expected)
+            got.append([t.clone() for t in (w.recv_x.view(torch.uint8), w.recv_scales_raw, w.recv_info, dst)])
+        vc.buffers[0].check_status()
+        assert all(torch.equal(a, b) for a, b in zip(*got)) and (got[0][3].view(-1) >= 0).sum() == (idx >= 0).sum()
+    finally:
+        vc.destroy()
