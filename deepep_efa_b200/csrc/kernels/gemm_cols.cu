@@ -4,7 +4,7 @@
 // A layer whose experts have about a tile of rows each is bound by its weights, which every row tile pulls anew from L2: with tiles
 // of 128 rows, an expert of 137 tokens costs two passes over them and 256 rows of products. Here a tile is 256 weight rows by ALL
 // tokens of the group up to `token_cap` (at most 224, in steps of 16), so the weights of such an expert are read once and the products are those of its
-// tokens; a longer group is cut into tiles of 128 tokens (64 where `token_cap` is below that) and a last one of up to `token_cap`.
+// tokens; a longer group is cut into several (see row_tiles).
 //
 // The issuer's and the loader's loops are run by whole warps, with one elected lane issuing. The same loops as a branch that only lane 0 takes
 // were slower, most of all here, where a K block of few tokens is eight short MMAs (one B200, both GEMMs, decode of 20 tokens, 64 experts of 4096 ->
@@ -17,7 +17,9 @@
 // A stage holds 32 KB of weights, `token_cap` rows of 128 bytes and the scale atoms; the ring has as many stages as fit (five for 64
 // tokens, four up to 160, three beyond), because bytes in flight are what streams weights. There is one accumulator window (two products of up
 // to 224 columns and the scale factors fill TMEM): the epilogue packs it to BF16 in registers, hands it back, and does the rest (row
-// maxima, quantisation, stores) while the next tile accumulates.
+// maxima, quantisation, stores) while the next tile accumulates. That rest still bounds tiles of many tokens and few K blocks: without it (timing only)
+// 64 experts of 188 rows, 4096 -> 1408, took 258 us instead of 358 for both GEMMs, and 256 experts of 128 rows, 7168 -> 2048, 1875 instead of 2100.
+// Two chunks of tokens per exchange, scales from the exponent's bits and stores of 16 bytes brought the first to 304 (tokens as rows: 341).
 //
 // Every wait is bounded, as in grouped_gemm.cu.
 #include <algorithm>
@@ -54,7 +56,8 @@ struct ColTile {
 };
 
 __host__ __device__ constexpr size_t cols_table_bytes(int groups) { return ((size_t)(groups + 1) * 4 + 15) / 16 * 16; }
-__host__ __device__ constexpr size_t cols_exchange_bytes(int cap, bool swiglu) { return swiglu ? (size_t)2 * cap * 16 : 0; }
+// SwiGLU: maxima of two tiles; else a block of 8 tokens x 32 features per epilogue warp
+__host__ __device__ constexpr size_t cols_exchange_bytes(int cap, bool swiglu) { return swiglu ? (size_t)2 * cap * 16 : (size_t)kColsEpiWarps * 512; }
 __host__ __device__ constexpr int cols_stage_bytes(int cap) { return kWeightBytes + cap * kKBlockBytes + kSfStageBytes; }
 
 template <bool kSwiGLU>
@@ -74,7 +77,8 @@ token_cols_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
     uint64_t* tile_free = tile_full + kTileSlots;
     static_assert(2 * kMaxStages + 2 + 2 * kTileSlots <= 32, "barrier block");
     int* tile_start = reinterpret_cast<int*>(bars + 32);  // [G+1]
-    volatile uint32_t* xch = reinterpret_cast<volatile uint32_t*>(reinterpret_cast<uint8_t*>(tile_start) + cols_table_bytes(G));  // [2][cap][4]
+    uint8_t* xch_base = reinterpret_cast<uint8_t*>(tile_start) + cols_table_bytes(G);
+    volatile uint32_t* xch = reinterpret_cast<volatile uint32_t*>(xch_base);  // SwiGLU: [2][cap][4]
     __shared__ uint32_t s_tmem_base;
     __shared__ int s_abort;
     __shared__ volatile int s_tile[kTileSlots];
@@ -106,9 +110,10 @@ token_cols_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
         pdl_wait_predecessor();
         if (!p.hold_successor) pdl_release_successor();
     }
-    // row tiles of a group: `step` tokens each and a last one of up to `cap`; a tile starts on a scale atom or in the middle of one
-    const int step = cap < 128 ? 64 : 128;
-    auto row_tiles = [&](int n) { return n <= 0 ? 0 : n <= cap ? 1 : 1 + (n - cap + step - 1) / step; };
+    // Row tiles of a group: one of up to `cap` tokens, or `step` of them each, the last one of up to `cap` where the step is a whole scale
+    // atom. A tile starts on an atom or in the middle of one, and touches two at most.
+    const int step = cap < 128 ? 64 : cap < 192 ? 128 : 192;
+    auto row_tiles = [&](int n) { return n <= 0 ? 0 : n <= cap ? 1 : step == 128 ? 1 + (n - cap + 127) / 128 : (n + step - 1) / step; };
     if (warp == 2) {
         int run = 0;
         for (int g0 = 0; g0 < G; g0 += 32) {
@@ -229,7 +234,7 @@ token_cols_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
                 if (lane == 0) atomicMin(&p.trace[0], global_timer_ns());
                 stamped = true;
             }
-            const int atoms = t.cols > 128 ? 2 : 1;
+            const int atoms = (t.row & 127) + t.cols > 128 ? 2 : 1;
             const uint32_t tx = kWeightBytes + t.cols * kKBlockBytes + 512 * (2 + atoms);
             const uint8_t* sfw = p.sfb_atoms + ((size_t)t.group * tiles_n + t.nt) * num_kb * 1024;
             const uint8_t* sft = p.sfa_atoms + (size_t)(t.row >> 7) * num_kb * 512;
@@ -292,7 +297,7 @@ token_cols_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
         for (int tile = blockIdx.x; tile < total_tiles && ok; tile = next_tile(tile)) {
             decode(tile, g, t);
             const uint32_t idesc = make_idesc_mx(t.cols, kBlockM);
-            const bool two_atoms = t.cols > 128;
+            const bool two_atoms = (t.row & 127) + t.cols > 128;
             if (!__all_sync(0xffffffffu, mbar_wait(tmem_empty, win_phase ^ 1, abort_flag, limit, note, wait_id(3, tile, 0, 0)))) break;
             win_phase ^= 1;
             for (int kb = 0; kb < num_kb; ++kb) {
@@ -422,72 +427,90 @@ token_cols_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
                         if ((lane & 3) < 2) xs[(t0 + (lane >> 2) * 2 + (lane & 1)) * 4 + q] = tag | bits;
                     }
                 }
+                // Two chunks at a time: lanes 0-15 have the tokens of the first, lanes 16-31 those of the second.
 #pragma unroll
-                for (int c = 0; c < kChunks; ++c) {
-                    const int t0 = (2 * c + half) * kChunk;
-                    if (t0 < t.cols && ok) {
+                for (int c2 = 0; c2 < kChunks; c2 += 2) {
+                    if ((2 * c2 + half) * kChunk < t.cols && ok) {
+                        const int tok = (2 * (c2 + (lane >> 4)) + half) * kChunk + (lane & 15);
                         uint32_t most = 0;
-                        if (lane < kChunk) {
-                            volatile uint32_t* slot = xs + (t0 + lane) * 4;
-                            const long long w0 = clock64();
-                            for (int i = 0; i < 4 && ok; ++i) {
-                                uint32_t w = slot[i];
-                                while ((w & 0xffff0000u) != tag) {
+                        if (tok < t.cols) {
+                            const uint32_t slot = smem_u32(const_cast<const uint32_t*>(xs) + tok * 4);
+                            uint32_t w[4];
+                            auto look = [&]() {
+                                asm volatile("ld.volatile.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]) : "r"(slot) : "memory");
+                                return (((w[0] ^ tag) | (w[1] ^ tag) | (w[2] ^ tag) | (w[3] ^ tag)) >> 16) == 0;
+                            };
+                            if (!look()) {
+                                const long long w0 = clock64();
+                                while (!look()) {
                                     if (*abort_flag || clock64() - w0 > limit) {
                                         if (!*abort_flag && note != nullptr) atomicCAS(note, 0ull, wait_id(7, tile, 0, warp));
                                         *abort_flag = 1;
                                         ok = false;
                                         break;
                                     }
-                                    w = slot[i];
                                 }
-                                most = max(most, w & 0xffffu);
                             }
+                            most = max(max(w[0], w[1]), max(w[2], w[3])) & 0xffffu;
                         }
                         ok = __all_sync(0xffffffffu, ok);
                         if (ok) {
                             float scale, inv;
                             fp8_scale_from_amax(__uint_as_float(most << 16), true, scale, inv);
-                            if (q == 0 && lane < kChunk && t0 + lane < t.valid) {
-                                const int row = t.row + t0 + lane;
+                            if (q == 0 && tok < t.valid) {
+                                const int row = t.row + tok;
                                 *reinterpret_cast<uint32_t*>(p.c_atoms + ((size_t)(row >> 7) * (ldc / 128) + t.nt) * 512 + (row & 31) * 16 + ((row >> 5) & 3) * 4) =
                                     ((__float_as_uint(scale) >> 23) & 0xffu) * 0x01010101u;
                             }
 #pragma unroll
-                            for (int i = 0; i < kChunk; i += 4) {
-                                const float2 lo = bf16x2_to_f2(keep[c][i / 2]), hi = bf16x2_to_f2(keep[c][i / 2 + 1]);
-                                const float x0 = lo.x * __shfl_sync(0xffffffffu, inv, i), x1 = lo.y * __shfl_sync(0xffffffffu, inv, i + 1);
-                                const float x2 = hi.x * __shfl_sync(0xffffffffu, inv, i + 2), x3 = hi.y * __shfl_sync(0xffffffffu, inv, i + 3);
-                                const uint32_t w = transpose_bytes_4x4(pack_e4m3x4(x0, x1, x2, x3), lane);
-                                const int tok = t0 + i + (lane & 3);
-                                if (tok < t.valid)
-                                    *reinterpret_cast<uint32_t*>(p.c_fp8 + (size_t)(t.row + tok) * ldc + t.nt * 128 + q * 32 + (lane & ~3)) = w;
+                            for (int c = c2; c < c2 + 2 && c < kChunks; ++c) {
+                                const int t0 = (2 * c + half) * kChunk;
+                                if (t0 >= t.cols) break;
+                                uint8_t* dst = p.c_fp8 + (size_t)(t.row + t0 + (lane & 3)) * ldc + t.nt * 128 + q * 32 + (lane & ~3);
+#pragma unroll
+                                for (int i = 0; i < kChunk; i += 4) {
+                                    const float2 lo = bf16x2_to_f2(keep[c][i / 2]), hi = bf16x2_to_f2(keep[c][i / 2 + 1]);
+                                    const int from = (c & 1) * 16 + i;
+                                    const float x0 = lo.x * __shfl_sync(0xffffffffu, inv, from), x1 = lo.y * __shfl_sync(0xffffffffu, inv, from + 1);
+                                    const float x2 = hi.x * __shfl_sync(0xffffffffu, inv, from + 2), x3 = hi.y * __shfl_sync(0xffffffffu, inv, from + 3);
+                                    const uint32_t w = transpose_bytes_4x4(pack_e4m3x4(x0, x1, x2, x3), lane);
+                                    if (t0 + i + (lane & 3) < t.valid) *reinterpret_cast<uint32_t*>(dst + (size_t)i * ldc) = w;
+                                }
                             }
                         }
                     }
                 }
             } else {
-                // two lanes exchange halves, so that each stores two neighbouring features of one token: 64 contiguous bytes per token
-                const int col = t.nt * kWeightRows + q * 32 + (lane & ~1);
+                // Two lanes exchange halves, so that each has two neighbouring features of one token; eight tokens then pass through shared
+                // memory, and every lane stores 16 bytes: 64 contiguous ones per token.
+                uint32_t* block = reinterpret_cast<uint32_t*>(xch_base) + (warp - 2) * 128;
+                const int col = t.nt * kWeightRows + q * 32 + (lane & 3) * 8;
 #pragma unroll
                 for (int c = 0; c < kChunks; ++c) {
                     const int t0 = (2 * c + half) * kChunk;
                     if (t0 < t.cols) {
 #pragma unroll
-                        for (int i = 0; i < 8; ++i) {
-                            const int tok = t0 + 2 * i + (lane & 1);
+                        for (int g8 = 0; g8 < 2; ++g8) {
+                            const int tok = t0 + g8 * 8 + (lane >> 2);
                             __nv_bfloat16* dst = nullptr;
                             if (scatter) {
-                                const int word = __shfl_sync(0xffffffffu, info[c], 2 * i + (lane & 1));
+                                const int word = __shfl_sync(0xffffffffu, info[c], g8 * 8 + (lane >> 2));
                                 if (word >= 0) dst = reinterpret_cast<__nv_bfloat16*>(p.scatter_bases[word >> 24]) + (size_t)(word & 0xffffff) * ldc + col;
                             } else if (tok < t.valid) {
                                 dst = reinterpret_cast<__nv_bfloat16*>(p.c) + (size_t)(t.row + tok) * ldc + col;
                             }
 #pragma unroll
                             for (int h = 0; h < 2; ++h) {
-                                const uint32_t w = keep[c][h * 8 + i];
-                                const uint32_t o = __shfl_xor_sync(0xffffffffu, w, 1);
-                                if (dst != nullptr) *reinterpret_cast<uint32_t*>(dst + h * 128) = __byte_perm(w, o, (lane & 1) ? 0x3276 : 0x5410);
+#pragma unroll
+                                for (int i = 0; i < 4; ++i) {
+                                    const uint32_t w = keep[c][h * 8 + g8 * 4 + i];
+                                    const uint32_t o = __shfl_xor_sync(0xffffffffu, w, 1);
+                                    block[(2 * i + (lane & 1)) * 16 + (lane >> 1)] = __byte_perm(w, o, (lane & 1) ? 0x3276 : 0x5410);
+                                }
+                                __syncwarp();
+                                const int4 piece = *reinterpret_cast<const int4*>(block + lane * 4);
+                                __syncwarp();
+                                if (dst != nullptr) *reinterpret_cast<int4*>(dst + h * 128) = piece;
                             }
                         }
                     }

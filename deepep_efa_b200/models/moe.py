@@ -327,18 +327,21 @@ UNIT_ROWS = 8  # rows of one expert a dispatch warp sends between two arrival-co
 # the register file, and next to the natively block-scaled kernel the dispatch was measured several times slower than on
 # SMs of its own. A GEMM that got every SM before the dispatch CTAs were placed would wait for rows that nobody can send.
 FUSE_CAST_INTO_GEMM1 = True  # wide natively block-scaled tiles: GEMM1's epilogue emits e4m3 + scale atoms itself
-# Average rows per expert up to which the natively block-scaled GEMMs take the tokens as columns, and up to which a tile has at most 64 of
-# them instead of 128 (five stages in flight instead of four). Both GEMMs of a layer, us, rows / columns by 64 / by 128: 256 experts of 7168 -> 2048 with 4
-# rows 1804 / 1692 / 1723; 64 experts of 4096 -> 1408 with 2 rows 219 / 191 / 191, 36 rows 220 / - / 219, 48 rows 224 / - / 224, 66 rows 226 / - / 245.
-# Skewed routing (popularity 1 / (e + 1)^1.2), average / most rows of an expert: 64 experts 19 / 192 224 / 222 / 218, 38 / 377 237 / 233 / 225; 32 experts
-# 24 / 125 160 / 147 / 135; 128 experts 6 / 121 331 / 319 / 319. The average is all the host knows.
-TOKEN_COLUMNS_MAX_ROWS = 44
-TOKEN_COLUMNS_SMALL_ROWS = 8
-
-
+# Natively block-scaled GEMMs: where the tokens are taken as columns, by the average rows per expert, which is all the host knows. Both GEMMs
+# of a layer, us, rows / columns (two boxes where two figures are given). As rows an expert takes tiles of 128 rows, so columns win
+# where few of those would be filled and, once most experts have a second tile with little in it, up to where a tile of columns ends.
+#   256 experts of 7168 -> 2048: 4 rows 1804 / 1692; 128 rows 2465, 2448 / 2127, 2192.
+#   128 experts of 7168 -> 2048: 38 rows 975 / 940; 75 rows 971 / 979 to 1074; 100 rows 1085 / 1119; 119 rows 1129 / 1119; 156 rows 1718 / 1310; 200 rows 1809 / 1383.
+#   64 experts of 4096 -> 1408: 2 rows 219 / 191; 48 rows 224 / 219; 73 rows 233 / 231; 94 rows 227 / 238; 117 rows 244 / 248; 131 rows 300 / 269; 150 rows 359 / 294;
+#   187 rows 341 / 304; 216 rows 355 / 362; 375 rows 503 / 500 to 594.
+# Skewed routing (popularity 1 / (e + 1)^1.2): 64 experts 38 rows 247 / 224, 75 rows 264 / 242, 150 rows 319 / 299, 188 rows 341 / 327; 128 experts 19 rows 973 / 927, 125
+# rows 1291 to 1354 / 1271 to 1385; 256 experts 128 rows 2825 to 3025 / 2905 to 3125.
+# A tile of 64 tokens leaves room for five stages instead of four: worth 2 % with 4 rows per expert, and lost again with 19 and skewed routing.
 def _token_columns(rows: float) -> int:
     """Tokens of a tile for the natively block-scaled GEMMs that take them as columns, or 0 for the form with tokens as rows."""
-    return 0 if rows > TOKEN_COLUMNS_MAX_ROWS else 64 if rows <= TOKEN_COLUMNS_SMALL_ROWS else 128
+    if rows <= 60:
+        return 64 if rows <= 8 else 128
+    return 0 if rows <= 120 or rows > 200 else 160 if rows <= 136 else 192 if rows <= 164 else 224
 
 
 # Natively block-scaled GEMMs: average rows per expert from which the 128x256 tiles are used instead of the 128x128 ones. Since the

@@ -345,8 +345,8 @@ def test_token_columns_tile_sizes(cap, scatter):
     C = _ext.load()
     C.gemm_clear_error(0)
     torch.manual_seed(cap)
-    step = 64 if cap < 128 else 128
-    counts = [1, 0, 16, 17, step - 1, step, step + 1, cap - 16, cap - 15, cap, cap + 1, cap + 15, cap + 16, step + cap, step + cap + 1, 384]
+    step = 64 if cap < 128 else 128 if cap < 192 else 192
+    counts = [1, 0, 16, 17, step - 1, step, step + 1, cap - 16, cap - 15, cap, cap + 1, cap + 15, cap + 16, step + cap, step + cap + 1, 384, 385, 448]
     G, stride, I = len(counts), 512, 256
     cnt = torch.tensor(counts, device="cuda", dtype=torch.int32)
     starts = torch.arange(G + 1, device="cuda", dtype=torch.int32) * stride
