@@ -1028,7 +1028,7 @@ __global__ void __launch_bounds__(kLLThreads, 2) combine_lone(const __grid_const
                     }
                 }
             }
-            if (early) pdl_wait_predecessor();  // from here on everything is final; returns at once in later rounds
+            if (early) pdl_wait_predecessor();  // from here on everything is final; returns at once from the second token on
             if (sure) break;
             if (early && slot >= 0) info = __ldcg(a.src_info + slot);
             const bool wrong = e >= 0 && (slot < 0 || info != t);

@@ -328,7 +328,7 @@ UNIT_ROWS = 8  # rows of one expert a dispatch warp sends between two arrival-co
 # SMs of its own. A GEMM that got every SM before the dispatch CTAs were placed would wait for rows that nobody can send.
 FUSE_CAST_INTO_GEMM1 = True  # wide natively block-scaled tiles: GEMM1's epilogue emits e4m3 + scale atoms itself
 # Natively block-scaled GEMMs: where the tokens are taken as columns, by the average rows per expert, which is all the host knows. Both GEMMs
-# of a layer, us, rows / columns (two boxes where two figures are given). As rows an expert takes tiles of 128 rows, so columns win
+# of a layer, us, rows / columns (two runs where two figures are given). As rows an expert takes tiles of 128 rows, so columns win
 # where few of those would be filled and, once most experts have a second tile with little in it, up to where a tile of columns ends.
 #   256 experts of 7168 -> 2048: 4 rows 1804 / 1692; 128 rows 2465, 2448 / 2127, 2192.
 #   128 experts of 7168 -> 2048: 38 rows 975 / 940; 75 rows 971 / 979 to 1074; 100 rows 1085 / 1119; 119 rows 1129 / 1119; 156 rows 1718 / 1310; 200 rows 1809 / 1383.
