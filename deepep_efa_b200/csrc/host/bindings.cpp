@@ -727,6 +727,7 @@ void fill_ll_combine(dx::LLCombineArgs& a, Runtime* rt, const torch::Tensor& x, 
     a.pull = pull ? 1 : 0;
     a.close_barrier = (pull && close_barrier) ? 1 : 0;
     a.x_off = 0;
+    a.settled = 0;
     a.send_row = nullptr;
     if (send_row.has_value()) {
         DX_CHECK(send_row->is_cuda() && send_row->scalar_type() == torch::kInt32 && send_row->is_contiguous() &&
@@ -738,6 +739,11 @@ void fill_ll_combine(dx::LLCombineArgs& a, Runtime* rt, const torch::Tensor& x, 
         DX_CHECK(xo >= 0 && xo % 16 == 0, "pull combine: x must live in this rank's symmetric buffer");
         DX_CHECK(send_row.has_value(), "pull combine: send_row is missing");
         a.x_off = (uint64_t)xo;
+        // Rows may be gathered beside the dispatch of their handle unless that dispatch is what writes them: of the low-latency region (where
+        // x may be the landing zone itself, as in a round trip without experts) only the combine buffers are the caller's to fill.
+        const uint64_t begin = (uint64_t)xo, end = begin + (uint64_t)x.numel() * x.element_size();
+        const bool in_region = begin < rt->core->ll_base() + rt->core->ll_bytes() && end > rt->core->ll_base();
+        a.settled = (!in_region || begin == lay.combine_src_off[0] || begin == lay.combine_src_off[1]) ? 1 : 0;
     }
 }
 

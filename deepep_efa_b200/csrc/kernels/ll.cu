@@ -793,8 +793,9 @@ __global__ void __launch_bounds__(kLLThreads, 1) combine_pull(const __grid_const
     const int n16 = H / 8;
     const int tid = threadIdx.x;
     // When this kernel directly follows the dispatch of its handle, programmatic dependent launch lets its CTAs start while
-    // that dispatch still waits for the last rows of the other ranks. Nothing this kernel reads depends on those rows: the
-    // expert outputs were final before the dispatch began, and the row numbers it needs are written early by the dispatch's
+    // that dispatch still waits for the last rows of the other ranks. Nothing this kernel reads depends on those rows as long as x is
+    // no memory that a dispatch writes (`settled`; the received rows themselves are, and a row number says nothing about them): the
+    // expert outputs were then final before the dispatch began, and the row numbers it needs are written early by the dispatch's
     // token CTAs, each word tagged with the call it belongs to. So a CTA that finds its dispatch still in flight (started, not
     // yet committed) does its work first and waits for the predecessor only before it exits, which keeps the stream's order of
     // completion. In every other case (dispatch already complete: an expert GEMM ran in between, or the launch is an ordinary
@@ -804,7 +805,7 @@ __global__ void __launch_bounds__(kLLThreads, 1) combine_pull(const __grid_const
     if (tid == 0) {
         const uint64_t started = *reinterpret_cast<volatile uint64_t*>(c.seq + kLLStartedWord0 + a.parity);
         const uint64_t committed = *reinterpret_cast<volatile uint64_t*>(c.seq + kFamLLDispatch);
-        s_early = committed < started ? 1 : 0;
+        s_early = (a.settled && committed < started) ? 1 : 0;
         s_seq_d = started;
     }
     __syncthreads();
@@ -957,9 +958,9 @@ __global__ void __launch_bounds__(kLLThreads, 1) combine_pull(const __grid_const
 
 // A lone rank's expert outputs are in its own memory wherever x lives, so the rows are read in place: no announcement, no copy into a
 // stage, no closing round. One thread has one 16-byte column of a token, with the loads of eight rows in flight; warps do not wait for
-// each other. A combine that directly follows the dispatch of its handle gathers beside it, as combine_pull does: the dispatch raises the
-// parity's in-flight word by its number of CTAs before any of them allows this launch, and each takes one off as its last act, so the
-// word is zero whenever anything came in between. Only reads happen early; results are stored after the predecessor has completed, because
+// each other. A combine that directly follows the dispatch of its handle gathers beside it, as combine_pull does (and with the same exception,
+// the received rows themselves): the dispatch raises the parity's in-flight word by its number of CTAs before any of them allows this
+// launch, and each takes one off as its last act, so the word is zero whenever a kernel that waits for its own predecessor came in between. Only reads happen early; results are stored after the predecessor has completed, because
 // their memory may be a block that the predecessor still reads (freed by the caller between the two calls).
 // kFind (x is an ordinary tensor): src_info decides which row of the expert is the token's, so that the selections of a token may come in
 // another order than at the dispatch, as with the staged form. It is loaded with the row itself; the search is for the odd case.
@@ -973,7 +974,7 @@ __global__ void __launch_bounds__(kLLThreads, 2) combine_lone(const __grid_const
     const bool traced = blockIdx.x == 0 || blockIdx.x == gridDim.x - 1;
     const int tslot = blockIdx.x == 0 ? 0 : 1;
     if (traced) trace_stamp(c, kFamLLCombine, tslot, 0);
-    bool early = *reinterpret_cast<volatile uint64_t*>(c.seq + kLLInFlightWord0 + a.parity) != 0;
+    bool early = (kFind || a.settled) && *reinterpret_cast<volatile uint64_t*>(c.seq + kLLInFlightWord0 + a.parity) != 0;
     early = __any_sync(0xffffffffu, early);
     if (!early) pdl_wait_predecessor();
     const int tag = ll_count_tag(*reinterpret_cast<volatile uint64_t*>(c.seq + kLLStartedWord0 + a.parity));

@@ -129,3 +129,58 @@ def test_lone_rank_that_masks_itself_sends_nothing():
         buf.check_status()
     finally:
         vc.destroy()
+
+
+@pytest.mark.parametrize("R,T,H", [(1, 128, 7168), (1, 3, 1024), (2, 40, 4096)])
+def test_combine_of_the_rows_just_received(R, T, H):
+    """The landing zone itself as the expert outputs, right behind the dispatch that fills it: a BF16 round trip without experts. Every call has
+    other data, so a row read before it has landed shows."""
+    from deepep_efa_b200 import Buffer
+    from deepep_efa_b200.parallel.virtual import VirtualCluster
+    E, K = 16, 4
+    vc = VirtualCluster(R, num_nvl_bytes=2 << 20, num_rdma_bytes=Buffer.get_low_latency_rdma_size_hint(T, H, R, E), timeout_ms=2000)
+    try:
+        routing = [make_routing(T, E, K, "cuda", seed=r, masked_fraction=0.05) for r in range(R)]
+        idxs, ws = [i for i, _ in routing], [w for _, w in routing]
+        share = [w.masked_fill(i == -1, 0).sum(dim=1, keepdim=True) for i, w in routing]
+        g = torch.Generator(device="cuda").manual_seed(T)
+
+        def data():
+            return [torch.randn(T, H, generator=g, device="cuda").to(torch.bfloat16) for _ in range(R)]
+
+        def step(xs, outs=None):
+            res = vc.low_latency_dispatch(xs, idxs, T, E, use_fp8=False)
+            return [c[0] for c in vc.low_latency_combine([r[0] for r in res], idxs, ws, [r[2] for r in res], outs=outs)]
+
+        def check(xs, outs):
+            for x, o, s in zip(xs, outs, share):
+                # K products of one BF16 value in fp32, then rounded to BF16
+                assert ((o.float() - x.float() * s).norm(dim=1) <= 4e-3 * (x.float() * s).norm(dim=1) + 1e-6).all()
+
+        batches = [data() for _ in range(24)]
+        torch.cuda.synchronize()
+        results = [step(b) for b in batches]
+        torch.cuda.synchronize()
+        for b, o in zip(batches, results):
+            check(b, o)
+        if R == 1:  # both parities from a graph, with other inputs in place before every replay
+            ins, outs = [data(), data()], [[torch.empty(T, H, dtype=torch.bfloat16, device="cuda")] for _ in range(2)]
+            s = torch.cuda.Stream()
+            s.wait_stream(torch.cuda.current_stream())
+            with torch.cuda.stream(s):
+                graph = torch.cuda.CUDAGraph()
+                with torch.cuda.graph(graph, stream=s):
+                    for x, o in zip(ins, outs):
+                        step(x, o)
+            torch.cuda.current_stream().wait_stream(s)
+            for _ in range(4):
+                for x in ins:
+                    x[0].copy_(data()[0])
+                graph.replay()
+                torch.cuda.synchronize()
+                for x, o in zip(ins, outs):
+                    check(x, o)
+        for b in vc.buffers:
+            b.check_status()
+    finally:
+        vc.destroy()
