@@ -958,12 +958,14 @@ __global__ void __launch_bounds__(kLLThreads, 1) combine_pull(const __grid_const
 
 // A lone rank's expert outputs are in its own memory wherever x lives, so the rows are read in place: no announcement, no copy into a
 // stage, no closing round. One thread has one 16-byte column of a token, with the loads of eight rows in flight; warps do not wait for
-// each other. A combine that directly follows the dispatch of its handle gathers beside it, as combine_pull does (and with the same exception,
-// the received rows themselves): the dispatch raises the parity's in-flight word by its number of CTAs before any of them allows this
-// launch, and each takes one off as its last act, so the word is zero whenever a kernel that waits for its own predecessor came in between. Only reads happen early; results are stored after the predecessor has completed, because
-// their memory may be a block that the predecessor still reads (freed by the caller between the two calls).
-// kFind (x is an ordinary tensor): src_info decides which row of the expert is the token's, so that the selections of a token may come in
-// another order than at the dispatch, as with the staged form. It is loaded with the row itself; the search is for the odd case.
+// each other. A combine in symmetric memory that directly follows the dispatch of its handle gathers beside it, as combine_pull does (and with
+// the same exception, the received rows themselves): the dispatch raises the parity's in-flight word by its number of CTAs before any of them
+// allows this launch, and each takes one off as its last act, so the word is zero whenever a kernel that waits for its own predecessor came
+// in between. Only reads happen early; results are stored after the predecessor has completed, because their memory may be a block that the
+// predecessor still reads (freed by the caller between the two calls).
+// kFind (x is an ordinary tensor): whatever launched in between may still be writing x, so the predecessor's end comes first, as for the
+// staged form. src_info decides which row of the expert is the token's, so that the selections of a token may come in another order than at
+// the dispatch, as there too. It is loaded with the row itself; the search is for the odd case.
 // (Two CTAs of 512 threads to an SM: the 64 registers that leaves let the 896 CTAs of 128 threads of 128 tokens x 7168 be resident at once.)
 template <bool kFind>
 __global__ void __launch_bounds__(kLLThreads, 2) combine_lone(const __grid_constant__ LLCombineArgs a, const int slices) {
@@ -974,8 +976,11 @@ __global__ void __launch_bounds__(kLLThreads, 2) combine_lone(const __grid_const
     const bool traced = blockIdx.x == 0 || blockIdx.x == gridDim.x - 1;
     const int tslot = blockIdx.x == 0 ? 0 : 1;
     if (traced) trace_stamp(c, kFamLLCombine, tslot, 0);
-    bool early = (kFind || a.settled) && *reinterpret_cast<volatile uint64_t*>(c.seq + kLLInFlightWord0 + a.parity) != 0;
-    early = __any_sync(0xffffffffu, early);
+    bool early = false;
+    if constexpr (!kFind) {
+        early = a.settled && *reinterpret_cast<volatile uint64_t*>(c.seq + kLLInFlightWord0 + a.parity) != 0;
+        early = __any_sync(0xffffffffu, early);
+    }
     if (!early) pdl_wait_predecessor();
     const int tag = ll_count_tag(*reinterpret_cast<volatile uint64_t*>(c.seq + kLLStartedWord0 + a.parity));
     const bool masked = __ldcg(&c.my_ctrl()->ll_mask[0]) != 0;
@@ -1003,7 +1008,7 @@ __global__ void __launch_bounds__(kLLThreads, 2) combine_lone(const __grid_const
             if (e >= 0 && row >= 0 && row < N) slot = e * N + row;
         }
         int info = t;
-        if (kFind && !early && slot >= 0) info = __ldcg(a.src_info + slot);
+        if (kFind && slot >= 0) info = __ldcg(a.src_info + slot);
         float acc[8];
         for (bool sure = !kFind;; sure = true) {
 #pragma unroll
@@ -1031,7 +1036,6 @@ __global__ void __launch_bounds__(kLLThreads, 2) combine_lone(const __grid_const
             }
             if (early) pdl_wait_predecessor();  // from here on everything is final; returns at once from the second token on
             if (sure) break;
-            if (early && slot >= 0) info = __ldcg(a.src_info + slot);
             const bool wrong = e >= 0 && (slot < 0 || info != t);
             if (!__any_sync(0xffffffffu, wrong)) break;
             if (wrong) {

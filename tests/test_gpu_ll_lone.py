@@ -184,3 +184,43 @@ def test_combine_of_the_rows_just_received(R, T, H):
             b.check_status()
     finally:
         vc.destroy()
+
+
+def _sums(y, idx, w):
+    """What a combine of y [E, N, H] returns when rows were numbered in token order, in fp32."""
+    rows, want = {}, torch.zeros(idx.size(0), y.size(2), device=y.device)
+    for t, es in enumerate(idx.tolist()):
+        for k, e in enumerate(es):
+            if e >= 0:
+                want[t] += w[t, k] * y[e, rows.setdefault(e, 0)].float()
+                rows[e] += 1
+    return want
+
+
+@pytest.mark.parametrize("memory", ["ordinary"])
+def test_combine_behind_a_kernel_that_lets_it_start(memory):
+    """The expert outputs are written between dispatch and combine by a kernel that allows its successor's launch before it has waited itself:
+    another combine of the same handle, whose result is the first rows of the second one's input."""
+    T, H, E, K = 96, 7168, 8, 4
+    vc = _cluster(T, H, E, arena=(2 << 20) + E * T * H * 2)
+    try:
+        buf = vc.buffers[0]
+        src = torch.randn(E, T, H, device="cuda").to(torch.bfloat16)
+        y = buf.empty_symmetric([E, T, H], torch.bfloat16) if memory == "symmetric" else torch.empty(E, T, H, dtype=torch.bfloat16, device="cuda")
+        for i in range(8):
+            idx, w = make_routing(T, E, K, "cuda", seed=i, masked_fraction=0.05)
+            x = make_tokens(T, H, "cuda", seed=i)
+            src.copy_(torch.randn(E, T, H, device="cuda"))
+            y.copy_(src)
+            torch.cuda.synchronize()
+            h = vc.low_latency_dispatch([x], [idx], T, E)[0][2]
+            first = vc.low_latency_combine([src], [idx], [w], [h], outs=[y[0]])[0][0]
+            second = vc.low_latency_combine([y], [idx], [w], [h])[0][0]
+            torch.cuda.synchronize()
+            want = _sums(src, idx, w)
+            assert (first.float() - want).norm() <= 4e-3 * want.norm()
+            want = _sums(torch.cat([first[None], src[1:]]), idx, w)
+            assert (second.float() - want).norm() <= 4e-3 * want.norm()
+        buf.check_status()
+    finally:
+        vc.destroy()
