@@ -32,6 +32,7 @@ struct Runtime {
     cudaStream_t comm_stream = nullptr;
     torch::Tensor layout_scratch;  // grows on demand
     bool all_tokens_sent = true;   // by the last dispatch of a lone rank (see normal_dispatch)
+    int ll_dispatched = -1;        // parity of the low-latency dispatch that no combine has followed yet
 
     Runtime(int rank, int num_ranks, int64_t num_nvl_bytes, int64_t num_ll_bytes, int device, double timeout_ms, bool mask_on_timeout)
         : core(std::make_shared<RuntimeCore>(rank, num_ranks, (uint64_t)num_nvl_bytes, (uint64_t)num_ll_bytes, device, timeout_ms,
@@ -657,6 +658,7 @@ void fill_ll_dispatch(dx::LLDispatchArgs& a, Runtime* rt, const torch::Tensor& x
         DX_CHECK(slot->is_cuda() && slot->scalar_type() == torch::kInt32 && slot->is_contiguous() && slot->numel() >= (int64_t)T * topk_idx.size(1), "send_row must be int32 [T,K] on the GPU");
     a.send_row = ptr_or_null<int>(slot);
     a.num_sms = num_sms;
+    rt->ll_dispatched = parity;
 }
 
 // Per rank tuple: (x, topk_idx, packed_recv_count, layout_range, cumulative_stats|None, wait_stats|None, send_row|None)
@@ -743,8 +745,10 @@ void fill_ll_combine(dx::LLCombineArgs& a, Runtime* rt, const torch::Tensor& x, 
         // x may be the landing zone itself, as in a round trip without experts) only the combine buffers are the caller's to fill.
         const uint64_t begin = (uint64_t)xo, end = begin + (uint64_t)x.numel() * x.element_size();
         const bool in_region = begin < rt->core->ll_base() + rt->core->ll_bytes() && end > rt->core->ll_base();
-        a.settled = (!in_region || begin == lay.combine_src_off[0] || begin == lay.combine_src_off[1]) ? 1 : 0;
+        // Nor where another combine came in between: it lets its successor start before its result is written, and that may be part of x.
+        a.settled = (rt->ll_dispatched == parity && (!in_region || begin == lay.combine_src_off[0] || begin == lay.combine_src_off[1])) ? 1 : 0;
     }
+    rt->ll_dispatched = -1;
 }
 
 // Per rank tuple: (x, topk_idx, topk_weights, src_info, layout_range, out, wait_stats|None, send_row|None)

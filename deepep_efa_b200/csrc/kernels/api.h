@@ -244,7 +244,7 @@ struct LLCombineArgs {
     uint64_t x_off;
     const int* send_row;
     int close_barrier;            // pull form: readers report back before the kernel ends (x is a caller-owned tensor)
-    int settled;                  // pull form: no dispatch writes x, so what a caller put there was final before the dispatch began
+    int settled;                  // pull form: neither the dispatch nor a combine behind it writes x, so x was final before the dispatch began
 };
 cudaError_t launch_ll_combine(const LLCombineArgs* a, int num_virtual, cudaStream_t stream);
 

@@ -197,7 +197,7 @@ def _sums(y, idx, w):
     return want
 
 
-@pytest.mark.parametrize("memory", ["ordinary"])
+@pytest.mark.parametrize("memory", ["ordinary", "symmetric"])
 def test_combine_behind_a_kernel_that_lets_it_start(memory):
     """The expert outputs are written between dispatch and combine by a kernel that allows its successor's launch before it has waited itself:
     another combine of the same handle, whose result is the first rows of the second one's input."""
