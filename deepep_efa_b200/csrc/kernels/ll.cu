@@ -994,7 +994,10 @@ __global__ void __launch_bounds__(kLLThreads, 2) combine_lone(const __grid_const
             const int64_t e64 = __ldg(a.topk_idx + (size_t)t * K + lane);
             unsigned word = (unsigned)ld_relaxed_sys(a.send_row + (size_t)t * K + lane);
             weight = __ldg(a.topk_weights + (size_t)t * K + lane);
-            if ((word >> 16) != (unsigned)tag) {
+            if (kFind) {
+                // other columns than at the dispatch may name a word of another call, or none: then the search finds the row
+                if ((word >> 16) != (unsigned)tag) word = 0;
+            } else if ((word >> 16) != (unsigned)tag) {
                 const long long t0 = clock64();
                 while (early && ((word = (unsigned)ld_relaxed_sys(a.send_row + (size_t)t * K + lane)) >> 16) != (unsigned)tag && clock64() - t0 <= c.timeout_cycles) {
                 }

@@ -224,3 +224,28 @@ def test_combine_behind_a_kernel_that_lets_it_start(memory):
         buf.check_status()
     finally:
         vc.destroy()
+
+
+def test_combine_with_other_columns_than_the_dispatch():
+    """A top-k list that is wider, narrower or longer than the dispatch's, filled up with -1: ordinary tensors allow it."""
+    T, H, E, K = 20, 1024, 8, 3
+    vc = _cluster(32, H, E)
+    try:
+        for i in range(4):
+            idx, w = make_routing(T, E, K, "cuda", seed=i, masked_fraction=0.1)
+            idx[:, 2] = -1
+            y = torch.randn(E, 32, H, device="cuda").to(torch.bfloat16)
+            h = vc.low_latency_dispatch([make_tokens(T, H, "cuda", seed=i)], [idx], 32, E)[0][2]
+            want = vc.low_latency_combine([y], [idx], [w], [h])[0][0]
+            none, zero = torch.full((T, 4), -1, device="cuda"), torch.zeros(T, 4, device="cuda")
+            order = [3, 0, 5, 4, 1, 6, 2]
+            wide = torch.cat([idx, none], 1)[:, order].contiguous(), torch.cat([w, zero], 1)[:, order].contiguous()
+            narrow = idx[:, :2].contiguous(), w[:, :2].contiguous()
+            long = torch.cat([idx, none[:7, :3]]), torch.cat([w, zero[:7, :3]])
+            for got in (vc.low_latency_combine([y], [wide[0]], [wide[1]], [h])[0][0], vc.low_latency_combine([y], [narrow[0]], [narrow[1]], [h])[0][0]):
+                assert torch.equal(got, want)  # two products: one order of summation
+            got = vc.low_latency_combine([y], [long[0]], [long[1]], [h])[0][0]
+            assert torch.equal(got[:T], want) and not got[T:].any()
+        vc.buffers[0].check_status(sync=True)
+    finally:
+        vc.destroy()
