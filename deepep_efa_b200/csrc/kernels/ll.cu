@@ -1010,7 +1010,9 @@ __global__ void __launch_bounds__(kLLThreads, 2) combine_lone(const __grid_const
             if (e64 >= 0 && e64 < E && !masked) e = (int)e64;
             if (e >= 0 && row >= 0 && row < N) slot = e * N + row;
         }
-        int info = t;
+        // the row is the token's if it is one of this call (behind the count lie those of earlier calls) and came from the token
+        int info = t, rows = N;
+        if (kFind && e >= 0) rows = min((int)(__ldcg(a.layout_range + e) & 0xffffffff), N);
         if (kFind && slot >= 0) info = __ldcg(a.src_info + slot);
         float acc[8];
         for (bool sure = !kFind;; sure = true) {
@@ -1039,11 +1041,10 @@ __global__ void __launch_bounds__(kLLThreads, 2) combine_lone(const __grid_const
             }
             if (early) pdl_wait_predecessor();  // from here on everything is final; returns at once from the second token on
             if (sure) break;
-            const bool wrong = e >= 0 && (slot < 0 || info != t);
+            const bool wrong = e >= 0 && (slot < 0 || info != t || slot - e * N >= rows);
             if (!__any_sync(0xffffffffu, wrong)) break;
             if (wrong) {
                 slot = -1;
-                const int rows = min((int)(a.layout_range[e] & 0xffffffff), N);
                 for (int n = 0; n < rows && slot < 0; ++n)
                     if (__ldcg(a.src_info + (size_t)e * N + n) == t) slot = e * N + n;
             }

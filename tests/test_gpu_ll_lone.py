@@ -249,3 +249,25 @@ def test_combine_with_other_columns_than_the_dispatch():
         vc.buffers[0].check_status(sync=True)
     finally:
         vc.destroy()
+
+
+def test_combine_in_another_order_ignores_rows_of_earlier_calls():
+    """Behind an expert's rows lie those of earlier calls, with their source tokens. Selections in another order than at the dispatch name such
+    a row here, once from the very token."""
+    T, H, E = 8, 256, 2
+    vc = _cluster(T, H, E)
+    try:
+        x, y = make_tokens(T, H, "cuda"), torch.randn(E, T, H, device="cuda").to(torch.bfloat16)
+        everything = torch.tensor([[0, 1]] * T, device="cuda")
+        one = torch.tensor([[0, 1 if t == 5 else -1] for t in range(T)], device="cuda")
+        w = torch.rand(T, 2, device="cuda") + 0.5
+        for _ in range(2):  # both parities
+            vc.low_latency_dispatch([x], [everything], T, E)
+        for _ in range(2):
+            h = vc.low_latency_dispatch([x], [one], T, E)[0][2]
+            got = vc.low_latency_combine([y], [one.flip(1).contiguous()], [w.flip(1).contiguous()], [h])[0][0]
+            want = _sums(y, one, w)
+            assert (got.float() - want).norm() <= 4e-3 * want.norm()
+        vc.buffers[0].check_status(sync=True)
+    finally:
+        vc.destroy()
