@@ -1047,6 +1047,7 @@ __global__ void __launch_bounds__(kLLThreads, 2) combine_lone(const __grid_const
                 slot = -1;
                 for (int n = 0; n < rows && slot < 0; ++n)
                     if (__ldcg(a.src_info + (size_t)e * N + n) == t) slot = e * N + n;
+                if (slot < 0) report(c.status, kTimeoutCombineData, 0, 0, 0);  // the token was never sent there: no row will come
             }
         }
         if (col < n16) {

@@ -271,3 +271,27 @@ def test_combine_in_another_order_ignores_rows_of_earlier_calls():
         vc.buffers[0].check_status(sync=True)
     finally:
         vc.destroy()
+
+
+def test_combine_of_a_selection_that_was_not_dispatched_is_reported():
+    """The staged form waits for a row that nobody sends and ends in a status; the rows that are there still come."""
+    from deepep_efa_b200 import EPTimeoutError
+    T, H, E, K = 12, 512, 8, 2
+    vc = _cluster(T, H, E)
+    try:
+        buf = vc.buffers[0]
+        idx, w = make_routing(T, E, K, "cuda", seed=5)
+        y = torch.randn(E, T, H, device="cuda").to(torch.bfloat16)
+        h = vc.low_latency_dispatch([make_tokens(T, H, "cuda")], [idx], T, E)[0][2]
+        want = vc.low_latency_combine([y], [idx], [w], [h])[0][0]
+        other = idx.clone()
+        other[3, 1] = next(e for e in range(E) if e not in idx[3].tolist())
+        got = vc.low_latency_combine([y], [other], [w], [h])[0][0]
+        with pytest.raises(EPTimeoutError):
+            buf.check_status(sync=True)
+        keep = torch.arange(T, device="cuda") != 3
+        assert torch.equal(got[keep], want[keep])
+        buf.recover()
+        buf.check_status(sync=True)
+    finally:
+        vc.destroy()
