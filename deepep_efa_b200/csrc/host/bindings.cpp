@@ -707,6 +707,11 @@ void fill_ll_combine(dx::LLCombineArgs& a, Runtime* rt, const torch::Tensor& x, 
     DX_CHECK(src_info.scalar_type() == torch::kInt32 && src_info.is_contiguous() && src_info.numel() == (int64_t)L * R * num_max_tokens, "src_info must be int32 [L,N]");
     DX_CHECK(range.scalar_type() == torch::kInt64 && range.is_contiguous() && range.numel() == (int64_t)L * R, "layout_range must be int64 [L,R]");
     DX_CHECK(out.scalar_type() == torch::kBFloat16 && out.is_contiguous() && out.size(0) == T && out.size(1) == H, "out must be bf16 [T,hidden]");
+    // A result that overwrites expert outputs: the staged form has copied every row before it stores one. (With peers the forms are
+    // different protocols, which a rank cannot choose by itself.)
+    const char *x0 = static_cast<const char*>(x.data_ptr()), *out0 = static_cast<const char*>(out.data_ptr());
+    a.in_place = R == 1 && out0 < x0 + x.nbytes() && out0 + out.nbytes() > x0 ? 1 : 0;
+    if (a.in_place) pull = close_barrier = false;
     dxh::LowLatencyLayout lay(rt->core->ll_base(), num_max_tokens, H, R, num_experts);
     DX_CHECK(lay.total_bytes <= rt->core->ll_bytes(), "low-latency region too small");
     a.ctx = rt->core->ctx();

@@ -245,6 +245,7 @@ struct LLCombineArgs {
     const int* send_row;
     int close_barrier;            // pull form: readers report back before the kernel ends (x is a caller-owned tensor)
     int settled;                  // pull form: neither the dispatch nor a combine behind it writes x, so x was final before the dispatch began
+    int in_place;                 // out lies in x: only the staged form may run
 };
 cudaError_t launch_ll_combine(const LLCombineArgs* a, int num_virtual, cudaStream_t stream);
 

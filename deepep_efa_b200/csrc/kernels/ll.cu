@@ -1066,7 +1066,7 @@ __global__ void __launch_bounds__(kLLThreads, 2) combine_lone(const __grid_const
 }  // namespace ll
 
 cudaError_t launch_ll_combine(const LLCombineArgs* a, int nv, cudaStream_t stream) {
-    if (nv == 1 && a->ctx.num_ranks == 1 && a->phases == 3 && a->send_row != nullptr) {
+    if (nv == 1 && a->ctx.num_ranks == 1 && a->phases == 3 && a->send_row != nullptr && !a->in_place) {
         if (a->num_tokens == 0 || a->hidden == 0) return cudaSuccess;
         // one column per thread in CTAs of 128 threads; a bounded grid takes as wide ones as there are
         const bool bounded = a->num_sms < kNumSms;

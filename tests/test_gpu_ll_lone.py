@@ -295,3 +295,23 @@ def test_combine_of_a_selection_that_was_not_dispatched_is_reported():
         buf.check_status(sync=True)
     finally:
         vc.destroy()
+
+
+@pytest.mark.parametrize("memory", ["ordinary", "symmetric"])
+def test_combine_into_its_own_input(memory):
+    """The result in the place of expert outputs that other tokens still need."""
+    T, H, E, K = 128, 4096, 8, 4
+    vc = _cluster(T, H, E, arena=(2 << 20) + E * T * H * 2)
+    try:
+        buf = vc.buffers[0]
+        y = buf.empty_symmetric([E, T, H], torch.bfloat16) if memory == "symmetric" else torch.empty(E, T, H, dtype=torch.bfloat16, device="cuda")
+        for i in range(4):
+            idx, w = make_routing(T, E, K, "cuda", seed=i)
+            y.copy_(torch.randn(E, T, H, device="cuda"))
+            h = vc.low_latency_dispatch([make_tokens(T, H, "cuda", seed=i)], [idx], T, E)[0][2]
+            want = _sums(y, idx, w)
+            vc.low_latency_combine([y], [idx], [w], [h], outs=[y[i]])
+            assert (y[i].float() - want).norm() <= 4e-3 * want.norm()
+        buf.check_status(sync=True)
+    finally:
+        vc.destroy()
