@@ -552,7 +552,8 @@ __global__ void __launch_bounds__(kLLThreads) dispatch_lone(const __grid_constan
 cudaError_t launch_ll_dispatch(const LLDispatchArgs* a, int nv, cudaStream_t stream) {
     int max_tokens = 0;
     for (int v = 0; v < nv; ++v) max_tokens = std::max(max_tokens, a[v].num_tokens);
-    if (nv == 1 && a->ctx.num_ranks == 1 && a->phases == 3 && a->hidden > 0 && a->num_tokens * a->num_topk <= kLoneMaxSelections && a->num_experts <= kLoneMaxExperts) {
+    // (the lone kernels wait for nothing; a caller who asks how long the waits take gets the general one's)
+    if (nv == 1 && a->ctx.num_ranks == 1 && a->phases == 3 && a->wait_cost_stats == nullptr && a->hidden > 0 && a->num_tokens * a->num_topk <= kLoneMaxSelections && a->num_experts <= kLoneMaxExperts) {
         int slices = (a->hidden + kLLThreads * 16 - 1) / (kLLThreads * 16);
         int grid = a->num_tokens * slices + 1;
         if (a->num_sms >= kNumSms) {
@@ -1066,7 +1067,7 @@ __global__ void __launch_bounds__(kLLThreads, 2) combine_lone(const __grid_const
 }  // namespace ll
 
 cudaError_t launch_ll_combine(const LLCombineArgs* a, int nv, cudaStream_t stream) {
-    if (nv == 1 && a->ctx.num_ranks == 1 && a->phases == 3 && a->send_row != nullptr && !a->in_place) {
+    if (nv == 1 && a->ctx.num_ranks == 1 && a->phases == 3 && a->send_row != nullptr && !a->in_place && a->wait_cost_stats == nullptr) {
         if (a->num_tokens == 0 || a->hidden == 0) return cudaSuccess;
         // one column per thread in CTAs of 128 threads; a bounded grid takes as wide ones as there are
         const bool bounded = a->num_sms < kNumSms;

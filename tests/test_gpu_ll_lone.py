@@ -315,3 +315,33 @@ def test_combine_into_its_own_input(memory):
         buf.check_status(sync=True)
     finally:
         vc.destroy()
+
+
+@pytest.mark.parametrize("symmetric", [False, True])
+def test_wait_statistics_of_a_lone_rank(symmetric):
+    """A lone rank that asks for the time it waits gets it (for its own signals), and the same results."""
+    from deepep_efa_b200 import Buffer
+    T, H, E, K = 64, 2048, 16, 4
+
+    class Solo:
+        Get_rank, Get_size, allgather = (lambda self: 0), (lambda self: 1), (lambda self, obj: [obj])
+
+    buf = Buffer(None, (2 << 20) + E * T * H * 2, Buffer.get_low_latency_rdma_size_hint(T, H, 1, E), low_latency_mode=True, explicitly_destroy=True, comm=Solo())
+    try:
+        idx, w = make_routing(T, E, K, "cuda", seed=1, masked_fraction=0.05)
+        x, y = make_tokens(T, H, "cuda"), torch.randn(E, T, H, device="cuda").to(torch.bfloat16)
+        if symmetric:
+            y = buf.empty_symmetric([E, T, H], torch.bfloat16).copy_(y)
+        h = buf.low_latency_dispatch(x, idx, T, E)[2]
+        want = buf.low_latency_combine(y, idx, w, h)[0]
+        waits = [torch.zeros(1, dtype=torch.int64, device="cuda") for _ in range(2)]
+        before = [0, 0]
+        for _ in range(3):
+            recv, _, h, _, _ = buf.low_latency_dispatch(x, idx, T, E, dispatch_wait_recv_cost_stats=waits[0])
+            assert torch.equal(buf.low_latency_combine(y, idx, w, h, combine_wait_recv_cost_stats=waits[1])[0], want)
+            now = [t.item() for t in waits]
+            assert all(n > b for n, b in zip(now, before))
+            before = now
+        buf.check_status(sync=True)
+    finally:
+        buf.destroy()
