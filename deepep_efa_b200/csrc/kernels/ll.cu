@@ -798,7 +798,7 @@ __global__ void __launch_bounds__(kLLThreads, 1) combine_pull(const __grid_const
     // no memory that a dispatch writes (`settled`; the received rows themselves are, and a row number says nothing about them): the
     // expert outputs were then final before the dispatch began, and the row numbers it needs are written early by the dispatch's
     // token CTAs, each word tagged with the call it belongs to. So a CTA that finds its dispatch still in flight (started, not
-    // yet committed) does its work first and waits for the predecessor only before it exits, which keeps the stream's order of
+    // yet committed) gathers first and waits for the predecessor only before it stores, which keeps the stream's order of
     // completion. In every other case (dispatch already complete: an expert GEMM ran in between, or the launch is an ordinary
     // one) the wait comes first, as for any dependent kernel. A stale read of either word can only choose the second way.
     __shared__ int s_early;
@@ -927,6 +927,8 @@ __global__ void __launch_bounds__(kLLThreads, 1) combine_pull(const __grid_const
                             }
                         }
                     }
+                    // Only reads happen early: the result may lie in a block that the dispatch still reads (freed by the caller in between).
+                    if (early) pdl_wait_predecessor();  // returns at once from the second time on
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {
                         const int i = h == 0 ? ia : ib;

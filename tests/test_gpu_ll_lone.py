@@ -345,3 +345,34 @@ def test_wait_statistics_of_a_lone_rank(symmetric):
         buf.check_status(sync=True)
     finally:
         buf.destroy()
+
+
+def test_pull_combine_stores_behind_its_dispatch():
+    """The general kernels right behind each other, more tokens than SMs, and a result in the block that held the dispatch's input: every row
+    still leaves as it was."""
+    from deepep_efa_b200 import Buffer
+    T, H, E, K = 400, 2048, 32, 4
+
+    class Solo:
+        Get_rank, Get_size, allgather = (lambda self: 0), (lambda self: 1), (lambda self, obj: [obj])
+
+    buf = Buffer(None, (2 << 20) + E * T * H * 2, Buffer.get_low_latency_rdma_size_hint(T, H, 1, E), low_latency_mode=True, explicitly_destroy=True, comm=Solo())
+    try:
+        y = buf.empty_symmetric([E, T, H], torch.bfloat16)
+        y.copy_(torch.randn(E, T, H, device="cuda"))
+        idx, w = make_routing(T, E, K, "cuda", seed=2)
+        want, waits = _sums(y, idx, w), torch.zeros(1, dtype=torch.int64, device="cuda")
+        data = make_tokens(T, H, "cuda")
+        for i in range(6):
+            x = data.roll(i, 0)
+            torch.cuda.synchronize()
+            recv, _, h, _, _ = buf.low_latency_dispatch(x, idx, T, E, use_fp8=False, dispatch_wait_recv_cost_stats=waits)
+            del x
+            out = buf.low_latency_combine(y, idx, w, h, combine_wait_recv_cost_stats=waits)[0]
+            rows, x = {}, data.roll(i, 0)
+            at = torch.tensor([[rows.setdefault(e, []).append(t) or len(rows[e]) - 1 for e in es] for t, es in enumerate(idx.tolist())], device="cuda")
+            assert torch.equal(recv[idx.view(-1), at.view(-1)].view(T, K, H), x[:, None].expand(T, K, H))
+            assert (out.float() - want).norm() <= 4e-3 * want.norm()
+        buf.check_status(sync=True)
+    finally:
+        buf.destroy()
