@@ -412,7 +412,9 @@ def run_ours(args):
         stamps = {"rank0": allst[0], f"rank{world - 1}": allst[-1],
                   "legend": {"ll_dispatch_first_cta": "start, idx loaded, counts of lower ranks, rows known, rows stored, release done, exit",
                              "ll_dispatch_last_cta": "start, -, counts sent, all counts, layout out, all rows in, exit",
-                             "ll_combine (pull)": "start, offset posted, -, -, peers' offsets known, rows reduced, exit"}}
+                             "ll_combine (pull)": "start, offset posted, -, -, peers' offsets known, rows reduced, exit",
+                             "one rank": "dispatch: start, -, -, rows known (first only), rows stored (first) or layout out (last), -, exit; "
+                                         "combine: start, -, -, -, places of the rows known, rows reduced, exit"}}
 
     # the same pair with the expert outputs in the zero-copy combine buffer (where the decode path's last GEMM writes them):
     # pulled like the symmetric tensor, without the closing "readers done" round a caller-owned tensor needs

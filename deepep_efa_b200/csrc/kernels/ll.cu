@@ -411,7 +411,7 @@ __global__ void __launch_bounds__(kLLThreads, 1) dispatch(const __grid_constant_
 // Sequence numbers, the started word and the tags of send_row are those of the kernel above, so calls of either kind follow each other
 // in any order; the sequence number advances when the last CTA has read it.
 template <bool kFp8>
-__global__ void __launch_bounds__(kLLThreads) dispatch_lone(const __grid_constant__ LLDispatchArgs a, const int slices) {
+__global__ void __launch_bounds__(kLLThreads, 2) dispatch_lone(const __grid_constant__ LLDispatchArgs a, const int slices) {
     pdl_wait_predecessor();
     const RankCtx& c = a.ctx;
     const int T = a.num_tokens, K = a.num_topk, E = a.num_experts, H = a.hidden, P = a.parity, N = a.num_max_tokens;
@@ -452,6 +452,7 @@ __global__ void __launch_bounds__(kLLThreads) dispatch_lone(const __grid_constan
             a.layout_range[e] = n;
             if (a.cumulative_stats != nullptr) a.cumulative_stats[e] += n;
         }
+        trace_stamp(c, kFamLLDispatch, 1, 4);
         trace_stamp(c, kFamLLDispatch, 1, 6);
     } else {
         const bool pow2 = a.round_scale != 0 || a.use_ue8m0 != 0;
@@ -516,6 +517,7 @@ __global__ void __launch_bounds__(kLLThreads) dispatch_lone(const __grid_constan
                 if (row >= 0) c.at<int>(0, a.region.recv_src_info_off[P])[(size_t)e * N + row] = t;
                 if (a.send_row != nullptr) a.send_row[t * K + lane] = (ll_count_tag(seq) << 16) | (row + 1);
             }
+            if (blockIdx.x == 1) trace_stamp(c, kFamLLDispatch, 0, 3);
             const int slot_of = row >= 0 ? e * N + row : -1;
 #pragma unroll 4
             for (int k = 0; k < K; ++k) {
@@ -536,6 +538,7 @@ __global__ void __launch_bounds__(kLLThreads) dispatch_lone(const __grid_constan
             }
             if (item + (int)gridDim.x - 1 < T * slices) __syncthreads();  // s_part is reused
         }
+        if (blockIdx.x == 1) trace_stamp(c, kFamLLDispatch, 0, 4);
         if (blockIdx.x == 1) trace_stamp(c, kFamLLDispatch, 0, 6);
     }
     if (tid == 0) {
@@ -1013,6 +1016,7 @@ __global__ void __launch_bounds__(kLLThreads, 2) combine_lone(const __grid_const
             if (e64 >= 0 && e64 < E && !masked) e = (int)e64;
             if (e >= 0 && row >= 0 && row < N) slot = e * N + row;
         }
+        if (traced) trace_stamp(c, kFamLLCombine, tslot, 4);
         // the row is the token's if it is one of this call (behind the count lie those of earlier calls) and came from the token
         int info = t, rows = N;
         if (kFind && e >= 0) rows = min((int)(__ldcg(a.layout_range + e) & 0xffffffff), N);
@@ -1062,8 +1066,9 @@ __global__ void __launch_bounds__(kLLThreads, 2) combine_lone(const __grid_const
             st_stream(reinterpret_cast<int4*>(a.out) + (size_t)t * n16 + col, o);
         }
     }
-    if (traced) trace_stamp(c, kFamLLCombine, tslot, 6);
+    if (traced) trace_stamp(c, kFamLLCombine, tslot, 5);
     if (early) pdl_wait_predecessor();  // also without an item: this kernel may not complete before its predecessor has
+    if (traced) trace_stamp(c, kFamLLCombine, tslot, 6);
 }
 
 }  // namespace ll

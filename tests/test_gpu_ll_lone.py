@@ -376,3 +376,24 @@ def test_pull_combine_stores_behind_its_dispatch():
         buf.check_status(sync=True)
     finally:
         buf.destroy()
+
+
+def test_phase_stamps_of_a_lone_rank():
+    T, H, E, K = 32, 2048, 16, 4
+    vc = _cluster(T, H, E, arena=(2 << 20) + E * T * H * 2)
+    try:
+        buf = vc.buffers[0]
+        idx, w = make_routing(T, E, K, "cuda", seed=2)
+        y = buf.empty_symmetric([E, T, H], torch.bfloat16)
+        buf.runtime.enable_trace(True)
+        h = vc.low_latency_dispatch([make_tokens(T, H, "cuda")], [idx], T, E)[0][2]
+        vc.low_latency_combine([y], [idx], [w], [h])
+        torch.cuda.synchronize()
+        trace = buf.runtime.read_trace()
+        buf.runtime.enable_trace(False)
+        # the two low-latency families, first and last CTA of each: the phases that a kernel without signalling has, in order
+        for slot, phases in ((8, (0, 3, 4, 6)), (9, (0, 4, 6)), (10, (0, 4, 5, 6)), (11, (0, 4, 5, 6))):
+            at = [trace[slot * 16 + p] for p in phases]
+            assert all(at) and at == sorted(at)
+    finally:
+        vc.destroy()
