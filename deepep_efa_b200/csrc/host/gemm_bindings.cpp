@@ -187,14 +187,14 @@ torch::Tensor grouped_gemm(const torch::Tensor& a, const torch::Tensor& b, const
     }
     // The caller says that groups have few rows, and how many a tile may have (1: the ordinary choice). The natively block-scaled 256-column
     // tiles have the form with the weights as M; SwiGLU then quantises its output.
-    const bool columns = tokens_as_columns != 0 && p.m_ends != nullptr && p.sfa_atoms != nullptr && p.mx_wide && p.n % 256 == 0 && (!swiglu || out_fp8.has_value());
+    const bool columns = tokens_as_columns != 0 && p.m_ends != nullptr && fp8 && sfa_atoms.has_value() && p.mx_wide && p.n % 256 == 0 && (!swiglu || out_fp8.has_value());
     if (columns) {
         p.token_cap = tokens_as_columns == 1 ? 128 : tokens_as_columns;
         DXG_CHECK(p.token_cap >= 64 && p.token_cap <= 224 && p.token_cap % 32 == 0, "tokens_as_columns must be 0, 1 or a multiple of 32 from 64 to 224");
     }
     if (out_fp8.has_value() || out_atoms.has_value()) {
         DXG_CHECK(out_fp8.has_value() && out_atoms.has_value() && same_dev(out_fp8) && same_dev(out_atoms), "out_fp8 and out_atoms go together, on A's device");
-        DXG_CHECK(mode == 0 && swiglu && p.sfa_atoms != nullptr && p.mx_wide == 1, "quantised output needs the natively block-scaled kernel with wide SwiGLU tiles");
+        DXG_CHECK(mode == 0 && swiglu && sfa_atoms.has_value() && p.mx_wide == 1, "quantised output needs the natively block-scaled kernel with wide SwiGLU tiles");
         const int64_t inter = p.n / 2;
         DXG_CHECK(out_fp8->element_size() == 1 && out_fp8->is_contiguous() && out_fp8->numel() == (int64_t)p.m_total * inter, "out_fp8 must be e4m3 [M, N/2]");
         DXG_CHECK(out_atoms->element_size() == 1 && out_atoms->is_contiguous() && out_atoms->numel() >= (((int64_t)p.m_total + 127) / 128) * (inter / 128) * 512,

@@ -557,11 +557,10 @@ cudaError_t launch_cols_impl(const GroupedGemmArgs& a, cudaStream_t stream) {
 }  // namespace
 
 cudaError_t launch_token_cols_gemm(const GroupedGemmArgs& a, cudaStream_t stream) {
-    if (a.num_groups < 1 || a.num_groups > kMaxGroups || a.num_sms < 1 || a.mode != 0 || !a.fp8 || a.sfa_atoms == nullptr || a.sfb_atoms == nullptr)
-        return cudaErrorInvalidValue;
+    if (a.num_groups < 1 || a.num_groups > kMaxGroups || a.num_sms < 1 || a.mode != 0 || !a.fp8) return cudaErrorInvalidValue;
     if (a.token_cap < 64 || a.token_cap > kMaxTokenCap || a.token_cap % 32 != 0 || a.k % 128 != 0 || a.k <= 0 || a.n % kWeightRows != 0) return cudaErrorInvalidValue;
-    if (a.swiglu && (a.c_fp8 == nullptr || a.c_atoms == nullptr)) return cudaErrorInvalidValue;
-    if (a.m_total <= 0) return cudaSuccess;
+    if (a.m_total <= 0) return cudaSuccess;  // (tensors without rows have no address)
+    if (a.sfa_atoms == nullptr || a.sfb_atoms == nullptr || (a.swiglu && (a.c_fp8 == nullptr || a.c_atoms == nullptr))) return cudaErrorInvalidValue;
     return a.swiglu ? launch_cols_impl<true>(a, stream) : launch_cols_impl<false>(a, stream);
 }
 

@@ -117,3 +117,24 @@ def test_moe_low_latency_decode_path():
             assert _rel(y, ref) < 8e-2, _rel(y, ref)
     finally:
         vc.destroy()
+
+
+@pytest.mark.parametrize("native", [False, True])
+@pytest.mark.parametrize("path", ["forward_fp8", "forward_fused"])
+def test_fp8_forward_of_a_rank_without_rows(native, path):
+    """Nobody selects an expert of this rank: an empty product per expert, and zeros."""
+    import deepep_efa_b200 as ep
+    from deepep_efa_b200.models.moe import MoEConfig, MoELayer
+    from deepep_efa_b200.parallel.virtual import VirtualCluster
+    vc = VirtualCluster(1, num_nvl_bytes=64 << 20)
+    try:
+        layer = MoELayer(MoEConfig(hidden=512, intermediate=256, num_experts=8, num_topk=2), vc.buffers[0])
+        layer.prepare_fp8(native_block_scaling=native)
+        x, idx, w = make_tokens(5, 512, "cuda"), torch.full((5, 2), -1, device="cuda"), torch.ones(5, 2, device="cuda")
+        y = getattr(layer, path)(x, idx, w)
+        torch.cuda.synchronize()
+        vc.buffers[0].check_status()
+        assert ep._ext.load().gemm_error(0) == 0
+        assert y.shape == x.shape and not y.any()
+    finally:
+        vc.destroy()
