@@ -474,9 +474,14 @@ def fused_forward_many(layers, xs, idxs, ws, overlap: bool = True, num_dispatch_
         ga = min(L, max(1, int(round(L * SPLIT_FRACTION)))) if overlapped else L
         if native:
             columns = _token_columns(R_ * w.num_tokens * K / E)
-            wide = R_ * w.num_tokens * K >= WIDE_TILE_MIN_ROWS_PER_EXPERT * E or columns != 0
+            wide2 = R_ * w.num_tokens * K >= WIDE_TILE_MIN_ROWS_PER_EXPERT * E
+            wide = wide2 or columns != 0
             sfb = l._mx[0 if wide else 2]
             fuse_cast = wide and FUSE_CAST_INTO_GEMM1
+            # as columns a row leaves in pieces of 64 bytes: fine for this GPU's memory, too short for NVLink. With peers the second GEMM
+            # takes tokens as rows, few of them in narrow tiles, whose scatter stores whole rows.
+            columns2 = columns if R_ == 1 else 0
+            wide2 = wide2 or columns2 != 0
         # (first group, number of groups, SMs): the early experts next to the dispatch, the rest on the whole GPU
         parts = [(0, ga, 148 - RESERVED_SMS), (ga, L - ga, 0)] if (overlapped and ga < L) else [(0, L, (148 - RESERVED_SMS) if overlapped else 0)]
         for pi, (g0, ng, sms1) in enumerate(parts):
@@ -501,10 +506,8 @@ def fused_forward_many(layers, xs, idxs, ws, overlap: bool = True, num_dispatch_
         if native:
             if not fuse_cast:
                 C.per_token_cast_to_fp8(w.h, True, False, None, 1, w.hq, w.hs, w.m_offsets[L:], True)
-            C.grouped_gemm(w.hq, w2, w.m_offsets, 0, False, None, None, None, 0, GEMM_TIMEOUT_MS, w.m_ends, w.hs, l._mx[3 if wide else 1],
-                           row_info=w.recv_info, scatter_bases=w.peer_bases[3 * R_:], sched=w.sched, early_table=True,
-                           # (as columns a row leaves in pieces of 64 bytes: fine for this GPU's memory, too short for NVLink)
-                           tokens_as_columns=columns if R_ == 1 else 0)
+            C.grouped_gemm(w.hq, w2, w.m_offsets, 0, False, None, None, None, 0, GEMM_TIMEOUT_MS, w.m_ends, w.hs, l._mx[3 if wide2 else 1],
+                           row_info=w.recv_info, scatter_bases=w.peer_bases[3 * R_:], sched=w.sched, early_table=True, tokens_as_columns=columns2)
         else:
             C.per_token_cast_to_fp8(w.h, False, False, None, 1, w.hq, w.hs, w.m_offsets[L:], False)
             C.grouped_gemm(w.hq, w2, w.m_offsets, 0, False, w.hs, s2, None, 0, GEMM_TIMEOUT_MS, w.m_ends, None, None,

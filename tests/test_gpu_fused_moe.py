@@ -193,3 +193,53 @@ def test_lone_dispatch_places_rows_like_the_general_one(T, H, E, K, native):
         assert all(torch.equal(a, b) for a, b in zip(*got)) and (got[0][3].view(-1) >= 0).sum() == (idx >= 0).sum()
     finally:
         vc.destroy()
+
+
+@pytest.mark.parametrize("R,T", [(1, 1), (1, 30), (1, 160), (1, 300), (1, 380), (1, 500), (2, 3), (2, 100), (2, 150), (2, 190)])
+def test_fused_forward_with_tokens_as_columns(monkeypatch, R, T):
+    """0.4 to 188 rows per expert, up to 60 and from 121 on with tokens as columns, alone and with a peer, whose second GEMM takes narrow tiles
+    of rows below 64 per expert and wide ones beyond: bit for bit the layer that takes rows."""
+    import deepep_efa_b200 as ep
+    from deepep_efa_b200.models import moe as moe_mod
+    H, I, E, K = 512, 384, 8, 3
+    vc, layers, xs, idxs, ws = _setup(R, T, H, I, E, K, True, seed=T)
+    calls = []
+
+    class Spy:
+        def __getattr__(self, name):
+            return getattr(ep._ext.load(), name)
+
+        def grouped_gemm(self, *args, **kw):
+            calls.append((args[4], args[12], kw.get("tokens_as_columns", 0)))
+            return ep._ext.load().grouped_gemm(*args, **kw)
+
+    monkeypatch.setattr(moe_mod.MoELayer, "_C", staticmethod(lambda: Spy()))
+    try:
+        def run():
+            outs = moe_mod.fused_forward_many(layers, xs, idxs, ws)
+            torch.cuda.synchronize()
+            for b in vc.buffers:
+                b.check_status(sync=True)
+            assert ep._ext.load().gemm_error(0) == 0
+            return outs
+
+        got = run()
+        rows = R * T * K / E
+        columns = moe_mod._token_columns(rows)
+        assert (columns != 0) == (rows <= 60 or 120 < rows <= 200)
+        for swiglu, atoms, given in calls:
+            if swiglu:
+                assert given == columns
+            else:
+                assert given == (columns if R == 1 else 0)
+                narrow = rows < moe_mod.WIDE_TILE_MIN_ROWS_PER_EXPERT and (R > 1 or not columns)
+                assert any(atoms is l._mx[1 if narrow else 3] for l in layers)
+        monkeypatch.setattr(moe_mod, "_token_columns", lambda rows: 0)
+        for a, b in zip(got, run()):
+            assert torch.equal(a, b) and a.any()
+        w13_all, w2_all = (torch.cat([getattr(l, n).detach().float() for l in layers]) for n in ("w13", "w2"))
+        for r in range(R):
+            ref = moe_mod.dense_reference(xs[r], idxs[r], ws[r].masked_fill(idxs[r] == -1, 0), w13_all, w2_all)
+            assert _rel(got[r], ref) < 8e-2  # as in the test of the whole pipeline above
+    finally:
+        vc.destroy()
