@@ -607,3 +607,81 @@ def test_tile_counter_after_a_launch_that_gave_up(kind):
         torch.cuda.synchronize()
         assert C.gemm_error(0) == 0 and sched.tolist() == [0, 0]
         assert torch.equal(got[live], want[live])
+
+
+@pytest.mark.parametrize("scatter", [False, True])
+def test_token_columns_tile_of_96(scatter):
+    """The one tile that is longer than the step of a cut group without being whole scale atoms."""
+    test_token_columns_tile_sizes(96, scatter)
+
+
+def _columns_case(counts, stride, K, I):
+    """Both natively block-scaled products of an expert layer, as functions of the launch's options, on groups of `stride` rows of which
+    `counts` count."""
+    from deepep_efa_b200 import _ext
+    from deepep_efa_b200.ops.grouped_gemm import build_sf_atoms_a, build_sf_atoms_b
+    C, G = _ext.load(), len(counts)
+    cnt = torch.tensor(counts, device="cuda", dtype=torch.int32)
+    starts = torch.arange(G + 1, device="cuda", dtype=torch.int32) * stride
+    a, a_s = C.per_token_cast_to_fp8(torch.randn(G * stride, K, device="cuda").to(torch.bfloat16), True, False)
+    b = torch.randn(G, 2 * I, K, device="cuda").to(torch.float8_e4m3fn)
+    b_s = torch.exp2(torch.randint(-8, -4, (G, 2 * I // 128, K // 128), device="cuda").float())
+    sfa, sfb, sfb_swiglu = build_sf_atoms_a(a_s), build_sf_atoms_b(b_s, 2 * I, False, True), build_sf_atoms_b(b_s, 2 * I, True, True)
+
+    def run(swiglu, timeout_ms=2000.0, sms=0, **how):
+        if not swiglu:
+            out = torch.zeros(G * stride, 2 * I, device="cuda", dtype=torch.bfloat16)
+            C.grouped_gemm(a, b, starts, 0, False, None, None, out, sms, timeout_ms, cnt, sfa, sfb, m_ends_are_counts=True, **how)
+            return (out,)
+        q, qs = torch.zeros(G * stride, I, dtype=torch.uint8, device="cuda"), torch.zeros(G * stride // 128, I // 128, 512, dtype=torch.uint8, device="cuda")
+        C.grouped_gemm(a, b, starts, 0, True, None, None, None, sms, timeout_ms, cnt, sfa, sfb_swiglu, out_fp8=q.view(torch.float8_e4m3fn), out_atoms=qs,
+                       m_ends_are_counts=True, **how)
+        return q, qs
+
+    return C, run
+
+
+@pytest.mark.parametrize("swiglu", [False, True])
+@pytest.mark.parametrize("cap", [64, 160])
+def test_token_columns_behind_an_arrival_gate(swiglu, cap):
+    """Gates that are open, and one that nobody opens: an error after the limit, the tile counter zero again, and the next launch right."""
+    torch.manual_seed(cap)
+    C, run = _columns_case([200, 0, 33, 128, 1], 256, 512, 256)
+    C.gemm_clear_error(0)
+    want = run(swiglu)
+    sched = torch.zeros(2, dtype=torch.int32, device="cuda")
+    expected = torch.tensor([3, 0, 1, 7, 2], dtype=torch.int64, device="cuda")
+    shut = expected.clone()
+    shut[3] -= 1
+
+    def check(got):
+        torch.cuda.synchronize()
+        assert C.gemm_error(0) == 0 and sched.tolist() == [0, 0]
+        assert all(torch.equal(g, w) for g, w in zip(got, want))
+
+    for _ in range(2):
+        check(run(swiglu, sched=sched, ready=expected, expected=expected, tokens_as_columns=cap))
+        run(swiglu, timeout_ms=20.0, sched=sched, ready=shut, expected=expected, tokens_as_columns=cap)
+        torch.cuda.synchronize()
+        assert C.gemm_error(0) == 1 and sched.tolist() == [0, 0]
+        C.gemm_clear_error(0)
+        for early in (False, True):
+            check(run(swiglu, sched=sched, early_table=early, tokens_as_columns=cap))
+
+
+def test_token_columns_hold_their_successor():
+    """On four SMs with tokens as columns: the kernel behind it, which would fit on the others, begins when it has ended."""
+    torch.manual_seed(31)
+    C, run = _columns_case([128] * 64, 128, 2048, 512)
+    C.gemm_clear_error(0)
+    small = torch.randn(148 * 128, 256, device="cuda").to(torch.bfloat16)
+    small_w = torch.randn(1, 256, 256, device="cuda").to(torch.bfloat16)
+    offs, out = _offsets([148 * 128]), torch.empty(148 * 128, 256, dtype=torch.bfloat16, device="cuda")
+    stamps = [torch.tensor([torch.iinfo(torch.int64).max, 0, 0, 0], dtype=torch.int64, device="cuda") for _ in range(2)]
+    for warm in (True, False):
+        torch.cuda.synchronize()
+        run(False, sms=4, tokens_as_columns=128, hold_successor=True, trace=None if warm else stamps[0])
+        C.grouped_gemm(small, small_w, offs, 0, False, None, None, out, 0, 2000.0, trace=None if warm else stamps[1])
+        torch.cuda.synchronize()
+    assert C.gemm_error(0) == 0
+    assert stamps[0][1].item() <= stamps[1][0].item()
