@@ -49,8 +49,6 @@ constexpr int kLLWarps = kLLThreads / 32;
 constexpr int kTicketLLDispatch = 3;
 constexpr int kTicketLLCombine = 4;
 constexpr int kNumSms = 148;
-// The kernels for a lone rank count the earlier selections of a token by looking at all of them. Up to this many (512 tokens with eight
-// experts each) that is a handful of loads per thread; longer batches keep the running histogram of the general kernel.
 constexpr int kLoneMaxSelections = 4096;
 constexpr int kLoneMaxExperts = 8192;  // their counts stay in the shared memory that needs no opt-in
 // rank-local u64 words after the family sequence numbers (RankCtx::seq + kNumFamilies):
@@ -552,24 +550,47 @@ __global__ void __launch_bounds__(kLLThreads, 2) dispatch_lone(const __grid_cons
 
 }  // namespace ll
 
+// Threads and row slices of a lone rank's dispatch.
+struct LoneShape {
+    int slices, threads;
+};
+static LoneShape lone_dispatch_shape(const LLDispatchArgs& a) {
+    int slices = (a.hidden + kLLThreads * 16 - 1) / (kLLThreads * 16);
+    // few tokens: slices of a row as small as 1024 channels, as long as every one of them has an SM for itself
+    if (a.num_sms >= kNumSms)
+        while (slices * 1024 < a.hidden && a.num_tokens * (slices + 1) < kNumSms) ++slices;
+    return {slices, ((a.hidden + 16 * slices - 1) / (16 * slices) + 31) / 32 * 32};
+}
+
+// Whether a lone rank's dispatch takes its own kernel. That one looks at all earlier selections of every token, K of them at a time in groups of
+// eight, with as many threads as a row has pieces of 16 channels; the general kernel advances one histogram per CTA, but waits for itself.
+// One B200, dispatch alone in a CUDA graph, us, general / lone. With an SM for every CTA the loads per thread of the longest scan decide, against
+// what the general kernel takes for its tokens: H 7168, K 8: T 128 12.6 / 5.9, 512 21.6 / 14.6; H 1024, K 8, BF16: T 256 (32 loads) 13.4 / 11.0, 384 (48)
+// 15.1 / 14.3, 512 (64) 17.3 / 18.0; H 512, K 8, BF16: T 128 (32) 11.1 / 10.7, 192 (48) 13.0 / 14.6, 256 (64) 13.3 / 17.9; H 1024, K 4, T 1024 (64) 24.9 / 17.6;
+// H 2048, T 128: K 16 (32) 12.8 / 9.7, K 32 (128) 14.7 / 20.0; T 48, K 32 (96) 14.6 / 16.9.
+// With fewer SMs every CTA scans once for each of its tokens: 64 SMs, BF16: T 128, K 8, H 2048 (8 loads) 13.5 / 8.9; T 256, K 8, H 1024 (32) 17.4 / 20.5; T 512, K 8,
+// H 1024 26.2 / 47.3; 4 SMs: T 128, K 8, H 2048 91.9 / 87.2, H 7168 (3) 152 / 151; T 256, K 8, H 7168 (5) 296 / 310; T 1024, K 1, H 2048 (8) 452 / 464.
+static bool lone_dispatch(const LLDispatchArgs& a) {
+    const int selections = a.num_tokens * a.num_topk;
+    if (selections > kLoneMaxSelections || a.num_experts > kLoneMaxExperts) return false;
+    if ((selections + a.num_experts) * (int)sizeof(int) > 40 * 1024) return true;  // more than the general kernel's lists may be
+    const int scans = selections * ((a.num_topk + 7) / 8);
+    const int threads = lone_dispatch_shape(a).threads;
+    if (a.num_sms >= kNumSms) return scans <= (30 + a.num_tokens / 20) * threads;
+    return scans <= 1024 && scans <= 8 * threads && a.num_tokens <= 512;
+}
+
 cudaError_t launch_ll_dispatch(const LLDispatchArgs* a, int nv, cudaStream_t stream) {
     int max_tokens = 0;
     for (int v = 0; v < nv; ++v) max_tokens = std::max(max_tokens, a[v].num_tokens);
     // (the lone kernels wait for nothing; a caller who asks how long the waits take gets the general one's)
-    if (nv == 1 && a->ctx.num_ranks == 1 && a->phases == 3 && a->wait_cost_stats == nullptr && a->hidden > 0 && a->num_tokens * a->num_topk <= kLoneMaxSelections && a->num_experts <= kLoneMaxExperts) {
-        int slices = (a->hidden + kLLThreads * 16 - 1) / (kLLThreads * 16);
-        int grid = a->num_tokens * slices + 1;
-        if (a->num_sms >= kNumSms) {
-            // few tokens: slices of a row as small as 1024 channels, as long as every one of them has an SM for itself
-            while (slices * 1024 < a->hidden && a->num_tokens * (slices + 1) < kNumSms) ++slices;
-            grid = a->num_tokens * slices + 1;
-        } else {
-            grid = std::min(grid, std::max(2, a->num_sms));
-        }
-        const int threads = ((a->hidden + 16 * slices - 1) / (16 * slices) + 31) / 32 * 32;
+    if (nv == 1 && a->ctx.num_ranks == 1 && a->phases == 3 && a->wait_cost_stats == nullptr && a->hidden > 0 && lone_dispatch(*a)) {
+        const LoneShape shape = lone_dispatch_shape(*a);
+        int grid = a->num_tokens * shape.slices + 1;
+        if (a->num_sms < kNumSms) grid = std::min(grid, std::max(2, a->num_sms));
         const size_t smem = (size_t)a->num_experts * sizeof(int);
-        return a->use_fp8 ? launch_dependent(ll::dispatch_lone<true>, dim3(grid), threads, smem, stream, *a, slices)
-                          : launch_dependent(ll::dispatch_lone<false>, dim3(grid), threads, smem, stream, *a, slices);
+        return a->use_fp8 ? launch_dependent(ll::dispatch_lone<true>, dim3(grid), shape.threads, smem, stream, *a, shape.slices)
+                          : launch_dependent(ll::dispatch_lone<false>, dim3(grid), shape.threads, smem, stream, *a, shape.slices);
     }
     const int grid = std::max(2, std::min(max_tokens + 1, a[0].num_sms));
     const size_t smem = ((size_t)a[0].num_tokens * a[0].num_topk + a[0].num_experts) * sizeof(int);

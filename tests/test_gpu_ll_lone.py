@@ -397,3 +397,11 @@ def test_phase_stamps_of_a_lone_rank():
             assert all(at) and at == sorted(at)
     finally:
         vc.destroy()
+
+
+# both sides of the lines between the two dispatch kernels: the longest lists, narrow rows, a bounded number of SMs, 32 selections per token
+@pytest.mark.parametrize("T,H,E,K,masked,sms", [(512, 2048, 32, 8, 0.0, None), (513, 2048, 32, 8, 0.1, None), (119, 512, 32, 8, 0.1, None), (192, 512, 32, 8, 0.0, None),
+                                                 (4, 1024, 64, 32, 0.2, None), (30, 2048, 64, 32, 0.2, None), (128, 2048, 16, 8, 0.1, 7), (129, 2048, 16, 8, 0.0, 7)])
+@pytest.mark.parametrize("wire", ["bf16", "fp8"])
+def test_lone_rank_around_the_lines_of_its_dispatch(T, H, E, K, masked, sms, wire):
+    test_lone_rank_matches_general_kernels(T, H, E, K, masked, sms, wire)
