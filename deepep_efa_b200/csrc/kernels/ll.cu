@@ -1094,8 +1094,18 @@ __global__ void __launch_bounds__(kLLThreads, 2) combine_lone(const __grid_const
 
 }  // namespace ll
 
+// Whether a lone rank's combine takes its own kernel. With a bounded number of SMs that one has a column per thread of one CTA per SM, the general
+// kernels two: in rows of more than 512 columns they keep more in flight, unless there is little to do. One B200, combine alone in a CUDA graph,
+// us, general / lone, outputs in ordinary and in symmetric memory, K 8: H 4096: T 128, 16 SMs 42.1 / 21.7 and 26.0 / 15.8, T 512, 4 SMs 543 / 380 and 356 / 283;
+// H 5120: T 128, 64 SMs 19.4 / 12.9 and 11.3 / 9.8, 16 SMs 45.7 / 42.6 and 26.4 / 30.7, T 512, 64 SMs 51.0 / 51.7 and 29.1 / 39.6; H 7168: T 256, 64 SMs 33.9 / 26.5 and 17.9 / 20.9,
+// 4 SMs 336 / 371 and 188 / 282; K 2, T 512, 64 SMs 33.6 / 38.9 and 24.3 / 30.9.
+static bool lone_combine(const LLCombineArgs& a) {
+    if (a.num_sms >= kNumSms || a.hidden / 8 <= kLLThreads || a.num_experts > kLoneMaxExperts) return true;  // (more experts than the general kernel's list takes)
+    return a.num_tokens <= 2 * a.num_sms;
+}
+
 cudaError_t launch_ll_combine(const LLCombineArgs* a, int nv, cudaStream_t stream) {
-    if (nv == 1 && a->ctx.num_ranks == 1 && a->phases == 3 && a->send_row != nullptr && !a->in_place && a->wait_cost_stats == nullptr) {
+    if (nv == 1 && a->ctx.num_ranks == 1 && a->phases == 3 && a->send_row != nullptr && !a->in_place && a->wait_cost_stats == nullptr && lone_combine(*a)) {
         if (a->num_tokens == 0 || a->hidden == 0) return cudaSuccess;
         // one column per thread in CTAs of 128 threads; a bounded grid takes as wide ones as there are
         const bool bounded = a->num_sms < kNumSms;

@@ -405,3 +405,9 @@ def test_phase_stamps_of_a_lone_rank():
 @pytest.mark.parametrize("wire", ["bf16", "fp8"])
 def test_lone_rank_around_the_lines_of_its_dispatch(T, H, E, K, masked, sms, wire):
     test_lone_rank_matches_general_kernels(T, H, E, K, masked, sms, wire)
+
+
+# rows of more than 512 columns on few SMs: both sides of the line between the two combine kernels, and the widest rows that have one side
+@pytest.mark.parametrize("T,H,sms", [(14, 4224, 7), (15, 4224, 7), (40, 4096, 7), (9, 7168, 4)])
+def test_lone_rank_around_the_lines_of_its_combine(T, H, sms):
+    test_lone_rank_matches_general_kernels(T, H, 16, 4, 0.1, sms, "fp8")
