@@ -220,7 +220,7 @@ class MoELayer(nn.Module):
         how = dict(m_ends=plan.m_ends, timeout_ms=GEMM_TIMEOUT_MS)
         if mx is not None:
             # padding rows of the plan carry all-zero data; whatever exponent their zero scale maps to does not matter
-            columns = _token_columns(buf.group_size * x.size(0) * self.cfg.num_topk / self.cfg.num_experts)
+            columns = _token_columns(buf.group_size * x.size(0) * self.cfg.num_topk / self.cfg.num_experts, w13.numel() + w2.numel(), self.cfg.hidden)
             a_atoms = gg.build_sf_atoms_a(a_s)
             if columns or plan.num_rows >= WIDE_TILE_MIN_ROWS_PER_EXPERT * self.num_local_experts:
                 # the first GEMM quantises its own output: a wide tile holds one whole scale block of a row
@@ -300,7 +300,7 @@ class MoELayer(nn.Module):
             ws[key] = w_
         w_ = ws[key]
         a, a_s = px.view(L * N, H), ps.view(L * N, H // 128)
-        columns = _token_columns(R * x.size(0) * cfg.num_topk / cfg.num_experts)
+        columns = _token_columns(R * x.size(0) * cfg.num_topk / cfg.num_experts, w13.numel() + w2.numel(), H)
         y = buf.get_next_low_latency_combine_buffer(handle)
         # rows per expert come as counts; both GEMMs read them where the dispatch left them
         if mx is not None:
@@ -337,11 +337,25 @@ FUSE_CAST_INTO_GEMM1 = True  # wide natively block-scaled tiles: GEMM1's epilogu
 # Skewed routing (popularity 1 / (e + 1)^1.2): 64 experts 38 rows 247 / 224, 75 rows 264 / 242, 150 rows 319 / 299, 188 rows 341 / 327; 128 experts 19 rows 973 / 927, 125
 # rows 1291 to 1354 / 1271 to 1385; 256 experts 128 rows 2825 to 3025 / 2905 to 3125.
 # A tile of 64 tokens leaves room for five stages instead of four: worth 2 % with 4 rows per expert, and lost again with 19 and skewed routing.
-def _token_columns(rows: float) -> int:
+# From 120 rows on this holds for layers whose weights are some times the 126 MB of the L2 and whose rows are long. Otherwise what the rows form pulls
+# again comes from L2 anyway, its shorter tiles spread better over the SMs, and the columns' epilogue is not covered by enough K blocks. Whole fused
+# layer, us, rows / columns, uniform and skewed: weights of 104 to 302 MB: 12 experts of 4096 -> 768, 190 rows 97 / 116 to 135, 97 / 108; 16 of 3328 -> 1408, 129 rows
+# 110 / 126; 32 of 4096 -> 768, 190 rows 168 / 185, 169 / 179; 352 MB: 8 of 7168 -> 2048, 150 rows, skewed, 159 / 171; 453 MB: 48 of 4096 -> 768, 130 to 190 rows 198
+# to 224 / 190 to 230, 205 to 238 / 196 to 235; 604 MB: 24 of 4096 -> 2048 189 to 241 / 197 to 244, 203 to 250 / 201 to 235, 64 of 4096 -> 768 225 to 293 / 234 to 291, 252 to 301 /
+# 246 to 292; 1.6 GB: 64 of 4096 -> 2048 471 to 606 / 411 to 526, 504 to 598 / 494 to 592. Hidden 2048, up to 0.8 GB: 96 of 2048 -> 1408, 130 rows 315 / 328 to 343, 312 to 325 / 337 to
+# 361, 150 rows 351 / 326 to 338, 350 / 343 to 361, 190 rows 384 / 390 to 398, 386 to 391 / 398 to 415; from 2304 on columns win again: 128 of 2304 -> 1664, 138 rows, skewed, 568 /
+# 538; 160 of 2560 -> 640, 135 rows, uniform, 387 / 362; FP8 layer, uniform: 128 of 2816 -> 896, 157 rows 499 / 414; 64 of 2304 -> 1280, 162 rows 333 / 298.
+SECOND_WINDOW_MIN_WEIGHT_BYTES = 400 << 20  # e4m3 bytes of this rank's experts
+SECOND_WINDOW_MIN_HIDDEN = 2304
+
+
+def _token_columns(rows: float, weight_bytes: int, hidden: int) -> int:
     """Tokens of a tile for the natively block-scaled GEMMs that take them as columns, or 0 for the form with tokens as rows."""
     if rows <= 60:
         return 64 if rows <= 8 else 128
-    return 0 if rows <= 120 or rows > 200 else 160 if rows <= 136 else 192 if rows <= 164 else 224
+    if rows <= 120 or rows > 200 or weight_bytes < SECOND_WINDOW_MIN_WEIGHT_BYTES or hidden < SECOND_WINDOW_MIN_HIDDEN:
+        return 0
+    return 160 if rows <= 136 else 192 if rows <= 164 else 224
 
 
 # Natively block-scaled GEMMs: average rows per expert from which the 128x256 tiles are used instead of the 128x128 ones. Since the
@@ -473,7 +487,7 @@ def fused_forward_many(layers, xs, idxs, ws, overlap: bool = True, num_dispatch_
         overlapped = comm is not cur
         ga = min(L, max(1, int(round(L * SPLIT_FRACTION)))) if overlapped else L
         if native:
-            columns = _token_columns(R_ * w.num_tokens * K / E)
+            columns = _token_columns(R_ * w.num_tokens * K / E, w13.numel() + w2.numel(), cfg.hidden)
             wide2 = R_ * w.num_tokens * K >= WIDE_TILE_MIN_ROWS_PER_EXPERT * E
             wide = wide2 or columns != 0
             sfb = l._mx[0 if wide else 2]

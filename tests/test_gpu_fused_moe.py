@@ -203,6 +203,9 @@ def test_fused_forward_with_tokens_as_columns(monkeypatch, R, T):
     from deepep_efa_b200.models import moe as moe_mod
     H, I, E, K = 512, 384, 8, 3
     vc, layers, xs, idxs, ws = _setup(R, T, H, I, E, K, True, seed=T)
+    # (from 120 rows on only large layers take columns; the kernels do not mind small ones)
+    monkeypatch.setattr(moe_mod, "SECOND_WINDOW_MIN_WEIGHT_BYTES", 0)
+    monkeypatch.setattr(moe_mod, "SECOND_WINDOW_MIN_HIDDEN", 0)
     calls = []
 
     class Spy:
@@ -225,7 +228,7 @@ def test_fused_forward_with_tokens_as_columns(monkeypatch, R, T):
 
         got = run()
         rows = R * T * K / E
-        columns = moe_mod._token_columns(rows)
+        columns = moe_mod._token_columns(rows, 0, 0)
         assert (columns != 0) == (rows <= 60 or 120 < rows <= 200)
         for swiglu, atoms, given in calls:
             if swiglu:
@@ -234,7 +237,7 @@ def test_fused_forward_with_tokens_as_columns(monkeypatch, R, T):
                 assert given == (columns if R == 1 else 0)
                 narrow = rows < moe_mod.WIDE_TILE_MIN_ROWS_PER_EXPERT and (R > 1 or not columns)
                 assert any(atoms is l._mx[1 if narrow else 3] for l in layers)
-        monkeypatch.setattr(moe_mod, "_token_columns", lambda rows: 0)
+        monkeypatch.setattr(moe_mod, "_token_columns", lambda *_: 0)
         for a, b in zip(got, run()):
             assert torch.equal(a, b) and a.any()
         w13_all, w2_all = (torch.cat([getattr(l, n).detach().float() for l in layers]) for n in ("w13", "w2"))
