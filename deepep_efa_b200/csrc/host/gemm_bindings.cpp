@@ -386,6 +386,22 @@ torch::Tensor build_sf_atoms_b(const torch::Tensor& scales, int64_t n, bool swig
     return atoms;
 }
 
+// Both natively block-scaled products of an expert layer whose first one quantises its own output (wide tiles, or tokens as columns): rows
+// a [M, H] with power-of-two scales, groups of whole 128-row tiles -> bf16 [M, H]. One call from the host's side, because a short prompt's
+// GPU waits for each of these launches (8 experts of 3072 -> 1920, 273 tokens: four calls and two allocations were 5 us more per layer).
+torch::Tensor fp8_experts(const torch::Tensor& a, const torch::Tensor& a_scales, const torch::Tensor& w13, const torch::Tensor& w2, const torch::Tensor& m_offsets,
+                          const torch::Tensor& m_ends, const torch::Tensor& atoms13, const torch::Tensor& atoms2, double timeout_ms, int tokens_as_columns) {
+    DXG_CHECK(a.dim() == 2 && a.size(0) % 128 == 0 && w13.dim() == 3, "a must be [M, H] in whole tiles of 128 rows, w13 [G, 2 I, H]");
+    const auto none = c10::nullopt;
+    const int64_t inter = w13.size(1) / 2;
+    const torch::Tensor a_atoms = build_sf_atoms_a(a_scales, none, 0);
+    const torch::Tensor h = torch::empty({a.size(0), inter}, a.options()), h_atoms = torch::empty({a.size(0) / 128, inter / 128, 512}, a_atoms.options());
+    grouped_gemm(a, w13, m_offsets, 0, true, none, none, none, 0, timeout_ms, m_ends, a_atoms, atoms13, none, none, none, none, none, false, h, h_atoms, false, none,
+                 false, tokens_as_columns, false);
+    return grouped_gemm(h, w2, m_offsets, 0, false, none, none, none, 0, timeout_ms, m_ends, h_atoms, atoms2, none, none, none, none, none, false, none, none, false, none,
+                        false, tokens_as_columns, false);
+}
+
 void bind_gemm(py::module_& m) {
     m.def("build_sf_atoms_a", &build_sf_atoms_a, py::arg("scales"), py::arg("group_counts") = py::none(), py::arg("rows_per_group") = 0);
     m.def("build_sf_atoms_b", &build_sf_atoms_b, py::arg("scales"), py::arg("n"), py::arg("swiglu") = false, py::arg("wide") = false);
@@ -401,6 +417,7 @@ void bind_gemm(py::module_& m) {
           py::arg("scatter_bases") = py::none(), py::arg("trace") = py::none(), py::arg("mn_major") = false,
           py::arg("out_fp8") = py::none(), py::arg("out_atoms") = py::none(), py::arg("m_ends_are_counts") = false, py::arg("sched") = py::none(),
           py::arg("early_table") = false, py::arg("tokens_as_columns") = 0, py::arg("hold_successor") = false);
+    m.def("fp8_experts", &fp8_experts);
     m.def("build_plan", &build_plan);
     m.def("gather_rows", &gather_rows, py::arg("src"), py::arg("src_row"), py::arg("scale") = py::none(), py::arg("out") = py::none());
     m.def("gather_reduce_rows", &gather_reduce_rows, py::arg("src"), py::arg("pos"), py::arg("w") = py::none(), py::arg("out") = py::none());

@@ -221,15 +221,11 @@ class MoELayer(nn.Module):
         if mx is not None:
             # padding rows of the plan carry all-zero data; whatever exponent their zero scale maps to does not matter
             columns = _token_columns(buf.group_size * x.size(0) * self.cfg.num_topk / self.cfg.num_experts, w13.numel() + w2.numel(), self.cfg.hidden)
-            a_atoms = gg.build_sf_atoms_a(a_s)
             if columns or plan.num_rows >= WIDE_TILE_MIN_ROWS_PER_EXPERT * self.num_local_experts:
                 # the first GEMM quantises its own output: a wide tile holds one whole scale block of a row
-                hq = torch.empty(plan.num_rows, self.cfg.intermediate, dtype=torch.float8_e4m3fn, device=a.device)
-                ha = torch.empty(plan.num_rows // 128, self.cfg.intermediate // 128, 512, dtype=torch.uint8, device=a.device)
-                C.grouped_gemm(a, w13, plan.m_offsets, 0, True, sfa_atoms=a_atoms, sfb_atoms=mx[0], out_fp8=hq, out_atoms=ha, tokens_as_columns=columns, **how)
-                y_perm = C.grouped_gemm(hq, w2, plan.m_offsets, 0, False, sfa_atoms=ha, sfb_atoms=mx[3], tokens_as_columns=columns, **how)
+                y_perm = C.fp8_experts(a, a_s, w13, w2, plan.m_offsets, plan.m_ends, mx[0], mx[3], GEMM_TIMEOUT_MS, columns)
             else:
-                h = C.grouped_gemm(a, w13, plan.m_offsets, 0, True, sfa_atoms=a_atoms, sfb_atoms=mx[2], **how)
+                h = C.grouped_gemm(a, w13, plan.m_offsets, 0, True, sfa_atoms=gg.build_sf_atoms_a(a_s), sfb_atoms=mx[2], **how)
                 hq, hs = C.per_token_cast_to_fp8(h, True, False)
                 y_perm = C.grouped_gemm(hq, w2, plan.m_offsets, 0, False, sfa_atoms=gg.build_sf_atoms_a(hs), sfb_atoms=mx[1], **how)
         else:
