@@ -1097,7 +1097,7 @@ cudaError_t launch_sel(const GroupedGemmArgs& a, cudaStream_t stream) {
 
 cudaError_t launch_grouped_gemm(const GroupedGemmArgs& a, cudaStream_t stream) {
     if (a.num_groups < 1 || a.num_groups > kMaxGroups || a.num_sms < 1) return cudaErrorInvalidValue;
-    // MN-major operands: bf16, no swiglu, single CTAs; mode 0 takes B that way (input gradients read the weight in place),
+    // MN-major operands: bf16, no swiglu, single CTAs or pairs (the caller's choice); mode 0 takes B that way (input gradients read the weight in place),
     // mode 1 takes both (weight gradients read the output gradient and the activation in place)
     if ((a.a_mn || a.b_mn) && (a.fp8 || a.swiglu || (a.mode == 0 && a.a_mn) || (a.mode == 1 && !(a.a_mn && a.b_mn)) || a.n % 64 != 0))
         return cudaErrorInvalidValue;

@@ -419,8 +419,8 @@ __global__ void __launch_bounds__(kDispatchThreads, 1) dispatch_kernel(const __g
 }
 
 // A lone rank that may use the whole GPU: the rows only move within its memory, at the speed of a copy. A warp takes one piece of one row
-// (2 KB to read when it casts, 4 KB otherwise), asks for all of it together with the row's place, stores it and ends; five or six CTAs of eight
-// such warps share an SM. With a warp per row that walked over its columns, 32 to an SM, a row of 14 KB was seven dependent steps (one B200,
+// (2 KB to read when it casts, 4 KB otherwise), asks for all of it together with the row's place, stores it and ends; five CTAs of eight such
+// warps share an SM when it casts, four when it copies or combines, three with two biases. With a warp per row that walked over its columns, 32 to an SM, a row of 14 KB was seven dependent steps (one B200,
 // 4096 x 7168: cast to FP8 31.4 -> 19.2 us, back in BF16 27.4 -> 17.5 us with what overlaps the predecessor; 3001 x 4096 in BF16 with one
 // bias 11.5 -> 8.0 and 18.3 -> 12.0 us).
 constexpr int kLoneThreads = 256;
