@@ -161,11 +161,19 @@ torch::Tensor grouped_gemm(const torch::Tensor& a, const torch::Tensor& b, const
         // the output of a weight gradient is the work. Single / pair, us, 64 experts of 4096 -> 2 x 1408 (first product, its input gradient,
         // its weight gradient), uniform but where noted: 128 rows 255 / 316, 242 / 298, 359 / 567; 242 rows 346 / 329, 403 / 331, 582 / 726; 308 rows 426 /
         // 406, 485 / 460, 683 / 778; 430 rows, skewed, 581 / 547, 661 / 617, 880 / 884; 512 rows 689 / 565, 754 / 619, 918 / 798; 838 rows, skewed, 1005 / 921,
-        // 1129 / 967, 1287 / 1226. The FP8 promotion hands a window to the epilogue every K block, and the cross-CTA handshake per
+        // 1129 / 967, 1287 / 1226. In a loop of whole training steps (power limit) a pair loses wherever most experts end in the first half of a pair's
+        // tile, three row tiles above all. Steps, us, single / pair: padded average 256 to 268: 32 experts of 2304 -> 1792 987 / 910 (single before whole warps
+        // issued), 64 of 4096 -> 1408 2623 / 2503; 270 to 290, skewed: 64 of 6144 -> 1280 3453 / 3548, 64 of 4864 -> 896 2085 / 2120, 32 of 4096 -> 1408 1387 / 1427; 344 to 395, uniform:
+        // 32 of 2560 -> 1792 1202 / 1270, 32 of 4096 -> 1408 1593 / 1670, 64 of it (308 rows) 3189 / 3437, 32 of 3072 -> 1536 1384 / 1466 and 1448 / 1492, skewed: 32 of 6400 -> 1280
+        // 2288 / 2237, 64 and 32 of 4096 -> 1408 3379 / 3387 and 1716 / 1720; from 456 on: 32 of 4096 -> 1408 1909 / 1834, 16 of 4352 -> 640 673 / 637, 60 of 5376 -> 1920 7000 /
+        // 6559, 16 of 3328 -> 768 792 / 720. The FP8 promotion hands a window to the epilogue every K block, and the cross-CTA handshake per
         // block costs more than the halved B traffic saves.
         const char* pr = std::getenv("DEEPEP_GEMM_PAIR");
         if (pr != nullptr && (pr[0] == '0' || pr[0] == '1')) p.cta_pairs = pr[0] == '1';
-        else if (!fp8 && p.m_ends == nullptr) p.cta_pairs = (mode == 1 ? !mn_major || (int64_t)p.m_total >= 480 * (int64_t)G : (int64_t)p.m_total >= 224 * (int64_t)G) ? 1 : 0;
+        else if (!fp8 && p.m_ends == nullptr) {
+            const double rows = (double)p.m_total / G;
+            p.cta_pairs = (mode == 1 ? !mn_major || rows >= 480 : (rows >= 224 && rows <= 270) || rows >= 430) ? 1 : 0;
+        }
         if (p.num_sms < 2) p.cta_pairs = 0;
         // natively block-scaled e4m3: a pair instantiation exists for the wide SwiGLU tile only
         if (fp8 && !(p.sfa_atoms != nullptr && p.mx_wide == 1)) p.cta_pairs = (pr != nullptr && pr[0] == '1' && p.sfa_atoms == nullptr) ? 1 : 0;

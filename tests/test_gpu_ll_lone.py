@@ -23,8 +23,8 @@ def _valid(res):
     return [p.clone() for p in parts]
 
 
-# one token and one selection; slices of a row (few tokens), whole rows, rows wider than a CTA, the last batch of the lone kernel
-# (512 x 8 selections) and the first past it, more selections than a group of eight, hidden sizes that end inside a slice
+# one token and one selection; slices of a row (few tokens), whole rows, rows wider than a CTA, long batches, more selections than a group of
+# eight, hidden sizes that end inside a slice
 @pytest.mark.parametrize("T,H,E,K,masked,sms", [(1, 7168, 256, 8, 0.0, None), (1, 128, 1, 1, 0.0, None), (5, 1152, 60, 6, 0.1, None), (77, 4096, 64, 6, 0.05, None),
                                                  (128, 7168, 16, 8, 0.0, None), (128, 7168, 16, 8, 0.1, 7), (20, 8320, 8, 3, 0.0, None),
                                                  (40, 1024, 64, 32, 0.2, None), (512, 512, 32, 8, 0.0, None), (513, 512, 32, 8, 0.0, None), (33, 512, 8, 2, 1.0, None)])
