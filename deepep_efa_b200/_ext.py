@@ -32,6 +32,7 @@ CUDA_SOURCES = [
     "kernels/ll.cu",
     "kernels/grouped_gemm.cu",
     "kernels/gemm_cols.cu",
+    "kernels/gemm_pairs.cu",
     "kernels/permute.cu",
     "kernels/noalloc.cu",
     "kernels/hier.cu",

@@ -66,7 +66,7 @@ torch::Tensor grouped_gemm(const torch::Tensor& a, const torch::Tensor& b, const
                            c10::optional<torch::Tensor> row_info, c10::optional<torch::Tensor> scatter_bases,
                            c10::optional<torch::Tensor> trace, bool mn_major, c10::optional<torch::Tensor> out_fp8,
                            c10::optional<torch::Tensor> out_atoms, bool m_ends_are_counts, c10::optional<torch::Tensor> sched, bool early_table, int tokens_as_columns,
-                           bool hold_successor) {
+                           bool hold_successor, bool zero_tail) {
     DXG_CHECK(a.is_cuda() && b.is_cuda() && m_offsets.is_cuda(), "operands must be CUDA tensors");
     DXG_CHECK(a.is_contiguous() && b.is_contiguous() && m_offsets.is_contiguous(), "operands must be contiguous");
     DXG_CHECK(m_offsets.scalar_type() == torch::kInt32 && m_offsets.dim() == 1 && m_offsets.numel() >= 2, "m_offsets must be int32 [G+1]");
@@ -148,32 +148,38 @@ torch::Tensor grouped_gemm(const torch::Tensor& a, const torch::Tensor& b, const
     p.m_offsets = m_offsets.data_ptr<int>();
     p.m_ends = nullptr;
     if (m_ends.has_value()) {
-        DXG_CHECK(mode == 0 && m_ends->is_cuda() && m_ends->scalar_type() == torch::kInt32 && m_ends->is_contiguous() && m_ends->numel() == G, "m_ends must be int32 [G] on the GPU (M-grouped mode only)");
+        DXG_CHECK(m_ends->is_cuda() && m_ends->scalar_type() == torch::kInt32 && m_ends->is_contiguous() && m_ends->numel() == G, "m_ends must be int32 [G] on the GPU");
         p.m_ends = m_ends->data_ptr<int>();
         p.m_ends_are_counts = m_ends_are_counts ? 1 : 0;
     }
+    DXG_CHECK(!zero_tail || (mode == 0 && !fp8 && !swiglu && p.m_ends != nullptr), "zero_tail needs m_ends (M-grouped mode, bf16, no swiglu)");
     p.num_sms = num_sms > 0 ? num_sms : sm_count(device);
     {
         const char* o = std::getenv("DEEPEP_GEMM_ORDER");
         p.tile_order = (o != nullptr && o[0] == '1') ? 1 : 0;
-        // CTA pairs (cta_group::2), BF16: half of the weight tile per CTA, so a third less to pull from L2. A pair's tile is two row tiles
-        // high, and with few rows per expert (the average of the padded ones is what the host knows) its second half multiplies nothing, or
-        // the output of a weight gradient is the work. Single / pair, us, 64 experts of 4096 -> 2 x 1408 (first product, its input gradient,
-        // its weight gradient), uniform but where noted: 128 rows 255 / 316, 242 / 298, 359 / 567; 242 rows 346 / 329, 403 / 331, 582 / 726; 308 rows 426 /
-        // 406, 485 / 460, 683 / 778; 430 rows, skewed, 581 / 547, 661 / 617, 880 / 884; 512 rows 689 / 565, 754 / 619, 918 / 798; 838 rows, skewed, 1005 / 921,
-        // 1129 / 967, 1287 / 1226. In a loop of whole training steps (power limit) a pair loses wherever most experts end in the first half of a pair's
-        // tile, three row tiles above all. Steps, us, single / pair: padded average 256 to 268: 32 experts of 2304 -> 1792 987 / 910 (single before whole warps
-        // issued), 64 of 4096 -> 1408 2623 / 2503; 270 to 290, skewed: 64 of 6144 -> 1280 3453 / 3548, 64 of 4864 -> 896 2085 / 2120, 32 of 4096 -> 1408 1387 / 1427; 344 to 395, uniform:
-        // 32 of 2560 -> 1792 1202 / 1270, 32 of 4096 -> 1408 1593 / 1670, 64 of it (308 rows) 3189 / 3437, 32 of 3072 -> 1536 1384 / 1466 and 1448 / 1492, skewed: 32 of 6400 -> 1280
-        // 2288 / 2237, 64 and 32 of 4096 -> 1408 3379 / 3387 and 1716 / 1720; from 456 on: 32 of 4096 -> 1408 1909 / 1834, 16 of 4352 -> 640 673 / 637, 60 of 5376 -> 1920 7000 /
-        // 6559, 16 of 3328 -> 768 792 / 720. The FP8 promotion hands a window to the epilogue every K block, and the cross-CTA handshake per
-        // block costs more than the halved B traffic saves.
+        // CTA pairs (cta_group::2) of the row form, BF16: weight gradients whose operands are read in place, from 480 padded rows per expert on (with
+        // fewer the output is the work), all others, and SwiGLU where a pair's tile of 256 rows has little padding. The FP8 promotion hands a window to
+        // the epilogue every K block, and the cross-CTA handshake per block costs more than the halved B traffic saves.
         const char* pr = std::getenv("DEEPEP_GEMM_PAIR");
-        if (pr != nullptr && (pr[0] == '0' || pr[0] == '1')) p.cta_pairs = pr[0] == '1';
-        else if (!fp8 && p.m_ends == nullptr) {
-            const double rows = (double)p.m_total / G;
-            p.cta_pairs = (mode == 1 ? !mn_major || rows >= 480 : (rows >= 224 && rows <= 270) || rows >= 430) ? 1 : 0;
+        const bool forced = pr != nullptr && (pr[0] == '0' || pr[0] == '1');
+        const double rows = (double)p.m_total / G;
+        if (forced) p.cta_pairs = pr[0] == '1';
+        else if (!fp8 && mode == 1) p.cta_pairs = !mn_major || rows >= 480;
+        else if (!fp8 && p.m_ends == nullptr) p.cta_pairs = (rows >= 224 && rows <= 270) || rows >= 430;
+        // Forward and input gradients in BF16: tokens as columns on CTA pairs, from 160 padded rows per expert on. One tile of rows of the other form is
+        // as good as a tile of columns (64 experts of 4096 -> 1408, 94 rows: 765 and 774 us; 128 of 2048 -> 512, 100 rows: 345 and 365); with more than one it is not
+        // (gemm_pairs.cu has both sides).
+        if (mode == 0 && !fp8 && !swiglu && p.num_sms >= 2 && p.n % 128 == 0 && p.k % 64 == 0 && !ready.has_value() && !expected.has_value() && !row_info.has_value() &&
+            !trace.has_value() && !sched.has_value() && !early_table && !hold_successor) {
+            p.token_pairs = forced ? p.cta_pairs : rows >= 160;
+            p.token_cap = 256;
         }
+        if (mode == 0 && !swiglu && !fp8) p.cta_pairs = 0;
+        // A weight gradient with about a tile of rows per expert is bound by what happens per tile; leaving out steps of its two K blocks cost more than it
+        // gave (64 experts of 4096 -> 1408, 94 rows: 562 and 573 us).
+        if (mode == 1 && !forced && rows < 160) p.m_ends = nullptr;
+        p.zero_tail = zero_tail ? 1 : 0;
+        if (zero_tail && !p.token_pairs) p.m_ends = nullptr;  // all rows up to the next group are computed: zeros in, zeros out
         if (p.num_sms < 2) p.cta_pairs = 0;
         // natively block-scaled e4m3: a pair instantiation exists for the wide SwiGLU tile only
         if (fp8 && !(p.sfa_atoms != nullptr && p.mx_wide == 1)) p.cta_pairs = (pr != nullptr && pr[0] == '1' && p.sfa_atoms == nullptr) ? 1 : 0;
@@ -222,7 +228,7 @@ torch::Tensor grouped_gemm(const torch::Tensor& a, const torch::Tensor& b, const
     }
     p.error_flag = error_flag(device).data_ptr<int>();
     p.timeout_cycles = (long long)(timeout_ms * (double)clock_khz(device));
-    const cudaError_t e = (columns ? dx::launch_token_cols_gemm : dx::launch_grouped_gemm)(p, at::cuda::getCurrentCUDAStream(device).stream());
+    const cudaError_t e = (p.token_pairs ? dx::launch_token_pairs_gemm : columns ? dx::launch_token_cols_gemm : dx::launch_grouped_gemm)(p, at::cuda::getCurrentCUDAStream(device).stream());
     if (e == cudaErrorInvalidValue) {
         cudaGetLastError();
         throw std::invalid_argument(
@@ -405,9 +411,9 @@ torch::Tensor fp8_experts(const torch::Tensor& a, const torch::Tensor& a_scales,
     const torch::Tensor a_atoms = build_sf_atoms_a(a_scales, none, 0);
     const torch::Tensor h = torch::empty({a.size(0), inter}, a.options()), h_atoms = torch::empty({a.size(0) / 128, inter / 128, 512}, a_atoms.options());
     grouped_gemm(a, w13, m_offsets, 0, true, none, none, none, 0, timeout_ms, m_ends, a_atoms, atoms13, none, none, none, none, none, false, h, h_atoms, false, none,
-                 false, tokens_as_columns, false);
+                 false, tokens_as_columns, false, false);
     return grouped_gemm(h, w2, m_offsets, 0, false, none, none, none, 0, timeout_ms, m_ends, h_atoms, atoms2, none, none, none, none, none, false, none, none, false, none,
-                        false, tokens_as_columns, false);
+                        false, tokens_as_columns, false, false);
 }
 
 void bind_gemm(py::module_& m) {
@@ -424,7 +430,7 @@ void bind_gemm(py::module_& m) {
           py::arg("ready") = py::none(), py::arg("expected") = py::none(), py::arg("row_info") = py::none(),
           py::arg("scatter_bases") = py::none(), py::arg("trace") = py::none(), py::arg("mn_major") = false,
           py::arg("out_fp8") = py::none(), py::arg("out_atoms") = py::none(), py::arg("m_ends_are_counts") = false, py::arg("sched") = py::none(),
-          py::arg("early_table") = false, py::arg("tokens_as_columns") = 0, py::arg("hold_successor") = false);
+          py::arg("early_table") = false, py::arg("tokens_as_columns") = 0, py::arg("hold_successor") = false, py::arg("zero_tail") = false);
     m.def("fp8_experts", &fp8_experts);
     m.def("build_plan", &build_plan);
     m.def("gather_rows", &gather_rows, py::arg("src"), py::arg("src_row"), py::arg("scale") = py::none(), py::arg("out") = py::none());

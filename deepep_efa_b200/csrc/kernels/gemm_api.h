@@ -35,6 +35,8 @@ struct GroupedGemmArgs {
     const int* m_offsets;     // [G+1] device memory
     const int* m_ends;        // optional [G]: group g covers rows [m_offsets[g], m_ends[g]) instead of up to m_offsets[g+1]
                               // (mode 0 only; the low-latency layout has fixed group starts and a count per expert)
+    int zero_tail;            // launch_token_pairs_gemm, with m_ends: 1 = rows from m_ends[g] to m_offsets[g+1] are zero in A, and in C they are
+                              // written as zeros; 0 = they are not touched
     int m_ends_are_counts;    // 1 = m_ends[g] is the number of rows of group g instead of its end
     int num_groups;
     int mode;                 // 0 = M-grouped, 1 = K-grouped
@@ -80,7 +82,8 @@ struct GroupedGemmArgs {
     // 1 = the next kernel in the stream gets no SM before this one has ended, also where it is a programmatic dependent launch: the SMs
     // that this launch leaves free are meant for another stream.
     int hold_successor;
-    // launch_token_cols_gemm: tokens of one tile at most (a multiple of 32 from 64 to 224)
+    int token_pairs;          // the caller's choice: launch_token_pairs_gemm takes this product
+    // launch_token_cols_gemm, launch_token_pairs_gemm: tokens of one tile at most (a multiple of 32 from 64 to 224, of 64 up to 256)
     int token_cap;
 };
 
@@ -89,6 +92,10 @@ cudaError_t launch_grouped_gemm(const GroupedGemmArgs& args, cudaStream_t stream
 // The same product for groups of few to some hundred rows (gemm_cols.cu): natively block-scaled operands with 256-column weight atoms,
 // mode 0, n % 256 == 0; SwiGLU writes c_fp8 and c_atoms, otherwise bf16 rows to c or through the scatter epilogue.
 cudaError_t launch_token_cols_gemm(const GroupedGemmArgs& args, cudaStream_t stream);
+
+// BF16 with the tokens as columns on CTA pairs (gemm_pairs.cu): mode 0, B [G, N, K] or with b_mn [G, K, N], n % 128 == 0, k % 64 == 0, any
+// group boundaries.
+cudaError_t launch_token_pairs_gemm(const GroupedGemmArgs& args, cudaStream_t stream);
 
 // Expert-major plan from local expert ids [N, K] (-1 = unselected) and 128-aligned group offsets [L+1] on the host:
 // m_offsets [L+1] (the offsets on the device), m_ends [L] (end of every group's rows in front of its padding), pos [N*K], src_row [m_pad]

@@ -108,6 +108,7 @@ __device__ __forceinline__ void store_rows_256(int4* stage, const int4 (&regs)[1
 struct TileInfo {
     int a_row, a_k0, b_row, b_row2, b_k0, num_kb, c_row, c_col, group, nblock, nblock2;
     int c_row_end;  // first output row this tile must not write (end of its group; groups need no 128-row alignment)
+    int k_rows;     // weight gradients: rows of the reduction
     int nt;         // n-tile index inside the group (kMx: selects the B scale atoms)
     int n_cols;     // columns of this tile: kBlockN, or half of it for the last column tile of an MN-major operand (kRagged)
     // MN-major operands: first tile row inside the tensor's contiguous dimension, and the tensor row of K index 0
@@ -282,6 +283,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             ti.a_k0 = 0;
             ti.b_k0 = 0;
             ti.num_kb = p.k / elem_per_kb;
+            ti.k_rows = 0;
             ti.c_row = ti.a_row;
             ti.c_row_end = min(m1, p.m_total);
             if (kSwiGLU) {
@@ -310,7 +312,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             ti.a_kbase = ti.b_kbase = m0;
             ti.a_k0 = m0;
             ti.b_k0 = m0;
-            ti.num_kb = (m1 - m0) / elem_per_kb;
+            ti.k_rows = p.m_ends != nullptr ? group_rows(p, g, m0) : m1 - m0;  // (the rows behind it are zero in both operands)
+            ti.num_kb = (ti.k_rows + elem_per_kb - 1) / elem_per_kb;
             ti.c_row = g * p.n + ti.a_row;
             ti.c_row_end = min((g + 1) * p.n, p.num_groups * p.n);
             ti.c_col = jt * kBlockN;
@@ -591,8 +594,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                                             (new_window && j == 0) ? 0u : 1u);
                             }
                         } else {
-#pragma unroll
-                            for (int j = 0; j < 4; ++j) {
+                            auto step = [&](int j) {
                                 // +32 bytes along K inside the swizzle atom = +2 in the 16-byte start-address field
                                 if constexpr (kPair)
                                     umma_pair<kFp8>(tmem_d, adesc + (uint64_t)j * a_kstep, bdesc + (uint64_t)j * b_kstep, idesc,
@@ -600,6 +602,17 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                                 else
                                     umma<kFp8>(tmem_d, adesc + (uint64_t)j * a_kstep, bdesc + (uint64_t)j * b_kstep, idesc,
                                                (new_window && j == 0) ? 0u : 1u);
+                            };
+                            // 16 K steps per MMA; those behind the last row of a weight gradient are left out, as are whole blocks of 64 (decode): both weight
+                            // gradients of 64 experts of 4096 -> 1408, us, in a loop: 190 rows 781 -> 726, 384 rows 1065 -> 1044, 768 rows 1649 -> 1605.
+                            // (Whole blocks keep their straight line of four: an MMA behind a branch costs three times as much to issue.)
+                            if (kMnMajor && p.mode == 1 && ti.k_rows - kb * 64 <= 48) {
+                                step(0);
+                                if (ti.k_rows - kb * 64 > 16) step(1);
+                                if (ti.k_rows - kb * 64 > 32) step(2);
+                            } else {
+#pragma unroll
+                                for (int j = 0; j < 4; ++j) step(j);
                             }
                         }
                         // smem stage reusable once these MMAs have read it (in both CTAs of a pair)
@@ -998,22 +1011,6 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 }
 
 // ---- host side ------------------------------------------------------------------------------
-// Row-major [k_rows, mn_cols] bf16 tensor whose contiguous dimension is the operand's row index (MN-major operand), seen as
-// [mn_cols / 64, k_rows, 64]: a box of `box_rows` operand rows x 64 K-steps lands as chunks of 64 rows (8 KiB each, 128B swizzle),
-// the order the matrix descriptor expects, in one copy. One copy per 64-row chunk cost the loading lane up to six instructions per
-// stage. Chunks past the last column read as zeros and touch no memory.
-bool make_map_mn(CUtensorMap* map, const void* ptr, uint64_t k_rows, uint64_t mn_cols, uint32_t box_rows) {
-    EncodeFn fn = get_encode_fn();
-    if (fn == nullptr) return false;
-    cuuint64_t dims[3] = {64, k_rows, mn_cols / 64};
-    cuuint64_t strides[2] = {mn_cols * 2, 128};
-    cuuint32_t box[3] = {64, 64, box_rows / 64};
-    cuuint32_t estr[3] = {1, 1, 1};
-    const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                          CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    return r == CUDA_SUCCESS;
-}
-
 // Scale atoms as a 2-D tensor of 32-bit words: one row per (tile, K block), `words` words per row (128 per 512-byte atom).
 bool make_map_sf(CUtensorMap* map, const void* ptr, uint64_t rows, uint32_t words) {
     EncodeFn fn = get_encode_fn();

@@ -216,6 +216,19 @@ __device__ __forceinline__ void tma_load_3d_pair(const CUtensorMap* map, uint32_
         "l"(reinterpret_cast<uint64_t>(map)), "r"(bar_cluster_addr), "r"(0), "r"(c1), "r"(c2)
         : "memory");
 }
+// The same with the shared-memory address as it is.
+__device__ __forceinline__ void tma_load_2d_pair_at(const CUtensorMap* map, uint32_t bar_cluster_addr, uint32_t dst, int c0, int c1) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(dst),
+        "l"(reinterpret_cast<uint64_t>(map)), "r"(bar_cluster_addr), "r"(c0), "r"(c1)
+        : "memory");
+}
+__device__ __forceinline__ void tma_load_3d_pair_at(const CUtensorMap* map, uint32_t bar_cluster_addr, uint32_t dst, int c0, int c1, int c2) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(dst),
+        "l"(reinterpret_cast<uint64_t>(map)), "r"(bar_cluster_addr), "r"(c0), "r"(c1), "r"(c2)
+        : "memory");
+}
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t* dst_smem, uint32_t ncols) {
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(dst_smem)), "r"(ncols) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
@@ -353,6 +366,22 @@ bool make_map(CUtensorMap* map, const void* ptr, bool fp8, uint64_t rows, uint64
     const CUresult r = fn(map, fp8 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims,
                           strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS;
+}
+
+// Row-major [k_rows, mn_cols] bf16 tensor whose contiguous dimension is the operand's row index (MN-major operand), seen as
+// [mn_cols / 64, k_rows, 64]: a box of `box_rows` operand rows x 64 K-steps lands as chunks of 64 rows (8 KiB each, 128B swizzle),
+// the order the matrix descriptor expects, in one copy. One copy per 64-row chunk cost the loading lane up to six instructions per
+// stage. Chunks past the last column read as zeros and touch no memory.
+bool make_map_mn(CUtensorMap* map, const void* ptr, uint64_t k_rows, uint64_t mn_cols, uint32_t box_rows) {
+    EncodeFn fn = get_encode_fn();
+    if (fn == nullptr) return false;
+    cuuint64_t dims[3] = {64, k_rows, mn_cols / 64};
+    cuuint64_t strides[2] = {mn_cols * 2, 128};
+    cuuint32_t box[3] = {64, 64, box_rows / 64};
+    cuuint32_t estr[3] = {1, 1, 1};
+    const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                          CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS;
 }
 

@@ -82,23 +82,24 @@ class _Combine(torch.autograd.Function):
 
 
 class _GroupedLinear(torch.autograd.Function):
-    """y[m] = x[m] @ w[g].T for the rows m of expert g (w: [G, N, K])."""
+    """y[m] = x[m] @ w[g].T for the rows m of expert g (w: [G, N, K]). With ``m_ends`` the rows of x from the end of an expert's own rows to
+    the next expert are zero, and so are those of the incoming gradient: nothing is multiplied there, and results have zeros there too."""
 
     @staticmethod
-    def forward(ctx, x, w, m_offsets):
-        ctx.save_for_backward(x, w, m_offsets)
+    def forward(ctx, x, w, m_offsets, m_ends):
+        ctx.save_for_backward(x, w, m_offsets, m_ends)
         if x.is_cuda:
-            return gg.grouped_gemm(x, w, m_offsets)
+            return gg.grouped_gemm(x, w, m_offsets, m_ends=m_ends, zero_tail=m_ends is not None)
         return gg.reference_grouped_gemm(x, w, m_offsets).to(x.dtype)
 
     @staticmethod
     def backward(ctx, grad):
-        x, w, m_offsets = ctx.saved_tensors
+        x, w, m_offsets, m_ends = ctx.saved_tensors
         grad = grad.contiguous()
         if x.is_cuda and x.size(1) % 128 == 0 and w.size(1) % 128 == 0:
             # weight, gradient and activation are read in place as MN-major operands: no transposed copies
-            dx = gg.grouped_gemm_dgrad(grad, w, m_offsets)
-            dw = gg.grouped_gemm_wgrad_inplace(grad, x, m_offsets)
+            dx = gg.grouped_gemm_dgrad(grad, w, m_offsets, m_ends=m_ends)
+            dw = gg.grouped_gemm_wgrad_inplace(grad, x, m_offsets, m_ends=m_ends)
         elif x.is_cuda:
             dx = gg.grouped_gemm(grad, gg.transpose_last2(w), m_offsets)
             dw = gg.grouped_gemm_wgrad(gg.transpose_last2(grad), gg.transpose_last2(x), m_offsets)
@@ -106,11 +107,11 @@ class _GroupedLinear(torch.autograd.Function):
             dx = gg.reference_grouped_gemm(grad, w.transpose(1, 2).contiguous(), m_offsets).to(x.dtype)
             offs = m_offsets.tolist()
             dw = torch.stack([grad[offs[g]:offs[g + 1]].float().t() @ x[offs[g]:offs[g + 1]].float() for g in range(w.size(0))]).to(w.dtype)
-        return dx, dw, None
+        return dx, dw, None, None
 
 
-def grouped_linear(x, w, m_offsets):
-    return _GroupedLinear.apply(x, w, m_offsets)
+def grouped_linear(x, w, m_offsets, m_ends=None):
+    return _GroupedLinear.apply(x, w, m_offsets, m_ends)
 
 
 # ---------------------------------------------------------------------------------------------------------
@@ -152,9 +153,9 @@ class MoELayer(nn.Module):
         recv_x, recv_w = _Dispatch.apply(x, topk_weights, topk_idx, self.buffer, self.cfg.num_experts, routing)
         plan = build_expert_plan(routing["recv_topk_idx"], routing["counts"])
         x_perm = permute(recv_x, plan)
-        h13 = grouped_linear(x_perm, self.w13, plan.m_offsets)
+        h13 = grouped_linear(x_perm, self.w13, plan.m_offsets, plan.m_ends)
         h = gg.swiglu(h13)
-        y_perm = grouped_linear(h, self.w2, plan.m_offsets)
+        y_perm = grouped_linear(h, self.w2, plan.m_offsets, plan.m_ends)
         out_buf = self._symmetric_like(recv_x)
         y_recv = unpermute_weighted(y_perm, recv_w, plan, out_buf)
         return _Combine.apply(y_recv, self.buffer, routing["handle"])

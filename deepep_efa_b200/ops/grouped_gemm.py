@@ -23,17 +23,18 @@ from .. import _ext
 def grouped_gemm(a: torch.Tensor, b: torch.Tensor, m_offsets: torch.Tensor, *, swiglu: bool = False,
                  a_scales: Optional[torch.Tensor] = None, b_scales: Optional[torch.Tensor] = None,
                  out: Optional[torch.Tensor] = None, num_sms: int = 0, m_ends: Optional[torch.Tensor] = None,
-                 sfa_atoms: Optional[torch.Tensor] = None, sfb_atoms: Optional[torch.Tensor] = None) -> torch.Tensor:
+                 sfa_atoms: Optional[torch.Tensor] = None, sfb_atoms: Optional[torch.Tensor] = None, zero_tail: bool = False) -> torch.Tensor:
     """M-grouped GEMM; see the module docstring. Returns bf16 ``[M, N]`` (``[M, N/2]`` with ``swiglu``).
 
     ``m_ends`` (int32 ``[G]``, optional) makes group g cover rows ``[m_offsets[g], m_ends[g])``: the "masked" form for the
     low-latency layout ``[L, N, hidden]``, where every expert starts at ``g * N`` and only ``packed_recv_count[g]`` rows
-    are valid; rows past ``m_ends[g]`` are never written.
+    are valid; rows past ``m_ends[g]`` are never written. ``zero_tail=True`` (bf16, no ``swiglu``) says that the rows of ``a`` from
+    ``m_ends[g]`` to the next group are zero and wants those of the result written as zeros.
 
     ``sfa_atoms`` / ``sfb_atoms`` (from :func:`build_sf_atoms_a` / :func:`build_sf_atoms_b`) select the natively block-scaled
     FP8 kernel: power-of-two scales are applied by the tensor core (``kind::mxf8f6f4.block_scale``) and a whole tile
     accumulates in TMEM. Every group must then start on a multiple of 128 rows."""
-    return _ext.load().grouped_gemm(a, b, m_offsets, 0, swiglu, a_scales, b_scales, out, num_sms, 2000.0, m_ends, sfa_atoms, sfb_atoms)
+    return _ext.load().grouped_gemm(a, b, m_offsets, 0, swiglu, a_scales, b_scales, out, num_sms, 2000.0, m_ends, sfa_atoms, sfb_atoms, zero_tail=zero_tail)
 
 
 def build_sf_atoms_a(a_scales: torch.Tensor) -> torch.Tensor:
@@ -61,16 +62,20 @@ def grouped_gemm_wgrad(a_t: torch.Tensor, b_t: torch.Tensor, m_offsets: torch.Te
     return _ext.load().grouped_gemm(a_t, b_t, m_offsets, 1, False, None, None, out, num_sms)
 
 
-def grouped_gemm_dgrad(grad: torch.Tensor, w: torch.Tensor, m_offsets: torch.Tensor, *, out: Optional[torch.Tensor] = None) -> torch.Tensor:
+def grouped_gemm_dgrad(grad: torch.Tensor, w: torch.Tensor, m_offsets: torch.Tensor, *, out: Optional[torch.Tensor] = None,
+                       m_ends: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Input gradient of ``y = grouped_gemm(x, w)``: ``dx[m] = grad[m] @ w[g]`` for the rows of expert g, with ``w``
-    ``[G, N, K]`` read in place as an MN-major operand (no transposed copy of the weight). bf16; ``grad`` is ``[M, N]``."""
-    return _ext.load().grouped_gemm(grad, w, m_offsets, 0, False, None, None, out, 0, 2000.0, mn_major=True)
+    ``[G, N, K]`` read in place as an MN-major operand (no transposed copy of the weight). bf16; ``grad`` is ``[M, N]``. With ``m_ends`` the rows of
+    ``grad`` from ``m_ends[g]`` to the next group are zero, as are those of the result."""
+    return _ext.load().grouped_gemm(grad, w, m_offsets, 0, False, None, None, out, 0, 2000.0, m_ends, mn_major=True, zero_tail=m_ends is not None)
 
 
-def grouped_gemm_wgrad_inplace(grad: torch.Tensor, x: torch.Tensor, m_offsets: torch.Tensor, *, out: Optional[torch.Tensor] = None) -> torch.Tensor:
+def grouped_gemm_wgrad_inplace(grad: torch.Tensor, x: torch.Tensor, m_offsets: torch.Tensor, *, out: Optional[torch.Tensor] = None,
+                               m_ends: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Weight gradient ``dw[g] = grad[rows of g].T @ x[rows of g]`` with ``grad`` ``[M, N_out]`` and ``x`` ``[M, K_out]`` read in
-    place as MN-major operands (no transposed copies). Group boundaries on multiples of 64 rows. Returns bf16 ``[G, N_out, K_out]``."""
-    return _ext.load().grouped_gemm(grad, x, m_offsets, 1, False, None, None, out, 0, 2000.0, mn_major=True)
+    place as MN-major operands (no transposed copies). Group boundaries on multiples of 64 rows. Returns bf16 ``[G, N_out, K_out]``. With
+    ``m_ends`` the rows of both from ``m_ends[g]`` to the next group are zero, and the reduction stops at the next multiple of 16 rows."""
+    return _ext.load().grouped_gemm(grad, x, m_offsets, 1, False, None, None, out, 0, 2000.0, m_ends, mn_major=True)
 
 
 def reference_grouped_gemm(a: torch.Tensor, b: torch.Tensor, m_offsets: torch.Tensor, swiglu: bool = False,

@@ -1,0 +1,104 @@
+"""BF16 expert GEMMs on CTA pairs with the tokens as columns, and weight gradients that stop at an expert's last row."""
+import pytest
+import torch
+
+pytestmark = [pytest.mark.gpu, pytest.mark.skipif(not torch.cuda.is_available(), reason="needs a GPU")]
+
+
+def _groups(rows, aligned):
+    starts = [0]
+    for n in rows:
+        starts.append(starts[-1] + ((n + 127) // 128 * 128 if aligned else n))
+    return starts, [starts[g] + n for g, n in enumerate(rows)]
+
+
+def _i32(v):
+    return torch.tensor(v, dtype=torch.int32, device="cuda")
+
+
+def _close(out, ref):
+    # fp32 sums of bf16 products, rounded once to bf16 (2^-9 relative of each value; the norm of the errors stays below 4e-3 of the norm)
+    assert ((out.float() - ref).norm() / ref.norm().clamp(min=1e-20)).item() < 4e-3
+
+
+@pytest.mark.parametrize("mn_major", [False, True])
+@pytest.mark.parametrize("how", ["whole", "ragged", "masked", "zero_tail"])
+@pytest.mark.parametrize("K,N,sms", [(64, 128, 0), (192, 384, 6), (512, 256, 0), (320, 1408, 0)])
+def test_tokens_as_columns_on_pairs(monkeypatch, K, N, sms, how, mn_major):
+    """Rows on both sides of the unit of 32, of a tile of 256 and of several equal tiles; odd counts of 128 features; empty groups."""
+    from deepep_efa_b200 import _ext
+    monkeypatch.setenv("DEEPEP_GEMM_PAIR", "1")
+    C = _ext.load()
+    C.gemm_clear_error(0)
+    torch.manual_seed(K + N)
+    rows = [1, 0, 31, 32, 33, 255, 256, 257, 300, 513, 128]
+    starts, ends = _groups(rows, how != "ragged")
+    if how == "zero_tail":  # a group of padding only
+        starts, ends = starts + [starts[-1] + 128], ends + [starts[-1]]
+        rows = rows + [0]
+    G, M = len(rows), starts[-1]
+    x = torch.randn(M, K, device="cuda").to(torch.bfloat16)
+    if how == "zero_tail":
+        for g in range(G):
+            x[ends[g]:starts[g + 1]] = 0
+    w = (torch.randn(G, N, K, device="cuda") * 0.1).to(torch.bfloat16)
+    b = w.transpose(1, 2).contiguous() if mn_major else w
+    out = torch.full((M, N), 7.0, dtype=torch.bfloat16, device="cuda")
+    kw = {} if how in ("whole", "ragged") else dict(m_ends=_i32(ends), zero_tail=how == "zero_tail")
+    C.grouped_gemm(x, b, _i32(starts), 0, False, None, None, out, sms, mn_major=mn_major, **kw)
+    torch.cuda.synchronize()
+    assert C.gemm_error(0) == 0
+    for g in range(G):
+        end = starts[g + 1] if how == "whole" else ends[g]
+        if end > starts[g]:
+            _close(out[starts[g]:end], x[starts[g]:end].float() @ w[g].float().t())
+        assert (out[end:starts[g + 1]] == (0.0 if how == "zero_tail" else 7.0)).all()
+
+
+def test_few_rows_take_the_other_form_with_the_same_padding():
+    """zero_tail below and above the line between the forms: the same rows are zero, the same values are there."""
+    from deepep_efa_b200.ops.grouped_gemm import grouped_gemm, grouped_gemm_dgrad
+    torch.manual_seed(5)
+    for rows in ([100, 20, 128], [300, 129, 200]):
+        starts, ends = _groups(rows, True)
+        x = torch.randn(starts[-1], 256, device="cuda").to(torch.bfloat16)
+        w = (torch.randn(3, 384, 256, device="cuda") * 0.1).to(torch.bfloat16)
+        dy = torch.randn(starts[-1], 384, device="cuda").to(torch.bfloat16)
+        for g in range(3):
+            x[ends[g]:starts[g + 1]] = dy[ends[g]:starts[g + 1]] = 0
+        y = grouped_gemm(x, w, _i32(starts), m_ends=_i32(ends), zero_tail=True)
+        dx = grouped_gemm_dgrad(dy, w, _i32(starts), m_ends=_i32(ends))
+        for g in range(3):
+            r = slice(starts[g], ends[g])
+            _close(y[r], x[r].float() @ w[g].float().t())
+            _close(dx[r], dy[r].float() @ w[g].float())
+            assert (y[ends[g]:starts[g + 1]] == 0).all() and (dx[ends[g]:starts[g + 1]] == 0).all()
+    with pytest.raises(ValueError):
+        grouped_gemm(x, w, _i32(starts), zero_tail=True)
+
+
+@pytest.mark.parametrize("pair", ["0", "1"])
+@pytest.mark.parametrize("N,K", [(128, 128), (256, 384), (384, 256)])
+def test_weight_gradient_stops_at_the_last_row(monkeypatch, N, K, pair):
+    """Rows that end inside every step of 16 of a K block, on its edges, and not at all; the rest of the group is zero."""
+    from deepep_efa_b200 import _ext
+    from deepep_efa_b200.ops.grouped_gemm import grouped_gemm_wgrad_inplace
+    monkeypatch.setenv("DEEPEP_GEMM_PAIR", pair)
+    C = _ext.load()
+    C.gemm_clear_error(0)
+    torch.manual_seed(N)
+    rows = [1, 0, 15, 16, 17, 47, 49, 63, 64, 65, 127, 128, 300]
+    starts, ends = _groups(rows, True)
+    starts, ends, rows = starts + [starts[-1] + 128], ends + [starts[-1]], rows + [0]  # (and a group of padding only)
+    dy, x = (torch.randn(starts[-1], c, device="cuda").to(torch.bfloat16) for c in (N, K))
+    for g in range(len(rows)):
+        dy[ends[g]:starts[g + 1]] = x[ends[g]:starts[g + 1]] = 0
+    dw = grouped_gemm_wgrad_inplace(dy, x, _i32(starts), m_ends=_i32(ends))
+    torch.cuda.synchronize()
+    assert C.gemm_error(0) == 0
+    for g, n in enumerate(rows):
+        r = slice(starts[g], ends[g])
+        if n == 0:
+            assert (dw[g] == 0).all()
+        else:
+            _close(dw[g], dy[r].float().t() @ x[r].float())
