@@ -198,6 +198,7 @@ torch::Tensor grouped_gemm(const torch::Tensor& a, const torch::Tensor& b, const
         DXG_CHECK(scatter_bases->element_size() == 8 && scatter_bases->is_contiguous() && scatter_bases->numel() >= 1, "scatter_bases must be 64-bit pointers");
         p.row_info = row_info->data_ptr<int>();
         p.scatter_bases = reinterpret_cast<const unsigned long long*>(scatter_bases->data_ptr());
+        p.scatter_to_peers = scatter_bases->numel() > 1 ? 1 : 0;
     }
     // The caller says that groups have few rows, and how many a tile may have (1: the ordinary choice). The natively block-scaled 256-column
     // tiles have the form with the weights as M; SwiGLU then quantises its output.

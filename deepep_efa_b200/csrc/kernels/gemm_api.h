@@ -60,6 +60,7 @@ struct GroupedGemmArgs {
     // is negative are dropped. Null = ordinary output.
     const int* row_info;
     const unsigned long long* scatter_bases;
+    int scatter_to_peers;     // 1 = some of them are other GPUs': pieces of a row should be long (FP8 with fp32 scales keeps tiles that store 128 bytes)
     unsigned long long* trace;  // optional [4]: earliest first-tile load / latest epilogue end (global timer, ns) / first wait that
                                 // gave up (role << 56 | tile << 24 | k block << 8 | slot; 0 = none) / what the loader was doing
                                 // then (state << 32 | tile; state 1 = arrival gate, 2 = waiting for a free stage, 3 = loads issued)

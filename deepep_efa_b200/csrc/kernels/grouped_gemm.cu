@@ -13,7 +13,7 @@
 // overlap the MMAs of window i+1. BF16: a window is a whole output tile. FP8 with DeepSeek-style fp32
 // scales (1x128 on activations, 128x128 on weights): a window is ONE K block; the epilogue multiplies it
 // by scale_a[row, kb] * scale_b[nblock, kb] and accumulates in fp32 registers (the MMA's native block
-// scaling wants power-of-two UE8M0 factors, which these scales are not).
+// scaling wants power-of-two UE8M0 factors, which these scales are not). Tiles of 256 columns where there are enough of them (wide_promotion).
 //
 // Every mbarrier wait is bounded; when a limit runs out the CTA raises a flag, all roles leave their
 // loops, TMEM is released and the kernel returns.
@@ -134,11 +134,12 @@ struct Cfg {
     // K blocks ahead of the promotion: four 128-column windows fill TMEM. BF16 hands over one window per tile: two.
     // kMx with 256-column tiles: ONE window (two would fill TMEM and leave no room for the scale columns); the epilogue of
     // that variant drains the accumulator into registers first and releases the window before it stores.
-    static constexpr int kWindows = kPromote ? 4 : ((kMx && kBlockN == 256) ? 1 : 2);
+    static constexpr int kWindows = kPromote ? (kBlockN == 256 ? 2 : 4) : ((kMx && kBlockN == 256) ? 1 : 2);
     static constexpr int kSfCol0 = kWindows * kBlockN;   // kMx: two alternating sets of (4 columns A + 4 per B atom) after the windows
     static constexpr int kSfColsPerBuf = 4 + 4 * kSfBAtoms;
     static constexpr int kTmemCols = kMx ? 512 : kWindows * kBlockN;
     static constexpr int kOutCols = kSwiGLU ? kBlockN / 2 : kBlockN;
+    // (Tiles of 256 columns have two windows, and 128 accumulators per thread.)
     // FP8 promotes every K block on the CUDA cores, so it gets two epilogue warps per TMEM lane quarter (each takes half
     // of the columns); BF16 reads the accumulator once per tile and one warp per quarter is plenty.
     // The single-window wide tile also gets two warps per quarter: each drains half of the columns RAW (128 fp32 registers per
@@ -148,7 +149,8 @@ struct Cfg {
     static constexpr bool kRagged = !kFp8 && !kSwiGLU && kBlockN == 256;
     static constexpr int kEpiWarps = (kPromote || kSplitDrain) ? 8 : 4;
     static constexpr int kThreads = 64 + 32 * kEpiWarps;
-    static constexpr int kOutStageBytes = kRowScatter ? 8192 : (kSplitDrain ? 2048 : 4096);    // per epilogue warp: 32 rows x 32 / 64 (128) BF16
+    static constexpr bool kWidePromote = kPromote && kBlockN == 256;
+    static constexpr int kOutStageBytes = kRowScatter ? 8192 : (kSplitDrain || kWidePromote ? 2048 : 4096);    // per epilogue warp: 32 rows x 32 / 64 (128) BF16
     // kSplitDrain with quantised output: the two warps of a quarter exchange their half-row maxima here (two tile parities)
     static constexpr int kXchBytes = (kMx && kSwiGLU && kBlockN == 256) ? 2 * 2 * kBlockM * 8 : 0;
     static constexpr size_t kSmemBytes =
@@ -340,6 +342,18 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         return t;
     };
 
+    auto next_tile_alone = [&](int tile) {  // for a single thread of a warp
+        if (!drawn) return tile + sched_stride;
+        if (!mbar_wait(&tile_full[tslot], tphase, abort_flag, limit, note, wait_id(8, tile, 0, tslot))) return total_tiles;
+        const int t = s_tile[tslot];
+        mbar_arrive(&tile_free[tslot]);
+        if (++tslot == kTileSlots) {
+            tslot = 0;
+            tphase ^= 1;
+        }
+        return t;
+    };
+
     if (p.early_table) {
         if (warp == 0 && lane == 0 && p.mode == 0 && sched_id < total_tiles) {
             // weights of the first tile -> L2 while the predecessor's last tiles leave most SMs idle
@@ -394,6 +408,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 return t;
             };
             int drawn_tile = 0;
+            const uint32_t full_u32 = smem_u32(full), stage_u32 = smem_u32(stage_base);
             unsigned stage_rows = 0;  // four bits per stage: 32-row pieces of A that are not zero
             for (int tile = sched_id; tile < total_tiles && ok; tile = hand_out(tile, drawn_tile)) {
                 if (drawn && lane == 0) drawn_tile = atomicAdd(p.sched, 1);  // used when this tile's loads have been issued
@@ -429,6 +444,50 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 // zeros). One or two copies of 32 rows replace the copy of 128; with three or four the loading lane would fall behind.
                 const int valid_rows = max(1, ti.c_row_end - ti.a_row);
                 const int edge = (!kPair && p.mode == 0 && p.m_ends != nullptr && valid_rows <= 2 * kEdgeRows) ? (valid_rows + kEdgeRows - 1) / kEdgeRows : 0;
+                if constexpr (kFp8 && !kPair) {
+                    // The same for e4m3 operands with everything that does not change from one K block to the next in front of the loop: what the
+                    // loading lane needs per K block is part of every stage's round trip.
+                    const uint8_t* sfa = kMx ? p.sfa_atoms + (size_t)(ti.a_row >> 7) * (size_t)(p.k / 128) * 512 : nullptr;
+                    const uint8_t* sfb = kMx ? p.sfb_atoms + ((size_t)ti.group * (p.n / kBlockN) + ti.nt) * (size_t)(p.k / 128) * (512 * C::kSfBAtoms) : nullptr;
+                    const bool whole = edge == 0 && p.m_ends == nullptr;
+                    if (note != nullptr && lane == 0) s_prod_state[0] = 2;
+                    for (int kb = 0; kb < ti.num_kb; ++kb) {
+                        if (!__all_sync(0xffffffffu, mbar_wait(&empty[stage], phase ^ 1, abort_flag, limit, note, wait_id(1, tile, kb, stage)))) {
+                            ok = false;
+                            break;
+                        }
+                        int pieces = kBlockM / kEdgeRows;
+                        if (!whole) {
+                            // 32-row pieces of A to write: the valid ones, then pieces an earlier tile left in this stage (zeroed by copies from
+                            // past the last row, which touch no memory)
+                            const int filled = (int)(stage_rows >> (4 * stage)) & 7;
+                            if (edge != 0) pieces = max(edge, filled);
+                            stage_rows = (stage_rows & ~(7u << (4 * stage))) | ((unsigned)(edge == 0 ? kBlockM / kEdgeRows : edge) << (4 * stage));
+                        }
+                        if (elect_one()) {
+                            const uint32_t bar = full_u32 + stage * 8, sa = stage_u32 + stage * C::kStageBytes, sb = sa + kATileBytes;
+                            mbar_expect_tx_at(bar, C::kStageTxBytes - kATileBytes + pieces * (kEdgeRows * kKBlockBytes));
+                            tma_load_2d_at(&map_b, bar, sb, kb * 128, ti.b_row);
+                            if (kSwiGLU) tma_load_2d_at(&map_b, bar, sb + C::kBTileBytes / 2, kb * 128, ti.b_row2);
+                            if (edge == 0) tma_load_2d_at(&map_a, bar, sa, kb * 128, ti.a_row);
+                            else
+                                for (int j = 0; j < pieces; ++j)
+                                    tma_load_2d_at(&map_sfa, bar, sa + j * kEdgeRows * kKBlockBytes, kb * 128, j < edge ? ti.a_row + j * kEdgeRows : p.m_total);
+                            if constexpr (kMx) {
+                                // scale atoms: [row tile][K block][512] for A, [group][n tile][K block][512] for B
+                                bulk_load_1d_at(sb + C::kBTileBytes, sfa + kb * 512, 512, bar);
+                                bulk_load_1d_at(sb + C::kBTileBytes + 512, sfb + kb * (512 * C::kSfBAtoms), 512 * C::kSfBAtoms, bar);
+                            }
+                        }
+                        __syncwarp();
+                        if (issued < C::kStages) ++issued;
+                        if (++stage == C::kStages) {
+                            stage = 0;
+                            phase ^= 1;
+                        }
+                    }
+                    continue;
+                }
                 for (int kb = 0; kb < ti.num_kb; ++kb) {
                     if (lane == 0) s_prod_state[0] = 2;
                     if (!__all_sync(0xffffffffu, mbar_wait(&empty[stage], phase ^ 1, abort_flag, limit, note, wait_id(1, tile, kb, stage)))) {
@@ -535,7 +594,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         }
     } else if (warp == 1) {
         // ================= MMA issuer =================
-        if (cta_rank == 0) {
+        if (cta_rank == 0 && elect_one()) {
             const uint32_t idesc_full = kMx ? make_idesc_mx(kBlockN, C::kTileRows) : make_idesc<kFp8>(kBlockN, C::kTileRows, p.a_mn, p.b_mn);
             const uint32_t idesc_half = make_idesc<kFp8>(kBlockN / 2, C::kTileRows, p.a_mn, p.b_mn);
             // bytes (in 16-byte units) one K = 16 step moves the operand's start address: 32 B inside the swizzle atom when K
@@ -546,21 +605,21 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             int win = 0, win_phase = 0;  // accumulator window ring
             TileInfo ti;
             bool ok = true;
-            for (int tile = sched_id; tile < total_tiles && ok; tile = next_tile(tile)) {
+            for (int tile = sched_id; tile < total_tiles && ok; tile = next_tile_alone(tile)) {
                 decode(tile, g, ti);
                 if (ti.num_kb == 0) continue;  // epilogue writes zeros on its own
                 const uint32_t idesc = (C::kRagged && ti.n_cols != kBlockN) ? idesc_half : idesc_full;
                 for (int kb = 0; kb < ti.num_kb; ++kb) {
                     const bool new_window = C::kPromote ? true : (kb == 0);
                     if (new_window) {
-                        if (!__all_sync(0xffffffffu, mbar_wait(&tmem_empty[win], win_phase ^ 1, abort_flag, limit, note, wait_id(3, tile, kb, win)))) {
+                        if (!(mbar_wait(&tmem_empty[win], win_phase ^ 1, abort_flag, limit, note, wait_id(3, tile, kb, win)))) {
                             ok = false;
                             break;
                         }
                         tc_fence_after();
                     }
-                    if (!__all_sync(0xffffffffu, mbar_wait(&full[stage], phase, abort_flag, limit, note, wait_id(4, tile, kb, stage)))) {
-                        if (note != nullptr && lane == 0) atomicCAS(note + 1, 0ull, ((unsigned long long)s_prod_state[0] << 32) | (unsigned)s_prod_state[1]);
+                    if (!(mbar_wait(&full[stage], phase, abort_flag, limit, note, wait_id(4, tile, kb, stage)))) {
+                        if (note != nullptr) atomicCAS(note + 1, 0ull, ((unsigned long long)s_prod_state[0] << 32) | (unsigned)s_prod_state[1]);
                         ok = false;
                         break;
                     }
@@ -571,7 +630,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                     const uint64_t bdesc = p.b_mn ? make_smem_desc_mn(sb) : make_smem_desc(sb);
                     const uint32_t tmem_d = tmem_base + (uint32_t)(win * kBlockN);
                     const bool window_done = C::kPromote ? true : (kb == ti.num_kb - 1);
-                    if (elect_one()) {
+                    {
                         if constexpr (kMx) {
                             // scale atoms of this stage -> TMEM (alternating column sets), then four K=32 MMAs that read them
                             const uint32_t ssf = sb + C::kBTileBytes;
@@ -631,7 +690,6 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                             }
                         }
                     }
-                    __syncwarp();
                     sf_buf ^= 1;
                     if (window_done) {
                         if (++win == C::kWindows) {
@@ -646,6 +704,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 }
             }
         }
+        __syncwarp();
     } else {
         // ================= epilogue =================
         const int q = warp & 3;                    // TMEM lane quarter this warp may read
@@ -677,7 +736,81 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                     for (int c = 0; c < (C::kRagged ? ti.n_cols : C::kOutCols); c += 8) *reinterpret_cast<int4*>(zrow + c) = make_int4(0, 0, 0, 0);
                 continue;
             }
-            if constexpr (C::kPromote) {
+            if constexpr (C::kWidePromote) {
+                // 256 columns: a warp promotes 128 of them, with SwiGLU 64 gate columns and the matching up columns, else one scale block. A K
+                // block costs its hand-overs (stage, window, scales) once for twice the columns, and twice the weights are on their way.
+                const int num_kscales = p.k / 128, n_blocks = p.n / 128;
+                const int c0 = half * (kSwiGLU ? 64 : 128), c1 = kSwiGLU ? 128 + half * 64 : half * 128 + 64;
+                const float* sa_row = p.a_scales + (size_t)min(row, p.m_total - 1) * num_kscales;
+                const float* sb0 = p.b_scales + ((size_t)ti.group * n_blocks + ti.nblock + (kSwiGLU ? 0 : half)) * num_kscales;
+                const float* sb1 = p.b_scales + ((size_t)ti.group * n_blocks + ti.nblock2) * num_kscales;
+                const bool warp_has_rows = ti.c_row + q * 32 < ti.c_row_end;  // else it only keeps the windows moving
+                float acc[2][64];
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+#pragma unroll
+                    for (int i = 0; i < 64; ++i) acc[h][i] = 0.f;
+                float n_a = 0.f, n_0 = 0.f, n_1 = 0.f;
+                auto fetch_scales = [&](int kb) {
+                    if (kb >= ti.num_kb || !warp_has_rows) return;
+                    n_a = __ldcg(sa_row + kb);
+                    n_0 = __ldg(sb0 + kb);
+                    if (kSwiGLU) n_1 = __ldg(sb1 + kb);
+                };
+                if (p.ready == nullptr) fetch_scales(0);  // (with arrival gating the rows' scales are there after the first wait: see below)
+                for (int kb = 0; kb < ti.num_kb; ++kb) {
+                    if (!mbar_wait(&tmem_full[win], win_phase, abort_flag, limit, note, wait_id(5, tile, kb, warp))) {
+                        ok = false;
+                        break;
+                    }
+                    if (kb == 0 && p.ready != nullptr) fetch_scales(0);
+                    if (warp_has_rows) {
+                        tc_fence_after();
+                        const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(win * kBlockN);
+                        const float s0 = n_a * n_0, s1 = kSwiGLU ? n_a * n_1 : s0;
+                        fetch_scales(kb + 1);
+#pragma unroll
+                        for (int c = 0; c < 8; ++c) {
+                            uint32_t v[16];
+                            tmem_ld16(taddr + (c < 4 ? c0 + c * 16 : c1 + (c - 4) * 16), v);
+                            tmem_ld_wait();
+                            if (c == 7) {
+                                tc_fence_before();
+                                __syncwarp();
+                                if (lane == 0) release_window(&tmem_empty[win]);
+                            }
+#pragma unroll
+                            for (int i = 0; i < 16; ++i) acc[c / 4][(c & 3) * 16 + i] = fmaf(__uint_as_float(v[i]), c < 4 ? s0 : s1, acc[c / 4][(c & 3) * 16 + i]);
+                        }
+                    } else {
+                        __syncwarp();
+                        if (lane == 0) release_window(&tmem_empty[win]);
+                    }
+                    if (++win == C::kWindows) {
+                        win = 0;
+                        win_phase ^= 1;
+                    }
+                }
+                if (!ok) break;
+                const int rows_valid = min(32, ti.c_row_end - (ti.c_row + q * 32));
+                __nv_bfloat16* wbase = cbase + (size_t)(ti.c_row + q * 32) * ldc + ti.c_col;
+                if (rows_valid > 0) {
+#pragma unroll
+                    for (int c = 0; c < (kSwiGLU ? 64 : 128); c += 32) {
+                        int4 regs[4];
+#pragma unroll
+                        for (int i = 0; i < 32; i += 8) {
+                            float o[8];
+#pragma unroll
+                            for (int j = 0; j < 8; ++j) o[j] = kSwiGLU ? silu(acc[0][(c + i + j) & 63]) * acc[1][(c + i + j) & 63] : acc[c / 64][(c + i + j) & 63];
+                            regs[i / 8] = pack8_bf16(o);
+                        }
+                        const int col = half * (kSwiGLU ? 64 : 128) + c;
+                        if (scatter) store_block_scattered<32>(out_stage, regs, scat_ptr != nullptr ? scat_ptr + col : nullptr, lane);
+                        else store_block_coalesced<32>(out_stage, regs, wbase + col, ldc, rows_valid, lane);
+                    }
+                }
+            } else if constexpr (C::kPromote) {
                 // One window per K block, promoted into fp32 registers with the two scales. A warp owns two 32-column
                 // chunks: with SwiGLU a gate chunk and the matching up chunk, otherwise two neighbouring chunks.
                 constexpr int kLo0 = 0, kHalfCols = kBlockN / 2;
@@ -1090,6 +1223,16 @@ cudaError_t launch_sel(const GroupedGemmArgs& a, cudaStream_t stream) {
     return launch_impl<kBlockN, kFp8, kSwiGLU, false>(a, stream);
 }
 
+// Whether FP8 with fp32 scales takes tiles of 256 columns, `col_tiles` to a row tile. A K block of such a tile takes 1.6 times that of one with 128
+// columns, so it pays unless twice as many tiles fill the SMs that much better. Both products, us, 128 / 256 columns: 64 experts of 4096 -> 1408 with 4 rows
+// 184 + 88 / 141 + 71, 73 rows 199 + 94 / 160 + 85, 768 rows 994 + 502 / 777 + 427; 32 of 2304 -> 1792, 200 rows 177 + 65 / 125 + 56; 8 of 7168 -> 2048, 100
+// rows 68 + 39 / 55 + 38; 16 of 1024 -> 640, 300 rows, where the second has 192 tiles: 35 + 15.5 / 27 + 17.9.
+bool wide_promotion(const GroupedGemmArgs& a, int col_tiles) {
+    if (a.cta_pairs) return false;
+    const long long tiles = ((long long)a.m_total + kBlockM - 1) / kBlockM * col_tiles, sms = a.num_sms;
+    return 8 * ((tiles + sms - 1) / sms) < 5 * ((2 * tiles + sms - 1) / sms);
+}
+
 }  // namespace
 
 cudaError_t launch_grouped_gemm(const GroupedGemmArgs& a, cudaStream_t stream) {
@@ -1119,9 +1262,11 @@ cudaError_t launch_grouped_gemm(const GroupedGemmArgs& a, cudaStream_t stream) {
             if (a.a_scales == nullptr || a.b_scales == nullptr || a.k % 128 != 0) return cudaErrorInvalidValue;
             if (a.swiglu) {
                 if ((a.n / 2) % 128 != 0) return cudaErrorInvalidValue;  // gate/up halves must start on scale-block boundaries
+                if (wide_promotion(a, a.n / 256)) return launch_impl<256, true, true, false>(a, stream);
                 return launch_sel<128, true, true>(a, stream);
             }
             if (a.n % 128 != 0) return cudaErrorInvalidValue;
+            if (a.n % 256 == 0 && !a.scatter_to_peers && wide_promotion(a, a.n / 256)) return launch_impl<256, true, false, false>(a, stream);
             return launch_sel<128, true, false>(a, stream);
         }
         if (a.swiglu) {

@@ -102,3 +102,65 @@ def test_weight_gradient_stops_at_the_last_row(monkeypatch, N, K, pair):
             assert (dw[g] == 0).all()
         else:
             _close(dw[g], dy[r].float().t() @ x[r].float())
+
+
+@pytest.mark.parametrize("swiglu,K,N", [(True, 128, 256), (True, 640, 768), (False, 384, 256), (False, 1280, 512)])
+@pytest.mark.parametrize("masked", [False, True])
+def test_promotion_with_256_columns_equals_128(swiglu, K, N, masked):
+    """FP8 with fp32 scales: few SMs make the wide tiles the better choice, all of them the narrow ones. Both add the K blocks in the same order
+    with the same fused multiply-adds, so the results are the same bit for bit; rows on both sides of a warp's 32 and of a tile's 128."""
+    from deepep_efa_b200 import _ext
+    from deepep_efa_b200.ops.grouped_gemm import reference_grouped_gemm
+    C = _ext.load()
+    C.gemm_clear_error(0)
+    torch.manual_seed(N)
+    rows = [1, 31, 33, 0, 127, 128, 129, 200]
+    starts, ends = _groups(rows, True)
+    G, M = len(rows), starts[-1]
+    a = torch.randn(M, K, device="cuda").to(torch.float8_e4m3fn)
+    b = torch.randn(G, N, K, device="cuda").to(torch.float8_e4m3fn)
+    a_s, b_s = torch.rand(M, K // 128, device="cuda") + 0.1, torch.rand(G, N // 128, K // 128, device="cuda") * 0.1
+    kw = dict(m_ends=_i32(ends)) if masked else {}
+    width = N // 2 if swiglu else N
+    outs = []
+    for sms in (1, 3, 0):
+        out = torch.full((M, width), 7.0, dtype=torch.bfloat16, device="cuda")
+        outs.append(C.grouped_gemm(a, b, _i32(starts), 0, swiglu, a_s, b_s, out, sms, **kw))
+    torch.cuda.synchronize()
+    assert C.gemm_error(0) == 0
+    assert torch.equal(outs[0], outs[2]) and torch.equal(outs[1], outs[2])
+    ref = reference_grouped_gemm(a, b, _i32(starts), swiglu=swiglu, a_scales=a_s, b_scales=b_s)
+    for g in range(G):
+        if rows[g]:
+            # exact products of e4m3 values, fp32 sums and scales, one rounding to bf16
+            _close(outs[0][starts[g]:ends[g]], ref[starts[g]:ends[g]])
+        if masked:
+            assert (outs[0][ends[g]:starts[g + 1]] == 7.0).all()
+
+
+@pytest.mark.parametrize("N", [256, 768])
+def test_promotion_with_256_columns_scatters_rows(N):
+    from deepep_efa_b200 import _ext
+    C = _ext.load()
+    C.gemm_clear_error(0)
+    torch.manual_seed(3)
+    rows, K = [40, 130, 0, 65], 512
+    starts, ends = _groups(rows, True)
+    M, valid = starts[-1], sum(rows)
+    a = torch.randn(M, K, device="cuda").to(torch.float8_e4m3fn)
+    b = torch.randn(len(rows), N, K, device="cuda").to(torch.float8_e4m3fn)
+    a_s, b_s = torch.rand(M, K // 128, device="cuda") + 0.1, torch.rand(len(rows), N // 128, K // 128, device="cuda") * 0.1
+    where, order = torch.full((M,), -1, dtype=torch.int32), torch.randperm(valid)
+    at = torch.cat([torch.arange(starts[g], ends[g]) for g in range(len(rows))])
+    where[at] = order.to(torch.int32)
+    where[at[::7]] = -1  # dropped rows
+    dst = torch.full((valid, N), 7.0, dtype=torch.bfloat16, device="cuda")
+    bases = torch.tensor([dst.data_ptr()], dtype=torch.int64, device="cuda")
+    plain = C.grouped_gemm(a, b, _i32(starts), 0, False, a_s, b_s)
+    C.grouped_gemm(a, b, _i32(starts), 0, False, a_s, b_s, None, 2, 2000.0, _i32(ends), row_info=where.cuda(), scatter_bases=bases)
+    torch.cuda.synchronize()
+    assert C.gemm_error(0) == 0
+    want = torch.full_like(dst, 7.0)
+    keep = where[at] >= 0
+    want[where[at][keep].long().cuda()] = plain[at[keep].cuda()]
+    assert torch.equal(dst, want)
