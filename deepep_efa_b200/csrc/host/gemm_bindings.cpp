@@ -166,13 +166,15 @@ torch::Tensor grouped_gemm(const torch::Tensor& a, const torch::Tensor& b, const
         if (forced) p.cta_pairs = pr[0] == '1';
         else if (!fp8 && mode == 1) p.cta_pairs = !mn_major || rows >= 480;
         else if (!fp8 && p.m_ends == nullptr) p.cta_pairs = (rows >= 224 && rows <= 270) || rows >= 430;
-        // Forward and input gradients in BF16: tokens as columns on CTA pairs, from 160 padded rows per expert on. One tile of rows of the other form is
-        // as good as a tile of columns (64 experts of 4096 -> 1408, 94 rows: 765 and 774 us; 128 of 2048 -> 512, 100 rows: 345 and 365); with more than one it is not
-        // (gemm_pairs.cu has both sides).
+        // Forward and input gradients in BF16: tokens as columns on CTA pairs, in tiles of up to 256 of them from 160 padded rows per expert on (gemm_pairs.cu has
+        // both sides), below it of up to 128, which leaves room for eight stages instead of six; but with one tile of rows per expert and few K blocks
+        // the other form's epilogue, which turns nothing over, is the better one. All four products of a layer in a loop, rows / columns, us: 64 experts of 4096 -> 1408
+        // with 5 rows 759 / 717, 20 rows 786 / 730, 60 rows 793 / 765, 94 rows 814 / 806, 110 rows 847 / 851; 60 of 2304 -> 640, 30 rows 247 / 222; single products,
+        // 100 rows: 128 of 2048 -> 512: K 2048 107.2 / 104.1, K 1024 100.7 / 103.4, K 512 60.1 / 67.9; 90 rows: K 640 41.6 / 44.4, K 1280 69.1 / 71.0.
         if (mode == 0 && !fp8 && !swiglu && p.num_sms >= 2 && p.n % 128 == 0 && p.k % 64 == 0 && !ready.has_value() && !expected.has_value() && !row_info.has_value() &&
             !trace.has_value() && !sched.has_value() && !early_table && !hold_successor) {
-            p.token_pairs = forced ? p.cta_pairs : rows >= 160;
-            p.token_cap = 256;
+            p.token_pairs = forced ? p.cta_pairs : (rows >= 160 || p.k >= 1024);
+            p.token_cap = rows >= 160 ? 256 : 128;
         }
         if (mode == 0 && !swiglu && !fp8) p.cta_pairs = 0;
         // A weight gradient with about a tile of rows per expert is bound by what happens per tile; leaving out steps of its two K blocks cost more than it
