@@ -316,8 +316,7 @@ token_cols_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
                     tmem_cp_sf(t_sfw + 4, make_sf_desc(ssf + 512));
                     tmem_cp_sf(t_sfw + 8, make_sf_desc(ssf + 1024));
                     if (two_atoms) tmem_cp_sf(t_sfw + 12, make_sf_desc(ssf + 1536));
-                    // The two products take turns: an MMA of so few columns ends long before the next one may add to the same accumulator
-                    // (144 tokens, no copies in flight: both GEMMs of 256 experts 2870 -> 1670 us; with the copies 2210 -> 2165).
+                    // The two products take turns (144 tokens, both GEMMs of 256 experts: 2210 -> 2165 us).
 #pragma unroll
                     for (int j = 0; j < 4; ++j)
 #pragma unroll
