@@ -989,17 +989,19 @@ __global__ void __launch_bounds__(kLLThreads, 1) combine_pull(const __grid_const
 // the same exception, the received rows themselves): the dispatch raises the parity's in-flight word by its number of CTAs before any of them
 // allows this launch, and each takes one off as its last act, so the word is zero whenever a kernel that waits for its own predecessor came
 // in between. Only reads happen early; results are stored after the predecessor has completed, because their memory may be a block that the
-// predecessor still reads (freed by the caller between the two calls). The successor is released only then: the next dispatch's CTAs, launched at
-// this kernel's start, took the places of CTAs of both kernels that still had work (128 tokens of 7168, 256 experts, top-8, FP8, launched one by
-// one: pair of dispatch and combine 15.1 -> 12.1 us; 33 tokens of 6144 in a graph, two pairs 14.3 -> 12.9; shapes whose CTAs are few: the same).
-// With kFind, which gathers nothing early, it made no difference, and the release stays in front.
+// predecessor still reads (freed by the caller between the two calls). The successor is released only then, where this kernel has
+// more than a CTA per SM: the next dispatch's CTAs, launched at its start, took the places of CTAs of both kernels that still had work (128 tokens of 7168, 256 experts, top-8, FP8, launched one by
+// one: pair of dispatch and combine 15.1 -> 12.1 us; 33 tokens of 6144 in a graph, two pairs 14.3 -> 12.9). With fewer CTAs nobody's place is taken, and
+// the early launch is worth a little (30 tokens of 2944, top-2, in a graph: 12.4, late 12.8). With kFind, which gathers nothing early, it made no
+// difference, and the release stays in front.
 // kFind (x is an ordinary tensor): whatever launched in between may still be writing x, so the predecessor's end comes first, as for the
 // staged form. src_info decides which row of the expert is the token's, so that the selections of a token may come in another order than at
 // the dispatch, as there too. It is loaded with the row itself; the search is for the odd case.
 // (Two CTAs of 512 threads to an SM: the 64 registers that leaves let the 896 CTAs of 128 threads of 128 tokens x 7168 be resident at once.)
 template <bool kFind>
 __global__ void __launch_bounds__(kLLThreads, 2) combine_lone(const __grid_constant__ LLCombineArgs a, const int slices) {
-    if constexpr (kFind) pdl_release_successor();
+    const bool release_first = kFind || gridDim.x <= kNumSms;
+    if (release_first) pdl_release_successor();
     const RankCtx& c = a.ctx;
     const int T = a.num_tokens, K = a.num_topk, E = a.num_experts, N = a.num_max_tokens, n16 = a.hidden / 8;
     const int tid = threadIdx.x, lane = tid & 31;
@@ -1013,7 +1015,7 @@ __global__ void __launch_bounds__(kLLThreads, 2) combine_lone(const __grid_const
     }
     if (!early) {
         pdl_wait_predecessor();
-        if constexpr (!kFind) pdl_release_successor();
+        if (!release_first) pdl_release_successor();
     }
     const int tag = ll_count_tag(*reinterpret_cast<volatile uint64_t*>(c.seq + kLLStartedWord0 + a.parity));
     const bool masked = __ldcg(&c.my_ctrl()->ll_mask[0]) != 0;
@@ -1075,7 +1077,7 @@ __global__ void __launch_bounds__(kLLThreads, 2) combine_lone(const __grid_const
             }
             if (early) {  // from here on everything is final; both return at once from the second token on
                 pdl_wait_predecessor();
-                pdl_release_successor();
+                if (!release_first) pdl_release_successor();
             }
             if (sure) break;
             const bool wrong = e >= 0 && (slot < 0 || info != t || slot - e * N >= rows);
