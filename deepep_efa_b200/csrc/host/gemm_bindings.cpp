@@ -5,6 +5,7 @@
 #include <pybind11/stl.h>
 #include <torch/extension.h>
 
+#include <algorithm>
 #include <map>
 #include <mutex>
 
@@ -66,7 +67,7 @@ torch::Tensor grouped_gemm(const torch::Tensor& a, const torch::Tensor& b, const
                            c10::optional<torch::Tensor> row_info, c10::optional<torch::Tensor> scatter_bases,
                            c10::optional<torch::Tensor> trace, bool mn_major, c10::optional<torch::Tensor> out_fp8,
                            c10::optional<torch::Tensor> out_atoms, bool m_ends_are_counts, c10::optional<torch::Tensor> sched, bool early_table, int tokens_as_columns,
-                           bool hold_successor, bool zero_tail) {
+                           bool hold_successor, bool zero_tail, int64_t rows_hint) {
     DXG_CHECK(a.is_cuda() && b.is_cuda() && m_offsets.is_cuda(), "operands must be CUDA tensors");
     DXG_CHECK(a.is_contiguous() && b.is_contiguous() && m_offsets.is_contiguous(), "operands must be contiguous");
     DXG_CHECK(m_offsets.scalar_type() == torch::kInt32 && m_offsets.dim() == 1 && m_offsets.numel() >= 2, "m_offsets must be int32 [G+1]");
@@ -153,6 +154,7 @@ torch::Tensor grouped_gemm(const torch::Tensor& a, const torch::Tensor& b, const
         p.m_ends_are_counts = m_ends_are_counts ? 1 : 0;
     }
     DXG_CHECK(!zero_tail || (mode == 0 && !fp8 && !swiglu && p.m_ends != nullptr), "zero_tail needs m_ends (M-grouped mode, bf16, no swiglu)");
+    p.rows_hint = (int)std::min<int64_t>(std::max<int64_t>(rows_hint, 0), p.m_total);
     p.num_sms = num_sms > 0 ? num_sms : sm_count(device);
     {
         const char* o = std::getenv("DEEPEP_GEMM_ORDER");
@@ -414,9 +416,9 @@ torch::Tensor fp8_experts(const torch::Tensor& a, const torch::Tensor& a_scales,
     const torch::Tensor a_atoms = build_sf_atoms_a(a_scales, none, 0);
     const torch::Tensor h = torch::empty({a.size(0), inter}, a.options()), h_atoms = torch::empty({a.size(0) / 128, inter / 128, 512}, a_atoms.options());
     grouped_gemm(a, w13, m_offsets, 0, true, none, none, none, 0, timeout_ms, m_ends, a_atoms, atoms13, none, none, none, none, none, false, h, h_atoms, false, none,
-                 false, tokens_as_columns, false, false);
+                 false, tokens_as_columns, false, false, 0);
     return grouped_gemm(h, w2, m_offsets, 0, false, none, none, none, 0, timeout_ms, m_ends, h_atoms, atoms2, none, none, none, none, none, false, none, none, false, none,
-                        false, tokens_as_columns, false, false);
+                        false, tokens_as_columns, false, false, 0);
 }
 
 void bind_gemm(py::module_& m) {
@@ -433,7 +435,7 @@ void bind_gemm(py::module_& m) {
           py::arg("ready") = py::none(), py::arg("expected") = py::none(), py::arg("row_info") = py::none(),
           py::arg("scatter_bases") = py::none(), py::arg("trace") = py::none(), py::arg("mn_major") = false,
           py::arg("out_fp8") = py::none(), py::arg("out_atoms") = py::none(), py::arg("m_ends_are_counts") = false, py::arg("sched") = py::none(),
-          py::arg("early_table") = false, py::arg("tokens_as_columns") = 0, py::arg("hold_successor") = false, py::arg("zero_tail") = false);
+          py::arg("early_table") = false, py::arg("tokens_as_columns") = 0, py::arg("hold_successor") = false, py::arg("zero_tail") = false, py::arg("rows_hint") = 0);
     m.def("fp8_experts", &fp8_experts);
     m.def("build_plan", &build_plan);
     m.def("gather_rows", &gather_rows, py::arg("src"), py::arg("src_row"), py::arg("scale") = py::none(), py::arg("out") = py::none());

@@ -307,10 +307,11 @@ class MoELayer(nn.Module):
             C.grouped_gemm(w_["hq"], w2, w_["starts"], 0, False, None, None, y.view(L * N, H), 0, GEMM_TIMEOUT_MS, cnt, w_["ha"], mx[3],
                            m_ends_are_counts=True, sched=w_["sched"], early_table=True, tokens_as_columns=columns)
         else:
-            C.grouped_gemm(a, w13, w_["starts"], 0, True, a_s, s13, w_["h"], 0, GEMM_TIMEOUT_MS, cnt, m_ends_are_counts=True, sched=w_["sched"])
+            arriving = max(1, R * x.size(0) * cfg.num_topk * L // cfg.num_experts)  # rows, on average
+            C.grouped_gemm(a, w13, w_["starts"], 0, True, a_s, s13, w_["h"], 0, GEMM_TIMEOUT_MS, cnt, m_ends_are_counts=True, sched=w_["sched"], rows_hint=arriving)
             C.per_token_cast_to_fp8(w_["h"], False, False, cnt, N, w_["hq"], w_["hs"])
             C.grouped_gemm(w_["hq"], w2, w_["starts"], 0, False, w_["hs"], s2, y.view(L * N, H), 0, GEMM_TIMEOUT_MS, cnt, m_ends_are_counts=True, sched=w_["sched"],
-                           early_table=True)
+                           early_table=True, rows_hint=arriving)
         out, _, _ = buf.low_latency_combine(y, topk_idx, topk_weights, handle, zero_copy=True)
         return out
 
@@ -498,7 +499,7 @@ def fused_forward_many(layers, xs, idxs, ws, overlap: bool = True, num_dispatch_
         for pi, (g0, ng, sms1) in enumerate(parts):
             tr = None if (w.trace is None or pi > 0) else w.trace[2:6]
             # what follows a part that leaves SMs to the dispatch must not take them early, while that part still waits for rows
-            gate = dict(trace=tr, sched=w.sched, early_table=not overlapped, hold_successor=sms1 > 0)
+            gate = dict(trace=tr, sched=w.sched, early_table=not overlapped, hold_successor=sms1 > 0, rows_hint=w.num_tokens * K * ng // L)
             if not lone:
                 # (a lone rank's rows are in place when its dispatch has run, which this stream already waits for. The words are the
                 # buffer's: the next call of another layer on another stream raises what is expected, and a GEMM on every SM that
