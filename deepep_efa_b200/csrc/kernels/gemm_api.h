@@ -64,7 +64,7 @@ struct GroupedGemmArgs {
     int scatter_to_peers;     // 1 = some of them are other GPUs': pieces of a row should be long (FP8 with fp32 scales keeps tiles that store 128 bytes)
     unsigned long long* trace;  // optional [4]: earliest first-tile load / latest epilogue end (global timer, ns) / first wait that
                                 // gave up (role << 56 | tile << 24 | k block << 8 | slot; 0 = none) / what the loader was doing
-                                // then (state << 32 | tile; state 1 = arrival gate, 2 = waiting for a free stage, 3 = loads issued)
+                                // then (state << 32 | tile; state 1 = arrival gate, 2 = waiting for a free stage, 3 = loads issued; e4m3 single CTAs: 2 from a tile's first wait on)
     // MN-major operands (bf16, no swiglu): the operand is read from a tensor whose contiguous dimension is the operand's row
     // index instead of K, so gradients need no transposed copies. mode 0: b_mn = 1, B given as [G, K, N] (input gradients:
     // the forward weight as it is). mode 1: a_mn = b_mn = 1, A given as [M_total, N_out], B as [M_total, K_out] (weight

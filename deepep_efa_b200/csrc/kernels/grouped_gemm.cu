@@ -3,7 +3,7 @@
 // persistent warp-specialised CTA per SM.
 //
 //   warp 0   : TMA producer   (one elected lane issues)  global -> smem ring, mbarrier complete_tx
-//   warp 1   : MMA issuer     (one elected lane issues)  tcgen05.mma, tcgen05.commit frees smem stages and publishes
+//   warp 1   : MMA issuer     (one elected thread)  tcgen05.mma, tcgen05.commit frees smem stages and publishes
 //                                         accumulator windows; also owns TMEM alloc / dealloc
 //   warps 2.. : epilogue (4 warps for BF16, 8 for FP8)  tcgen05.ld -> registers -> (scale | SwiGLU) -> BF16 ->
 //                                         per-warp smem transpose -> coalesced global stores
@@ -533,14 +533,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                     stage_rows = (stage_rows & ~(7u << (4 * stage))) | ((unsigned)(edge == 0 ? kBlockM / kEdgeRows : edge) << (4 * stage));
                     if (elect_one()) {
                         mbar_expect_tx(&full[stage], C::kStageTxBytes - kATileBytes + pieces * kEdgeRows * kKBlockBytes);
-                        if constexpr (kMx) {
-                            // scale atoms: [row tile][K block][512] for A, [group][n tile][K block][512] for B
-                            uint8_t* ssf = sb + C::kBTileBytes;
-                            const size_t nkb = (size_t)(p.k / 128);
-                            bulk_load_1d(ssf, p.sfa_atoms + ((size_t)(ti.a_row >> 7) * nkb + kb) * 512, 512, &full[stage]);
-                            bulk_load_1d(ssf + 512, p.sfb_atoms + (((size_t)ti.group * (p.n / kBlockN) + ti.nt) * nkb + kb) * (512 * C::kSfBAtoms),
-                                         512 * C::kSfBAtoms, &full[stage]);
-                        }
+                        // (BF16 from here on)
                         if (kMnMajor && p.a_mn) tma_load_3d(&map_a, &full[stage], sa, ti.a_kbase + kb * 64, ti.a_mn0 / 64);
                         else if (edge == 0) tma_load_2d(&map_a, &full[stage], sa, ti.a_k0 + kb * elem_per_kb, ti.a_row);
                         else
