@@ -499,7 +499,7 @@ def fused_forward_many(layers, xs, idxs, ws, overlap: bool = True, num_dispatch_
         for pi, (g0, ng, sms1) in enumerate(parts):
             tr = None if (w.trace is None or pi > 0) else w.trace[2:6]
             # what follows a part that leaves SMs to the dispatch must not take them early, while that part still waits for rows
-            gate = dict(trace=tr, sched=w.sched, early_table=not overlapped, hold_successor=sms1 > 0, rows_hint=w.num_tokens * K * ng // L)
+            gate = dict(trace=tr, sched=w.sched, early_table=not overlapped, hold_successor=sms1 > 0, rows_hint=max(1, w.num_tokens * K * ng // L))
             if not lone:
                 # (a lone rank's rows are in place when its dispatch has run, which this stream already waits for. The words are the
                 # buffer's: the next call of another layer on another stream raises what is expected, and a GEMM on every SM that
@@ -523,7 +523,7 @@ def fused_forward_many(layers, xs, idxs, ws, overlap: bool = True, num_dispatch_
         else:
             C.per_token_cast_to_fp8(w.h, False, False, None, 1, w.hq, w.hs, w.m_offsets[L:], False)
             C.grouped_gemm(w.hq, w2, w.m_offsets, 0, False, w.hs, s2, None, 0, GEMM_TIMEOUT_MS, w.m_ends, None, None,
-                           row_info=w.recv_info, scatter_bases=w.peer_bases[3 * R_:], sched=w.sched, early_table=True)
+                           row_info=w.recv_info, scatter_bases=w.peer_bases[3 * R_:], sched=w.sched, early_table=True, rows_hint=max(1, w.num_tokens * K))
     # every rank's second GEMM has finished scattering before anybody sums its stage
     if not lone:
         C.barrier(rts)

@@ -246,3 +246,30 @@ def test_fused_forward_with_tokens_as_columns(monkeypatch, R, T):
             assert _rel(got[r], ref) < 8e-2  # as in the test of the whole pipeline above
     finally:
         vc.destroy()
+
+
+@pytest.mark.parametrize("R,T", [(1, 9), (2, 40)])
+def test_fused_products_say_how_many_rows_come(monkeypatch, R, T):
+    """The workspace has room for many more rows than come, and FP8 with fp32 scales chooses its tiles by their number: both products name it."""
+    from deepep_efa_b200.models import moe
+    E, K, I = 16, 2, 384
+    vc, layers, xs, idxs, ws = _setup(R, T, 512, I, E, K, native=False)
+    try:
+        C, hints = layers[0]._C(), []
+
+        class Recorder:
+            def __getattr__(self, name):
+                return getattr(C, name)
+
+            def grouped_gemm(self, a, b, *args, **kw):
+                hints.append((b.size(0), b.size(1) == 2 * I, kw.get("rows_hint")))
+                return C.grouped_gemm(a, b, *args, **kw)
+
+        monkeypatch.setattr(moe.MoELayer, "_C", staticmethod(lambda: Recorder()))
+        moe.fused_forward_many(layers, xs, idxs, ws, overlap=False)
+        torch.cuda.synchronize()
+        assert len(hints) == 2 * R and {swiglu for _, swiglu, _ in hints} == {True, False}
+        for groups, _, hint in hints:
+            assert hint == T * K * groups // (E // R)
+    finally:
+        vc.destroy()
