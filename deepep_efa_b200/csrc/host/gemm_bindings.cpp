@@ -10,6 +10,7 @@
 #include <mutex>
 
 #include "../kernels/gemm_api.h"
+#include "../kernels/gemm_choice.h"
 
 namespace py = pybind11;
 
@@ -421,7 +422,24 @@ torch::Tensor fp8_experts(const torch::Tensor& a, const torch::Tensor& a_scales,
                         false, tokens_as_columns, false, false, 0);
 }
 
+// What the rules of gemm_choice.h say about a product of these sizes (for the tests: they need no GPU). ends: whether m_ends is given.
+int promotion_columns(int64_t rows, int64_t groups, int64_t n, int64_t k, bool swiglu, bool ends, int64_t rows_hint, int num_sms) {
+    dx::GroupedGemmArgs p{};
+    const int there = 0;
+    p.m_total = (int)rows;
+    p.num_groups = (int)groups;
+    p.n = (int)n;
+    p.k = (int)k;
+    p.swiglu = swiglu ? 1 : 0;
+    p.m_ends = ends ? &there : nullptr;
+    p.rows_hint = (int)rows_hint;
+    p.num_sms = num_sms;
+    return dx::wide_promotion(p) ? 256 : 128;
+}
+
 void bind_gemm(py::module_& m) {
+    m.def("promotion_columns", &promotion_columns, py::arg("rows"), py::arg("groups"), py::arg("n"), py::arg("k"), py::arg("swiglu") = false, py::arg("ends") = false,
+          py::arg("rows_hint") = 0, py::arg("num_sms") = 148);
     m.def("build_sf_atoms_a", &build_sf_atoms_a, py::arg("scales"), py::arg("group_counts") = py::none(), py::arg("rows_per_group") = 0);
     m.def("build_sf_atoms_b", &build_sf_atoms_b, py::arg("scales"), py::arg("n"), py::arg("swiglu") = false, py::arg("wide") = false);
     m.def("transpose_bf16", &transpose_bf16);

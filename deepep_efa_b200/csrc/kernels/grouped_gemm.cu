@@ -19,10 +19,9 @@
 // loops, TMEM is released and the kernel returns.
 //
 // The reference has no GEMM: its users run their expert FFN between dispatch and combine themselves.
-#include <algorithm>
-#include <cmath>
 #include <cstring>
 
+#include "gemm_choice.h"
 #include "launch.cuh"
 #include "tc_prims.cuh"
 
@@ -1218,22 +1217,6 @@ cudaError_t launch_sel(const GroupedGemmArgs& a, cudaStream_t stream) {
     return launch_impl<kBlockN, kFp8, kSwiGLU, false>(a, stream);
 }
 
-// Whether FP8 with fp32 scales takes tiles of 256 columns, `col_tiles` to a row tile. A K block of such a tile takes 1.6 times that of one with 128
-// columns, so it pays unless twice as many tiles fill the SMs that much better. Both products, us, 128 / 256 columns: 64 experts of 4096 -> 1408 with 4 rows
-// 184 + 88 / 141 + 71, 73 rows 199 + 94 / 160 + 85, 768 rows 994 + 502 / 777 + 427; 32 of 2304 -> 1792, 200 rows 177 + 65 / 125 + 56; 8 of 7168 -> 2048, 100
-// rows 68 + 39 / 55 + 38; 16 of 1024 -> 640, 300 rows, where the second has 192 tiles: 35 + 15.5 / 27 + 17.9. A decode layout has room for many more rows than
-// come, so its caller says how many do (a step of the layer with 3 of 256 experts of 2048 -> 896 in use, 128 / 256 columns: 61 / 72 us).
-bool wide_promotion(const GroupedGemmArgs& a, int col_tiles) {
-    if (a.cta_pairs) return false;
-    long long row_tiles = ((long long)a.m_total + kBlockM - 1) / kBlockM;
-    if (a.rows_hint > 0) {
-        const double groups = a.num_groups, used = groups * (1.0 - std::exp(-a.rows_hint / groups));  // that get a row
-        row_tiles = std::min<long long>(row_tiles, a.rows_hint / kBlockM + (long long)(used + 0.5));
-    }
-    const long long tiles = row_tiles * col_tiles, sms = a.num_sms;
-    return 8 * ((tiles + sms - 1) / sms) < 5 * ((2 * tiles + sms - 1) / sms);
-}
-
 }  // namespace
 
 cudaError_t launch_grouped_gemm(const GroupedGemmArgs& a, cudaStream_t stream) {
@@ -1263,11 +1246,11 @@ cudaError_t launch_grouped_gemm(const GroupedGemmArgs& a, cudaStream_t stream) {
             if (a.a_scales == nullptr || a.b_scales == nullptr || a.k % 128 != 0) return cudaErrorInvalidValue;
             if (a.swiglu) {
                 if ((a.n / 2) % 128 != 0) return cudaErrorInvalidValue;  // gate/up halves must start on scale-block boundaries
-                if (wide_promotion(a, a.n / 256)) return launch_impl<256, true, true, false>(a, stream);
+                if (wide_promotion(a)) return launch_impl<256, true, true, false>(a, stream);
                 return launch_sel<128, true, true>(a, stream);
             }
             if (a.n % 128 != 0) return cudaErrorInvalidValue;
-            if (a.n % 256 == 0 && !a.scatter_to_peers && wide_promotion(a, a.n / 256)) return launch_impl<256, true, false, false>(a, stream);
+            if (!a.scatter_to_peers && wide_promotion(a)) return launch_impl<256, true, false, false>(a, stream);
             return launch_sel<128, true, false>(a, stream);
         }
         if (a.swiglu) {

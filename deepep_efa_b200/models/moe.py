@@ -230,6 +230,7 @@ class MoELayer(nn.Module):
                 hq, hs = C.per_token_cast_to_fp8(h, True, False)
                 y_perm = C.grouped_gemm(hq, w2, plan.m_offsets, 0, False, sfa_atoms=gg.build_sf_atoms_a(hs), sfb_atoms=mx[1], **how)
         else:
+            how["rows_hint"] = plan.num_rows  # its row tiles are all in use
             h = C.grouped_gemm(a, w13, plan.m_offsets, 0, True, a_s, s13, **how)
             hq, hs = C.per_token_cast_to_fp8(h, False, False)
             y_perm = C.grouped_gemm(hq, w2, plan.m_offsets, 0, False, hs, s2, **how)

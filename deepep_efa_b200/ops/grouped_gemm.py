@@ -23,18 +23,21 @@ from .. import _ext
 def grouped_gemm(a: torch.Tensor, b: torch.Tensor, m_offsets: torch.Tensor, *, swiglu: bool = False,
                  a_scales: Optional[torch.Tensor] = None, b_scales: Optional[torch.Tensor] = None,
                  out: Optional[torch.Tensor] = None, num_sms: int = 0, m_ends: Optional[torch.Tensor] = None,
-                 sfa_atoms: Optional[torch.Tensor] = None, sfb_atoms: Optional[torch.Tensor] = None, zero_tail: bool = False) -> torch.Tensor:
+                 sfa_atoms: Optional[torch.Tensor] = None, sfb_atoms: Optional[torch.Tensor] = None, zero_tail: bool = False,
+                 rows_hint: int = 0) -> torch.Tensor:
     """M-grouped GEMM; see the module docstring. Returns bf16 ``[M, N]`` (``[M, N/2]`` with ``swiglu``).
 
     ``m_ends`` (int32 ``[G]``, optional) makes group g cover rows ``[m_offsets[g], m_ends[g])``: the "masked" form for the
     low-latency layout ``[L, N, hidden]``, where every expert starts at ``g * N`` and only ``packed_recv_count[g]`` rows
     are valid; rows past ``m_ends[g]`` are never written. ``zero_tail=True`` (bf16, no ``swiglu``) says that the rows of ``a`` from
-    ``m_ends[g]`` to the next group are zero and wants those of the result written as zeros.
+    ``m_ends[g]`` to the next group are zero and wants those of the result written as zeros. ``rows_hint``: how many rows the groups have together
+    where ``a`` has room for more (a low-latency layout); FP8 with fp32 scales chooses its tiles by it and keeps the narrow ones without it.
 
     ``sfa_atoms`` / ``sfb_atoms`` (from :func:`build_sf_atoms_a` / :func:`build_sf_atoms_b`) select the natively block-scaled
     FP8 kernel: power-of-two scales are applied by the tensor core (``kind::mxf8f6f4.block_scale``) and a whole tile
     accumulates in TMEM. Every group must then start on a multiple of 128 rows."""
-    return _ext.load().grouped_gemm(a, b, m_offsets, 0, swiglu, a_scales, b_scales, out, num_sms, 2000.0, m_ends, sfa_atoms, sfb_atoms, zero_tail=zero_tail)
+    return _ext.load().grouped_gemm(a, b, m_offsets, 0, swiglu, a_scales, b_scales, out, num_sms, 2000.0, m_ends, sfa_atoms, sfb_atoms, zero_tail=zero_tail,
+                                    rows_hint=rows_hint)
 
 
 def build_sf_atoms_a(a_scales: torch.Tensor) -> torch.Tensor:

@@ -104,8 +104,8 @@ def test_weight_gradient_stops_at_the_last_row(monkeypatch, N, K, pair):
             _close(dw[g], dy[r].float().t() @ x[r].float())
 
 
-@pytest.mark.parametrize("swiglu,K,N", [(True, 128, 256), (True, 640, 768), (False, 384, 256), (False, 1280, 512)])
-@pytest.mark.parametrize("masked", [False, True])
+@pytest.mark.parametrize("swiglu,K,N,masked", [(True, 1152, 512, False), (False, 1280, 512, False), (True, 128, 256, True), (True, 640, 768, True),
+                                               (False, 512, 256, True), (False, 1280, 512, True)])
 def test_promotion_with_256_columns_equals_128(swiglu, K, N, masked):
     """FP8 with fp32 scales: few SMs make the wide tiles the better choice, all of them the narrow ones. Both add the K blocks in the same order
     with the same fused multiply-adds, so the results are the same bit for bit; rows on both sides of a warp's 32 and of a tile's 128."""
@@ -120,7 +120,8 @@ def test_promotion_with_256_columns_equals_128(swiglu, K, N, masked):
     a = torch.randn(M, K, device="cuda").to(torch.float8_e4m3fn)
     b = torch.randn(G, N, K, device="cuda").to(torch.float8_e4m3fn)
     a_s, b_s = torch.rand(M, K // 128, device="cuda") + 0.1, torch.rand(G, N // 128, K // 128, device="cuda") * 0.1
-    kw = dict(m_ends=_i32(ends)) if masked else {}
+    kw = dict(m_ends=_i32(ends), rows_hint=sum(rows)) if masked else {}
+    assert [C.promotion_columns(M, G, N, K, swiglu, masked, kw.get("rows_hint", 0), sms) for sms in (1, 148)] == [256, 128]
     width = N // 2 if swiglu else N
     outs = []
     for sms in (1, 3, 0):
@@ -157,7 +158,8 @@ def test_promotion_with_256_columns_scatters_rows(N):
     dst = torch.full((valid, N), 7.0, dtype=torch.bfloat16, device="cuda")
     bases = torch.tensor([dst.data_ptr()], dtype=torch.int64, device="cuda")
     plain = C.grouped_gemm(a, b, _i32(starts), 0, False, a_s, b_s)
-    C.grouped_gemm(a, b, _i32(starts), 0, False, a_s, b_s, None, 2, 2000.0, _i32(ends), row_info=where.cuda(), scatter_bases=bases)
+    assert C.promotion_columns(M, len(rows), N, K, False, True, valid, 2) == 256
+    C.grouped_gemm(a, b, _i32(starts), 0, False, a_s, b_s, None, 2, 2000.0, _i32(ends), row_info=where.cuda(), scatter_bases=bases, rows_hint=valid)
     torch.cuda.synchronize()
     assert C.gemm_error(0) == 0
     want = torch.full_like(dst, 7.0)
