@@ -160,30 +160,19 @@ torch::Tensor grouped_gemm(const torch::Tensor& a, const torch::Tensor& b, const
     {
         const char* o = std::getenv("DEEPEP_GEMM_ORDER");
         p.tile_order = (o != nullptr && o[0] == '1') ? 1 : 0;
-        // CTA pairs (cta_group::2) of the row form, BF16: weight gradients whose operands are read in place, from 480 padded rows per expert on (with
-        // fewer the output is the work), all others, and SwiGLU where a pair's tile of 256 rows has little padding. The FP8 promotion hands a window to
-        // the epilogue every K block, and the cross-CTA handshake per block costs more than the halved B traffic saves.
         const char* pr = std::getenv("DEEPEP_GEMM_PAIR");
         const bool forced = pr != nullptr && (pr[0] == '0' || pr[0] == '1');
-        const double rows = (double)p.m_total / G;
-        if (forced) p.cta_pairs = pr[0] == '1';
-        else if (!fp8 && mode == 1) p.cta_pairs = !mn_major || rows >= 480;
-        else if (!fp8 && p.m_ends == nullptr) p.cta_pairs = (rows >= 224 && rows <= 270) || rows >= 430;
-        // Forward and input gradients in BF16: tokens as columns on CTA pairs, in tiles of up to 256 of them from 160 padded rows per expert on (gemm_pairs.cu has
-        // both sides), below it of up to 128, which leaves room for eight stages instead of six; but with one tile of rows per expert and few K blocks
-        // the other form's epilogue, which turns nothing over, is the better one. All four products of a layer in a loop, rows / columns, us: 64 experts of 4096 -> 1408
-        // with 5 rows 759 / 717, 20 rows 786 / 730, 60 rows 793 / 765, 94 rows 814 / 806, 110 rows 847 / 851; 60 of 2304 -> 640, 30 rows 247 / 222; single products,
-        // 100 rows: 128 of 2048 -> 512: K 2048 107.2 / 104.1, K 1024 100.7 / 103.4, K 512 60.1 / 67.9; 90 rows: K 640 41.6 / 44.4, K 1280 69.1 / 71.0.
+        p.zero_tail = zero_tail ? 1 : 0;
         if (mode == 0 && !fp8 && !swiglu && p.num_sms >= 2 && p.n % 128 == 0 && p.k % 64 == 0 && !ready.has_value() && !expected.has_value() && !row_info.has_value() &&
             !trace.has_value() && !sched.has_value() && !early_table && !hold_successor) {
-            p.token_pairs = forced ? p.cta_pairs : (rows >= 160 || p.k >= 1024);
-            p.token_cap = rows >= 160 ? 256 : 128;
+            p.token_cap = !forced ? dx::token_columns(p) : pr[0] == '1' ? (p.m_total <= 128ll * G ? 128 : 256) : 0;
+            p.token_pairs = p.token_cap != 0;
         }
-        if (mode == 0 && !swiglu && !fp8) p.cta_pairs = 0;
+        // The FP8 promotion hands a window to the epilogue every K block, and the cross-CTA handshake per block costs more than the halved B traffic saves.
+        if (!p.token_pairs) p.cta_pairs = forced ? pr[0] == '1' : dx::rows_on_pairs(p);
         // A weight gradient with about a tile of rows per expert is bound by what happens per tile; leaving out steps of its two K blocks cost more than it
         // gave (64 experts of 4096 -> 1408, 94 rows: 562 and 573 us).
-        if (mode == 1 && !forced && rows < 160) p.m_ends = nullptr;
-        p.zero_tail = zero_tail ? 1 : 0;
+        if (mode == 1 && !forced && (double)p.m_total / G < 160) p.m_ends = nullptr;
         if (zero_tail && !p.token_pairs) p.m_ends = nullptr;  // all rows up to the next group are computed: zeros in, zeros out
         if (p.num_sms < 2) p.cta_pairs = 0;
         // natively block-scaled e4m3: a pair instantiation exists for the wide SwiGLU tile only
@@ -437,7 +426,24 @@ int promotion_columns(int64_t rows, int64_t groups, int64_t n, int64_t k, bool s
     return dx::wide_promotion(p) ? 256 : 128;
 }
 
+std::string bf16_form(int64_t rows, int64_t groups, int64_t n, int64_t k, bool mn_major, bool ends, bool zero_tail, int num_sms) {
+    dx::GroupedGemmArgs p{};
+    const int there = 0;
+    p.m_total = (int)rows;
+    p.num_groups = (int)groups;
+    p.n = (int)n;
+    p.k = (int)k;
+    p.b_mn = mn_major ? 1 : 0;
+    p.m_ends = ends ? &there : nullptr;
+    p.zero_tail = zero_tail ? 1 : 0;
+    p.num_sms = num_sms;
+    const int cap = dx::token_columns(p);
+    return cap != 0 ? "columns " + std::to_string(cap) : dx::rows_on_pairs(p) ? "row pairs" : "rows";
+}
+
 void bind_gemm(py::module_& m) {
+    m.def("bf16_form", &bf16_form, py::arg("rows"), py::arg("groups"), py::arg("n"), py::arg("k"), py::arg("mn_major") = false, py::arg("ends") = false,
+          py::arg("zero_tail") = false, py::arg("num_sms") = 148);
     m.def("promotion_columns", &promotion_columns, py::arg("rows"), py::arg("groups"), py::arg("n"), py::arg("k"), py::arg("swiglu") = false, py::arg("ends") = false,
           py::arg("rows_hint") = 0, py::arg("num_sms") = 148);
     m.def("build_sf_atoms_a", &build_sf_atoms_a, py::arg("scales"), py::arg("group_counts") = py::none(), py::arg("rows_per_group") = 0);

@@ -35,3 +35,33 @@ C = _ext.load()
 ])
 def test_promotion_tile_width(rows, groups, n, k, swiglu, how, columns):
     assert C.promotion_columns(rows, groups, n, k, swiglu, **how) == columns
+
+
+@pytest.mark.parametrize("rows,groups,n,k,how,form", [
+    # few K blocks stay rows, as pairs where two tiles of rows are full (us, rows / columns: 11.6 / 15.9, 7.4 / 11.6, 124 / 132)
+    (64 * 256, 64, 512, 256, {}, "row pairs"),
+    (64 * 300, 64, 512, 256, {}, "rows"),
+    (64 * 128, 64, 512, 128, dict(ends=True, zero_tail=True), "rows"),
+    (64 * 800, 64, 1408, 512, dict(mn_major=True), "row pairs"),
+    # two rounds of small tiles against one of large ones (16.3 / 19.2; 18.2 / 20.2), and a single one of either (13.9 / 12.0)
+    (64 * 100, 64, 512, 1024, dict(mn_major=True), "rows"),
+    (64 * 128, 64, 512, 1024, dict(ends=True, zero_tail=True), "rows"),
+    (8 * 128, 8, 2048, 1024, dict(ends=True, zero_tail=True), "columns 128"),
+    # half of an odd last tile of 256 features is empty (41 / 47; 29.4 / 42.7)
+    (64 * 210, 64, 128, 5056, dict(ends=True, zero_tail=True), "rows"),
+    # the layers of the training step
+    (64 * 128, 64, 2816, 4096, dict(ends=True, zero_tail=True), "columns 128"),
+    (64 * 128, 64, 4096, 1408, dict(ends=True, zero_tail=True), "columns 128"),
+    (64 * 832, 64, 4096, 1408, dict(ends=True, zero_tail=True), "columns 256"),
+    (64 * 832, 64, 1408, 4096, dict(mn_major=True, ends=True, zero_tail=True), "columns 256"),
+    # a layout with room for more rows than come
+    (64 * 256, 64, 1408, 512, dict(ends=True), "rows"),
+    (64 * 256, 64, 1408, 2048, dict(ends=True), "columns 256"),
+    (64 * 128, 64, 512, 1024, dict(ends=True), "rows"),
+    (160 * 128, 160, 128, 2240, dict(ends=True), "rows"),
+    # what the columns' kernel does not take, and one SM
+    (8 * 512, 8, 192, 4096, {}, "row pairs"),
+    (8 * 512, 8, 256, 4096, dict(num_sms=1), "rows"),
+])
+def test_form_of_bf16_products(rows, groups, n, k, how, form):
+    assert C.bf16_form(rows, groups, n, k, **how) == form

@@ -55,24 +55,39 @@ def test_tokens_as_columns_on_pairs(monkeypatch, K, N, sms, how, mn_major):
         assert (out[end:starts[g + 1]] == (0.0 if how == "zero_tail" else 7.0)).all()
 
 
-def test_few_rows_take_the_other_form_with_the_same_padding():
-    """zero_tail below and above the line between the forms: the same rows are zero, the same values are there."""
+@pytest.mark.parametrize("rows,K,N,forward,gradient", [
+    ([100, 20, 128], 256, 384, "rows", "rows"),
+    ([100, 20, 128], 1024, 768, "columns 128", "rows"),
+    ([1, 0, 33, 128], 768, 1088, "rows", "columns 128"),
+    ([300, 129, 200], 256, 384, "rows", "rows"),
+    ([300, 129, 200], 1088, 1024, "columns 256", "columns 256"),
+    ([500, 460, 430, 0], 256, 384, "rows", "rows"),
+    ([500, 460, 430], 256, 384, "row pairs", "row pairs"),
+])
+def test_every_form_leaves_the_same_padding(rows, K, N, forward, gradient):
+    """zero_tail on both sides of the lines between the forms: the same rows are zero, the same values are there."""
+    from deepep_efa_b200 import _ext
     from deepep_efa_b200.ops.grouped_gemm import grouped_gemm, grouped_gemm_dgrad
+    C = _ext.load()
+    C.gemm_clear_error(0)
     torch.manual_seed(5)
-    for rows in ([100, 20, 128], [300, 129, 200]):
-        starts, ends = _groups(rows, True)
-        x = torch.randn(starts[-1], 256, device="cuda").to(torch.bfloat16)
-        w = (torch.randn(3, 384, 256, device="cuda") * 0.1).to(torch.bfloat16)
-        dy = torch.randn(starts[-1], 384, device="cuda").to(torch.bfloat16)
-        for g in range(3):
-            x[ends[g]:starts[g + 1]] = dy[ends[g]:starts[g + 1]] = 0
-        y = grouped_gemm(x, w, _i32(starts), m_ends=_i32(ends), zero_tail=True)
-        dx = grouped_gemm_dgrad(dy, w, _i32(starts), m_ends=_i32(ends))
-        for g in range(3):
+    starts, ends = _groups(rows, True)
+    G, M = len(rows), starts[-1]
+    n = N // 128 * 128  # (an output has a multiple of 128 columns, a reduction of 64)
+    assert C.bf16_form(M, G, n, K, False, True, True) == forward and C.bf16_form(M, G, K // 128 * 128, N, True, True, True) == gradient
+    for g_of, k, cols in (("forward", K, n), ("gradient", N, K // 128 * 128)):
+        x = torch.randn(M, k, device="cuda").to(torch.bfloat16)
+        for g in range(G):
+            x[ends[g]:starts[g + 1]] = 0
+        w = (torch.randn(G, cols, k, device="cuda") * 0.1).to(torch.bfloat16)
+        y = grouped_gemm(x, w, _i32(starts), m_ends=_i32(ends), zero_tail=True) if g_of == "forward" else \
+            grouped_gemm_dgrad(x, w.transpose(1, 2).contiguous(), _i32(starts), m_ends=_i32(ends))
+        assert C.gemm_error(0) == 0
+        for g in range(G):
             r = slice(starts[g], ends[g])
-            _close(y[r], x[r].float() @ w[g].float().t())
-            _close(dx[r], dy[r].float() @ w[g].float())
-            assert (y[ends[g]:starts[g + 1]] == 0).all() and (dx[ends[g]:starts[g + 1]] == 0).all()
+            if rows[g]:
+                _close(y[r], x[r].float() @ w[g].float().t())
+            assert (y[ends[g]:starts[g + 1]] == 0).all()
     with pytest.raises(ValueError):
         grouped_gemm(x, w, _i32(starts), zero_tail=True)
 
