@@ -160,12 +160,15 @@ torch::Tensor grouped_gemm(const torch::Tensor& a, const torch::Tensor& b, const
     {
         const char* o = std::getenv("DEEPEP_GEMM_ORDER");
         p.tile_order = (o != nullptr && o[0] == '1') ? 1 : 0;
+        // DEEPEP_GEMM_PAIR: 0 = single CTAs, 1 = CTA pairs with tokens as rows, 2 = tokens as columns on CTA pairs wherever that kernel takes the
+        // product (BF16 forward products and input gradients); DEEPEP_GEMM_ORDER is of the forms with tokens as rows.
         const char* pr = std::getenv("DEEPEP_GEMM_PAIR");
+        const bool columns_forced = pr != nullptr && pr[0] == '2';
         const bool forced = pr != nullptr && (pr[0] == '0' || pr[0] == '1');
         p.zero_tail = zero_tail ? 1 : 0;
         if (mode == 0 && !fp8 && !swiglu && p.num_sms >= 2 && p.n % 128 == 0 && p.k % 64 == 0 && !ready.has_value() && !expected.has_value() && !row_info.has_value() &&
             !trace.has_value() && !sched.has_value() && !early_table && !hold_successor) {
-            p.token_cap = !forced ? dx::token_columns(p) : pr[0] == '1' ? (p.m_total <= 128ll * G ? 128 : 256) : 0;
+            p.token_cap = columns_forced ? (p.m_total <= 128ll * G ? 128 : 256) : forced ? 0 : dx::token_columns(p);
             p.token_pairs = p.token_cap != 0;
         }
         // The FP8 promotion hands a window to the epilogue every K block, and the cross-CTA handshake per block costs more than the halved B traffic saves.

@@ -27,7 +27,7 @@ def _close(out, ref):
 def test_tokens_as_columns_on_pairs(monkeypatch, K, N, sms, how, mn_major):
     """Rows on both sides of the unit of 32, of a tile of 256 and of several equal tiles; odd counts of 128 features; empty groups."""
     from deepep_efa_b200 import _ext
-    monkeypatch.setenv("DEEPEP_GEMM_PAIR", "1")
+    monkeypatch.setenv("DEEPEP_GEMM_PAIR", "2")
     C = _ext.load()
     C.gemm_clear_error(0)
     torch.manual_seed(K + N)
@@ -53,6 +53,46 @@ def test_tokens_as_columns_on_pairs(monkeypatch, K, N, sms, how, mn_major):
         if end > starts[g]:
             _close(out[starts[g]:end], x[starts[g]:end].float() @ w[g].float().t())
         assert (out[end:starts[g + 1]] == (0.0 if how == "zero_tail" else 7.0)).all()
+
+
+def _launched(call):
+    """Names of the kernels that a call launches."""
+    from torch.profiler import ProfilerActivity, profile
+    call()
+    torch.cuda.synchronize()
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        call()
+        torch.cuda.synchronize()
+    names = " ".join(e.key for e in prof.key_averages())
+    if "gemm_kernel" not in names:
+        pytest.skip("the profiler records no kernels here")
+    return names
+
+
+@pytest.mark.parametrize("gradient", [False, True])
+def test_forms_that_the_environment_asks_for(monkeypatch, gradient):
+    """0: single CTAs, 1: pairs with tokens as rows, 2: tokens as columns; a product with a trace has the rows' forms only."""
+    from deepep_efa_b200 import _ext
+    C = _ext.load()
+    C.gemm_clear_error(0)
+    torch.manual_seed(2)
+    offs = _i32([0, 256, 512])
+    x = torch.randn(512, 256, device="cuda").to(torch.bfloat16)
+    w = (torch.randn(2, 256, 256, device="cuda") * 0.1).to(torch.bfloat16)
+    ref = torch.cat([x[g * 256:(g + 1) * 256].float() @ (w[g].float() if gradient else w[g].float().t()) for g in range(2)])
+    trace = torch.zeros(4, dtype=torch.int64, device="cuda")
+
+    def run(**kw):
+        return C.grouped_gemm(x, w, offs, 0, False, mn_major=gradient, **kw)
+
+    for value, kw, kernel in (("0", {}, "grouped_gemm_kernel<256, false, false, false"), ("1", {}, "grouped_gemm_kernel<256, false, false, true"),
+                              ("2", {}, "token_pairs_gemm_kernel"), (None, dict(trace=trace), "grouped_gemm_kernel<256, false, false, true")):
+        monkeypatch.delenv("DEEPEP_GEMM_PAIR", raising=False)
+        if value is not None:
+            monkeypatch.setenv("DEEPEP_GEMM_PAIR", value)
+        assert kernel in _launched(lambda: run(**kw)), (value, kw)
+        _close(run(**kw), ref)
+    assert C.gemm_error(0) == 0
 
 
 @pytest.mark.parametrize("rows,K,N,forward,gradient", [
