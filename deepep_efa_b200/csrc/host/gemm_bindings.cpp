@@ -154,7 +154,9 @@ torch::Tensor grouped_gemm(const torch::Tensor& a, const torch::Tensor& b, const
         p.m_ends = m_ends->data_ptr<int>();
         p.m_ends_are_counts = m_ends_are_counts ? 1 : 0;
     }
-    DXG_CHECK(!zero_tail || (mode == 0 && !fp8 && !swiglu && p.m_ends != nullptr), "zero_tail needs m_ends (M-grouped mode, bf16, no swiglu)");
+    // (a form that computes the padding would send it where row_info says, which names no place for it)
+    DXG_CHECK(!zero_tail || (mode == 0 && !fp8 && !swiglu && p.m_ends != nullptr && !row_info.has_value()),
+              "zero_tail needs m_ends (M-grouped mode, bf16, no swiglu, no scatter epilogue)");
     p.rows_hint = (int)std::min<int64_t>(std::max<int64_t>(rows_hint, 0), p.m_total);
     p.num_sms = num_sms > 0 ? num_sms : sm_count(device);
     {

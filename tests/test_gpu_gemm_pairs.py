@@ -132,6 +132,21 @@ def test_every_form_leaves_the_same_padding(rows, K, N, forward, gradient):
         grouped_gemm(x, w, _i32(starts), zero_tail=True)
 
 
+def test_padding_is_not_scattered():
+    """Rows behind an expert's end have no destination, so zeros for them and the scatter epilogue do not go together."""
+    from deepep_efa_b200 import _ext
+    C = _ext.load()
+    starts, ends = [0, 128, 256], [100, 256]
+    x, w = torch.zeros(256, 128, device="cuda", dtype=torch.bfloat16), torch.zeros(2, 128, 128, device="cuda", dtype=torch.bfloat16)
+    dst = torch.full((256, 128), 7.0, device="cuda", dtype=torch.bfloat16)
+    info, bases = torch.arange(256, dtype=torch.int32, device="cuda"), torch.tensor([dst.data_ptr()], dtype=torch.int64, device="cuda")
+    with pytest.raises(ValueError, match="zero_tail"):
+        C.grouped_gemm(x, w, _i32(starts), 0, False, m_ends=_i32(ends), row_info=info, scatter_bases=bases, zero_tail=True)
+    C.grouped_gemm(x, w, _i32(starts), 0, False, m_ends=_i32(ends), row_info=info, scatter_bases=bases)
+    torch.cuda.synchronize()
+    assert (dst[100:128] == 7.0).all() and (dst[:100] == 0).all() and (dst[128:] == 0).all()
+
+
 @pytest.mark.parametrize("pair", ["0", "1"])
 @pytest.mark.parametrize("N,K", [(128, 128), (256, 384), (384, 256)])
 def test_weight_gradient_stops_at_the_last_row(monkeypatch, N, K, pair):
