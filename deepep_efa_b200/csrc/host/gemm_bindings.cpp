@@ -151,6 +151,7 @@ torch::Tensor grouped_gemm(const torch::Tensor& a, const torch::Tensor& b, const
     p.m_ends = nullptr;
     if (m_ends.has_value()) {
         DXG_CHECK(m_ends->is_cuda() && m_ends->scalar_type() == torch::kInt32 && m_ends->is_contiguous() && m_ends->numel() == G, "m_ends must be int32 [G] on the GPU");
+        DXG_CHECK(mode == 0 || mn_major, "m_ends in the K-grouped mode needs operands that are read in place");
         p.m_ends = m_ends->data_ptr<int>();
         p.m_ends_are_counts = m_ends_are_counts ? 1 : 0;
     }

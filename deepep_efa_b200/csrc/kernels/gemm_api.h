@@ -34,7 +34,8 @@ struct GroupedGemmArgs {
     int mx_wide;              // swiglu only: 1 = 256-column tiles (one accumulator window; large groups), 0 = 128-column tiles
     const int* m_offsets;     // [G+1] device memory
     const int* m_ends;        // optional [G]: group g covers rows [m_offsets[g], m_ends[g]) instead of up to m_offsets[g+1]
-                              // (mode 0 only; the low-latency layout has fixed group starts and a count per expert)
+                              // (the low-latency layout has fixed group starts and a count per expert). mode 1, MN-major operands: the rows
+                              // behind it are zero in both, and the reduction may stop there or go over them
     int zero_tail;            // launch_token_pairs_gemm, with m_ends: 1 = rows from m_ends[g] to m_offsets[g+1] are zero in A, and in C they are
                               // written as zeros; 0 = they are not touched
     int m_ends_are_counts;    // 1 = m_ends[g] is the number of rows of group g instead of its end

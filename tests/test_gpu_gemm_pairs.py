@@ -174,6 +174,14 @@ def test_weight_gradient_stops_at_the_last_row(monkeypatch, N, K, pair):
             _close(dw[g], dy[r].float().t() @ x[r].float())
 
 
+def test_ends_of_weight_gradients_need_operands_in_place():
+    from deepep_efa_b200 import _ext
+    C = _ext.load()
+    a = torch.zeros(128, 256, device="cuda", dtype=torch.bfloat16)
+    with pytest.raises(ValueError, match="m_ends"):
+        C.grouped_gemm(a, a, _i32([0, 128, 256]), 1, False, m_ends=_i32([100, 256]))
+
+
 @pytest.mark.parametrize("swiglu,K,N,masked", [(True, 1152, 512, False), (False, 1280, 512, False), (True, 128, 256, True), (True, 640, 768, True),
                                                (False, 512, 256, True), (False, 1280, 512, True)])
 def test_promotion_with_256_columns_equals_128(swiglu, K, N, masked):
