@@ -85,7 +85,8 @@ struct GroupedGemmArgs {
     // 1 = the next kernel in the stream gets no SM before this one has ended, also where it is a programmatic dependent launch: the SMs
     // that this launch leaves free are meant for another stream.
     int hold_successor;
-    int token_pairs;          // the caller's choice: launch_token_pairs_gemm takes this product
+    int token_pairs;          // the caller's choice: launch_token_pairs_gemm takes this product (gemm_choice.h; never with gates, the scatter epilogue, a
+                              // trace, a tile counter, early_table or hold_successor, which that kernel does not have: a traced product takes rows)
     // launch_token_cols_gemm, launch_token_pairs_gemm: tokens of one tile at most (a multiple of 32 from 64 to 224, of 64 up to 256)
     int token_cap;
 };

@@ -21,17 +21,11 @@ def _close(out, ref):
     assert ((out.float() - ref).norm() / ref.norm().clamp(min=1e-20)).item() < 4e-3
 
 
-@pytest.mark.parametrize("mn_major", [False, True])
-@pytest.mark.parametrize("how", ["whole", "ragged", "masked", "zero_tail"])
-@pytest.mark.parametrize("K,N,sms", [(64, 128, 0), (192, 384, 6), (512, 256, 0), (320, 1408, 0)])
-def test_tokens_as_columns_on_pairs(monkeypatch, K, N, sms, how, mn_major):
-    """Rows on both sides of the unit of 32, of a tile of 256 and of several equal tiles; odd counts of 128 features; empty groups."""
+def _check_columns(rows, K, N, sms, how, mn_major):
     from deepep_efa_b200 import _ext
-    monkeypatch.setenv("DEEPEP_GEMM_PAIR", "2")
     C = _ext.load()
     C.gemm_clear_error(0)
     torch.manual_seed(K + N)
-    rows = [1, 0, 31, 32, 33, 255, 256, 257, 300, 513, 128]
     starts, ends = _groups(rows, how != "ragged")
     if how == "zero_tail":  # a group of padding only
         starts, ends = starts + [starts[-1] + 128], ends + [starts[-1]]
@@ -53,6 +47,30 @@ def test_tokens_as_columns_on_pairs(monkeypatch, K, N, sms, how, mn_major):
         if end > starts[g]:
             _close(out[starts[g]:end], x[starts[g]:end].float() @ w[g].float().t())
         assert (out[end:starts[g + 1]] == (0.0 if how == "zero_tail" else 7.0)).all()
+    return C.bf16_form(M, G, N, K, mn_major, bool(kw), how == "zero_tail", sms or 148)
+
+
+@pytest.mark.parametrize("mn_major", [False, True])
+@pytest.mark.parametrize("how", ["whole", "ragged", "masked", "zero_tail"])
+@pytest.mark.parametrize("K,N,sms", [(64, 128, 0), (192, 384, 6), (512, 256, 0), (320, 1408, 0)])
+def test_tokens_as_columns_on_pairs(monkeypatch, K, N, sms, how, mn_major):
+    """Rows on both sides of the unit of 32, of a tile of 256 and of several equal tiles; odd counts of 128 features; empty groups."""
+    monkeypatch.setenv("DEEPEP_GEMM_PAIR", "2")
+    _check_columns([1, 0, 31, 32, 33, 255, 256, 257, 300, 513, 128], K, N, sms, how, mn_major)
+
+
+@pytest.mark.parametrize("mn_major", [False, True])
+@pytest.mark.parametrize("how", ["whole", "ragged", "masked", "zero_tail"])
+@pytest.mark.parametrize("K,N,sms", [(64, 128, 2), (576, 384, 6), (1024, 256, 0), (1088, 384, 0)])
+def test_tokens_as_columns_in_tiles_of_128(monkeypatch, K, N, sms, how, mn_major):
+    """With up to 128 rows per group on average: rows on both sides of a unit and of a tile, K blocks fewer than, as many as and more than the eight
+    stages, tiles enough on few SMs for both windows to go round. From K 1024 on this is what the product takes by itself."""
+    if K < 1024:
+        monkeypatch.setenv("DEEPEP_GEMM_PAIR", "2")
+    else:
+        monkeypatch.delenv("DEEPEP_GEMM_PAIR", raising=False)
+    form = _check_columns([1, 0, 31, 0, 33, 64, 0, 65, 127, 128, 129, 257, 0, 0], K, N, sms, how, mn_major)
+    assert K < 1024 or form == "columns 128"
 
 
 def _launched(call):
