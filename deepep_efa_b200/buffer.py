@@ -406,40 +406,37 @@ class Buffer:
         if self._cpu is not None:
             return self._cpu.dispatch(x, handle, num_tokens_per_rank, is_token_in_rank, num_tokens_per_expert, topk_idx,
                                       topk_weights, expert_alignment, num_worst_tokens)
-        if not (_DEBUG_CHECKS or NVTX_ENABLED):
-            # what _dispatch_many does, for one rank, in a straight line (see _on_callers_stream)
-            self.check_status()
-            used = config if config is not None else self.get_dispatch_config(self.group_size)
-            num_sms, num_channels = _normal_sms(used, config is not None, [self]), _num_channels(used)
-            cached = handle is not None
-            if cached:
-                assert topk_idx is None and topk_weights is None, "cached dispatch carries no top-k data"
-            else:
-                assert num_tokens_per_rank is not None and is_token_in_rank is not None and num_tokens_per_expert is not None
-            rows, scales = x if isinstance(x, tuple) else (x, None)
-            call = (rows, scales, num_tokens_per_rank, num_tokens_per_expert, is_token_in_rank, topk_idx, topk_weights, handle)
-            how = (num_channels, expert_alignment, quantize_fp8, round_scale, 0 if cached else num_worst_tokens, num_sms)
-            if not allocate_on_comm_stream and _on_callers_stream(previous_event, async_finish):
-                event = None
-                recv_x, recv_scales, recv_idx, recv_w, per_expert, new_handle = self._C.normal_dispatch([self.runtime], [call], *how)[0]
-            else:
-                with _CommScope(self, previous_event, async_finish, allocate_on_comm_stream, call[:7]) as scope:
-                    recv_x, recv_scales, recv_idx, recv_w, per_expert, new_handle = self._C.normal_dispatch([self.runtime], [call], *how)[0]
-                    if not cached:
-                        rpm, cpm, rcpm, _, _, send_head = new_handle
-                        scope.outputs(rpm, cpm, rcpm, send_head)
-                event = scope.event
-            event = EventOverlap() if event is None else event
-            if recv_scales is not None:
-                recv_x = (recv_x, recv_scales)
-            if cached:
-                return recv_x, None, None, None, None, event
-            return recv_x, recv_idx, recv_w, per_expert, new_handle, event
-        req = _DispatchReq(x, handle, num_tokens_per_rank, is_token_in_rank, num_tokens_per_expert, topk_idx, topk_weights,
-                           expert_alignment, num_worst_tokens, quantize_fp8, round_scale)
-        own_config = config is not None
-        config = config if own_config else self.get_dispatch_config(self.group_size)
-        return _dispatch_many([self], [req], config, previous_event, async_finish, allocate_on_comm_stream, own_config)[0]
+        # what _dispatch_many does for several emulated ranks, for one, in a straight line (see _on_callers_stream)
+        self.check_status()
+        used = config if config is not None else self.get_dispatch_config(self.group_size)
+        num_sms, num_channels = _normal_sms(used, config is not None, [self]), _num_channels(used)
+        cached = handle is not None
+        if cached:
+            assert topk_idx is None and topk_weights is None, "cached dispatch carries no top-k data"
+            if _DEBUG_CHECKS:
+                validate_handle(handle, self.rank, self.group_size)
+        else:
+            assert num_tokens_per_rank is not None and is_token_in_rank is not None and num_tokens_per_expert is not None
+        rows, scales = x if isinstance(x, tuple) else (x, None)
+        call = (rows, scales, num_tokens_per_rank, num_tokens_per_expert, is_token_in_rank, topk_idx, topk_weights, handle)
+        how = (num_channels, expert_alignment, quantize_fp8, round_scale, 0 if cached else num_worst_tokens, num_sms)
+        native = _named("ep.dispatch", self._C.normal_dispatch)
+        if not allocate_on_comm_stream and _on_callers_stream(previous_event, async_finish):
+            event = None
+            recv_x, recv_scales, recv_idx, recv_w, per_expert, new_handle = native([self.runtime], [call], *how)[0]
+        else:
+            with _CommScope(self, previous_event, async_finish, allocate_on_comm_stream, call[:7]) as scope:
+                recv_x, recv_scales, recv_idx, recv_w, per_expert, new_handle = native([self.runtime], [call], *how)[0]
+                if not cached:
+                    rpm, cpm, rcpm, _, _, send_head = new_handle
+                    scope.outputs(rpm, cpm, rcpm, send_head)
+            event = scope.event
+        event = EventOverlap() if event is None else event
+        if recv_scales is not None:
+            recv_x = (recv_x, recv_scales)
+        if cached:
+            return recv_x, None, None, None, None, event
+        return recv_x, recv_idx, recv_w, per_expert, new_handle, event
 
     def combine(self, x: torch.Tensor, handle: Tuple, topk_weights: Optional[torch.Tensor] = None,
                 bias: Union[torch.Tensor, Tuple[torch.Tensor, torch.Tensor], None] = None, config: Optional[Config] = None,
@@ -455,33 +452,31 @@ class Buffer:
             return self.internode_combine(x, handle, topk_weights, bias, config, previous_event, async_finish, allocate_on_comm_stream)
         if self._cpu is not None:
             return self._cpu.combine(x, handle, topk_weights, bias)
-        if not (_DEBUG_CHECKS or NVTX_ENABLED):
-            self.check_status()
-            num_sms = _normal_sms(config if config is not None else self.get_combine_config(self.group_size), config is not None, [self])
-            direct = not allocate_on_comm_stream and _on_callers_stream(previous_event, async_finish)
-            scope = None if direct else _CommScope(self, previous_event, async_finish, allocate_on_comm_stream)
-            rpm, _, _, src_idx, _, send_head = handle
-            assert x.dim() == 2 and x.dtype == torch.bfloat16 and x.size(0) == src_idx.size(0)
-            b0, b1 = Buffer._unpack_bias(bias)
-            if direct:
-                out, out_w = self._C.normal_combine([self.runtime], [(x, topk_weights, send_head, rpm, b0, b1, None, None)], num_sms)[0]
-                return out, out_w, EventOverlap()
-            out = out_w = None
-            if not allocate_on_comm_stream:
-                # results are allocated here, on the caller's stream (see _CommScope.outputs_from_caller_stream)
-                out = torch.empty((send_head.size(0), x.size(1)), dtype=torch.bfloat16, device=x.device)
-                out_w = torch.empty((send_head.size(0), topk_weights.size(1)), dtype=torch.float32, device=x.device) if topk_weights is not None else None
-                scope.outputs_from_caller_stream(out, out_w)
-            scope.inputs = [t for t in (x, topk_weights, b0, b1) if t is not None]
-            with scope:
-                out, out_w = self._C.normal_combine([self.runtime], [(x, topk_weights, send_head, rpm, b0, b1, out, out_w)], num_sms)[0]
-                if allocate_on_comm_stream:
-                    scope.outputs(out, out_w)
-            return out, out_w, scope.event
-        own_config = config is not None
-        config = config if own_config else self.get_combine_config(self.group_size)
-        return _combine_many([self], [(x, handle, topk_weights, bias)], config, previous_event, async_finish,
-                             allocate_on_comm_stream, own_config)[0]
+        self.check_status()
+        num_sms = _normal_sms(config if config is not None else self.get_combine_config(self.group_size), config is not None, [self])
+        direct = not allocate_on_comm_stream and _on_callers_stream(previous_event, async_finish)
+        scope = None if direct else _CommScope(self, previous_event, async_finish, allocate_on_comm_stream)
+        rpm, _, _, src_idx, _, send_head = handle
+        if _DEBUG_CHECKS:
+            validate_handle(handle, self.rank, self.group_size)
+        assert x.dim() == 2 and x.dtype == torch.bfloat16 and x.size(0) == src_idx.size(0)
+        b0, b1 = Buffer._unpack_bias(bias)
+        native = _named("ep.combine", self._C.normal_combine)
+        if direct:
+            out, out_w = native([self.runtime], [(x, topk_weights, send_head, rpm, b0, b1, None, None)], num_sms)[0]
+            return out, out_w, EventOverlap()
+        out = out_w = None
+        if not allocate_on_comm_stream:
+            # results are allocated here, on the caller's stream (see _CommScope.outputs_from_caller_stream)
+            out = torch.empty((send_head.size(0), x.size(1)), dtype=torch.bfloat16, device=x.device)
+            out_w = torch.empty((send_head.size(0), topk_weights.size(1)), dtype=torch.float32, device=x.device) if topk_weights is not None else None
+            scope.outputs_from_caller_stream(out, out_w)
+        scope.inputs = [t for t in (x, topk_weights, b0, b1) if t is not None]
+        with scope:
+            out, out_w = native([self.runtime], [(x, topk_weights, send_head, rpm, b0, b1, out, out_w)], num_sms)[0]
+            if allocate_on_comm_stream:
+                scope.outputs(out, out_w)
+        return out, out_w, scope.event
 
     # Groups that span several NVLink domains (the reference's "internode" paths).
     def internode_dispatch(self, x, handle: Optional[Tuple] = None, num_tokens_per_rank: Optional[torch.Tensor] = None,
@@ -720,6 +715,17 @@ def _as_topk_idx(topk_idx):
     if topk_idx is not None and topk_idx.dtype != torch.int64:
         return topk_idx.to(torch.int64)
     return topk_idx
+
+
+def _named(name: str, call):
+    """The native call, in an NVTX range of that name where ranges are on: what is profiled is what runs without them."""
+    if not NVTX_ENABLED:
+        return call
+
+    def ranged(*args):
+        with nvtx_range(name):
+            return call(*args)
+    return ranged
 
 
 def _on_callers_stream(previous_event, async_finish) -> bool:

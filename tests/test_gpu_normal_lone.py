@@ -51,3 +51,53 @@ def test_lone_rank_matches_general_kernels(T, H, masked, wire):
             assert len(a) == len(b) and all(torch.equal(p, q) for p, q in zip(a, b))
     finally:
         vc.destroy()
+
+
+@pytest.mark.parametrize("async_finish", [False, True])
+def test_named_ranges_and_handle_checks_are_of_the_path_that_runs(monkeypatch, async_finish):
+    """With NVTX ranges and the debug checks on, dispatch and combine take the same path as without them."""
+    from deepep_efa_b200 import buffer as module
+    from deepep_efa_b200.parallel.virtual import VirtualCluster
+    from deepep_efa_b200.utils import profiler
+    T, H, E, K = 40, 512, 8, 2
+    vc = VirtualCluster(1, num_nvl_bytes=64 << 20, timeout_ms=2000)
+    try:
+        buf, names = vc.buffers[0], []
+        idx, w = make_routing(T, E, K, "cuda", seed=1)
+        x = make_tokens(T, H, "cuda", seed=2)
+        per_rank, _, per_expert, in_rank, _ = buf.get_dispatch_layout(idx, E)
+        how = dict(async_finish=async_finish)
+        fresh = dict(num_tokens_per_rank=per_rank, is_token_in_rank=in_rank, num_tokens_per_expert=per_expert, topk_idx=idx, topk_weights=w, **how)
+
+        def steps():
+            rx, _, rw, _, handle, e0 = buf.dispatch(x, **fresh)
+            e0.current_stream_wait()
+            again, _, _, _, _, e1 = buf.dispatch(x, handle=handle, **how)
+            e1.current_stream_wait()
+            out, _, e2 = buf.combine(again, handle, **how)
+            e2.current_stream_wait()
+            torch.cuda.synchronize()
+            return handle, [rx.clone(), again.clone(), out.clone()]
+
+        _, plain = steps()
+
+        def other_path(*args, **kw):
+            raise AssertionError("the path of several emulated ranks")
+
+        monkeypatch.setattr(module, "_dispatch_many", other_path)
+        monkeypatch.setattr(module, "_combine_many", other_path)
+        for m in (module, profiler):
+            monkeypatch.setattr(m, "NVTX_ENABLED", True)
+        monkeypatch.setattr(module, "_DEBUG_CHECKS", True)
+        monkeypatch.setattr(torch.cuda.nvtx, "range_push", names.append)
+        monkeypatch.setattr(torch.cuda.nvtx, "range_pop", lambda: None)
+        handle, named = steps()
+        assert names == ["ep.dispatch", "ep.dispatch", "ep.combine"]
+        assert all(torch.equal(a, b) for a, b in zip(plain, named))
+        foreign = handle[:3] + (handle[3][:-1],) + handle[4:]  # one row short
+        with pytest.raises(AssertionError, match="receive count"):
+            buf.dispatch(x, handle=foreign, **how)
+        with pytest.raises(AssertionError, match="receive count"):
+            buf.combine(x[:T - 1], foreign, **how)
+    finally:
+        vc.destroy()
