@@ -11,23 +11,26 @@ inline long long tiles_up(long long a, long long b) { return (a + b - 1) / b; }
 
 // Whether FP8 with fp32 scales takes tiles of 256 columns instead of 128 (n % 256 == 0). Half as many tiles, each of which takes less than twice as
 // long: it pays unless the narrow ones fill the SMs that much better. With q = rounds of wide tiles / rounds of narrow ones (0.5 with many, 1
-// where both are dealt out at once), time wide / narrow over 9300 products of random sizes and routings, geometric mean and in brackets the worst tenth:
+// where both are dealt out at once):
 //
-//   K blocks                                             1 to 3      4-7         8-15        16-31       32 on
-//   whole groups, plain,  q 0.5                       1.04 (1.08) 0.98 (1.02) 0.93 (1.00) 0.87 (0.96) 0.80 (0.89)
-//                         q 0.56 to 0.61              1.16        1.11        1.07        1.02        0.92
-//                         q 1                         1.27        1.41        1.39        1.32        1.25
-//   whole groups, SwiGLU, q 0.5                       1.01 (1.02) 1.00 (1.03) 0.96 (1.03) 0.91 (0.98) 0.86 (0.94)
-//   ends given,   plain,  q 0.5, tiles full           1.04 (1.10) 0.97 (1.00) 0.89 (0.95) 0.83 (0.88) 0.75 (0.85)
-//                         q 0.51 to 0.56, tiles full  1.06        1.01        0.93        0.88        0.78
-//                         q 0.56 to 0.61, tiles full  1.14        1.08        1.01        0.94        0.86
-//                         q 0.56 to 0.61, up to 24    0.92        0.89        0.91        0.93        0.89      rows in a tile
-//                         q 0.61 to 0.68, up to 24    1.02        0.98        0.94        0.99        0.95
-//   ends given,   SwiGLU, q 0.56 to 0.61              0.69        0.76        0.84        0.88        0.91
-//                         q 0.61 to 0.68              0.77        0.84        0.87        0.96        0.99
+// Whole groups, time of the product wide / narrow over 3400 of random sizes, geometric mean and in brackets the worst tenth
+//   K blocks                          1 to 3      4-7         8-15        16-31       32 on
+//   plain,  q 0.5                   1.04 (1.08) 0.98 (1.02) 0.93 (1.00) 0.87 (0.96) 0.80 (0.89)
+//           q 0.56 to 0.61          1.16        1.11        1.07        1.02        0.92
+//           q 1                     1.27        1.41        1.39        1.32        1.25
+//   SwiGLU, q 0.5                   1.01 (1.02) 1.00 (1.03) 0.96 (1.03) 0.91 (0.98) 0.86 (0.94)
 //
-// (With the ends of the groups given, warps without rows promote nothing.) A layout that has room for more rows than come (m_ends without
-// rows_hint) says nothing about the tiles: where two of 32 experts are in use, 1.2 to 1.36, where all are, 0.5 to 1; it keeps the narrow ones.
+// Ends given, change of a whole layer's time in per cent (1700 decode steps, fused and step-by-step layers of random sizes and routings)
+//   q                               to 0.53   0.53-0.56   0.56-0.6   0.6-0.63   0.63-0.7   1
+//   SwiGLU,  8 to 15 K blocks        -2.7      +0.1        +3.1       +5.0       +6.9     +13.8
+//           16 to 31                 -3.4      -0.4        +2.3       +4.9       +8.5     +20.4
+//           32 on                    -6.5      -2.8        -0.2       +2.7       +7.4     +20.0
+//   plain,   4 to 7                  -4.0      -3.7        -2.3       -0.7       -0.1      +2.1
+//            8 on                    -4.6      -3.7        -2.1       -1.6       -0.1      +3.7
+//
+// Alone, with plain tiles of one to three K blocks: 1.04 where they are full of rows, 0.9 with up to 24 rows in one. SwiGLU alone gains more than in
+// a layer where the rows of the padding are not zero. A layout that has room for more rows than come (m_ends without rows_hint) says nothing about
+// the tiles: where two of 32 experts are in use, 1.2 to 1.36, where all are, 0.5 to 1; it keeps the narrow ones.
 inline bool wide_promotion(const GroupedGemmArgs& a) {
     const bool ends = a.m_ends != nullptr;
     if (a.cta_pairs || a.n % 256 != 0 || (ends && a.rows_hint <= 0)) return false;
@@ -40,9 +43,9 @@ inline bool wide_promotion(const GroupedGemmArgs& a) {
     const int kb = a.k / 128;
     double most;
     if (!ends) most = kb < 8 ? 0.0 : kb < 16 ? 0.53 : kb < 32 ? 0.56 : 0.6;
-    else if (a.swiglu) most = 0.625;
-    else if (a.rows_hint <= 48 * row_tiles) most = kb < 4 ? 0.58 : 0.625;
-    else most = kb < 4 ? 0.0 : kb < 8 ? 0.51 : kb < 16 ? 0.56 : 0.6;
+    else if (a.swiglu) most = kb < 16 ? 0.55 : kb < 32 ? 0.56 : 0.6;
+    else if (a.rows_hint <= 48 * row_tiles) most = kb < 4 ? 0.58 : 0.67;
+    else most = kb < 4 ? 0.0 : kb < 8 ? 0.58 : 0.625;
     auto pays = [&](long long rt) {
         const long long tiles = rt * (a.n / 256);
         return (double)tiles_up(tiles, a.num_sms) <= most * (double)tiles_up(2 * tiles, a.num_sms);
