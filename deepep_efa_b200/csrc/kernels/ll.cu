@@ -991,7 +991,7 @@ __global__ void __launch_bounds__(kLLThreads, 1) combine_pull(const __grid_const
 // in between. Only reads happen early; results are stored after the predecessor has completed, because their memory may be a block that the
 // predecessor still reads (freed by the caller between the two calls). The successor is released only then, where this kernel has
 // more than a CTA per SM: the next dispatch's CTAs, launched at its start, took the places of CTAs of both kernels that still had work (128 tokens of 7168, 256 experts, top-8, FP8, launched one by
-// one: pair of dispatch and combine 15.1 -> 12.1 us; 33 tokens of 6144 in a graph, two pairs 14.3 -> 12.9). With fewer CTAs nobody's place is taken, and
+// one: pair of dispatch and combine 14.4 -> 12.0 to 12.2 us, on one B200 13.3; 33 tokens of 6144 in a graph, two pairs 14.3 -> 12.9). With fewer CTAs nobody's place is taken, and
 // the early launch is worth a little (30 tokens of 2944, top-2, in a graph: 12.4, late 12.8). With kFind, which gathers nothing early, it made no
 // difference, and the release stays in front.
 // kFind (x is an ordinary tensor): whatever launched in between may still be writing x, so the predecessor's end comes first, as for the
