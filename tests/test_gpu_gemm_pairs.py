@@ -78,7 +78,7 @@ def _launched(call):
     from torch.profiler import ProfilerActivity, profile
     call()
     torch.cuda.synchronize()
-    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+    with profile(activities=[ProfilerActivity.CUDA], acc_events=True) as prof:
         call()
         torch.cuda.synchronize()
     names = " ".join(e.key for e in prof.key_averages())
