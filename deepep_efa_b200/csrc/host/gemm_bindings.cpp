@@ -176,9 +176,6 @@ torch::Tensor grouped_gemm(const torch::Tensor& a, const torch::Tensor& b, const
         }
         // The FP8 promotion hands a window to the epilogue every K block, and the cross-CTA handshake per block costs more than the halved B traffic saves.
         if (!p.token_pairs) p.cta_pairs = forced ? pr[0] == '1' : dx::rows_on_pairs(p);
-        // A weight gradient with about a tile of rows per expert is bound by what happens per tile; leaving out steps of its two K blocks cost more than it
-        // gave (64 experts of 4096 -> 1408, 94 rows: 562 and 573 us).
-        if (mode == 1 && !forced && (double)p.m_total / G < 160) p.m_ends = nullptr;
         if (zero_tail && !p.token_pairs) p.m_ends = nullptr;  // all rows up to the next group are computed: zeros in, zeros out
         if (p.num_sms < 2) p.cta_pairs = 0;
         // natively block-scaled e4m3: a pair instantiation exists for the wide SwiGLU tile only

@@ -192,6 +192,49 @@ def test_weight_gradient_stops_at_the_last_row(monkeypatch, N, K, pair):
             _close(dw[g], dy[r].float().t() @ x[r].float())
 
 
+@pytest.mark.parametrize("pair", ["0", "1"])
+@pytest.mark.parametrize("N,K", [(128, 128), (256, 384)])
+def test_outputs_that_start_between_sectors_equal_aligned_ones(monkeypatch, N, K, pair):
+    """Rows leave in pieces of 32 bytes where the output starts on such a boundary, and through a staging buffer elsewhere. Odd numbers of rows: the
+    last row of a pair of lanes is not there."""
+    from deepep_efa_b200 import _ext
+    monkeypatch.setenv("DEEPEP_GEMM_PAIR", pair)
+    C = _ext.load()
+    C.gemm_clear_error(0)
+    torch.manual_seed(N + K)
+
+    def outputs(shape):
+        n = shape[0] * shape[1] * (shape[2] if len(shape) == 3 else 1)
+        for shift in (0, 8):
+            flat = torch.full((n + 32,), 7.0, device="cuda", dtype=torch.bfloat16)
+            yield flat, flat[shift:shift + n].view(shape), shift
+
+    rows = [1, 31, 33, 0, 129, 2]
+    starts, _ = _groups(rows, False)
+    x, w = (torch.randn(s, device="cuda").to(torch.bfloat16) for s in ((starts[-1], K), (len(rows), N, K)))
+    forward = []
+    for flat, out, shift in outputs((starts[-1], N)):
+        C.grouped_gemm(x, w, _i32(starts), 0, False, None, None, out)
+        assert (flat[:shift] == 7.0).all() and (flat[shift + out.numel():] == 7.0).all()
+        forward.append(out)
+    starts, _ = _groups([70, 0, 1, 128], True)
+    dy, h = (torch.randn(starts[-1], c, device="cuda").to(torch.bfloat16) for c in (N, K))
+    grads = []
+    for flat, out, shift in outputs((4, N, K)):
+        C.grouped_gemm(dy, h, _i32(starts), 1, False, None, None, out, mn_major=True)
+        assert (flat[:shift] == 7.0).all() and (flat[shift + out.numel():] == 7.0).all()
+        grads.append(out)
+    torch.cuda.synchronize()
+    assert C.gemm_error(0) == 0
+    assert torch.equal(*forward) and torch.equal(*grads)
+    for g in range(4):
+        r = slice(starts[g], starts[g + 1])
+        if starts[g + 1] > starts[g]:
+            _close(grads[0][g], dy[r].float().t() @ h[r].float())
+        else:
+            assert (grads[0][g] == 0).all()
+
+
 def test_ends_of_weight_gradients_need_operands_in_place():
     from deepep_efa_b200 import _ext
     C = _ext.load()
