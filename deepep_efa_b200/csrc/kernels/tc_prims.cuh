@@ -7,6 +7,7 @@
 
 #include "gemm_api.h"
 #include "prims.cuh"
+#include "sigmoid.cuh"
 
 namespace dx {
 
@@ -338,8 +339,6 @@ __device__ __forceinline__ void st_global_256(void* p, const uint32_t* v) {
                  "r"(v[6]), "r"(v[7])
                  : "memory");
 }
-
-__device__ __forceinline__ float silu(float x) { return x / (1.f + __expf(-x)); }
 
 // Four lanes hold one byte of each of four tokens (byte t of the word) for neighbouring features: afterwards lane j of the four holds
 // the four features of token j.

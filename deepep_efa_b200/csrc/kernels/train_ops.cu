@@ -11,6 +11,7 @@
 // dominated the training step.
 #include "gemm_api.h"
 #include "launch.cuh"
+#include "sigmoid.cuh"
 
 #include <cuda_bf16.h>
 
@@ -50,8 +51,6 @@ __global__ void __launch_bounds__(256) transpose_bf16_kernel(const __nv_bfloat16
     }
 }
 
-__device__ __forceinline__ float silu_f(float x) { return x / (1.f + __expf(-x)); }
-
 // One thread per eight columns; `I` is a 32-bit index wherever the sizes allow (a 64-bit division per thread costs more than the
 // arithmetic of the eight elements).
 template <typename I>
@@ -70,7 +69,7 @@ __global__ void __launch_bounds__(256) swiglu_fwd_kernel(const __nv_bfloat16* __
     const __nv_bfloat16* up = reinterpret_cast<const __nv_bfloat16*>(&u);
     __align__(16) __nv_bfloat16 o[8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) o[j] = __float2bfloat16(silu_f(__bfloat162float(gp[j])) * __bfloat162float(up[j]));
+    for (int j = 0; j < 8; ++j) o[j] = __float2bfloat16(silu(__bfloat162float(gp[j])) * __bfloat162float(up[j]));
     *reinterpret_cast<int4*>(h + (size_t)r * inter + c) = *reinterpret_cast<const int4*>(o);
 }
 
@@ -95,7 +94,7 @@ __global__ void __launch_bounds__(256) swiglu_bwd_kernel(const __nv_bfloat16* __
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
         const float x = __bfloat162float(gp[j]), uu = __bfloat162float(up[j]), dd = __bfloat162float(dp[j]);
-        const float sig = 1.f / (1.f + __expf(-x));
+        const float sig = sigmoid(x);
         og[j] = __float2bfloat16(dd * uu * sig * (1.f + x * (1.f - sig)));  // d silu(x)/dx = sig * (1 + x * (1 - sig))
         ou[j] = __float2bfloat16(dd * x * sig);
     }

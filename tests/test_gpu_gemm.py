@@ -156,6 +156,32 @@ def test_swiglu_kernels_match_autograd():
     assert _rel_err(h13.grad, ref_in.grad) < 4e-3
 
 
+def test_swiglu_of_zeros_infinities_and_the_far_ends():
+    """Gates whose quotient x / (1 + e^-x) is a zero of either sign, infinite, not a number, or has a denominator near the end of the range."""
+    from deepep_efa_b200.ops import grouped_gemm as gg
+    inf, nan = float("inf"), float("nan")
+    gates = [0.0, -0.0, inf, -inf, nan, 88.0, -87.0, -88.0, -89.0, -100.0, 3e38, -3e38, 1e-30, -1e-30, 20.0, -20.0]
+    gate = torch.tensor([gates, [g / 8 for g in gates]], device="cuda").to(torch.bfloat16)
+    h13 = torch.cat([gate, torch.ones_like(gate)], dim=1).requires_grad_(True)
+    h = gg.swiglu(h13)
+    h.backward(torch.ones_like(h))
+    x = gate.double()
+    sig = 1 / (1 + torch.exp(-x))
+    want = torch.where(x == -inf, nan, x * sig)  # (-inf * 0)
+    finite = torch.isfinite(x)
+
+    def close(out, ref):
+        # fp32 values with a few units of error, rounded to BF16 (2^-9); below 2^-126 only the magnitude counts
+        assert ((out.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-36).all()
+
+    h = h.detach()
+    close(h[finite], want[finite])
+    close(h13.grad[:, 16:][finite], want[finite])
+    close(h13.grad[:, :16][finite], (sig * (1 + x * (1 - sig)))[finite])
+    assert torch.equal(torch.isnan(h), torch.isnan(want)) and torch.equal(torch.isinf(h), torch.isinf(want))
+    assert torch.equal(torch.signbit(h[:, :2]), torch.signbit(gate[:, :2]))
+
+
 def test_rowdot_kernel():
     from deepep_efa_b200 import _ext
     torch.manual_seed(9)
