@@ -75,23 +75,29 @@ __device__ __forceinline__ void store_block_coalesced(int4* stage, const int4 (&
 // cycles (20 to 94 rows per expert), now 3100. Both weight gradients of 64 experts of 4096 -> 1408 in a loop, us, before / after: 20 rows 559 / 453, 94 rows
 // 623 / 538, 190 rows 753 / 671, 384 rows 1061 / 1041, on pairs 768 rows 1563 / 1567. Whole lines of 128 bytes by two exchanges are no faster (94 rows 343 / 343
 // for the first), neither are eight epilogue warps on alternate tiles (361 / 369) or columns read from TMEM ahead (343 / 398).
-__device__ __forceinline__ void store_block_direct(const int4* regs, __nv_bfloat16* gbase, int ldc, int rows_valid, int lane) {
-    const bool odd = lane & 1;
-    const uint32_t w[16] = {(uint32_t)regs[0].x, (uint32_t)regs[0].y, (uint32_t)regs[0].z, (uint32_t)regs[0].w, (uint32_t)regs[1].x, (uint32_t)regs[1].y,
-                            (uint32_t)regs[1].z, (uint32_t)regs[1].w, (uint32_t)regs[2].x, (uint32_t)regs[2].y, (uint32_t)regs[2].z, (uint32_t)regs[2].w,
-                            (uint32_t)regs[3].x, (uint32_t)regs[3].y, (uint32_t)regs[3].z, (uint32_t)regs[3].w};
-    uint32_t first[8], second[8];  // what this lane stores of the even row and of the odd one
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        const uint32_t got = __shfl_xor_sync(0xffffffffu, odd ? w[j] : w[8 + j], 1);
-        first[j] = odd ? got : w[j];
-        second[j] = odd ? w[8 + j] : got;
+struct RowPair {
+    __nv_bfloat16 *even, *odd;  // this lane's half of 32 columns of the rows of lanes 2i and 2i + 1 (nullptr: no such row)
+    bool upper;
+    __device__ __forceinline__ RowPair(__nv_bfloat16* mine, int lane) : upper(lane & 1) {
+        __nv_bfloat16* other = reinterpret_cast<__nv_bfloat16*>(__shfl_xor_sync(0xffffffffu, reinterpret_cast<unsigned long long>(mine), 1));
+        even = upper ? other : mine;
+        odd = upper ? mine : other;
+        if (upper && even != nullptr) even += 16;
+        if (upper && odd != nullptr) odd += 16;
     }
-    const int even_row = lane & ~1;
-    __nv_bfloat16* dst = gbase + (size_t)even_row * ldc + (odd ? 16 : 0);
-    if (even_row < rows_valid) st_global_256(dst, first);
-    if (even_row + 1 < rows_valid) st_global_256(dst + ldc, second);
-}
+    __device__ __forceinline__ void store(const int4 (&regs)[4], int column) const {
+        uint32_t w[16], first[8], second[8];
+        memcpy(w, regs, sizeof(w));
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const uint32_t got = __shfl_xor_sync(0xffffffffu, upper ? w[j] : w[8 + j], 1);
+            first[j] = upper ? got : w[j];
+            second[j] = upper ? w[8 + j] : got;
+        }
+        st_global_256(even + column, first, even != nullptr);
+        st_global_256(odd + column, second, odd != nullptr);
+    }
+};
 
 // Same block, but every row goes to its own destination: lane l holds the address of row l (nullptr = drop the row).
 template <int kCols>
@@ -178,11 +184,17 @@ struct Cfg {
     // plain BF16 with MN-major B: a column count that is an odd multiple of 128 ends in one tile of half the width
     static constexpr bool kRagged = !kFp8 && !kSwiGLU && kBlockN == 256;
     static constexpr int kEpiWarps = (kPromote || kSplitDrain) ? 8 : 4;
-    static constexpr int kThreads = 64 + 32 * kEpiWarps;
     // first row and rows of every group in shared memory too: read from global memory they cost an epilogue that has little else to do 500 cycles a tile
-    static constexpr bool kGroupTable = !kFp8 && !kSwiGLU;
+    static constexpr bool kGroupTable = !kMx;
     static constexpr bool kWidePromote = kPromote && kBlockN == 256;
-    static constexpr int kOutStageBytes = kRowScatter ? 8192 : (kSplitDrain || kWidePromote ? 2048 : 4096);    // per epilogue warp: 32 rows x 32 / 64 (128) BF16
+    // 128 accumulators per thread and two buffers of 32 columns do not fit the 168 registers that ten warps get: with the epilogue in warpgroups of its own, the
+    // loader's and issuer's (and two warps that have nothing to do) hand theirs over. The sum is what the block was launched with: 3 x 168.
+    static constexpr bool kMoveRegs = kWidePromote;
+    static constexpr int kLaunchRegs = 168, kSmallRegs = 56, kEpiRegs = 224;
+    static_assert(kSmallRegs + 2 * kEpiRegs <= 3 * kLaunchRegs, "a split above the launch's registers waits forever");
+    static constexpr int kFirstEpi = kMoveRegs ? 4 : 2;  // first warp of the epilogue
+    static constexpr int kThreads = 32 * (kFirstEpi + kEpiWarps);
+    static constexpr int kOutStageBytes = kWidePromote ? 0 : kRowScatter ? 8192 : (kSplitDrain ? 2048 : 4096);    // per epilogue warp: 32 rows x 32 / 64 (128) BF16
     // kSplitDrain with quantised output: the two warps of a quarter exchange their half-row maxima here (two tile parities)
     static constexpr int kXchBytes = (kMx && kSwiGLU && kBlockN == 256) ? 2 * 2 * kBlockM * 8 : 0;
     static constexpr size_t kSmemBytes =
@@ -419,7 +431,9 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         }
     };
 
-    if (warp == 0) {
+    if (warp < C::kFirstEpi) {
+        if constexpr (C::kMoveRegs) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(C::kSmallRegs));
+        if (warp == 0) {
         // ================= TMA producer =================
         {
             int stage = 0, phase = 0, g = 0;
@@ -624,7 +638,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 }
             }
         }
-    } else if (warp == 1) {
+        } else if (warp == 1) {
         // ================= MMA issuer =================
         if (cta_rank == 0 && elect_one()) {
             const uint32_t idesc_full = kMx ? make_idesc_mx(kBlockN, C::kTileRows) : make_idesc<kFp8>(kBlockN, C::kTileRows, p.a_mn, p.b_mn);
@@ -737,12 +751,14 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             }
         }
         __syncwarp();
+        }
     } else {
         // ================= epilogue =================
+        if constexpr (C::kMoveRegs) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(C::kEpiRegs));
         const int q = warp & 3;                    // TMEM lane quarter this warp may read
-        const int half = (warp - 2) >> 2;          // FP8 only: which half of the columns this warp promotes
+        const int half = (warp - C::kFirstEpi) >> 2;          // FP8 only: which half of the columns this warp promotes
         const int row_in_tile = q * 32 + lane;
-        int4* out_stage = reinterpret_cast<int4*>(out_stage_base + (size_t)(warp - 2) * C::kOutStageBytes);
+        int4* out_stage = reinterpret_cast<int4*>(out_stage_base + (size_t)(warp - C::kFirstEpi) * C::kOutStageBytes);
         int g = 0, win = 0, win_phase = 0;
         int xch_iter = 0;  // split drain: tiles whose row maxima went through the exchange so far
         (void)xch_iter;
@@ -783,37 +799,48 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 for (int h = 0; h < 2; ++h)
 #pragma unroll
                     for (int i = 0; i < 64; ++i) acc[h][i] = 0.f;
-                float n_a = 0.f, n_0 = 0.f, n_1 = 0.f;
-                auto fetch_scales = [&](int kb) {
-                    if (kb >= ti.num_kb || !warp_has_rows) return;
-                    n_a = __ldcg(sa_row + kb);
-                    n_0 = __ldg(sb0 + kb);
-                    if (kSwiGLU) n_1 = __ldg(sb1 + kb);
+                // scales are fetched two K blocks ahead: with one an L2 round trip under load is part of every block
+                float s_next[3] = {0.f, 0.f, 0.f}, s_far[3] = {0.f, 0.f, 0.f};
+                auto fetch_scales = [&](int kb, float (&s)[3]) {
+                    if (kb >= ti.num_kb) return;
+                    s[0] = __ldcg(sa_row + kb);
+                    s[1] = __ldg(sb0 + kb);
+                    if (kSwiGLU) s[2] = __ldg(sb1 + kb);
                 };
-                if (p.ready == nullptr) fetch_scales(0);  // (with arrival gating the rows' scales are there after the first wait: see below)
+                if (warp_has_rows && p.ready == nullptr) {  // (with arrival gating the rows' scales are there after the first wait: see below)
+                    fetch_scales(0, s_next);
+                    fetch_scales(1, s_far);
+                }
                 for (int kb = 0; kb < ti.num_kb; ++kb) {
                     if (!mbar_wait(&tmem_full[win], win_phase, abort_flag, limit, note, wait_id(5, tile, kb, warp))) {
                         ok = false;
                         break;
                     }
-                    if (kb == 0 && p.ready != nullptr) fetch_scales(0);
                     if (warp_has_rows) {
+                        if (kb == 0 && p.ready != nullptr) {
+                            fetch_scales(0, s_next);
+                            fetch_scales(1, s_far);
+                        }
                         tc_fence_after();
                         const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(win * kBlockN);
-                        const float s0 = n_a * n_0, s1 = kSwiGLU ? n_a * n_1 : s0;
-                        fetch_scales(kb + 1);
+                        uint32_t v[2][32];
+                        tmem_ld32(taddr + c0, v[0]);
+                        const float s0 = s_next[0] * s_next[1], s1 = kSwiGLU ? s_next[0] * s_next[2] : s0;
 #pragma unroll
-                        for (int c = 0; c < 8; ++c) {
-                            uint32_t v[16];
-                            tmem_ld16(taddr + (c < 4 ? c0 + c * 16 : c1 + (c - 4) * 16), v);
+                        for (int i = 0; i < 3; ++i) s_next[i] = s_far[i];
+                        fetch_scales(kb + 2, s_far);
+#pragma unroll
+                        for (int c = 0; c < 4; ++c) {
                             tmem_ld_wait();
-                            if (c == 7) {
+                            if (c < 3) {  // the next 32 columns are on their way while these are added
+                                tmem_ld32(taddr + (c + 1 < 2 ? c0 + 32 : c1 + (c - 1) * 32), v[(c + 1) & 1]);
+                            } else {
                                 tc_fence_before();
                                 __syncwarp();
                                 if (lane == 0) release_window(&tmem_empty[win]);
                             }
 #pragma unroll
-                            for (int i = 0; i < 16; ++i) acc[c / 4][(c & 3) * 16 + i] = fmaf(__uint_as_float(v[i]), c < 4 ? s0 : s1, acc[c / 4][(c & 3) * 16 + i]);
+                            for (int i = 0; i < 32; ++i) acc[c / 2][(c & 1) * 32 + i] = fmaf(__uint_as_float(v[c & 1][i]), c < 2 ? s0 : s1, acc[c / 2][(c & 1) * 32 + i]);
                         }
                     } else {
                         __syncwarp();
@@ -825,12 +852,13 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                     }
                 }
                 if (!ok) break;
-                const int rows_valid = min(32, ti.c_row_end - (ti.c_row + q * 32));
-                __nv_bfloat16* wbase = cbase + (size_t)(ti.c_row + q * 32) * ldc + ti.c_col;
-                if (rows_valid > 0) {
-#pragma unroll
-                    for (int c = 0; c < (kSwiGLU ? 64 : 128); c += 32) {
-                        int4 regs[4];
+                // Straight on, without branches: while a warp is here the tensor core runs two K blocks ahead at most, and a jump to instructions that
+                // were last fetched a tile ago takes some 800 cycles. 64 experts of 4096 -> 1408, 73 rows: 7400 -> 3000 cycles a tile with SwiGLU, 8000 -> 1500
+                // without; a K block 1430 -> 1150 with the columns below read ahead. Both products, us: 73 rows 227 / 223, 300 rows (second) 245 / 216.
+                if (warp_has_rows) {
+                    __nv_bfloat16* mine = scatter ? scat_ptr : row < ti.c_row_end ? crow : nullptr;
+                    if (mine != nullptr) mine += half * (kSwiGLU ? 64 : 128);
+                    auto columns = [&](int c, int4 (&regs)[4]) {
 #pragma unroll
                         for (int i = 0; i < 32; i += 8) {
                             float o[8];
@@ -838,9 +866,23 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                             for (int j = 0; j < 8; ++j) o[j] = kSwiGLU ? silu(acc[0][(c + i + j) & 63]) * acc[1][(c + i + j) & 63] : acc[c / 64][(c + i + j) & 63];
                             regs[i / 8] = pack8_bf16(o);
                         }
-                        const int col = half * (kSwiGLU ? 64 : 128) + c;
-                        if (scatter) store_block_scattered<32>(out_stage, regs, scat_ptr != nullptr ? scat_ptr + col : nullptr, lane);
-                        else store_block_coalesced<32>(out_stage, regs, wbase + col, ldc, rows_valid, lane);
+                    };
+                    if (__all_sync(0xffffffffu, (reinterpret_cast<uintptr_t>(mine) & 31) == 0)) {
+                        const RowPair rows(mine, lane);
+#pragma unroll
+                        for (int c = 0; c < (kSwiGLU ? 64 : 128); c += 32) {
+                            int4 regs[4];
+                            columns(c, regs);
+                            rows.store(regs, c);
+                        }
+                    } else if (mine != nullptr) {
+#pragma unroll
+                        for (int c = 0; c < (kSwiGLU ? 64 : 128); c += 32) {
+                            int4 regs[4];
+                            columns(c, regs);
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) reinterpret_cast<int4*>(mine + c)[i] = regs[i];
+                        }
                     }
                 }
             } else if constexpr (C::kPromote) {
@@ -1127,6 +1169,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                         if (dst != nullptr) *reinterpret_cast<int4*>(dst + piece * 8) = val;
                     }
                 } else {
+                    const RowPair rows(row < ti.c_row_end ? crow : nullptr, lane);
 #pragma unroll 1
                     for (int c = 0; c < (C::kRagged ? ti.n_cols : C::kOutCols); c += 64) {
                         uint32_t v[32], u[32];
@@ -1148,8 +1191,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                         if (scatter) {
                             store_block_scattered<64>(out_stage, regs, scat_ptr != nullptr ? scat_ptr + c : nullptr, lane);
                         } else if (direct) {
-                            store_block_direct(regs, wbase + c, ldc, rows_valid, lane);
-                            store_block_direct(regs + 4, wbase + c + 32, ldc, rows_valid, lane);
+                            rows.store(*reinterpret_cast<const int4(*)[4]>(regs), c);
+                            rows.store(*reinterpret_cast<const int4(*)[4]>(regs + 4), c + 32);
                         } else {
                             store_block_coalesced<64>(out_stage, regs, wbase + c, ldc, rows_valid, lane);
                         }
@@ -1166,10 +1209,10 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         }
     }
 
-    if (warp >= 2) {
+    if (warp >= C::kFirstEpi) {
         // rows scattered into other GPUs' memory are performed there before this kernel counts as finished
         if (p.row_info != nullptr) __threadfence_system();
-        if (p.trace != nullptr && warp == 2 && lane == 0) atomicMax(&p.trace[1], global_timer_ns());
+        if (p.trace != nullptr && warp == C::kFirstEpi && lane == 0) atomicMax(&p.trace[1], global_timer_ns());
     }
     tc_fence_before();
     __syncthreads();
@@ -1225,12 +1268,18 @@ cudaError_t launch_impl(const GroupedGemmArgs& a, cudaStream_t stream) {
     }
     if (!ok) return cudaErrorInvalidValue;
     auto kernel = grouped_gemm_kernel<kBlockN, kFp8, kSwiGLU, kPair, kMx, kRowScatter>;
-    static bool smem_opted_in[64] = {};  // per device, once: the attribute is sticky
+    static bool smem_opted_in[64] = {};  // per device, once: the attribute is sticky (and the registers do not change)
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64 || !smem_opted_in[dev]) {
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::kSmemBytes);
         if (e != cudaSuccess) return e;
+        if constexpr (C::kMoveRegs) {  // launched with fewer registers the epilogue would wait for more forever
+            cudaFuncAttributes attributes;
+            e = cudaFuncGetAttributes(&attributes, kernel);
+            if (e != cudaSuccess) return e;
+            if (attributes.numRegs != C::kLaunchRegs) return cudaErrorLaunchOutOfResources;
+        }
         if (dev >= 0 && dev < 64) smem_opted_in[dev] = true;
     }
     if constexpr (kPair) {

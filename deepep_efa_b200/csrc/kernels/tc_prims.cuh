@@ -333,10 +333,10 @@ __device__ __forceinline__ unsigned long long global_timer_ns() {
     return t;
 }
 
-// 32 bytes per lane; the address is a multiple of 32
-__device__ __forceinline__ void st_global_256(void* p, const uint32_t* v) {
-    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]),
-                 "r"(v[6]), "r"(v[7])
+// 32 bytes per lane where `on`; the address is a multiple of 32
+__device__ __forceinline__ void st_global_256(void* p, const uint32_t (&v)[8], bool on) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %9, 0;\n\t@p st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};\n\t}" ::"l"(p), "r"(v[0]), "r"(v[1]),
+                 "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"((uint32_t)on)
                  : "memory");
 }
 

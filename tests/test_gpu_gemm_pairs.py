@@ -305,3 +305,30 @@ def test_promotion_with_256_columns_scatters_rows(N):
     keep = where[at] >= 0
     want[where[at][keep].long().cuda()] = plain[at[keep].cuda()]
     assert torch.equal(dst, want)
+
+
+@pytest.mark.parametrize("swiglu,N,K", [(True, 512, 384), (False, 256, 128)])
+def test_promotion_with_256_columns_between_sectors(swiglu, N, K):
+    """Outputs that start on a multiple of 16 bytes only are stored by other instructions, with the same values."""
+    from deepep_efa_b200 import _ext
+    C = _ext.load()
+    C.gemm_clear_error(0)
+    torch.manual_seed(K)
+    rows = [1, 0, 31, 129]
+    starts, ends = _groups(rows, True)
+    G, M, width = len(rows), starts[-1], N // 2 if swiglu else N
+    a, b = torch.randn(M, K, device="cuda").to(torch.float8_e4m3fn), torch.randn(G, N, K, device="cuda").to(torch.float8_e4m3fn)
+    a_s, b_s = torch.rand(M, K // 128, device="cuda") + 0.1, torch.rand(G, N // 128, K // 128, device="cuda") * 0.1
+    assert C.promotion_columns(M, G, N, K, swiglu, True, sum(rows), 1) == 256
+    outs = []
+    for shift in (0, 8):
+        flat = torch.full((M * width + 16,), 7.0, dtype=torch.bfloat16, device="cuda")
+        out = flat[shift:shift + M * width].view(M, width)
+        C.grouped_gemm(a, b, _i32(starts), 0, swiglu, a_s, b_s, out, 1, m_ends=_i32(ends), rows_hint=sum(rows))
+        assert (flat[:shift] == 7.0).all() and (flat[shift + M * width:] == 7.0).all()
+        outs.append(out)
+    torch.cuda.synchronize()
+    assert C.gemm_error(0) == 0
+    assert torch.equal(*outs)
+    for g in range(G):
+        assert (outs[0][ends[g]:starts[g + 1]] == 7.0).all()
