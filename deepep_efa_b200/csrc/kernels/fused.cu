@@ -398,7 +398,7 @@ __global__ void __launch_bounds__(kEmLoneThreads, 3) em_dispatch_lone_kernel(con
                 if (i0 + k * 32 < n16) v[k] = ld_cached(src + i0 + k * 32);
 #pragma unroll
             for (int k = 0; k < kEmLoneLoads; ++k)
-                if (i0 + k * 32 < n16) st_stream(dst + i0 + k * 32, v[k]);
+                if (i0 + k * 32 < n16) st_once(dst + i0 + k * 32, v[k]);
         }
         for (int kb = lane; kb < num_kb; kb += 32) {
             const float scale = a.x_scales[(size_t)t * num_kb + kb];

@@ -36,7 +36,7 @@ __device__ __forceinline__ void reduce_row_span(const int4* __restrict__ src, in
             const int row = __shfl_sync(0xffffffffu, my_row, (k0 + kk) & 31);
             const bool ok = k0 + kk < num_k && row >= 0;
 #pragma unroll
-            for (int u = 0; u < U; ++u) v[kk][u] = (ok && i0 + u * 32 < n16) ? ld_stream(src + (size_t)row * n16 + i0 + u * 32) : make_int4(0, 0, 0, 0);
+            for (int u = 0; u < U; ++u) v[kk][u] = (ok && i0 + u * 32 < n16) ? ld_once(src + (size_t)row * n16 + i0 + u * 32) : make_int4(0, 0, 0, 0);
         }
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk) {

@@ -176,7 +176,7 @@ __global__ void __launch_bounds__(256) unpermute_bwd_kernel(const __nv_bfloat16*
 #pragma unroll
             for (int u = 0; u < U; ++u) {
                 const int i = i0 + u * 32 + lane;
-                x[u] = i < n16 ? ld_stream(ar + i) : make_int4(0, 0, 0, 0);
+                x[u] = i < n16 ? ld_once(ar + i) : make_int4(0, 0, 0, 0);
                 y[u] = i < n16 ? gr[i] : make_int4(0, 0, 0, 0);
             }
 #pragma unroll
@@ -190,7 +190,7 @@ __global__ void __launch_bounds__(256) unpermute_bwd_kernel(const __nv_bfloat16*
                     acc = fmaf(xf.x, yf.x, fmaf(xf.y, yf.y, acc));
                     yw[j] = f2_to_bf16x2(yf.x * sc, yf.y * sc);
                 }
-                if (i < n16) dr[i] = make_int4((int)yw[0], (int)yw[1], (int)yw[2], (int)yw[3]);
+                if (i < n16) st_once(dr + i, make_int4((int)yw[0], (int)yw[1], (int)yw[2], (int)yw[3]));
             }
         }
     }
