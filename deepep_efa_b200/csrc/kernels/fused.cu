@@ -356,41 +356,61 @@ __global__ void __launch_bounds__(kEmDispatchThreads, 6) em_dispatch_kernel(cons
     }
 }
 
-// A lone rank with the GPU to itself copies its quantised rows within its own memory, so experts need not complete in order: a CTA takes
-// one unit, a warp of it a row with all loads in flight. A warp that copied the eight rows of a unit one after the other waited for the
-// selection and twice for the row, eight times over (one B200, 4096 x 8 rows of 7 KB: 94 -> 83 us, 2.8 TB/s of writes).
+// A lone rank with the GPU to itself copies its quantised rows within its own memory, so experts need not complete in order: resident warps
+// walk over the rows of all units, each with all loads of a row in flight, and look the next row's selection up while they copy. A CTA per unit spent
+// two thirds of its life on finding the expert, the selection and the row one after the other (4096 x 8 rows of 7 KB 68 -> 61 us behind the exchange, 4000 x 8 of
+// 2 KB 36 -> 23).
 constexpr int kEmLoneThreads = 256;
 constexpr int kEmLoneLoads = 14;  // 7168 channels in one pass
+constexpr int kEmLoneCtasPerSm = 3;
+__host__ __device__ constexpr size_t em_lone_smem(int num_experts) { return (size_t)(3 * num_experts + 1) * sizeof(int); }
 
-__global__ void __launch_bounds__(kEmLoneThreads, 3) em_dispatch_lone_kernel(const __grid_constant__ EmDispatchArgs a) {
+__global__ void __launch_bounds__(kEmLoneThreads, kEmLoneCtasPerSm) em_dispatch_lone_kernel(const __grid_constant__ EmDispatchArgs a) {
     pdl_wait_predecessor();
     pdl_release_successor();
     const RankCtx& c = a.ctx;
     const int T = a.num_tokens, K = a.num_topk, E = a.num_experts, H = a.hidden;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    __shared__ int s_expert, s_first;
-    const int u = blockIdx.x;  // units of expert e: [unit_start[e], unit_start[e + 1])
-    if (tid == 0) s_expert = -1;
-    __syncthreads();
-    for (int e = tid; e < E; e += kEmLoneThreads) {
-        const int from = __ldg(a.unit_start + e);
-        if (from <= u && u < __ldg(a.unit_start + e + 1)) {
-            s_expert = e;
-            s_first = (u - from) * a.unit_rows;
+    const int tid = threadIdx.x, lane = tid & 31;
+    extern __shared__ int s_lone[];
+    int *s_start = s_lone, *s_count = s_lone + E + 1, *s_base = s_count + E;  // units of expert e: [s_start[e], s_start[e + 1])
+    for (int e = tid; e <= E; e += kEmLoneThreads) {
+        s_start[e] = a.unit_start[e];
+        if (e < E) {
+            s_count[e] = a.my_counts[e];
+            s_base[e] = a.send_base[e];
         }
     }
     __syncthreads();
-    const int e = s_expert, s0 = s_first;
-    if (e < 0) return;  // the grid is sized for the most units there can be
-    const int n = min(a.unit_rows, a.my_counts[e] - s0), base_row = a.send_base[e] + s0;
     char* rows = reinterpret_cast<char*>(a.peer_bases[0]);
     char* scales = reinterpret_cast<char*>(a.peer_bases[1]);
     int* info = reinterpret_cast<int*>(a.peer_bases[2]);
     const int n16 = H / 16, num_kb = H / 128;
-    for (int s = warp; s < n; s += kEmLoneThreads / 32) {
-        const int sel = a.sel_list[(size_t)e * T + s0 + s], t = sel / K, row = base_row + s;
+    const int items = s_start[E] * a.unit_rows, step = gridDim.x * (kEmLoneThreads / 32);
+    int sel = -1, row = 0;
+    auto find = [&](int item) {  // selection and row of an item, -1 where a unit has no such row
+        sel = -1;
+        if (item >= items) return;
+        const int u = item / a.unit_rows;
+        int lo = 0, hi = E;  // the last expert whose units start at or before u (experts without rows have none)
+        while (hi - lo > 1) {
+            const int mid = (lo + hi) / 2;
+            if (s_start[mid] <= u) lo = mid;
+            else hi = mid;
+        }
+        const int s = (u - s_start[lo]) * a.unit_rows + item % a.unit_rows;
+        if (s >= s_count[lo]) return;
+        sel = a.sel_list[(size_t)lo * T + s];
+        row = s_base[lo] + s;
+    };
+    int item = blockIdx.x * (kEmLoneThreads / 32) + (tid >> 5);
+    find(item);
+    for (; item < items; item += step) {
+        const int mine = sel, dst_row = row;
+        find(item + step);
+        if (mine < 0) continue;
+        const int t = mine / K;
         const int4* src = reinterpret_cast<const int4*>(reinterpret_cast<const char*>(a.x) + (size_t)t * H);
-        int4* dst = reinterpret_cast<int4*>(rows + (size_t)row * H);
+        int4* dst = reinterpret_cast<int4*>(rows + (size_t)dst_row * H);
         for (int i0 = lane; i0 < n16; i0 += 32 * kEmLoneLoads) {
             int4 v[kEmLoneLoads];
 #pragma unroll
@@ -403,24 +423,28 @@ __global__ void __launch_bounds__(kEmLoneThreads, 3) em_dispatch_lone_kernel(con
         for (int kb = lane; kb < num_kb; kb += 32) {
             const float scale = a.x_scales[(size_t)t * num_kb + kb];
             if (a.native_atoms)
-                *reinterpret_cast<uint32_t*>(scales + ((size_t)(row >> 7) * num_kb + kb) * 512 + (row & 31) * 16 + ((row >> 5) & 3) * 4) =
+                *reinterpret_cast<uint32_t*>(scales + ((size_t)(dst_row >> 7) * num_kb + kb) * 512 + (dst_row & 31) * 16 + ((dst_row >> 5) & 3) * 4) =
                     ((__float_as_uint(scale) >> 23) & 0xffu) * 0x01010101u;
-            else reinterpret_cast<float*>(scales)[(size_t)row * num_kb + kb] = scale;
+            else reinterpret_cast<float*>(scales)[(size_t)dst_row * num_kb + kb] = scale;
         }
         if (lane == 0) {
-            info[row] = sel;  // (source rank 0 << 24) | selection
-            if (a.dst_row != nullptr) a.dst_row[sel] = row;
+            info[dst_row] = mine;  // (source rank 0 << 24) | selection
+            if (a.dst_row != nullptr) a.dst_row[mine] = dst_row;
         }
     }
-    __syncthreads();
-    if (tid == 0) red_add_release_gpu(&c.my_ctrl()->em_arrived[e], (uint64_t)n);
+    // (nobody waits for a lone rank's arrivals within this kernel)
+    if (blockIdx.x == 0)
+        for (int e = tid; e < E; e += kEmLoneThreads)  // (without units after an overflow)
+            if (s_start[e + 1] > s_start[e]) red_add_release_gpu(&c.my_ctrl()->em_arrived[e], (uint64_t)s_count[e]);
 }
 
 cudaError_t launch_em_dispatch(const EmDispatchArgs* a, int nv, cudaStream_t stream) {
     if (a[0].hidden % 128 != 0 || a[0].num_sms < 1) return cudaErrorInvalidValue;
-    if (nv == 1 && a->ctx.num_ranks == 1 && a->num_sms >= 148 && a->x_scales != nullptr && a->ctx.debug_extent == 0 && a->trace == nullptr) {
-        const long long units = ((long long)a->num_tokens * a->num_topk + a->unit_rows - 1) / a->unit_rows + a->num_experts;
-        return launch_dependent(em_dispatch_lone_kernel, dim3((unsigned)units), kEmLoneThreads, 0, stream, *a);
+    if (nv == 1 && a->ctx.num_ranks == 1 && a->num_sms >= 148 && a->x_scales != nullptr && a->ctx.debug_extent == 0 && a->trace == nullptr &&
+        em_lone_smem(a->num_experts) <= 48 * 1024) {
+        const long long warps = (long long)a->num_tokens * a->num_topk + (long long)a->num_experts * (a->unit_rows - 1);  // at most
+        const int ctas = (int)std::min<long long>(148 * kEmLoneCtasPerSm, (warps + kEmLoneThreads / 32 - 1) / (kEmLoneThreads / 32));
+        return launch_dependent(em_dispatch_lone_kernel, dim3((unsigned)ctas), kEmLoneThreads, em_lone_smem(a->num_experts), stream, *a);
     }
     const size_t smem = (size_t)(a[0].num_experts + 1) * sizeof(int);
     return DX_LAUNCH_RANKED_PDL(em_dispatch_kernel, EmDispatchArgs, a, nv, a[0].num_sms, kEmDispatchThreads, smem, stream);
