@@ -420,18 +420,14 @@ class Buffer:
         rows, scales = x if isinstance(x, tuple) else (x, None)
         call = (rows, scales, num_tokens_per_rank, num_tokens_per_expert, is_token_in_rank, topk_idx, topk_weights, handle)
         how = (num_channels, expert_alignment, quantize_fp8, round_scale, 0 if cached else num_worst_tokens, num_sms)
-        native = _named("ep.dispatch", self._C.normal_dispatch)
         if not allocate_on_comm_stream and _on_callers_stream(previous_event, async_finish):
-            event = None
-            recv_x, recv_scales, recv_idx, recv_w, per_expert, new_handle = native([self.runtime], [call], *how)[0]
+            event = EventOverlap()
+            recv_x, recv_scales, recv_idx, recv_w, per_expert, new_handle = _named("ep.dispatch", self._C.normal_dispatch)([self.runtime], [call], *how)[0]
         else:
-            with _CommScope(self, previous_event, async_finish, allocate_on_comm_stream, call[:7]) as scope:
-                recv_x, recv_scales, recv_idx, recv_w, per_expert, new_handle = native([self.runtime], [call], *how)[0]
-                if not cached:
-                    rpm, cpm, rcpm, _, _, send_head = new_handle
-                    scope.outputs(rpm, cpm, rcpm, send_head)
-            event = scope.event
-        event = EventOverlap() if event is None else event
+            _check_comm_arguments(previous_event, async_finish, allocate_on_comm_stream)
+            native = _named("ep.dispatch", self._C.normal_dispatch_on)
+            recv_x, recv_scales, recv_idx, recv_w, per_expert, new_handle = native(self._comm_key(), _event_of(previous_event), async_finish, self.runtime, call, *how)
+            event = self._comm_event(async_finish, call[:7])
         if recv_scales is not None:
             recv_x = (recv_x, recv_scales)
         if cached:
@@ -454,29 +450,28 @@ class Buffer:
             return self._cpu.combine(x, handle, topk_weights, bias)
         self.check_status()
         num_sms = _normal_sms(config if config is not None else self.get_combine_config(self.group_size), config is not None, [self])
-        direct = not allocate_on_comm_stream and _on_callers_stream(previous_event, async_finish)
-        scope = None if direct else _CommScope(self, previous_event, async_finish, allocate_on_comm_stream)
         rpm, _, _, src_idx, _, send_head = handle
         if _DEBUG_CHECKS:
             validate_handle(handle, self.rank, self.group_size)
         assert x.dim() == 2 and x.dtype == torch.bfloat16 and x.size(0) == src_idx.size(0)
         b0, b1 = Buffer._unpack_bias(bias)
-        native = _named("ep.combine", self._C.normal_combine)
-        if direct:
-            out, out_w = native([self.runtime], [(x, topk_weights, send_head, rpm, b0, b1, None, None)], num_sms)[0]
+        call = (x, topk_weights, send_head, rpm, b0, b1)
+        if not allocate_on_comm_stream and _on_callers_stream(previous_event, async_finish):
+            out, out_w = _named("ep.combine", self._C.normal_combine)([self.runtime], [(*call, None, None)], num_sms)[0]
             return out, out_w, EventOverlap()
-        out = out_w = None
-        if not allocate_on_comm_stream:
-            # results are allocated here, on the caller's stream (see _CommScope.outputs_from_caller_stream)
-            out = torch.empty((send_head.size(0), x.size(1)), dtype=torch.bfloat16, device=x.device)
-            out_w = torch.empty((send_head.size(0), topk_weights.size(1)), dtype=torch.float32, device=x.device) if topk_weights is not None else None
-            scope.outputs_from_caller_stream(out, out_w)
-        scope.inputs = [t for t in (x, topk_weights, b0, b1) if t is not None]
-        with scope:
-            out, out_w = native([self.runtime], [(x, topk_weights, send_head, rpm, b0, b1, out, out_w)], num_sms)[0]
-            if allocate_on_comm_stream:
-                scope.outputs(out, out_w)
-        return out, out_w, scope.event
+        _check_comm_arguments(previous_event, async_finish, allocate_on_comm_stream)
+        native = _named("ep.combine", self._C.normal_combine_on)
+        out, out_w = native(self._comm_key(), _event_of(previous_event), async_finish, allocate_on_comm_stream, self.runtime, call, num_sms)
+        return out, out_w, self._comm_event(async_finish, (x, topk_weights, b0, b1))
+
+    def _comm_key(self) -> Tuple[int, int]:
+        stream = self._comm_stream
+        return stream.stream_id, stream.device_index
+
+    def _comm_event(self, async_finish: bool, inputs) -> EventOverlap:
+        if not async_finish:
+            return EventOverlap()
+        return EventOverlap(EventHandle(self._comm_stream), tuple(t for t in inputs if isinstance(t, torch.Tensor)))
 
     # Groups that span several NVLink domains (the reference's "internode" paths).
     def internode_dispatch(self, x, handle: Optional[Tuple] = None, num_tokens_per_rank: Optional[torch.Tensor] = None,
@@ -731,8 +726,8 @@ def _named(name: str, call):
 def _on_callers_stream(previous_event, async_finish) -> bool:
     """A call without ``previous_event`` and without ``async_finish`` is ordered behind the caller's stream on both sides, so it runs on that
     stream itself: no events, no ``record_stream``, no scope. Together with the straight line that a call of one rank takes in ``dispatch`` and ``combine``,
-    layout, dispatch and combine of 61 tokens, which wait for the host, went from 59 to 49 us. (A cached dispatch and a combine of 3001 tokens on the
-    communication stream, which take the line but not this form, went from 82 to 79, with runs that differ by as much.)"""
+    layout, dispatch and combine of 61 tokens, which wait for the host, went from 59 to 49 us. Other calls do the same in native code on the communication
+    stream (OnCommStream in bindings.cpp): a cached dispatch and a combine of 3001 tokens went from 77 to 52 us."""
     return not async_finish and (previous_event is None or previous_event.event is None or previous_event.event.event is None)
 
 
@@ -749,6 +744,18 @@ class _DispatchReq:
         self.quantize_fp8, self.round_scale = quantize_fp8, round_scale
 
 
+def _check_comm_arguments(previous_event, async_finish, allocate_on_comm_stream) -> None:
+    if allocate_on_comm_stream:
+        assert previous_event is not None and async_finish, "allocate_on_comm_stream requires previous_event and async_finish"
+
+
+def _event_of(previous_event) -> Optional[int]:
+    """The CUDA event that the communication stream waits for, None where it waits for the caller's stream."""
+    if previous_event is None or previous_event.event is None or previous_event.event.event is None:
+        return None
+    return previous_event.event.event.cuda_event
+
+
 class _CommScope:
     """Stream choreography of one collective call (reference contract: csrc/deep_ep.cpp:526-578, 845-876).
 
@@ -761,9 +768,7 @@ class _CommScope:
     GPU a few microseconds per hop. The native call keeps it in order with calls on the communication stream."""
 
     def __init__(self, buf: Buffer, previous_event, async_finish, allocate_on_comm_stream, inputs=()):
-        if allocate_on_comm_stream:
-            assert previous_event is not None and async_finish, \
-                "allocate_on_comm_stream requires previous_event and async_finish"
+        _check_comm_arguments(previous_event, async_finish, allocate_on_comm_stream)
         self.buf, self.prev, self.async_finish = buf, previous_event, async_finish
         self.inputs = [t for t in inputs if isinstance(t, torch.Tensor)]
         self._outputs: List[torch.Tensor] = []

@@ -51,6 +51,8 @@ struct NotifyArgs {
 };
 cudaError_t launch_notify(const NotifyArgs* a, int num_virtual, cudaStream_t stream);
 
+constexpr uint64_t kNoOffset = ~0ull;
+
 struct DispatchArgs {
     RankCtx ctx;
     const void* x;                // [T,hidden] bf16, or e4m3 when x_scales != nullptr
@@ -65,7 +67,7 @@ struct DispatchArgs {
     const int* rank_prefix_matrix;  // [R,R]
     int num_tokens, hidden, num_experts;
     int num_sms;
-    // Where MY received rows go (offsets inside my symmetric buffer); published to all peers.
+    // Where MY received rows go (offsets inside my symmetric buffer); published to all peers. A lone rank that has the source indices (cached) takes none.
     uint64_t recv_x_off, recv_scales_off, recv_topk_idx_off, recv_topk_w_off, recv_src_idx_off;
     int num_worst_tokens;         // >0: fill recv_topk_idx rows [num_recv, num_worst_tokens) with -1
 };

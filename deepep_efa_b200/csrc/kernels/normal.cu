@@ -344,7 +344,7 @@ __device__ __forceinline__ void dispatch_rows(const DispatchArgs& a, const PeerD
                 if (a.topk_weights != nullptr) s_dst[d].topk_w[(size_t)rows[d] * K + lane] = mine ? w : 0.f;
             }
         }
-        if (lane == 0) {
+        if (lane == 0 && a.recv_src_idx_off != kNoOffset) {
 #pragma unroll
             for (int d = 0; d < kRanks; ++d)
                 if (rows[d] >= 0) s_dst[d].src_idx[rows[d]] = t;
@@ -503,7 +503,7 @@ __global__ void __launch_bounds__(kLoneThreads, kQuant ? 5 : 4) dispatch_lone_ke
                     c.at<int64_t>(0, a.recv_topk_idx_off)[(size_t)row * K + lane] = mine ? e : -1;
                     if (a.topk_weights != nullptr) c.at<float>(0, a.recv_topk_w_off)[(size_t)row * K + lane] = mine ? a.topk_weights[(size_t)t * K + lane] : 0.f;
                 }
-                if (lane == 0) c.at<int>(0, a.recv_src_idx_off)[row] = t;
+                if (lane == 0 && a.recv_src_idx_off != kNoOffset) c.at<int>(0, a.recv_src_idx_off)[row] = t;
             }
         }
     }

@@ -10,7 +10,7 @@ Reference counterparts: ``EventHandle`` (csrc/event.hpp:9-40) and ``EventOverlap
 """
 from __future__ import annotations
 
-from typing import Any, Optional, Tuple
+from typing import Any, Dict, Optional, Tuple
 
 import torch
 
@@ -26,10 +26,20 @@ def _has_cuda() -> bool:
     return _HAS_CUDA
 
 
+_STREAMS: Dict[Tuple[int, int], "torch.cuda.Stream"] = {}
+
+
 def current_stream() -> "torch.cuda.Stream":
-    """``torch.cuda.current_stream()``. Told the device by number it need not work out which one is meant, which takes longer (about 4 us)
-    than all the rest."""
-    return torch.cuda.current_stream(torch.cuda.current_device())
+    """``torch.cuda.current_stream()``, which builds an object on every call (1.5 us, of which a call on the communication stream asks for four): the object
+    of a CUDA stream is kept by its address. PyTorch's streams live as long as the process, and for others the address is all that the object holds."""
+    device = torch.cuda.current_device()
+    key = (device, torch._C._cuda_getCurrentRawStream(device))
+    stream = _STREAMS.get(key)
+    if stream is None:
+        if len(_STREAMS) >= 256:
+            _STREAMS.clear()
+        stream = _STREAMS[key] = torch.cuda.current_stream(device)
+    return stream
 
 
 class EventHandle:

@@ -380,3 +380,37 @@ def test_captured_layout_replayed_after_larger_ones(warm):
             assert all(bool((t == 7).all()) for t in keep)
     finally:
         vc.destroy()
+
+
+@pytest.mark.parametrize("form", ["asynchronous", "allocated_there", "with_event_only"])
+def test_inputs_dropped_behind_calls_on_the_communication_stream(form):
+    """Inputs that die while the communication stream has yet to read them, results used on the caller's stream, and an event that was never recorded."""
+    from deepep_efa_b200 import Buffer
+    from deepep_efa_b200.utils.event import EventHandle, EventOverlap
+    vc, buf = _buffer()
+    try:
+        idx, _ = make_routing(T, E, K, "cuda", seed=3, masked_fraction=0.2)
+        x, y, bias = (make_tokens(T, H, "cuda", seed=s) for s in (3, 4, 5))
+        lay, _ = _layout(buf, idx)
+        recv, _, _, _, handle, _ = buf.dispatch(x, **lay)
+        y = y[:recv.size(0)].contiguous()
+        want = recv.clone(), buf.combine(y, handle, bias=bias)[0].clone()
+        how = dict(async_finish=form != "with_event_only", allocate_on_comm_stream=form == "allocated_there")
+        for _ in range(3):
+            parts = [t.clone() for t in (x, y, bias)]
+            torch.cuda.synchronize()
+            _delay(buf.comm_stream)
+            rows, _, _, _, _, first = buf.dispatch(parts[0], handle=handle, previous_event=Buffer.capture(), **how)
+            out, _, second = buf.combine(parts[1], handle, bias=parts[2], previous_event=EventOverlap(EventHandle(record=False)), **how)
+            extra = [first.extra_tensors, second.extra_tensors]
+            assert (extra == [None, None]) == (form == "with_event_only")
+            waits = first.event, second.event  # (without the objects that keep the inputs alive)
+            del parts, first, second, extra
+            keep = _overwrite([(T, H // 2), (want[0].size(0), H // 2)])
+            for event in waits:
+                if event is not None:
+                    event.current_stream_wait()
+            assert torch.equal(rows, want[0]) and torch.equal(out, want[1])
+            del rows, out, keep
+    finally:
+        vc.destroy()
