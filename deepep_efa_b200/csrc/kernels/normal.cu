@@ -154,7 +154,63 @@ __global__ void __launch_bounds__(kNotifyThreads, 1) notify_kernel(const __grid_
     if (cta_is_last(c.local_scratch + kTicketNotify, gridDim.x) && tid == 0) commit_seq(c, kFamNotify, seq);
 }
 
+// A lone rank exchanges nothing: the counts go from the layout's tensors to the host, and one CTA numbers the tokens. The general kernel takes the counts through
+// the words that peers would write, and reads every flag three times (us, before / after: 1 token 6.2 / 4.7, 777 5.7 / 4.6, 4096 6.0 / 4.9, 8192 9.0 / 8.1).
+__global__ void __launch_bounds__(kNotifyThreads, 1) notify_lone_kernel(const __grid_constant__ NotifyArgs a) {
+    pdl_wait_predecessor();
+    pdl_release_successor();
+    const int T = a.num_tokens, C = a.num_channels, tid = threadIdx.x;
+    __shared__ int s_warp_sums[kNotifyThreads / 32];
+    __shared__ int s_off[kNotifyThreads + 1];
+    // flags of this thread's tokens; up to 8192 tokens they stay in a register
+    const int per = (T + kNotifyThreads - 1) / kNotifyThreads;
+    const int begin = min(tid * per, T), end = min(begin + per, T);
+    auto flag = [&](int t) { return a.is_token_in_rank[t] ? 1u : 0u; };
+    unsigned bits = 0;
+    int cnt = 0;
+    if (per <= 8) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            if (begin + j < end) bits |= flag(begin + j) << j;
+        cnt = __popc(bits);
+    } else {
+        for (int t = begin; t < end; ++t) cnt += (int)flag(t);
+    }
+    if (tid == 0) {
+        const int total = a.num_tokens_per_rank[0];
+        a.rank_prefix_matrix[0] = total;
+        if (a.host_recv_counter != nullptr) *a.host_recv_counter = total;
+    }
+    const int al = a.expert_alignment;
+    for (int e = tid; e < a.num_experts && a.host_expert_counter != nullptr; e += kNotifyThreads)
+        a.host_expert_counter[e] = (a.num_tokens_per_expert[e] + al - 1) / al * al;
+    const int incl = warp_incl_scan(cnt);
+    if ((tid & 31) == 31) s_warp_sums[tid >> 5] = incl;
+    __syncthreads();
+    const int before = warp_incl_scan(s_warp_sums[tid & 31]);  // every warp for itself
+    int pos = incl - cnt + ((tid >> 5) > 0 ? __shfl_sync(0xffffffffu, before, (tid >> 5) - 1) : 0);
+    s_off[tid] = pos;
+    if (tid == kNotifyThreads - 1) s_off[kNotifyThreads] = pos + cnt;
+    for (int t = begin; t < end; ++t) {
+        const bool in = per <= 8 ? (bits >> (t - begin)) & 1u : flag(t) != 0;
+        a.send_head[t] = in ? pos : -1;
+        pos += in ? 1 : 0;
+    }
+    __syncthreads();
+    const int tpc = (T + C - 1) / C;  // channel ch covers the tokens [ch * tpc, (ch + 1) * tpc)
+    if (tid < C) {
+        const int b = min((tid + 1) * tpc, T);
+        const int owner = per > 0 ? min(b / per, kNotifyThreads) : 0;
+        int prefix = s_off[owner];
+        if (owner < kNotifyThreads)
+            for (int t = owner * per; t < b; ++t) prefix += (int)flag(t);
+        a.channel_prefix_matrix[tid] = prefix;
+        a.recv_channel_prefix_matrix[tid] = prefix;
+    }
+}
+
 cudaError_t launch_notify(const NotifyArgs* a, int nv, cudaStream_t stream) {
+    if (nv == 1 && a->ctx.num_ranks == 1) return launch_dependent(notify_lone_kernel, dim3(1), kNotifyThreads, 0, stream, *a);
     return DX_LAUNCH_RANKED_PDL(notify_kernel, NotifyArgs, a, nv, 1 + a[0].ctx.num_ranks, kNotifyThreads, 0, stream);
 }
 

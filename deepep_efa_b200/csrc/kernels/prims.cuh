@@ -99,6 +99,19 @@ __device__ __forceinline__ void st_stream(int4* p, const int4& v) {
                  : "memory");
 }
 
+// ---- thread-block clusters ----
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// The word that CTA `rank` of the cluster has at shared-memory address `own`.
+__device__ __forceinline__ int ld_cluster_s32(uint32_t own, int rank) {
+    uint32_t at;
+    int v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(own), "r"(rank));
+    asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(at) : "memory");
+    return v;
+}
+
 // ---------------------------------------------------------------------------------------------
 // bounded waiting
 // ---------------------------------------------------------------------------------------------

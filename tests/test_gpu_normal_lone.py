@@ -101,3 +101,34 @@ def test_named_ranges_and_handle_checks_are_of_the_path_that_runs(monkeypatch, a
             buf.combine(x[:T - 1], foreign, **how)
     finally:
         vc.destroy()
+
+
+@pytest.mark.parametrize("T", [0, 31, 256, 1024, 1025, 1056, 8192, 8193, 8200, 20000])
+@pytest.mark.parametrize("masked", [0.0, 0.7])
+def test_counts_and_positions_of_a_lone_rank(T, masked):
+    """Layout by one CTA, by a cluster and by tickets, and the numbering of the tokens that are sent, with the flags of up to eight tokens per thread and of more."""
+    from deepep_efa_b200.parallel.virtual import VirtualCluster
+    E, K, H = 72, 6, 128
+    vc = VirtualCluster(1, num_nvl_bytes=128 << 20, timeout_ms=5000)
+    buf = vc.buffers[0]
+    try:
+        gen = torch.Generator(device="cuda").manual_seed(T)
+        idx = torch.rand(T, E, device="cuda", generator=gen).topk(K, dim=1).indices
+        idx[torch.rand(T, device="cuda", generator=gen) < masked] = -1  # tokens that stay at home
+        x = torch.randn(T, H, device="cuda", generator=gen).to(torch.bfloat16)
+        per_rank, _, per_expert, in_rank, _ = buf.get_dispatch_layout(idx, E)
+        sent = (idx >= 0).any(dim=1)
+        counts = torch.bincount(idx[idx >= 0], minlength=E)
+        assert per_rank.tolist() == [int(sent.sum())] and torch.equal(per_expert.long(), counts) and torch.equal(in_rank[:, 0], sent)
+        recv, recv_idx, _, per_expert_list, handle, _ = buf.dispatch(x, num_tokens_per_rank=per_rank, is_token_in_rank=in_rank, num_tokens_per_expert=per_expert,
+                                                                     topk_idx=idx, topk_weights=torch.ones(T, K, device="cuda"), expert_alignment=8)
+        rpm, cpm, rcpm, src_idx, _, head = handle
+        assert per_expert_list == ((counts + 7) // 8 * 8).tolist() and rpm.tolist() == [[int(sent.sum())]]
+        position = torch.where(sent, sent.cumsum(0) - 1, -1)
+        assert torch.equal(head[:, 0].long(), position) and torch.equal(src_idx.long(), sent.nonzero()[:, 0])
+        channels = cpm.size(1)
+        ends = [min((c + 1) * -(-T // channels), T) for c in range(channels)]
+        assert cpm[0].tolist() == [int(sent[:e].sum()) for e in ends] and torch.equal(cpm, rcpm)
+        assert torch.equal(recv, x[sent]) and torch.equal(recv_idx, idx[sent])
+    finally:
+        vc.destroy()
