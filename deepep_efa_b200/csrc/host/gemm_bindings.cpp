@@ -9,6 +9,7 @@
 #include <map>
 #include <mutex>
 
+#include "../kernels/api.h"
 #include "../kernels/gemm_api.h"
 #include "../kernels/gemm_choice.h"
 
@@ -68,7 +69,7 @@ torch::Tensor grouped_gemm(const torch::Tensor& a, const torch::Tensor& b, const
                            c10::optional<torch::Tensor> row_info, c10::optional<torch::Tensor> scatter_bases,
                            c10::optional<torch::Tensor> trace, bool mn_major, c10::optional<torch::Tensor> out_fp8,
                            c10::optional<torch::Tensor> out_atoms, bool m_ends_are_counts, c10::optional<torch::Tensor> sched, bool early_table, int tokens_as_columns,
-                           bool hold_successor, bool zero_tail, int64_t rows_hint) {
+                           bool hold_successor, bool zero_tail, int64_t rows_hint, c10::optional<torch::Tensor> out_scales = c10::nullopt) {
     DXG_CHECK(a.is_cuda() && b.is_cuda() && m_offsets.is_cuda(), "operands must be CUDA tensors");
     DXG_CHECK(a.is_contiguous() && b.is_contiguous() && m_offsets.is_contiguous(), "operands must be contiguous");
     DXG_CHECK(m_offsets.scalar_type() == torch::kInt32 && m_offsets.dim() == 1 && m_offsets.numel() >= 2, "m_offsets must be int32 [G+1]");
@@ -204,15 +205,46 @@ torch::Tensor grouped_gemm(const torch::Tensor& a, const torch::Tensor& b, const
         p.token_cap = tokens_as_columns == 1 ? 128 : tokens_as_columns;
         DXG_CHECK(p.token_cap >= 64 && p.token_cap <= 224 && p.token_cap % 32 == 0, "tokens_as_columns must be 0, 1 or a multiple of 32 from 64 to 224");
     }
-    if (out_fp8.has_value() || out_atoms.has_value()) {
-        DXG_CHECK(out_fp8.has_value() && out_atoms.has_value() && same_dev(out_fp8) && same_dev(out_atoms), "out_fp8 and out_atoms go together, on A's device");
-        DXG_CHECK(mode == 0 && swiglu && sfa_atoms.has_value() && p.mx_wide == 1, "quantised output needs the natively block-scaled kernel with wide SwiGLU tiles");
+    dx::Fp8CastArgs cast_after{};
+    if (out_fp8.has_value() || out_atoms.has_value() || out_scales.has_value()) {
+        DXG_CHECK(out_fp8.has_value() && out_atoms.has_value() != out_scales.has_value() && same_dev(out_fp8) && same_dev(out_atoms) && same_dev(out_scales),
+                  "out_fp8 goes with out_atoms or out_scales, on A's device");
         const int64_t inter = p.n / 2;
         DXG_CHECK(out_fp8->element_size() == 1 && out_fp8->is_contiguous() && out_fp8->numel() == (int64_t)p.m_total * inter, "out_fp8 must be e4m3 [M, N/2]");
-        DXG_CHECK(out_atoms->element_size() == 1 && out_atoms->is_contiguous() && out_atoms->numel() >= (((int64_t)p.m_total + 127) / 128) * (inter / 128) * 512,
-                  "out_atoms must be uint8 [ceil(M/128), N/2/128, 512]");
         p.c_fp8 = reinterpret_cast<uint8_t*>(out_fp8->data_ptr());
-        p.c_atoms = reinterpret_cast<uint8_t*>(out_atoms->data_ptr());
+        if (out_atoms.has_value()) {
+            DXG_CHECK(mode == 0 && swiglu && sfa_atoms.has_value() && p.mx_wide == 1, "quantised output needs the natively block-scaled kernel with wide SwiGLU tiles");
+            DXG_CHECK(out_atoms->element_size() == 1 && out_atoms->is_contiguous() && out_atoms->numel() >= (((int64_t)p.m_total + 127) / 128) * (inter / 128) * 512,
+                      "out_atoms must be uint8 [ceil(M/128), N/2/128, 512]");
+            p.c_atoms = reinterpret_cast<uint8_t*>(out_atoms->data_ptr());
+        } else {
+            // where tiles are narrow, a cast of BF16 rows follows
+            DXG_CHECK(mode == 0 && swiglu && fp8 && !sfa_atoms.has_value(), "out_scales is of products with fp32 scales and SwiGLU");
+            DXG_CHECK((reinterpret_cast<uintptr_t>(p.c_fp8) & 31) == 0 && inter % 128 == 0, "out_fp8 must be 32-byte aligned, N/2 a multiple of 128");
+            DXG_CHECK(out_scales->scalar_type() == torch::kFloat32 && out_scales->is_contiguous() && out_scales->numel() == (int64_t)p.m_total * (inter / 128),
+                      "out_scales must be f32 [M, N/2/128]");
+            if (dx::wide_promotion(p)) {
+                p.c_scales = out_scales->data_ptr<float>();
+            } else {
+                c = out.has_value() ? *out : torch::empty({p.m_total, inter}, c.options());
+                DXG_CHECK(c.numel() == (int64_t)p.m_total * inter, "out must be contiguous bf16 [M, N/2]");
+                p.c = c.data_ptr();
+                cast_after.x = reinterpret_cast<const __nv_bfloat16*>(p.c);
+                cast_after.out = p.c_fp8;
+                cast_after.scales = out_scales->data_ptr<float>();
+                cast_after.num_rows = p.m_total;
+                cast_after.hidden = (int)inter;
+                cast_after.rows_per_group = 1;
+                if (m_ends_are_counts) {
+                    DXG_CHECK(p.m_total % G == 0, "counts are of groups of equal room");
+                    cast_after.group_counts = p.m_ends;
+                    cast_after.rows_per_group = p.m_total / G;
+                } else {
+                    cast_after.num_rows_dev = p.m_offsets + G;
+                }
+                p.c_fp8 = nullptr;
+            }
+        }
     }
     p.early_table = early_table ? 1 : 0;
     p.hold_successor = hold_successor ? 1 : 0;
@@ -237,6 +269,8 @@ torch::Tensor grouped_gemm(const torch::Tensor& a, const torch::Tensor& b, const
         cudaGetLastError();
         throw std::runtime_error(std::string("deepep_efa_b200.grouped_gemm: launch failed: ") + cudaGetErrorString(e));
     }
+    if (cast_after.x != nullptr && dx::launch_fp8_cast(cast_after, at::cuda::getCurrentCUDAStream(device).stream()) != cudaSuccess)
+        throw std::runtime_error("deepep_efa_b200.grouped_gemm: launch of the cast failed");
     return c;
 }
 
@@ -398,20 +432,60 @@ torch::Tensor build_sf_atoms_b(const torch::Tensor& scales, int64_t n, bool swig
     return atoms;
 }
 
-// Both natively block-scaled products of an expert layer whose first one quantises its own output (wide tiles, or tokens as columns): rows
-// a [M, H] with power-of-two scales, groups of whole 128-row tiles -> bf16 [M, H]. One call from the host's side, because a short prompt's
-// GPU waits for each of these launches (8 experts of 3072 -> 1920, 273 tokens: four calls and two allocations were 5 us more per layer).
-torch::Tensor fp8_experts(const torch::Tensor& a, const torch::Tensor& a_scales, const torch::Tensor& w13, const torch::Tensor& w2, const torch::Tensor& m_offsets,
-                          const torch::Tensor& m_ends, const torch::Tensor& atoms13, const torch::Tensor& atoms2, double timeout_ms, int tokens_as_columns) {
-    DXG_CHECK(a.dim() == 2 && a.size(0) % 128 == 0 && w13.dim() == 3, "a must be [M, H] in whole tiles of 128 rows, w13 [G, 2 I, H]");
+// Expert-major rows of a dispatch result in e4m3 and their scales in one launch: (rows [M, H], scales [M, H/128], or scale atoms [M/128, H/128, 512]).
+std::tuple<torch::Tensor, torch::Tensor> gather_quantised(const torch::Tensor& rows, const torch::Tensor& scales, const torch::Tensor& src_row, bool atoms,
+                                                          c10::optional<torch::Tensor> sched) {
+    DXG_CHECK(rows.is_cuda() && rows.dim() == 2 && rows.is_contiguous() && rows.scalar_type() == torch::kFloat8_e4m3fn && rows.size(1) % 128 == 0,
+              "rows must be contiguous e4m3 [N, H] on the GPU, H in whole scale blocks");
+    DXG_CHECK(scales.device() == rows.device() && scales.scalar_type() == torch::kFloat32 && scales.is_contiguous() && scales.dim() == 2 && scales.size(0) == rows.size(0) &&
+                  scales.size(1) == rows.size(1) / 128, "scales must be f32 [N, H/128] on the rows' GPU");
+    DXG_CHECK(src_row.device() == rows.device() && src_row.scalar_type() == torch::kInt32 && src_row.is_contiguous() && src_row.dim() == 1, "src_row must be int32 [M]");
+    const int64_t M = src_row.numel(), H = rows.size(1);
+    DXG_CHECK(!atoms || M % 128 == 0, "scale atoms need whole tiles of 128 rows");
+    c10::cuda::CUDAGuard guard(rows.device());
+    const torch::Tensor out = torch::empty({M, H}, rows.options());
+    const torch::Tensor s = atoms ? torch::empty({M / 128, H / 128, 512}, rows.options().dtype(torch::kUInt8)) : torch::empty({M, H / 128}, scales.options());
+    const cudaError_t e = dx::launch_gather_quantised(rows.data_ptr(), scales.data_ptr<float>(), out.data_ptr(), atoms ? nullptr : s.data_ptr<float>(),
+                                                      atoms ? s.data_ptr<uint8_t>() : nullptr, src_row.data_ptr<int>(), (int)M, (int)H,
+                                                      sched.has_value() ? sched->data_ptr<int>() : nullptr, at::cuda::getCurrentCUDAStream(rows.get_device()).stream());
+    if (e != cudaSuccess) throw std::runtime_error(std::string("gather_quantised: ") + cudaGetErrorString(e));
+    return {out, s};
+}
+
+// Gather and both natively block-scaled products of an expert layer whose first one quantises its own output (wide tiles, or tokens as columns): the
+// received rows [N, H] with power-of-two scales -> bf16 [M, H] in the plan's order, groups of whole 128-row tiles. One call from the host's side, because a short
+// prompt's GPU waits for each of these launches. The plan was complete before the gather began, so the first product builds its table and
+// fetches weights beside it; tiles are drawn from a counter that the gather clears.
+torch::Tensor fp8_experts(const torch::Tensor& rows, const torch::Tensor& scales, const torch::Tensor& src_row, const torch::Tensor& w13, const torch::Tensor& w2,
+                          const torch::Tensor& m_offsets, const torch::Tensor& m_ends, const torch::Tensor& atoms13, const torch::Tensor& atoms2, double timeout_ms,
+                          int tokens_as_columns) {
+    DXG_CHECK(w13.dim() == 3 && w2.dim() == 3, "w13 must be [G, 2 I, H], w2 [G, H, I]");
     const auto none = c10::nullopt;
-    const int64_t inter = w13.size(1) / 2;
-    const torch::Tensor a_atoms = build_sf_atoms_a(a_scales, none, 0);
-    const torch::Tensor h = torch::empty({a.size(0), inter}, a.options()), h_atoms = torch::empty({a.size(0) / 128, inter / 128, 512}, a_atoms.options());
-    grouped_gemm(a, w13, m_offsets, 0, true, none, none, none, 0, timeout_ms, m_ends, a_atoms, atoms13, none, none, none, none, none, false, h, h_atoms, false, none,
-                 false, tokens_as_columns, false, false, 0);
-    return grouped_gemm(h, w2, m_offsets, 0, false, none, none, none, 0, timeout_ms, m_ends, h_atoms, atoms2, none, none, none, none, none, false, none, none, false, none,
-                        false, tokens_as_columns, false, false, 0);
+    const int64_t M = src_row.numel(), inter = w13.size(1) / 2;
+    if (M == 0) return torch::empty({0, w2.size(1)}, rows.options().dtype(torch::kBFloat16));
+    const torch::Tensor sched = torch::empty({2}, m_offsets.options());
+    const auto [a, a_atoms] = gather_quantised(rows, scales, src_row, true, sched);
+    const torch::Tensor h = torch::empty({M, inter}, a.options()), h_atoms = torch::empty({M / 128, inter / 128, 512}, a_atoms.options());
+    grouped_gemm(a, w13, m_offsets, 0, true, none, none, none, 0, timeout_ms, m_ends, a_atoms, atoms13, none, none, none, none, none, false, h, h_atoms, false, sched,
+                 true, tokens_as_columns, false, false, 0);
+    return grouped_gemm(h, w2, m_offsets, 0, false, none, none, none, 0, timeout_ms, m_ends, h_atoms, atoms2, none, none, none, none, none, false, none, none, false, sched,
+                        true, tokens_as_columns, false, false, 0);
+}
+
+// The same with fp32 scales.
+torch::Tensor fp8_experts_promoted(const torch::Tensor& rows, const torch::Tensor& scales, const torch::Tensor& src_row, const torch::Tensor& w13, const torch::Tensor& s13,
+                                   const torch::Tensor& w2, const torch::Tensor& s2, const torch::Tensor& m_offsets, const torch::Tensor& m_ends, double timeout_ms) {
+    DXG_CHECK(w13.dim() == 3 && w2.dim() == 3, "w13 must be [G, 2 I, H], w2 [G, H, I]");
+    const auto none = c10::nullopt;
+    const int64_t M = src_row.numel(), inter = w13.size(1) / 2;
+    if (M == 0) return torch::empty({0, w2.size(1)}, rows.options().dtype(torch::kBFloat16));
+    const torch::Tensor sched = torch::empty({2}, m_offsets.options());
+    const auto [a, a_scales] = gather_quantised(rows, scales, src_row, false, sched);
+    const torch::Tensor hq = torch::empty({M, inter}, a.options()), hs = torch::empty({M, inter / 128}, a_scales.options());
+    grouped_gemm(a, w13, m_offsets, 0, true, a_scales, s13, none, 0, timeout_ms, m_ends, none, none, none, none, none, none, none, false, hq, none, false, sched, true, 0, false,
+                 false, M, hs);
+    return grouped_gemm(hq, w2, m_offsets, 0, false, hs, s2, none, 0, timeout_ms, m_ends, none, none, none, none, none, none, none, false, none, none, false, sched, true, 0, false,
+                        false, M);
 }
 
 // What the rules of gemm_choice.h say about a product of these sizes (for the tests: they need no GPU). ends: whether m_ends is given.
@@ -462,8 +536,11 @@ void bind_gemm(py::module_& m) {
           py::arg("ready") = py::none(), py::arg("expected") = py::none(), py::arg("row_info") = py::none(),
           py::arg("scatter_bases") = py::none(), py::arg("trace") = py::none(), py::arg("mn_major") = false,
           py::arg("out_fp8") = py::none(), py::arg("out_atoms") = py::none(), py::arg("m_ends_are_counts") = false, py::arg("sched") = py::none(),
-          py::arg("early_table") = false, py::arg("tokens_as_columns") = 0, py::arg("hold_successor") = false, py::arg("zero_tail") = false, py::arg("rows_hint") = 0);
+          py::arg("early_table") = false, py::arg("tokens_as_columns") = 0, py::arg("hold_successor") = false, py::arg("zero_tail") = false, py::arg("rows_hint") = 0,
+          py::arg("out_scales") = py::none());
     m.def("fp8_experts", &fp8_experts);
+    m.def("fp8_experts_promoted", &fp8_experts_promoted);
+    m.def("gather_quantised", &gather_quantised, py::arg("rows"), py::arg("scales"), py::arg("src_row"), py::arg("atoms"), py::arg("sched") = py::none());
     m.def("build_plan", &build_plan);
     m.def("gather_rows", &gather_rows, py::arg("src"), py::arg("src_row"), py::arg("scale") = py::none(), py::arg("out") = py::none());
     m.def("gather_reduce_rows", &gather_reduce_rows, py::arg("src"), py::arg("pos"), py::arg("w") = py::none(), py::arg("out") = py::none());

@@ -76,6 +76,7 @@ struct GroupedGemmArgs {
     // c_atoms: the activation operand of the next natively block-scaled GEMM, without a cast pass in between.
     uint8_t* c_fp8;
     uint8_t* c_atoms;
+    float* c_scales;          // fp32 scales [M_total, N/2/128] instead of atoms, where tiles are promoted in 256 columns; c_fp8 32-byte aligned then
     // Optional [2], zero: tiles are drawn from a counter instead of dealt out in strides (single CTAs only; pairs ignore it). The
     // kernel leaves both words zero. Launches that may run at the same time need words of their own.
     int* sched;
@@ -113,6 +114,10 @@ cudaError_t launch_build_plan(const int64_t* topk_idx, const int* host_offsets, 
 //   are multiples of 4 bytes (of 16 when scaled).
 cudaError_t launch_gather_rows(const void* src, void* dst, const int* src_row, const float* scale, int num_dst_rows, int row_bytes,
                                cudaStream_t stream);
+// Rows of e4m3 with their fp32 scales per 128 channels (hidden % 128 == 0), gathered in one launch: scales as they are [num_dst_rows, hidden/128], or with
+// `atoms` as scale atoms (powers of two; whole tiles of 128 rows). Clears the two words at `sched` (may be null), for the products behind it.
+cudaError_t launch_gather_quantised(const void* src, const float* src_scales, void* dst, float* scales, uint8_t* atoms, const int* src_row, int num_dst_rows, int hidden,
+                                    int* sched, cudaStream_t stream);
 //   dst[n] = sum_k w[n,k] * src[pos[n,k]]  (bf16 rows, fp32 accumulate; pos < 0 skipped; w may be null = 1)
 cudaError_t launch_gather_reduce_rows(const void* src, void* dst, const int* pos, const float* w, int num_dst_rows, int num_k, int hidden,
                                       cudaStream_t stream);

@@ -196,7 +196,7 @@ struct Cfg {
     static constexpr int kThreads = 32 * (kFirstEpi + kEpiWarps);
     static constexpr int kOutStageBytes = kWidePromote ? 0 : kRowScatter ? 8192 : (kSplitDrain ? 2048 : 4096);    // per epilogue warp: 32 rows x 32 / 64 (128) BF16
     // kSplitDrain with quantised output: the two warps of a quarter exchange their half-row maxima here (two tile parities)
-    static constexpr int kXchBytes = (kMx && kSwiGLU && kBlockN == 256) ? 2 * 2 * kBlockM * 8 : 0;
+    static constexpr int kXchBytes = ((kMx || kPromote) && kSwiGLU && kBlockN == 256) ? 2 * 2 * kBlockM * 8 : 0;
     static constexpr size_t kSmemBytes =
         (size_t)kStages * kStageBytes + (size_t)kEpiWarps * kOutStageBytes + 1024 /*align*/ + 256 /*barriers*/ + (kMaxGroups + 2) * 4 + kXchBytes +
         (kGroupTable ? kMaxGroups * 8 : 0);
@@ -767,6 +767,31 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         __nv_bfloat16* cbase = reinterpret_cast<__nv_bfloat16*>(p.c);
         const int ldc = p.mode == 0 ? (kSwiGLU ? p.n / 2 : p.n) : p.k;
         const bool scatter = !kSwiGLU && p.mode == 0 && p.row_info != nullptr;
+        // Maximum over a row's 128 columns, whose other 64 are the partner warp's of this quarter: the two exchange theirs through shared memory,
+        // tagged with the tile's number, two tile parities.
+        auto row_maximum = [&](float& amax, int tile) {
+            const int par = xch_iter & 1;
+            ++xch_iter;
+            const unsigned tag = (unsigned)tile + 1u;
+            xch[(par * 2 + half) * kBlockM + row_in_tile] = ((unsigned long long)tag << 32) | __float_as_uint(amax);
+            volatile unsigned long long* other = xch + (par * 2 + (half ^ 1)) * kBlockM + row_in_tile;
+            unsigned long long w = *other;
+            bool there = true;
+            if ((unsigned)(w >> 32) != tag) {
+                const long long t0 = clock64();
+                while ((unsigned)((w = *other) >> 32) != tag) {
+                    if (*abort_flag || clock64() - t0 > limit) {
+                        if (!*abort_flag && note != nullptr) atomicCAS(note, 0ull, wait_id(7, tile, 0, warp));
+                        *abort_flag = 1;
+                        there = false;
+                        break;
+                    }
+                }
+            }
+            amax = fmaxf(amax, __uint_as_float((unsigned)w));
+            return __all_sync(0xffffffffu, there) != 0;
+        };
+        (void)row_maximum;
         const bool direct = (reinterpret_cast<uintptr_t>(p.c) & 31) == 0;  // (rows are multiples of 256 bytes apart)
         for (int tile = sched_id; tile < total_tiles && ok; tile = next_tile(tile)) {
             decode(tile, g, ti);
@@ -867,7 +892,55 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                             regs[i / 8] = pack8_bf16(o);
                         }
                     };
-                    if (__all_sync(0xffffffffu, (reinterpret_cast<uintptr_t>(mine) & 31) == 0)) {
+                    bool quantised = false;
+                    if constexpr (kSwiGLU) {
+                        if (p.c_fp8 != nullptr) {
+                            // the 128 output columns are one scale block of the next product's activations: what a cast of the BF16 rows would write
+                            quantised = true;
+                            int4 keep[8];
+                            float amax = 0.f;
+#pragma unroll
+                            for (int c = 0; c < 2; ++c) {
+                                int4 regs[4];
+                                columns(c * 32, regs);
+#pragma unroll
+                                for (int i = 0; i < 4; ++i) {
+                                    keep[c * 4 + i] = regs[i];
+                                    const uint32_t w4[4] = {(uint32_t)regs[i].x, (uint32_t)regs[i].y, (uint32_t)regs[i].z, (uint32_t)regs[i].w};
+#pragma unroll
+                                    for (int t = 0; t < 4; ++t) {
+                                        const float2 f = bf16x2_to_f2(w4[t]);
+                                        amax = fmaxf(amax, fmaxf(fabsf(f.x), fabsf(f.y)));
+                                    }
+                                }
+                            }
+                            ok = row_maximum(amax, tile);
+                            if (!ok) break;
+                            float scale, inv;
+                            fp8_scale_from_amax(amax, false, scale, inv);
+                            int4 q8[4];
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) {
+                                uint32_t out[4];
+#pragma unroll
+                                for (int h = 0; h < 2; ++h) {
+                                    const int4 v = keep[2 * i + h];
+                                    const float2 f0 = bf16x2_to_f2((uint32_t)v.x), f1 = bf16x2_to_f2((uint32_t)v.y);
+                                    const float2 f2 = bf16x2_to_f2((uint32_t)v.z), f3 = bf16x2_to_f2((uint32_t)v.w);
+                                    out[2 * h] = pack_e4m3x4(f0.x * inv, f0.y * inv, f1.x * inv, f1.y * inv);
+                                    out[2 * h + 1] = pack_e4m3x4(f2.x * inv, f2.y * inv, f3.x * inv, f3.y * inv);
+                                }
+                                q8[i] = make_int4((int)out[0], (int)out[1], (int)out[2], (int)out[3]);
+                            }
+                            const bool row_there = row < ti.c_row_end;
+                            uint8_t* dst = row_there ? p.c_fp8 + (size_t)row * ldc + ti.c_col + half * 64 : nullptr;
+                            // 64 bytes per row, like 32 BF16 columns
+                            RowPair(reinterpret_cast<__nv_bfloat16*>(dst), lane).store(q8, 0);
+                            if (half == 0 && row_there) p.c_scales[(size_t)row * (ldc / 128) + (ti.c_col >> 7)] = scale;
+                        }
+                    }
+                    if (quantised) {
+                    } else if (__all_sync(0xffffffffu, (reinterpret_cast<uintptr_t>(mine) & 31) == 0)) {
                         const RowPair rows(mine, lane);
 #pragma unroll
                         for (int c = 0; c < (kSwiGLU ? 64 : 128); c += 32) {
@@ -1041,26 +1114,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                                         amax = fmaxf(amax, fmaxf(fabsf(f.x), fabsf(f.y)));
                                     }
                                 }
-                            const int par = xch_iter & 1;
-                            ++xch_iter;
-                            const unsigned tag = (unsigned)tile + 1u;
-                            xch[(par * 2 + half) * kBlockM + row_in_tile] = ((unsigned long long)tag << 32) | __float_as_uint(amax);
-                            volatile unsigned long long* other = xch + (par * 2 + (half ^ 1)) * kBlockM + row_in_tile;
-                            unsigned long long w = *other;
-                            if ((unsigned)(w >> 32) != tag) {
-                                const long long t0 = clock64();
-                                while ((unsigned)((w = *other) >> 32) != tag) {
-                                    if (*abort_flag || clock64() - t0 > limit) {
-                                        if (!*abort_flag && note != nullptr) atomicCAS(note, 0ull, wait_id(7, tile, 0, warp));
-                                        *abort_flag = 1;
-                                        ok = false;
-                                        break;
-                                    }
-                                }
-                            }
-                            ok = __all_sync(0xffffffffu, ok);
+                            ok = row_maximum(amax, tile);
                             if (!ok) break;
-                            amax = fmaxf(amax, __uint_as_float((unsigned)w));
                             float scale, inv;
                             fp8_scale_from_amax(amax, true, scale, inv);
                             int4 q8[4];
@@ -1341,6 +1396,7 @@ cudaError_t launch_grouped_gemm(const GroupedGemmArgs& a, cudaStream_t stream) {
             if (a.swiglu) {
                 if ((a.n / 2) % 128 != 0) return cudaErrorInvalidValue;  // gate/up halves must start on scale-block boundaries
                 if (wide_promotion(a)) return launch_impl<256, true, true, false>(a, stream);
+                if (a.c_fp8 != nullptr) return cudaErrorInvalidValue;  // (a narrow tile holds half of a scale block)
                 return launch_sel<128, true, true>(a, stream);
             }
             if (a.n % 128 != 0) return cudaErrorInvalidValue;

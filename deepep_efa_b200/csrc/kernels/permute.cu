@@ -193,6 +193,50 @@ cudaError_t launch_gather_rows(const void* src, void* dst, const int* src_row, c
                             static_cast<const char*>(src), static_cast<char*>(dst), src_row, scale, num_dst_rows, row_bytes);
 }
 
+// e4m3 rows and their scales (num_kb per row) together: the scales of a row come and go with its first span, as floats or as the words of scale atoms (row r of
+// a tile at (r & 31) * 16 + (r >> 5) * 4 of the K block's 512 bytes). Two launches, or three with the atoms, cost a short prompt more than the copies.
+__global__ void __launch_bounds__(kPermThreads) gather_quantised_kernel(const char* __restrict__ src, const float* __restrict__ src_scales, char* __restrict__ dst,
+                                                                       float* __restrict__ scales, uint8_t* __restrict__ atoms, const int* __restrict__ src_row,
+                                                                       int* __restrict__ sched, int num_dst_rows, int hidden) {
+    pdl_wait_predecessor();
+    pdl_release_successor();
+    if (sched != nullptr && blockIdx.x == 0 && threadIdx.x < 2) sched[threadIdx.x] = 0;
+    const int lane = threadIdx.x & 31;
+    const int n16 = hidden / 16, num_kb = hidden / 128, spans = (n16 + kGatherSpan - 1) / kGatherSpan;
+    const int item = blockIdx.x * (kPermThreads / 32) + (threadIdx.x >> 5);
+    const int m = item / spans, span = item % spans;
+    if (m >= num_dst_rows) return;
+    const int s = src_row[m];
+    const int i0 = span * kGatherSpan + lane;
+    constexpr int U = kGatherSpan / 32;
+    int4 v[U];
+    const int4* p = reinterpret_cast<const int4*>(src + (size_t)max(s, 0) * hidden);
+#pragma unroll
+    for (int u = 0; u < U; ++u) v[u] = (s >= 0 && i0 + u * 32 < n16) ? __ldg(p + i0 + u * 32) : make_int4(0, 0, 0, 0);
+    if (span == 0) {
+        for (int kb = lane; kb < num_kb; kb += 32) {
+            const float f = s >= 0 ? src_scales[(size_t)s * num_kb + kb] : 0.f;
+            if (atoms != nullptr)
+                *reinterpret_cast<uint32_t*>(atoms + ((size_t)(m >> 7) * num_kb + kb) * 512 + (m & 31) * 16 + ((m >> 5) & 3) * 4) = ((__float_as_uint(f) >> 23) & 0xffu) * 0x01010101u;
+            else scales[(size_t)m * num_kb + kb] = f;
+        }
+    }
+    int4* d = reinterpret_cast<int4*>(dst + (size_t)m * hidden);
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+        if (i0 + u * 32 < n16) st_once(d + i0 + u * 32, v[u]);
+}
+
+cudaError_t launch_gather_quantised(const void* src, const float* src_scales, void* dst, float* scales, uint8_t* atoms, const int* src_row, int num_dst_rows, int hidden,
+                                    int* sched, cudaStream_t stream) {
+    if (num_dst_rows <= 0) return cudaSuccess;
+    if (hidden % 128 != 0 || hidden == 0 || (scales == nullptr) == (atoms == nullptr)) return cudaErrorInvalidValue;
+    const int spans = (hidden / 16 + kGatherSpan - 1) / kGatherSpan;
+    const long long warps = (long long)num_dst_rows * spans;
+    return launch_dependent(gather_quantised_kernel, dim3((unsigned)((warps + kPermThreads / 32 - 1) / (kPermThreads / 32))), kPermThreads, 0, stream,
+                            static_cast<const char*>(src), src_scales, static_cast<char*>(dst), scales, atoms, src_row, sched, num_dst_rows, hidden);
+}
+
 cudaError_t launch_gather_reduce_rows(const void* src, void* dst, const int* pos, const float* w, int num_dst_rows, int num_k, int hidden,
                                       cudaStream_t stream) {
     if (num_dst_rows <= 0) return cudaSuccess;

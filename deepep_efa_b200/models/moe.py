@@ -29,7 +29,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from ..ops import grouped_gemm as gg
-from ..ops.permute import build_expert_plan, gather_rows, permute, unpermute_weighted
+from ..ops.permute import build_expert_plan, permute, unpermute_weighted
 
 EXPERT_ALIGNMENT = 128
 
@@ -216,24 +216,20 @@ class MoELayer(nn.Module):
             x, num_tokens_per_rank=per_rank, is_token_in_rank=in_rank, num_tokens_per_expert=per_expert, topk_idx=topk_idx,
             topk_weights=topk_weights, expert_alignment=EXPERT_ALIGNMENT, quantize_fp8=True, round_scale=mx is not None)
         plan = build_expert_plan(recv_idx, counts)
-        a = gather_rows(rx, plan.src_row)
-        a_s = gather_rows(rs, plan.src_row)
-        how = dict(m_ends=plan.m_ends, timeout_ms=GEMM_TIMEOUT_MS)
         if mx is not None:
             # padding rows of the plan carry all-zero data; whatever exponent their zero scale maps to does not matter
             columns = _token_columns(buf.group_size * x.size(0) * self.cfg.num_topk / self.cfg.num_experts, w13.numel() + w2.numel(), self.cfg.hidden)
             if columns or plan.num_rows >= WIDE_TILE_MIN_ROWS_PER_EXPERT * self.num_local_experts:
                 # the first GEMM quantises its own output: a wide tile holds one whole scale block of a row
-                y_perm = C.fp8_experts(a, a_s, w13, w2, plan.m_offsets, plan.m_ends, mx[0], mx[3], GEMM_TIMEOUT_MS, columns)
+                y_perm = C.fp8_experts(rx, rs, plan.src_row, w13, w2, plan.m_offsets, plan.m_ends, mx[0], mx[3], GEMM_TIMEOUT_MS, columns)
             else:
-                h = C.grouped_gemm(a, w13, plan.m_offsets, 0, True, sfa_atoms=gg.build_sf_atoms_a(a_s), sfb_atoms=mx[2], **how)
+                how = dict(m_ends=plan.m_ends, timeout_ms=GEMM_TIMEOUT_MS)
+                a, a_atoms = C.gather_quantised(rx, rs, plan.src_row, True)
+                h = C.grouped_gemm(a, w13, plan.m_offsets, 0, True, sfa_atoms=a_atoms, sfb_atoms=mx[2], **how)
                 hq, hs = C.per_token_cast_to_fp8(h, True, False)
                 y_perm = C.grouped_gemm(hq, w2, plan.m_offsets, 0, False, sfa_atoms=gg.build_sf_atoms_a(hs), sfb_atoms=mx[1], **how)
         else:
-            how["rows_hint"] = plan.num_rows  # its row tiles are all in use
-            h = C.grouped_gemm(a, w13, plan.m_offsets, 0, True, a_s, s13, **how)
-            hq, hs = C.per_token_cast_to_fp8(h, False, False)
-            y_perm = C.grouped_gemm(hq, w2, plan.m_offsets, 0, False, hs, s2, **how)
+            y_perm = C.fp8_experts_promoted(rx, rs, plan.src_row, w13, s13, w2, s2, plan.m_offsets, plan.m_ends, GEMM_TIMEOUT_MS)
         y_recv = unpermute_weighted(y_perm, recv_w, plan, buf.empty_symmetric([rx.size(0), self.cfg.hidden], torch.bfloat16))
         out, _, _ = buf.combine(y_recv, handle)
         return out
@@ -309,8 +305,8 @@ class MoELayer(nn.Module):
                            m_ends_are_counts=True, sched=w_["sched"], early_table=True, tokens_as_columns=columns)
         else:
             arriving = max(1, R * x.size(0) * cfg.num_topk * L // cfg.num_experts)  # rows, on average
-            C.grouped_gemm(a, w13, w_["starts"], 0, True, a_s, s13, w_["h"], 0, GEMM_TIMEOUT_MS, cnt, m_ends_are_counts=True, sched=w_["sched"], rows_hint=arriving)
-            C.per_token_cast_to_fp8(w_["h"], False, False, cnt, N, w_["hq"], w_["hs"])
+            C.grouped_gemm(a, w13, w_["starts"], 0, True, a_s, s13, w_["h"], 0, GEMM_TIMEOUT_MS, cnt, m_ends_are_counts=True, sched=w_["sched"], rows_hint=arriving,
+                           out_fp8=w_["hq"], out_scales=w_["hs"])
             C.grouped_gemm(w_["hq"], w2, w_["starts"], 0, False, w_["hs"], s2, y.view(L * N, H), 0, GEMM_TIMEOUT_MS, cnt, m_ends_are_counts=True, sched=w_["sched"],
                            early_table=True, rows_hint=arriving)
         out, _, _ = buf.low_latency_combine(y, topk_idx, topk_weights, handle, zero_copy=True)
@@ -515,14 +511,17 @@ def fused_forward_many(layers, xs, idxs, ws, overlap: bool = True, num_dispatch_
                 else:
                     C.grouped_gemm(w.recv_x, w13[g0:g0 + ng], mo, 0, True, None, None, w.h, sms1, GEMM_TIMEOUT_MS, me_, w.recv_scales, sfb[g0:g0 + ng], **gate)
             else:
-                C.grouped_gemm(w.recv_x, w13[g0:g0 + ng], mo, 0, True, w.recv_scales, s13[g0:g0 + ng], w.h, sms1, GEMM_TIMEOUT_MS, me_, None, None, **gate)
+                # (a part of the experts alone does not say which rows to cast)
+                quantised = dict(out_fp8=w.hq, out_scales=w.hs) if len(parts) == 1 else {}
+                C.grouped_gemm(w.recv_x, w13[g0:g0 + ng], mo, 0, True, w.recv_scales, s13[g0:g0 + ng], w.h, sms1, GEMM_TIMEOUT_MS, me_, None, None, **gate, **quantised)
         if native:
             if not fuse_cast:
                 C.per_token_cast_to_fp8(w.h, True, False, None, 1, w.hq, w.hs, w.m_offsets[L:], True)
             C.grouped_gemm(w.hq, w2, w.m_offsets, 0, False, None, None, None, 0, GEMM_TIMEOUT_MS, w.m_ends, w.hs, l._mx[3 if wide2 else 1],
                            row_info=w.recv_info, scatter_bases=w.peer_bases[3 * R_:], sched=w.sched, early_table=True, tokens_as_columns=columns2)
         else:
-            C.per_token_cast_to_fp8(w.h, False, False, None, 1, w.hq, w.hs, w.m_offsets[L:], False)
+            if len(parts) > 1:
+                C.per_token_cast_to_fp8(w.h, False, False, None, 1, w.hq, w.hs, w.m_offsets[L:], False)
             C.grouped_gemm(w.hq, w2, w.m_offsets, 0, False, w.hs, s2, None, 0, GEMM_TIMEOUT_MS, w.m_ends, None, None,
                            row_info=w.recv_info, scatter_bases=w.peer_bases[3 * R_:], sched=w.sched, early_table=True, rows_hint=max(1, w.num_tokens * K))
     # every rank's second GEMM has finished scattering before anybody sums its stage

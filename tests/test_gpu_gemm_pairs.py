@@ -332,3 +332,53 @@ def test_promotion_with_256_columns_between_sectors(swiglu, N, K):
     assert torch.equal(*outs)
     for g in range(G):
         assert (outs[0][ends[g]:starts[g + 1]] == 7.0).all()
+
+
+@pytest.mark.parametrize("sms", [1, 148])  # tiles of 256 columns, which quantise their own output, and of 128 with a cast behind
+@pytest.mark.parametrize("counts", [False, True])
+def test_promotion_writes_quantised_output(sms, counts):
+    """The same e4m3 rows and scales, byte for byte, as a cast of the BF16 output; nothing behind a group's last row where the tiles write them."""
+    from deepep_efa_b200 import _ext
+    C = _ext.load()
+    C.gemm_clear_error(0)
+    torch.manual_seed(sms)
+    rows, K, inter = [1, 0, 31, 33, 128, 97], 384, 256
+    starts = list(range(0, 128 * len(rows) + 1, 128))
+    G, M = len(rows), starts[-1]
+    a, b = torch.randn(M, K, device="cuda").to(torch.float8_e4m3fn), torch.randn(G, 2 * inter, K, device="cuda").to(torch.float8_e4m3fn)
+    a_s, b_s = torch.rand(M, K // 128, device="cuda") * 0.02, torch.rand(G, 2 * inter // 128, K // 128, device="cuda") * 0.1
+    a.view(torch.uint8)[128 * 3 + 2] = 0  # a row of zeros: the smallest scale
+    assert C.promotion_columns(M, G, 2 * inter, K, True, True, sum(rows), sms) == (256 if sms == 1 else 128)
+    how = dict(m_ends=_i32(rows if counts else [s + n for s, n in zip(starts, rows)]), m_ends_are_counts=counts, rows_hint=sum(rows))
+    plain = torch.zeros(M, inter, device="cuda", dtype=torch.bfloat16)
+    C.grouped_gemm(a, b, _i32(starts), 0, True, a_s, b_s, plain, sms, **how)
+    want_q, want_s = C.per_token_cast_to_fp8(plain, False, False)
+    q, s = torch.full((M, inter), 7, device="cuda", dtype=torch.uint8), torch.full((M, inter // 128), 7.0, device="cuda")
+    C.grouped_gemm(a, b, _i32(starts), 0, True, a_s, b_s, torch.zeros_like(plain), sms, out_fp8=q.view(torch.float8_e4m3fn), out_scales=s, **how)
+    torch.cuda.synchronize()
+    assert C.gemm_error(0) == 0
+    for g, n in enumerate(rows):
+        r = slice(starts[g], starts[g] + n)
+        assert torch.equal(q[r], want_q.view(torch.uint8)[r]) and torch.equal(s[r], want_s[r])
+        if sms == 1:
+            assert (q[starts[g] + n:starts[g + 1]] == 7).all() and (s[starts[g] + n:starts[g + 1]] == 7).all()
+
+
+@pytest.mark.parametrize("H", [128, 1408, 4096, 7168])
+@pytest.mark.parametrize("atoms", [False, True])
+def test_gather_of_quantised_rows(H, atoms):
+    from deepep_efa_b200 import _ext
+    from deepep_efa_b200.ops.grouped_gemm import build_sf_atoms_a
+    from deepep_efa_b200.ops.permute import gather_rows
+    C = _ext.load()
+    torch.manual_seed(H)
+    N, M = 77, 384
+    rows = torch.randint(0, 255, (N, H), device="cuda", dtype=torch.uint8).view(torch.float8_e4m3fn)
+    scales = torch.exp2(torch.randint(-20, 20, (N, H // 128), device="cuda").float()) if atoms else torch.rand(N, H // 128, device="cuda")
+    src = torch.randint(-1, N, (M,), device="cuda", dtype=torch.int32)
+    sched = torch.full((2,), 9, device="cuda", dtype=torch.int32)
+    got, got_s = C.gather_quantised(rows, scales, src, atoms, sched)
+    want_s = gather_rows(scales, src)
+    assert torch.equal(got.view(torch.uint8), gather_rows(rows, src).view(torch.uint8)) and sched.tolist() == [0, 0]
+    assert torch.equal(got_s, build_sf_atoms_a(want_s) if atoms else want_s)
+    assert C.gather_quantised(rows, scales, src[:0], atoms)[0].shape == (0, H)
