@@ -58,8 +58,8 @@ inline bool wide_promotion(const GroupedGemmArgs& a) {
 
 // BF16 products with tokens as rows: whether a CTA pair shares a tile of 256 of them. For weight gradients all but those that read their operands in
 // place, which take pairs from 480 padded rows per expert on (with fewer the output is the work; both of 64 experts of 4096 -> 1408 in a loop, single / pair, us:
-// 242 rows 814 / 860, 384 rows 1041 / 1027, 512 rows 1297 / 1172; of 70 products of random sizes pairs take 1.2 to 1.5 of the time up to 350 padded rows, 0.97 to 1.15 up to 460,
-// 0.86 to 1.03 from 490 on); else where a pair's tile has little padding (first product of the same layer, 128 rows 255 / 316,
+// 242 rows 779 / 818, 384 rows 1025 / 963, 512 rows 1266 / 1131; of 160 products of random sizes pairs take 1.04 to 1.4 of the time up to 370 padded rows, 0.94 to 1.1 from 390 to
+// 470, 0.86 to 1.1 and 0.97 on average from 490 on); else where a pair's tile has little padding (first product of the same layer, 128 rows 255 / 316,
 // 242 rows 346 / 329, 512 rows 689 / 565; in whole steps at the power limit 270 to 430 rows lose 2 to 8 %). With ends and no zeros behind them
 // the number of rows is not known.
 inline bool rows_on_pairs(const GroupedGemmArgs& a) {

@@ -30,6 +30,9 @@ namespace dx {
 namespace {
 
 constexpr int kEdgeRows = 32;          // rows of one copy when a tile of A is fetched in part
+// Of the last K block of a weight gradient, where its reduction has no more left: half the bytes of a block that short reductions have two or three of (both of
+// 64 experts of 4096 -> 1408 in a loop, 94 rows 518 -> 490 us).
+constexpr int kTailRows = 32;
 constexpr int kAheadBlocks = 10;       // K blocks of weights per CTA fetched into L2 before the predecessor ends: 48 MB of the 126 MB
 
 __device__ __forceinline__ int4 pack8_bf16(const float* o) {
@@ -72,8 +75,8 @@ __device__ __forceinline__ void store_block_coalesced(int4* stage, const int4 (&
 // 32 rows x 32 BF16 columns, one row per lane, without shared memory: lanes 2i and 2i + 1 exchange halves, so that each store instruction writes 64
 // contiguous bytes of 16 rows. `gbase` and the row stride are multiples of 32 bytes.
 // Where the reduction is short the epilogue is the tile: through the staging buffer, with the group's table in global memory, a tile of 128 x 256 took 4500
-// cycles (20 to 94 rows per expert), now 3100. Both weight gradients of 64 experts of 4096 -> 1408 in a loop, us, before / after: 20 rows 559 / 453, 94 rows
-// 623 / 538, 190 rows 753 / 671, 384 rows 1061 / 1041, on pairs 768 rows 1563 / 1567. Whole lines of 128 bytes by two exchanges are no faster (94 rows 343 / 343
+// cycles (20 to 94 rows per expert), now 3100. Both weight gradients of 64 experts of 4096 -> 1408 in a loop, us, before / with this, kTailRows and kWgrad: 20 rows
+// 559 / 440, 94 rows 623 / 490, 190 rows 753 / 663, 384 rows 1061 / 1025, on pairs 768 rows 1563 / 1484. Whole lines of 128 bytes by two exchanges are no faster (94 rows 343 / 343
 // for the first), neither are eight epilogue warps on alternate tiles (361 / 369) or columns read from TMEM ahead (343 / 398).
 struct RowPair {
     __nv_bfloat16 *even, *odd;  // this lane's half of 32 columns of the rows of lanes 2i and 2i + 1 (nullptr: no such row)
@@ -145,6 +148,7 @@ struct TileInfo {
     int a_row, a_k0, b_row, b_row2, b_k0, num_kb, c_row, c_col, group, nblock, nblock2;
     int c_row_end;  // first output row this tile must not write (end of its group; groups need no 128-row alignment)
     int k_rows;     // weight gradients: rows of the reduction
+    int tail_kb;    // and the K block that holds at most kTailRows of them, MN-major (-1: none)
     int nt;         // n-tile index inside the group (kMx: selects the B scale atoms)
     int n_cols;     // columns of this tile: kBlockN, or half of it for the last column tile of an MN-major operand (kRagged)
     // MN-major operands: first tile row inside the tensor's contiguous dimension, and the tensor row of K index 0
@@ -202,11 +206,16 @@ struct Cfg {
         (kGroupTable ? kMaxGroups * 8 : 0);
 };
 
-template <int kBlockN, bool kFp8, bool kSwiGLU, bool kPair, bool kMx = false, bool kRowScatter = false>
+// kWgrad: weight gradients with both operands read in place. What is fixed for them costs no instructions (every launch fetches its code anew, and an MMA whose
+// operands are not known costs more to issue): 8 experts, 1408 x 1024, 512 rows 15.9 -> 15.5 us, 16 experts, 2816 x 1024, 320 rows 37.2 -> 36.1.
+template <int kBlockN, bool kFp8, bool kSwiGLU, bool kPair, bool kMx = false, bool kRowScatter = false, bool kWgrad = false>
 __global__ void __launch_bounds__((Cfg<kBlockN, kFp8, kSwiGLU, kPair, kMx, kRowScatter>::kThreads), 1)
 grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                     const __grid_constant__ CUtensorMap map_sfa, const __grid_constant__ CUtensorMap map_sfb, const GroupedGemmArgs p) {
     using C = Cfg<kBlockN, kFp8, kSwiGLU, kPair, kMx, kRowScatter>;
+    static_assert(!kWgrad || (!kFp8 && !kSwiGLU), "weight gradients are BF16");
+    const int mode = kWgrad ? 1 : p.mode, b_mn = kWgrad ? 1 : p.b_mn;
+    constexpr int a_mn = kWgrad ? 1 : 0;  // (nothing else takes A that way)
     static_assert(!kRowScatter || (kMx && !kSwiGLU && !kPair && kBlockN == 128), "whole-row scatter: natively block-scaled 128-column tiles");
     static_assert(!kMx || (kFp8 && ((!kPair && kBlockN == 128) || (kBlockN == 256 && (kSwiGLU || !kPair)))),
                   "native block scaling: e4m3 operands; 128-column tiles, 256-column tiles, or 256-column SwiGLU tiles on a CTA pair");
@@ -237,7 +246,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     const int G = p.num_groups;
     const int elem_per_kb = kFp8 ? 128 : 64;
     constexpr bool kMnMajor = !kFp8 && !kSwiGLU;    // instantiations that take MN-major operands
-    const int out_width = p.mode == 0 ? p.n : p.k;  // columns that the column tiles cover
+    const int out_width = mode == 0 ? p.n : p.k;  // columns that the column tiles cover
     const int col_tiles = C::kRagged ? (out_width + kBlockN - 1) / kBlockN : out_width / kBlockN;
 
     if (threadIdx.x == 0) {
@@ -258,7 +267,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         tma_prefetch_desc(&map_a);
         tma_prefetch_desc(&map_b);
     }
-    if (!kPair && p.mode == 0 && p.m_ends != nullptr) {  // see `edge` below
+    if (!kPair && mode == 0 && p.m_ends != nullptr) {  // see `edge` below
         for (int s = 0; s < C::kStages; ++s)
             for (int i = threadIdx.x; i < kATileBytes / 16; i += C::kThreads)
                 reinterpret_cast<int4*>(stage_base + (size_t)s * C::kStageBytes)[i] = make_int4(0, 0, 0, 0);
@@ -273,8 +282,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     }
     if (warp == 2) {
         // tile table: one warp scans the groups (one thread walking 256 groups through dependent loads took about 10 us)
-        const int tiles_n = p.mode == 0 ? col_tiles : 0;
-        const int tiles_fixed = p.mode == 1 ? ((p.n + C::kTileRows - 1) / C::kTileRows) * col_tiles : 0;
+        const int tiles_n = mode == 0 ? col_tiles : 0;
+        const int tiles_fixed = mode == 1 ? ((p.n + C::kTileRows - 1) / C::kTileRows) * col_tiles : 0;
         int run = 0;
         for (int g0 = 0; g0 < G; g0 += 32) {
             const int g = g0 + lane;
@@ -286,7 +295,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 if (kMx && (begin & 127) != 0 && p.error_flag != nullptr) atomicExch(p.error_flag, 2);
                 const int rows = group_rows(p, g, begin);
                 if (C::kGroupTable) group_table[g] = make_int2(begin, rows);
-                if (p.mode == 0) tiles = ((rows + C::kTileRows - 1) / C::kTileRows) * tiles_n;
+                if (mode == 0) tiles = ((rows + C::kTileRows - 1) / C::kTileRows) * tiles_n;
                 else tiles = tiles_fixed;
             }
             const int incl = warp_incl_scan(tiles);
@@ -321,7 +330,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         else own = make_int2(p.m_offsets[g], group_rows(p, g, p.m_offsets[g]));
         const int m0 = own.x, m1 = own.x + own.y;
         ti.group = g;
-        if (p.mode == 0) {
+        if (mode == 0) {
             const int tiles_m = (m1 - m0 + C::kTileRows - 1) / C::kTileRows;
             const int tiles_n_ = col_tiles;
             // order 0: consecutive tiles share the weight tile (n outer); order 1: they share the activation tile (m outer)
@@ -337,6 +346,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             ti.b_k0 = 0;
             ti.num_kb = p.k / elem_per_kb;
             ti.k_rows = 0;
+            ti.tail_kb = -1;
             ti.c_row = ti.a_row;
             ti.c_row_end = min(m1, p.m_total);
             if (kSwiGLU) {
@@ -367,6 +377,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             ti.b_k0 = m0;
             ti.k_rows = own.y;  // (with p.m_ends the rows behind it are zero in both operands)
             ti.num_kb = (ti.k_rows + elem_per_kb - 1) / elem_per_kb;
+            ti.tail_kb = kWgrad && ti.num_kb * 64 - ti.k_rows >= 64 - kTailRows ? ti.num_kb - 1 : -1;
             ti.c_row = g * p.n + ti.a_row;
             ti.c_row_end = min((g + 1) * p.n, p.num_groups * p.n);
             ti.c_col = jt * kBlockN;
@@ -406,13 +417,13 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     };
 
     if (p.early_table) {
-        if (warp == 0 && lane == 0 && p.mode == 0 && sched_id < total_tiles) {
+        if (warp == 0 && lane == 0 && mode == 0 && sched_id < total_tiles) {
             // weights of the first tile -> L2 while the predecessor's last tiles leave most SMs idle
             int g = 0;
             TileInfo ti;
             decode(sched_id, g, ti);
             for (int kb = 0; kb < min(ti.num_kb, kAheadBlocks); ++kb) {
-                if (kMnMajor && p.b_mn) break;
+                if (kMnMajor && b_mn) break;
                 tma_prefetch_2d(&map_b, ti.b_k0 + kb * elem_per_kb, (kSwiGLU && kPair && cta_rank == 1) ? ti.b_row2 : ti.b_row);
                 if (kSwiGLU && !kPair) tma_prefetch_2d(&map_b, ti.b_k0 + kb * elem_per_kb, ti.b_row2);
             }
@@ -467,7 +478,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 if (drawn && lane == 0) drawn_tile = atomicAdd(p.sched, 1);  // used when this tile's loads have been issued
                 decode(tile, g, ti);
                 if (lane == 0) s_prod_state[1] = tile;
-                if (p.ready != nullptr && ti.group != gated_group) {
+                if (!kWgrad && p.ready != nullptr && ti.group != gated_group) {
                     if (lane == 0) s_prod_state[0] = 1;
                     // the rows of this group come from other GPUs: wait until all of them have landed
                     const unsigned long long want = p.expected[ti.group];
@@ -496,7 +507,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 // clock (decode, 20 tokens: 177 us for the first GEMM over stale bytes, 142 with all 128 rows fetched, 138 over
                 // zeros). One or two copies of 32 rows replace the copy of 128; with three or four the loading lane would fall behind.
                 const int valid_rows = max(1, ti.c_row_end - ti.a_row);
-                const int edge = (!kPair && p.mode == 0 && p.m_ends != nullptr && valid_rows <= 2 * kEdgeRows) ? (valid_rows + kEdgeRows - 1) / kEdgeRows : 0;
+                const int edge = (!kPair && mode == 0 && p.m_ends != nullptr && valid_rows <= 2 * kEdgeRows) ? (valid_rows + kEdgeRows - 1) / kEdgeRows : 0;
                 if constexpr (kFp8 && !kPair) {
                     // The same for e4m3 operands with everything that does not change from one K block to the next in front of the loop: what the
                     // loading lane needs per K block is part of every stage's round trip.
@@ -552,11 +563,14 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                     if constexpr (kPair) {
                         // both CTAs fill their own stage and signal the LEADER's barrier, which expects the bytes of both
                         const uint32_t leader_full = mapa_shared(smem_u32(&full[stage]), 0);
+                        const bool tail = kWgrad && kb == ti.tail_kb;
                         if (elect_one()) {
-                            if (cta_rank == 0) mbar_expect_tx(&full[stage], 2 * C::kStageTxBytes);
-                            if (kMnMajor && p.a_mn) tma_load_3d_pair(&map_a, leader_full, sa, ti.a_kbase + kb * 64, ti.a_mn0 / 64);
+                            if (cta_rank == 0) mbar_expect_tx(&full[stage], tail ? C::kStageTxBytes : 2 * C::kStageTxBytes);
+                            if (tail) tma_load_3d_pair(&map_sfa, leader_full, sa, ti.a_kbase + kb * 64, ti.a_mn0 / 64);
+                            else if (kMnMajor && a_mn) tma_load_3d_pair(&map_a, leader_full, sa, ti.a_kbase + kb * 64, ti.a_mn0 / 64);
                             else tma_load_2d_pair(&map_a, leader_full, sa, ti.a_k0 + kb * elem_per_kb, ti.a_row);
-                            if (kMnMajor && p.b_mn) tma_load_3d_pair(&map_b, leader_full, sb, ti.b_kbase + kb * 64, ti.b_mn0 / 64);
+                            if (tail) tma_load_3d_pair(&map_sfb, leader_full, sb, ti.b_kbase + kb * 64, ti.b_mn0 / 64);
+                            else if (kMnMajor && b_mn) tma_load_3d_pair(&map_b, leader_full, sb, ti.b_kbase + kb * 64, ti.b_mn0 / 64);
                             else
                                 tma_load_2d_pair(&map_b, leader_full, sb, ti.b_k0 + kb * elem_per_kb,
                                                  (kSwiGLU && cta_rank == 1) ? ti.b_row2 : ti.b_row);  // SwiGLU: gate half / up half
@@ -582,16 +596,20 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                     const int filled = (int)(stage_rows >> (4 * stage)) & 7;
                     const int pieces = edge == 0 ? kBlockM / kEdgeRows : max(edge, filled);
                     stage_rows = (stage_rows & ~(7u << (4 * stage))) | ((unsigned)(edge == 0 ? kBlockM / kEdgeRows : edge) << (4 * stage));
+                    const bool tail = kWgrad && kb == ti.tail_kb;
                     if (elect_one()) {
-                        mbar_expect_tx(&full[stage], C::kStageTxBytes - kATileBytes + pieces * kEdgeRows * kKBlockBytes);
+                        mbar_expect_tx(&full[stage], tail ? C::kStageTxBytes / 2 : C::kStageTxBytes - kATileBytes + pieces * kEdgeRows * kKBlockBytes);
                         // (BF16 from here on)
-                        if (kMnMajor && p.a_mn) tma_load_3d(&map_a, &full[stage], sa, ti.a_kbase + kb * 64, ti.a_mn0 / 64);
+                        if (tail) tma_load_3d(&map_sfa, &full[stage], sa, ti.a_kbase + kb * 64, ti.a_mn0 / 64);
+                        else if (kMnMajor && a_mn) tma_load_3d(&map_a, &full[stage], sa, ti.a_kbase + kb * 64, ti.a_mn0 / 64);
                         else if (edge == 0) tma_load_2d(&map_a, &full[stage], sa, ti.a_k0 + kb * elem_per_kb, ti.a_row);
                         else
                             for (int j = 0; j < pieces; ++j)
                                 tma_load_2d(&map_sfa, &full[stage], sa + j * kEdgeRows * kKBlockBytes, ti.a_k0 + kb * elem_per_kb,
                                             j < edge ? ti.a_row + j * kEdgeRows : p.m_total);
-                        if (kMnMajor && p.b_mn) {
+                        if (tail) {
+                            tma_load_3d(&map_sfb, &full[stage], sb, ti.b_kbase + kb * 64, ti.b_mn0 / 64);
+                        } else if (kMnMajor && b_mn) {
                             tma_load_3d(&map_b, &full[stage], sb, ti.b_kbase + kb * 64, ti.b_mn0 / 64);
                         } else if (kSwiGLU) {
                             tma_load_2d(&map_b, &full[stage], sb, ti.b_k0 + kb * elem_per_kb, ti.b_row);
@@ -641,11 +659,11 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         } else if (warp == 1) {
         // ================= MMA issuer =================
         if (cta_rank == 0 && elect_one()) {
-            const uint32_t idesc_full = kMx ? make_idesc_mx(kBlockN, C::kTileRows) : make_idesc<kFp8>(kBlockN, C::kTileRows, p.a_mn, p.b_mn);
-            const uint32_t idesc_half = make_idesc<kFp8>(kBlockN / 2, C::kTileRows, p.a_mn, p.b_mn);
+            const uint32_t idesc_full = kMx ? make_idesc_mx(kBlockN, C::kTileRows) : make_idesc<kFp8>(kBlockN, C::kTileRows, a_mn, b_mn);
+            const uint32_t idesc_half = make_idesc<kFp8>(kBlockN / 2, C::kTileRows, a_mn, b_mn);
             // bytes (in 16-byte units) one K = 16 step moves the operand's start address: 32 B inside the swizzle atom when K
             // is contiguous, 16 K-steps of 128 B when the rows are
-            const uint64_t a_kstep = p.a_mn ? 128 : 2, b_kstep = p.b_mn ? 128 : 2;
+            const uint64_t a_kstep = a_mn ? 128 : 2, b_kstep = b_mn ? 128 : 2;
             int sf_buf = 0;  // native block scaling: which set of scale columns
             int stage = 0, phase = 0, g = 0;
             int win = 0, win_phase = 0;  // accumulator window ring
@@ -672,8 +690,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                     tc_fence_after();
                     const uint32_t sa = smem_u32(stage_base) + (uint32_t)(stage * C::kStageBytes);
                     const uint32_t sb = sa + kATileBytes;
-                    const uint64_t adesc = p.a_mn ? make_smem_desc_mn(sa) : make_smem_desc(sa);
-                    const uint64_t bdesc = p.b_mn ? make_smem_desc_mn(sb) : make_smem_desc(sb);
+                    const uint64_t adesc = a_mn ? make_smem_desc_mn(sa) : make_smem_desc(sa);
+                    const uint64_t bdesc = b_mn ? make_smem_desc_mn(sb) : make_smem_desc(sb);
                     const uint32_t tmem_d = tmem_base + (uint32_t)(win * kBlockN);
                     const bool window_done = C::kPromote ? true : (kb == ti.num_kb - 1);
                     {
@@ -699,7 +717,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                                             (new_window && j == 0) ? 0u : 1u);
                             }
                         } else {
-                            auto step = [&](int j) {
+                            auto step_at = [&](uint64_t adesc, uint64_t bdesc, int j) {
                                 // +32 bytes along K inside the swizzle atom = +2 in the 16-byte start-address field
                                 if constexpr (kPair)
                                     umma_pair<kFp8>(tmem_d, adesc + (uint64_t)j * a_kstep, bdesc + (uint64_t)j * b_kstep, idesc,
@@ -708,10 +726,15 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                                     umma<kFp8>(tmem_d, adesc + (uint64_t)j * a_kstep, bdesc + (uint64_t)j * b_kstep, idesc,
                                                (new_window && j == 0) ? 0u : 1u);
                             };
+                            auto step = [&](int j) { step_at(adesc, bdesc, j); };
                             // 16 K steps per MMA; those behind the last row of a weight gradient are left out, as are whole blocks of 64 (decode): both weight
                             // gradients of 64 experts of 4096 -> 1408, us, in a loop: 190 rows 781 -> 726, 384 rows 1065 -> 1044, 768 rows 1649 -> 1605.
                             // (Whole blocks keep their straight line of four: an MMA behind a branch costs three times as much to issue.)
-                            if (kMnMajor && p.mode == 1 && ti.k_rows - kb * 64 <= 48) {
+                            if (kWgrad && kb == ti.tail_kb) {
+                                const uint64_t at = make_smem_desc_mn(sa, kTailRows * 128), bt = make_smem_desc_mn(sb, kTailRows * 128);
+                                step_at(at, bt, 0);
+                                if (ti.k_rows - kb * 64 > 16) step_at(at, bt, 1);
+                            } else if (kMnMajor && mode == 1 && ti.k_rows - kb * 64 <= 48) {
                                 step(0);
                                 if (ti.k_rows - kb * 64 > 16) step(1);
                                 if (ti.k_rows - kb * 64 > 32) step(2);
@@ -765,8 +788,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         TileInfo ti;
         bool ok = true;
         __nv_bfloat16* cbase = reinterpret_cast<__nv_bfloat16*>(p.c);
-        const int ldc = p.mode == 0 ? (kSwiGLU ? p.n / 2 : p.n) : p.k;
-        const bool scatter = !kSwiGLU && p.mode == 0 && p.row_info != nullptr;
+        const int ldc = mode == 0 ? (kSwiGLU ? p.n / 2 : p.n) : p.k;
+        const bool scatter = !kSwiGLU && mode == 0 && p.row_info != nullptr;
         // Maximum over a row's 128 columns, whose other 64 are the partner warp's of this quarter: the two exchange theirs through shared memory,
         // tagged with the tile's number, two tile parities.
         auto row_maximum = [&](float& amax, int tile) {
@@ -1266,7 +1289,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 
     if (warp >= C::kFirstEpi) {
         // rows scattered into other GPUs' memory are performed there before this kernel counts as finished
-        if (p.row_info != nullptr) __threadfence_system();
+        if (!kWgrad && p.row_info != nullptr) __threadfence_system();
         if (p.trace != nullptr && warp == C::kFirstEpi && lane == 0) atomicMax(&p.trace[1], global_timer_ns());
     }
     tc_fence_before();
@@ -1294,7 +1317,7 @@ bool make_map_sf(CUtensorMap* map, const void* ptr, uint64_t rows, uint32_t word
     return r == CUDA_SUCCESS;
 }
 
-template <int kBlockN, bool kFp8, bool kSwiGLU, bool kPair, bool kMx = false, bool kRowScatter = false>
+template <int kBlockN, bool kFp8, bool kSwiGLU, bool kPair, bool kMx = false, bool kRowScatter = false, bool kWgrad = false>
 cudaError_t launch_impl(const GroupedGemmArgs& a, cudaStream_t stream) {
     using C = Cfg<kBlockN, kFp8, kSwiGLU, kPair, kMx, kRowScatter>;
     CUtensorMap map_a, map_b, map_sfa, map_sfb;
@@ -1320,9 +1343,12 @@ cudaError_t launch_impl(const GroupedGemmArgs& a, cudaStream_t stream) {
                      : make_map(&map_a, a.a, kFp8, (uint64_t)a.n, (uint64_t)a.m_total, kBlockM)) &&
              (a.b_mn ? make_map_mn(&map_b, a.b, (uint64_t)a.m_total, (uint64_t)a.k, C::kBRows)   // B given as [M, K_out]
                      : make_map(&map_b, a.b, kFp8, (uint64_t)a.k, (uint64_t)a.m_total, b_box_rows));
+        if (ok && a.a_mn)  // the maps of scale atoms are free: boxes of a reduction's last rows
+            ok = make_map_mn(&map_sfa, a.a, (uint64_t)a.m_total, (uint64_t)a.n, kBlockM, kTailRows) &&
+                 make_map_mn(&map_sfb, a.b, (uint64_t)a.m_total, (uint64_t)a.k, C::kBRows, kTailRows);
     }
     if (!ok) return cudaErrorInvalidValue;
-    auto kernel = grouped_gemm_kernel<kBlockN, kFp8, kSwiGLU, kPair, kMx, kRowScatter>;
+    auto kernel = grouped_gemm_kernel<kBlockN, kFp8, kSwiGLU, kPair, kMx, kRowScatter, kWgrad>;
     static bool smem_opted_in[64] = {};  // per device, once: the attribute is sticky (and the registers do not change)
     int dev = 0;
     cudaGetDevice(&dev);
@@ -1360,10 +1386,10 @@ cudaError_t launch_impl(const GroupedGemmArgs& a, cudaStream_t stream) {
 }
 
 // kPair chosen at run time (GroupedGemmArgs::cta_pairs)
-template <int kBlockN, bool kFp8, bool kSwiGLU>
+template <int kBlockN, bool kFp8, bool kSwiGLU, bool kWgrad = false>
 cudaError_t launch_sel(const GroupedGemmArgs& a, cudaStream_t stream) {
-    if (a.cta_pairs) return launch_impl<kBlockN, kFp8, kSwiGLU, true>(a, stream);
-    return launch_impl<kBlockN, kFp8, kSwiGLU, false>(a, stream);
+    if (a.cta_pairs) return launch_impl<kBlockN, kFp8, kSwiGLU, true, false, false, kWgrad>(a, stream);
+    return launch_impl<kBlockN, kFp8, kSwiGLU, false, false, false, kWgrad>(a, stream);
 }
 
 }  // namespace
@@ -1416,10 +1442,14 @@ cudaError_t launch_grouped_gemm(const GroupedGemmArgs& a, cudaStream_t stream) {
     }
     // K-grouped (weight gradients), bf16 only
     if (a.fp8 || a.swiglu || a.n % kBlockM != 0) return cudaErrorInvalidValue;
-    // as above (weight gradient of the same layer: 880 -> 680 us; with 128 rows per expert 216 -> 201 us)
-    if (a.k % 256 == 0 || (a.b_mn && a.k > 256 && a.k % 128 == 0)) return launch_sel<256, false, false>(a, stream);
-    if (a.k % 128 == 0) return launch_sel<128, false, false>(a, stream);
-    return cudaErrorInvalidValue;
+    if (a.k % 128 != 0) return cudaErrorInvalidValue;
+    if (a.a_mn) {
+        // 256-column tiles as above (weight gradient of the same layer: 880 -> 680 us; with 128 rows per expert 216 -> 201 us)
+        if (a.k >= 256) return launch_sel<256, false, false, true>(a, stream);
+        return launch_sel<128, false, false, true>(a, stream);
+    }
+    if (a.k % 256 == 0) return launch_sel<256, false, false>(a, stream);
+    return launch_sel<128, false, false>(a, stream);
 }
 
 }  // namespace dx

@@ -170,10 +170,10 @@ __device__ __forceinline__ uint64_t make_smem_desc(uint32_t smem_addr) {
 // MN-major operand tile (the tensor's contiguous dimension is the tile's row index, not K): the tile is stored as chunks of
 // 64 rows; a chunk is 64 K-steps of 128 bytes (64 BF16 row elements), 128B-swizzled in groups of 8 K-steps. Stride byte
 // offset = distance between 8-K-step groups (1024), leading byte offset = distance between 64-row chunks (8192).
-__device__ __forceinline__ uint64_t make_smem_desc_mn(uint32_t smem_addr) {
+__device__ __forceinline__ uint64_t make_smem_desc_mn(uint32_t smem_addr, uint32_t chunk_bytes = 8192) {
     uint64_t d = 0;
     d |= (uint64_t)((smem_addr & 0x3FFFF) >> 4);
-    d |= (uint64_t)(8192 >> 4) << 16;              // leading byte offset: next 64-row chunk
+    d |= (uint64_t)(chunk_bytes >> 4) << 16;       // leading byte offset: next 64-row chunk
     d |= (uint64_t)(1024 >> 4) << 32;              // stride byte offset: next group of 8 K-steps
     d |= (uint64_t)1 << 46;
     d |= (uint64_t)2 << 61;                        // SWIZZLE_128B
@@ -391,12 +391,12 @@ bool make_map(CUtensorMap* map, const void* ptr, bool fp8, uint64_t rows, uint64
 // [mn_cols / 64, k_rows, 64]: a box of `box_rows` operand rows x 64 K-steps lands as chunks of 64 rows (8 KiB each, 128B swizzle),
 // the order the matrix descriptor expects, in one copy. One copy per 64-row chunk cost the loading lane up to six instructions per
 // stage. Chunks past the last column read as zeros and touch no memory.
-bool make_map_mn(CUtensorMap* map, const void* ptr, uint64_t k_rows, uint64_t mn_cols, uint32_t box_rows) {
+bool make_map_mn(CUtensorMap* map, const void* ptr, uint64_t k_rows, uint64_t mn_cols, uint32_t box_rows, uint32_t k_steps = 64) {
     EncodeFn fn = get_encode_fn();
     if (fn == nullptr) return false;
     cuuint64_t dims[3] = {64, k_rows, mn_cols / 64};
     cuuint64_t strides[2] = {mn_cols * 2, 128};
-    cuuint32_t box[3] = {64, 64, box_rows / 64};
+    cuuint32_t box[3] = {64, k_steps, box_rows / 64};
     cuuint32_t estr[3] = {1, 1, 1};
     const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                           CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
