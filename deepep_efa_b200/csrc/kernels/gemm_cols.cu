@@ -105,6 +105,7 @@ token_cols_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
     if constexpr (kSwiGLU) {
         for (int i = threadIdx.x; i < 2 * cap * 4; i += kColsThreads) xch[i] = 0u;
     }
+    if (warp == 1) tmem_alloc(&s_tmem_base, 512);
     // early_table and hold_successor: see grouped_gemm.cu
     if (!p.early_table) {
         pdl_wait_predecessor();
@@ -115,22 +116,11 @@ token_cols_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
     const int step = cap < 128 ? 64 : cap < 192 ? 128 : 192;
     auto row_tiles = [&](int n) { return n <= 0 ? 0 : n <= cap ? 1 : step == 128 ? 1 + (n - cap + 127) / 128 : (n + step - 1) / step; };
     if (warp == 2) {
-        int run = 0;
-        for (int g0 = 0; g0 < G; g0 += 32) {
-            const int g = g0 + lane;
-            int tiles = 0;
-            if (g < G) {
-                const int begin = p.m_offsets[g];
-                if ((begin & 127) != 0 && p.error_flag != nullptr) atomicExch(p.error_flag, 2);
-                tiles = row_tiles(group_rows(p, g, begin)) * tiles_n;
-            }
-            const int incl = warp_incl_scan(tiles);
-            if (g < G) tile_start[g] = run + incl - tiles;
-            run += __shfl_sync(0xffffffffu, incl, 31);
-        }
-        if (lane == 0) tile_start[G] = run;
+        build_tile_table(p, tile_start, lane, [&](int, int begin, int rows) {
+            if ((begin & 127) != 0 && p.error_flag != nullptr) atomicExch(p.error_flag, 2);
+            return row_tiles(rows) * tiles_n;
+        });
     }
-    if (warp == 1) tmem_alloc(&s_tmem_base, 512);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();

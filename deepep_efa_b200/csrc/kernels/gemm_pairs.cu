@@ -86,6 +86,8 @@ token_pairs_gemm_kernel(const __grid_constant__ PairMaps maps, const GroupedGemm
         tma_prefetch_desc(&maps.w);
         for (int i = 0; i < 4; ++i) tma_prefetch_desc(&maps.t[i]);
     }
+    if (warp == 1) tmem_alloc_pair(&s_tmem_base, 2 * kPairWindowCols);
+    cluster_sync_all();  // the peer's barriers exist before anything signals them
     pdl_wait_predecessor();
     pdl_release_successor();
     // A group's rows in units of 32, cut into tiles of at most token_cap of them that differ by a unit at most. A group that has no rows but
@@ -97,24 +99,10 @@ token_pairs_gemm_kernel(const __grid_constant__ PairMaps maps, const GroupedGemm
         return (units + most - 1) / most;
     };
     if (warp == 2) {
-        int run = 0;
-        for (int g0 = 0; g0 < G; g0 += 32) {
-            const int g = g0 + lane;
-            int tiles = 0;
-            if (g < G) {
-                const int begin = p.m_offsets[g];
-                tiles = row_tiles(g, begin, group_rows(p, g, begin)) * feature_tiles;
-            }
-            const int incl = warp_incl_scan(tiles);
-            if (g < G) tile_start[g] = run + incl - tiles;
-            run += __shfl_sync(0xffffffffu, incl, 31);
-        }
-        if (lane == 0) tile_start[G] = run;
+        build_tile_table(p, tile_start, lane, [&](int g, int begin, int rows) { return row_tiles(g, begin, rows) * feature_tiles; });
     }
-    if (warp == 1) tmem_alloc_pair(&s_tmem_base, 2 * kPairWindowCols);
     tc_fence_before();
     __syncthreads();
-    cluster_sync_all();  // the peer's barriers exist before anything signals them
     tc_fence_after();
     const uint32_t tmem_base = s_tmem_base;
     const int total_tiles = tile_start[G];

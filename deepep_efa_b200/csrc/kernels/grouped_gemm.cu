@@ -273,6 +273,11 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 reinterpret_cast<int4*>(stage_base + (size_t)s * C::kStageBytes)[i] = make_int4(0, 0, 0, 0);
         fence_proxy_async();
     }
+    if (warp == 1) {
+        if constexpr (kPair) tmem_alloc_pair(&s_tmem_base, C::kTmemCols);
+        else tmem_alloc(&s_tmem_base, C::kTmemCols);
+    }
+    if constexpr (kPair) cluster_sync_all();  // the peer's barriers exist before anything signals them
     // What precedes overlaps the end of the previous kernel (programmatic dependent launch); from here on its results are read.
     // The successor is released only now, so that a kernel that starts early finds every kernel before this one complete.
     // With p.early_table the group table is older than the predecessor, so the tile table and the first weights do not wait for it.
@@ -281,39 +286,21 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         if (!p.hold_successor) pdl_release_successor();
     }
     if (warp == 2) {
-        // tile table: one warp scans the groups (one thread walking 256 groups through dependent loads took about 10 us)
         const int tiles_n = mode == 0 ? col_tiles : 0;
         const int tiles_fixed = mode == 1 ? ((p.n + C::kTileRows - 1) / C::kTileRows) * col_tiles : 0;
-        int run = 0;
-        for (int g0 = 0; g0 < G; g0 += 32) {
-            const int g = g0 + lane;
-            int tiles = 0;
-            if (g < G) {
-                const int begin = p.m_offsets[g];
-                // native block scaling reads one scale atom per 128-row tile, so a group that does not start on a tile boundary
-                // would be scaled with its neighbour's factors: flag it (value 2) instead of returning silently wrong numbers
-                if (kMx && (begin & 127) != 0 && p.error_flag != nullptr) atomicExch(p.error_flag, 2);
-                const int rows = group_rows(p, g, begin);
-                if (C::kGroupTable) group_table[g] = make_int2(begin, rows);
-                if (mode == 0) tiles = ((rows + C::kTileRows - 1) / C::kTileRows) * tiles_n;
-                else tiles = tiles_fixed;
-            }
-            const int incl = warp_incl_scan(tiles);
-            if (g < G) tile_start[g] = run + incl - tiles;
-            run += __shfl_sync(0xffffffffu, incl, 31);
-        }
-        if (lane == 0) tile_start[G] = run;
+        build_tile_table(p, tile_start, lane, [&](int g, int begin, int rows) {
+            // native block scaling reads one scale atom per 128-row tile, so a group that does not start on a tile boundary
+            // would be scaled with its neighbour's factors: flag it (value 2) instead of returning silently wrong numbers
+            if (kMx && (begin & 127) != 0 && p.error_flag != nullptr) atomicExch(p.error_flag, 2);
+            if (C::kGroupTable) group_table[g] = make_int2(begin, rows);
+            return mode == 0 ? ((rows + C::kTileRows - 1) / C::kTileRows) * tiles_n : tiles_fixed;
+        });
     }
     if constexpr (C::kXchBytes > 0) {
         for (int i = threadIdx.x; i < C::kXchBytes / 8; i += C::kThreads) xch[i] = 0ull;
     }
-    if (warp == 1) {
-        if constexpr (kPair) tmem_alloc_pair(&s_tmem_base, C::kTmemCols);
-        else tmem_alloc(&s_tmem_base, C::kTmemCols);
-    }
     tc_fence_before();
     __syncthreads();
-    if constexpr (kPair) cluster_sync_all();  // the peer's barriers exist before anything signals them
     tc_fence_after();
     const uint32_t tmem_base = s_tmem_base;
     const int total_tiles = tile_start[G];

@@ -355,6 +355,26 @@ __device__ __forceinline__ int group_rows(const GroupedGemmArgs& p, int g, int b
     return max(p.m_ends_are_counts ? p.m_ends[g] : p.m_ends[g] - begin, 0);
 }
 
+// Tile table, by one warp: tile_start[g] = tiles of the groups before g, tile_start[G] = all; tiles(g, first row, rows) says how many a group has.
+template <typename Tiles>
+__device__ __forceinline__ void build_tile_table(const GroupedGemmArgs& p, int* tile_start, int lane, Tiles&& tiles) {
+    const int G = p.num_groups;
+    int run = 0;
+#pragma unroll 1
+    for (int g0 = 0; g0 < G; g0 += 32) {
+        const int g = g0 + lane;
+        int n = 0;
+        if (g < G) {
+            const int begin = p.m_offsets[g];
+            n = tiles(g, begin, group_rows(p, g, begin));
+        }
+        const int incl = warp_incl_scan(n);
+        if (g < G) tile_start[g] = run + incl - n;
+        run += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    if (lane == 0) tile_start[G] = run;
+}
+
 // ---- host side ------------------------------------------------------------------------------
 using EncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                               const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
