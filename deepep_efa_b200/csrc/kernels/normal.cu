@@ -475,42 +475,56 @@ __global__ void __launch_bounds__(kDispatchThreads, 1) dispatch_kernel(const __g
 }
 
 // A lone rank that may use the whole GPU: the rows only move within its memory, at the speed of a copy. A warp takes one piece of one row
-// (2 KB to read when it casts, 4 KB otherwise), asks for all of it together with the row's place, stores it and ends; five CTAs of eight such
-// warps share an SM when it casts, four when it copies or combines, three with two biases. With a warp per row that walked over its columns, 32 to an SM, a row of 14 KB was seven dependent steps (one B200,
+// (2 KB to read when it casts, 4 KB otherwise), asks for all of it together with the row's place, stores it and ends; four CTAs of eight such
+// warps share an SM, three when it combines with two biases. Casting, resident warps go on to their next piece, which is on its way while this one is
+// cast (4096 x 7168 19.2 -> 17.0 us, 8192 x 7168 34.3 -> 31.1 beside one piece per warp and five CTAs; copies have no registers for that: 19.6 -> 24). With a warp per row that walked over its columns, 32 to an SM, a row of 14 KB was seven dependent steps (one B200,
 // 4096 x 7168: cast to FP8 31.4 -> 19.2 us, back in BF16 27.4 -> 17.5 us with what overlaps the predecessor; 3001 x 4096 in BF16 with one
 // bias 11.5 -> 8.0 and 18.3 -> 12.0 us).
 constexpr int kLoneThreads = 256;
 constexpr int kLoneWarps = kLoneThreads / 32;
 
 template <bool kQuant>
-__global__ void __launch_bounds__(kLoneThreads, kQuant ? 5 : 4) dispatch_lone_kernel(const __grid_constant__ DispatchArgs a, const int pieces) {
+__global__ void __launch_bounds__(kLoneThreads, 4) dispatch_lone_kernel(const __grid_constant__ DispatchArgs a, const int pieces) {
     pdl_wait_predecessor();
     pdl_release_successor();
     const RankCtx& c = a.ctx;
     const int T = a.num_tokens, K = a.num_topk, H = a.hidden;
     const int lane = threadIdx.x & 31;
-    const long long item = (long long)blockIdx.x * kLoneWarps + (threadIdx.x >> 5);
-    if (item < (long long)T * pieces) {
-        const int t = (int)(item / pieces), piece = (int)(item % pieces);
-        const size_t out_row_bytes = (size_t)H * (kQuant ? 1 : a.x_elem_bytes);
-        char* out = c.at<char>(0, a.recv_x_off);
-        float* scales = c.at<float>(0, a.recv_scales_off);
-        constexpr int U = kQuant ? 4 : 8;
-        int4 v[U];
-        const int n16 = (int)(out_row_bytes / 16);
-        const int ch = piece * 1024 + lane * 16;  // casting: 16 channels here and 16 in the other half of the piece
-        const int col = piece * 32 * U + lane;    // copying
+    const size_t out_row_bytes = (size_t)H * (kQuant ? 1 : a.x_elem_bytes);
+    char* out = c.at<char>(0, a.recv_x_off);
+    float* scales = c.at<float>(0, a.recv_scales_off);
+    constexpr int U = kQuant ? 4 : 8;
+    const int n16 = (int)(out_row_bytes / 16);
+    const unsigned items = (unsigned)T * (unsigned)pieces, step = gridDim.x * kLoneWarps;
+    int4 next[U];
+    int next_row = -1;
+    auto fetch = [&](unsigned item) {
+        const int t = (int)(item / (unsigned)pieces), piece = (int)(item % (unsigned)pieces);
+        const int ch = piece * 1024 + lane * 16, col = piece * 32 * U + lane;
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            v[u] = make_int4(0, 0, 0, 0);
+            next[u] = make_int4(0, 0, 0, 0);
+            if (item >= items) continue;
             if constexpr (kQuant) {
                 const int at = ch + (u >> 1) * 512;
-                if (at < H) v[u] = ld_stream(reinterpret_cast<const int4*>(reinterpret_cast<const char*>(a.x) + ((size_t)t * H + at) * 2) + (u & 1));
+                if (at < H) next[u] = ld_stream(reinterpret_cast<const int4*>(reinterpret_cast<const char*>(a.x) + ((size_t)t * H + at) * 2) + (u & 1));
             } else {
-                if (col + u * 32 < n16) v[u] = ld_stream(reinterpret_cast<const int4*>(reinterpret_cast<const char*>(a.x) + (size_t)t * out_row_bytes) + col + u * 32);
+                if (col + u * 32 < n16) next[u] = ld_stream(reinterpret_cast<const int4*>(reinterpret_cast<const char*>(a.x) + (size_t)t * out_row_bytes) + col + u * 32);
             }
         }
-        int row = a.send_head[t];
+        next_row = item < items ? a.send_head[t] : -1;
+    };
+    unsigned item = blockIdx.x * kLoneWarps + (threadIdx.x >> 5);
+    fetch(item);
+    for (; item < items; item += step) {
+        const int t = (int)(item / (unsigned)pieces), piece = (int)(item % (unsigned)pieces);
+        const int ch = piece * 1024 + lane * 16;  // casting: 16 channels here and 16 in the other half of the piece
+        const int col = piece * 32 * U + lane;    // copying
+        int4 v[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) v[u] = next[u];
+        int row = next_row;
+        if constexpr (kQuant) fetch(item + step);  // (copying, a warp has one piece)
         if (row >= 0 && !peer_range_ok(c, 0, out + (size_t)row * out_row_bytes, out_row_bytes, 1)) row = -1;
         if (row >= 0) {
             char* dst = out + (size_t)row * out_row_bytes;
@@ -582,7 +596,7 @@ cudaError_t launch_dispatch(const DispatchArgs* a, int nv, cudaStream_t stream) 
         const long long ids = (long long)a->num_worst_tokens * (a->topk_idx != nullptr ? a->num_topk : 0);
         const long long moving = ((long long)a->num_tokens * std::max(pieces, 1) + kLoneWarps - 1) / kLoneWarps;
         const long long marking = std::min<long long>((ids + 8 * kLoneThreads - 1) / (8 * kLoneThreads), 4 * 148);
-        const unsigned ctas = (unsigned)std::max<long long>(1, std::max(moving, marking));
+        const unsigned ctas = (unsigned)std::max<long long>(1, std::max(quant ? std::min<long long>(moving, 148 * 4) : moving, marking));
         return quant ? launch_dependent(dispatch_lone_kernel<true>, dim3(ctas), kLoneThreads, 0, stream, *a, std::max(pieces, 1))
                      : launch_dependent(dispatch_lone_kernel<false>, dim3(ctas), kLoneThreads, 0, stream, *a, std::max(pieces, 1));
     }
