@@ -579,6 +579,17 @@ def test_expert_plan_matches_the_cpu_plan(L, N, K):
     assert torch.equal(build_expert_plan(beyond.cuda(), counts.tolist()).pos.cpu(), want.pos)
 
 
+@pytest.mark.parametrize("N", [1, 31, 8191, 8192, 8193, 16385, 24577, 40961])
+def test_expert_plan_where_parts_of_a_chunk_are_empty(N):
+    """CTAs start at different quarters of 32768 selections, some of which have none."""
+    from deepep_efa_b200.ops.permute import build_expert_plan
+    L = 9
+    idx = torch.randint(0, L, (N, 1), generator=torch.Generator().manual_seed(N))
+    counts = ((torch.bincount(idx.view(-1), minlength=L) + 127) // 128 * 128).tolist()
+    want, got = build_expert_plan(idx, counts), build_expert_plan(idx.cuda(), counts)
+    assert torch.equal(got.pos.cpu(), want.pos) and torch.equal(got.src_row.cpu(), want.src_row)
+
+
 def test_gathers_of_rows_without_columns():
     """Nothing to move, as with the scale rows of fewer than 128 channels: no launch, and no error from one."""
     from deepep_efa_b200 import _ext
