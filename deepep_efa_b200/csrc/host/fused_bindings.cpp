@@ -45,6 +45,12 @@ int64_t sym_off(dxh::RuntimeCore* core, const torch::Tensor& t, const char* name
 }
 
 // Per rank tuple: (topk_idx, recv_x, recv_scales, recv_info, stage, my_counts, sel_list, send_base, unit_start, m_offsets, m_ends, peer_bases)
+// Behind the [E, T] words of sel_list, where the tensor has room for it: [T*K, 2], which expert's how manieth a selection is.
+int2* places_of(const torch::Tensor& sel_list, int64_t listed, int64_t selections) {
+    listed = (listed + 1) / 2 * 2;
+    return sel_list.numel() >= listed + 2 * selections ? reinterpret_cast<int2*>(sel_list.data_ptr<int>() + listed) : nullptr;
+}
+
 void em_notify(std::vector<py::object> rts, std::vector<py::tuple> per_rank, int num_experts, int unit_rows) {
     const int V = (int)rts.size();
     DXF_CHECK(V >= 1 && V <= dx::kMaxVirtualRanks && (int)per_rank.size() == V, "em_notify: one entry per rank");
@@ -99,6 +105,7 @@ void em_notify(std::vector<py::object> rts, std::vector<py::tuple> per_rank, int
         a.stage_off = (uint64_t)sym_off(core, stage, "stage");
         a.my_counts = my_counts.data_ptr<int>();
         a.sel_list = sel_list.data_ptr<int>();
+        a.places = places_of(sel_list, num_experts * T, T * K);
         a.send_base = send_base.data_ptr<int>();
         a.unit_start = unit_start.data_ptr<int>();
         a.unit_counter = unit_start.data_ptr<int>() + num_experts + 1;  // the tensor's last int is the hand-out counter
@@ -160,6 +167,7 @@ void em_dispatch(std::vector<py::object> rts, std::vector<py::tuple> per_rank, i
         a.native_atoms = native_atoms ? 1 : 0;
         a.my_counts = my_counts.data_ptr<int>();
         a.sel_list = sel_list.data_ptr<int>();
+        a.places = num_topk <= dx::kMaxTopk ? places_of(sel_list, num_experts * T, T * num_topk) : nullptr;
         a.send_base = send_base.data_ptr<int>();
         a.unit_start = unit_start.data_ptr<int>();
         a.unit_counter = unit_start.data_ptr<int>() + num_experts + 1;

@@ -147,6 +147,7 @@ struct EmNotifyArgs {
     // outputs, rank-local device memory
     int* my_counts;               // [E] my selections per expert
     int* sel_list;                // [E, T] selection ids (t*K + k) of every expert in token order
+    int2* places;                 // [T*K] or nullptr: expert of each selection (-1: none) and which of the expert's it is
     int* send_base;               // [E] row of my first selection of expert e inside e's rank
     int* unit_start;              // [E+1] exclusive prefix of work units in send order (local expert major, rank minor)
     int* unit_counter;            // [1] next work unit of the dispatch kernel, reset here
@@ -165,6 +166,7 @@ struct EmDispatchArgs {
     int native_atoms;             // 1: scales are written as the UE8M0 words of [row tile][K block][512] scale atoms
     const int* my_counts;
     const int* sel_list;
+    const int2* places;           // of em_notify, or nullptr
     const int* send_base;
     const int* unit_start;
     int* unit_counter;            // [1] next unit to hand out (zeroed by the count exchange)

@@ -57,11 +57,12 @@ __global__ void __launch_bounds__(kEmNotifyThreads, 1) em_notify_kernel(const __
         uint32_t* s_vote = reinterpret_cast<uint32_t*>(s_dyn + kScanBatch);
         for (int b0 = 0; b0 < ne; b0 += kScanBatch) {
             const int nb = min(kScanBatch, ne - b0);
-            scan_selections(a.topk_idx, T * K, E, e0 + b0, nb, s_vote, s_run, false,
+            scan_selections(a.topk_idx, T * K, E, e0 + b0, nb, s_vote, s_run, a.places != nullptr && e0 + b0 == 0,
                             [&](int j, int n, int i) {
                                 if (n < T) a.sel_list[(size_t)(e0 + b0 + j) * T + n] = i;  // an expert is selected at most once per token
+                                if (a.places != nullptr) a.places[i] = make_int2(e0 + b0 + j, n);
                             },
-                            [](int) {});
+                            [&](int i) { a.places[i] = make_int2(-1, 0); });
             for (int j = tid; j < nb; j += kEmNotifyThreads) a.my_counts[e0 + b0 + j] = min(s_run[j], T);
         }
     }
@@ -358,96 +359,73 @@ __global__ void __launch_bounds__(kEmDispatchThreads, 6) em_dispatch_kernel(cons
     }
 }
 
-// A lone rank with the GPU to itself copies its quantised rows within its own memory, so experts need not complete in order: resident warps
-// walk over the rows of all units, each with all loads of a row in flight, and look the next row's selection up while they copy. A CTA per unit spent
-// two thirds of its life on finding the expert, the selection and the row one after the other (4096 x 8 rows of 7 KB 68 -> 61 us behind the exchange, 4000 x 8 of
-// 2 KB 36 -> 23).
+// A lone rank copies its quantised rows within its own memory, so experts need not complete in order: a warp loads a span of a token's row once and stores it to
+// all of the token's rows. Expert by expert the rows were read again for each selection, from HBM, since what is written pushes them out of the L2 (rows of
+// 52736 x 8 KB written at 3.2 TB/s with reads from 67 MB, at 6.5 without). Behind the exchange, 4096 x 8 rows of 1 KB 38.4 -> 26.8 us, 4096 x 6 27.4 -> 19.5; in a layer
+// at the power limit, 4096 x 8 rows of 7 KB 96 -> 55.
 constexpr int kEmLoneThreads = 256;
-constexpr int kEmLoneLoads = 14;  // 7168 channels in one pass
-constexpr int kEmLoneCtasPerSm = 3;
-__host__ __device__ constexpr size_t em_lone_smem(int num_experts) { return (size_t)(3 * num_experts + 1) * sizeof(int); }
+constexpr int kEmLoneLoads = 4;
+constexpr int kEmLoneSpan = 32 * kEmLoneLoads * 16;  // bytes of a row per warp: 16 of its scales
+inline long long em_lone_ctas(const EmDispatchArgs& a) {
+    const long long warps = (long long)a.num_tokens * ((a.hidden + kEmLoneSpan - 1) / kEmLoneSpan);
+    return std::max(1ll, (warps + kEmLoneThreads / 32 - 1) / (kEmLoneThreads / 32));
+}
 
-__global__ void __launch_bounds__(kEmLoneThreads, kEmLoneCtasPerSm) em_dispatch_lone_kernel(const __grid_constant__ EmDispatchArgs a) {
+__global__ void __launch_bounds__(kEmLoneThreads) em_dispatch_lone_kernel(const __grid_constant__ EmDispatchArgs a) {
     pdl_wait_predecessor();
     pdl_release_successor();
-    const RankCtx& c = a.ctx;
     const int T = a.num_tokens, K = a.num_topk, E = a.num_experts, H = a.hidden;
     const int tid = threadIdx.x, lane = tid & 31;
-    extern __shared__ int s_lone[];
-    int *s_start = s_lone, *s_count = s_lone + E + 1, *s_base = s_count + E;  // units of expert e: [s_start[e], s_start[e + 1])
-    for (int e = tid; e <= E; e += kEmLoneThreads) {
-        s_start[e] = a.unit_start[e];
-        if (e < E) {
-            s_count[e] = a.my_counts[e];
-            s_base[e] = a.send_base[e];
-        }
-    }
-    __syncthreads();
-    char* rows = reinterpret_cast<char*>(a.peer_bases[0]);
-    char* scales = reinterpret_cast<char*>(a.peer_bases[1]);
-    int* info = reinterpret_cast<int*>(a.peer_bases[2]);
-    const int n16 = H / 16, num_kb = H / 128;
-    const int items = s_start[E] * a.unit_rows, step = gridDim.x * (kEmLoneThreads / 32);
-    int sel = -1, row = 0;
-    auto find = [&](int item) {  // selection and row of an item, -1 where a unit has no such row
-        sel = -1;
-        if (item >= items) return;
-        const int u = item / a.unit_rows;
-        int lo = 0, hi = E;  // the last expert whose units start at or before u (experts without rows have none)
-        while (hi - lo > 1) {
-            const int mid = (lo + hi) / 2;
-            if (s_start[mid] <= u) lo = mid;
-            else hi = mid;
-        }
-        const int s = (u - s_start[lo]) * a.unit_rows + item % a.unit_rows;
-        if (s >= s_count[lo]) return;
-        sel = a.sel_list[(size_t)lo * T + s];
-        row = s_base[lo] + s;
-    };
-    int item = blockIdx.x * (kEmLoneThreads / 32) + (tid >> 5);
-    find(item);
-    for (; item < items; item += step) {
-        const int mine = sel, dst_row = row;
-        find(item + step);
-        if (mine < 0) continue;
-        const int t = mine / K;
-        const int4* src = reinterpret_cast<const int4*>(reinterpret_cast<const char*>(a.x) + (size_t)t * H);
-        int4* dst = reinterpret_cast<int4*>(rows + (size_t)dst_row * H);
-        for (int i0 = lane; i0 < n16; i0 += 32 * kEmLoneLoads) {
-            int4 v[kEmLoneLoads];
+    const int n16 = H / 16, num_kb = H / 128, spans = (H + kEmLoneSpan - 1) / kEmLoneSpan;
+    const long long item = (long long)blockIdx.x * (kEmLoneThreads / 32) + (tid >> 5);
+    const int t = (int)(item / spans), span = (int)(item % spans);
+    const bool any = a.unit_start[E] > 0;  // (no units after an overflow)
+    if (t < T && any) {
+        const int i0 = span * (kEmLoneSpan / 16) + lane, kb = span * (kEmLoneSpan / 128) + (lane & 15);
+        const int4* src = reinterpret_cast<const int4*>(reinterpret_cast<const char*>(a.x) + (size_t)t * H) + i0;
+        int4 v[kEmLoneLoads];
 #pragma unroll
-            for (int k = 0; k < kEmLoneLoads; ++k)
-                if (i0 + k * 32 < n16) v[k] = ld_cached(src + i0 + k * 32);
-#pragma unroll
-            for (int k = 0; k < kEmLoneLoads; ++k)
-                if (i0 + k * 32 < n16) st_once(dst + i0 + k * 32, v[k]);
+        for (int u = 0; u < kEmLoneLoads; ++u)
+            if (i0 + u * 32 < n16) v[u] = ld_once(src + u * 32);
+        const float scale = kb < num_kb ? a.x_scales[(size_t)t * num_kb + kb] : 0.f;
+        int row = -1;
+        if (lane < K) {
+            const int2 place = a.places[(size_t)t * K + lane];
+            if (place.x >= 0 && place.y < a.my_counts[place.x]) row = a.send_base[place.x] + place.y;
         }
-        for (int kb = lane; kb < num_kb; kb += 32) {
-            const float scale = a.x_scales[(size_t)t * num_kb + kb];
+        char* rows = reinterpret_cast<char*>(a.peer_bases[0]);
+        char* scales = reinterpret_cast<char*>(a.peer_bases[1]);
+        for (int k = 0; k < K; ++k) {
+            const int dst_row = __shfl_sync(0xffffffffu, row, k);
+            if (dst_row < 0) continue;
+            int4* dst = reinterpret_cast<int4*>(rows + (size_t)dst_row * H) + i0;
+#pragma unroll
+            for (int u = 0; u < kEmLoneLoads; ++u)
+                if (i0 + u * 32 < n16) st_once(dst + u * 32, v[u]);
+        }
+        for (int k0 = 0; k0 < K; k0 += 2) {  // two rows' scales at a time
+            const int dst_row = __shfl_sync(0xffffffffu, row, (k0 + (lane >> 4)) & 31);
+            if (k0 + (lane >> 4) >= K || dst_row < 0 || kb >= num_kb) continue;
             if (a.native_atoms)
                 *reinterpret_cast<uint32_t*>(scales + ((size_t)(dst_row >> 7) * num_kb + kb) * 512 + (dst_row & 31) * 16 + ((dst_row >> 5) & 3) * 4) =
                     ((__float_as_uint(scale) >> 23) & 0xffu) * 0x01010101u;
             else reinterpret_cast<float*>(scales)[(size_t)dst_row * num_kb + kb] = scale;
         }
-        if (lane == 0) {
-            info[dst_row] = mine;  // (source rank 0 << 24) | selection
-            if (a.dst_row != nullptr) a.dst_row[mine] = dst_row;
+        if (span == 0 && row >= 0) {
+            reinterpret_cast<int*>(a.peer_bases[2])[row] = t * K + lane;  // (source rank 0 << 24) | selection
+            if (a.dst_row != nullptr) a.dst_row[t * K + lane] = row;
         }
     }
     // (nobody waits for a lone rank's arrivals within this kernel)
-    if (blockIdx.x == 0)
-        for (int e = tid; e < E; e += kEmLoneThreads)  // (without units after an overflow)
-            if (s_start[e + 1] > s_start[e]) red_add_release_gpu(&c.my_ctrl()->em_arrived[e], (uint64_t)s_count[e]);
+    if (blockIdx.x == 0 && any)
+        for (int e = tid; e < E; e += kEmLoneThreads)
+            if (a.my_counts[e] > 0) red_add_release_gpu(&a.ctx.my_ctrl()->em_arrived[e], (uint64_t)a.my_counts[e]);
 }
 
 cudaError_t launch_em_dispatch(const EmDispatchArgs* a, int nv, cudaStream_t stream) {
     if (a[0].hidden % 128 != 0 || a[0].num_sms < 1) return cudaErrorInvalidValue;
-    if (nv == 1 && a->ctx.num_ranks == 1 && a->num_sms >= 148 && a->x_scales != nullptr && a->ctx.debug_extent == 0 && a->trace == nullptr &&
-        em_lone_smem(a->num_experts) <= 48 * 1024) {
-        const long long warps = (long long)a->num_tokens * a->num_topk + (long long)a->num_experts * (a->unit_rows - 1);  // at most
-        const int ctas = (int)std::min<long long>(148 * kEmLoneCtasPerSm, (warps + kEmLoneThreads / 32 - 1) / (kEmLoneThreads / 32));
-        return launch_dependent(em_dispatch_lone_kernel, dim3((unsigned)ctas), kEmLoneThreads, em_lone_smem(a->num_experts), stream, *a);
-    }
+    if (nv == 1 && a->ctx.num_ranks == 1 && a->num_sms >= 148 && a->places != nullptr && a->x_scales != nullptr && a->ctx.debug_extent == 0 && a->trace == nullptr)
+        return launch_dependent(em_dispatch_lone_kernel, dim3((unsigned)em_lone_ctas(*a)), kEmLoneThreads, 0, stream, *a);
     const size_t smem = (size_t)(a[0].num_experts + 1) * sizeof(int);
     return DX_LAUNCH_RANKED_PDL(em_dispatch_kernel, EmDispatchArgs, a, nv, a[0].num_sms, kEmDispatchThreads, smem, stream);
 }

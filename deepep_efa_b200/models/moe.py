@@ -391,7 +391,7 @@ class _FusedWorkspace:
         self.stage = sym([T * K, H], torch.bfloat16)
         i32 = dict(dtype=torch.int32, device=dev)
         self.my_counts = torch.zeros(E, **i32)
-        self.sel_list = torch.zeros(E * T, **i32)
+        self.sel_list = torch.zeros(E * T + (2 * T * K + 1 if R == 1 else 0), **i32)  # a lone rank also keeps the selections' places
         self.send_base = torch.zeros(E, **i32)
         self.unit_start = torch.zeros(E + 2, **i32)  # prefix of work units [E + 1] and the hand-out counter
         self.m_offsets = torch.zeros(L + 1, **i32)

@@ -169,8 +169,8 @@ def test_expert_major_dispatch_with_many_experts_per_cta():
 
 @pytest.mark.parametrize("T,H,E,K,native", [(1, 128, 4, 1, True), (5, 512, 300, 3, False), (77, 4224, 6, 4, True), (130, 7296, 5, 5, False), (40, 7168, 16, 8, True)])
 def test_lone_dispatch_places_rows_like_the_general_one(T, H, E, K, native):
-    """The dispatch of a lone rank that may use the whole GPU against the one with a bounded number of CTAs: rows, scales, row words, places
-    and arrival counts; hidden sizes below, at and past one pass of a warp, fewer and more experts than a CTA has threads."""
+    """The dispatch of a lone rank that may use the whole GPU (token by token) against the one with a bounded number of CTAs (expert by expert): rows,
+    scales, row words, places and arrival counts; hidden sizes below, at and past a warp's span, fewer and more experts than a CTA has threads."""
     import deepep_efa_b200 as ep
     from deepep_efa_b200.models.moe import UNIT_ROWS
     vc, layers, xs, idxs, ws = _setup(1, T, H, 256, E, K, native)
