@@ -432,6 +432,21 @@ torch::Tensor build_sf_atoms_b(const torch::Tensor& scales, int64_t n, bool swig
     return atoms;
 }
 
+// src [N, H] in a plan's order [M, H], zero rows as padding; pos [N, K] and src_row [M] are the plan's maps.
+torch::Tensor permute_rows(const torch::Tensor& src, const torch::Tensor& pos, const torch::Tensor& src_row) {
+    DXG_CHECK(src.is_cuda() && src.dim() == 2 && src.is_contiguous(), "src must be a contiguous CUDA matrix");
+    const int64_t row_bytes = src.size(1) * src.element_size();
+    DXG_CHECK(row_bytes % 4 == 0, "row size must be a multiple of 4 bytes");
+    DXG_CHECK(src_row.device() == src.device() && src_row.scalar_type() == torch::kInt32 && src_row.is_contiguous() && src_row.dim() == 1, "src_row must be int32 [M]");
+    DXG_CHECK(pos.device() == src.device() && pos.scalar_type() == torch::kInt32 && pos.is_contiguous() && pos.dim() == 2 && pos.size(0) == src.size(0), "pos must be int32 [N, K]");
+    c10::cuda::CUDAGuard guard(src.device());
+    const torch::Tensor dst = torch::empty({src_row.numel(), src.size(1)}, src.options());
+    const cudaError_t e = dx::launch_permute_rows(src.data_ptr(), dst.data_ptr(), pos.data_ptr<int>(), src_row.data_ptr<int>(), (int)src.size(0), (int)pos.size(1),
+                                                  (int)src_row.numel(), (int)row_bytes, at::cuda::getCurrentCUDAStream(src.get_device()).stream());
+    if (e != cudaSuccess) throw std::runtime_error(std::string("permute_rows: ") + cudaGetErrorString(e));
+    return dst;
+}
+
 // Expert-major rows of a dispatch result in e4m3 and their scales in one launch: (rows [M, H], scales [M, H/128], or scale atoms [M/128, H/128, 512]).
 std::tuple<torch::Tensor, torch::Tensor> gather_quantised(const torch::Tensor& rows, const torch::Tensor& scales, const torch::Tensor& src_row, bool atoms,
                                                           c10::optional<torch::Tensor> sched) {
@@ -543,6 +558,7 @@ void bind_gemm(py::module_& m) {
     m.def("gather_quantised", &gather_quantised, py::arg("rows"), py::arg("scales"), py::arg("src_row"), py::arg("atoms"), py::arg("sched") = py::none());
     m.def("build_plan", &build_plan);
     m.def("gather_rows", &gather_rows, py::arg("src"), py::arg("src_row"), py::arg("scale") = py::none(), py::arg("out") = py::none());
+    m.def("permute_rows", &permute_rows);
     m.def("gather_reduce_rows", &gather_reduce_rows, py::arg("src"), py::arg("pos"), py::arg("w") = py::none(), py::arg("out") = py::none());
     m.def("gemm_error", &gemm_error);
     m.def("gemm_clear_error", &gemm_clear_error);

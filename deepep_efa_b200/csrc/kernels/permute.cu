@@ -3,6 +3,7 @@
 //
 //   build_plan:           the maps between the two orders, in one launch
 //   gather_rows:          dst[m] = scale[m] * src[src_row[m]]            (src_row < 0 -> zero row)
+//   permute_rows:         the unweighted gather of a plan, by whichever of its maps is the faster
 //   gather_reduce_rows:   dst[n] = sum_k w[n,k] * src[pos[n,k]]          (pos < 0 skipped), fp32 accumulate
 //
 // The gathers are pure bandwidth kernels: a warp per span of columns of an output row, 16-byte accesses, no atomics. The
@@ -193,6 +194,41 @@ cudaError_t launch_gather_rows(const void* src, void* dst, const int* src_row, c
                             static_cast<const char*>(src), static_cast<char*>(dst), src_row, scale, num_dst_rows, row_bytes);
 }
 
+// dst[pos[n, k]] = src[n] for all k, zero rows where src_row says padding: rows in the plan's order, each source row read once. A warp takes a span of a row and
+// stores it to all its places, or clears a padding row.
+constexpr int kSpreadLoads = 4;
+constexpr int kSpreadSpan = 32 * kSpreadLoads;  // 16-byte columns
+
+__global__ void __launch_bounds__(kPermThreads) spread_rows_kernel(const char* __restrict__ src, char* __restrict__ dst, const int* __restrict__ pos,
+                                                                  const int* __restrict__ src_row, int num_src_rows, int num_k, int num_dst_rows, int n16) {
+    pdl_wait_predecessor();
+    pdl_release_successor();
+    const int lane = threadIdx.x & 31, spans = (n16 + kSpreadSpan - 1) / kSpreadSpan;
+    const long long item = (long long)blockIdx.x * (kPermThreads / 32) + (threadIdx.x >> 5), spread = (long long)num_src_rows * spans;
+    if (item >= spread) {
+        const long long m = item - spread;
+        if (m >= num_dst_rows || src_row[m] >= 0) return;
+        int4* d = reinterpret_cast<int4*>(dst) + (size_t)m * n16;
+        for (int i = lane; i < n16; i += 32) st_once(d + i, make_int4(0, 0, 0, 0));
+        return;
+    }
+    const int n = (int)(item / spans), i0 = (int)(item % spans) * kSpreadSpan + lane;
+    const int4* p = reinterpret_cast<const int4*>(src) + (size_t)n * n16 + i0;
+    int4 v[kSpreadLoads];
+#pragma unroll
+    for (int u = 0; u < kSpreadLoads; ++u)
+        if (i0 + u * 32 < n16) v[u] = ld_once(p + u * 32);
+    const int place = lane < num_k ? pos[(size_t)n * num_k + lane] : -1;
+    for (int k = 0; k < num_k; ++k) {
+        const int row = __shfl_sync(0xffffffffu, place, k);
+        if (row < 0 || row >= num_dst_rows) continue;
+        int4* d = reinterpret_cast<int4*>(dst) + (size_t)row * n16 + i0;
+#pragma unroll
+        for (int u = 0; u < kSpreadLoads; ++u)
+            if (i0 + u * 32 < n16) st_once(d + u * 32, v[u]);
+    }
+}
+
 // e4m3 rows and their scales (num_kb per row) together: the scales of a row come and go with its first span, as floats or as the words of scale atoms (row r of
 // a tile at (r & 31) * 16 + (r >> 5) * 4 of the K block's 512 bytes). Two launches, or three with the atoms, cost a short prompt more than the copies.
 __global__ void __launch_bounds__(kPermThreads) gather_quantised_kernel(const char* __restrict__ src, const float* __restrict__ src_scales, char* __restrict__ dst,
@@ -225,6 +261,22 @@ __global__ void __launch_bounds__(kPermThreads) gather_quantised_kernel(const ch
 #pragma unroll
     for (int u = 0; u < U; ++u)
         if (i0 + u * 32 < n16) st_once(d + i0 + u * 32, v[u]);
+}
+
+// Sources that the rows written would push out of the L2 between one reading and the next go the other way round, each row read once (52736 rows of 8 KB are
+// written at 3.2 TB/s with gathered reads from 67 MB, at 6.5 without reads). Time spread / gathered, rows of 2 to 14 KB, 2 to 8 places each:
+//   source MB   8          16         24         32         40         48         56         64         80
+//               0.89-1.13  0.96-1.13  0.99-1.09  0.94-1.05  0.90-1.04  0.88-1.00  0.85-1.01  0.82-0.97  0.78-0.95
+constexpr long long kSpreadMinBytes = 48ll << 20;
+
+cudaError_t launch_permute_rows(const void* src, void* dst, const int* pos, const int* src_row, int num_src_rows, int num_k, int num_dst_rows, int row_bytes, cudaStream_t stream) {
+    if (num_dst_rows <= 0 || row_bytes == 0) return cudaSuccess;
+    if (row_bytes % 16 != 0 || num_k < 1 || num_k > 32 || (long long)num_src_rows * row_bytes < kSpreadMinBytes)
+        return launch_gather_rows(src, dst, src_row, nullptr, num_dst_rows, row_bytes, stream);
+    const int n16 = row_bytes / 16;
+    const long long warps = (long long)num_src_rows * ((n16 + kSpreadSpan - 1) / kSpreadSpan) + num_dst_rows;
+    return launch_dependent(spread_rows_kernel, dim3((unsigned)((warps + kPermThreads / 32 - 1) / (kPermThreads / 32))), kPermThreads, 0, stream, static_cast<const char*>(src),
+                            static_cast<char*>(dst), pos, src_row, num_src_rows, num_k, num_dst_rows, n16);
 }
 
 cudaError_t launch_gather_quantised(const void* src, const float* src_scales, void* dst, float* scales, uint8_t* atoms, const int* src_row, int num_dst_rows, int hidden,

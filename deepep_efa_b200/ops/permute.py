@@ -102,6 +102,8 @@ class _Permute(torch.autograd.Function):
     @staticmethod
     def forward(ctx, recv_x, plan: ExpertPlan):
         ctx.plan = plan
+        if recv_x.is_cuda and plan.pos.size(0) == recv_x.size(0):
+            return _ext.load().permute_rows(recv_x.contiguous(), plan.pos, plan.src_row)
         return gather_rows(recv_x, plan.src_row)
 
     @staticmethod

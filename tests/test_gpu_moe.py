@@ -40,6 +40,20 @@ def test_permute_kernels_match_indexing():
     assert torch.equal(gather_rows(q, plan.src_row).view(torch.uint8)[o[1]:o[1] + 3], q.view(torch.uint8)[plan.src_row[o[1]:o[1] + 3].long()])
 
 
+@pytest.mark.parametrize("N,H,K,L", [(50, 256, 3, 4), (49153, 512, 1, 3), (25000, 1032, 3, 200), (6200, 4096, 32, 40), (3100, 8200, 8, 9)])
+def test_rows_of_a_plan_by_either_map(N, H, K, L):
+    """Small sources are gathered, large ones spread to their places: rows below, at and past a warp's span; experts without rows, tiles of padding, and
+    selections that the plan has no room for."""
+    from deepep_efa_b200.ops.permute import build_expert_plan, gather_rows, permute
+    g = torch.Generator(device="cuda").manual_seed(N)
+    idx = torch.randint(-1, L - 1, (N, K), generator=g, device="cuda")
+    counts = ((torch.bincount(idx[idx >= 0], minlength=L) + 255) // 128 * 128).tolist()
+    counts[1] = 128
+    plan = build_expert_plan(idx, counts)
+    x = torch.randn(N, H, generator=g, device="cuda").to(torch.bfloat16)
+    assert torch.equal(permute(x, plan), gather_rows(x, plan.src_row))
+
+
 def test_moe_layer_forward_backward_gpu():
     import deepep_efa_b200 as ep
     from deepep_efa_b200.models.moe import MoEConfig, MoELayer, dense_reference
