@@ -48,7 +48,8 @@ int64_t sym_off(dxh::RuntimeCore* core, const torch::Tensor& t, const char* name
 // Behind the [E, T] words of sel_list, where the tensor has room for it: [T*K, 2], which expert's how manieth a selection is.
 int2* places_of(const torch::Tensor& sel_list, int64_t listed, int64_t selections) {
     listed = (listed + 1) / 2 * 2;
-    return sel_list.numel() >= listed + 2 * selections ? reinterpret_cast<int2*>(sel_list.data_ptr<int>() + listed) : nullptr;
+    int* at = sel_list.data_ptr<int>() + listed;
+    return sel_list.numel() >= listed + 2 * selections && (reinterpret_cast<uintptr_t>(at) & 7) == 0 ? reinterpret_cast<int2*>(at) : nullptr;
 }
 
 void em_notify(std::vector<py::object> rts, std::vector<py::tuple> per_rank, int num_experts, int unit_rows) {
