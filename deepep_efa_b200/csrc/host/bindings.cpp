@@ -595,7 +595,10 @@ py::tuple normal_dispatch_on(const py::tuple& stream, py::object previous, bool 
 py::tuple normal_combine_on(const py::tuple& stream, py::object previous, bool async_finish, bool results_on_stream, Runtime* rt, const py::tuple& req, int num_sms) {
     OnCommStream scope(stream, previous, async_finish);
     py::object out = py::none(), out_w = py::none();
-    if (!results_on_stream) {  // on the caller's stream, freed on which they are reusable at once
+    // Results of a call that follows the caller's stream are allocated there, freed on which they are reusable at once. Behind an event they are the communication
+    // stream's: a block that the caller's stream gave up after the event may still be in use there.
+    results_on_stream = results_on_stream || !previous.is_none();
+    if (!results_on_stream) {
         const auto x = req[0].cast<torch::Tensor>();
         const int64_t rows = req[2].cast<torch::Tensor>().size(0);
         out = py::cast(torch::empty({rows, x.size(1)}, x.options().dtype(torch::kBFloat16)));

@@ -414,3 +414,40 @@ def test_inputs_dropped_behind_calls_on_the_communication_stream(form):
             del rows, out, keep
     finally:
         vc.destroy()
+
+
+@pytest.mark.parametrize("asynchronous", [False, True])
+@pytest.mark.parametrize("entry", ["one", "many"])
+def test_results_of_a_combine_behind_an_event(entry, asynchronous):
+    """A block that the caller's stream gave up after the event, but has yet to write and read, does not become a result of a combine that waits for the
+    event alone."""
+    from deepep_efa_b200 import Buffer
+    from deepep_efa_b200.buffer import _combine_many
+    vc, buf = _buffer()
+    try:
+        idx, w = make_routing(T, E, K, "cuda", seed=7, masked_fraction=0.2)
+        x = make_tokens(T, H, "cuda", seed=7)
+        lay, _ = _layout(buf, idx)
+        y, _, rw, _, handle, _ = buf.dispatch(x, topk_weights=w, **lay)
+        want, want_w = (t.clone() for t in buf.combine(y, handle, topk_weights=rw)[:2])
+        fives, kept = torch.full_like(want, 5.0), torch.zeros_like(want)
+        sixes, kept_w = torch.full_like(want_w, 6.0), torch.zeros_like(want_w)
+        torch.cuda.synchronize()
+        how = dict(previous_event=Buffer.capture(), async_finish=asynchronous)
+        _delay(torch.cuda.current_stream())
+        blocks = torch.empty_like(want), torch.empty_like(want_w)
+        for block, value, copy in zip(blocks, (fives, sixes), (kept, kept_w)):
+            block.copy_(value)
+            copy.copy_(block)
+        del blocks, block
+        if entry == "one":
+            out, out_w, ev = buf.combine(y, handle, topk_weights=rw, **how)
+        else:
+            out, out_w, ev = _combine_many([buf], [(y, handle, rw, None)], Buffer.get_combine_config(1), how["previous_event"], asynchronous, False)[0]
+        ev.current_stream_wait()
+        torch.cuda.synchronize()
+        buf.check_status()
+        assert torch.equal(kept, fives) and torch.equal(kept_w, sixes)
+        assert torch.equal(out, want) and torch.equal(out_w, want_w)
+    finally:
+        vc.destroy()
