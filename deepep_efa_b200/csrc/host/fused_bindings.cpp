@@ -44,14 +44,16 @@ int64_t sym_off(dxh::RuntimeCore* core, const torch::Tensor& t, const char* name
     return (int64_t)off;
 }
 
-// Per rank tuple: (topk_idx, recv_x, recv_scales, recv_info, stage, my_counts, sel_list, send_base, unit_start, m_offsets, m_ends, peer_bases)
-// Behind the [E, T] words of sel_list, where the tensor has room for it: [T*K, 2], which expert's how manieth a selection is.
-int2* places_of(const torch::Tensor& sel_list, int64_t listed, int64_t selections) {
-    listed = (listed + 1) / 2 * 2;
-    int* at = sel_list.data_ptr<int>() + listed;
-    return sel_list.numel() >= listed + 2 * selections && (reinterpret_cast<uintptr_t>(at) & 7) == 0 ? reinterpret_cast<int2*>(at) : nullptr;
+// Optional last entry of a per-rank tuple: int32 [T*K, 2], which expert's how manieth each selection is. Not inferred from room behind another tensor, whose
+// tail is its owner's.
+int2* places_of(const py::tuple& t, size_t entry, const torch::Device& dev, int64_t selections) {
+    if (t.size() <= entry || t[entry].is_none()) return nullptr;
+    const auto places = t[entry].cast<torch::Tensor>();
+    DXF_CHECK(i32_on(places, dev, 2 * selections) && (reinterpret_cast<uintptr_t>(places.data_ptr()) & 7) == 0, "places must be int32 [T*K, 2], 8-byte aligned");
+    return reinterpret_cast<int2*>(places.data_ptr<int>());
 }
 
+// Per rank tuple: (topk_idx, recv_x, recv_scales, recv_info, stage, my_counts, sel_list, send_base, unit_start, m_offsets, m_ends, peer_bases[, places|None])
 void em_notify(std::vector<py::object> rts, std::vector<py::tuple> per_rank, int num_experts, int unit_rows) {
     const int V = (int)rts.size();
     DXF_CHECK(V >= 1 && V <= dx::kMaxVirtualRanks && (int)per_rank.size() == V, "em_notify: one entry per rank");
@@ -63,7 +65,7 @@ void em_notify(std::vector<py::object> rts, std::vector<py::tuple> per_rank, int
         dxh::RuntimeCore* core = dx_core_of(rts[v]);
         order.add(core);
         const py::tuple& t = per_rank[v];
-        DXF_CHECK(t.size() == 12, "em_notify: per-rank tuple must have 12 entries");
+        DXF_CHECK(t.size() == 12 || t.size() == 13, "em_notify: per-rank tuple must have 12 entries, or 13 with places");
         auto topk_idx = t[0].cast<torch::Tensor>();
         auto recv_x = t[1].cast<torch::Tensor>();
         auto recv_scales = t[2].cast<torch::Tensor>();
@@ -106,7 +108,7 @@ void em_notify(std::vector<py::object> rts, std::vector<py::tuple> per_rank, int
         a.stage_off = (uint64_t)sym_off(core, stage, "stage");
         a.my_counts = my_counts.data_ptr<int>();
         a.sel_list = sel_list.data_ptr<int>();
-        a.places = places_of(sel_list, num_experts * T, T * K);
+        a.places = places_of(t, 12, dev, T * K);
         a.send_base = send_base.data_ptr<int>();
         a.unit_start = unit_start.data_ptr<int>();
         a.unit_counter = unit_start.data_ptr<int>() + num_experts + 1;  // the tensor's last int is the hand-out counter
@@ -118,8 +120,9 @@ void em_notify(std::vector<py::object> rts, std::vector<py::tuple> per_rank, int
     check(dx::launch_em_notify(args.data(), V, order.stream), "em_notify");
 }
 
-// Per rank tuple: (x, my_counts, sel_list, send_base, unit_start, peer_bases, dst_row|None, trace|None, x_scales|None)
-// x is bf16 (rows are quantised by the kernel) or, with x_scales, e4m3 rows quantised beforehand (copied as they are).
+// Per rank tuple: (x, my_counts, sel_list, send_base, unit_start, peer_bases, dst_row|None, trace|None, x_scales|None[, places|None])
+// x is bf16 (rows are quantised by the kernel) or, with x_scales, e4m3 rows quantised beforehand (copied as they are). With `places`, as em_notify has
+// written them, a lone rank that may use every SM sends such rows token by token and reads no sel_list.
 void em_dispatch(std::vector<py::object> rts, std::vector<py::tuple> per_rank, int num_experts, int num_topk, int unit_rows,
                  bool round_scale, bool native_atoms, int num_sms) {
     const int V = (int)rts.size();
@@ -133,7 +136,7 @@ void em_dispatch(std::vector<py::object> rts, std::vector<py::tuple> per_rank, i
         dxh::RuntimeCore* core = dx_core_of(rts[v]);
         order.add(core);
         const py::tuple& t = per_rank[v];
-        DXF_CHECK(t.size() == 9, "em_dispatch: per-rank tuple must have 9 entries");
+        DXF_CHECK(t.size() == 9 || t.size() == 10, "em_dispatch: per-rank tuple must have 9 entries, or 10 with places");
         auto x = t[0].cast<torch::Tensor>();
         auto my_counts = t[1].cast<torch::Tensor>();
         auto sel_list = t[2].cast<torch::Tensor>();
@@ -168,7 +171,7 @@ void em_dispatch(std::vector<py::object> rts, std::vector<py::tuple> per_rank, i
         a.native_atoms = native_atoms ? 1 : 0;
         a.my_counts = my_counts.data_ptr<int>();
         a.sel_list = sel_list.data_ptr<int>();
-        a.places = num_topk <= dx::kMaxTopk ? places_of(sel_list, num_experts * T, T * num_topk) : nullptr;
+        a.places = num_topk <= dx::kMaxTopk ? places_of(t, 9, dev, T * num_topk) : nullptr;
         a.send_base = send_base.data_ptr<int>();
         a.unit_start = unit_start.data_ptr<int>();
         a.unit_counter = unit_start.data_ptr<int>() + num_experts + 1;

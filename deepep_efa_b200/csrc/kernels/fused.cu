@@ -391,7 +391,7 @@ __global__ void __launch_bounds__(kEmLoneThreads) em_dispatch_lone_kernel(const 
         int row = -1;
         if (lane < K) {
             const int2 place = a.places[(size_t)t * K + lane];
-            if (place.x >= 0 && place.y < a.my_counts[place.x]) row = a.send_base[place.x] + place.y;
+            if ((unsigned)place.x < (unsigned)E && (unsigned)place.y < (unsigned)a.my_counts[place.x]) row = a.send_base[place.x] + place.y;
         }
         char* rows = reinterpret_cast<char*>(a.peer_bases[0]);
         char* scales = reinterpret_cast<char*>(a.peer_bases[1]);

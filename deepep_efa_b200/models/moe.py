@@ -361,8 +361,9 @@ RESERVED_SMS = 16
 # The gated GEMM runs as two launches when it overlaps the dispatch: the first part of the experts (arrival order = expert
 # order) on the SMs the dispatch does not use, the rest on all SMs once the dispatch is about done.
 SPLIT_FRACTION = 0.5
-# CTAs of the expert-major dispatch per SM when nothing runs beside it (four warps each; six fit an SM): with one the copy of 32768
-# rows of 7 KB took 162 us, bound by the loads four warps keep in flight.
+# CTAs of the general expert-major dispatch per SM when nothing runs beside it (four warps each; six fit an SM): with one the copy of 32768
+# rows of 7 KB took 162 us, bound by the loads four warps keep in flight. A lone rank's kernel for rows quantised beforehand sizes its own grid
+# and is only told by 148 CTAs or more that every SM is its own; the number itself counts with a trace or without PREQUANTIZE.
 DISPATCH_CTAS_PER_SM = 6
 PREQUANTIZE = True  # cast every token to e4m3 once before the dispatch, which then only copies rows (8 selections share a cast)
 GEMM_TIMEOUT_MS = 2000.0  # bound of every wait inside the gated GEMMs (pipeline barriers and arrival counters)
@@ -391,7 +392,9 @@ class _FusedWorkspace:
         self.stage = sym([T * K, H], torch.bfloat16)
         i32 = dict(dtype=torch.int32, device=dev)
         self.my_counts = torch.zeros(E, **i32)
-        self.sel_list = torch.zeros(E * T + (2 * T * K + 1 if R == 1 else 0), **i32)  # a lone rank also keeps the selections' places
+        self.sel_list = torch.zeros(E * T, **i32)
+        # a lone rank's dispatch goes by these; the lists are for what it leaves to the general kernel (a trace, rows not quantised beforehand)
+        self.places = torch.zeros(T * K, 2, **i32) if R == 1 else None
         self.send_base = torch.zeros(E, **i32)
         self.unit_start = torch.zeros(E + 2, **i32)  # prefix of work units [E + 1] and the hand-out counter
         self.m_offsets = torch.zeros(L + 1, **i32)
@@ -464,14 +467,14 @@ def fused_forward_many(layers, xs, idxs, ws, overlap: bool = True, num_dispatch_
             quantised.record(cur)
     with torch.cuda.stream(comm):
         C.em_notify(rts, [(i, w.recv_x, w.recv_scales_raw, w.recv_info, w.stage, w.my_counts, w.sel_list, w.send_base, w.unit_start,
-                           w.m_offsets, w.m_ends, w.peer_bases) for i, w in zip(idxs, wss)], E, UNIT_ROWS)
+                           w.m_offsets, w.m_ends, w.peer_bases, w.places) for i, w in zip(idxs, wss)], E, UNIT_ROWS)
         planned = torch.cuda.Event()
         planned.record(comm)
         if quantised is not None:
             comm.wait_event(quantised)
         sms = num_dispatch_sms or (148 * DISPATCH_CTAS_PER_SM if lone else 148 if V == 1 else max(1, 148 // V - 1))
         C.em_dispatch(rts, [(w.xq if PREQUANTIZE else x, w.my_counts, w.sel_list, w.send_base, w.unit_start, w.peer_bases, None,
-                             None if w.trace is None else w.trace[0:2], w.xs if PREQUANTIZE else None) for x, w in zip(xs, wss)],
+                             None if w.trace is None else w.trace[0:2], w.xs if PREQUANTIZE else None, w.places) for x, w in zip(xs, wss)],
                       E, K, UNIT_ROWS, native, native, sms)
     if comm is not cur:
         cur.wait_event(planned)

@@ -273,3 +273,44 @@ def test_fused_products_say_how_many_rows_come(monkeypatch, R, T):
             assert hint == T * K * groups // (E // R)
     finally:
         vc.destroy()
+
+
+@pytest.mark.parametrize("T,H,E,K,native", [(1, 128, 4, 1, True), (77, 4224, 6, 4, True), (130, 7296, 300, 5, False)])
+def test_places_are_kept_where_they_are_asked_for(T, H, E, K, native):
+    """A lone rank's dispatch with places reads no lists, one without them goes by the lists alone, and nothing is written behind a list with room to spare."""
+    import deepep_efa_b200 as ep
+    from deepep_efa_b200.models.moe import UNIT_ROWS
+    vc, layers, xs, idxs, ws = _setup(1, T, H, 256, E, K, native)
+    try:
+        C = ep._ext.load()
+        rt, w, idx = vc.buffers[0].runtime, layers[0].fused_workspace(T), idxs[0]
+        assert w.places.shape == (T * K, 2) and w.sel_list.numel() == E * T
+        q, s = C.per_token_cast_to_fp8(xs[0], native, False)
+        roomy = torch.full((E * T + 4 * T * K + 8,), 7, dtype=torch.int32, device="cuda")
+        got = []
+        for places, lists in ((w.places, False), (None, True), (w.places, True)):
+            for t in (w.recv_x.view(torch.uint8), w.recv_scales_raw, w.recv_info):
+                t.zero_()
+            w.places.fill_(-1)
+            C.em_notify([rt], [(idx, w.recv_x, w.recv_scales_raw, w.recv_info, w.stage, w.my_counts, roomy, w.send_base, w.unit_start, w.m_offsets, w.m_ends,
+                                w.peer_bases, places)], E, UNIT_ROWS)
+            assert (w.places[:, 0] >= 0).sum() == (0 if places is None else (idx >= 0).sum())
+            if places is None:
+                w.places.fill_(-1)  # no row would move by them
+            if not lists:
+                roomy[:E * T] = 0   # every row would be token 0's by them
+            dst = torch.full((T * K,), -1, dtype=torch.int32, device="cuda")
+            C.em_dispatch([rt], [(q, w.my_counts, roomy, w.send_base, w.unit_start, w.peer_bases, dst, None, s, places)], E, K, UNIT_ROWS, native, native, 148 * 6)
+            torch.cuda.synchronize()
+            assert torch.equal(w.arrived, w.expected) and (roomy[E * T:] == 7).all()
+            got.append([t.clone() for t in (w.recv_x.view(torch.uint8), w.recv_scales_raw, w.recv_info, dst)])
+        vc.buffers[0].check_status()
+        for other in got[1:]:
+            assert all(torch.equal(a, b) for a, b in zip(got[0], other))
+        assert (got[0][3] >= 0).sum() == (idx >= 0).sum()
+        for bad in (w.places[:, 0], w.places.view(-1)[1:], w.places.long()):
+            with pytest.raises(ValueError):
+                C.em_notify([rt], [(idx, w.recv_x, w.recv_scales_raw, w.recv_info, w.stage, w.my_counts, roomy, w.send_base, w.unit_start, w.m_offsets,
+                                    w.m_ends, w.peer_bases, bad)], E, UNIT_ROWS)
+    finally:
+        vc.destroy()
