@@ -416,8 +416,8 @@ __global__ void __launch_bounds__(kEmLoneThreads) em_dispatch_lone_kernel(const 
             if (a.dst_row != nullptr) a.dst_row[t * K + lane] = row;
         }
     }
-    // (nobody waits for a lone rank's arrivals within this kernel)
-    if (blockIdx.x == 0 && any)
+    // The last CTA says what has arrived: whoever waits for these words finds every row in place, as behind the general kernel, whose units say it one by one.
+    if (any && cta_is_last(a.ctx.local_scratch + kTicketFused, gridDim.x))
         for (int e = tid; e < E; e += kEmLoneThreads)
             if (a.my_counts[e] > 0) red_add_release_gpu(&a.ctx.my_ctrl()->em_arrived[e], (uint64_t)a.my_counts[e]);
 }

@@ -314,3 +314,31 @@ def test_places_are_kept_where_they_are_asked_for(T, H, E, K, native):
                                     w.m_ends, w.peer_bases, bad)], E, UNIT_ROWS)
     finally:
         vc.destroy()
+
+
+@pytest.mark.parametrize("T,H,masked", [(1, 128, 0.0), (700, 4224, 0.05), (300, 7168, 1.0)])
+def test_lone_dispatches_in_a_row_count_their_arrivals(T, H, masked):
+    """One CTA to some hundred, none with a row to send: the last one of each call raises the words, and leaves the ticket that the exchange shares as it was."""
+    import deepep_efa_b200 as ep
+    from deepep_efa_b200.models.moe import UNIT_ROWS
+    E, K = 40, 3
+    vc, layers, xs, idxs, ws = _setup(1, T, H, 256, E, K, False, masked=masked)
+    try:
+        C = ep._ext.load()
+        rt, w, idx = vc.buffers[0].runtime, layers[0].fused_workspace(T), idxs[0]
+        q, s = C.per_token_cast_to_fp8(xs[0], False, False)
+        counts = torch.bincount(idx[idx >= 0], minlength=E)
+        before = w.arrived.clone()
+        for _ in range(5):
+            C.em_notify([rt], [(idx, w.recv_x, w.recv_scales_raw, w.recv_info, w.stage, w.my_counts, w.sel_list, w.send_base, w.unit_start, w.m_offsets,
+                                w.m_ends, w.peer_bases, w.places)], E, UNIT_ROWS)
+            C.em_dispatch([rt], [(q, w.my_counts, w.sel_list, w.send_base, w.unit_start, w.peer_bases, None, None, s, w.places)], E, K, UNIT_ROWS, False, False, 148)
+        torch.cuda.synchronize()
+        vc.buffers[0].check_status()
+        assert torch.equal(w.arrived - before, 5 * counts) and torch.equal(w.arrived, w.expected)
+        for e in range(E):
+            toks = (idx == e).nonzero()[:, 0]
+            row = int(w.m_offsets[e])
+            assert torch.equal(w.recv_x[row:row + toks.numel()].view(torch.uint8), q.view(torch.uint8)[toks])
+    finally:
+        vc.destroy()
