@@ -362,6 +362,16 @@ torch::Tensor swiglu_fwd(const torch::Tensor& h13) {
     return h;
 }
 
+// f32 [N] -> [4, N], see launch_logistic
+torch::Tensor logistic(const torch::Tensor& x) {
+    DXG_CHECK(x.is_cuda() && x.is_contiguous() && x.scalar_type() == torch::kFloat32 && x.dim() == 1, "logistic: contiguous CUDA f32 [N]");
+    c10::cuda::CUDAGuard guard(x.device());
+    auto out = torch::empty({4, x.size(0)}, x.options());
+    const cudaError_t e = dx::launch_logistic(x.data_ptr<float>(), out.data_ptr<float>(), x.size(0), at::cuda::getCurrentCUDAStream(x.get_device()).stream());
+    DXG_CHECK(e == cudaSuccess, "logistic launch failed");
+    return out;
+}
+
 torch::Tensor swiglu_bwd(const torch::Tensor& h13, const torch::Tensor& dh) {
     DXG_CHECK(h13.is_cuda() && h13.is_contiguous() && h13.scalar_type() == torch::kBFloat16 && h13.dim() == 2 && h13.size(1) % 16 == 0, "swiglu_bwd: contiguous CUDA bf16 [M, 2*I]");
     DXG_CHECK(dh.is_cuda() && dh.is_contiguous() && dh.scalar_type() == torch::kBFloat16 && dh.dim() == 2 && dh.size(0) == h13.size(0) && dh.size(1) * 2 == h13.size(1), "swiglu_bwd: dh must be bf16 [M, I]");
@@ -543,6 +553,7 @@ void bind_gemm(py::module_& m) {
     m.def("transpose_bf16", &transpose_bf16);
     m.def("swiglu_fwd", &swiglu_fwd);
     m.def("swiglu_bwd", &swiglu_bwd);
+    m.def("logistic", &logistic);
     m.def("unpermute_bwd", &unpermute_bwd);
     m.def("rowdot", &rowdot);
     m.def("grouped_gemm", &grouped_gemm, py::arg("a"), py::arg("b"), py::arg("m_offsets"), py::arg("mode") = 0, py::arg("swiglu") = false,

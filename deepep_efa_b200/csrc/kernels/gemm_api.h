@@ -128,6 +128,7 @@ cudaError_t launch_gather_reduce_rows(const void* src, void* dst, const int* pos
 //   out[b, c, r] = in[b, r, c]                     rows and cols multiples of 8
 cudaError_t launch_transpose_bf16(const void* in, void* out, int batch, int rows, int cols, cudaStream_t stream);
 //   h[m, i] = silu(h13[m, i]) * h13[m, inter + i]
+cudaError_t launch_logistic(const float* x, float* out, long long n, cudaStream_t stream);
 cudaError_t launch_swiglu_fwd(const void* h13, void* h, long long rows, int inter, cudaStream_t stream);
 //   dh13 = d/dh13 of the above given dh
 cudaError_t launch_swiglu_bwd(const void* h13, const void* dh, void* dh13, long long rows, int inter, cudaStream_t stream);

@@ -230,6 +230,23 @@ cudaError_t launch_swiglu_fwd(const void* h13, void* h, long long rows, int inte
     return launch_dependent(swiglu_fwd_kernel<long long>, grid, 256, 0, stream, in, out, work, inter);
 }
 
+// What the epilogues compute in fp32, beside the same with a division: [4, n] = silu, silu by division, sigmoid, sigmoid by division (for the tests).
+__global__ void __launch_bounds__(256) logistic_kernel(const float* __restrict__ x, float* __restrict__ out, long long n) {
+    for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < n; i += (long long)gridDim.x * 256) {
+        const float v = x[i], d = 1.f + __expf(-v);
+        out[i] = silu(v);
+        out[n + i] = v / d;
+        out[2 * n + i] = sigmoid(v);
+        out[3 * n + i] = 1.f / d;
+    }
+}
+
+cudaError_t launch_logistic(const float* x, float* out, long long n, cudaStream_t stream) {
+    if (n <= 0) return cudaSuccess;
+    logistic_kernel<<<148, 256, 0, stream>>>(x, out, n);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_swiglu_bwd(const void* h13, const void* dh, void* dh13, long long rows, int inter, cudaStream_t stream) {
     if (rows <= 0) return cudaSuccess;
     if ((inter & 7) != 0) return cudaErrorInvalidValue;
