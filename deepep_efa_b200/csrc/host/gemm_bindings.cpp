@@ -182,6 +182,7 @@ torch::Tensor grouped_gemm(const torch::Tensor& a, const torch::Tensor& b, const
         // natively block-scaled e4m3: a pair instantiation exists for the wide SwiGLU tile only
         if (fp8 && !(p.sfa_atoms != nullptr && p.mx_wide == 1)) p.cta_pairs = (pr != nullptr && pr[0] == '1' && p.sfa_atoms == nullptr) ? 1 : 0;
     }
+    p.narrow_promotion = fp8 && p.sfa_atoms == nullptr && !dx::wide_promotion_fits(swiglu) ? 1 : 0;
     if (ready.has_value() || expected.has_value()) {
         DXG_CHECK(mode == 0 && ready.has_value() && expected.has_value(), "ready and expected go together (M-grouped mode)");
         DXG_CHECK(ready->element_size() == 8 && expected->element_size() == 8 && ready->is_contiguous() && expected->is_contiguous() &&
@@ -514,7 +515,7 @@ torch::Tensor fp8_experts_promoted(const torch::Tensor& rows, const torch::Tenso
 }
 
 // What the rules of gemm_choice.h say about a product of these sizes (for the tests: they need no GPU). ends: whether m_ends is given.
-int promotion_columns(int64_t rows, int64_t groups, int64_t n, int64_t k, bool swiglu, bool ends, int64_t rows_hint, int num_sms) {
+int promotion_columns(int64_t rows, int64_t groups, int64_t n, int64_t k, bool swiglu, bool ends, int64_t rows_hint, int num_sms, bool fits) {
     dx::GroupedGemmArgs p{};
     const int there = 0;
     p.m_total = (int)rows;
@@ -525,6 +526,7 @@ int promotion_columns(int64_t rows, int64_t groups, int64_t n, int64_t k, bool s
     p.m_ends = ends ? &there : nullptr;
     p.rows_hint = (int)rows_hint;
     p.num_sms = num_sms;
+    p.narrow_promotion = fits ? 0 : 1;
     return dx::wide_promotion(p) ? 256 : 128;
 }
 
@@ -547,7 +549,8 @@ void bind_gemm(py::module_& m) {
     m.def("bf16_form", &bf16_form, py::arg("rows"), py::arg("groups"), py::arg("n"), py::arg("k"), py::arg("mn_major") = false, py::arg("ends") = false,
           py::arg("zero_tail") = false, py::arg("num_sms") = 148);
     m.def("promotion_columns", &promotion_columns, py::arg("rows"), py::arg("groups"), py::arg("n"), py::arg("k"), py::arg("swiglu") = false, py::arg("ends") = false,
-          py::arg("rows_hint") = 0, py::arg("num_sms") = 148);
+          py::arg("rows_hint") = 0, py::arg("num_sms") = 148, py::arg("fits") = true);
+    m.def("wide_promotion_fits", &dx::wide_promotion_fits);
     m.def("build_sf_atoms_a", &build_sf_atoms_a, py::arg("scales"), py::arg("group_counts") = py::none(), py::arg("rows_per_group") = 0);
     m.def("build_sf_atoms_b", &build_sf_atoms_b, py::arg("scales"), py::arg("n"), py::arg("swiglu") = false, py::arg("wide") = false);
     m.def("transpose_bf16", &transpose_bf16);

@@ -50,6 +50,7 @@ struct GroupedGemmArgs {
     int rows_hint;            // how many rows all groups have together, where that is less than m_total (0 = not known)
     int tile_order;           // mode 0: 0 = weight tile shared by consecutive CTAs, 1 = activation tile shared
     int cta_pairs;            // 1 = two CTAs of a cluster share one 256-row MMA (cta_group::2), each staging half of the B tile
+    int narrow_promotion;     // 1 = this build's 256-column promotion cannot run (wide_promotion_fits), 128 columns take its place
     int* error_flag;          // device int, set non-zero when a bounded pipeline wait ran out
     long long timeout_cycles;
     // Arrival gating (mode 0): the rows of group g are written by other GPUs while this kernel runs. Before the first tile
@@ -94,6 +95,8 @@ struct GroupedGemmArgs {
 
 // Returns cudaErrorInvalidValue for unsupported shapes (divisibility rules are in grouped_gemm.cu).
 cudaError_t launch_grouped_gemm(const GroupedGemmArgs& args, cudaStream_t stream);
+// Whether the compiler gave the 256-column promotion the registers that its warps move between them (another toolkit, -G or -maxrregcount may not).
+bool wide_promotion_fits(bool swiglu);
 // The same product for groups of few to some hundred rows (gemm_cols.cu): natively block-scaled operands with 256-column weight atoms,
 // mode 0, n % 256 == 0; SwiGLU writes c_fp8 and c_atoms, otherwise bf16 rows to c or through the scatter epilogue.
 cudaError_t launch_token_cols_gemm(const GroupedGemmArgs& args, cudaStream_t stream);

@@ -33,7 +33,7 @@ inline long long tiles_up(long long a, long long b) { return (a + b - 1) / b; }
 // the tiles: where two of 32 experts are in use, 1.2 to 1.36, where all are, 0.5 to 1; it keeps the narrow ones.
 inline bool wide_promotion(const GroupedGemmArgs& a) {
     const bool ends = a.m_ends != nullptr;
-    if (a.cta_pairs || a.n % 256 != 0 || (ends && a.rows_hint <= 0)) return false;
+    if (a.narrow_promotion || a.cta_pairs || a.n % 256 != 0 || (ends && a.rows_hint <= 0)) return false;
     long long row_tiles = tiles_up(a.m_total, 128);
     if (a.rows_hint > 0) {
         // groups that get a row, each with half a tile to spare, but one tile at least

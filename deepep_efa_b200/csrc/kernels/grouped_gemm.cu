@@ -1304,6 +1304,16 @@ bool make_map_sf(CUtensorMap* map, const void* ptr, uint64_t rows, uint32_t word
     return r == CUDA_SUCCESS;
 }
 
+template <typename C, typename Kernel>
+bool has_registers(Kernel kernel) {
+    cudaFuncAttributes attributes;
+    if (cudaFuncGetAttributes(&attributes, kernel) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return attributes.numRegs == C::kLaunchRegs;
+}
+
 template <int kBlockN, bool kFp8, bool kSwiGLU, bool kPair, bool kMx = false, bool kRowScatter = false, bool kWgrad = false>
 cudaError_t launch_impl(const GroupedGemmArgs& a, cudaStream_t stream) {
     using C = Cfg<kBlockN, kFp8, kSwiGLU, kPair, kMx, kRowScatter>;
@@ -1342,11 +1352,8 @@ cudaError_t launch_impl(const GroupedGemmArgs& a, cudaStream_t stream) {
     if (dev < 0 || dev >= 64 || !smem_opted_in[dev]) {
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::kSmemBytes);
         if (e != cudaSuccess) return e;
-        if constexpr (C::kMoveRegs) {  // launched with fewer registers the epilogue would wait for more forever
-            cudaFuncAttributes attributes;
-            e = cudaFuncGetAttributes(&attributes, kernel);
-            if (e != cudaSuccess) return e;
-            if (attributes.numRegs != C::kLaunchRegs) return cudaErrorLaunchOutOfResources;
+        if constexpr (C::kMoveRegs) {  // launched with fewer registers the epilogue would wait for more forever; the choice has asked (wide_promotion_fits)
+            if (!has_registers<C>(kernel)) return cudaErrorLaunchOutOfResources;
         }
         if (dev >= 0 && dev < 64) smem_opted_in[dev] = true;
     }
@@ -1380,6 +1387,15 @@ cudaError_t launch_sel(const GroupedGemmArgs& a, cudaStream_t stream) {
 }
 
 }  // namespace
+
+bool wide_promotion_fits(bool swiglu) {
+    if (swiglu) {  // (once each: every device runs the same code)
+        static const bool fits = has_registers<Cfg<256, true, true, false>>(grouped_gemm_kernel<256, true, true, false>);
+        return fits;
+    }
+    static const bool fits = has_registers<Cfg<256, true, false, false>>(grouped_gemm_kernel<256, true, false, false>);
+    return fits;
+}
 
 cudaError_t launch_grouped_gemm(const GroupedGemmArgs& a, cudaStream_t stream) {
     if (a.num_groups < 1 || a.num_groups > kMaxGroups || a.num_sms < 1) return cudaErrorInvalidValue;

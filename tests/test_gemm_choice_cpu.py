@@ -65,3 +65,11 @@ def test_promotion_tile_width(rows, groups, n, k, swiglu, how, columns):
 ])
 def test_form_of_bf16_products(rows, groups, n, k, how, form):
     assert C.bf16_form(rows, groups, n, k, **how) == form
+
+
+@pytest.mark.parametrize("swiglu,how", [(True, {}), (False, {}), (True, dict(ends=True, rows_hint=64 * 512))])
+def test_promotion_without_registers_for_wide_tiles(swiglu, how):
+    """A build whose 256-column kernel did not get the registers that its warps move between them takes 128 columns, which compute the same."""
+    size = (64 * 512, 64, 4096, 4096, swiglu)
+    assert C.promotion_columns(*size, **how) == 256
+    assert C.promotion_columns(*size, fits=False, **how) == 128

@@ -212,6 +212,13 @@ def test_logistic_in_fp32_like_the_division(which):
             assert off.square().mean() <= 1.0001 * off_plain.square().mean() and off.max() <= off_plain.max() + 2
 
 
+@pytest.mark.parametrize("swiglu", [False, True])
+def test_wide_promotion_has_its_registers(swiglu):
+    """In this build the choice is free to take tiles of 256 columns."""
+    from deepep_efa_b200 import _ext
+    assert _ext.load().wide_promotion_fits(swiglu)
+
+
 def test_rowdot_kernel():
     from deepep_efa_b200 import _ext
     torch.manual_seed(9)
