@@ -530,7 +530,7 @@ cudaError_t launch_cols_impl(const GroupedGemmArgs& a, cudaStream_t stream) {
         if (!make_map(&maps_t.m[i], a.a, true, (uint64_t)a.m_total, (uint64_t)a.k, 128 >> i)) return cudaErrorInvalidValue;
     const size_t fixed = 1024 /*align*/ + 256 /*barriers*/ + cols_table_bytes(a.num_groups) + cols_exchange_bytes(a.token_cap, kSwiGLU);
     const int stages = std::min(kMaxStages, (int)((kMaxSmem - 512 /*static*/ - fixed) / cols_stage_bytes(a.token_cap)));
-    const size_t smem = fixed + (size_t)stages * cols_stage_bytes(a.token_cap);
+    const size_t smem = std::max(kTensorKernelSmem, fixed + (size_t)stages * cols_stage_bytes(a.token_cap));
     auto kernel = token_cols_gemm_kernel<kSwiGLU>;
     static bool smem_opted_in[64] = {};  // per device, once: the attribute is sticky
     int dev = 0;

@@ -309,7 +309,7 @@ cudaError_t launch_pairs_impl(const GroupedGemmArgs& a, cudaStream_t stream) {
         if (!make_map(&maps.t[i], a.a, false, (uint64_t)a.m_total, (uint64_t)a.k, 128 >> i)) return cudaErrorInvalidValue;
     const size_t fixed = 1024 /*align*/ + kPairEpiWarps * kBlockBytes + 256 /*barriers*/ + ((size_t)(a.num_groups + 1) * 4 + 15) / 16 * 16;
     const int stages = std::min(kPairMaxStages, (int)((kPairMaxSmem - fixed) / pair_stage_bytes(a.token_cap)));
-    const size_t smem = fixed + (size_t)stages * pair_stage_bytes(a.token_cap);
+    const size_t smem = std::max(kTensorKernelSmem, fixed + (size_t)stages * pair_stage_bytes(a.token_cap));
     auto kernel = token_pairs_gemm_kernel<kMn>;
     static bool smem_opted_in[64] = {};  // per device, once: the attribute is sticky
     int dev = 0;

@@ -204,6 +204,7 @@ struct Cfg {
     static constexpr size_t kSmemBytes =
         (size_t)kStages * kStageBytes + (size_t)kEpiWarps * kOutStageBytes + 1024 /*align*/ + 256 /*barriers*/ + (kMaxGroups + 2) * 4 + kXchBytes +
         (kGroupTable ? kMaxGroups * 8 : 0);
+    static_assert(kSmemBytes >= kTensorKernelSmem, "kernels with tensor memory must not share an SM");
 };
 
 // kWgrad: weight gradients with both operands read in place. What is fixed for them costs no instructions (every launch fetches its code anew, and an MMA whose

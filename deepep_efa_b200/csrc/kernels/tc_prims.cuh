@@ -107,6 +107,12 @@ __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* map) {
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
+// Kernels allocate tensor memory in front of their wait for the predecessor, and an allocation blocks, without a limit, until the columns are free. Were a CTA
+// of the predecessor still to allocate on the same SM, each would wait for the other; a predecessor's other warps may release the successor before that. So no
+// two of these kernels share an SM: each takes at least this much of its 228 KB of shared memory (1 KB more per CTA is the system's).
+constexpr size_t kTensorKernelSmem = 114 * 1024;
+static_assert(2 * (kTensorKernelSmem + 1024) > 228 * 1024, "two kernels with tensor memory must not fit one SM");
+
 __device__ __forceinline__ void tmem_alloc(uint32_t* dst_smem, uint32_t ncols) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(dst_smem)), "r"(ncols) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
