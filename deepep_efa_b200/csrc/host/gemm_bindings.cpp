@@ -270,6 +270,7 @@ torch::Tensor grouped_gemm(const torch::Tensor& a, const torch::Tensor& b, const
         cudaGetLastError();
         throw std::runtime_error(std::string("deepep_efa_b200.grouped_gemm: launch failed: ") + cudaGetErrorString(e));
     }
+    if (mode == 1 && p.m_total == 0) c.zero_();  // sums over no rows, for which nothing was launched
     if (cast_after.x != nullptr && dx::launch_fp8_cast(cast_after, at::cuda::getCurrentCUDAStream(device).stream()) != cudaSuccess)
         throw std::runtime_error("deepep_efa_b200.grouped_gemm: launch of the cast failed");
     return c;

@@ -152,3 +152,34 @@ def test_fp8_forward_of_a_rank_without_rows(native, path):
         assert y.shape == x.shape and not y.any()
     finally:
         vc.destroy()
+
+
+@pytest.mark.parametrize("hidden,inter", [(512, 256), (256, 128)])
+def test_training_step_of_a_rank_without_rows(hidden, inter):
+    """Nobody selects an expert of this rank: zeros, and gradients that are zeros too, those of the weights among them."""
+    from deepep_efa_b200.models.moe import MoEConfig, MoELayer
+    from deepep_efa_b200.parallel.virtual import VirtualCluster
+    vc = VirtualCluster(1, num_nvl_bytes=64 << 20)
+    try:
+        layer = MoELayer(MoEConfig(hidden=hidden, intermediate=inter, num_experts=8, num_topk=2), vc.buffers[0])
+        x, idx, w = make_tokens(5, hidden, "cuda").requires_grad_(True), torch.full((5, 2), -1, device="cuda"), torch.ones(5, 2, device="cuda", requires_grad=True)
+        dirt = [torch.full_like(p, float("nan")) for p in (layer.w13, layer.w2)]  # what the gradients' memory held before
+        del dirt
+        y = layer(x, idx, w)
+        y.backward(torch.ones_like(y))
+        torch.cuda.synchronize()
+        vc.buffers[0].check_status()
+        for t in (y, x.grad, w.grad, layer.w13.grad, layer.w2.grad):
+            assert (t == 0).all()
+    finally:
+        vc.destroy()
+
+
+@pytest.mark.parametrize("in_place", [False, True])
+def test_weight_gradient_over_no_rows(in_place):
+    from deepep_efa_b200.ops import grouped_gemm as gg
+    offs = torch.zeros(4, dtype=torch.int32, device="cuda")
+    out = torch.full((3, 128, 256), float("nan"), dtype=torch.bfloat16, device="cuda")
+    a, b = (torch.empty((0, n) if in_place else (n, 0), dtype=torch.bfloat16, device="cuda") for n in (128, 256))
+    got = (gg.grouped_gemm_wgrad_inplace if in_place else gg.grouped_gemm_wgrad)(a, b, offs, out=out)
+    assert got.data_ptr() == out.data_ptr() and (out == 0).all()
