@@ -360,10 +360,10 @@ class Buffer:
         event)``; the second entry (tokens per RDMA rank = per NVLink domain, i32 ``[domains]``) is ``None`` when the
         group is a single NVLink domain (deep_ep/buffer.py:422-448).
         """
-        topk_idx = _as_topk_idx(topk_idx)
         if self._hier is not None:
             _wait_previous(previous_event)
-            return self._hier.get_dispatch_layout(topk_idx, num_experts)
+            return self._hier.get_dispatch_layout(_as_topk_idx(topk_idx), num_experts)
+        topk_idx = self._ids_behind(previous_event, topk_idx)
         if self._cpu is not None:
             a, b, c = self._cpu.get_dispatch_layout(topk_idx, num_experts)
             return a, None, b, c, EventOverlap()
@@ -397,16 +397,16 @@ class Buffer:
         Rows of ``recv_x`` are ordered by source rank, then by token order at the source. The returned
         tensors live in this rank's symmetric arena; their memory returns to the arena when they die.
         """
-        topk_idx = _as_topk_idx(topk_idx)
         if self._hier is not None:
             return self.internode_dispatch(x, handle, num_tokens_per_rank, num_tokens_per_rdma_rank, is_token_in_rank,
                                            num_tokens_per_expert, topk_idx, topk_weights, expert_alignment, num_worst_tokens, config,
                                            previous_event, async_finish, allocate_on_comm_stream, quantize_fp8=quantize_fp8,
                                            round_scale=round_scale)
         if self._cpu is not None:
-            return self._cpu.dispatch(x, handle, num_tokens_per_rank, is_token_in_rank, num_tokens_per_expert, topk_idx,
+            return self._cpu.dispatch(x, handle, num_tokens_per_rank, is_token_in_rank, num_tokens_per_expert, _as_topk_idx(topk_idx),
                                       topk_weights, expert_alignment, num_worst_tokens)
         # what _dispatch_many does for several emulated ranks, for one, in a straight line (see _on_callers_stream)
+        topk_idx = self._ids_behind(previous_event, topk_idx)
         self.check_status()
         used = config if config is not None else self.get_dispatch_config(self.group_size)
         num_sms, num_channels = _normal_sms(used, config is not None, [self]), _num_channels(used)
@@ -463,6 +463,17 @@ class Buffer:
         native = _named("ep.combine", self._C.normal_combine_on)
         out, out_w = native(self._comm_key(), _event_of(previous_event), async_finish, allocate_on_comm_stream, self.runtime, call, num_sms)
         return out, out_w, self._comm_event(async_finish, (x, topk_weights, b0, b1))
+
+    def _ids_behind(self, previous_event, topk_idx):
+        """Expert ids as the kernels take them. Where the communication stream waits for an event alone, ids that have to be widened are so on that stream:
+        the caller's may be short of the event, or behind work that the event does not cover."""
+        if topk_idx is None or topk_idx.dtype == torch.int64 or not topk_idx.is_cuda or _event_of(previous_event) is None:
+            return _as_topk_idx(topk_idx)
+        with torch.cuda.stream(self._comm_stream):
+            previous_event.current_stream_wait()
+            wide = _as_topk_idx(topk_idx)
+        topk_idx.record_stream(self._comm_stream)
+        return wide
 
     def _comm_key(self) -> Tuple[int, int]:
         stream = self._comm_stream

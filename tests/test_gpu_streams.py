@@ -451,3 +451,45 @@ def test_results_of_a_combine_behind_an_event(entry, asynchronous):
         assert torch.equal(out, want) and torch.equal(out_w, want_w)
     finally:
         vc.destroy()
+
+
+@pytest.mark.parametrize("asynchronous", [False, True])
+def test_ids_of_32_bits_behind_an_event(asynchronous):
+    """Written on a third stream and covered by the event, while the caller's stream is busy with something else: they are widened behind the event, not
+    behind (or in front of) the caller's work, and may be dropped."""
+    from deepep_efa_b200.utils.event import EventHandle, EventOverlap
+    vc, buf = _buffer()
+    try:
+        idx, w = make_routing(T, E, K, "cuda", seed=8, masked_fraction=0.2)
+        x = make_tokens(T, H, "cuda", seed=8)
+        lay, _ = _layout(buf, idx)
+        want = [t.clone() for t in (lay["num_tokens_per_expert"], lay["is_token_in_rank"])]
+        y, want_idx, want_w, counts, handle, _ = buf.dispatch(x, topk_weights=w, **lay)
+        narrow, side = idx.int(), torch.cuda.Stream()
+        for caller_busy in (False, True):
+            ids = torch.full_like(narrow, -1)
+            torch.cuda.synchronize()
+            with torch.cuda.stream(side):
+                torch.cuda._sleep(DELAY)
+                ids.copy_(narrow)
+                written = EventOverlap(EventHandle())
+            if caller_busy:
+                _delay(torch.cuda.current_stream())
+                torch.cuda._sleep(DELAY)
+            per_rank, _, per_expert, in_rank, ev = buf.get_dispatch_layout(ids, E, previous_event=written, async_finish=asynchronous)
+            ev = ev if asynchronous else written
+            got = buf.dispatch(x, num_tokens_per_rank=per_rank, is_token_in_rank=in_rank, num_tokens_per_expert=per_expert, topk_idx=ids, topk_weights=w,
+                               previous_event=ev if asynchronous else None, async_finish=asynchronous)
+            got_event = buf.dispatch(x, num_tokens_per_rank=per_rank, is_token_in_rank=in_rank, num_tokens_per_expert=per_expert, topk_idx=ids, topk_weights=w,
+                                     previous_event=ev, async_finish=asynchronous)
+            del ids
+            keep = _overwrite([(T, K)])
+            for out in (got, got_event):
+                out[5].current_stream_wait()
+            assert torch.equal(per_expert, want[0]) and torch.equal(in_rank, want[1])
+            for out in (got, got_event):
+                assert out[3] == counts and torch.equal(out[0], y) and torch.equal(out[1], want_idx) and torch.equal(out[2], want_w)
+            del keep
+        buf.check_status(sync=True)
+    finally:
+        vc.destroy()
