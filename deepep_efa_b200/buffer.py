@@ -975,6 +975,7 @@ def _ll_stream_enter(buf: Buffer, async_finish: bool):
 
 
 def _ll_stream_exit(buf: Buffer, ctx, tensors) -> EventOverlap:
+    """``tensors``: all that the caller may drop while the communication stream has yet to use it (the stream waits for the caller's, not the other way)."""
     if ctx is None:
         return EventOverlap()
     ctx.__exit__(None, None, None)
@@ -1018,7 +1019,7 @@ def _ll_dispatch_many(bufs: List[Buffer], calls, num_max_tokens: int, num_expert
     ctx, _ = _ll_stream_enter(bufs[0], async_finish)
     with nvtx_range("ep.ll_dispatch"):
         launch(1 if return_recv_hook else 3)
-    event = _ll_stream_exit(bufs[0], ctx, [c[0] for c in calls] + [c[1] for c in calls])
+    event = _ll_stream_exit(bufs[0], ctx, [t for c in calls for t in c])
     hook = (lambda: launch(2)) if return_recv_hook else None
     return [(rx, cnt, handle, event, hook) for rx, cnt, handle in results]
 
@@ -1057,6 +1058,6 @@ def _ll_combine_many(bufs: List[Buffer], calls, zero_copy: bool, async_finish: b
     ctx, _ = _ll_stream_enter(bufs[0], async_finish)
     with nvtx_range("ep.ll_combine"):
         launch(1 if return_recv_hook else 3)
-    event = _ll_stream_exit(bufs[0], ctx, [c[0] for c in calls] + [o for o in outs if o.is_cuda])
+    event = _ll_stream_exit(bufs[0], ctx, [t for c in calls for t in c] + outs)
     hook = (lambda: launch(2)) if return_recv_hook else None
     return [(o, event, hook) for o in outs]

@@ -493,3 +493,43 @@ def test_ids_of_32_bits_behind_an_event(asynchronous):
         buf.check_status(sync=True)
     finally:
         vc.destroy()
+
+
+@pytest.mark.parametrize("ids", [torch.int64, torch.int32])
+def test_inputs_dropped_behind_asynchronous_low_latency_calls(ids):
+    """Tokens, ids (widened or not), weights and counters that die while the communication stream has yet to use them."""
+    import deepep_efa_b200 as ep
+    from deepep_efa_b200.parallel.virtual import VirtualCluster
+    n, hidden = 64, 1024
+    vc = VirtualCluster(1, num_nvl_bytes=64 << 20, num_rdma_bytes=ep.Buffer.get_low_latency_rdma_size_hint(n, hidden, 1, E), timeout_ms=5000)
+    try:
+        buf = vc.buffers[0]
+        idx, w = make_routing(n, E, K, "cuda", seed=9, masked_fraction=0.2)
+        x, y = make_tokens(n, hidden, "cuda", seed=9), make_tokens(E * n, hidden, "cuda", seed=10).view(E, n, hidden)
+
+        def step(given, **how):
+            x, idx, w, y, seen = given
+            recv, count, handle, first, _ = buf.low_latency_dispatch(x, idx, n, E, cumulative_local_expert_recv_stats=seen, use_fp8=False, **how)
+            out, second, _ = buf.low_latency_combine(y, idx, w, handle, **how)
+            return recv, count, out, (first, second)
+
+        def fresh():
+            return [x.clone(), idx.to(ids), w.clone(), y.clone(), torch.zeros(E, dtype=torch.int32, device="cuda")]
+
+        _, _, want, _ = step(fresh())
+        for _ in range(3):
+            given = fresh()
+            torch.cuda.synchronize()
+            _delay(buf.comm_stream)
+            recv, count, out, events = step(given, async_finish=True)
+            del given
+            keep = _overwrite([(n, K), (n, 2 * K), (E,), (n, hidden // 2)]) + _overwrite([(E, n, hidden // 2)], copies=2)
+            for event in events:
+                event.current_stream_wait()
+            torch.cuda.synchronize()
+            assert torch.equal(out, want) and count.sum() == (idx >= 0).sum()
+            assert not any(bool(t.any()) for t in keep)
+            del keep, out
+        buf.check_status(sync=True)
+    finally:
+        vc.destroy()
