@@ -444,16 +444,18 @@ torch::Tensor build_sf_atoms_b(const torch::Tensor& scales, int64_t n, bool swig
     return atoms;
 }
 
-// src [N, H] in a plan's order [M, H], zero rows as padding; pos [N, K] and src_row [M] are the plan's maps.
-torch::Tensor permute_rows(const torch::Tensor& src, const torch::Tensor& pos, const torch::Tensor& src_row) {
+// src [N, H] in a plan's order [M, H], zero rows as padding; src_row [M] and pos [N, K] are the plan's maps. What pos says is only another way to the same rows:
+// one of another type or shape, or none, is no error.
+torch::Tensor permute_rows(const torch::Tensor& src, const c10::optional<torch::Tensor>& pos, const torch::Tensor& src_row) {
     DXG_CHECK(src.is_cuda() && src.dim() == 2 && src.is_contiguous(), "src must be a contiguous CUDA matrix");
     const int64_t row_bytes = src.size(1) * src.element_size();
     DXG_CHECK(row_bytes % 4 == 0, "row size must be a multiple of 4 bytes");
     DXG_CHECK(src_row.device() == src.device() && src_row.scalar_type() == torch::kInt32 && src_row.is_contiguous() && src_row.dim() == 1, "src_row must be int32 [M]");
-    DXG_CHECK(pos.device() == src.device() && pos.scalar_type() == torch::kInt32 && pos.is_contiguous() && pos.dim() == 2 && pos.size(0) == src.size(0), "pos must be int32 [N, K]");
+    const bool usable = pos.has_value() && pos->device() == src.device() && pos->scalar_type() == torch::kInt32 && pos->is_contiguous() && pos->dim() == 2 &&
+                        pos->size(0) == src.size(0);
     c10::cuda::CUDAGuard guard(src.device());
     const torch::Tensor dst = torch::empty({src_row.numel(), src.size(1)}, src.options());
-    const cudaError_t e = dx::launch_permute_rows(src.data_ptr(), dst.data_ptr(), pos.data_ptr<int>(), src_row.data_ptr<int>(), (int)src.size(0), (int)pos.size(1),
+    const cudaError_t e = dx::launch_permute_rows(src.data_ptr(), dst.data_ptr(), usable ? pos->data_ptr<int>() : nullptr, src_row.data_ptr<int>(), (int)src.size(0), usable ? (int)pos->size(1) : 0,
                                                   (int)src_row.numel(), (int)row_bytes, at::cuda::getCurrentCUDAStream(src.get_device()).stream());
     if (e != cudaSuccess) throw std::runtime_error(std::string("permute_rows: ") + cudaGetErrorString(e));
     return dst;

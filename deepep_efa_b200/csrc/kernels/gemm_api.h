@@ -117,7 +117,7 @@ cudaError_t launch_build_plan(const int64_t* topk_idx, const int* host_offsets, 
 //   are multiples of 4 bytes (of 16 when scaled).
 cudaError_t launch_gather_rows(const void* src, void* dst, const int* src_row, const float* scale, int num_dst_rows, int row_bytes,
                                cudaStream_t stream);
-// The same without a scale for a plan's two maps: src_row, and pos [num_src_rows, num_k], where each row goes (-1: nowhere).
+// The same without a scale for a plan's two maps: src_row, which decides, and pos [num_src_rows, num_k] (may be null), where each row goes (-1: nowhere).
 cudaError_t launch_permute_rows(const void* src, void* dst, const int* pos, const int* src_row, int num_src_rows, int num_k, int num_dst_rows, int row_bytes, cudaStream_t stream);
 // Rows of e4m3 with their fp32 scales per 128 channels (hidden % 128 == 0), gathered in one launch: scales as they are [num_dst_rows, hidden/128], or with
 // `atoms` as scale atoms (powers of two; whole tiles of 128 rows). Clears the two words at `sched` (may be null), for the products behind it.

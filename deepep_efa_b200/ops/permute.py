@@ -102,7 +102,7 @@ class _Permute(torch.autograd.Function):
     @staticmethod
     def forward(ctx, recv_x, plan: ExpertPlan):
         ctx.plan = plan
-        if recv_x.is_cuda and plan.pos.size(0) == recv_x.size(0):
+        if recv_x.is_cuda:
             return _ext.load().permute_rows(recv_x.contiguous(), plan.pos, plan.src_row)
         return gather_rows(recv_x, plan.src_row)
 

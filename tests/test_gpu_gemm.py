@@ -759,3 +759,28 @@ def test_token_columns_hold_their_successor():
         torch.cuda.synchronize()
     assert C.gemm_error(0) == 0
     assert stamps[0][1].item() <= stamps[1][0].item()
+
+
+@pytest.mark.parametrize("N,K,H", [(6300, 6, 4096), (6300, 1, 4096), (3600, 8, 7176), (700, 6, 1024)])
+def test_permutation_by_changed_plans(N, K, H):
+    """Above and below the size from which rows are spread instead of gathered: what src_row says decides, whatever was done to either map since."""
+    import dataclasses
+    from deepep_efa_b200.ops.permute import build_expert_plan, gather_rows, permute
+    torch.manual_seed(3)
+    idx = torch.rand(N, 16, device="cuda").topk(K, dim=1).indices
+    idx[torch.rand(N, K, device="cuda") < 0.1] = -1
+    counts = [(int((idx == e).sum()) + 127) // 128 * 128 for e in range(16)]
+    plan, x = build_expert_plan(idx, counts), torch.randn(N, H, device="cuda").to(torch.bfloat16)
+    M = plan.num_rows
+    dropped, other, short = plan.src_row.clone(), plan.src_row.clone(), plan.pos.clone()
+    dropped[torch.rand(M, device="cuda") < 0.2] = -1
+    some = torch.rand(M, device="cuda") < 0.2
+    other[some] = torch.randint(0, N, (M,), device="cuda", dtype=torch.int32)[some]
+    short[torch.rand(N, K, device="cuda") < 0.2] = -1
+    wild = torch.randint(-5, 2 * M, (N, K), device="cuda", dtype=torch.int32)
+    for change in ({}, dict(src_row=dropped), dict(src_row=other), dict(pos=short), dict(pos=wild), dict(pos=plan.pos[:0]), dict(pos=plan.pos.long()), dict(pos=None),
+                   dict(pos=plan.pos.t().contiguous().t()), dict(src_row=plan.src_row[: M - 77].contiguous()), dict(src_row=dropped, pos=wild)):
+        changed = dataclasses.replace(plan, **change)
+        dirt = torch.full((M, H), float("nan"), dtype=torch.bfloat16, device="cuda")
+        del dirt
+        assert torch.equal(permute(x, changed), gather_rows(x, changed.src_row)), change.keys()
