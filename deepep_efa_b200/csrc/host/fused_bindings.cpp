@@ -122,7 +122,8 @@ void em_notify(std::vector<py::object> rts, std::vector<py::tuple> per_rank, int
 
 // Per rank tuple: (x, my_counts, sel_list, send_base, unit_start, peer_bases, dst_row|None, trace|None, x_scales|None[, places|None])
 // x is bf16 (rows are quantised by the kernel) or, with x_scales, e4m3 rows quantised beforehand (copied as they are). With `places`, as em_notify has
-// written them, a lone rank that may use every SM sends such rows token by token and reads no sel_list.
+// written them, a lone rank that may use every SM sends such rows token by token, reads no sel_list and
+// leaves the arrival counters to the next em_notify: no product may be gated on that call.
 void em_dispatch(std::vector<py::object> rts, std::vector<py::tuple> per_rank, int num_experts, int num_topk, int unit_rows,
                  bool round_scale, bool native_atoms, int num_sms) {
     const int V = (int)rts.size();
@@ -195,7 +196,8 @@ void em_dispatch(std::vector<py::object> rts, std::vector<py::tuple> per_rank, i
 }
 
 // Views of the expert-major control words of this rank: (arrival counters [kMaxLocalExperts] u64 inside the symmetric
-// control block, expected totals [kMaxLocalExperts] u64 in rank-local memory), as int64 tensors that the gated GEMM reads.
+// control block, expected totals [kMaxLocalExperts] u64 in rank-local memory), as int64 tensors that the gated GEMM reads. After an em_dispatch of a lone rank
+// with places the counters stay behind, so that a gate gives up instead of letting a product read early.
 std::pair<torch::Tensor, torch::Tensor> em_gate_words(py::object rt) {
     dxh::RuntimeCore* core = dx_core_of(rt);
     auto opts = torch::TensorOptions().dtype(torch::kInt64).device(torch::kCUDA, core->device());

@@ -166,7 +166,7 @@ struct EmDispatchArgs {
     int native_atoms;             // 1: scales are written as the UE8M0 words of [row tile][K block][512] scale atoms
     const int* my_counts;
     const int* sel_list;
-    const int2* places;           // of em_notify, or nullptr
+    const int2* places;           // of em_notify, or nullptr; a lone rank's kernel that goes by them does not count arrivals
     const int* send_base;
     const int* unit_start;
     int* unit_counter;            // [1] next unit to hand out (zeroed by the count exchange)

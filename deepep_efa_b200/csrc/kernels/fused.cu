@@ -156,8 +156,11 @@ __global__ void __launch_bounds__(kEmNotifyThreads, 1) em_notify_kernel(const __
             const int g = me * L + le;
             a.m_offsets[le] = s_base[g];
             a.m_ends[le] = s_base[g] + s_total[g];
-            // rows this expert will have received once this call's dispatch is complete (monotonic over the calls)
-            c.seq[kFusedExpectedWord0 + le] += (uint64_t)s_total[g];
+            // rows this expert will have received once this call's dispatch is complete (monotonic over the calls). What a lone rank was to receive by now is
+            // in place: the kernels of earlier calls are complete, also those that count no arrivals (em_dispatch_lone_kernel).
+            const uint64_t expected = c.seq[kFusedExpectedWord0 + le];
+            if (R == 1) my->em_arrived[le] = expected;
+            c.seq[kFusedExpectedWord0 + le] = expected + (uint64_t)s_total[g];
         }
         if (tid == 0) a.m_offsets[L] = s_rank_rows[me];
         if (tid == 0) *a.unit_counter = 0;
@@ -361,11 +364,16 @@ __global__ void __launch_bounds__(kEmDispatchThreads, 6) em_dispatch_kernel(cons
 
 // A lone rank copies its quantised rows within its own memory, so experts need not complete in order: a warp loads a span of a token's row once and stores it to
 // all of the token's rows. Expert by expert the rows were read again for each selection, from HBM, since what is written pushes them out of the L2 (rows of
-// 52736 x 8 KB written at 3.2 TB/s with reads from 67 MB, at 6.5 without). Behind the exchange, 4096 x 8 rows of 1 KB 38.4 -> 26.8 us, 4096 x 6 27.4 -> 19.5; in a layer
-// at the power limit, 4096 x 8 rows of 7 KB 96 -> 55.
+// 52736 x 8 KB written at 3.2 TB/s with reads from 67 MB, at 6.5 without). Behind the exchange, 4096 x 8 rows of 1 KB 38.4 -> 25.3 us, 4096 x 6 27.4 -> 19.0; in a layer
+// at the power limit, 4096 x 8 rows of 7 KB 96 -> 55. No CTA knows when an expert's rows are complete, so arrivals are not counted here: nothing on this GPU may
+// gate on them (a gate would run into its limit), and the next exchange makes up for it. Counted by the last CTA to finish, with a ticket, the kernel
+// itself took 11.4 -> 13.8 us with rows of 1 KB, 46.4 -> 47.8 with 7 KB.
+// Four CTAs share an SM, by shared memory that none of them uses: more of them write more rows at a time than the memory takes well (4096 x 8 rows of 1 / 2 / 7 KB, CTAs
+// per SM 6: 13.3 / 23.7 / 45.4 us, 5: 11.7 / 20.5 / 46.3, 4: 9.9 / 17.4 / 45.9).
 constexpr int kEmLoneThreads = 256;
 constexpr int kEmLoneLoads = 4;
 constexpr int kEmLoneSpan = 32 * kEmLoneLoads * 16;  // bytes of a row per warp: 16 of its scales
+constexpr int kEmLoneSmem = 46 * 1024;  // of the 228 KB of an SM, 1 KB more per CTA is the system's
 inline long long em_lone_ctas(const EmDispatchArgs& a) {
     const long long warps = (long long)a.num_tokens * ((a.hidden + kEmLoneSpan - 1) / kEmLoneSpan);
     return std::max(1ll, (warps + kEmLoneThreads / 32 - 1) / (kEmLoneThreads / 32));
@@ -379,8 +387,7 @@ __global__ void __launch_bounds__(kEmLoneThreads) em_dispatch_lone_kernel(const 
     const int n16 = H / 16, num_kb = H / 128, spans = (H + kEmLoneSpan - 1) / kEmLoneSpan;
     const long long item = (long long)blockIdx.x * (kEmLoneThreads / 32) + (tid >> 5);
     const int t = (int)(item / spans), span = (int)(item % spans);
-    const bool any = a.unit_start[E] > 0;  // (no units after an overflow)
-    if (t < T && any) {
+    if (t < T && a.unit_start[E] > 0) {  // (no units after an overflow)
         const int i0 = span * (kEmLoneSpan / 16) + lane, kb = span * (kEmLoneSpan / 128) + (lane & 15);
         const int4* src = reinterpret_cast<const int4*>(reinterpret_cast<const char*>(a.x) + (size_t)t * H) + i0;
         int4 v[kEmLoneLoads];
@@ -416,16 +423,12 @@ __global__ void __launch_bounds__(kEmLoneThreads) em_dispatch_lone_kernel(const 
             if (a.dst_row != nullptr) a.dst_row[t * K + lane] = row;
         }
     }
-    // The last CTA says what has arrived: whoever waits for these words finds every row in place, as behind the general kernel, whose units say it one by one.
-    if (any && cta_is_last(a.ctx.local_scratch + kTicketFused, gridDim.x))
-        for (int e = tid; e < E; e += kEmLoneThreads)
-            if (a.my_counts[e] > 0) red_add_release_gpu(&a.ctx.my_ctrl()->em_arrived[e], (uint64_t)a.my_counts[e]);
 }
 
 cudaError_t launch_em_dispatch(const EmDispatchArgs* a, int nv, cudaStream_t stream) {
     if (a[0].hidden % 128 != 0 || a[0].num_sms < 1) return cudaErrorInvalidValue;
     if (nv == 1 && a->ctx.num_ranks == 1 && a->num_sms >= 148 && a->places != nullptr && a->x_scales != nullptr && a->ctx.debug_extent == 0 && a->trace == nullptr)
-        return launch_dependent(em_dispatch_lone_kernel, dim3((unsigned)em_lone_ctas(*a)), kEmLoneThreads, 0, stream, *a);
+        return launch_dependent(em_dispatch_lone_kernel, dim3((unsigned)em_lone_ctas(*a)), kEmLoneThreads, kEmLoneSmem, stream, *a);
     const size_t smem = (size_t)(a[0].num_experts + 1) * sizeof(int);
     return DX_LAUNCH_RANKED_PDL(em_dispatch_kernel, EmDispatchArgs, a, nv, a[0].num_sms, kEmDispatchThreads, smem, stream);
 }

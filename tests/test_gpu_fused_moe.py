@@ -302,7 +302,7 @@ def test_places_are_kept_where_they_are_asked_for(T, H, E, K, native):
             dst = torch.full((T * K,), -1, dtype=torch.int32, device="cuda")
             C.em_dispatch([rt], [(q, w.my_counts, roomy, w.send_base, w.unit_start, w.peer_bases, dst, None, s, places)], E, K, UNIT_ROWS, native, native, 148 * 6)
             torch.cuda.synchronize()
-            assert torch.equal(w.arrived, w.expected) and (roomy[E * T:] == 7).all()
+            assert (roomy[E * T:] == 7).all()
             got.append([t.clone() for t in (w.recv_x.view(torch.uint8), w.recv_scales_raw, w.recv_info, dst)])
         vc.buffers[0].check_status()
         for other in got[1:]:
@@ -317,8 +317,9 @@ def test_places_are_kept_where_they_are_asked_for(T, H, E, K, native):
 
 
 @pytest.mark.parametrize("T,H,masked", [(1, 128, 0.0), (700, 4224, 0.05), (300, 7168, 1.0)])
-def test_lone_dispatches_in_a_row_count_their_arrivals(T, H, masked):
-    """One CTA to some hundred, none with a row to send: the last one of each call raises the words, and leaves the ticket that the exchange shares as it was."""
+def test_arrivals_of_a_lone_rank(T, H, masked):
+    """The dispatch with places counts no arrivals, so that nothing that waits for them reads early; the next exchange makes up for it, and a dispatch that does
+    count finds the words as if all calls had."""
     import deepep_efa_b200 as ep
     from deepep_efa_b200.models.moe import UNIT_ROWS
     E, K = 40, 3
@@ -328,17 +329,22 @@ def test_lone_dispatches_in_a_row_count_their_arrivals(T, H, masked):
         rt, w, idx = vc.buffers[0].runtime, layers[0].fused_workspace(T), idxs[0]
         q, s = C.per_token_cast_to_fp8(xs[0], False, False)
         counts = torch.bincount(idx[idx >= 0], minlength=E)
-        before = w.arrived.clone()
-        for _ in range(5):
+        due = w.arrived.clone()
+        assert torch.equal(due, w.expected)
+        for counted in (False, False, True, True, False, True):
+            places = None if counted else w.places
+            w.recv_x.view(torch.uint8).zero_()
             C.em_notify([rt], [(idx, w.recv_x, w.recv_scales_raw, w.recv_info, w.stage, w.my_counts, w.sel_list, w.send_base, w.unit_start, w.m_offsets,
-                                w.m_ends, w.peer_bases, w.places)], E, UNIT_ROWS)
-            C.em_dispatch([rt], [(q, w.my_counts, w.sel_list, w.send_base, w.unit_start, w.peer_bases, None, None, s, w.places)], E, K, UNIT_ROWS, False, False, 148)
-        torch.cuda.synchronize()
+                                w.m_ends, w.peer_bases, places)], E, UNIT_ROWS)
+            assert torch.equal(w.arrived, due) and torch.equal(w.expected, due + counts)
+            C.em_dispatch([rt], [(q, w.my_counts, w.sel_list, w.send_base, w.unit_start, w.peer_bases, None, None, s, places)], E, K, UNIT_ROWS, False, False, 148)
+            torch.cuda.synchronize()
+            assert torch.equal(w.arrived, due + counts if counted else due)
+            due += counts
+            for e in range(E):
+                toks = (idx == e).nonzero()[:, 0]
+                row = int(w.m_offsets[e])
+                assert torch.equal(w.recv_x[row:row + toks.numel()].view(torch.uint8), q.view(torch.uint8)[toks])
         vc.buffers[0].check_status()
-        assert torch.equal(w.arrived - before, 5 * counts) and torch.equal(w.arrived, w.expected)
-        for e in range(E):
-            toks = (idx == e).nonzero()[:, 0]
-            row = int(w.m_offsets[e])
-            assert torch.equal(w.recv_x[row:row + toks.numel()].view(torch.uint8), q.view(torch.uint8)[toks])
     finally:
         vc.destroy()
