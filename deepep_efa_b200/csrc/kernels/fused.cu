@@ -368,8 +368,10 @@ __global__ void __launch_bounds__(kEmDispatchThreads, 6) em_dispatch_kernel(cons
 // at the power limit, 4096 x 8 rows of 7 KB 96 -> 55. No CTA knows when an expert's rows are complete, so arrivals are not counted here: nothing on this GPU may
 // gate on them (a gate would run into its limit), and the next exchange makes up for it. Counted by the last CTA to finish, with a ticket, the kernel
 // itself took 11.4 -> 13.8 us with rows of 1 KB, 46.4 -> 47.8 with 7 KB.
-// Four CTAs share an SM, by shared memory that none of them uses: more of them write more rows at a time than the memory takes well (4096 x 8 rows of 1 / 2 / 7 KB, CTAs
-// per SM 6: 13.3 / 23.7 / 45.4 us, 5: 11.7 / 20.5 / 46.3, 4: 9.9 / 17.4 / 45.9).
+// With more than four places per token four CTAs share an SM instead of six, by shared memory that none of them uses: more write more rows at a time than the memory takes
+// well. With fewer places the loads want more of them. Exchange and dispatch, us, CTAs per SM 6 / 5 / 4 (rows x places of a size): 7000 x 2 of 2 KB 18.3 / 19.8 / 20.3, 4096 x 2
+// of 7 KB 24.3 / 24.9 / 26.1, 7000 x 4 of 2 KB 26.1 / 26.4 / 27.6; 2000 x 6 of 4 KB 26.2 / 25.4 / 22.9, 4096 x 8 of 1 KB 28.5 / 27.0 / 25.0, of 2 KB 39.8 / 36.7 / 33.0, of 7 KB
+// 60.9 / 61.7 / 61.6, 7000 x 8 of 2 KB 40.6 / 40.2 / 40.4.
 constexpr int kEmLoneThreads = 256;
 constexpr int kEmLoneLoads = 4;
 constexpr int kEmLoneSpan = 32 * kEmLoneLoads * 16;  // bytes of a row per warp: 16 of its scales
@@ -428,7 +430,7 @@ __global__ void __launch_bounds__(kEmLoneThreads) em_dispatch_lone_kernel(const 
 cudaError_t launch_em_dispatch(const EmDispatchArgs* a, int nv, cudaStream_t stream) {
     if (a[0].hidden % 128 != 0 || a[0].num_sms < 1) return cudaErrorInvalidValue;
     if (nv == 1 && a->ctx.num_ranks == 1 && a->num_sms >= 148 && a->places != nullptr && a->x_scales != nullptr && a->ctx.debug_extent == 0 && a->trace == nullptr)
-        return launch_dependent(em_dispatch_lone_kernel, dim3((unsigned)em_lone_ctas(*a)), kEmLoneThreads, kEmLoneSmem, stream, *a);
+        return launch_dependent(em_dispatch_lone_kernel, dim3((unsigned)em_lone_ctas(*a)), kEmLoneThreads, a->num_topk > 4 ? kEmLoneSmem : 0, stream, *a);
     const size_t smem = (size_t)(a[0].num_experts + 1) * sizeof(int);
     return DX_LAUNCH_RANKED_PDL(em_dispatch_kernel, EmDispatchArgs, a, nv, a[0].num_sms, kEmDispatchThreads, smem, stream);
 }
