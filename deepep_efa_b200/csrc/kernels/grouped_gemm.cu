@@ -73,11 +73,12 @@ __device__ __forceinline__ void store_block_coalesced(int4* stage, const int4 (&
 }
 
 // 32 rows x 32 BF16 columns, one row per lane, without shared memory: lanes 2i and 2i + 1 exchange halves, so that each store instruction writes 64
-// contiguous bytes of 16 rows. `gbase` and the row stride are multiples of 32 bytes.
-// Where the reduction is short the epilogue is the tile: through the staging buffer, with the group's table in global memory, a tile of 128 x 256 took 4500
-// cycles (20 to 94 rows per expert), now 3100. Both weight gradients of 64 experts of 4096 -> 1408 in a loop, us, before / with this, kTailRows and kWgrad: 20 rows
-// 559 / 440, 94 rows 623 / 490, 190 rows 753 / 663, 384 rows 1061 / 1025, on pairs 768 rows 1563 / 1484. Whole lines of 128 bytes by two exchanges are no faster (94 rows 343 / 343
-// for the first), neither are eight epilogue warps on alternate tiles (361 / 369) or columns read from TMEM ahead (343 / 398).
+// contiguous bytes of 16 rows. Every row's address is a multiple of 32 bytes, and the columns are stored at multiples of 16.
+// Where the reduction is short the epilogue is the tile: 4500 cycles for 128 x 256 outputs through the staging buffer of store_block_coalesced and with the group's
+// table in global memory (20 to 94 rows per expert), 3100 with these stores and the table in shared memory. Both weight gradients of 64 experts of 4096 -> 1408 in a
+// loop, us, before / with that and reductions that stop at the last row: 20 rows 559 / 453, 94 rows 623 / 538, 190 rows 753 / 671, 384 rows 1061 / 1041, on pairs 768 rows
+// 1563 / 1567 (what came since stands at kTailRows and kWgrad). Other forms of the store, the first of the two, 94 rows, us: these 343, whole lines of 128 bytes by two
+// exchanges 343, columns read from TMEM ahead 398.
 struct RowPair {
     __nv_bfloat16 *even, *odd;  // this lane's half of 32 columns of the rows of lanes 2i and 2i + 1 (nullptr: no such row)
     bool upper;
